@@ -138,9 +138,10 @@ size_t spc_rulebook_workspace_bytes(const spc_geometry* g, int64_t n_in);
  * gives the reference) and numbers them.  Writes the number of output rows
  * to *n_out_host after synchronising `stream` (subm: n_out = n_in, no
  * synchronisation).  n_out == 0 is the reference's "points vanished" case.
- * The synchronisation spins (cudaStreamSynchronize) unless the environment holds
- * SPC_HOST_WAIT=block when the first call is made: then the thread sleeps on a
- * blocking event, which suits processes with more waiting threads than cores. */
+ * The wait ends when the count has arrived, work queued after it may still run; it
+ * spins unless the environment holds SPC_HOST_WAIT=block when the first call is
+ * made: then the thread sleeps on a blocking event, which suits processes with
+ * more waiting threads than cores. */
 int spc_rulebook_prepare(const spc_geometry* g, const int32_t* indices, int64_t n_in,
                          void* workspace, size_t workspace_bytes, int64_t* n_out_host,
                          void* stream);
@@ -180,6 +181,21 @@ int spc_rulebook_igemm_backward(const spc_geometry* g, const int32_t* indices, i
                                 int32_t* pair_bwd, int32_t* mask_bwd, int32_t* argsort_bwd,
                                 const uint32_t* split_masks, int n_split, int do_sort,
                                 int32_t* pair_bwd_rowmajor, void* stream);
+
+/* Phase 2 for callers that run the GEMMs of this library and nothing else: the
+ * tables of spc_rulebook_igemm without the sorted masks, which only the reference's
+ * interface needs (they are the stable sort of the mask words of a row-major table,
+ * bit k of a row's word = entry k >= 0).  Every output may be NULL and is then not made.
+ *   order_fwd [n_out] / order_bwd [n_in] (kv <= 32): an order of the rows for the
+ *   `mask_argsort` argument of the GEMMs, in which the 128 rows of a tile share
+ *   kernel offsets; rows of the same offsets come in any order.
+ * The input side (pair_bwd, pair_bwd_rowmajor, order_bwd) exists for strided and
+ * transposed layers only; it may be asked for by a later call of its own with the
+ * same workspace. */
+int spc_rulebook_tables(const spc_geometry* g, const int32_t* indices, int64_t n_in, int64_t n_out,
+                        void* workspace, size_t workspace_bytes, int32_t* out_indices,
+                        int32_t* pair_fwd, int32_t* pair_fwd_rowmajor, int32_t* order_fwd,
+                        int32_t* pair_bwd, int32_t* pair_bwd_rowmajor, int32_t* order_bwd, void* stream);
 
 /* Row-major copy [n, kvp] of a pair table [kv, n] that was not produced by
  * spc_rulebook_igemm (tables converted from the Native format, user tables). */
@@ -481,17 +497,8 @@ typedef struct {
                                             rulebook reads it (spc_conv_forward_needs_colmajor): it is
                                             the transpose of pair_fwd_rowmajor[:, :kv] */
   uint64_t pair_fwd_rowmajor;            /* [n_out, kvp] int32 */
-  uint64_t pair_mask;                    /* [n_out] int32 (one split, one word) */
-  uint64_t mask_argsort;                 /* [n_out] int32 */
-  uint64_t num_per_loc;                  /* [kv] int32, zeros (as igemm_pairs returns) */
+  uint64_t mask_argsort;                 /* [n_out] int32: the order of spc_rulebook_tables */
   uint64_t features;                     /* [n_out, c_out], dtype */
-  int64_t masks_are_exact;               /* 1: pair_mask / mask_argsort are what spc_rulebook_igemm emits (the
-                                            mask words sorted ascending, stable, and their argsort); 0: the pass
-                                            ordered the rows for its own GEMMs by a key that packs rows with
-                                            common kernel offsets into the same 128-row tile: mask_argsort is
-                                            that order, pair_mask the sorted keys, and the exact pair is the
-                                            stable sort of the mask words of pair_fwd_rowmajor (bit k of a
-                                            row's word = entry k >= 0) */
 } spc_seq_result;
 
 /* Inference forward of `n_layers` convolutions applied one after the other to

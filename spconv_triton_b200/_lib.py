@@ -104,6 +104,7 @@ _PROTOTYPES = {
     "spc_voxelize": (c_int, [_P, c_int64, c_int, c_int, c_int, POINTER(ctypes.c_float), POINTER(ctypes.c_float),
                              POINTER(ctypes.c_int32), c_int64, c_int, c_int, c_int, _P, c_size_t, _P, _P, _P, _P,
                              POINTER(c_int64), _P]),
+    "spc_rulebook_tables": (c_int, [POINTER(Geometry), _P, c_int64, c_int64, _P, c_size_t] + [_P] * 8),
     "spc_rulebook_native": (c_int, [POINTER(Geometry), _P, c_int64, c_int64, _P, c_size_t, _P, _P, _P, _P]),
     "spc_native_to_tables": (c_int, [_P, c_int, c_int64, c_int, _P, c_int64, _P, c_int64, _P]),
     "spc_conv_forward": (c_int, [_P, _P, _P, _P, _P, _P, _P, c_int64, c_int64, c_int, c_int, c_int, c_int, c_int,

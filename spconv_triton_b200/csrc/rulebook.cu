@@ -14,9 +14,9 @@
 // output coordinates, which reproduces the ascending row numbering that
 // torch.unique gives the reference.
 #include <cub/device/device_radix_sort.cuh>
-#include <cub/device/device_scan.cuh>
 
 #include <algorithm>
+#include <atomic>
 #include <climits>
 #include <type_traits>
 
@@ -26,6 +26,7 @@
 #include "common.cuh"
 #include "gemm_internal.cuh"
 #include "rulebook_internal.cuh"
+#include "tile_order.cuh"
 
 namespace spc {
 namespace {
@@ -36,27 +37,11 @@ struct Geo {
   int ndim, batch, subm, transpose, kv;
   int in_shape[SPC_MAX_NDIM], out_shape[SPC_MAX_NDIM];
   int ksize[SPC_MAX_NDIM], stride[SPC_MAX_NDIM], pad[SPC_MAX_NDIM], dil[SPC_MAX_NDIM];
-  // Tile key (kv <= 32 only, off unless a caller of rulebook_igemm_chained asks for it): the mask
-  // sort then orders the rows by a transformed mask word instead of the word itself, see below.
-  int tile_key;
-  unsigned char key_pos[32];  // bit k of the mask word goes to bit key_pos[k] of the key
+  int shift[SPC_MAX_NDIM];    // log2 of a stride that is a power of two, else -1
+  int axes_fit;               // every axis has at most 32 offsets: the valid ones are a bitmask
+  int window;                 // the cells of a line of offsets lie in one 64-bit window of the occupancy bitmap
+  unsigned char key_pos[32];  // bit k of the mask word goes to bit key_pos[k] of the tile-order word (kv <= 32)
 };
-
-// The order the gather-GEMM wants is not the numeric order of the mask words but one in which the
-// 128 rows of a tile share as many kernel offsets as possible.  Two cheap changes to the sort key
-// get most of what a data-dependent order would: the offsets far from the kernel's centre (the
-// corners of the window, the rarest in surface-like data) become the most significant bits, so that
-// rows are grouped by their rare offsets first, and the key is Gray-decoded, so that neighbouring
-// keys (hence neighbouring tiles) differ in few offsets.  On the VoxelNet-style backbone: 6 - 9 % fewer
-// (tile, offset) stages on the submanifold levels, 2 - 16 % on the strided ones.
-__device__ __forceinline__ uint32_t gray_decode(uint32_t key) {
-  key ^= key >> 1;
-  key ^= key >> 2;
-  key ^= key >> 4;
-  key ^= key >> 8;
-  key ^= key >> 16;
-  return key;
-}
 
 // ------------------------------------------------------------------------
 // Hash tables.  K64 = false: key < 2^31, slot = (key << 32) | value in one
@@ -88,11 +73,10 @@ struct Table<false> {
   uint32_t* obits = nullptr;
   const uint32_t* oprefix = nullptr;
   // Input side: rows equal ranks only when the rows came in ascending key order (the outputs of an
-  // earlier layer do); `unsorted` points at a device flag that says they did not.
+  // earlier layer do); where `unsorted` points at a device flag that says they did not, row = perm[rank].
   const int* unsorted = nullptr;
-  __device__ __forceinline__ bool ranked() const {
-    return obits != nullptr && (unsorted == nullptr || *unsorted == 0);
-  }
+  const int32_t* perm = nullptr;
+  __device__ __forceinline__ bool permuted() const { return unsorted != nullptr && *unsorted != 0; }
   __device__ __forceinline__ int rank_of(key_t key) const {
     const uint32_t w = __ldg(&obits[key >> 5]);
     if (!((w >> (key & 31u)) & 1u)) return -1;
@@ -136,7 +120,10 @@ struct Table<false> {
     return -1;
   }
   __device__ int find(key_t key) const {
-    if (ranked()) return rank_of(key);
+    if (obits != nullptr) {
+      const int rank = rank_of(key);
+      return rank >= 0 && permuted() ? __ldg(&perm[rank]) : rank;
+    }
     uint32_t s = home(key);
     for (uint32_t probe = 0; probe <= (cap_mask >> 2); ++probe) {
       const unsigned long long v = __ldg(&slots[s]);
@@ -348,37 +335,97 @@ __device__ __forceinline__ void delinearize_out(const Geo& g, long long lin, int
   c[0] = static_cast<int>(lin);
 }
 
-enum Counter { kUniqueCount = 0, kStatus = 1, kUnsorted = 2 };
+enum Counter { kUniqueCount = 0, kStatus = 1, kUnsorted = 2, kTicket = 3 };
 
 // ------------------------------------------------------------------------
 // Phase 1 kernels
 // ------------------------------------------------------------------------
-template <int ND, bool K64>
-__global__ void __launch_bounds__(kThreads)
-insert_inputs_kernel(const __grid_constant__ Geo g, const int32_t* __restrict__ idx, long long n,
-                     Table<K64> tin, int* counters, uint32_t* __restrict__ bitmap, int* dev_status) {
-  const long long j = blockIdx.x * static_cast<long long>(kThreads) + threadIdx.x;
-  if (j >= n) return;
-  if (bitmap != nullptr && counters[kUnsorted] == 0) return;  // rows are ranks of the bitmap
-  int c[ND + 1];
-  load_coord<ND>(idx, j, c);
-  if (!coord_in_grid<ND>(g, c)) {
-    flag_bad_row(counters, dev_status);
-    return;
+// Scratch regions are cleared by a kernel rather than by cudaMemsetAsync, and all of them by one launch: a
+// kernel can neither be routed to a copy engine (where it would queue behind a large transfer of the
+// application) nor cost a driver memset's set-up.  Regions are 16-byte multiples at 16-byte offsets.
+struct Clear {
+  static constexpr int kMost = 8;
+  uint4* at[kMost];
+  long long n16[kMost];
+  uint32_t word[kMost];
+  int n = 0;
+  long long total = 0;
+  void add(void* p, int byte, size_t bytes) {
+    if (bytes == 0) return;
+    at[n] = static_cast<uint4*>(p);
+    n16[n] = static_cast<long long>((bytes + 15) / 16);
+    word[n] = 0x01010101u * (static_cast<uint32_t>(byte) & 0xffu);
+    total += n16[n++];
   }
-  using key_t = typename Table<K64>::key_t;
-  const long long key = in_key_of<ND>(g, c);
-  if (!tin.insert_min(static_cast<key_t>(key), static_cast<uint32_t>(j)))
-    atomicExch(&counters[kStatus], SPC_ERR_HASH_TABLE_FULL);
+};
+__global__ void __launch_bounds__(256) clear_kernel(const __grid_constant__ Clear c) {
+  const long long stride = static_cast<long long>(gridDim.x) * 256;
+  for (int s = 0; s < c.n; ++s) {
+    const uint4 v = make_uint4(c.word[s], c.word[s], c.word[s], c.word[s]);
+    uint4* __restrict__ dst = c.at[s];
+    for (long long i = blockIdx.x * 256ll + threadIdx.x; i < c.n16[s]; i += stride) dst[i] = v;
+  }
 }
 
-// With a bitmap of the input grid: sets the bit of every input cell and notes whether the rows are in
-// strictly ascending key order.  If they are, a row number is the rank of its bit and the hash table
-// is not needed (insert_inputs_kernel then returns at once).
-template <int ND>
+__device__ __forceinline__ uint32_t* dense_bits(const Table<false>& t) { return t.obits; }
+__device__ __forceinline__ uint32_t* dense_bits(const Table<true>&) { return nullptr; }
+__device__ __forceinline__ const uint32_t* dense_prefix(const Table<false>& t) { return t.oprefix; }
+__device__ __forceinline__ const uint32_t* dense_prefix(const Table<true>&) { return nullptr; }
+__device__ __forceinline__ const int32_t* row_permutation(const Table<false>& t) { return t.permuted() ? t.perm : nullptr; }
+__device__ __forceinline__ const int32_t* row_permutation(const Table<true>&) { return nullptr; }
+
+__device__ __forceinline__ void set_bit(uint32_t* bits, long long cell) {
+  uint32_t* word = bits + (cell >> 5);
+  const uint32_t bit = 1u << (cell & 31);
+  if (!(*word & bit)) atomicOr(word, bit);
+}
+
+// The cells an own coordinate meets along axis d: `div` = the cell is what this coordinate was reached from
+// ((own + pad - k * dil) / stride, if that divides), else own * stride - pad + k * dil.
+// Returns -1 where there is none.
+__device__ __forceinline__ int axis_cell(const Geo& g, bool div, int d, int own, int k, int limit) {
+  int x;
+  if (div) {
+    x = own + g.pad[d] - k * g.dil[d];
+    if (x < 0) return -1;
+    if (g.shift[d] >= 0) {
+      if (x & ((1 << g.shift[d]) - 1)) return -1;
+      x >>= g.shift[d];
+    } else {
+      const int q = x / g.stride[d];
+      if (q * g.stride[d] != x) return -1;
+      x = q;
+    }
+  } else {
+    x = own * g.stride[d] - g.pad[d] + k * g.dil[d];
+  }
+  return x >= 0 && x < limit ? x : -1;
+}
+
+// The bits of every output cell an input row reaches.  Per axis only the kernel offsets that land on an
+// output coordinate are kept (a bitmask over the offsets of that axis: with stride 2 and a 3-wide kernel
+// one or two of three), and the cells are the product of the axes, so a k3 s2 layer visits at most 8
+// candidates per input instead of testing all 27.
+template <int D, int ND>
+__device__ __forceinline__ void mark_cells(const Geo& g, const int* c, const uint32_t* mask, long long lin,
+                                           uint32_t* __restrict__ bits) {
+  if constexpr (D == ND) {
+    set_bit(bits, lin);
+  } else {
+    for (uint32_t m = mask[D]; m != 0; m &= m - 1)
+      mark_cells<D + 1, ND>(g, c, mask,
+                            lin * g.out_shape[D] + axis_cell(g, !g.transpose, D, c[D + 1], __ffs(m) - 1, g.out_shape[D]), bits);
+  }
+}
+
+// First pass over the input rows: checks them, enters them into the input table (`in_bits`: the bit of the
+// cell, noting whether the rows are in strictly ascending key order; else the hash table, if `insert`) and,
+// with `out_bits`, marks the output cells.  One pass instead of one each: the coordinates are read once and
+// a small rulebook is three launches shorter.
+template <int ND, bool K64>
 __global__ void __launch_bounds__(kThreads)
-mark_inputs_kernel(const __grid_constant__ Geo g, const int32_t* __restrict__ idx, long long n,
-                   uint32_t* __restrict__ bitmap, int* counters, int* dev_status) {
+ingest_kernel(const __grid_constant__ Geo g, const int32_t* __restrict__ idx, long long n, Table<K64> tin, int insert,
+              uint32_t* __restrict__ in_bits, uint32_t* __restrict__ out_bits, int* counters, int* dev_status) {
   const long long j = blockIdx.x * static_cast<long long>(kThreads) + threadIdx.x;
   if (j >= n) return;
   int c[ND + 1];
@@ -389,102 +436,200 @@ mark_inputs_kernel(const __grid_constant__ Geo g, const int32_t* __restrict__ id
     return;
   }
   const long long key = in_key_of<ND>(g, c);
-  atomicOr(&bitmap[key >> 5], 1u << (key & 31));
-  if (j > 0) {
-    load_coord<ND>(idx, j - 1, c);
-    if (in_key_of<ND>(g, c) >= key) counters[kUnsorted] = 1;
-  }
-}
-
-// One thread per input row walks the kv offsets and inserts each candidate
-// output coordinate into the output table.  Offsets are handled in groups of
-// 32: a thread remembers in a bitmask which of its candidates were first-time
-// inserts, the warp reserves room for all of them in `uniq` with ONE atomicAdd
-// per group (a per-insert counter serialises on a single address), and a
-// second walk over the group writes the keys.
-__device__ __forceinline__ uint32_t* dense_bits(const Table<false>& t) { return t.obits; }
-__device__ __forceinline__ uint32_t* dense_bits(const Table<true>&) { return nullptr; }
-
-__device__ __forceinline__ bool table_ranked(const Table<false>& t) { return t.ranked(); }
-__device__ __forceinline__ bool table_ranked(const Table<true>&) { return false; }
-__device__ __forceinline__ uint32_t rank_prefix(const Table<false>& t, long long key) { return __ldg(&t.oprefix[key >> 5]); }
-__device__ __forceinline__ uint32_t rank_prefix(const Table<true>&, long long) { return 0; }
-
-// Dense numbering, step 2: set bits per word (scanned in place afterwards).
-__global__ void __launch_bounds__(kThreads)
-count_bits_kernel(const uint32_t* __restrict__ bits, long long words, uint32_t* __restrict__ counts) {
-  const long long i = blockIdx.x * static_cast<long long>(kThreads) + threadIdx.x;
-  if (i < words) counts[i] = __popc(bits[i]);
-}
-
-// Dense numbering, step 3: the keys of the set bits in ascending order, and their total.
-__global__ void __launch_bounds__(kThreads)
-expand_bits_kernel(const uint32_t* __restrict__ bits, const uint32_t* __restrict__ prefix, long long words,
-                   long long limit, uint32_t* __restrict__ sorted, int* counters) {
-  const long long i = blockIdx.x * static_cast<long long>(kThreads) + threadIdx.x;
-  if (i >= words) return;
-  uint32_t w = bits[i];
-  long long at = prefix[i];
-  if (i == words - 1) counters[kUniqueCount] = static_cast<int>(at + __popc(w));
-  while (w != 0 && at < limit) {
-    const int b = __ffs(w) - 1;
-    sorted[at++] = static_cast<uint32_t>(i * 32 + b);
-    w &= w - 1;
-  }
-}
-
-// Dense numbering, step 1: the bits of every output cell an input row reaches.  Per axis only the
-// kernel offsets that land on an output coordinate are kept (a bitmask over the offsets of that axis:
-// with stride 2 and a 3-wide kernel one or two of three), and the cells are the product of the axes,
-// so a k3 s2 layer visits at most 8 candidates per input instead of testing all 27.
-template <int D, int ND>
-__device__ __forceinline__ void mark_cells(const Geo& g, const int* c, const uint32_t* mask, long long lin,
-                                           uint32_t* __restrict__ bits) {
-  if constexpr (D == ND) {
-    uint32_t* word = bits + (lin >> 5);
-    const uint32_t bit = 1u << (lin & 31);
-    if (!(*word & bit)) atomicOr(word, bit);
-  } else {
-    for (uint32_t m = mask[D]; m != 0; m &= m - 1) {
-      const int k = __ffs(m) - 1;
-      const int o = g.transpose ? c[D + 1] * g.stride[D] + k * g.dil[D] - g.pad[D]
-                                : (c[D + 1] + g.pad[D] - k * g.dil[D]) / g.stride[D];
-      mark_cells<D + 1, ND>(g, c, mask, lin * g.out_shape[D] + o, bits);
+  if (in_bits != nullptr) {
+    set_bit(in_bits, key);
+    if (j > 0) {
+      int p[ND + 1];
+      load_coord<ND>(idx, j - 1, p);
+      if (in_key_of<ND>(g, p) >= key) counters[kUnsorted] = 1;
     }
+  } else if (insert) {
+    using key_t = typename Table<K64>::key_t;
+    if (!tin.insert_min(static_cast<key_t>(key), static_cast<uint32_t>(j)))
+      atomicExch(&counters[kStatus], SPC_ERR_HASH_TABLE_FULL);
   }
-}
-
-template <int ND>
-__global__ void __launch_bounds__(kThreads)
-mark_outputs_kernel(const __grid_constant__ Geo g, const int32_t* __restrict__ idx, long long n,
-                    uint32_t* __restrict__ bits) {
-  const long long j = blockIdx.x * static_cast<long long>(kThreads) + threadIdx.x;
-  if (j >= n) return;
-  int c[ND + 1];
-  load_coord<ND>(idx, j, c);
-  if (!coord_in_grid<ND>(g, c)) return;  // recorded by the input pass
+  if (out_bits == nullptr) return;
   uint32_t mask[ND];
 #pragma unroll
   for (int d = 0; d < ND; ++d) {
     uint32_t m = 0;
-    for (int k = 0; k < g.ksize[d]; ++k) {
-      int o;
-      if (g.transpose) {
-        o = c[d + 1] * g.stride[d] + k * g.dil[d] - g.pad[d];
-      } else {
-        const int num = c[d + 1] + g.pad[d] - k * g.dil[d];
-        if (num < 0) continue;
-        o = num / g.stride[d];
-        if (o * g.stride[d] != num) continue;
-      }
-      if (o >= 0 && o < g.out_shape[d]) m |= 1u << k;
-    }
+    for (int k = 0; k < g.ksize[d]; ++k)
+      m |= static_cast<uint32_t>(axis_cell(g, !g.transpose, d, c[d + 1], k, g.out_shape[d]) >= 0) << k;
     if (m == 0) return;
     mask[d] = m;
   }
-  mark_cells<0, ND>(g, c, mask, c[0], bits);
+  mark_cells<0, ND>(g, c, mask, c[0], out_bits);
 }
 
+// ------------------------------------------------------------------------
+// Numbering the set bits of the input and the output bitmap in ascending cell order.  A block owns 4096
+// words.  count_cells_kernel adds up every block's bits; its last block to finish turns the sums into
+// starts and hands the output count to the host, which can then allocate while number_cells_kernel gives
+// every word the number of bits before it and lists the output cells.  (A library scan over the words plus
+// separate counting, listing and publishing kernels was five launches more per bitmap.)
+// ------------------------------------------------------------------------
+constexpr int kCellBlock = 4096;
+constexpr int kWordsPerThread = kCellBlock / kThreads;
+
+struct Cells {
+  const uint32_t* bits[2];  // input, output (null: not there)
+  uint32_t* prefix[2];
+  uint32_t* starts[2];      // per block: its bits, then the bits before it; one more entry for the total
+  long long words[2];
+  int blocks[2];
+};
+
+// counters[kUniqueCount], counters[kStatus] and the device status word -> page-locked host memory; the
+// ticket last, so that a host that sees it sees the rest.
+__device__ void publish(const int* counters, const int* dev_status, volatile int* host_box, int ticket) {
+  host_box[1] = counters[kUniqueCount];
+  host_box[2] = counters[kStatus];
+  host_box[3] = dev_status != nullptr ? *dev_status : 0;
+  __threadfence_system();
+  host_box[0] = ticket;
+}
+__global__ void publish_counters_kernel(const int* counters, const int* dev_status, int* host_box, int ticket) {
+  if (threadIdx.x == 0) publish(counters, dev_status, host_box, ticket);
+}
+
+__device__ __forceinline__ uint32_t block_exclusive_sum(uint32_t v, uint32_t* warp_sums, uint32_t* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t incl = v;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += t;
+  }
+  __syncthreads();  // warp_sums may still be read from a previous call
+  if (lane == 31) warp_sums[warp] = incl;
+  __syncthreads();
+  uint32_t before = 0, all = 0;
+#pragma unroll
+  for (int w = 0; w < kThreads / 32; ++w) {
+    if (w < warp) before += warp_sums[w];
+    all += warp_sums[w];
+  }
+  *total = all;
+  return before + incl - v;
+}
+
+__global__ void __launch_bounds__(kThreads)
+count_cells_kernel(const __grid_constant__ Cells c, int* counters, const int* dev_status, int* host_box, int ticket) {
+  __shared__ uint32_t warp_sums[kThreads / 32];
+  __shared__ int last;
+  const int side = blockIdx.x < static_cast<unsigned>(c.blocks[0]) ? 0 : 1;
+  const int block = blockIdx.x - (side ? c.blocks[0] : 0);
+  const uint32_t* bits = c.bits[side];
+  const long long first = static_cast<long long>(block) * kCellBlock;
+  uint32_t sum = 0;
+#pragma unroll
+  for (int i = 0; i < kWordsPerThread; ++i) {
+    const long long w = first + i * kThreads + threadIdx.x;
+    if (w < c.words[side]) sum += __popc(bits[w]);
+  }
+  uint32_t total;
+  block_exclusive_sum(sum, warp_sums, &total);
+  if (threadIdx.x == 0) {
+    c.starts[side][block] = total;
+    __threadfence();
+    last = atomicAdd(&counters[kTicket], 1) == static_cast<int>(gridDim.x) - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int s = 0; s < 2; ++s) {
+    volatile uint32_t* starts = c.starts[s];
+    uint32_t carry = 0;
+    for (int b0 = 0; b0 < c.blocks[s]; b0 += kThreads) {
+      const int b = b0 + threadIdx.x;
+      const uint32_t v = b < c.blocks[s] ? starts[b] : 0u;
+      uint32_t all;
+      const uint32_t before = block_exclusive_sum(v, warp_sums, &all);
+      if (b < c.blocks[s]) starts[b] = carry + before;
+      carry += all;
+    }
+    if (threadIdx.x == 0 && c.blocks[s] != 0) {
+      starts[c.blocks[s]] = carry;
+      if (s == 1) counters[kUniqueCount] = static_cast<int>(carry);
+    }
+  }
+  if (threadIdx.x == 0 && host_box != nullptr) {
+    __threadfence();
+    publish(counters, dev_status, host_box, ticket);
+  }
+}
+
+__global__ void __launch_bounds__(kThreads)
+number_cells_kernel(const __grid_constant__ Cells c, long long limit, uint32_t* __restrict__ sorted) {
+  __shared__ uint32_t warp_sums[kThreads / 32];
+  const int side = blockIdx.x < static_cast<unsigned>(c.blocks[0]) ? 0 : 1;
+  const int block = blockIdx.x - (side ? c.blocks[0] : 0);
+  const uint32_t start = c.starts[side][block];
+  if (c.starts[side][block + 1] == start) return;  // an empty block: nobody asks for the prefix of a zero word
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t* bits = c.bits[side];
+  uint32_t* prefix = c.prefix[side];
+  const long long first = static_cast<long long>(block) * kCellBlock + warp * (kCellBlock / (kThreads / 32)) + lane;
+  uint32_t word[kWordsPerThread], sum = 0;
+#pragma unroll
+  for (int i = 0; i < kWordsPerThread; ++i) {
+    const long long w = first + i * 32;
+    word[i] = w < c.words[side] ? bits[w] : 0u;
+    sum += __popc(word[i]);
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+  if (lane == 0) warp_sums[warp] = sum;
+  __syncthreads();
+  uint32_t at = start;
+  for (int w = 0; w < warp; ++w) at += warp_sums[w];
+#pragma unroll
+  for (int i = 0; i < kWordsPerThread; ++i) {
+    const uint32_t mine = __popc(word[i]);
+    uint32_t incl = mine;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, off);
+      if (lane >= off) incl += t;
+    }
+    const uint32_t before = at + incl - mine;
+    at += __shfl_sync(0xffffffffu, incl, 31);
+    if (word[i] != 0) prefix[first + i * 32] = before;
+    if (side == 0) continue;
+    // the warp lists one word's cells at a time: consecutive lanes write consecutive entries
+    unsigned some = __ballot_sync(0xffffffffu, word[i] != 0);
+    while (some != 0) {
+      const int src = __ffs(some) - 1;
+      some &= some - 1;
+      const uint32_t w = __shfl_sync(0xffffffffu, word[i], src);
+      const uint32_t to = __shfl_sync(0xffffffffu, before, src) + __popc(w & ((1u << lane) - 1u));
+      if (((w >> lane) & 1u) && to < limit)
+        sorted[to] = static_cast<uint32_t>((first - lane + i * 32 + src) * 32 + lane);
+    }
+  }
+}
+
+// perm[rank of a row's cell] = the row (the lowest one of equal coordinates, as a stable sort and a lower
+// bound give in the reference), where the rows did not come in ascending order.
+template <int ND>
+__global__ void __launch_bounds__(kThreads)
+permute_rows_kernel(const __grid_constant__ Geo g, const int32_t* __restrict__ idx, long long n, Table<false> tin,
+                    int32_t* __restrict__ perm) {
+  if (!tin.permuted()) return;
+  const long long j = blockIdx.x * static_cast<long long>(kThreads) + threadIdx.x;
+  if (j >= n) return;
+  int c[ND + 1];
+  load_coord<ND>(idx, j, c);
+  if (!coord_in_grid<ND>(g, c)) return;
+  atomicMin(&perm[tin.rank_of(static_cast<uint32_t>(in_key_of<ND>(g, c)))], static_cast<int32_t>(j));
+}
+
+// One thread per input row walks the kv offsets and inserts each candidate
+// output coordinate into the output table (grids too large for a bitmap).  Offsets are handled in groups of
+// 32: a thread remembers in a bitmask which of its candidates were first-time
+// inserts, the warp reserves room for all of them in `uniq` with ONE atomicAdd
+// per group (a per-insert counter serialises on a single address), and a
+// second walk over the group writes the keys.
 template <int ND, bool K64>
 __global__ void __launch_bounds__(kThreads)
 enumerate_outputs_kernel(const __grid_constant__ Geo g, const int32_t* __restrict__ idx, long long n,
@@ -509,9 +654,7 @@ enumerate_outputs_kernel(const __grid_constant__ Geo g, const int32_t* __restric
         const long long key = out_key_from_input<ND>(g, c, od.pos);
         if (key >= 0) {
           if (dense_bits(tout) != nullptr) {
-            uint32_t* word = dense_bits(tout) + (key >> 5);
-            const uint32_t bit = 1u << (key & 31);
-            if (!(*word & bit)) atomicOr(word, bit);
+            set_bit(dense_bits(tout), key);
           } else {
             const int r = tout.insert_unique(static_cast<key_t>(key));
             if (r < 0) atomicExch(&counters[kStatus], SPC_ERR_HASH_TABLE_FULL);
@@ -544,17 +687,6 @@ enumerate_outputs_kernel(const __grid_constant__ Geo g, const int32_t* __restric
   }
 }
 
-// counters[kUniqueCount], counters[kStatus] and the device status word -> page-locked host memory.
-__global__ void publish_counters_kernel(const int* __restrict__ counters, const int* __restrict__ dev_status,
-                                        int* __restrict__ host_box) {
-  if (threadIdx.x == 0) {
-    host_box[0] = counters[0];
-    host_box[1] = counters[1];
-    host_box[2] = dev_status != nullptr ? *dev_status : 0;
-    __threadfence_system();
-  }
-}
-
 template <bool K64>
 __global__ void __launch_bounds__(kThreads)
 assign_ranks_kernel(Table<K64> tout, const typename Table<K64>::key_t* __restrict__ sorted,
@@ -566,269 +698,297 @@ assign_ranks_kernel(Table<K64> tout, const typename Table<K64>::key_t* __restric
 // ------------------------------------------------------------------------
 // Phase 2 kernels (implicit-gemm tables)
 // ------------------------------------------------------------------------
-// Column r of pair_fwd: for each offset the input row that feeds output row r.
-// SUBM_BWD additionally writes pair_bwd, which for a submanifold layer is
-// pair_fwd with the offset axis reversed (offset k seen from the input side is
-// offset kv-1-k seen from the output side).
-template <int ND, bool K64, bool SUBM_BWD>
-__global__ void __launch_bounds__(kThreads)
-fill_fwd_kernel(const __grid_constant__ Geo g, const int32_t* __restrict__ idx,
-                const typename Table<K64>::key_t* __restrict__ sorted_out, long long n_out,
-                Table<K64> tin, int32_t* __restrict__ out_indices, int32_t* __restrict__ pair_fwd,
-                int32_t* __restrict__ pair_bwd, uint32_t* __restrict__ words, int mic,
-                int32_t* __restrict__ fwd_rm, int32_t* __restrict__ bwd_rm, int kvp,
-                const uint32_t* __restrict__ bitmap, int32_t* __restrict__ iota, int staged) {
-  using key_t = typename Table<K64>::key_t;
-  const long long r = blockIdx.x * static_cast<long long>(kThreads) + threadIdx.x;
-  // Row-major copies: a thread owns one row of kvp entries, so direct stores are 16 (or 4) bytes at
-  // a stride of kvp * 4 bytes -- a warp-wide store then touches 32 sectors and writes half (an
-  // eighth) of each.  With `staged` the warp collects its 32 rows in shared memory and writes the
-  // 32 * kvp * 4 contiguous bytes with full 16-byte-per-lane stores.
-  extern __shared__ int32_t stage_s[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int32_t* tile_f = stage_s + static_cast<size_t>(warp) * (SUBM_BWD ? 2 : 1) * 32 * kvp;
-  int32_t* tile_b = tile_f + 32 * kvp;
-  const bool live = r < n_out;
-  if (live) {
-  if (iota != nullptr) iota[r] = static_cast<int32_t>(r);  // the values the mask sort permutes
-  int o[ND + 1];
-  int quad[4] = {-1, -1, -1, -1};  // four consecutive offsets of the row-major copy
-  bool row_ok = true;
-  if (g.subm) {
-    load_coord<ND>(idx, r, o);
-    row_ok = coord_in_grid<ND>(g, o);  // a row outside the grid gets no pairs
-  } else {
-    delinearize_out<ND>(g, static_cast<long long>(sorted_out[r]), o);
-#pragma unroll
-    for (int d = 0; d <= ND; ++d) out_indices[r * (ND + 1) + d] = o[d];
-  }
-  Odometer<ND> od;
-  od.reset();
-  uint32_t word = 0;
-  // Non-transposed layers: the input cell of offset (p_0, .., p_last) is base + sum p_d * step_d, and
-  // whether it lies inside the grid is one bit per dimension; both are set up once per row so that
-  // the loop over the kv offsets does no coordinate arithmetic.
-  bool fast = !g.transpose;
-  long long base = o[0];
-  long long step[ND];
-  uint32_t inside[ND];
-  if (fast) {
-    long long mult = 1;
-#pragma unroll
-    for (int d = ND - 1; d >= 0; --d) {
-      step[d] = mult * g.dil[d];
-      mult *= g.in_shape[d];
-      if (g.ksize[d] > 32) fast = false;
-    }
-  }
-  if (fast) {
-#pragma unroll
-    for (int d = 0; d < ND; ++d) {
-      const int x0 = o[d + 1] * g.stride[d] - g.pad[d];
-      base = base * g.in_shape[d] + x0;
-      uint32_t m = 0;
-      for (int q = 0; q < g.ksize[d]; ++q) {
-        const int x = x0 + q * g.dil[d];
-        m |= static_cast<uint32_t>(x >= 0 && x < g.in_shape[d]) << q;
-      }
-      inside[d] = m;
-    }
-  }
-  // rows in ascending key order: a neighbour's row is the rank of its bit (one load of the word's prefix)
-  const bool ranked = bitmap != nullptr && table_ranked(tin);
-  // what is written for offset k once its input row j (-1: none) is known
-  auto emit = [&](int k, int j) {
-    if (pair_fwd != nullptr) pair_fwd[static_cast<long long>(k) * n_out + r] = j;
-    if (SUBM_BWD) {
-      pair_bwd[static_cast<long long>(g.kv - 1 - k) * n_out + r] = j;
-      if (bwd_rm != nullptr) {
-        if (staged) tile_b[lane * kvp + (g.kv - 1 - k)] = j;
-        else bwd_rm[r * kvp + (g.kv - 1 - k)] = j;
-      }
-    }
-    if (fwd_rm != nullptr) {
-      if (staged) {
-        tile_f[lane * kvp + k] = j;
-      } else {
-        quad[k & 3] = j;
-        if ((k & 3) == 3 || k == g.kv - 1) {
-          *reinterpret_cast<int4*>(&fwd_rm[r * kvp + (k & ~3)]) = make_int4(quad[0], quad[1], quad[2], quad[3]);
-          quad[0] = quad[1] = quad[2] = quad[3] = -1;
-        }
-      }
-    }
-    // with the tile key the bit goes straight to its place in the key (single word)
-    word |= static_cast<uint32_t>(j >= 0) << (g.tile_key ? g.key_pos[k] : (k & 31));
-    if ((k & 31) == 31 || k == g.kv - 1) {
-      words[r * mic + (k >> 5)] = g.tile_key ? gray_decode(word) : word;
-      word = 0;
-    }
-  };
-  const int kl = g.ksize[ND - 1];
-  if (fast && row_ok && bitmap != nullptr && g.dil[ND - 1] == 1) {
-    // Window path.  The kl offsets along the last axis are kl consecutive cells, i.e. consecutive
-    // bits of the occupancy bitmap: one (at a word boundary two) loads test all of them, and in
-    // ranked mode one prefix load numbers all of them, since the prefix of the next word is this
-    // word's prefix plus its population count.  A scattered load costs an L1 wavefront per lane, so
-    // 2-3 loads per axis line instead of one or two per offset is what this kernel's time follows.
-    const uint32_t in_mask = inside[ND - 1] & (kl >= 32 ? 0xffffffffu : ((1u << kl) - 1u));
-    for (int k0 = 0; k0 < g.kv; k0 += kl) {
-      uint32_t ok = in_mask != 0;
-      long long kk = base;
-#pragma unroll
-      for (int d = 0; d < ND - 1; ++d) {
-        ok &= inside[d] >> od.pos[d];
-        kk += od.pos[d] * step[d];
-      }
-      uint32_t present = 0, w0 = 0, w1 = 0, pfx0 = 0;
-      int qlo = 0, sh = 0;
-      long long kb = 0;
-      if (ok & 1u) {
-        qlo = __ffs(in_mask) - 1;                 // first offset of the line that lies inside the grid
-        const int qhi = 31 - __clz(in_mask);      // and the last one
-        kb = kk + qlo;                            // its cell: a valid key
-        const long long wi = kb >> 5;
-        sh = static_cast<int>(kb & 31);
-        w0 = __ldg(&bitmap[wi]);
-        if (sh + (qhi - qlo) >= 32) w1 = __ldg(&bitmap[wi + 1]);  // the word of a valid cell as well
-        const unsigned long long win = ((static_cast<unsigned long long>(w1) << 32) | w0) >> sh;
-        present = (static_cast<uint32_t>(win) << qlo) & in_mask;
-        if (present != 0 && ranked) pfx0 = rank_prefix(tin, kb);
-      }
-      for (int q = 0; q < kl; ++q) {
-        int j = -1;
-        if ((present >> q) & 1u) {
-          if (ranked) {
-            const int bit = sh + (q - qlo);
-            j = bit < 32 ? static_cast<int>(pfx0) + __popc(w0 & ((1u << bit) - 1u))
-                         : static_cast<int>(pfx0) + __popc(w0) + __popc(w1 & ((1u << (bit - 32)) - 1u));
-          } else {
-            j = tin.find(static_cast<key_t>(kb + (q - qlo)));
-          }
-        }
-        emit(k0 + q, j);
-        od.next(g);
-      }
-    }
-  } else {
-  // Offsets are handled three at a time (the three neighbours along the last axis of a 3^3
-  // kernel): their bitmap words, then their first hash probes, are requested together, so a row
-  // has up to three L2 accesses in flight instead of one after the other.
-  constexpr int kBatch = 3;
-  for (int k0 = 0; k0 < g.kv; k0 += kBatch) {
-    long long key[kBatch];
-    uint32_t bits[kBatch];
-    unsigned long long probe[kBatch];
-#pragma unroll
-    for (int b = 0; b < kBatch; ++b) {
-      key[b] = -1;
-      if (k0 + b < g.kv) {
-        if (!row_ok) {
-        } else if (fast) {
-          uint32_t ok = 1u;
-          long long kk = base;
-#pragma unroll
-          for (int d = 0; d < ND; ++d) {
-            ok &= inside[d] >> od.pos[d];
-            kk += od.pos[d] * step[d];
-          }
-          if (ok & 1u) key[b] = kk;
-        } else {
-          key[b] = in_key_from_output<ND>(g, o, od.pos);
-        }
-        od.next(g);
-      }
-    }
-#pragma unroll
-    for (int b = 0; b < kBatch; ++b)
-      bits[b] = (key[b] >= 0 && bitmap != nullptr) ? __ldg(&bitmap[key[b] >> 5]) : 0xffffffffu;
-#pragma unroll
-    for (int b = 0; b < kBatch; ++b) {
-      if (key[b] >= 0 && !((bits[b] >> (key[b] & 31)) & 1u)) key[b] = -1;
-      probe[b] = key[b] < 0 ? 0ull
-                 : ranked  ? static_cast<unsigned long long>(rank_prefix(tin, key[b]))
-                           : tin.first_probe(static_cast<key_t>(key[b]));
-    }
-#pragma unroll
-    for (int b = 0; b < kBatch; ++b) {
-      const int k = k0 + b;
-      if (k >= g.kv) break;
-      const int j = key[b] < 0 ? -1
-                    : ranked  ? static_cast<int>(probe[b]) + __popc(bits[b] & ((1u << (key[b] & 31)) - 1u))
-                              : tin.finish(static_cast<key_t>(key[b]), probe[b]);
-      emit(k, j);
-    }
-  }
-  }
-  if (staged) {
-    for (int k = g.kv; k < kvp; ++k) {
-      if (fwd_rm != nullptr) tile_f[lane * kvp + k] = -1;
-      if (SUBM_BWD && bwd_rm != nullptr) tile_b[lane * kvp + k] = -1;
-    }
-  } else if (SUBM_BWD && bwd_rm != nullptr) {
-    for (int k = g.kv; k < kvp; ++k) bwd_rm[r * kvp + k] = -1;
-  }
-  }  // live
-  if (staged) {
-    __syncwarp();
-    const long long row0 = r - lane;  // first row of this warp
-    const long long left = n_out - row0;
-    if (left > 0) {
-      const int n4 = static_cast<int>(left < 32 ? left : 32) * kvp / 4;  // kvp is a multiple of 4
-      if (fwd_rm != nullptr) {
-        int4* dst = reinterpret_cast<int4*>(fwd_rm + row0 * kvp);
-        const int4* src = reinterpret_cast<const int4*>(tile_f);
-        for (int i = lane; i < n4; i += 32) dst[i] = src[i];
-      }
-      if (SUBM_BWD && bwd_rm != nullptr) {
-        int4* dst = reinterpret_cast<int4*>(bwd_rm + row0 * kvp);
-        const int4* src = reinterpret_cast<const int4*>(tile_b);
-        for (int i = lane; i < n4; i += 32) dst[i] = src[i];
-      }
-    }
-  }
+// What a fill kernel writes for its rows; every pointer may be null.
+struct FillOut {
+  int32_t* out_indices;  // coordinates of the output rows (strided layers, output side)
+  int32_t* cm;           // [kv, n]: the neighbour table, column-major
+  int32_t* rm;           // [n, kvp]: the same, row-major, padded with -1
+  int32_t* cm_rev;       // both with the offset axis reversed: the input side of a submanifold layer, whose
+  int32_t* rm_rev;       //   offset k seen from the input is offset kv - 1 - k seen from the output
+  uint32_t* words;       // [n, mic]: bit k = offset k has a neighbour
+  int32_t* iota;         // 0..n-1 (values of the exact mask sort)
+  uint32_t* keys;        // [n]: key of the tile order (kv <= 32)
+  uint32_t* counts;      // rows per bucket of that order (kTileBuckets, zeroed), or null
+};
+
+// A thread owns one row and looks its neighbours up; a warp's 32 rows are collected in shared memory (up to
+// 32 offsets at a time), where absent entries are pre-filled, so that only neighbours that exist cost an
+// entry, and leave it as full 16-byte-per-lane stores (row-major) and coalesced columns.
+// BWD = false: the rows are output rows (of `sorted`, or of `idx` for a submanifold layer) and `table` holds
+// the input cells; BWD = true: input rows, and `table` holds the output cells (rows from n_limit on are cut).
+//
+// The row's kl offsets along the last axis meet cells that lie close together in the occupancy bitmap: one
+// (at a word boundary two) loads test all of them, and one prefix load numbers all of them, since the prefix
+// of the next word is this word's prefix plus its population count.  Three such lines are requested together:
+// the kernel waits on L2 latency otherwise.  A submanifold or strided k3 layer so has 9 + 9 loads in flight in
+// three rounds instead of 27 probes of a hash table.
+constexpr int kLines = 3;
+constexpr int kBucketSlots = 512;  // of the CTA's own bucket counts: at most 256 distinct buckets
+
+__host__ __device__ __forceinline__ int fill_pitch(int kvp) {
+  // row pitch of the shared tile in entries: 4 mod 8, so that a warp's rows start in eight different bank groups
+  const int w = kvp < 32 ? kvp : 32;
+  return (w & 7) == 4 ? w : w + 4;
 }
 
-// Column j of pair_bwd (strided / transposed layers): for each offset the
-// output row that input row j contributes to.
-template <int ND, bool K64>
+template <int ND, bool K64, bool BWD>
 __global__ void __launch_bounds__(kThreads)
-fill_bwd_kernel(const __grid_constant__ Geo g, const int32_t* __restrict__ idx, long long n_in,
-                long long n_out, Table<K64> tout, int32_t* __restrict__ pair_bwd,
-                uint32_t* __restrict__ words, int mic, int32_t* __restrict__ bwd_rm, int kvp,
-                int32_t* __restrict__ iota) {
+fill_kernel(const __grid_constant__ Geo g, const int32_t* __restrict__ idx,
+            const typename Table<K64>::key_t* __restrict__ sorted, long long n, long long n_limit, Table<K64> table,
+            const __grid_constant__ FillOut out, int mic, int kvp) {
   using key_t = typename Table<K64>::key_t;
-  const long long j = blockIdx.x * static_cast<long long>(kThreads) + threadIdx.x;
-  if (j >= n_in) return;
-  if (iota != nullptr) iota[j] = static_cast<int32_t>(j);
-  int quad[4] = {-1, -1, -1, -1};
-  int c[ND + 1];
-  load_coord<ND>(idx, j, c);
-  const bool row_ok = coord_in_grid<ND>(g, c);  // a row outside the grid contributes to no output
-  Odometer<ND> od;
-  od.reset();
-  uint32_t word = 0;
-  for (int k = 0; k < g.kv; ++k) {
-    const long long key = row_ok ? out_key_from_input<ND>(g, c, od.pos) : -1;
-    int r = key >= 0 ? tout.find(static_cast<key_t>(key)) : -1;
-    if (r >= n_out) r = -1;  // rows cut off by num_out_act_bound
-    pair_bwd[static_cast<long long>(k) * n_in + j] = r;
-    if (bwd_rm != nullptr) {
-      quad[k & 3] = r;
-      if ((k & 3) == 3 || k == g.kv - 1) {
-        *reinterpret_cast<int4*>(&bwd_rm[j * kvp + (k & ~3)]) = make_int4(quad[0], quad[1], quad[2], quad[3]);
-        quad[0] = quad[1] = quad[2] = quad[3] = -1;
-      }
+  extern __shared__ __align__(16) int32_t fill_s[];
+  __shared__ int slot_bucket[kBucketSlots];
+  __shared__ uint32_t slot_count[kBucketSlots];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int pitch = fill_pitch(kvp);
+  int32_t* tile = fill_s + warp * 32 * pitch;
+  int32_t* mine = tile + lane * pitch;
+  if (out.counts != nullptr) {
+    for (int i = threadIdx.x; i < kBucketSlots; i += kThreads) {
+      slot_bucket[i] = -1;
+      slot_count[i] = 0;
     }
-    if (words != nullptr) {
-      word |= static_cast<uint32_t>(r >= 0) << (k & 31);
-      if ((k & 31) == 31 || k == g.kv - 1) {
-        words[j * mic + (k >> 5)] = word;
-        word = 0;
-      }
-    }
-    od.next(g);
+    __syncthreads();
   }
+  const long long r = blockIdx.x * static_cast<long long>(kThreads) + threadIdx.x;
+  const long long row0 = r - lane;
+  const bool live = r < n;
+  const bool from_idx = BWD || g.subm;
+  const bool div = BWD ? !g.transpose : g.transpose != 0;
+  const int* __restrict__ limit = BWD ? g.out_shape : g.in_shape;
+
+  int own[ND + 1];
+  bool ok = live;  // a row outside the grid gets no neighbours
+  if (live) {
+    if (from_idx) {
+      load_coord<ND>(idx, r, own);
+      ok = coord_in_grid<ND>(g, own);
+    } else {
+      key_t lin = sorted[r];
+#pragma unroll
+      for (int d = ND - 1; d >= 0; --d) {
+        const key_t q = lin / static_cast<key_t>(g.out_shape[d]);
+        own[d + 1] = static_cast<int>(lin - q * static_cast<key_t>(g.out_shape[d]));
+        lin = q;
+      }
+      own[0] = static_cast<int>(lin);
+      if (out.out_indices != nullptr) {
+        if (ND == 3 && (reinterpret_cast<uintptr_t>(out.out_indices) & 15u) == 0) {
+          reinterpret_cast<int4*>(out.out_indices)[r] = make_int4(own[0], own[1], own[ND > 1 ? 2 : 0], own[ND > 2 ? 3 : 0]);
+        } else {
+#pragma unroll
+          for (int d = 0; d <= ND; ++d) out.out_indices[r * (ND + 1) + d] = own[d];
+        }
+      }
+    }
+    if (out.iota != nullptr) out.iota[r] = static_cast<int32_t>(r);
+  }
+  uint32_t valid[ND];  // per axis: the offsets that meet a cell of the grid
+#pragma unroll
+  for (int d = 0; d < ND; ++d) {
+    uint32_t m = 0;
+    if (ok && g.axes_fit)
+      for (int k = 0; k < g.ksize[d]; ++k)
+        m |= static_cast<uint32_t>(axis_cell(g, div, d, own[d + 1], k, limit[d]) >= 0) << k;
+    valid[d] = m;
+  }
+  const uint32_t* bits = dense_bits(table);
+  const uint32_t* prefix = dense_prefix(table);
+  const int32_t* perm = row_permutation(table);
+  const int kl = g.ksize[ND - 1];
+  const int q_lo = valid[ND - 1] ? __ffs(valid[ND - 1]) - 1 : 0;
+  const int q_hi = valid[ND - 1] ? 31 - __clz(valid[ND - 1]) : -1;
+  // lowest and highest cell of a line of offsets along the last axis
+  int x_lo = 0, x_span = 0;
+  if (q_hi >= 0) {
+    const int xa = axis_cell(g, div, ND - 1, own[ND], q_lo, limit[ND - 1]);
+    const int xb = axis_cell(g, div, ND - 1, own[ND], q_hi, limit[ND - 1]);
+    x_lo = xa < xb ? xa : xb;
+    x_span = (xa < xb ? xb : xa) - x_lo;
+  }
+  uint32_t order_word = 0;
+  for (int c0 = 0; c0 < g.kv; c0 += 32) {
+    const int width = min(32, kvp - c0);           // entries of a row in this piece, a multiple of four
+    const int c1 = min(g.kv, c0 + 32);
+    __syncwarp();  // the previous piece has been copied out
+    {
+      const int4 none = make_int4(-1, -1, -1, -1);
+      for (int i = lane; i < 8 * pitch; i += 32) reinterpret_cast<int4*>(tile)[i] = none;
+    }
+    __syncwarp();
+    uint32_t word = 0;
+    auto emit = [&](int k, int j) {
+      if (k < c0 || k >= c1 || j < 0 || (BWD && j >= n_limit)) return;
+      mine[k - c0] = j;
+      word |= 1u << (k - c0);
+      if (out.keys != nullptr) order_word |= 1u << g.key_pos[k];
+    };
+    if (ok && g.axes_fit && q_hi >= 0) {
+      int pos[ND];  // offsets of the leading axes
+      const int l0 = c0 / kl, l1 = (c1 - 1) / kl;
+      {
+        int rest = l0;
+#pragma unroll
+        for (int d = ND - 2; d >= 0; --d) {
+          pos[d] = rest % g.ksize[d];
+          rest /= g.ksize[d];
+        }
+      }
+      for (int l = l0; l <= l1; l += kLines) {
+        bool on[kLines];
+        key_t base[kLines];
+#pragma unroll
+        for (int b = 0; b < kLines; ++b) {
+          on[b] = l + b <= l1;
+          key_t key = static_cast<key_t>(own[0]);
+#pragma unroll
+          for (int d = 0; d < ND - 1; ++d) {
+            on[b] = on[b] && ((valid[d] >> pos[d]) & 1u);
+            const int x = on[b] ? axis_cell(g, div, d, own[d + 1], pos[d], limit[d]) : 0;
+            key = key * static_cast<key_t>(limit[d]) + static_cast<key_t>(x);
+          }
+          base[b] = key * static_cast<key_t>(limit[ND - 1]);
+          // next line
+          bool carry = true;
+#pragma unroll
+          for (int d = ND - 2; d >= 0; --d) {
+            if (carry) {
+              carry = ++pos[d] == g.ksize[d];
+              if (carry) pos[d] = 0;
+            }
+          }
+        }
+        if (bits != nullptr && g.window) {
+          uint32_t w0[kLines], w1[kLines], hits[kLines], before[kLines];
+#pragma unroll
+          for (int b = 0; b < kLines; ++b) {
+            w0[b] = w1[b] = 0;
+            if (on[b]) {
+              const key_t at = base[b] + static_cast<key_t>(x_lo);
+              w0[b] = __ldg(&bits[at >> 5]);
+              if (static_cast<int>(at & 31) + x_span >= 32) w1[b] = __ldg(&bits[(at >> 5) + 1]);
+            }
+          }
+#pragma unroll
+          for (int b = 0; b < kLines; ++b) {
+            hits[b] = before[b] = 0;
+            const key_t at = base[b] + static_cast<key_t>(x_lo);
+            if ((w0[b] | w1[b]) != 0) {
+              const unsigned long long win = ((static_cast<unsigned long long>(w1[b]) << 32) | w0[b]) >> (at & 31);
+              for (uint32_t m = valid[ND - 1]; m != 0; m &= m - 1) {
+                const int q = __ffs(m) - 1;
+                const int x = axis_cell(g, div, ND - 1, own[ND], q, limit[ND - 1]) - x_lo;
+                hits[b] |= static_cast<uint32_t>((win >> x) & 1ull) << q;
+              }
+              // (a word without bits has no prefix: the second word's rows then come first)
+              if (hits[b] != 0) before[b] = __ldg(&prefix[(at >> 5) + (w0[b] == 0 ? 1 : 0)]);
+            }
+          }
+#pragma unroll
+          for (int b = 0; b < kLines; ++b) {
+            const int sh = static_cast<int>((base[b] + static_cast<key_t>(x_lo)) & 31);
+            for (uint32_t m = hits[b]; m != 0; m &= m - 1) {
+              const int q = __ffs(m) - 1;
+              const int bit = sh + axis_cell(g, div, ND - 1, own[ND], q, limit[ND - 1]) - x_lo;
+              int j = static_cast<int>(before[b]) +
+                      (bit < 32 ? __popc(w0[b] & ((1u << bit) - 1u)) : __popc(w0[b]) + __popc(w1[b] & ((1u << (bit - 32)) - 1u)));
+              if (perm != nullptr) j = __ldg(&perm[j]);
+              emit((l + b) * kl + q, j);
+            }
+          }
+        } else {
+          // hash table (or cells too far apart for a window): up to three probes in flight
+#pragma unroll
+          for (int b = 0; b < kLines; ++b) {
+            if (!on[b]) continue;
+            uint32_t m = valid[ND - 1];
+            while (m != 0) {
+              key_t key[3];
+              int q[3];
+              unsigned long long probe[3];
+#pragma unroll
+              for (int u = 0; u < 3; ++u) {
+                q[u] = m != 0 ? __ffs(m) - 1 : -1;
+                m &= m - 1;
+                probe[u] = 0;
+                if (q[u] >= 0) {
+                  key[u] = base[b] + static_cast<key_t>(axis_cell(g, div, ND - 1, own[ND], q[u], limit[ND - 1]));
+                  if (bits == nullptr) probe[u] = table.first_probe(key[u]);
+                }
+              }
+#pragma unroll
+              for (int u = 0; u < 3; ++u)
+                if (q[u] >= 0) emit((l + b) * kl + q[u], bits == nullptr ? table.finish(key[u], probe[u]) : table.find(key[u]));
+            }
+          }
+        }
+      }
+    } else if (ok && !g.axes_fit) {
+      // an axis of more than 32 offsets: one offset after the other
+      Odometer<ND> od;
+      od.set(g, c0);
+      for (int k = c0; k < c1; ++k) {
+        long long key = own[0];
+#pragma unroll
+        for (int d = 0; d < ND; ++d) {
+          const int x = axis_cell(g, div, d, own[d + 1], od.pos[d], limit[d]);
+          key = key < 0 || x < 0 ? -1 : key * limit[d] + x;
+        }
+        if (key >= 0) emit(k, table.find(static_cast<key_t>(key)));
+        od.next(g);
+      }
+    }
+    if (live && out.words != nullptr) out.words[r * mic + (c0 >> 5)] = word;
+    __syncwarp();
+    const int rows = static_cast<int>(n - row0 < 32 ? (n - row0 > 0 ? n - row0 : 0) : 32);
+    if (out.rm != nullptr) {
+      const int quads = width / 4;
+      if (pitch == kvp) {
+        int4* dst = reinterpret_cast<int4*>(out.rm + row0 * kvp);
+        for (int i = lane; i < rows * quads; i += 32) dst[i] = reinterpret_cast<const int4*>(tile)[i];
+      } else {
+        for (int i = lane; i < rows * quads; i += 32) {
+          const int row = i / quads, q = i - row * quads;
+          *reinterpret_cast<int4*>(out.rm + (row0 + row) * kvp + c0 + 4 * q) =
+              *reinterpret_cast<const int4*>(tile + row * pitch + 4 * q);
+        }
+      }
+    }
+    if (out.rm_rev != nullptr) {
+      for (int row = 0; row < rows; ++row)
+        if (lane < c1 - c0) out.rm_rev[(row0 + row) * kvp + g.kv - 1 - (c0 + lane)] = tile[row * pitch + lane];
+      if (c1 == g.kv && live)
+        for (int k = g.kv; k < kvp; ++k) out.rm_rev[r * kvp + k] = -1;
+    }
+    if (live) {
+      if (out.cm != nullptr)
+        for (int k = c0; k < c1; ++k) out.cm[static_cast<long long>(k) * n + r] = mine[k - c0];
+      if (out.cm_rev != nullptr)
+        for (int k = c0; k < c1; ++k) out.cm_rev[static_cast<long long>(g.kv - 1 - k) * n + r] = mine[k - c0];
+    }
+  }
+  if (out.keys == nullptr) return;
+  if (live) out.keys[r] = gray_decode(order_word);
+  if (out.counts == nullptr) return;
+  // rows per bucket: first inside the warp, then inside the CTA, so that a bucket most rows fall into is
+  // one global addition per CTA
+  const int bucket = live ? bucket_of(order_word) : -1;
+  const unsigned same = __match_any_sync(0xffffffffu, bucket);
+  if (bucket >= 0 && __ffs(same) - 1 == lane) {
+    uint32_t s = (static_cast<uint32_t>(bucket) * 2654435761u) >> 23;
+    for (int probe = 0; probe < kBucketSlots; ++probe) {
+      const int old = atomicCAS(&slot_bucket[s], -1, bucket);
+      if (old == -1 || old == bucket) {
+        atomicAdd(&slot_count[s], static_cast<uint32_t>(__popc(same)));
+        break;
+      }
+      s = (s + 1) & (kBucketSlots - 1);
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kBucketSlots; i += kThreads)
+    if (slot_bucket[i] >= 0) atomicAdd(&out.counts[slot_bucket[i]], slot_count[i]);
 }
 
 // keys[i] = words[rows[i], w] & and_mask ; rows == nullptr means identity.
@@ -987,20 +1147,48 @@ struct Layout {
   int key_bits;
   int mic;
   int64_t bound;  // upper bound on n_out
-  int64_t obits_words = 0;  // dense numbering of the outputs: words of the bitmap (0 = hash table + sort)
-  size_t off_obits = 0, off_oprefix = 0, off_scan = 0, scan_bytes = 0, off_iprefix = 0;
+  // Occupancy bitmaps (words; 0 = that side uses a hash table): the output side of a strided layer is
+  // numbered and looked up through its bitmap, the input side looked up.
+  int64_t ibits_words = 0, obits_words = 0;
+  size_t off_ibits = 0, off_iprefix = 0, off_istarts = 0, off_perm = 0;
+  size_t off_obits = 0, off_oprefix = 0, off_ostarts = 0;
   uint32_t cap_in, cap_out;
   int64_t n_blocks_native;
   size_t off_counters, off_tin, off_tin_vals, off_tout, off_tout_vals, off_uniq, off_sorted;
   size_t off_words, off_keys_a, off_keys_b, off_vals_a, off_vals_b, off_cub, off_native;
+  size_t off_order_pairs, off_order_counts;
   size_t cub_bytes, total;
-  size_t off_bitmap, bitmap_bytes;  // occupancy bitmap of the input grid (0 bytes: not used)
   // Chained rulebooks: the input rows are exactly the output rows of an earlier strided layer whose
   // output bitmap and prefix (in ITS workspace) then serve as this layer's input bitmap; rows are
   // ranks by construction, and no input hash table is built.
   const uint32_t* shared_bits = nullptr;
   const uint32_t* shared_prefix = nullptr;
 };
+// counts and taken of the tile order
+constexpr size_t kOrderCountBytes = 2 * ((kTileBuckets * 4 + 255) / 256) * 256;
+
+inline int cell_blocks(int64_t words) { return static_cast<int>(ceil_div(words, kCellBlock)); }
+
+// Scratch of the library's radix sort for n (key, row) pairs: asked for once per power of two.
+size_t radix_sort_bytes(int64_t n, bool keys64) {
+  static std::atomic<size_t> known[2][64];
+  int e = 0;
+  while ((1ll << e) < n) ++e;
+  size_t have = known[keys64][e].load(std::memory_order_relaxed);
+  if (have != 0) return have;
+  const int64_t most = std::min<int64_t>(1ll << e, INT32_MAX);
+  size_t keys = 0, pairs = 0;
+  if (keys64)
+    cub::DeviceRadixSort::SortKeys(nullptr, keys, static_cast<unsigned long long*>(nullptr),
+                                   static_cast<unsigned long long*>(nullptr), most);
+  else
+    cub::DeviceRadixSort::SortKeys(nullptr, keys, static_cast<uint32_t*>(nullptr), static_cast<uint32_t*>(nullptr), most);
+  cub::DeviceRadixSort::SortPairs(nullptr, pairs, static_cast<uint32_t*>(nullptr), static_cast<uint32_t*>(nullptr),
+                                  static_cast<int32_t*>(nullptr), static_cast<int32_t*>(nullptr), most);
+  have = std::max<size_t>(std::max(keys, pairs), 16);
+  known[keys64][e].store(have, std::memory_order_relaxed);
+  return have;
+}
 
 uint32_t pow2_at_least(int64_t v) {
   uint64_t c = 64;
@@ -1035,7 +1223,14 @@ bool make_geo(const spc_geometry* s, Geo* g) {
     }
     g->kv *= g->ksize[d];
   }
-  g->tile_key = 0;
+  g->axes_fit = 1;
+  for (int d = 0; d < SPC_MAX_NDIM; ++d) {
+    g->axes_fit = g->axes_fit && g->ksize[d] <= 32;
+    g->shift[d] = -1;
+    for (int b = 0; b < 31; ++b)
+      if (g->stride[d] == (1 << b)) g->shift[d] = b;
+  }
+  g->window = static_cast<int64_t>(g->ksize[s->ndim - 1] - 1) * g->dil[s->ndim - 1] <= 32;
   for (int k = 0; k < 32; ++k) g->key_pos[k] = static_cast<unsigned char>(k);
   if (g->kv <= 32) {
     // distance of every offset from the kernel's centre (sum over the axes), then positions in
@@ -1084,23 +1279,21 @@ Layout make_layout(const Geo& g, int64_t n_in) {
     const double b = std::min(static_cast<double>(n_in) * per_input, vol_out);
     L.bound = static_cast<int64_t>(std::max(b, 1.0));
   }
-  L.cap_in = pow2_at_least(4 * n_in);  // load <= 0.25: most neighbour look-ups miss, keep their probe chains short
-  L.cap_out = g.subm ? 0 : pow2_at_least(2 * L.bound);
+  // The input side through a bitmap of the grid (most neighbour cells of a voxel are empty, a bit test
+  // answers for a whole line of them, and a row is its rank) where the bitmap is no dearer to clear and
+  // count than a hash table (512 cells or 64 bytes a voxel), small enough to stay in L2 beside the tables
+  // (24 MB), and there are enough rows for the looks-up to outweigh three more launches.
+  const double max_bits = 24.0 * 1024 * 1024 * 8;
+  if (!L.k64 && vol_in <= max_bits && vol_in <= 512.0 * n_in && n_in >= 16384)
+    L.ibits_words = static_cast<int64_t>(vol_in / 32.0) + 1;
+  // the output bitmap also numbers the outputs, which a hash table needs a sort for
+  if (!g.subm && !L.k64 && vol_out <= max_bits) L.obits_words = static_cast<int64_t>(vol_out / 32.0) + 1;
+  L.cap_in = L.ibits_words ? 0 : pow2_at_least(4 * n_in);  // load <= 0.25: most look-ups miss, keep their probe chains short
+  L.cap_out = g.subm || L.obits_words ? 0 : pow2_at_least(2 * L.bound);
   const int64_t n_max = std::max<int64_t>(n_in, L.bound);
   L.n_blocks_native = ceil_div(std::max<int64_t>(n_in, 1), kThreads);
   const size_t key_sz = L.k64 ? 8 : 4;
-
-  size_t sort_keys_bytes = 0, sort_pairs_bytes = 0;
-  if (L.k64)
-    cub::DeviceRadixSort::SortKeys(nullptr, sort_keys_bytes, static_cast<unsigned long long*>(nullptr),
-                                   static_cast<unsigned long long*>(nullptr), L.bound);
-  else
-    cub::DeviceRadixSort::SortKeys(nullptr, sort_keys_bytes, static_cast<uint32_t*>(nullptr),
-                                   static_cast<uint32_t*>(nullptr), L.bound);
-  cub::DeviceRadixSort::SortPairs(nullptr, sort_pairs_bytes, static_cast<uint32_t*>(nullptr),
-                                  static_cast<uint32_t*>(nullptr), static_cast<int32_t*>(nullptr),
-                                  static_cast<int32_t*>(nullptr), n_max);
-  L.cub_bytes = std::max(sort_keys_bytes, sort_pairs_bytes);
+  L.cub_bytes = radix_sort_bytes(n_max, L.k64);
 
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -1122,24 +1315,15 @@ Layout make_layout(const Geo& g, int64_t n_in) {
   L.off_vals_b = take(static_cast<size_t>(n_max) * 4);
   L.off_cub = take(L.cub_bytes);
   L.off_native = take(static_cast<size_t>(L.n_blocks_native) * g.kv * 4);
-  // One bit per input cell, when that is small enough to live in L2 beside the hash table: most of
-  // the kv neighbour cells of a voxel are empty, and a bit test (neighbours share bytes) then
-  // answers "absent" without a hash probe.
-  L.bitmap_bytes = (!L.k64 && vol_in / 8.0 <= 24.0 * 1024 * 1024) ? align_up(static_cast<size_t>(vol_in / 8.0) + 4, 256) : 0;
-  L.off_bitmap = take(L.bitmap_bytes);
-  L.off_iprefix = take(L.bitmap_bytes);  // set bits before each word of the input bitmap
-  // The same for the output grid of a strided layer; there the bitmap also numbers the outputs.
-  L.obits_words = (!g.subm && !L.k64 && vol_out / 8.0 <= 24.0 * 1024 * 1024) ? static_cast<int64_t>(vol_out / 32.0) + 1 : 0;
+  L.off_order_pairs = take(g.kv <= 32 ? static_cast<size_t>(n_max) * 8 : 0);
+  L.off_order_counts = take(kOrderCountBytes);
+  L.off_ibits = take(static_cast<size_t>(L.ibits_words) * 4);
+  L.off_iprefix = take(static_cast<size_t>(L.ibits_words) * 4);
+  L.off_istarts = take(L.ibits_words ? static_cast<size_t>(cell_blocks(L.ibits_words) + 1) * 4 : 0);
+  L.off_perm = take(L.ibits_words ? static_cast<size_t>(n_in) * 4 : 0);
   L.off_obits = take(static_cast<size_t>(L.obits_words) * 4);
   L.off_oprefix = take(static_cast<size_t>(L.obits_words) * 4);
-  const int64_t scan_words = std::max<int64_t>(L.obits_words, static_cast<int64_t>(L.bitmap_bytes / 4));
-  if (scan_words) {
-    size_t scan_bytes = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, static_cast<uint32_t*>(nullptr), static_cast<uint32_t*>(nullptr),
-                                  static_cast<int>(scan_words));
-    L.off_scan = take(scan_bytes);
-    L.scan_bytes = scan_bytes;
-  }
+  L.off_ostarts = take(L.obits_words ? static_cast<size_t>(cell_blocks(L.obits_words) + 1) * 4 : 0);
   L.total = off;
   return L;
 }
@@ -1172,10 +1356,11 @@ Table<false> tin_at<false>(char* ws, const Layout& L) {
     t.oprefix = L.shared_prefix;
     return t;  // `unsorted` stays null: the rows are the ranks
   }
-  if (L.bitmap_bytes) {
-    t.obits = reinterpret_cast<uint32_t*>(ws + L.off_bitmap);
+  if (L.ibits_words) {
+    t.obits = reinterpret_cast<uint32_t*>(ws + L.off_ibits);
     t.oprefix = reinterpret_cast<const uint32_t*>(ws + L.off_iprefix);
     t.unsorted = reinterpret_cast<const int*>(ws + L.off_counters) + kUnsorted;
+    t.perm = reinterpret_cast<const int32_t*>(ws + L.off_perm);
   }
   return t;
 }
@@ -1200,61 +1385,55 @@ Table<true> tout_at<true>(char* ws, const Layout& L) {
   return table_at<true>(ws, L.off_tout, L.off_tout_vals, L.cap_out);
 }
 
-// Byte fill of scratch regions by a kernel of this library rather than cudaMemsetAsync: the
-// regions are 16-byte multiples at 16-byte aligned offsets, and a kernel can neither be routed
-// to a copy engine (where it would queue behind a large transfer of the application) nor
-// cost a driver memset's set-up.
-__global__ void __launch_bounds__(256) fill_bytes_kernel(uint4* __restrict__ dst, uint32_t word, long long n16) {
-  const long long stride = static_cast<long long>(gridDim.x) * 256;
-  const uint4 v = make_uint4(word, word, word, word);
-  for (long long i = blockIdx.x * 256ll + threadIdx.x; i < n16; i += stride) dst[i] = v;
-}
-int fill_bytes(void* dst, int byte, size_t bytes, cudaStream_t st) {
-  if (bytes == 0) return SPC_OK;
-  if ((reinterpret_cast<uintptr_t>(dst) & 15u) != 0 || bytes % 16 != 0) {
-    SPC_CUDA_OK(cudaMemsetAsync(dst, byte, bytes, st));
-    return SPC_OK;
-  }
-  const long long n16 = static_cast<long long>(bytes / 16);
-  const uint32_t b = static_cast<uint32_t>(byte) & 0xffu;
-  const unsigned blocks = static_cast<unsigned>(std::min<long long>(ceil_div(n16, 256), 16ll * sm_count()));
-  fill_bytes_kernel<<<blocks, 256, 0, st>>>(static_cast<uint4*>(dst), b * 0x01010101u, n16);
+int launch_clear(const Clear& c, cudaStream_t st) {
+  const unsigned blocks = static_cast<unsigned>(std::max<long long>(1, std::min<long long>(ceil_div(c.total, 256), 16ll * sm_count())));
+  clear_kernel<<<blocks, 256, 0, st>>>(c);
   SPC_LAUNCH_OK();
   return SPC_OK;
 }
-#define SPC_FILL(dst, byte, bytes, st)                              \
-  do {                                                              \
-    const int rc__ = fill_bytes((dst), (byte), (bytes), (st));      \
-    if (rc__ != SPC_OK) return rc__;                                \
-  } while (0)
 
 // A few page-locked words per host thread and device that kernels write and the host reads after
 // synchronising (host memory: the library still allocates no device memory).
-int host_mailbox(volatile int** out) {
+// One per host thread and device, with the ticket of the next message.
+int host_mailbox(volatile int** out, int* ticket) {
   static thread_local int* boxes[kMaxDevices] = {nullptr};
+  static thread_local int tickets[kMaxDevices] = {0};
   const int dev = current_device_slot();
   if (dev < 0) return fail(SPC_ERR_CUDA, "rulebook: no current device");
   if (boxes[dev] == nullptr) {
     void* p = nullptr;
     SPC_CUDA_OK(cudaHostAlloc(&p, 64, cudaHostAllocPortable | cudaHostAllocMapped));
     boxes[dev] = static_cast<int*>(p);
+    boxes[dev][0] = 0;
   }
   *out = boxes[dev];
+  tickets[dev] = (tickets[dev] + 1) & 0x7fffffff;
+  if (tickets[dev] == 0) tickets[dev] = 1;
+  *ticket = tickets[dev];
   return SPC_OK;
 }
 
-// How the host waits for a count.  cudaStreamSynchronize spins on a core for the whole wait, which is
-// the fastest wake-up (a pass alone: 2.28 ms against 2.59 ms with a blocking event) but needs an idle
-// core per pass in flight; with SPC_HOST_WAIT=block in the environment (read once) the thread sleeps
-// on a blocking event instead, for processes that keep several passes in flight on few cores (one
-// process per GPU, eight GPUs, three host threads each).  One event per host thread and device.
-int wait_for_stream(cudaStream_t st) {
+// How the host waits for a count: it spins on the page-locked ticket that the publishing kernel writes last,
+// which is the fastest wake-up (the count is there before the stream has drained and without the driver's
+// completion signal) but needs an idle core per pass in flight; with SPC_HOST_WAIT=block in the
+// environment (read once) the thread sleeps on a blocking event instead, for processes that keep several
+// passes in flight on few cores (one process per GPU, eight GPUs, three host threads each).  A stream that
+// has drained, or failed, without the ticket ends the spin.  One event per host thread and device.
+int wait_for_ticket(volatile int* box, int ticket, cudaStream_t st) {
   static const bool block = [] {
     const char* v = std::getenv("SPC_HOST_WAIT");
     return v != nullptr && std::strcmp(v, "block") == 0;
   }();
   if (!block) {
-    SPC_CUDA_OK(cudaStreamSynchronize(st));
+    for (unsigned spin = 1; box[0] != ticket; ++spin) {
+      __builtin_ia32_pause();
+      if ((spin & 0xfffu) != 0) continue;
+      const cudaError_t e = cudaStreamQuery(st);
+      if (e == cudaErrorNotReady) continue;
+      SPC_CUDA_OK(e);
+      if (box[0] != ticket) return fail(SPC_ERR_CUDA, "rulebook: the output count did not arrive");
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
     return SPC_OK;
   }
   static thread_local cudaEvent_t events[kMaxDevices] = {nullptr};
@@ -1264,6 +1443,7 @@ int wait_for_stream(cudaStream_t st) {
     SPC_CUDA_OK(cudaEventCreateWithFlags(&events[dev], cudaEventBlockingSync | cudaEventDisableTiming));
   SPC_CUDA_OK(cudaEventRecord(events[dev], st));
   SPC_CUDA_OK(cudaEventSynchronize(events[dev]));
+  if (box[0] != ticket) return fail(SPC_ERR_CUDA, "rulebook: the output count did not arrive");
   return SPC_OK;
 }
 
@@ -1280,80 +1460,92 @@ int prepare_impl(const Geo& g, const Layout& L, const int32_t* idx, int64_t n_in
   // Submanifold layers return without a host read, so a row outside the grid is also recorded in the
   // device status word, which the host reads at its next synchronisation point.
   int* dev_status = device_status_ptr();
-  SPC_FILL(counters, 0, 256, st);
   const bool chained = L.shared_bits != nullptr;  // input bitmap and prefix exist already, no input table
-  if (!chained) {
-    SPC_FILL(ws + L.off_tin, 0xFF, static_cast<size_t>(L.cap_in) * 8, st);
-    if (K64) SPC_FILL(ws + L.off_tin_vals, 0x7F, static_cast<size_t>(L.cap_in) * 4, st);
+  const bool dense_in = !chained && L.ibits_words != 0, dense_out = L.obits_words != 0;
+  Clear clear;
+  clear.add(counters, 0, 256);
+  if (dense_in) {
+    clear.add(ws + L.off_ibits, 0, static_cast<size_t>(L.ibits_words) * 4);
+    clear.add(ws + L.off_perm, 0x7F, static_cast<size_t>(n_in) * 4);
+  } else if (!chained) {
+    clear.add(ws + L.off_tin, 0xFF, static_cast<size_t>(L.cap_in) * 8);
+    if (K64) clear.add(ws + L.off_tin_vals, 0x7F, static_cast<size_t>(L.cap_in) * 4);
   }
+  if (dense_out) {
+    clear.add(ws + L.off_obits, 0, static_cast<size_t>(L.obits_words) * 4);
+  } else if (!g.subm) {
+    clear.add(ws + L.off_tout, 0xFF, static_cast<size_t>(L.cap_out) * 8);
+    if (K64) clear.add(ws + L.off_tout_vals, 0x7F, static_cast<size_t>(L.cap_out) * 4);
+  }
+  clear.add(ws + L.off_order_counts, 0, kOrderCountBytes);
+  int rc = launch_clear(clear, st);
+  if (rc != SPC_OK) return rc;
   Table<K64> tin = tin_at<K64>(ws, L);
-  uint32_t* bitmap = (L.bitmap_bytes && !chained) ? reinterpret_cast<uint32_t*>(ws + L.off_bitmap) : nullptr;
-  if (bitmap != nullptr) {
-    SPC_FILL(bitmap, 0, L.bitmap_bytes, st);
-    mark_inputs_kernel<ND><<<blocks_for(n_in), kThreads, 0, st>>>(g, idx, n_in, bitmap, counters, dev_status);
+  Table<K64> tout = tout_at<K64>(ws, L);
+  uint32_t* ibits = dense_in ? reinterpret_cast<uint32_t*>(ws + L.off_ibits) : nullptr;
+  uint32_t* obits = dense_out ? reinterpret_cast<uint32_t*>(ws + L.off_obits) : nullptr;
+  key_t* uniq = reinterpret_cast<key_t*>(ws + L.off_uniq);
+  key_t* sorted = reinterpret_cast<key_t*>(ws + L.off_sorted);
+  if (!chained || (dense_out && g.axes_fit)) {
+    ingest_kernel<ND, K64><<<blocks_for(n_in), kThreads, 0, st>>>(g, idx, n_in, tin, !chained, ibits,
+                                                                  g.axes_fit ? obits : nullptr, counters, dev_status);
     SPC_LAUNCH_OK();
-    const int64_t words = static_cast<int64_t>(L.bitmap_bytes / 4);
-    uint32_t* iprefix = reinterpret_cast<uint32_t*>(ws + L.off_iprefix);
-    count_bits_kernel<<<blocks_for(words), kThreads, 0, st>>>(bitmap, words, iprefix);
-    SPC_LAUNCH_OK();
-    size_t scan_bytes = L.scan_bytes;
-    SPC_CUDA_OK(cub::DeviceScan::ExclusiveSum(ws + L.off_scan, scan_bytes, iprefix, iprefix, static_cast<int>(words), st));
   }
-  if (!chained) {
-    insert_inputs_kernel<ND, K64><<<blocks_for(n_in), kThreads, 0, st>>>(g, idx, n_in, tin, counters, bitmap,
-                                                                         dev_status);
+  if (!g.subm && !(dense_out && g.axes_fit)) {
+    enumerate_outputs_kernel<ND, K64><<<blocks_for(n_in), kThreads, 0, st>>>(g, idx, n_in, tout, uniq, counters);
     SPC_LAUNCH_OK();
+  }
+  // The output count reaches the host through a page-locked word that a kernel writes, not through a
+  // device-to-host copy: a copy would queue on the copy engine behind whatever transfer the
+  // application has in flight (a previous result going back to the host, say) and stall the whole
+  // rulebook chain for its duration.
+  volatile int* box = nullptr;
+  int ticket = 0;
+  if (!g.subm) {
+    rc = host_mailbox(&box, &ticket);
+    if (rc != SPC_OK) return rc;
+  }
+  if (dense_in || dense_out) {
+    Cells c{};
+    if (dense_in) {
+      c.bits[0] = ibits;
+      c.prefix[0] = reinterpret_cast<uint32_t*>(ws + L.off_iprefix);
+      c.starts[0] = reinterpret_cast<uint32_t*>(ws + L.off_istarts);
+      c.words[0] = L.ibits_words;
+      c.blocks[0] = cell_blocks(L.ibits_words);
+    }
+    if (dense_out) {
+      c.bits[1] = obits;
+      c.prefix[1] = reinterpret_cast<uint32_t*>(ws + L.off_oprefix);
+      c.starts[1] = reinterpret_cast<uint32_t*>(ws + L.off_ostarts);
+      c.words[1] = L.obits_words;
+      c.blocks[1] = cell_blocks(L.obits_words);
+    }
+    const unsigned blocks = static_cast<unsigned>(c.blocks[0] + c.blocks[1]);
+    count_cells_kernel<<<blocks, kThreads, 0, st>>>(c, counters, dev_status, dense_out ? const_cast<int*>(box) : nullptr, ticket);
+    SPC_LAUNCH_OK();
+    number_cells_kernel<<<blocks, kThreads, 0, st>>>(c, L.bound, reinterpret_cast<uint32_t*>(sorted));
+    SPC_LAUNCH_OK();
+    if constexpr (!K64) {
+      if (dense_in) {
+        permute_rows_kernel<ND><<<blocks_for(n_in), kThreads, 0, st>>>(g, idx, n_in, tin,
+                                                                       reinterpret_cast<int32_t*>(ws + L.off_perm));
+        SPC_LAUNCH_OK();
+      }
+    }
   }
   if (g.subm) {
     *n_out_host = n_in;
     return SPC_OK;
   }
-  const bool dense_out = L.obits_words != 0;
-  if (dense_out) {
-    SPC_FILL(ws + L.off_obits, 0, align_up(static_cast<size_t>(L.obits_words) * 4, 16), st);
-  } else {
-    SPC_FILL(ws + L.off_tout, 0xFF, static_cast<size_t>(L.cap_out) * 8, st);
-    if (K64) SPC_FILL(ws + L.off_tout_vals, 0x7F, static_cast<size_t>(L.cap_out) * 4, st);
-  }
-  Table<K64> tout = tout_at<K64>(ws, L);
-  key_t* uniq = reinterpret_cast<key_t*>(ws + L.off_uniq);
-  key_t* sorted = reinterpret_cast<key_t*>(ws + L.off_sorted);
-  bool axes_fit = true;  // mark_outputs_kernel keeps one bit per kernel offset of an axis
-  for (int d = 0; d < ND; ++d) axes_fit = axes_fit && g.ksize[d] <= 32;
-  if (dense_out && axes_fit) {
-    mark_outputs_kernel<ND><<<blocks_for(n_in), kThreads, 0, st>>>(
-        g, idx, n_in, reinterpret_cast<uint32_t*>(ws + L.off_obits));
-  } else {
-    enumerate_outputs_kernel<ND, K64><<<blocks_for(n_in), kThreads, 0, st>>>(g, idx, n_in, tout, uniq, counters);
-  }
-  SPC_LAUNCH_OK();
-  if (dense_out) {
-    uint32_t* bits = reinterpret_cast<uint32_t*>(ws + L.off_obits);
-    uint32_t* prefix = reinterpret_cast<uint32_t*>(ws + L.off_oprefix);
-    count_bits_kernel<<<blocks_for(L.obits_words), kThreads, 0, st>>>(bits, L.obits_words, prefix);
-    SPC_LAUNCH_OK();
-    size_t scan_bytes = L.scan_bytes;
-    SPC_CUDA_OK(cub::DeviceScan::ExclusiveSum(ws + L.off_scan, scan_bytes, prefix, prefix,
-                                              static_cast<int>(L.obits_words), st));
-    expand_bits_kernel<<<blocks_for(L.obits_words), kThreads, 0, st>>>(
-        bits, prefix, L.obits_words, L.bound, reinterpret_cast<uint32_t*>(sorted), counters);
+  if (!dense_out) {
+    publish_counters_kernel<<<1, 32, 0, st>>>(counters, dev_status, const_cast<int*>(box), ticket);
     SPC_LAUNCH_OK();
   }
-  // The output count reaches the host through a page-locked word that a one-thread kernel writes,
-  // not through a device-to-host copy: a copy would queue on the copy engine behind whatever
-  // transfer the application has in flight (a previous result going back to the host, say) and
-  // stall the whole rulebook chain for its duration.
-  volatile int* box = nullptr;
-  int rc_box = host_mailbox(&box);
-  if (rc_box != SPC_OK) return rc_box;
-  publish_counters_kernel<<<1, 32, 0, st>>>(counters, dev_status, const_cast<int*>(box));
-  SPC_LAUNCH_OK();
-  {
-    const int rc_wait = wait_for_stream(st);
-    if (rc_wait != SPC_OK) return rc_wait;
-  }
-  int host[2] = {box[kUniqueCount], box[kStatus]};
-  const int sticky = box[2];  // the device status word: a bounded wait of an earlier kernel, or a bad row of an earlier layer
+  rc = wait_for_ticket(box, ticket, st);
+  if (rc != SPC_OK) return rc;
+  int host[2] = {box[1], box[2]};
+  const int sticky = box[3];  // the device status word: a bounded wait of an earlier kernel, or a bad row of an earlier layer
   if (host[kStatus] != 0 || sticky != 0) {
     if (dev_status != nullptr && sticky != 0) SPC_CUDA_OK(cudaMemsetAsync(dev_status, 0, sizeof(int), st));
     const int code = host[kStatus] != 0 ? host[kStatus] : sticky;
@@ -1432,22 +1624,65 @@ int emit_masks(const Layout& L, char* ws, int64_t n, int kv, const uint32_t* spl
   return SPC_OK;
 }
 
-// Input-side tables of a strided / transposed layer: pair_bwd and its masks.
-// Reads the output hash the forward phase ranked; shares the mask scratch with
+size_t fill_smem_bytes(int kvp) { return static_cast<size_t>(kThreads / 32) * 32 * fill_pitch(kvp) * 4; }
+
+// Keys and bucket counts of the tile order for a fill kernel, then the order itself.
+void want_order(const Layout& L, char* ws, int64_t n, FillOut* out) {
+  out->keys = reinterpret_cast<uint32_t*>(ws + L.off_keys_a);
+  if (tile_order_needs_buckets(n)) out->counts = reinterpret_cast<uint32_t*>(ws + L.off_order_counts);
+}
+int emit_order(const Layout& L, char* ws, int64_t n, int kv, int32_t* order, cudaStream_t st) {
+  uint32_t* counts = reinterpret_cast<uint32_t*>(ws + L.off_order_counts);
+  return tile_order(reinterpret_cast<const uint32_t*>(ws + L.off_keys_a), n, kv, counts, counts + kOrderCountBytes / 8,
+                    reinterpret_cast<uint2*>(ws + L.off_order_pairs), order, st);
+}
+
+// Input-side tables of a strided / transposed layer: pair_bwd, its masks or its tile order.
+// Reads the output table the forward phase numbered; shares the mask scratch with
 // it, so it must follow the forward phase of the same workspace.
 template <int ND, bool K64>
 int igemm_backward_impl(const Geo& g, const Layout& L, const int32_t* idx, int64_t n_in, int64_t n_out, char* ws,
                         int32_t* pair_bwd, int32_t* mask_bwd, int32_t* argsort_bwd, const uint32_t* split_masks,
-                        int n_split, int do_sort, int32_t* bwd_rm, cudaStream_t st) {
+                        int n_split, int do_sort, int32_t* bwd_rm, int32_t* order_bwd, cudaStream_t st) {
   const int kvp = (g.kv + 3) & ~3;
-  Table<K64> tout = tout_at<K64>(ws, L);
-  uint32_t* words = reinterpret_cast<uint32_t*>(ws + L.off_words);
-  int32_t* iota = mask_bwd != nullptr ? mask_iota(L, ws, split_masks, n_split, do_sort) : nullptr;
-  fill_bwd_kernel<ND, K64><<<blocks_for(n_in), kThreads, 0, st>>>(
-      g, idx, n_in, n_out, tout, pair_bwd, mask_bwd ? words : nullptr, L.mic, bwd_rm, kvp, iota);
+  FillOut out{};
+  out.cm = pair_bwd;
+  out.rm = bwd_rm;
+  if (mask_bwd != nullptr) {
+    out.words = reinterpret_cast<uint32_t*>(ws + L.off_words);
+    out.iota = mask_iota(L, ws, split_masks, n_split, do_sort);
+  }
+  if (order_bwd != nullptr) {
+    // the counts of the output side's order are still there
+    if (tile_order_needs_buckets(n_in)) {
+      Clear c;
+      c.add(ws + L.off_order_counts, 0, kOrderCountBytes);
+      const int rc = launch_clear(c, st);
+      if (rc != SPC_OK) return rc;
+    }
+    want_order(L, ws, n_in, &out);
+  }
+  fill_kernel<ND, K64, true><<<blocks_for(n_in), kThreads, fill_smem_bytes(kvp), st>>>(
+      g, idx, nullptr, n_in, n_out, tout_at<K64>(ws, L), out, L.mic, kvp);
   SPC_LAUNCH_OK();
+  if (order_bwd != nullptr) {
+    const int rc = emit_order(L, ws, n_in, g.kv, order_bwd, st);
+    if (rc != SPC_OK) return rc;
+  }
   if (mask_bwd != nullptr) return emit_masks(L, ws, n_in, g.kv, split_masks, n_split, do_sort, mask_bwd, argsort_bwd, st);
   return SPC_OK;
+}
+
+template <int ND, bool K64>
+int igemm_forward_impl(const Geo& g, const Layout& L, const int32_t* idx, int64_t n_out, char* ws, FillOut out,
+                       int32_t* order_fwd, cudaStream_t st) {
+  using key_t = typename Table<K64>::key_t;
+  const int kvp = (g.kv + 3) & ~3;
+  if (order_fwd != nullptr) want_order(L, ws, n_out, &out);
+  fill_kernel<ND, K64, false><<<blocks_for(n_out), kThreads, fill_smem_bytes(kvp), st>>>(
+      g, idx, reinterpret_cast<const key_t*>(ws + L.off_sorted), n_out, n_out, tin_at<K64>(ws, L), out, L.mic, kvp);
+  SPC_LAUNCH_OK();
+  return order_fwd != nullptr ? emit_order(L, ws, n_out, g.kv, order_fwd, st) : SPC_OK;
 }
 
 template <int ND, bool K64>
@@ -1456,37 +1691,23 @@ int igemm_impl(const Geo& g, const Layout& L, const int32_t* idx, int64_t n_in, 
                int32_t* argsort_fwd, int32_t* mask_bwd, int32_t* argsort_bwd,
                const uint32_t* split_masks, int n_split, int do_sort, int32_t* fwd_rm, int32_t* bwd_rm,
                cudaStream_t st) {
-  using key_t = typename Table<K64>::key_t;
-  const int kvp = (g.kv + 3) & ~3;
-  Table<K64> tin = tin_at<K64>(ws, L);
-  Table<K64> tout = tout_at<K64>(ws, L);
-  const key_t* sorted = reinterpret_cast<const key_t*>(ws + L.off_sorted);
-  uint32_t* words = reinterpret_cast<uint32_t*>(ws + L.off_words);
-  const uint32_t* bitmap = L.shared_bits != nullptr ? L.shared_bits
-                           : (L.bitmap_bytes ? reinterpret_cast<const uint32_t*>(ws + L.off_bitmap) : nullptr);
-  int32_t* iota = mask_iota(L, ws, split_masks, n_split, do_sort);
-  // the row-major copies go through shared memory when a warp's 32 rows fit (kernel volumes up to 32)
-  const bool with_bwd = g.subm && pair_bwd != nullptr;
-  const int staged = (fwd_rm != nullptr && kvp <= 32 && (reinterpret_cast<uintptr_t>(fwd_rm) & 15u) == 0 &&
-                      (!with_bwd || bwd_rm == nullptr || (reinterpret_cast<uintptr_t>(bwd_rm) & 15u) == 0)) ? 1 : 0;
-  const size_t stage_bytes = staged ? static_cast<size_t>(kThreads / 32) * (with_bwd ? 2 : 1) * 32 * kvp * 4 : 0;
-  if (with_bwd) {
-    static bool configured[kMaxDevices] = {false};
-    SPC_CUDA_OK(ensure_dynamic_smem(fill_fwd_kernel<ND, K64, true>, 64 * 1024, configured));
-    fill_fwd_kernel<ND, K64, true><<<blocks_for(n_out), kThreads, stage_bytes, st>>>(
-        g, idx, sorted, n_out, tin, out_indices, pair_fwd, pair_bwd, words, L.mic, fwd_rm, bwd_rm, kvp, bitmap, iota,
-        staged);
-  } else {
-    fill_fwd_kernel<ND, K64, false><<<blocks_for(n_out), kThreads, stage_bytes, st>>>(
-        g, idx, sorted, n_out, tin, out_indices, pair_fwd, nullptr, words, L.mic, fwd_rm, nullptr, kvp, bitmap, iota,
-        staged);
+  FillOut out{};
+  out.out_indices = g.subm ? nullptr : out_indices;
+  out.cm = pair_fwd;
+  out.rm = fwd_rm;
+  if (g.subm && pair_bwd != nullptr) {
+    out.cm_rev = pair_bwd;
+    out.rm_rev = bwd_rm;
   }
-  SPC_LAUNCH_OK();
-  int rc = emit_masks(L, ws, n_out, g.kv, split_masks, n_split, do_sort, mask_fwd, argsort_fwd, st);
+  out.words = reinterpret_cast<uint32_t*>(ws + L.off_words);
+  out.iota = mask_iota(L, ws, split_masks, n_split, do_sort);
+  int rc = igemm_forward_impl<ND, K64>(g, L, idx, n_out, ws, out, nullptr, st);
+  if (rc != SPC_OK) return rc;
+  rc = emit_masks(L, ws, n_out, g.kv, split_masks, n_split, do_sort, mask_fwd, argsort_fwd, st);
   if (rc != SPC_OK) return rc;
   if (!g.subm && pair_bwd != nullptr)
     return igemm_backward_impl<ND, K64>(g, L, idx, n_in, n_out, ws, pair_bwd, mask_bwd, argsort_bwd, split_masks,
-                                        n_split, do_sort, bwd_rm, st);
+                                        n_split, do_sort, bwd_rm, nullptr, st);
   return SPC_OK;
 }
 
@@ -1544,9 +1765,7 @@ int dispatch(int ndim, bool k64, F&& f) {
 // Points `L` at the output bitmap of `producer` if that strided layer numbered its outputs through
 // one and its output grid is this layer's input grid.
 void adopt_producer_bits(const Geo& g, Layout* L, const RulebookProducer* producer) {
-  if (producer == nullptr || producer->geom == nullptr || producer->workspace == nullptr || L->k64 ||
-      L->bitmap_bytes == 0)
-    return;
+  if (producer == nullptr || producer->geom == nullptr || producer->workspace == nullptr || L->k64) return;
   Geo gp;
   if (!make_geo(producer->geom, &gp) || gp.subm || gp.ndim != g.ndim || gp.batch != g.batch) return;
   for (int d = 0; d < g.ndim; ++d)
@@ -1578,44 +1797,41 @@ int rulebook_prepare_chained(const spc_geometry* sg, const int32_t* indices, int
   });
 }
 
-int rulebook_igemm_chained(const spc_geometry* sg, const int32_t* indices, int64_t n_in, int64_t n_out,
-                           void* workspace, size_t workspace_bytes, int32_t* out_indices, int32_t* pair_fwd,
-                           int32_t* pair_bwd, int32_t* mask_fwd, int32_t* argsort_fwd, int32_t* mask_bwd,
-                           int32_t* argsort_bwd, const uint32_t* split_masks, int n_split, int do_sort,
-                           int32_t* pair_fwd_rowmajor, int32_t* pair_bwd_rowmajor, const RulebookProducer* producer,
-                           cudaStream_t st) {
+int rulebook_tables_chained(const spc_geometry* sg, const int32_t* indices, int64_t n_in, int64_t n_out,
+                            void* workspace, size_t workspace_bytes, const RulebookTables& t,
+                            const RulebookProducer* producer, cudaStream_t st) {
   Geo g;
   if (!make_geo(sg, &g)) return fail(SPC_ERR_INVALID_ARGUMENT, "rulebook: bad geometry");
-  // pair_fwd may be absent when the row-major copy is all the caller's GEMMs read (native pass)
-  if (n_in <= 0 || n_out <= 0 || !indices || !workspace || (!pair_fwd && (!pair_fwd_rowmajor || pair_bwd)) || !mask_fwd ||
-      !argsort_fwd || !split_masks || n_split < 1 || n_split > 2)
-    return fail(SPC_ERR_INVALID_ARGUMENT, "rulebook igemm: bad arguments");
-  if (!g.subm && out_indices == nullptr)
-    return fail(SPC_ERR_INVALID_ARGUMENT, "rulebook igemm: out_indices required for non-subm layers");
-  if (g.subm && n_out != n_in) return fail(SPC_ERR_INVALID_ARGUMENT, "rulebook igemm: subm needs n_out == n_in");
-  if ((mask_bwd == nullptr) != (argsort_bwd == nullptr))
-    return fail(SPC_ERR_INVALID_ARGUMENT, "rulebook igemm: mask_bwd and argsort_bwd go together");
+  const bool input_side = t.bwd_colmajor || t.bwd_rowmajor || t.bwd_order;
+  if (n_in <= 0 || n_out <= 0 || !indices || !workspace)
+    return fail(SPC_ERR_INVALID_ARGUMENT, "rulebook tables: bad arguments");
+  if (g.subm && (n_out != n_in || input_side))
+    return fail(SPC_ERR_INVALID_ARGUMENT, "rulebook tables: a submanifold layer has one side");
+  if ((t.fwd_order || t.bwd_order) && g.kv > 32)
+    return fail(SPC_ERR_UNSUPPORTED, "rulebook tables: tile order of %d offsets (32 at most)", g.kv);
+  if ((reinterpret_cast<uintptr_t>(t.fwd_rowmajor) | reinterpret_cast<uintptr_t>(t.bwd_rowmajor)) & 15u)
+    return fail(SPC_ERR_INVALID_ARGUMENT, "rulebook tables: row-major tables must be 16-byte aligned");
   Layout L = make_layout(g, n_in);
   if (workspace_bytes < L.total)
     return fail(SPC_ERR_WORKSPACE_TOO_SMALL, "rulebook: workspace %zu < %zu bytes", workspace_bytes, L.total);
-  if (n_out > L.bound) return fail(SPC_ERR_INVALID_ARGUMENT, "rulebook igemm: n_out exceeds prepared bound");
+  if (n_out > L.bound) return fail(SPC_ERR_INVALID_ARGUMENT, "rulebook tables: n_out exceeds prepared bound");
   adopt_producer_bits(g, &L, producer);
-  // do_sort == 2 (callers inside the library only): order the rows by the tile key.  mask_fwd then
-  // receives the sorted KEYS, not the sorted mask words, and argsort_fwd the tile order.
-  g.tile_key = do_sort == 2 && rulebook_tile_key_applies(sg, pair_bwd != nullptr || mask_bwd != nullptr, split_masks, n_split);
-  do_sort = do_sort != 0;
   char* ws = static_cast<char*>(workspace);
-  return dispatch(g.ndim, L.k64, [&](auto nd, auto k64) {
-    return igemm_impl<decltype(nd)::value, decltype(k64)::value>(
-        g, L, indices, n_in, n_out, ws, out_indices, pair_fwd, pair_bwd, mask_fwd, argsort_fwd, mask_bwd,
-        argsort_bwd, split_masks, n_split, do_sort, pair_fwd_rowmajor, pair_bwd_rowmajor, st);
+  return dispatch(g.ndim, L.k64, [&](auto nd, auto k64) -> int {
+    constexpr int ND = decltype(nd)::value;
+    constexpr bool K64 = decltype(k64)::value;
+    if (t.fwd_colmajor || t.fwd_rowmajor || t.fwd_order || t.out_indices) {
+      FillOut out{};
+      out.out_indices = g.subm ? nullptr : t.out_indices;
+      out.cm = t.fwd_colmajor;
+      out.rm = t.fwd_rowmajor;
+      const int rc = igemm_forward_impl<ND, K64>(g, L, indices, n_out, ws, out, t.fwd_order, st);
+      if (rc != SPC_OK) return rc;
+    }
+    if (!input_side) return SPC_OK;
+    return igemm_backward_impl<ND, K64>(g, L, indices, n_in, n_out, ws, t.bwd_colmajor, nullptr, nullptr, nullptr, 1, 0,
+                                        t.bwd_rowmajor, t.bwd_order, st);
   });
-}
-
-bool rulebook_tile_key_applies(const spc_geometry* sg, bool with_backward, const uint32_t* split_masks, int n_split) {
-  Geo g;
-  return make_geo(sg, &g) && g.kv > 1 && g.kv <= 31 && !with_backward && n_split == 1 && split_masks != nullptr &&
-         split_masks[0] == 0xffffffffu;
 }
 
 }  // namespace spc
@@ -1635,6 +1851,15 @@ extern "C" int spc_rulebook_prepare(const spc_geometry* sg, const int32_t* indic
                                   static_cast<cudaStream_t>(stream));
 }
 
+extern "C" int spc_rulebook_tables(const spc_geometry* sg, const int32_t* indices, int64_t n_in, int64_t n_out,
+                                   void* workspace, size_t workspace_bytes, int32_t* out_indices,
+                                   int32_t* pair_fwd, int32_t* pair_fwd_rowmajor, int32_t* order_fwd,
+                                   int32_t* pair_bwd, int32_t* pair_bwd_rowmajor, int32_t* order_bwd, void* stream) {
+  const RulebookTables t{out_indices, pair_fwd, pair_fwd_rowmajor, order_fwd, pair_bwd, pair_bwd_rowmajor, order_bwd};
+  return rulebook_tables_chained(sg, indices, n_in, n_out, workspace, workspace_bytes, t, nullptr,
+                                 static_cast<cudaStream_t>(stream));
+}
+
 extern "C" int spc_rulebook_igemm(const spc_geometry* sg, const int32_t* indices, int64_t n_in,
                                   int64_t n_out, void* workspace, size_t workspace_bytes,
                                   int32_t* out_indices, int32_t* pair_fwd, int32_t* pair_bwd,
@@ -1642,10 +1867,27 @@ extern "C" int spc_rulebook_igemm(const spc_geometry* sg, const int32_t* indices
                                   int32_t* argsort_bwd, const uint32_t* split_masks, int n_split,
                                   int do_sort, int32_t* pair_fwd_rowmajor, int32_t* pair_bwd_rowmajor,
                                   void* stream) {
-  if (!pair_fwd) return fail(SPC_ERR_INVALID_ARGUMENT, "rulebook igemm: bad arguments");
-  return rulebook_igemm_chained(sg, indices, n_in, n_out, workspace, workspace_bytes, out_indices, pair_fwd, pair_bwd,
-                                mask_fwd, argsort_fwd, mask_bwd, argsort_bwd, split_masks, n_split, do_sort != 0,
-                                pair_fwd_rowmajor, pair_bwd_rowmajor, nullptr, static_cast<cudaStream_t>(stream));
+  Geo g;
+  if (!make_geo(sg, &g)) return fail(SPC_ERR_INVALID_ARGUMENT, "rulebook: bad geometry");
+  if (n_in <= 0 || n_out <= 0 || !indices || !workspace || !pair_fwd || !mask_fwd || !argsort_fwd || !split_masks ||
+      n_split < 1 || n_split > 2)
+    return fail(SPC_ERR_INVALID_ARGUMENT, "rulebook igemm: bad arguments");
+  if (!g.subm && out_indices == nullptr)
+    return fail(SPC_ERR_INVALID_ARGUMENT, "rulebook igemm: out_indices required for non-subm layers");
+  if (g.subm && n_out != n_in) return fail(SPC_ERR_INVALID_ARGUMENT, "rulebook igemm: subm needs n_out == n_in");
+  if ((mask_bwd == nullptr) != (argsort_bwd == nullptr))
+    return fail(SPC_ERR_INVALID_ARGUMENT, "rulebook igemm: mask_bwd and argsort_bwd go together");
+  const Layout L = make_layout(g, n_in);
+  if (workspace_bytes < L.total)
+    return fail(SPC_ERR_WORKSPACE_TOO_SMALL, "rulebook: workspace %zu < %zu bytes", workspace_bytes, L.total);
+  if (n_out > L.bound) return fail(SPC_ERR_INVALID_ARGUMENT, "rulebook igemm: n_out exceeds prepared bound");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  char* ws = static_cast<char*>(workspace);
+  return dispatch(g.ndim, L.k64, [&](auto nd, auto k64) {
+    return igemm_impl<decltype(nd)::value, decltype(k64)::value>(
+        g, L, indices, n_in, n_out, ws, out_indices, pair_fwd, pair_bwd, mask_fwd, argsort_fwd, mask_bwd,
+        argsort_bwd, split_masks, n_split, do_sort, pair_fwd_rowmajor, pair_bwd_rowmajor, st);
+  });
 }
 
 extern "C" int spc_rulebook_igemm_backward(const spc_geometry* sg, const int32_t* indices, int64_t n_in,
@@ -1669,7 +1911,7 @@ extern "C" int spc_rulebook_igemm_backward(const spc_geometry* sg, const int32_t
   return dispatch(g.ndim, L.k64, [&](auto nd, auto k64) {
     return igemm_backward_impl<decltype(nd)::value, decltype(k64)::value>(
         g, L, indices, n_in, n_out, ws, pair_bwd, mask_bwd, argsort_bwd, split_masks, n_split, do_sort,
-        pair_bwd_rowmajor, st);
+        pair_bwd_rowmajor, nullptr, st);
   });
 }
 

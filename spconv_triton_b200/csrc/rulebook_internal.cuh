@@ -21,20 +21,23 @@ struct RulebookProducer {
   int64_t n_in;           // the n_in that workspace was laid out for
 };
 
-// spc_rulebook_prepare / spc_rulebook_igemm with an optional producer (nullptr = the plain calls).
+// What rulebook_tables_chained writes; every pointer may be null, the row-major tables are 16-byte aligned.
+struct RulebookTables {
+  int32_t* out_indices;   // [n_out, ndim + 1], strided / transposed layers
+  int32_t* fwd_colmajor;  // [kv, n_out]
+  int32_t* fwd_rowmajor;  // [n_out, kvp], -1 padded
+  int32_t* fwd_order;     // [n_out]: rows grouped so that the 128 rows of a gather-GEMM tile share offsets (kv <= 32)
+  int32_t* bwd_colmajor;  // the same for the input side of a strided / transposed layer
+  int32_t* bwd_rowmajor;
+  int32_t* bwd_order;
+};
+
+// spc_rulebook_prepare / spc_rulebook_tables with an optional producer (nullptr = the plain calls).
 int rulebook_prepare_chained(const spc_geometry* g, const int32_t* indices, int64_t n_in, void* workspace,
                              size_t workspace_bytes, int64_t* n_out_host, const RulebookProducer* producer,
                              cudaStream_t stream);
-int rulebook_igemm_chained(const spc_geometry* g, const int32_t* indices, int64_t n_in, int64_t n_out,
-                           void* workspace, size_t workspace_bytes, int32_t* out_indices, int32_t* pair_fwd,
-                           int32_t* pair_bwd, int32_t* mask_fwd, int32_t* argsort_fwd, int32_t* mask_bwd,
-                           int32_t* argsort_bwd, const uint32_t* split_masks, int n_split, int do_sort,
-                           int32_t* pair_fwd_rowmajor, int32_t* pair_bwd_rowmajor,
-                           const RulebookProducer* producer, cudaStream_t stream);
-// do_sort == 2 in rulebook_igemm_chained asks for the tile-key order (rows grouped so that the 128
-// rows of a gather-GEMM tile share kernel offsets; mask_fwd then holds sorted keys, not sorted mask
-// words).  It applies to single-word masks, one split that keeps every bit and no input-side tables;
-// otherwise 2 means 1.  This tells a caller in advance which of the two it will get.
-bool rulebook_tile_key_applies(const spc_geometry* g, bool with_backward, const uint32_t* split_masks, int n_split);
+int rulebook_tables_chained(const spc_geometry* g, const int32_t* indices, int64_t n_in, int64_t n_out, void* workspace,
+                            size_t workspace_bytes, const RulebookTables& tables, const RulebookProducer* producer,
+                            cudaStream_t stream);
 
 }  // namespace spc

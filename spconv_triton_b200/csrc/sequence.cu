@@ -87,7 +87,6 @@ extern "C" int spc_sequence_forward(const spc_seq_layer* layers, int n_layers, c
 
   Arena arena{static_cast<char*>(arena_ptr), arena_bytes};
   const size_t esize = dtype_size(dtype);
-  const uint32_t split_word = 0xFFFFFFFFu;
 
   // the caller's stream has produced indices and features: the rulebook streams start after it
   SPC_CUDA_OK(cudaEventRecord(ev_input, main));
@@ -141,20 +140,16 @@ extern "C" int spc_sequence_forward(const spc_seq_layer* layers, int n_layers, c
           colmajor = true;
       if (colmajor) R.pair_fwd = arena.take(static_cast<size_t>(kv) * n_out * 4);
       R.pair_fwd_rowmajor = arena.take(static_cast<size_t>(n_out) * kvp * 4);
-      R.pair_mask = arena.take(static_cast<size_t>(n_out) * 4);
       R.mask_argsort = arena.take(static_cast<size_t>(n_out) * 4);
-      R.num_per_loc = arena.take(static_cast<size_t>(kv) * 4);
       if (arena.overflow) break;
-      SPC_CUDA_OK(cudaMemsetAsync(arena.at(R.num_per_loc), 0, static_cast<size_t>(kv) * 4, st));
-      rc = rulebook_igemm_chained(&L.geom, cur_indices, cur_n, n_out, arena.at(R.workspace), ws_bytes,
-                                  subm ? nullptr : static_cast<int32_t*>(arena.at(R.out_indices)),
-                                  colmajor ? static_cast<int32_t*>(arena.at(R.pair_fwd)) : nullptr, nullptr,
-                                  static_cast<int32_t*>(arena.at(R.pair_mask)),
-                                  static_cast<int32_t*>(arena.at(R.mask_argsort)), nullptr, nullptr, &split_word, 1,
-                                  /*do_sort=*/2, static_cast<int32_t*>(arena.at(R.pair_fwd_rowmajor)), nullptr,
-                                  have_producer ? &producer : nullptr, st);
+      RulebookTables t{};
+      t.out_indices = subm ? nullptr : static_cast<int32_t*>(arena.at(R.out_indices));
+      t.fwd_colmajor = colmajor ? static_cast<int32_t*>(arena.at(R.pair_fwd)) : nullptr;
+      t.fwd_rowmajor = static_cast<int32_t*>(arena.at(R.pair_fwd_rowmajor));
+      t.fwd_order = static_cast<int32_t*>(arena.at(R.mask_argsort));
+      rc = rulebook_tables_chained(&L.geom, cur_indices, cur_n, n_out, arena.at(R.workspace), ws_bytes, t,
+                                   have_producer ? &producer : nullptr, st);
       if (rc != SPC_OK) return rc;
-      R.masks_are_exact = rulebook_tile_key_applies(&L.geom, false, &split_word, 1) ? 0 : 1;
       SPC_CUDA_OK(cudaEventRecord(ev[i], st));
       if (!subm) {
         producer = RulebookProducer{&L.geom, arena.at(R.workspace), cur_n};

@@ -48,9 +48,7 @@ class SeqResult(ctypes.Structure):
 
     _fields_ = [("n_in", ctypes.c_int64), ("n_out", ctypes.c_int64), ("workspace", ctypes.c_uint64),
                 ("workspace_bytes", ctypes.c_uint64), ("out_indices", ctypes.c_uint64), ("pair_fwd", ctypes.c_uint64),
-                ("pair_fwd_rowmajor", ctypes.c_uint64), ("pair_mask", ctypes.c_uint64),
-                ("mask_argsort", ctypes.c_uint64), ("num_per_loc", ctypes.c_uint64), ("features", ctypes.c_uint64),
-                ("masks_are_exact", ctypes.c_int64)]
+                ("pair_fwd_rowmajor", ctypes.c_uint64), ("mask_argsort", ctypes.c_uint64), ("features", ctypes.c_uint64)]
 
 
 class _Step:
@@ -246,7 +244,7 @@ def forward(container, x):
         # from its free list without splitting or growing
         arena_bytes = plan.arena_bytes = floor[0] = max(arena_bytes, plan.arena_bytes, floor[0])
         needed = ctypes.c_size_t(0)
-        for _attempt in range(4):
+        for _attempt in range(8):
             # The rulebook streams touch the arena and the indices only inside the call, and the
             # caller's stream joins both before the call returns: to the caching allocator the
             # arena is a block of the caller's stream like any other (no record_stream, whose
@@ -327,15 +325,11 @@ def _wrap(plan, x, indices, arena, dev, keep):
             pair_fwd = _column_major(rowmajor, kv, late, _view(arena, R.pair_fwd, kv * n_out, torch.int32, (kv, n_out)))
         else:
             pair_fwd = None  # not written: no layer of the pass reads it
-        exact = int(R.masks_are_exact) != 0
-        pm = [_view(arena, R.pair_mask, n_out, torch.int32, (n_out, 1))] if exact else None
-        ma = [_view(arena, R.mask_argsort, n_out, torch.int32, (n_out,))] if exact else None
         masks = [np.array([0xFFFFFFFF], dtype=np.uint32)]
         data = ImplicitGemmIndiceData(
-            in_indices if c.subm else cur_indices, in_indices, pair_fwd, torch.Tensor(), pm, [], ma, [], masks,
+            in_indices if c.subm else cur_indices, in_indices, pair_fwd, torch.Tensor(), None, [], None, [], masks,
             st.in_shape, st.out_shape, c.subm, c.algo, c.kernel_size, c.stride, c.dilation, c.padding)
-        if not exact:
-            data._masks_fwd_thunk = functools.partial(_exact_masks, rowmajor, kv)
+        data._masks_fwd_thunk = functools.partial(_exact_masks, rowmajor, kv)
         if pair_fwd is None:
             data._pair_fwd_thunk = functools.partial(_column_major, rowmajor, kv, late)
         data._late = late
