@@ -462,13 +462,13 @@ ingest_kernel(const __grid_constant__ Geo g, const int32_t* __restrict__ idx, lo
 }
 
 // ------------------------------------------------------------------------
-// Numbering the set bits of the input and the output bitmap in ascending cell order.  A block owns 4096
+// Numbering the set bits of the input and the output bitmap in ascending cell order.  A block owns 2048
 // words.  count_cells_kernel adds up every block's bits; its last block to finish turns the sums into
 // starts and hands the output count to the host, which can then allocate while number_cells_kernel gives
 // every word the number of bits before it and lists the output cells.  (A library scan over the words plus
 // separate counting, listing and publishing kernels was five launches more per bitmap.)
 // ------------------------------------------------------------------------
-constexpr int kCellBlock = 4096;
+constexpr int kCellBlock = 2048;
 constexpr int kWordsPerThread = kCellBlock / kThreads;
 
 struct Cells {
@@ -540,12 +540,22 @@ count_cells_kernel(const __grid_constant__ Cells c, int* counters, const int* de
   for (int s = 0; s < 2; ++s) {
     volatile uint32_t* starts = c.starts[s];
     uint32_t carry = 0;
-    for (int b0 = 0; b0 < c.blocks[s]; b0 += kThreads) {
-      const int b = b0 + threadIdx.x;
-      const uint32_t v = b < c.blocks[s] ? starts[b] : 0u;
-      uint32_t all;
-      const uint32_t before = block_exclusive_sum(v, warp_sums, &all);
-      if (b < c.blocks[s]) starts[b] = carry + before;
+    constexpr int kEach = 4;
+    for (int b0 = 0; b0 < c.blocks[s]; b0 += kEach * kThreads) {
+      uint32_t v[kEach], sum4 = 0, all;
+#pragma unroll
+      for (int q = 0; q < kEach; ++q) {
+        const int b = b0 + threadIdx.x * kEach + q;
+        v[q] = b < c.blocks[s] ? starts[b] : 0u;
+        sum4 += v[q];
+      }
+      uint32_t before = carry + block_exclusive_sum(sum4, warp_sums, &all);
+#pragma unroll
+      for (int q = 0; q < kEach; ++q) {
+        const int b = b0 + threadIdx.x * kEach + q;
+        if (b < c.blocks[s]) starts[b] = before;
+        before += v[q];
+      }
       carry += all;
     }
     if (threadIdx.x == 0 && c.blocks[s] != 0) {
@@ -596,7 +606,15 @@ number_cells_kernel(const __grid_constant__ Cells c, long long limit, uint32_t* 
     at += __shfl_sync(0xffffffffu, incl, 31);
     if (word[i] != 0) prefix[first + i * 32] = before;
     if (side == 0) continue;
-    // the warp lists one word's cells at a time: consecutive lanes write consecutive entries
+    const uint32_t in_warp = __shfl_sync(0xffffffffu, incl, 31);
+    if (in_warp <= 8 * 32) {
+      // few cells a word: every lane lists those of its own
+      uint32_t to = before;
+      for (uint32_t w = word[i]; w != 0 && to < limit; w &= w - 1)
+        sorted[to++] = static_cast<uint32_t>((first + i * 32) * 32 + __ffs(w) - 1);
+      continue;
+    }
+    // many: the warp lists one word's cells at a time, consecutive lanes to consecutive entries
     unsigned some = __ballot_sync(0xffffffffu, word[i] != 0);
     while (some != 0) {
       const int src = __ffs(some) - 1;
@@ -731,7 +749,120 @@ __host__ __device__ __forceinline__ int fill_pitch(int kvp) {
   return (w & 7) == 4 ? w : w + 4;
 }
 
-template <int ND, bool K64, bool BWD>
+// Looks a row's K^ND neighbours up, everything about the offsets known at compile time: the cells of every
+// axis are found once, and the loads of up to nine lines (bitmap) or nine cells (hash table) are requested
+// together, so that a row waits for the L2 three times, not once a line.  With the offsets in loops the kernel
+// took 32 us for 2 000 rows, all of it latency; the common kernels (2 and 3 wide) are worth the code.
+template <int ND, bool K64, int K, typename Emit>
+__device__ __forceinline__ void look_up_cube(const Geo& g, bool div, const int* own, const int* limit,
+                                             const Table<K64>& table, const Emit& emit) {
+  using key_t = typename Table<K64>::key_t;
+  constexpr int kAll = ND == 1 ? 1 : ND == 2 ? K : K * K;  // lines along the last axis
+  constexpr int kGroup = K64 || kAll < 3 ? 1 : 3;          // lines probed together without a bitmap
+  int x[ND][K];
+#pragma unroll
+  for (int d = 0; d < ND; ++d)
+#pragma unroll
+    for (int k = 0; k < K; ++k) x[d][k] = axis_cell(g, div, d, own[d + 1], k, limit[d]);
+  bool on[kAll];
+  key_t base[kAll];
+#pragma unroll
+  for (int l = 0; l < kAll; ++l) {
+    const int p0 = ND == 3 ? l / K : l, p1 = l % K;
+    key_t key = static_cast<key_t>(own[0]);
+    on[l] = true;
+    if (ND >= 2) {
+      on[l] = x[0][p0] >= 0;
+      key = key * static_cast<key_t>(limit[0]) + static_cast<key_t>(x[0][p0]);
+    }
+    if (ND == 3) {
+      on[l] = on[l] && x[ND > 1 ? 1 : 0][p1] >= 0;
+      key = key * static_cast<key_t>(limit[ND > 1 ? 1 : 0]) + static_cast<key_t>(x[ND > 1 ? 1 : 0][p1]);
+    }
+    base[l] = key * static_cast<key_t>(limit[ND - 1]);
+  }
+  const uint32_t* bits = dense_bits(table);
+  if (bits != nullptr) {
+    const uint32_t* prefix = dense_prefix(table);
+    const int32_t* perm = row_permutation(table);
+    int lo = INT_MAX, hi = -1;
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      if (x[ND - 1][k] >= 0) {
+        lo = min(lo, x[ND - 1][k]);
+        hi = max(hi, x[ND - 1][k]);
+      }
+    if (hi < 0) return;
+    uint32_t w0[kAll], w1[kAll], before[kAll];
+#pragma unroll
+    for (int l = 0; l < kAll; ++l) {
+      const key_t at = base[l] + static_cast<key_t>(lo);
+      w0[l] = on[l] ? __ldg(&bits[at >> 5]) : 0u;
+      w1[l] = on[l] && static_cast<int>(at & 31) + hi - lo >= 32 ? __ldg(&bits[(at >> 5) + 1]) : 0u;
+    }
+    uint32_t hits[kAll];
+#pragma unroll
+    for (int l = 0; l < kAll; ++l) {
+      const key_t at = base[l] + static_cast<key_t>(lo);
+      const unsigned long long win = ((static_cast<unsigned long long>(w1[l]) << 32) | w0[l]) >> (at & 31);
+      hits[l] = 0;
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (x[ND - 1][k] >= 0) hits[l] |= static_cast<uint32_t>((win >> (x[ND - 1][k] - lo)) & 1ull) << k;
+      // (a word without bits has no prefix: the second word's rows then come first)
+      before[l] = hits[l] != 0 ? __ldg(&prefix[(at >> 5) + (w0[l] == 0 ? 1 : 0)]) : 0u;
+    }
+#pragma unroll
+    for (int l0 = 0; l0 < kAll; l0 += (kAll < 3 ? 1 : 3)) {
+      constexpr int kStep = kAll < 3 ? 1 : 3;
+      int row[kStep * K];
+#pragma unroll
+      for (int b = 0; b < kStep; ++b) {
+        const int l = l0 + b < kAll ? l0 + b : kAll - 1;
+        const int sh = static_cast<int>((base[l] + static_cast<key_t>(lo)) & 31);
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          int j = -1;
+          if (l0 + b < kAll && ((hits[l] >> k) & 1u)) {
+            const int bit = sh + x[ND - 1][k] - lo;
+            j = static_cast<int>(before[l]) + (bit < 32 ? __popc(w0[l] & ((1u << bit) - 1u))
+                                                        : __popc(w0[l]) + __popc(w1[l] & ((1u << (bit - 32)) - 1u)));
+            if (perm != nullptr) j = __ldg(&perm[j]);
+          }
+          row[b * K + k] = j;
+        }
+      }
+#pragma unroll
+      for (int b = 0; b < kStep; ++b)
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+          if (l0 + b < kAll) emit((l0 + b) * K + k, row[b * K + k]);
+    }
+    return;
+  }
+#pragma unroll
+  for (int l0 = 0; l0 < kAll; l0 += kGroup) {
+    unsigned long long probe[kGroup * K];
+#pragma unroll
+    for (int b = 0; b < kGroup; ++b)
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const int l = l0 + b < kAll ? l0 + b : kAll - 1;
+        const bool want = l0 + b < kAll && on[l] && x[ND - 1][k] >= 0;
+        probe[b * K + k] = want ? table.first_probe(base[l] + static_cast<key_t>(x[ND - 1][k])) : 0ull;
+      }
+#pragma unroll
+    for (int b = 0; b < kGroup; ++b)
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const int l = l0 + b < kAll ? l0 + b : kAll - 1;
+        if (l0 + b < kAll && on[l] && x[ND - 1][k] >= 0)
+          emit(l * K + k, table.finish(base[l] + static_cast<key_t>(x[ND - 1][k]), probe[b * K + k]));
+      }
+  }
+}
+
+template <int ND, bool K64, bool BWD, int K>
 __global__ void __launch_bounds__(kThreads)
 fill_kernel(const __grid_constant__ Geo g, const int32_t* __restrict__ idx,
             const typename Table<K64>::key_t* __restrict__ sorted, long long n, long long n_limit, Table<K64> table,
@@ -788,7 +919,7 @@ fill_kernel(const __grid_constant__ Geo g, const int32_t* __restrict__ idx,
 #pragma unroll
   for (int d = 0; d < ND; ++d) {
     uint32_t m = 0;
-    if (ok && g.axes_fit)
+    if (K == 0 && ok && g.axes_fit)
       for (int k = 0; k < g.ksize[d]; ++k)
         m |= static_cast<uint32_t>(axis_cell(g, div, d, own[d + 1], k, limit[d]) >= 0) << k;
     valid[d] = m;
@@ -824,7 +955,9 @@ fill_kernel(const __grid_constant__ Geo g, const int32_t* __restrict__ idx,
       word |= 1u << (k - c0);
       if (out.keys != nullptr) order_word |= 1u << g.key_pos[k];
     };
-    if (ok && g.axes_fit && q_hi >= 0) {
+    if constexpr (K != 0) {
+      if (ok) look_up_cube<ND, K64, K>(g, div, own, limit, table, emit);
+    } else if (ok && g.axes_fit && q_hi >= 0) {
       int pos[ND];  // offsets of the leading axes
       const int l0 = c0 / kl, l1 = (c1 - 1) / kl;
       {
@@ -1624,7 +1757,32 @@ int emit_masks(const Layout& L, char* ws, int64_t n, int kv, const uint32_t* spl
   return SPC_OK;
 }
 
+// Kernel width of a cube-shaped kernel with a fill kernel of its own, else 0.
+int cube_width(const Geo& g) {
+  for (int d = 0; d < g.ndim; ++d)
+    if (g.ksize[d] != g.ksize[0] || g.dil[d] != 1) return 0;
+  return g.ndim <= 3 && (g.ksize[0] == 2 || g.ksize[0] == 3) ? g.ksize[0] : 0;
+}
 size_t fill_smem_bytes(int kvp) { return static_cast<size_t>(kThreads / 32) * 32 * fill_pitch(kvp) * 4; }
+
+template <int ND, bool K64, bool BWD>
+int launch_fill(const Geo& g, const int32_t* idx, const typename Table<K64>::key_t* sorted, int64_t n, int64_t n_limit,
+                const Table<K64>& table, const FillOut& out, int mic, cudaStream_t st) {
+  const int kvp = (g.kv + 3) & ~3;
+  const unsigned blocks = blocks_for(n);
+  const size_t smem = fill_smem_bytes(kvp);
+  const int width = cube_width(g);
+  if constexpr (ND <= 3) {
+    if (width == 3)
+      fill_kernel<ND, K64, BWD, 3><<<blocks, kThreads, smem, st>>>(g, idx, sorted, n, n_limit, table, out, mic, kvp);
+    else if (width == 2)
+      fill_kernel<ND, K64, BWD, 2><<<blocks, kThreads, smem, st>>>(g, idx, sorted, n, n_limit, table, out, mic, kvp);
+  }
+  if (ND > 3 || width == 0)
+    fill_kernel<ND, K64, BWD, 0><<<blocks, kThreads, smem, st>>>(g, idx, sorted, n, n_limit, table, out, mic, kvp);
+  SPC_LAUNCH_OK();
+  return SPC_OK;
+}
 
 // Keys and bucket counts of the tile order for a fill kernel, then the order itself.
 void want_order(const Layout& L, char* ws, int64_t n, FillOut* out) {
@@ -1644,7 +1802,6 @@ template <int ND, bool K64>
 int igemm_backward_impl(const Geo& g, const Layout& L, const int32_t* idx, int64_t n_in, int64_t n_out, char* ws,
                         int32_t* pair_bwd, int32_t* mask_bwd, int32_t* argsort_bwd, const uint32_t* split_masks,
                         int n_split, int do_sort, int32_t* bwd_rm, int32_t* order_bwd, cudaStream_t st) {
-  const int kvp = (g.kv + 3) & ~3;
   FillOut out{};
   out.cm = pair_bwd;
   out.rm = bwd_rm;
@@ -1662,9 +1819,8 @@ int igemm_backward_impl(const Geo& g, const Layout& L, const int32_t* idx, int64
     }
     want_order(L, ws, n_in, &out);
   }
-  fill_kernel<ND, K64, true><<<blocks_for(n_in), kThreads, fill_smem_bytes(kvp), st>>>(
-      g, idx, nullptr, n_in, n_out, tout_at<K64>(ws, L), out, L.mic, kvp);
-  SPC_LAUNCH_OK();
+  const int rc_fill = launch_fill<ND, K64, true>(g, idx, nullptr, n_in, n_out, tout_at<K64>(ws, L), out, L.mic, st);
+  if (rc_fill != SPC_OK) return rc_fill;
   if (order_bwd != nullptr) {
     const int rc = emit_order(L, ws, n_in, g.kv, order_bwd, st);
     if (rc != SPC_OK) return rc;
@@ -1677,11 +1833,10 @@ template <int ND, bool K64>
 int igemm_forward_impl(const Geo& g, const Layout& L, const int32_t* idx, int64_t n_out, char* ws, FillOut out,
                        int32_t* order_fwd, cudaStream_t st) {
   using key_t = typename Table<K64>::key_t;
-  const int kvp = (g.kv + 3) & ~3;
   if (order_fwd != nullptr) want_order(L, ws, n_out, &out);
-  fill_kernel<ND, K64, false><<<blocks_for(n_out), kThreads, fill_smem_bytes(kvp), st>>>(
-      g, idx, reinterpret_cast<const key_t*>(ws + L.off_sorted), n_out, n_out, tin_at<K64>(ws, L), out, L.mic, kvp);
-  SPC_LAUNCH_OK();
+  const int rc = launch_fill<ND, K64, false>(g, idx, reinterpret_cast<const key_t*>(ws + L.off_sorted), n_out, n_out,
+                                             tin_at<K64>(ws, L), out, L.mic, st);
+  if (rc != SPC_OK) return rc;
   return order_fwd != nullptr ? emit_order(L, ws, n_out, g.kv, order_fwd, st) : SPC_OK;
 }
 

@@ -11,41 +11,43 @@
 // order, so the result is the exact sort except inside buckets longer than a piece: 0 - 3 % more
 // (tile, offset) stages than the exact order of the tile key on every level of the backbone and UNet
 // workloads (two offsets instead of three: up to 7 %; no buckets, only pieces: 100 - 500 %).
-#include <cub/block/block_radix_sort.cuh>
-
 #include "common.cuh"
 #include "tile_order.cuh"
 
 namespace spc {
 namespace {
 
+constexpr int kDealThreads = 512;
+constexpr int kDealItems = 8;
 constexpr int kPieceThreads = 1024;
-constexpr int kPieceItems = kTileOrderPiece / kPieceThreads;
+constexpr int kPieceWarps = kPieceThreads / 32;
+constexpr int kDigitBits = 9;
+constexpr int kDigits = 1 << kDigitBits;
 
-// One CTA deals 8192 rows: counts them per bucket in shared memory, reserves that much of every bucket it
+// One CTA deals 4096 rows: counts them per bucket in shared memory, reserves that much of every bucket it
 // meets with one atomic, and writes (key, row) to its places.  Rows of a bucket come in any order.
-__global__ void __launch_bounds__(kPieceThreads)
+__global__ void __launch_bounds__(kDealThreads)
 deal_rows_kernel(const uint32_t* __restrict__ keys, long long n, const uint32_t* __restrict__ counts,
                  uint32_t* __restrict__ taken, uint2* __restrict__ pairs) {
   __shared__ uint32_t place[kTileBuckets];  // rows of this CTA in the bucket, then where they go
-  __shared__ uint32_t warp_sum[32];
+  __shared__ uint32_t warp_sum[kDealThreads / 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int b = tid; b < kTileBuckets; b += kPieceThreads) place[b] = 0;
+  for (int b = tid; b < kTileBuckets; b += kDealThreads) place[b] = 0;
   __syncthreads();
-  const long long first = blockIdx.x * static_cast<long long>(kTileOrderPiece);
-  uint32_t key[kPieceItems];
-  int bucket[kPieceItems];
-  uint32_t rank[kPieceItems];
+  const long long first = blockIdx.x * static_cast<long long>(kDealThreads * kDealItems);
+  uint32_t key[kDealItems];
+  int bucket[kDealItems];
+  uint32_t rank[kDealItems];
 #pragma unroll
-  for (int i = 0; i < kPieceItems; ++i) {
-    const long long r = first + i * kPieceThreads + tid;
+  for (int i = 0; i < kDealItems; ++i) {
+    const long long r = first + i * kDealThreads + tid;
     key[i] = r < n ? keys[r] : 0u;
     bucket[i] = r < n ? bucket_of(gray_encode(key[i])) : -1;
   }
 #pragma unroll
-  for (int i = 0; i < kPieceItems; ++i) rank[i] = bucket[i] >= 0 ? atomicAdd(&place[bucket[i]], 1u) : 0u;
-  // start of every bucket: exclusive sum of all rows' counts, six consecutive buckets a thread
-  constexpr int kPer = (kTileBuckets + kPieceThreads - 1) / kPieceThreads;
+  for (int i = 0; i < kDealItems; ++i) rank[i] = bucket[i] >= 0 ? atomicAdd(&place[bucket[i]], 1u) : 0u;
+  // start of every bucket: exclusive sum of all rows' counts, eleven consecutive buckets a thread
+  constexpr int kPer = (kTileBuckets + kDealThreads - 1) / kDealThreads;
   uint32_t mine[kPer], sum = 0;
 #pragma unroll
   for (int q = 0; q < kPer; ++q) {
@@ -75,53 +77,107 @@ deal_rows_kernel(const uint32_t* __restrict__ keys, long long n, const uint32_t*
   }
   __syncthreads();
 #pragma unroll
-  for (int i = 0; i < kPieceItems; ++i) {
+  for (int i = 0; i < kDealItems; ++i) {
     if (bucket[i] < 0) continue;
     const long long at = static_cast<long long>(place[bucket[i]]) + rank[i];
-    if (at < n) pairs[at] = make_uint2(key[i], static_cast<uint32_t>(first + i * kPieceThreads + tid));
+    if (at < n) pairs[at] = make_uint2(key[i], static_cast<uint32_t>(first + i * kDealThreads + tid));
   }
 }
 
 // order[piece] = the piece's rows in ascending key order.  `pairs` null: the rows are 0..n-1 with `keys`.
+// A least-significant-digit radix sort in shared memory: nine bits a pass, so three passes for the 27
+// offsets of a 3x3x3 kernel.  A warp ranks its rows 32 at a time (lanes with the same digit find each other
+// with a match, the first of them adds to the warp's count of that digit), then the counts of all warps
+// become places by one block-wide sum in (digit, warp) order, which keeps the sort stable.
 template <int ITEMS>
 __global__ void __launch_bounds__(kPieceThreads)
 sort_piece_kernel(const uint32_t* __restrict__ keys, const uint2* __restrict__ pairs, long long n, int key_bits,
                   int32_t* __restrict__ order) {
-  using Sort = cub::BlockRadixSort<uint32_t, kPieceThreads, ITEMS, int32_t>;
-  extern __shared__ __align__(16) unsigned char temp[];
+  extern __shared__ __align__(16) unsigned char smem[];
+  uint2* item = reinterpret_cast<uint2*>(smem);                                   // [kPieceThreads * ITEMS]
+  uint16_t* count = reinterpret_cast<uint16_t*>(item + kPieceThreads * ITEMS);    // [kDigits][kPieceWarps]
+  __shared__ uint32_t warp_sum[kPieceWarps];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const long long first = blockIdx.x * static_cast<long long>(kPieceThreads * ITEMS);
-  const long long left = n - first;
-  uint32_t key[ITEMS];
-  int32_t row[ITEMS];
+  const int left = static_cast<int>(n - first < kPieceThreads * ITEMS ? n - first : kPieceThreads * ITEMS);
+  uint2 mine[ITEMS];
+  const int at0 = warp * 32 * ITEMS + lane;  // a warp's rows are consecutive
 #pragma unroll
   for (int i = 0; i < ITEMS; ++i) {
-    const int at = threadIdx.x * ITEMS + i;
-    key[i] = 0xffffffffu;  // past the end: sorts behind every key and is not written
-    row[i] = -1;
-    if (at < left) {
-      if (pairs != nullptr) {
-        const uint2 p = pairs[first + at];
-        key[i] = p.x;
-        row[i] = static_cast<int32_t>(p.y);
-      } else {
-        key[i] = keys[at];
-        row[i] = at;
-      }
+    const int at = at0 + i * 32;
+    mine[i] = make_uint2(0u, 0u);
+    if (at < left) mine[i] = pairs != nullptr ? pairs[first + at] : make_uint2(keys[at], static_cast<uint32_t>(at));
+  }
+  for (int bit = 0; bit < key_bits; bit += kDigitBits) {
+    for (int i = tid; i < kDigits * kPieceWarps / 8; i += kPieceThreads)
+      reinterpret_cast<uint4*>(count)[i] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+    uint32_t rank[ITEMS];
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+      const bool live = at0 + i * 32 < left;
+      const int digit = live ? static_cast<int>((mine[i].x >> bit) & (kDigits - 1)) : kDigits;
+      const unsigned same = __match_any_sync(0xffffffffu, digit);
+      uint32_t before = 0;
+      if (live) before = count[digit * kPieceWarps + warp];
+      __syncwarp();
+      if (live && __ffs(same) - 1 == lane) count[digit * kPieceWarps + warp] = static_cast<uint16_t>(before + __popc(same));
+      __syncwarp();
+      rank[i] = before + __popc(same & ((1u << lane) - 1u));
     }
-  }
-  Sort(*reinterpret_cast<typename Sort::TempStorage*>(temp)).SortBlockedToStriped(key, row, 0, key_bits);
+    __syncthreads();
+    // exclusive sum over the counts, sixteen consecutive ones a thread
+    constexpr int kEach = kDigits * kPieceWarps / kPieceThreads;
+    uint32_t sum = 0;
+    uint16_t c[kEach];
+    static_assert(kEach == 16, "two 16-byte words of counts a thread");
+    reinterpret_cast<uint4*>(c)[0] = reinterpret_cast<const uint4*>(count)[2 * tid];
+    reinterpret_cast<uint4*>(c)[1] = reinterpret_cast<const uint4*>(count)[2 * tid + 1];
 #pragma unroll
-  for (int i = 0; i < ITEMS; ++i) {
-    const int at = i * kPieceThreads + threadIdx.x;
-    if (at < left) order[first + at] = row[i];
+    for (int q = 0; q < kEach; ++q) sum += c[q];
+    uint32_t incl = sum;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, off);
+      if (lane >= off) incl += t;
+    }
+    if (lane == 31) warp_sum[warp] = incl;
+    __syncthreads();
+    uint32_t total = warp_sum[lane];
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, total, off);
+      if (lane >= off) total += t;
+    }
+    uint32_t start = __shfl_sync(0xffffffffu, total, warp > 0 ? warp - 1 : 0);
+    start = (warp > 0 ? start : 0u) + incl - sum;
+#pragma unroll
+    for (int q = 0; q < kEach; ++q) {
+      const uint32_t v = c[q];
+      c[q] = static_cast<uint16_t>(start);
+      start += v;
+    }
+    reinterpret_cast<uint4*>(count)[2 * tid] = reinterpret_cast<const uint4*>(c)[0];
+    reinterpret_cast<uint4*>(count)[2 * tid + 1] = reinterpret_cast<const uint4*>(c)[1];
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i)
+      if (at0 + i * 32 < left)
+        item[count[((mine[i].x >> bit) & (kDigits - 1)) * kPieceWarps + warp] + rank[i]] = mine[i];
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i)
+      if (at0 + i * 32 < left) mine[i] = item[at0 + i * 32];
   }
+#pragma unroll
+  for (int i = 0; i < ITEMS; ++i)
+    if (at0 + i * 32 < left) order[first + at0 + i * 32] = static_cast<int32_t>(mine[i].y);
 }
 
 template <int ITEMS>
 int launch_sort(const uint32_t* keys, const uint2* pairs, int64_t n, int key_bits, int32_t* order, cudaStream_t st) {
-  using Sort = cub::BlockRadixSort<uint32_t, kPieceThreads, ITEMS, int32_t>;
   static bool configured[kMaxDevices] = {false};
-  constexpr int bytes = static_cast<int>(sizeof(typename Sort::TempStorage));
+  constexpr int bytes = kPieceThreads * ITEMS * static_cast<int>(sizeof(uint2)) + kDigits * kPieceWarps * 2;
   SPC_CUDA_OK(ensure_dynamic_smem(sort_piece_kernel<ITEMS>, bytes, configured));
   const unsigned blocks = static_cast<unsigned>(ceil_div(n, kPieceThreads * ITEMS));
   sort_piece_kernel<ITEMS><<<blocks, kPieceThreads, bytes, st>>>(keys, pairs, n, key_bits, order);
@@ -133,19 +189,18 @@ int launch_sort(const uint32_t* keys, const uint2* pairs, int64_t n, int key_bit
 
 int tile_order(const uint32_t* keys, int64_t n, int kv, const uint32_t* counts, uint32_t* taken, uint2* pairs,
                int32_t* order, cudaStream_t st) {
-  // one more bit than the keys have, so that the filler of the last piece sorts behind them
-  const int bits = kv < 32 ? kv + 1 : 32;
+  constexpr int kItems = kTileOrderPiece / kPieceThreads;
   if (!tile_order_needs_buckets(n)) {
     // one piece: exact, and no larger than it has to be (the fewer rows a thread holds, the sooner it is done)
-    if (n <= kPieceThreads) return launch_sort<1>(keys, nullptr, n, bits, order, st);
-    if (n <= 2 * kPieceThreads) return launch_sort<2>(keys, nullptr, n, bits, order, st);
-    if (n <= 4 * kPieceThreads) return launch_sort<4>(keys, nullptr, n, bits, order, st);
-    return launch_sort<kPieceItems>(keys, nullptr, n, bits, order, st);
+    if (n <= kPieceThreads) return launch_sort<1>(keys, nullptr, n, kv, order, st);
+    if (n <= 2 * kPieceThreads) return launch_sort<2>(keys, nullptr, n, kv, order, st);
+    if (n <= 4 * kPieceThreads) return launch_sort<4>(keys, nullptr, n, kv, order, st);
+    return launch_sort<kItems>(keys, nullptr, n, kv, order, st);
   }
-  const unsigned blocks = static_cast<unsigned>(ceil_div(n, kTileOrderPiece));
-  deal_rows_kernel<<<blocks, kPieceThreads, 0, st>>>(keys, n, counts, taken, pairs);
+  const unsigned blocks = static_cast<unsigned>(ceil_div(n, kDealThreads * kDealItems));
+  deal_rows_kernel<<<blocks, kDealThreads, 0, st>>>(keys, n, counts, taken, pairs);
   SPC_LAUNCH_OK();
-  return launch_sort<kPieceItems>(keys, pairs, n, bits, order, st);
+  return launch_sort<kItems>(keys, pairs, n, kv, order, st);
 }
 
 }  // namespace spc
