@@ -508,8 +508,8 @@ typedef struct {
  * and ops.implicit_gemm for such a chain.  Every output, table and workspace is
  * placed in `arena` (256-byte aligned device memory owned by the caller, which
  * must stay alive while the results are used); `results[i]` says where.
- * Rulebooks of strided layers are generated on `stream_chain`, those of
- * submanifold layers on `stream_side`, the GEMMs on `stream_main`, ordered by
+ * The outputs of strided layers are found and numbered on `stream_chain`, the tables
+ * of all layers made on `stream_side`, the GEMMs run on `stream_main`, ordered by
  * events; on return `stream_main` has been made to wait for both other streams.
  * The call blocks on `stream_chain` once per strided layer (the read of its
  * output count, as _impl/pairs.py:209 does).

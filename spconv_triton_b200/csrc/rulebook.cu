@@ -136,6 +136,11 @@ struct Table<false> {
   // A look-up split in two so that several keys' first probes can be in flight at once:
   // first_probe() returns the home slot's word, finish() resolves it (almost always at once).
   __device__ __forceinline__ unsigned long long first_probe(key_t key) const { return __ldg(&slots[home(key)]); }
+  // Whether a home slot's word that is not empty is the key's; *row = its row then.
+  __device__ __forceinline__ bool settled(key_t key, unsigned long long v, int* row) const {
+    *row = static_cast<int>(v & 0xffffffffu);
+    return static_cast<key_t>(v >> 32) == key;
+  }
   __device__ __forceinline__ int finish(key_t key, unsigned long long v) const {
     if (v == kEmpty) return -1;
     if (static_cast<key_t>(v >> 32) == key) return static_cast<int>(v & 0xffffffffu);
@@ -209,6 +214,7 @@ struct Table<true> {
     return -1;
   }
   __device__ __forceinline__ unsigned long long first_probe(key_t) const { return 0; }
+  __device__ __forceinline__ bool settled(key_t, unsigned long long, int*) const { return false; }
   __device__ __forceinline__ int finish(key_t key, unsigned long long) const { return find(key); }
   __device__ void set_value(key_t key, uint32_t val) const {
     uint32_t s = home(key);
@@ -270,28 +276,6 @@ __device__ __forceinline__ long long out_key_from_input(const Geo& g, const int*
     }
     if (o < 0 || o >= g.out_shape[d]) return -1;
     lin = lin * g.out_shape[d] + o;
-  }
-  return lin;
-}
-
-// Input linear coordinate that feeds output coordinate `o` through kernel
-// offset `kp` (the inverse map of out_key_from_input), or -1.
-template <int ND>
-__device__ __forceinline__ long long in_key_from_output(const Geo& g, const int* o, const int* kp) {
-  long long lin = o[0];
-#pragma unroll
-  for (int d = 0; d < ND; ++d) {
-    int x;
-    if (g.transpose) {
-      const int num = o[d + 1] + g.pad[d] - kp[d] * g.dil[d];
-      if (num < 0) return -1;
-      x = num / g.stride[d];
-      if (x * g.stride[d] != num) return -1;
-    } else {
-      x = o[d + 1] * g.stride[d] - g.pad[d] + kp[d] * g.dil[d];
-    }
-    if (x < 0 || x >= g.in_shape[d]) return -1;
-    lin = lin * g.in_shape[d] + x;
   }
   return lin;
 }
@@ -420,16 +404,28 @@ __device__ __forceinline__ void mark_cells(const Geo& g, const int* c, const uin
 
 // First pass over the input rows: checks them, enters them into the input table (`in_bits`: the bit of the
 // cell, noting whether the rows are in strictly ascending key order; else the hash table, if `insert`) and,
-// with `out_bits`, marks the output cells.  One pass instead of one each: the coordinates are read once and
+// with `out_bits`, marks the output cells.  `cells`: the rows' cells, where an earlier layer has listed them
+// (its coordinates need not have been written yet).  One pass instead of one each: the coordinates are read once and
 // a small rulebook is three launches shorter.
 template <int ND, bool K64>
 __global__ void __launch_bounds__(kThreads)
-ingest_kernel(const __grid_constant__ Geo g, const int32_t* __restrict__ idx, long long n, Table<K64> tin, int insert,
-              uint32_t* __restrict__ in_bits, uint32_t* __restrict__ out_bits, int* counters, int* dev_status) {
+ingest_kernel(const __grid_constant__ Geo g, const int32_t* __restrict__ idx, const uint32_t* __restrict__ cells,
+              long long n, Table<K64> tin, int insert, uint32_t* __restrict__ in_bits, uint32_t* __restrict__ out_bits, int* counters, int* dev_status) {
   const long long j = blockIdx.x * static_cast<long long>(kThreads) + threadIdx.x;
   if (j >= n) return;
   int c[ND + 1];
-  load_coord<ND>(idx, j, c);
+  if (cells != nullptr) {
+    uint32_t lin = cells[j];
+#pragma unroll
+    for (int d = ND - 1; d >= 0; --d) {
+      const uint32_t q = lin / static_cast<uint32_t>(g.in_shape[d]);
+      c[d + 1] = static_cast<int>(lin - q * static_cast<uint32_t>(g.in_shape[d]));
+      lin = q;
+    }
+    c[0] = static_cast<int>(lin);
+  } else {
+    load_coord<ND>(idx, j, c);
+  }
   if (!coord_in_grid<ND>(g, c)) {
     flag_bad_row(counters, dev_status);
     counters[kUnsorted] = 1;  // a skipped row breaks "row number = rank of its bit"
@@ -718,7 +714,6 @@ assign_ranks_kernel(Table<K64> tout, const typename Table<K64>::key_t* __restric
 // ------------------------------------------------------------------------
 // What a fill kernel writes for its rows; every pointer may be null.
 struct FillOut {
-  int32_t* out_indices;  // coordinates of the output rows (strided layers, output side)
   int32_t* cm;           // [kv, n]: the neighbour table, column-major
   int32_t* rm;           // [n, kvp]: the same, row-major, padded with -1
   int32_t* cm_rev;       // both with the offset axis reversed: the input side of a submanifold layer, whose
@@ -727,13 +722,25 @@ struct FillOut {
   int32_t* iota;         // 0..n-1 (values of the exact mask sort)
   uint32_t* keys;        // [n]: key of the tile order (kv <= 32)
   uint32_t* counts;      // rows per bucket of that order (kTileBuckets, zeroed), or null
+  // Input side only: the output side's tables, pre-filled with -1 (words: 0), to which every pair found is
+  // scattered.  The lowest input row wins an entry, as equal coordinates resolve elsewhere (-1 is the
+  // largest unsigned number).
+  int32_t* out_cm;       // [kv, n_limit]
+  int32_t* out_rm;       // [n_limit, kvp]
+  uint32_t* out_words;   // [n_limit, mic]: mask words, or tile-order words with `order_bits`
+  int order_bits;
 };
 
 // A thread owns one row and looks its neighbours up; a warp's 32 rows are collected in shared memory (up to
 // 32 offsets at a time), where absent entries are pre-filled, so that only neighbours that exist cost an
 // entry, and leave it as full 16-byte-per-lane stores (row-major) and coalesced columns.
-// BWD = false: the rows are output rows (of `sorted`, or of `idx` for a submanifold layer) and `table` holds
-// the input cells; BWD = true: input rows, and `table` holds the output cells (rows from n_limit on are cut).
+// BWD = false: the rows of a submanifold layer, and `table` holds the same cells.
+// BWD = true: the input rows of a strided or transposed layer, and `table` holds the output cells (rows from
+// n_limit on are cut).  The output side's tables are made by the same pass, by scattering: an input reaches at
+// most 8 of 27 offsets' outputs of a k3 s2 layer, and they are bits of the output bitmap that also numbers
+// them, so the input cells need no table at all.  Gathering (every output row looks its 27 input cells up)
+// took 350 us for 480 k -> 1.36 M rows and an input hash table; clearing 152 MB and scattering 1.6 M pairs
+// takes 73.
 //
 // The row's kl offsets along the last axis meet cells that lie close together in the occupancy bitmap: one
 // (at a word boundary two) loads test all of them, and one prefix load numbers all of them, since the prefix
@@ -749,123 +756,141 @@ __host__ __device__ __forceinline__ int fill_pitch(int kvp) {
   return (w & 7) == 4 ? w : w + 4;
 }
 
-// Looks a row's K^ND neighbours up, everything about the offsets known at compile time: the cells of every
-// axis are found once, and the loads of up to nine lines (bitmap) or nine cells (hash table) are requested
-// together, so that a row waits for the L2 three times, not once a line.  With the offsets in loops the kernel
-// took 32 us for 2 000 rows, all of it latency; the common kernels (2 and 3 wide) are worth the code.
+__device__ __forceinline__ void clear_buckets(int* slot_bucket, uint32_t* slot_count) {
+  for (int i = threadIdx.x; i < kBucketSlots; i += kThreads) {
+    slot_bucket[i] = -1;
+    slot_count[i] = 0;
+  }
+  __syncthreads();
+}
+// Rows per bucket (-1: no row), by all threads of a CTA: first inside the warp, then inside the CTA, so that a
+// bucket most rows fall into is one global addition per CTA.
+__device__ __forceinline__ void count_buckets(int bucket, int* slot_bucket, uint32_t* slot_count, uint32_t* counts) {
+  const unsigned same = __match_any_sync(0xffffffffu, bucket);
+  if (bucket >= 0 && __ffs(same) - 1 == static_cast<int>(threadIdx.x & 31)) {
+    uint32_t s = (static_cast<uint32_t>(bucket) * 2654435761u) >> 23;
+    for (int probe = 0; probe < kBucketSlots; ++probe) {
+      const int old = atomicCAS(&slot_bucket[s], -1, bucket);
+      if (old == -1 || old == bucket) {
+        atomicAdd(&slot_count[s], static_cast<uint32_t>(__popc(same)));
+        break;
+      }
+      s = (s + 1) & (kBucketSlots - 1);
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kBucketSlots; i += kThreads)
+    if (slot_bucket[i] >= 0) atomicAdd(&counts[slot_bucket[i]], slot_count[i]);
+}
+
+// Looks a row's K^ND neighbours up.  The offsets of the last two axes are known at compile time, so that
+// the loads of K lines (bitmap) or of their K * K cells (hash table) are requested together: the kernel waits
+// on L2 latency otherwise (32 us for 2 000 rows with one line at a time).  The first of three axes stays a
+// loop, and a hash chain is followed in a loop of its own: unrolled completely the code no longer fits the
+// instruction cache, and on few rows fetching it is what takes the time (20 us for the same rows).
 template <int ND, bool K64, int K, typename Emit>
 __device__ __forceinline__ void look_up_cube(const Geo& g, bool div, const int* own, const int* limit,
                                              const Table<K64>& table, const Emit& emit) {
   using key_t = typename Table<K64>::key_t;
-  constexpr int kAll = ND == 1 ? 1 : ND == 2 ? K : K * K;  // lines along the last axis
-  constexpr int kGroup = K64 || kAll < 3 ? 1 : 3;          // lines probed together without a bitmap
-  int x[ND][K];
+  constexpr int kLast = ND - 1, kMid = ND >= 2 ? ND - 2 : 0;
+  constexpr int kLinesHere = ND == 1 ? 1 : K;
+  int xm[K], xl[K];
+  int lo = INT_MAX, hi = -1;
 #pragma unroll
-  for (int d = 0; d < ND; ++d)
-#pragma unroll
-    for (int k = 0; k < K; ++k) x[d][k] = axis_cell(g, div, d, own[d + 1], k, limit[d]);
-  bool on[kAll];
-  key_t base[kAll];
-#pragma unroll
-  for (int l = 0; l < kAll; ++l) {
-    const int p0 = ND == 3 ? l / K : l, p1 = l % K;
-    key_t key = static_cast<key_t>(own[0]);
-    on[l] = true;
-    if (ND >= 2) {
-      on[l] = x[0][p0] >= 0;
-      key = key * static_cast<key_t>(limit[0]) + static_cast<key_t>(x[0][p0]);
+  for (int k = 0; k < K; ++k) {
+    xm[k] = ND >= 2 ? axis_cell(g, div, kMid, own[kMid + 1], k, limit[kMid]) : 0;
+    xl[k] = axis_cell(g, div, kLast, own[kLast + 1], k, limit[kLast]);
+    if (xl[k] >= 0) {
+      lo = min(lo, xl[k]);
+      hi = max(hi, xl[k]);
     }
-    if (ND == 3) {
-      on[l] = on[l] && x[ND > 1 ? 1 : 0][p1] >= 0;
-      key = key * static_cast<key_t>(limit[ND > 1 ? 1 : 0]) + static_cast<key_t>(x[ND > 1 ? 1 : 0][p1]);
-    }
-    base[l] = key * static_cast<key_t>(limit[ND - 1]);
   }
+  if (hi < 0) return;
   const uint32_t* bits = dense_bits(table);
-  if (bits != nullptr) {
-    const uint32_t* prefix = dense_prefix(table);
-    const int32_t* perm = row_permutation(table);
-    int lo = INT_MAX, hi = -1;
+  const uint32_t* prefix = dense_prefix(table);
+  const int32_t* perm = row_permutation(table);
+#pragma unroll 1
+  for (int p = 0; p < (ND == 3 ? K : 1); ++p) {
+    key_t lead = static_cast<key_t>(own[0]);
+    if (ND == 3) {
+      const int x0 = axis_cell(g, div, 0, own[1], p, limit[0]);
+      if (x0 < 0) continue;
+      lead = lead * static_cast<key_t>(limit[0]) + static_cast<key_t>(x0);
+    }
+    const int k0 = p * K * K;
+    key_t base[kLinesHere];
 #pragma unroll
-    for (int k = 0; k < K; ++k)
-      if (x[ND - 1][k] >= 0) {
-        lo = min(lo, x[ND - 1][k]);
-        hi = max(hi, x[ND - 1][k]);
+    for (int l = 0; l < kLinesHere; ++l)
+      base[l] = (ND >= 2 ? lead * static_cast<key_t>(limit[kMid]) + static_cast<key_t>(xm[l]) : lead) * static_cast<key_t>(limit[kLast]);
+    if (bits != nullptr) {
+      uint32_t w0[kLinesHere], w1[kLinesHere], before[kLinesHere], hits[kLinesHere];
+#pragma unroll
+      for (int l = 0; l < kLinesHere; ++l) {
+        const key_t at = base[l] + static_cast<key_t>(lo);
+        w0[l] = xm[l] >= 0 ? __ldg(&bits[at >> 5]) : 0u;
+        w1[l] = xm[l] >= 0 && static_cast<int>(at & 31) + hi - lo >= 32 ? __ldg(&bits[(at >> 5) + 1]) : 0u;
       }
-    if (hi < 0) return;
-    uint32_t w0[kAll], w1[kAll], before[kAll];
 #pragma unroll
-    for (int l = 0; l < kAll; ++l) {
-      const key_t at = base[l] + static_cast<key_t>(lo);
-      w0[l] = on[l] ? __ldg(&bits[at >> 5]) : 0u;
-      w1[l] = on[l] && static_cast<int>(at & 31) + hi - lo >= 32 ? __ldg(&bits[(at >> 5) + 1]) : 0u;
-    }
-    uint32_t hits[kAll];
+      for (int l = 0; l < kLinesHere; ++l) {
+        const key_t at = base[l] + static_cast<key_t>(lo);
+        const unsigned long long win = ((static_cast<unsigned long long>(w1[l]) << 32) | w0[l]) >> (at & 31);
+        hits[l] = 0;
 #pragma unroll
-    for (int l = 0; l < kAll; ++l) {
-      const key_t at = base[l] + static_cast<key_t>(lo);
-      const unsigned long long win = ((static_cast<unsigned long long>(w1[l]) << 32) | w0[l]) >> (at & 31);
-      hits[l] = 0;
+        for (int k = 0; k < K; ++k)
+          if (xl[k] >= 0) hits[l] |= static_cast<uint32_t>((win >> (xl[k] - lo)) & 1ull) << k;
+        // (a word without bits has no prefix: the second word's rows then come first)
+        before[l] = hits[l] != 0 ? __ldg(&prefix[(at >> 5) + (w0[l] == 0 ? 1 : 0)]) : 0u;
+      }
+      int row[kLinesHere * K];
 #pragma unroll
-      for (int k = 0; k < K; ++k)
-        if (x[ND - 1][k] >= 0) hits[l] |= static_cast<uint32_t>((win >> (x[ND - 1][k] - lo)) & 1ull) << k;
-      // (a word without bits has no prefix: the second word's rows then come first)
-      before[l] = hits[l] != 0 ? __ldg(&prefix[(at >> 5) + (w0[l] == 0 ? 1 : 0)]) : 0u;
-    }
-#pragma unroll
-    for (int l0 = 0; l0 < kAll; l0 += (kAll < 3 ? 1 : 3)) {
-      constexpr int kStep = kAll < 3 ? 1 : 3;
-      int row[kStep * K];
-#pragma unroll
-      for (int b = 0; b < kStep; ++b) {
-        const int l = l0 + b < kAll ? l0 + b : kAll - 1;
+      for (int l = 0; l < kLinesHere; ++l) {
         const int sh = static_cast<int>((base[l] + static_cast<key_t>(lo)) & 31);
 #pragma unroll
         for (int k = 0; k < K; ++k) {
           int j = -1;
-          if (l0 + b < kAll && ((hits[l] >> k) & 1u)) {
-            const int bit = sh + x[ND - 1][k] - lo;
+          if ((hits[l] >> k) & 1u) {
+            const int bit = sh + xl[k] - lo;
             j = static_cast<int>(before[l]) + (bit < 32 ? __popc(w0[l] & ((1u << bit) - 1u))
                                                         : __popc(w0[l]) + __popc(w1[l] & ((1u << (bit - 32)) - 1u)));
             if (perm != nullptr) j = __ldg(&perm[j]);
           }
-          row[b * K + k] = j;
+          row[l * K + k] = j;
         }
       }
 #pragma unroll
-      for (int b = 0; b < kStep; ++b)
+      for (int q = 0; q < kLinesHere * K; ++q) emit(k0 + q, row[q]);
+    } else {
+      unsigned long long probe[kLinesHere * K];
+      uint32_t far = 0;  // cells whose home slot holds another key
+#pragma unroll
+      for (int l = 0; l < kLinesHere; ++l)
 #pragma unroll
         for (int k = 0; k < K; ++k)
-          if (l0 + b < kAll) emit((l0 + b) * K + k, row[b * K + k]);
+          probe[l * K + k] = xm[l] >= 0 && xl[k] >= 0 ? table.first_probe(base[l] + static_cast<key_t>(xl[k])) : Table<K64>::kEmpty;
+#pragma unroll
+      for (int l = 0; l < kLinesHere; ++l)
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          const int q = l * K + k;
+          if (probe[q] == Table<K64>::kEmpty) continue;
+          int j;
+          if (table.settled(base[l] + static_cast<key_t>(xl[k]), probe[q], &j)) emit(k0 + q, j);
+          else far |= 1u << q;
+        }
+#pragma unroll 1
+      for (; far != 0; far &= far - 1) {
+        const int q = __ffs(far) - 1, l = q / K, k = q % K;
+        const key_t line = ND >= 2 ? lead * static_cast<key_t>(limit[kMid]) + static_cast<key_t>(axis_cell(g, div, kMid, own[kMid + 1], l, limit[kMid])) : lead;
+        emit(k0 + q, table.find(line * static_cast<key_t>(limit[kLast]) +
+                                static_cast<key_t>(axis_cell(g, div, kLast, own[kLast + 1], k, limit[kLast]))));
+      }
     }
-    return;
-  }
-#pragma unroll
-  for (int l0 = 0; l0 < kAll; l0 += kGroup) {
-    unsigned long long probe[kGroup * K];
-#pragma unroll
-    for (int b = 0; b < kGroup; ++b)
-#pragma unroll
-      for (int k = 0; k < K; ++k) {
-        const int l = l0 + b < kAll ? l0 + b : kAll - 1;
-        const bool want = l0 + b < kAll && on[l] && x[ND - 1][k] >= 0;
-        probe[b * K + k] = want ? table.first_probe(base[l] + static_cast<key_t>(x[ND - 1][k])) : 0ull;
-      }
-#pragma unroll
-    for (int b = 0; b < kGroup; ++b)
-#pragma unroll
-      for (int k = 0; k < K; ++k) {
-        const int l = l0 + b < kAll ? l0 + b : kAll - 1;
-        if (l0 + b < kAll && on[l] && x[ND - 1][k] >= 0)
-          emit(l * K + k, table.finish(base[l] + static_cast<key_t>(x[ND - 1][k]), probe[b * K + k]));
-      }
   }
 }
 
 template <int ND, bool K64, bool BWD, int K>
 __global__ void __launch_bounds__(kThreads)
-fill_kernel(const __grid_constant__ Geo g, const int32_t* __restrict__ idx,
-            const typename Table<K64>::key_t* __restrict__ sorted, long long n, long long n_limit, Table<K64> table,
+fill_kernel(const __grid_constant__ Geo g, const int32_t* __restrict__ idx, long long n, long long n_limit, Table<K64> table,
             const __grid_constant__ FillOut out, int mic, int kvp) {
   using key_t = typename Table<K64>::key_t;
   extern __shared__ __align__(16) int32_t fill_s[];
@@ -875,44 +900,18 @@ fill_kernel(const __grid_constant__ Geo g, const int32_t* __restrict__ idx,
   const int pitch = fill_pitch(kvp);
   int32_t* tile = fill_s + warp * 32 * pitch;
   int32_t* mine = tile + lane * pitch;
-  if (out.counts != nullptr) {
-    for (int i = threadIdx.x; i < kBucketSlots; i += kThreads) {
-      slot_bucket[i] = -1;
-      slot_count[i] = 0;
-    }
-    __syncthreads();
-  }
+  if (out.counts != nullptr) clear_buckets(slot_bucket, slot_count);
   const long long r = blockIdx.x * static_cast<long long>(kThreads) + threadIdx.x;
   const long long row0 = r - lane;
   const bool live = r < n;
-  const bool from_idx = BWD || g.subm;
-  const bool div = BWD ? !g.transpose : g.transpose != 0;
+  const bool div = BWD && !g.transpose;
   const int* __restrict__ limit = BWD ? g.out_shape : g.in_shape;
 
   int own[ND + 1];
   bool ok = live;  // a row outside the grid gets no neighbours
   if (live) {
-    if (from_idx) {
-      load_coord<ND>(idx, r, own);
-      ok = coord_in_grid<ND>(g, own);
-    } else {
-      key_t lin = sorted[r];
-#pragma unroll
-      for (int d = ND - 1; d >= 0; --d) {
-        const key_t q = lin / static_cast<key_t>(g.out_shape[d]);
-        own[d + 1] = static_cast<int>(lin - q * static_cast<key_t>(g.out_shape[d]));
-        lin = q;
-      }
-      own[0] = static_cast<int>(lin);
-      if (out.out_indices != nullptr) {
-        if (ND == 3 && (reinterpret_cast<uintptr_t>(out.out_indices) & 15u) == 0) {
-          reinterpret_cast<int4*>(out.out_indices)[r] = make_int4(own[0], own[1], own[ND > 1 ? 2 : 0], own[ND > 2 ? 3 : 0]);
-        } else {
-#pragma unroll
-          for (int d = 0; d <= ND; ++d) out.out_indices[r * (ND + 1) + d] = own[d];
-        }
-      }
-    }
+    load_coord<ND>(idx, r, own);
+    ok = coord_in_grid<ND>(g, own);
     if (out.iota != nullptr) out.iota[r] = static_cast<int32_t>(r);
   }
   uint32_t valid[ND];  // per axis: the offsets that meet a cell of the grid
@@ -954,6 +953,12 @@ fill_kernel(const __grid_constant__ Geo g, const int32_t* __restrict__ idx,
       mine[k - c0] = j;
       word |= 1u << (k - c0);
       if (out.keys != nullptr) order_word |= 1u << g.key_pos[k];
+      if (BWD && out.out_rm != nullptr)
+        atomicMin(reinterpret_cast<unsigned*>(&out.out_rm[static_cast<long long>(j) * kvp + k]), static_cast<unsigned>(r));
+      if (BWD && out.out_cm != nullptr)
+        atomicMin(reinterpret_cast<unsigned*>(&out.out_cm[k * n_limit + j]), static_cast<unsigned>(r));
+      if (BWD && out.out_words != nullptr)
+        atomicOr(&out.out_words[static_cast<long long>(j) * mic + (k >> 5)], 1u << (out.order_bits ? g.key_pos[k] : (k & 31)));
     };
     if constexpr (K != 0) {
       if (ok) look_up_cube<ND, K64, K>(g, div, own, limit, table, emit);
@@ -1103,25 +1108,44 @@ fill_kernel(const __grid_constant__ Geo g, const int32_t* __restrict__ idx,
   }
   if (out.keys == nullptr) return;
   if (live) out.keys[r] = gray_decode(order_word);
-  if (out.counts == nullptr) return;
-  // rows per bucket: first inside the warp, then inside the CTA, so that a bucket most rows fall into is
-  // one global addition per CTA
-  const int bucket = live ? bucket_of(order_word) : -1;
-  const unsigned same = __match_any_sync(0xffffffffu, bucket);
-  if (bucket >= 0 && __ffs(same) - 1 == lane) {
-    uint32_t s = (static_cast<uint32_t>(bucket) * 2654435761u) >> 23;
-    for (int probe = 0; probe < kBucketSlots; ++probe) {
-      const int old = atomicCAS(&slot_bucket[s], -1, bucket);
-      if (old == -1 || old == bucket) {
-        atomicAdd(&slot_count[s], static_cast<uint32_t>(__popc(same)));
-        break;
-      }
-      s = (s + 1) & (kBucketSlots - 1);
+  if (out.counts != nullptr) count_buckets(live ? bucket_of(order_word) : -1, slot_bucket, slot_count, out.counts);
+}
+
+// The output rows of a strided or transposed layer, after the scatter: their coordinates and, from the
+// scattered tile-order words, the keys and bucket counts of their order.
+template <int ND, bool K64>
+__global__ void __launch_bounds__(kThreads)
+finish_outputs_kernel(const __grid_constant__ Geo g, const typename Table<K64>::key_t* __restrict__ sorted, long long n,
+                      int32_t* __restrict__ out_indices, int32_t* __restrict__ iota, const uint32_t* __restrict__ order_words,
+                      uint32_t* __restrict__ keys, uint32_t* __restrict__ counts) {
+  using key_t = typename Table<K64>::key_t;
+  __shared__ int slot_bucket[kBucketSlots];
+  __shared__ uint32_t slot_count[kBucketSlots];
+  if (counts != nullptr) clear_buckets(slot_bucket, slot_count);
+  const long long r = blockIdx.x * static_cast<long long>(kThreads) + threadIdx.x;
+  const bool live = r < n;
+  if (live && out_indices != nullptr) {
+    int o[ND + 1];
+    key_t lin = sorted[r];
+#pragma unroll
+    for (int d = ND - 1; d >= 0; --d) {
+      const key_t q = lin / static_cast<key_t>(g.out_shape[d]);
+      o[d + 1] = static_cast<int>(lin - q * static_cast<key_t>(g.out_shape[d]));
+      lin = q;
+    }
+    o[0] = static_cast<int>(lin);
+    if (ND == 3 && (reinterpret_cast<uintptr_t>(out_indices) & 15u) == 0) {
+      reinterpret_cast<int4*>(out_indices)[r] = make_int4(o[0], o[1], o[ND > 1 ? 2 : 0], o[ND > 2 ? 3 : 0]);
+    } else {
+#pragma unroll
+      for (int d = 0; d <= ND; ++d) out_indices[r * (ND + 1) + d] = o[d];
     }
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < kBucketSlots; i += kThreads)
-    if (slot_bucket[i] >= 0) atomicAdd(&out.counts[slot_bucket[i]], slot_count[i]);
+  if (live && iota != nullptr) iota[r] = static_cast<int32_t>(r);
+  if (order_words == nullptr) return;
+  const uint32_t word = live ? order_words[r] : 0u;
+  if (live) keys[r] = gray_decode(word);
+  if (counts != nullptr) count_buckets(live ? bucket_of(word) : -1, slot_bucket, slot_count, counts);
 }
 
 // keys[i] = words[rows[i], w] & and_mask ; rows == nullptr means identity.
@@ -1296,6 +1320,7 @@ struct Layout {
   // ranks by construction, and no input hash table is built.
   const uint32_t* shared_bits = nullptr;
   const uint32_t* shared_prefix = nullptr;
+  const uint32_t* shared_cells = nullptr;  // the cells of those rows
 };
 // counts and taken of the tile order
 constexpr size_t kOrderCountBytes = 2 * ((kTileBuckets * 4 + 255) / 256) * 256;
@@ -1412,16 +1437,16 @@ Layout make_layout(const Geo& g, int64_t n_in) {
     const double b = std::min(static_cast<double>(n_in) * per_input, vol_out);
     L.bound = static_cast<int64_t>(std::max(b, 1.0));
   }
-  // The input side through a bitmap of the grid (most neighbour cells of a voxel are empty, a bit test
+  // The rows of a submanifold layer through a bitmap of the grid (most neighbour cells of a voxel are empty, a bit test
   // answers for a whole line of them, and a row is its rank) where the bitmap is no dearer to clear and
   // count than a hash table (512 cells or 64 bytes a voxel), small enough to stay in L2 beside the tables
   // (24 MB), and there are enough rows for the looks-up to outweigh three more launches.
   const double max_bits = 24.0 * 1024 * 1024 * 8;
-  if (!L.k64 && vol_in <= max_bits && vol_in <= 512.0 * n_in && n_in >= 16384)
+  if (g.subm && !L.k64 && vol_in <= max_bits && vol_in <= 512.0 * n_in && n_in >= 16384)
     L.ibits_words = static_cast<int64_t>(vol_in / 32.0) + 1;
   // the output bitmap also numbers the outputs, which a hash table needs a sort for
   if (!g.subm && !L.k64 && vol_out <= max_bits) L.obits_words = static_cast<int64_t>(vol_out / 32.0) + 1;
-  L.cap_in = L.ibits_words ? 0 : pow2_at_least(4 * n_in);  // load <= 0.25: most look-ups miss, keep their probe chains short
+  L.cap_in = !g.subm || L.ibits_words ? 0 : pow2_at_least(4 * n_in);  // load <= 0.25: most look-ups miss, keep their probe chains short
   L.cap_out = g.subm || L.obits_words ? 0 : pow2_at_least(2 * L.bound);
   const int64_t n_max = std::max<int64_t>(n_in, L.bound);
   L.n_blocks_native = ceil_div(std::max<int64_t>(n_in, 1), kThreads);
@@ -1600,7 +1625,7 @@ int prepare_impl(const Geo& g, const Layout& L, const int32_t* idx, int64_t n_in
   if (dense_in) {
     clear.add(ws + L.off_ibits, 0, static_cast<size_t>(L.ibits_words) * 4);
     clear.add(ws + L.off_perm, 0x7F, static_cast<size_t>(n_in) * 4);
-  } else if (!chained) {
+  } else if (g.subm && !chained) {
     clear.add(ws + L.off_tin, 0xFF, static_cast<size_t>(L.cap_in) * 8);
     if (K64) clear.add(ws + L.off_tin_vals, 0x7F, static_cast<size_t>(L.cap_in) * 4);
   }
@@ -1620,7 +1645,7 @@ int prepare_impl(const Geo& g, const Layout& L, const int32_t* idx, int64_t n_in
   key_t* uniq = reinterpret_cast<key_t*>(ws + L.off_uniq);
   key_t* sorted = reinterpret_cast<key_t*>(ws + L.off_sorted);
   if (!chained || (dense_out && g.axes_fit)) {
-    ingest_kernel<ND, K64><<<blocks_for(n_in), kThreads, 0, st>>>(g, idx, n_in, tin, !chained, ibits,
+    ingest_kernel<ND, K64><<<blocks_for(n_in), kThreads, 0, st>>>(g, idx, L.shared_cells, n_in, tin, g.subm && !chained, ibits,
                                                                   g.axes_fit ? obits : nullptr, counters, dev_status);
     SPC_LAUNCH_OK();
   }
@@ -1766,104 +1791,135 @@ int cube_width(const Geo& g) {
 size_t fill_smem_bytes(int kvp) { return static_cast<size_t>(kThreads / 32) * 32 * fill_pitch(kvp) * 4; }
 
 template <int ND, bool K64, bool BWD>
-int launch_fill(const Geo& g, const int32_t* idx, const typename Table<K64>::key_t* sorted, int64_t n, int64_t n_limit,
-                const Table<K64>& table, const FillOut& out, int mic, cudaStream_t st) {
+int launch_fill(const Geo& g, const int32_t* idx, int64_t n, int64_t n_limit, const Table<K64>& table, const FillOut& out,
+                int mic, cudaStream_t st) {
   const int kvp = (g.kv + 3) & ~3;
   const unsigned blocks = blocks_for(n);
   const size_t smem = fill_smem_bytes(kvp);
   const int width = cube_width(g);
   if constexpr (ND <= 3) {
     if (width == 3)
-      fill_kernel<ND, K64, BWD, 3><<<blocks, kThreads, smem, st>>>(g, idx, sorted, n, n_limit, table, out, mic, kvp);
-    else if (width == 2)
-      fill_kernel<ND, K64, BWD, 2><<<blocks, kThreads, smem, st>>>(g, idx, sorted, n, n_limit, table, out, mic, kvp);
+      fill_kernel<ND, K64, BWD, 3><<<blocks, kThreads, smem, st>>>(g, idx, n, n_limit, table, out, mic, kvp);
+    else if (width == 2 && BWD)  // (submanifold kernels are odd)
+      fill_kernel<ND, K64, BWD, BWD ? 2 : 0><<<blocks, kThreads, smem, st>>>(g, idx, n, n_limit, table, out, mic, kvp);
   }
-  if (ND > 3 || width == 0)
-    fill_kernel<ND, K64, BWD, 0><<<blocks, kThreads, smem, st>>>(g, idx, sorted, n, n_limit, table, out, mic, kvp);
+  if (ND > 3 || width == 0 || (width == 2 && !BWD))
+    fill_kernel<ND, K64, BWD, 0><<<blocks, kThreads, smem, st>>>(g, idx, n, n_limit, table, out, mic, kvp);
   SPC_LAUNCH_OK();
   return SPC_OK;
 }
 
-// Keys and bucket counts of the tile order for a fill kernel, then the order itself.
-void want_order(const Layout& L, char* ws, int64_t n, FillOut* out) {
-  out->keys = reinterpret_cast<uint32_t*>(ws + L.off_keys_a);
-  if (tile_order_needs_buckets(n)) out->counts = reinterpret_cast<uint32_t*>(ws + L.off_order_counts);
+// One side's tables, as the callers ask for them.
+struct SideTables {
+  int32_t* cm = nullptr;
+  int32_t* rm = nullptr;
+  int32_t* order = nullptr;        // the tile order, or
+  int32_t* mask = nullptr;         // the exactly sorted masks
+  int32_t* argsort = nullptr;
+  bool wanted() const { return cm || rm || order || mask; }
+};
+struct MaskSplits {
+  const uint32_t* words = nullptr;
+  int n = 1, do_sort = 0;
+};
+
+uint32_t* bucket_counts(const Layout& L, char* ws, int64_t n) {
+  return tile_order_needs_buckets(n) ? reinterpret_cast<uint32_t*>(ws + L.off_order_counts) : nullptr;
 }
 int emit_order(const Layout& L, char* ws, int64_t n, int kv, int32_t* order, cudaStream_t st) {
   uint32_t* counts = reinterpret_cast<uint32_t*>(ws + L.off_order_counts);
   return tile_order(reinterpret_cast<const uint32_t*>(ws + L.off_keys_a), n, kv, counts, counts + kOrderCountBytes / 8,
                     reinterpret_cast<uint2*>(ws + L.off_order_pairs), order, st);
 }
-
-// Input-side tables of a strided / transposed layer: pair_bwd, its masks or its tile order.
-// Reads the output table the forward phase numbered; shares the mask scratch with
-// it, so it must follow the forward phase of the same workspace.
-template <int ND, bool K64>
-int igemm_backward_impl(const Geo& g, const Layout& L, const int32_t* idx, int64_t n_in, int64_t n_out, char* ws,
-                        int32_t* pair_bwd, int32_t* mask_bwd, int32_t* argsort_bwd, const uint32_t* split_masks,
-                        int n_split, int do_sort, int32_t* bwd_rm, int32_t* order_bwd, cudaStream_t st) {
-  FillOut out{};
-  out.cm = pair_bwd;
-  out.rm = bwd_rm;
-  if (mask_bwd != nullptr) {
-    out.words = reinterpret_cast<uint32_t*>(ws + L.off_words);
-    out.iota = mask_iota(L, ws, split_masks, n_split, do_sort);
+// Keys or words of the rows that a fill kernel owns.
+void ask_fill(const Layout& L, char* ws, int64_t n, const SideTables& t, const MaskSplits& m, FillOut* out) {
+  out->cm = t.cm;
+  out->rm = t.rm;
+  if (t.order != nullptr) {
+    out->keys = reinterpret_cast<uint32_t*>(ws + L.off_keys_a);
+    out->counts = bucket_counts(L, ws, n);
   }
-  if (order_bwd != nullptr) {
-    // the counts of the output side's order are still there
-    if (tile_order_needs_buckets(n_in)) {
-      Clear c;
-      c.add(ws + L.off_order_counts, 0, kOrderCountBytes);
-      const int rc = launch_clear(c, st);
-      if (rc != SPC_OK) return rc;
-    }
-    want_order(L, ws, n_in, &out);
+  if (t.mask != nullptr) {
+    out->words = reinterpret_cast<uint32_t*>(ws + L.off_words);
+    out->iota = mask_iota(L, ws, m.words, m.n, m.do_sort);
   }
-  const int rc_fill = launch_fill<ND, K64, true>(g, idx, nullptr, n_in, n_out, tout_at<K64>(ws, L), out, L.mic, st);
-  if (rc_fill != SPC_OK) return rc_fill;
-  if (order_bwd != nullptr) {
-    const int rc = emit_order(L, ws, n_in, g.kv, order_bwd, st);
+}
+int emit_side(const Geo& g, const Layout& L, char* ws, int64_t n, const SideTables& t, const MaskSplits& m, cudaStream_t st) {
+  if (t.order != nullptr) {
+    const int rc = emit_order(L, ws, n, g.kv, t.order, st);
     if (rc != SPC_OK) return rc;
   }
-  if (mask_bwd != nullptr) return emit_masks(L, ws, n_in, g.kv, split_masks, n_split, do_sort, mask_bwd, argsort_bwd, st);
-  return SPC_OK;
+  return t.mask != nullptr ? emit_masks(L, ws, n, g.kv, m.words, m.n, m.do_sort, t.mask, t.argsort, st) : SPC_OK;
 }
 
+// Input side of a strided / transposed layer on its own (its output side was made by an earlier call).
 template <int ND, bool K64>
-int igemm_forward_impl(const Geo& g, const Layout& L, const int32_t* idx, int64_t n_out, char* ws, FillOut out,
-                       int32_t* order_fwd, cudaStream_t st) {
-  using key_t = typename Table<K64>::key_t;
-  if (order_fwd != nullptr) want_order(L, ws, n_out, &out);
-  const int rc = launch_fill<ND, K64, false>(g, idx, reinterpret_cast<const key_t*>(ws + L.off_sorted), n_out, n_out,
-                                             tin_at<K64>(ws, L), out, L.mic, st);
-  if (rc != SPC_OK) return rc;
-  return order_fwd != nullptr ? emit_order(L, ws, n_out, g.kv, order_fwd, st) : SPC_OK;
-}
-
-template <int ND, bool K64>
-int igemm_impl(const Geo& g, const Layout& L, const int32_t* idx, int64_t n_in, int64_t n_out, char* ws,
-               int32_t* out_indices, int32_t* pair_fwd, int32_t* pair_bwd, int32_t* mask_fwd,
-               int32_t* argsort_fwd, int32_t* mask_bwd, int32_t* argsort_bwd,
-               const uint32_t* split_masks, int n_split, int do_sort, int32_t* fwd_rm, int32_t* bwd_rm,
-               cudaStream_t st) {
-  FillOut out{};
-  out.out_indices = g.subm ? nullptr : out_indices;
-  out.cm = pair_fwd;
-  out.rm = fwd_rm;
-  if (g.subm && pair_bwd != nullptr) {
-    out.cm_rev = pair_bwd;
-    out.rm_rev = bwd_rm;
+int backward_impl(const Geo& g, const Layout& L, const int32_t* idx, int64_t n_in, int64_t n_out, char* ws,
+                  const SideTables& bwd, const MaskSplits& m, cudaStream_t st) {
+  if (bwd.order != nullptr && tile_order_needs_buckets(n_in)) {  // the counts of the output side's order are still there
+    Clear c;
+    c.add(ws + L.off_order_counts, 0, kOrderCountBytes);
+    const int rc = launch_clear(c, st);
+    if (rc != SPC_OK) return rc;
   }
-  out.words = reinterpret_cast<uint32_t*>(ws + L.off_words);
-  out.iota = mask_iota(L, ws, split_masks, n_split, do_sort);
-  int rc = igemm_forward_impl<ND, K64>(g, L, idx, n_out, ws, out, nullptr, st);
+  FillOut out{};
+  ask_fill(L, ws, n_in, bwd, m, &out);
+  const int rc = launch_fill<ND, K64, true>(g, idx, n_in, n_out, tout_at<K64>(ws, L), out, L.mic, st);
+  return rc != SPC_OK ? rc : emit_side(g, L, ws, n_in, bwd, m, st);
+}
+
+// Both sides of a strided / transposed layer: clear the output side's tables, one pass over the input rows,
+// one over the output rows.  The input side's keys or words wait for their sort until the output side's is
+// done with the shared scratch, so an ordered or masked input side is a pass of its own.
+template <int ND, bool K64>
+int strided_impl(const Geo& g, const Layout& L, const int32_t* idx, int64_t n_in, int64_t n_out, char* ws,
+                 int32_t* out_indices, const SideTables& fwd, const SideTables& bwd, const MaskSplits& m, cudaStream_t st) {
+  using key_t = typename Table<K64>::key_t;
+  const int kvp = (g.kv + 3) & ~3;
+  uint32_t* words = fwd.order || fwd.mask ? reinterpret_cast<uint32_t*>(ws + L.off_words) : nullptr;
+  Clear c;
+  c.add(fwd.rm, 0xFF, fwd.rm ? static_cast<size_t>(n_out) * kvp * 4 : 0);
+  c.add(words, 0, words ? static_cast<size_t>(n_out) * L.mic * 4 : 0);
+  int rc = SPC_OK;
+  if (fwd.cm != nullptr) {
+    // (a table of the caller's: neither its start nor its size need be a multiple of 16 bytes)
+    const size_t bytes = static_cast<size_t>(g.kv) * n_out * 4;
+    if ((reinterpret_cast<uintptr_t>(fwd.cm) | bytes) & 15u)
+      SPC_CUDA_OK(cudaMemsetAsync(fwd.cm, 0xFF, bytes, st));
+    else
+      c.add(fwd.cm, 0xFF, bytes);
+  }
+  if (c.total != 0) rc = launch_clear(c, st);
   if (rc != SPC_OK) return rc;
-  rc = emit_masks(L, ws, n_out, g.kv, split_masks, n_split, do_sort, mask_fwd, argsort_fwd, st);
+  FillOut out{};
+  const bool together = bwd.wanted() && bwd.order == nullptr && bwd.mask == nullptr;
+  if (together) ask_fill(L, ws, n_in, bwd, m, &out);
+  out.out_cm = fwd.cm;
+  out.out_rm = fwd.rm;
+  out.out_words = words;
+  out.order_bits = fwd.order != nullptr;
+  rc = launch_fill<ND, K64, true>(g, idx, n_in, n_out, tout_at<K64>(ws, L), out, L.mic, st);
   if (rc != SPC_OK) return rc;
-  if (!g.subm && pair_bwd != nullptr)
-    return igemm_backward_impl<ND, K64>(g, L, idx, n_in, n_out, ws, pair_bwd, mask_bwd, argsort_bwd, split_masks,
-                                        n_split, do_sort, bwd_rm, nullptr, st);
-  return SPC_OK;
+  finish_outputs_kernel<ND, K64><<<blocks_for(n_out), kThreads, 0, st>>>(
+      g, reinterpret_cast<const key_t*>(ws + L.off_sorted), n_out, out_indices,
+      fwd.mask ? mask_iota(L, ws, m.words, m.n, m.do_sort) : nullptr, fwd.order ? words : nullptr,
+      reinterpret_cast<uint32_t*>(ws + L.off_keys_a), bucket_counts(L, ws, n_out));
+  SPC_LAUNCH_OK();
+  rc = emit_side(g, L, ws, n_out, fwd, m, st);
+  if (rc != SPC_OK || !bwd.wanted() || together) return rc;
+  return backward_impl<ND, K64>(g, L, idx, n_in, n_out, ws, bwd, m, st);
+}
+
+// A submanifold layer; rev_cm / rev_rm: its input side.
+template <int ND, bool K64>
+int subm_impl(const Geo& g, const Layout& L, const int32_t* idx, int64_t n, char* ws, const SideTables& fwd, int32_t* rev_cm,
+              int32_t* rev_rm, const MaskSplits& m, cudaStream_t st) {
+  FillOut out{};
+  ask_fill(L, ws, n, fwd, m, &out);
+  out.cm_rev = rev_cm;
+  out.rm_rev = rev_rm;
+  const int rc = launch_fill<ND, K64, false>(g, idx, n, n, tin_at<K64>(ws, L), out, L.mic, st);
+  return rc != SPC_OK ? rc : emit_side(g, L, ws, n, fwd, m, st);
 }
 
 template <int ND, bool K64>
@@ -1930,6 +1986,7 @@ void adopt_producer_bits(const Geo& g, Layout* L, const RulebookProducer* produc
   const char* wp = static_cast<const char*>(producer->workspace);
   L->shared_bits = reinterpret_cast<const uint32_t*>(wp + Lp.off_obits);
   L->shared_prefix = reinterpret_cast<const uint32_t*>(wp + Lp.off_oprefix);
+  L->shared_cells = reinterpret_cast<const uint32_t*>(wp + Lp.off_sorted);
 }
 
 }  // namespace
@@ -1950,6 +2007,14 @@ int rulebook_prepare_chained(const spc_geometry* sg, const int32_t* indices, int
   return dispatch(g.ndim, L.k64, [&](auto nd, auto k64) {
     return prepare_impl<decltype(nd)::value, decltype(k64)::value>(g, L, indices, n_in, ws, n_out_host, st);
   });
+}
+
+bool rulebook_adopts(const spc_geometry* sg, int64_t n_in, const RulebookProducer* producer) {
+  Geo g;
+  if (!make_geo(sg, &g)) return false;
+  Layout L = make_layout(g, n_in);
+  adopt_producer_bits(g, &L, producer);
+  return L.shared_bits != nullptr;
 }
 
 int rulebook_tables_chained(const spc_geometry* sg, const int32_t* indices, int64_t n_in, int64_t n_out,
@@ -1975,17 +2040,17 @@ int rulebook_tables_chained(const spc_geometry* sg, const int32_t* indices, int6
   return dispatch(g.ndim, L.k64, [&](auto nd, auto k64) -> int {
     constexpr int ND = decltype(nd)::value;
     constexpr bool K64 = decltype(k64)::value;
-    if (t.fwd_colmajor || t.fwd_rowmajor || t.fwd_order || t.out_indices) {
-      FillOut out{};
-      out.out_indices = g.subm ? nullptr : t.out_indices;
-      out.cm = t.fwd_colmajor;
-      out.rm = t.fwd_rowmajor;
-      const int rc = igemm_forward_impl<ND, K64>(g, L, indices, n_out, ws, out, t.fwd_order, st);
-      if (rc != SPC_OK) return rc;
-    }
-    if (!input_side) return SPC_OK;
-    return igemm_backward_impl<ND, K64>(g, L, indices, n_in, n_out, ws, t.bwd_colmajor, nullptr, nullptr, nullptr, 1, 0,
-                                        t.bwd_rowmajor, t.bwd_order, st);
+    SideTables fwd, bwd;
+    fwd.cm = t.fwd_colmajor;
+    fwd.rm = t.fwd_rowmajor;
+    fwd.order = t.fwd_order;
+    bwd.cm = t.bwd_colmajor;
+    bwd.rm = t.bwd_rowmajor;
+    bwd.order = t.bwd_order;
+    if (g.subm) return subm_impl<ND, K64>(g, L, indices, n_in, ws, fwd, nullptr, nullptr, MaskSplits{}, st);
+    if (!fwd.wanted() && t.out_indices == nullptr)
+      return backward_impl<ND, K64>(g, L, indices, n_in, n_out, ws, bwd, MaskSplits{}, st);
+    return strided_impl<ND, K64>(g, L, indices, n_in, n_out, ws, t.out_indices, fwd, bwd, MaskSplits{}, st);
   });
 }
 
@@ -2038,10 +2103,21 @@ extern "C" int spc_rulebook_igemm(const spc_geometry* sg, const int32_t* indices
   if (n_out > L.bound) return fail(SPC_ERR_INVALID_ARGUMENT, "rulebook igemm: n_out exceeds prepared bound");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   char* ws = static_cast<char*>(workspace);
+  SideTables fwd, bwd;
+  fwd.cm = pair_fwd;
+  fwd.rm = pair_fwd_rowmajor;
+  fwd.mask = mask_fwd;
+  fwd.argsort = argsort_fwd;
+  bwd.cm = pair_bwd;
+  bwd.rm = pair_bwd_rowmajor;
+  bwd.mask = mask_bwd;
+  bwd.argsort = argsort_bwd;
+  const MaskSplits m{split_masks, n_split, do_sort};
   return dispatch(g.ndim, L.k64, [&](auto nd, auto k64) {
-    return igemm_impl<decltype(nd)::value, decltype(k64)::value>(
-        g, L, indices, n_in, n_out, ws, out_indices, pair_fwd, pair_bwd, mask_fwd, argsort_fwd, mask_bwd,
-        argsort_bwd, split_masks, n_split, do_sort, pair_fwd_rowmajor, pair_bwd_rowmajor, st);
+    constexpr int ND = decltype(nd)::value;
+    constexpr bool K64 = decltype(k64)::value;
+    if (g.subm) return subm_impl<ND, K64>(g, L, indices, n_in, ws, fwd, pair_bwd, pair_bwd_rowmajor, m, st);
+    return strided_impl<ND, K64>(g, L, indices, n_in, n_out, ws, out_indices, fwd, pair_bwd ? bwd : SideTables{}, m, st);
   });
 }
 
@@ -2063,10 +2139,14 @@ extern "C" int spc_rulebook_igemm_backward(const spc_geometry* sg, const int32_t
   if (n_out > L.bound) return fail(SPC_ERR_INVALID_ARGUMENT, "rulebook igemm backward: n_out exceeds prepared bound");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   char* ws = static_cast<char*>(workspace);
+  SideTables bwd;
+  bwd.cm = pair_bwd;
+  bwd.rm = pair_bwd_rowmajor;
+  bwd.mask = mask_bwd;
+  bwd.argsort = argsort_bwd;
+  const MaskSplits m{split_masks, n_split, do_sort};
   return dispatch(g.ndim, L.k64, [&](auto nd, auto k64) {
-    return igemm_backward_impl<decltype(nd)::value, decltype(k64)::value>(
-        g, L, indices, n_in, n_out, ws, pair_bwd, mask_bwd, argsort_bwd, split_masks, n_split, do_sort,
-        pair_bwd_rowmajor, nullptr, st);
+    return backward_impl<decltype(nd)::value, decltype(k64)::value>(g, L, indices, n_in, n_out, ws, bwd, m, st);
   });
 }
 

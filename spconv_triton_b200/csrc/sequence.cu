@@ -10,14 +10,15 @@
 // this library, with every table, workspace and activation carved out of ONE
 // caller-provided arena, on three streams:
 //
-//   chain   strided / transposed rulebooks, each of which needs the previous
-//           one's output coordinates and one host read of its output count;
-//   side    submanifold rulebooks (no host read), which only need the
-//           coordinates of their level;
+//   chain   the output cells of strided / transposed layers, found, numbered and
+//           counted, each from the cells of the one before, with one host read of
+//           the count: four short kernels a level;
+//   side    the tables and row orders of all rulebooks;
 //   main    the GEMMs, each waiting (cudaStreamWaitEvent) for its rulebook.
 //
-// So the rulebook chain runs ahead of the GEMMs as far as its host reads allow
-// and the submanifold rulebooks fill the gaps.  Results are the same tensors the
+// So the numbering chain, which everything else and the host wait for, runs ahead
+// of the tables and the GEMMs as far as its host reads allow.  (With the tables
+// of the strided layers on the chain a one-sample pass took 590 us.)  Results are the same tensors the
 // layer-by-layer path produces (same kernels, same arguments).
 #include <cstring>
 #include <vector>
@@ -32,7 +33,7 @@ namespace {
 constexpr int kMaxSeqLayers = 64;
 
 struct EventPool {
-  cudaEvent_t ev[kMaxSeqLayers + 2];
+  cudaEvent_t ev[2 * kMaxSeqLayers + 2];
   bool ready = false;
 };
 
@@ -83,7 +84,8 @@ extern "C" int spc_sequence_forward(const spc_seq_layer* layers, int n_layers, c
   cudaEvent_t* ev = nullptr;
   int rc = events_for_current_device(&ev);
   if (rc != SPC_OK) return rc;
-  cudaEvent_t ev_input = ev[kMaxSeqLayers];
+  cudaEvent_t ev_input = ev[2 * kMaxSeqLayers];
+  cudaEvent_t* ev_numbered = ev + kMaxSeqLayers;  // per strided layer: its outputs are numbered
 
   Arena arena{static_cast<char*>(arena_ptr), arena_bytes};
   const size_t esize = dtype_size(dtype);
@@ -95,7 +97,7 @@ extern "C" int spc_sequence_forward(const spc_seq_layer* layers, int n_layers, c
 
   const int32_t* cur_indices = indices;   // coordinates of the current level
   int64_t cur_n = n_in;
-  cudaEvent_t cur_indices_ready = ev_input;
+  int cur_indices_from = -1;              // the layer whose tables step writes them (-1: the caller)
   const void* cur_features = features;
   int cur_channels = layers[0].c_in;
   // the strided layer that produced the current level's coordinates: its output bitmap doubles as
@@ -119,7 +121,9 @@ extern "C" int spc_sequence_forward(const spc_seq_layer* layers, int n_layers, c
       // ---- generate this layer's rulebook --------------------------------------------------
       const bool subm = L.geom.subm != 0;
       cudaStream_t st = subm ? side : chain;
-      if (subm) SPC_CUDA_OK(cudaStreamWaitEvent(side, cur_indices_ready, 0));
+      // outputs of a layer that did not number them through a bitmap come as coordinates, from its tables step
+      if (!subm && cur_indices_from >= 0 && !rulebook_adopts(&L.geom, cur_n, &producer))
+        SPC_CUDA_OK(cudaStreamWaitEvent(chain, ev[cur_indices_from], 0));
       const size_t ws_bytes = spc_rulebook_workspace_bytes(&L.geom, cur_n);
       if (ws_bytes == 0) return fail(SPC_ERR_INVALID_ARGUMENT, "sequence_forward: layer %d: geometry rejected", i);
       R.workspace = arena.take(ws_bytes);
@@ -147,16 +151,20 @@ extern "C" int spc_sequence_forward(const spc_seq_layer* layers, int n_layers, c
       t.fwd_colmajor = colmajor ? static_cast<int32_t*>(arena.at(R.pair_fwd)) : nullptr;
       t.fwd_rowmajor = static_cast<int32_t*>(arena.at(R.pair_fwd_rowmajor));
       t.fwd_order = static_cast<int32_t*>(arena.at(R.mask_argsort));
+      if (!subm) {
+        SPC_CUDA_OK(cudaEventRecord(ev_numbered[i], chain));
+        SPC_CUDA_OK(cudaStreamWaitEvent(side, ev_numbered[i], 0));
+      }
       rc = rulebook_tables_chained(&L.geom, cur_indices, cur_n, n_out, arena.at(R.workspace), ws_bytes, t,
-                                   have_producer ? &producer : nullptr, st);
+                                   have_producer ? &producer : nullptr, side);
       if (rc != SPC_OK) return rc;
-      SPC_CUDA_OK(cudaEventRecord(ev[i], st));
+      SPC_CUDA_OK(cudaEventRecord(ev[i], side));
       if (!subm) {
         producer = RulebookProducer{&L.geom, arena.at(R.workspace), cur_n};
         have_producer = true;
         cur_indices = static_cast<const int32_t*>(arena.at(R.out_indices));
         cur_n = n_out;
-        cur_indices_ready = ev[i];
+        cur_indices_from = i;
       }
     } else {
       const spc_seq_result& G = results[L.rulebook];
@@ -184,8 +192,8 @@ extern "C" int spc_sequence_forward(const spc_seq_layer* layers, int n_layers, c
   *arena_needed = arena.used;
   // work queued on the rulebook streams must be over before the caller may free or reuse the arena
   // on its own stream: the caller's stream joins both
-  SPC_CUDA_OK(cudaEventRecord(ev[kMaxSeqLayers + 1], chain));
-  SPC_CUDA_OK(cudaStreamWaitEvent(main, ev[kMaxSeqLayers + 1], 0));
+  SPC_CUDA_OK(cudaEventRecord(ev[2 * kMaxSeqLayers + 1], chain));
+  SPC_CUDA_OK(cudaStreamWaitEvent(main, ev[2 * kMaxSeqLayers + 1], 0));
   SPC_CUDA_OK(cudaEventRecord(ev_input, side));
   SPC_CUDA_OK(cudaStreamWaitEvent(main, ev_input, 0));
   if (arena.overflow) {

@@ -66,13 +66,14 @@ deal_rows_kernel(const uint32_t* __restrict__ keys, long long n, const uint32_t*
   uint32_t before = 0;
   for (int w = 0; w < warp; ++w) before += warp_sum[w];
   uint32_t start = before + incl - sum;
+  uint32_t have[kPer], at_least[kPer];
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) have[q] = tid * kPer + q < kTileBuckets ? place[tid * kPer + q] : 0u;
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) at_least[q] = have[q] != 0 ? atomicAdd(&taken[tid * kPer + q], have[q]) : 0u;  // all in flight
 #pragma unroll
   for (int q = 0; q < kPer; ++q) {
-    const int b = tid * kPer + q;
-    if (b < kTileBuckets) {
-      const uint32_t have = place[b];
-      place[b] = have != 0 ? start + atomicAdd(&taken[b], have) : 0u;
-    }
+    if (have[q] != 0) place[tid * kPer + q] = start + at_least[q];
     start += mine[q];
   }
   __syncthreads();
@@ -87,7 +88,7 @@ deal_rows_kernel(const uint32_t* __restrict__ keys, long long n, const uint32_t*
 // order[piece] = the piece's rows in ascending key order.  `pairs` null: the rows are 0..n-1 with `keys`.
 // A least-significant-digit radix sort in shared memory: nine bits a pass, so three passes for the 27
 // offsets of a 3x3x3 kernel.  A warp ranks its rows 32 at a time (lanes with the same digit find each other
-// with a match, the first of them adds to the warp's count of that digit), then the counts of all warps
+// with nine ballots, the first of them adds to the warp's count of that digit), then the counts of all warps
 // become places by one block-wide sum in (digit, warp) order, which keeps the sort stable.
 template <int ITEMS>
 __global__ void __launch_bounds__(kPieceThreads)
@@ -117,7 +118,12 @@ sort_piece_kernel(const uint32_t* __restrict__ keys, const uint2* __restrict__ p
     for (int i = 0; i < ITEMS; ++i) {
       const bool live = at0 + i * 32 < left;
       const int digit = live ? static_cast<int>((mine[i].x >> bit) & (kDigits - 1)) : kDigits;
-      const unsigned same = __match_any_sync(0xffffffffu, digit);
+      unsigned same = __ballot_sync(0xffffffffu, live);
+#pragma unroll
+      for (int b = 0; b < kDigitBits; ++b) {
+        const unsigned ones = __ballot_sync(0xffffffffu, (digit >> b) & 1);
+        same &= (digit >> b) & 1 ? ones : ~ones;
+      }
       uint32_t before = 0;
       if (live) before = count[digit * kPieceWarps + warp];
       __syncwarp();
@@ -197,10 +203,12 @@ int tile_order(const uint32_t* keys, int64_t n, int kv, const uint32_t* counts, 
     if (n <= 4 * kPieceThreads) return launch_sort<4>(keys, nullptr, n, kv, order, st);
     return launch_sort<kItems>(keys, nullptr, n, kv, order, st);
   }
+  // pieces of 4096 rows where they still fit one wave of CTAs: the sort is as long as one piece takes
+  const bool small = n <= static_cast<int64_t>(sm_count()) * kTileOrderPiece / 2;
   const unsigned blocks = static_cast<unsigned>(ceil_div(n, kDealThreads * kDealItems));
   deal_rows_kernel<<<blocks, kDealThreads, 0, st>>>(keys, n, counts, taken, pairs);
   SPC_LAUNCH_OK();
-  return launch_sort<kItems>(keys, pairs, n, kv, order, st);
+  return small ? launch_sort<kItems / 2>(keys, pairs, n, kv, order, st) : launch_sort<kItems>(keys, pairs, n, kv, order, st);
 }
 
 }  // namespace spc
