@@ -201,6 +201,9 @@ int spc_rulebook_tables(const spc_geometry* g, const int32_t* indices, int64_t n
  * spc_rulebook_igemm (tables converted from the Native format, user tables). */
 int spc_pairs_to_rowmajor(const int32_t* pairs, int kv, int64_t n, int32_t* out, void* stream);
 
+/* ... and back: the column-major table [kv, n] of a row-major one. */
+int spc_rowmajor_to_pairs(const int32_t* rowmajor, int kv, int64_t n, int32_t* pairs, void* stream);
+
 /* Phase 2, Native format: replaces native_pairs, _impl/pairs.py:223-278.
  *   pair [2, kv, n_in] (-1 fill): per offset the contributing input rows in
  *   ascending order and their output rows; indice_num_per_loc [kv]. */
@@ -398,14 +401,31 @@ int spc_conv_backward_input(const void* grad_out, const void* weight,
  * fp32 layers (the reference's default, _impl/gemm.py:11-13) run on tcgen05.
  * spc_tf32_prepare_weight does the same for a KRSC weight [c_out, kv, c_in] ->
  * [c_out, kv, m c_in], or with `transpose` -> [c_in, kv, m c_out] (the operand
- * of the input gradient written as a forward convolution of grad_out), m = 1
- * (ROUND) or 3 (SPLIT_*).  No counterpart in the reference. */
+ * of the input gradient written as a forward convolution of grad_out; 2: with the
+ * offsets in reverse order as well), m = 1 (ROUND) or 3 (SPLIT_*).  No counterpart in the reference. */
 int spc_tf32_prepare(const float* src, float* dst, int64_t rows, int cols, int mode, void* stream);
 int spc_tf32_prepare_weight(const float* weight, float* dst, int c_out, int kv, int c_in,
                             int transpose, int mode, void* stream);
 
 /* Bytes of device scratch spc_conv_backward_weight needs (fp32 partial sums
  * of the split reduction). */
+/* spc_conv_backward_input for callers that hold one table: pair_bwd may be NULL when
+ * pair_bwd_rowmajor is given and spc_conv_backward_input_needs_colmajor says 0.  With
+ * `reversed` the tables are the forward tables of a submanifold layer, whose input
+ * side is the same with the kernel offsets in reverse order (offset k of the table
+ * meets weight kv - 1 - k), so that no table of that side has to exist. */
+int spc_conv_backward_input_tables(const void* grad_out, const void* weight, const int32_t* pair_bwd,
+                                   const int32_t* pair_bwd_rowmajor, const int32_t* mask_argsort, void* din,
+                                   int64_t n_in, int64_t n_out, int c_in, int c_out, int kv, int reversed, int dtype,
+                                   int precision, int path, void* stream);
+int spc_conv_backward_input_needs_colmajor(int c_in, int c_out, int kv, int dtype, int precision, int path);
+
+/* Column sums of x [rows, cols] (the gradient of a bias), added in fp32 in a fixed
+ * order; out [cols] of out_dtype (fp16, bf16 or fp32, as x). */
+size_t spc_column_sums_workspace_bytes(int64_t rows, int cols);
+int spc_column_sums(const void* x, int64_t rows, int cols, int dtype, void* out, int out_dtype, void* workspace,
+                    size_t workspace_bytes, void* stream);
+
 size_t spc_conv_backward_weight_workspace_bytes(int64_t n_out, int c_in, int c_out, int kv);
 
 /* Weight gradient: replaces conv_backward_weight, _impl/gemm.py:634-713.
@@ -464,6 +484,20 @@ int spc_avgpool_forward(const void* features, const int32_t* pair_fwd, void* out
 int spc_avgpool_backward(const void* grad_out, const int32_t* pair_bwd, const int32_t* count,
                          void* din, int64_t n_in, int channels, int kv, int dtype,
                          void* stream);
+
+/* The same four operators over a row-major table [n_rows, pitch] (pitch 0: column-major
+ * [kv, n_rows]).  src: features forward, grad_out backward; own / ref: features and
+ * pooled output (max backward); aux_in / aux_out: the counts of the average.  Every
+ * element of dst (and aux_out) is written. */
+typedef enum {
+  SPC_POOL_MAX_FORWARD = 0,
+  SPC_POOL_AVG_FORWARD = 1,
+  SPC_POOL_AVG_BACKWARD = 2,
+  SPC_POOL_MAX_BACKWARD = 3
+} spc_pool_op;
+int spc_pool(int op, const void* src, const void* own, const void* ref, const int32_t* table, int pitch,
+             const int32_t* aux_in, void* dst, int32_t* aux_out, int64_t n_rows, int channels, int kv, int dtype,
+             void* stream);
 
 /* ---- a chain of convolutions in one call --------------------------------- */
 

@@ -80,9 +80,9 @@ inline cudaError_t ensure_dynamic_smem(Kernel kernel, int bytes, bool (&done)[kM
 }
 
 // What happens to an accumulator row before it is stored:
-//   v = acc (+ bias[n]);  v = v * scale[n] + shift[n] (if scale);  v = act(v);  v += residual[row, n]
+//   v = acc (+ bias[n]);  v = v * scale[n] (if scale) + shift[n] (if shift);  v = act(v);  v += residual[row, n]
 // bias has the dtype of the inputs; scale and shift are fp32 (a folded
-// inference BatchNorm); act is an spc_activation; residual is a row-major
+// inference BatchNorm; shift alone: a bias in fp32); act is an spc_activation; residual is a row-major
 // [rows, n_dim] matrix of the OUTPUT dtype, added in fp32 before the one rounding
 // of the store (a residual connection fused into the convolution).
 struct Epilogue {
@@ -158,6 +158,7 @@ template <typename T>
 __device__ __forceinline__ float apply_epilogue(float v, const Epilogue& e, int n) {
   if (e.bias != nullptr) v += to_float(static_cast<const T*>(e.bias)[n]);
   if (e.scale != nullptr) v = fmaf(v, __ldg(&e.scale[n]), __ldg(&e.shift[n]));
+  else if (e.shift != nullptr) v += __ldg(&e.shift[n]);
   if (e.act == SPC_ACT_RELU) v = fmaxf(v, 0.f);
   else if (e.act == SPC_ACT_LEAKY_RELU) v = v > 0.f ? v : v * e.alpha;
   else if (e.act == SPC_ACT_SIGMOID) v = 1.f / (1.f + __expf(-v));

@@ -56,8 +56,8 @@ extern "C" int spc_conv_forward_residual(const void* features, const void* weigh
   if (!pair_fwd && (!pair_fwd_rowmajor ||
                     spc_conv_forward_needs_colmajor(c_in, c_out, kv, dtype, out_dtype, precision, path)))
     return fail(SPC_ERR_INVALID_ARGUMENT, "conv_forward: this layer reads the column-major table");
-  if ((out_scale == nullptr) != (out_shift == nullptr))
-    return fail(SPC_ERR_INVALID_ARGUMENT, "conv_forward: out_scale and out_shift go together");
+  if (out_scale != nullptr && out_shift == nullptr)
+    return fail(SPC_ERR_INVALID_ARGUMENT, "conv_forward: out_scale needs out_shift");
   if (n_out == 0) return SPC_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   Epilogue epi;
@@ -70,9 +70,9 @@ extern "C" int spc_conv_forward_residual(const void* features, const void* weigh
     if (path != SPC_GEMM_TCGEN05_CPASYNC &&
         gather_gemm_tma_supported(c_out, c_in, kv, dtype, out_dtype, precision, false))
       return gather_gemm_tma(features, weight, epi, pair_fwd, pair_fwd_rowmajor, mask_argsort, out, n_in, n_out, c_out, c_in, kv,
-                             /*transposed_weight=*/false, dtype, out_dtype, precision, st);
+                             /*transposed_weight=*/false, /*reversed=*/false, dtype, out_dtype, precision, st);
     return gather_gemm_tc(features, weight, epi, pair_fwd, mask_argsort, out, n_out, c_out, c_in, kv,
-                          /*transposed_weight=*/false, dtype, out_dtype, precision, st);
+                          /*transposed_weight=*/false, /*reversed=*/false, dtype, out_dtype, precision, st);
   }
   if (status != SPC_OK) return status;
   // weight[n, k, c]: reduction index c has stride 1, output channel n stride kv*c_in.
@@ -85,23 +85,42 @@ extern "C" int spc_conv_backward_input(const void* grad_out, const void* weight,
                                        const int32_t* pair_bwd_rowmajor, const int32_t* mask_argsort, void* din, int64_t n_in, int64_t n_out,
                                        int c_in, int c_out, int kv, int dtype, int precision, int path,
                                        void* stream) {
-  if (!grad_out || !weight || !pair_bwd || !din || n_in < 0 || n_out < 0 || c_in <= 0 || c_out <= 0 || kv <= 0)
+  if (!pair_bwd) return fail(SPC_ERR_INVALID_ARGUMENT, "conv_backward_input: bad arguments");
+  return spc_conv_backward_input_tables(grad_out, weight, pair_bwd, pair_bwd_rowmajor, mask_argsort, din, n_in, n_out, c_in, c_out,
+                                        kv, 0, dtype, precision, path, stream);
+}
+
+extern "C" int spc_conv_backward_input_needs_colmajor(int c_in, int c_out, int kv, int dtype, int precision, int path) {
+  const bool tma = path != SPC_GEMM_SIMT && path != SPC_GEMM_TCGEN05_CPASYNC &&
+                   gather_gemm_tc_supported(c_in, c_out, kv, dtype, dtype, precision, true) &&
+                   gather_gemm_tma_supported(c_in, c_out, kv, dtype, dtype, precision, true);
+  return tma ? 0 : 1;
+}
+
+extern "C" int spc_conv_backward_input_tables(const void* grad_out, const void* weight, const int32_t* pair_bwd,
+                                              const int32_t* pair_bwd_rowmajor, const int32_t* mask_argsort, void* din,
+                                              int64_t n_in, int64_t n_out, int c_in, int c_out, int kv, int reversed, int dtype,
+                                              int precision, int path, void* stream) {
+  if (!grad_out || !weight || !din || n_in < 0 || n_out < 0 || c_in <= 0 || c_out <= 0 || kv <= 0)
     return fail(SPC_ERR_INVALID_ARGUMENT, "conv_backward_input: bad arguments");
+  if (!pair_bwd && (!pair_bwd_rowmajor || spc_conv_backward_input_needs_colmajor(c_in, c_out, kv, dtype, precision, path)))
+    return fail(SPC_ERR_INVALID_ARGUMENT, "conv_backward_input: this layer reads the column-major table");
   if (n_in == 0) return SPC_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int status;
   if (want_tc(path, c_in, c_out, kv, dtype, dtype, precision, true, &status)) {
     if (path != SPC_GEMM_TCGEN05_CPASYNC && gather_gemm_tma_supported(c_in, c_out, kv, dtype, dtype, precision, true))
       return gather_gemm_tma(grad_out, weight, Epilogue{}, pair_bwd, pair_bwd_rowmajor, mask_argsort, din, n_out, n_in, c_in, c_out, kv,
-                             /*transposed_weight=*/true, dtype, dtype, precision, st);
+                             /*transposed_weight=*/true, reversed != 0, dtype, dtype, precision, st);
     return gather_gemm_tc(grad_out, weight, Epilogue{}, pair_bwd, mask_argsort, din, n_in, c_in, c_out, kv,
-                          /*transposed_weight=*/true, dtype, dtype, precision, st);
+                          /*transposed_weight=*/true, reversed != 0, dtype, dtype, precision, st);
   }
   if (status != SPC_OK) return status;
-  // output channel is c (stride 1), reduction index is n (stride kv*c_in).
-  return gather_gemm_simt(grad_out, weight, Epilogue{}, pair_bwd, mask_argsort, din, n_in, c_in, c_out, kv,
-                          /*s_wk=*/c_in, /*s_wr=*/static_cast<long long>(kv) * c_in, /*s_wn=*/1, dtype, dtype,
-                          st);
+  // output channel is c (stride 1), reduction index is n (stride kv*c_in); reversed offsets: from the last one down
+  const char* w = static_cast<const char*>(weight) + (reversed ? static_cast<size_t>(kv - 1) * c_in * dtype_size(dtype) : 0);
+  return gather_gemm_simt(grad_out, w, Epilogue{}, pair_bwd, mask_argsort, din, n_in, c_in, c_out, kv,
+                          /*s_wk=*/reversed ? -static_cast<long long>(c_in) : c_in, /*s_wr=*/static_cast<long long>(kv) * c_in, /*s_wn=*/1,
+                          dtype, dtype, st);
 }
 
 extern "C" size_t spc_conv_backward_weight_workspace_bytes(int64_t n_out, int c_in, int c_out, int kv) {

@@ -28,12 +28,12 @@ int wgrad_simt(const void* feats, const void* gout, const int32_t* pair_fwd, voi
                int64_t n_out, int c_in, int c_out, int kv, int dtype, cudaStream_t st);
 
 // tcgen05 kernels (gemm_tc.cu).  `transposed_weight` selects the input-gradient
-// view of the KRSC weight.  Return SPC_ERR_UNSUPPORTED for shapes they do not take.
+// view of the KRSC weight; `reversed`: offset k of the table meets weight kv - 1 - k.  Return SPC_ERR_UNSUPPORTED for shapes they do not take.
 bool gather_gemm_tc_supported(int n_dim, int r_dim, int kv, int dtype, int out_dtype, int precision,
                               bool transposed_weight);
 int gather_gemm_tc(const void* src, const void* w, const Epilogue& epi, const int32_t* pairs,
                    const int32_t* order, void* out, long long m_rows, int n_dim, int r_dim, int kv,
-                   bool transposed_weight, int dtype, int out_dtype, int precision, cudaStream_t st);
+                   bool transposed_weight, bool reversed, int dtype, int out_dtype, int precision, cudaStream_t st);
 
 // dw[e] = sum over splits of partial[s, e], added in split order (deterministic).
 int wgrad_reduce(const float* partial, void* dw, long long elems, int splits, int dtype, cudaStream_t st);
@@ -52,6 +52,6 @@ bool gather_gemm_tma_supported(int n_dim, int r_dim, int kv, int dtype, int out_
                                bool transposed_weight);
 int gather_gemm_tma(const void* src, const void* w, const Epilogue& epi, const int32_t* pairs,
                     const int32_t* pairs_rowmajor, const int32_t* order, void* out, long long src_rows, long long m_rows, int n_dim, int r_dim,
-                    int kv, bool transposed_weight, int dtype, int out_dtype, int precision, cudaStream_t st);
+                    int kv, bool transposed_weight, bool reversed, int dtype, int out_dtype, int precision, cudaStream_t st);
 
 }  // namespace spc

@@ -54,6 +54,7 @@ struct TcParams {
   void* out;
   long long m_rows;
   int n_dim, r_dim, kv;
+  int reversed;  // offset k of the table meets weight kv - 1 - k
   int stages, b_stage_bytes, tmem_cols;
   int* status;
 };
@@ -105,7 +106,7 @@ gather_gemm_tc_kernel(const __grid_constant__ TcParams p) {
     tmem_alloc(smem_u32(tmem_slot), static_cast<uint32_t>(p.tmem_cols));
     tmem_relinquish();
   }
-  const bool has_epilogue = p.epi.bias != nullptr || p.epi.scale != nullptr || p.epi.act != SPC_ACT_NONE;
+  const bool has_epilogue = p.epi.bias != nullptr || p.epi.shift != nullptr || p.epi.act != SPC_ACT_NONE;
   if (has_epilogue) stage_epilogue<T>(p.epi, p.n_dim, epi_scale, epi_shift, tid, kThreadsTc);
   tc_fence_before();
   __syncthreads();
@@ -145,7 +146,7 @@ gather_gemm_tc_kernel(const __grid_constant__ TcParams p) {
 
       for (uint32_t rest = active; rest != 0; rest &= rest - 1) {
         const int kk = __ffs(rest) - 1;
-        const int k = k0 + kk;
+        const int k = p.reversed ? p.kv - 1 - (k0 + kk) : k0 + kk;  // of the weight
         for (int rc = 0; rc < n_rchunks; ++rc) {
           ++real_stages;
           if (ok && !mbar_wait(bar_empty + 8 * stage, empty_parity)) ok = false;
@@ -380,14 +381,14 @@ bool gather_gemm_tc_supported(int n_dim, int r_dim, int kv, int dtype, int out_d
 
 int gather_gemm_tc(const void* src, const void* w, const Epilogue& epi, const int32_t* pairs,
                    const int32_t* order, void* out, long long m_rows, int n_dim, int r_dim, int kv,
-                   bool transposed_weight, int dtype, int out_dtype, int precision, cudaStream_t st) {
+                   bool transposed_weight, bool reversed, int dtype, int out_dtype, int precision, cudaStream_t st) {
   if (!gather_gemm_tc_supported(n_dim, r_dim, kv, dtype, out_dtype, precision, transposed_weight))
     return fail(SPC_ERR_UNSUPPORTED, "tcgen05 gather-GEMM: unsupported shape");
   if ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(out)) & 15u)
     return fail(SPC_ERR_UNSUPPORTED, "tcgen05 gather-GEMM: operands must be 16-byte aligned");
   TcParams p{};
   p.src = src; p.w = w; p.epi = epi; p.pairs = pairs; p.order = order; p.out = out;
-  p.m_rows = m_rows; p.n_dim = n_dim; p.r_dim = r_dim; p.kv = kv;
+  p.m_rows = m_rows; p.n_dim = n_dim; p.r_dim = r_dim; p.kv = kv; p.reversed = reversed;
   p.status = device_status_ptr();
   if (p.status == nullptr) return fail(SPC_ERR_CUDA, "tcgen05 gather-GEMM: no device status word");
 #define SPC_TC(T, TO)                                                        \

@@ -83,6 +83,7 @@ struct TmaParams {
   int kvp;
   int src_rows;  // rows of the gathered matrix; also the "absent row" index
   int n_dim, r_dim, kv;
+  int reversed;  // offset k of the table meets weight kv - 1 - k
   int stages, a_stage_bytes, b_stage_bytes, tmem_cols;
   int group_rows;  // kernel offsets voted on together: min(kv, 32); sizes the table tile in shared memory
   int epi_pad;     // output channels rounded up to 16; sizes the epilogue scale / shift arrays
@@ -174,7 +175,7 @@ gather_gemm_tma_kernel(const __grid_constant__ TmaParams p, const __grid_constan
     tmem_alloc(smem_u32(tmem_slot), static_cast<uint32_t>(p.tmem_cols));
     tmem_relinquish();
   }
-  const bool has_epilogue = p.epi.bias != nullptr || p.epi.scale != nullptr || p.epi.act != SPC_ACT_NONE;
+  const bool has_epilogue = p.epi.bias != nullptr || p.epi.shift != nullptr || p.epi.act != SPC_ACT_NONE;
   if (has_epilogue) stage_epilogue<T>(p.epi, p.n_dim, epi_scale, epi_shift, tid, kThreadsHybrid);
   tc_fence_before();
   __syncthreads();
@@ -257,7 +258,7 @@ gather_gemm_tma_kernel(const __grid_constant__ TmaParams p, const __grid_constan
 
       for (uint32_t rest = ok ? active : 0u; rest != 0; rest &= rest - 1) {
         const int kk = __ffs(rest) - 1;
-        const int k = k0 + kk;
+        const int k = p.reversed ? p.kv - 1 - (k0 + kk) : k0 + kk;  // of the weight
         // this group's stages of the offset: every other one
         if (n_rchunks == 1 && turn != static_cast<uint32_t>(grp)) {
           turn ^= 1u;
@@ -443,6 +444,10 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 EncodeTiledFn encode_fn() {
+  // The driver call needs the thread's context, which a thread that has made no runtime call yet (autograd's,
+  // whose first step may be an input gradient) does not have: an empty free makes it current.
+  static thread_local bool current = false;
+  if (!current) current = cudaFree(nullptr) == cudaSuccess;
   static EncodeTiledFn fn = nullptr;
   static bool tried = false;
   if (!tried) {
@@ -505,7 +510,7 @@ bool gather_gemm_tma_supported(int n_dim, int r_dim, int kv, int dtype, int out_
 
 int gather_gemm_tma(const void* src, const void* w, const Epilogue& epi, const int32_t* pairs,
                     const int32_t* pairs_rowmajor, const int32_t* order, void* out, long long src_rows, long long m_rows, int n_dim, int r_dim,
-                    int kv, bool transposed_weight, int dtype, int out_dtype, int precision, cudaStream_t st) {
+                    int kv, bool transposed_weight, bool reversed, int dtype, int out_dtype, int precision, cudaStream_t st) {
   if (!gather_gemm_tma_supported(n_dim, r_dim, kv, dtype, out_dtype, precision, transposed_weight))
     return fail(SPC_ERR_UNSUPPORTED, "TMA gather-GEMM: unsupported shape");
   if (src_rows <= 0 || src_rows >= (1ll << 31) - 1)
@@ -518,7 +523,7 @@ int gather_gemm_tma(const void* src, const void* w, const Epilogue& epi, const i
   TmaParams p{};
   p.src = src; p.epi = epi; p.pairs = pairs; p.pairs_rm = pairs_rowmajor; p.kvp = (kv + 3) & ~3; p.order = order; p.out = out;
   p.m_rows = m_rows; p.src_rows = static_cast<int>(src_rows);
-  p.n_dim = n_dim; p.r_dim = r_dim; p.kv = kv;
+  p.n_dim = n_dim; p.r_dim = r_dim; p.kv = kv; p.reversed = reversed;
   p.a_row_bytes = row_span(r_dim, elem);
   p.b_row_bytes = transposed_weight ? row_span(n_dim, elem) : p.a_row_bytes;
   const int epr = p.a_row_bytes / elem;

@@ -1,0 +1,555 @@
+// Host side of the layers: rulebook, allocations, kernels and the autograd node of a sparse convolution or
+// pooling layer in one call each, over the C ABI of this library.
+//
+// Written in Python, these steps were 40 - 100 us of interpreter, ctypes and allocator calls a layer and
+// direction, more than the kernels of a layer of a few thousand voxels take.  Here a layer is two calls (its
+// rulebook, its arithmetic) that release the interpreter lock; backward never enters Python.
+#include <ATen/autocast_mode.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
+#include <torch/extension.h>
+
+#include <memory>
+#include <mutex>
+#include <unordered_map>
+
+#include "../../include/spconv_b200.h"
+
+namespace {
+
+using at::Tensor;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+
+struct Failure : std::runtime_error {
+  int status;
+  Failure(int s, const std::string& m) : std::runtime_error(m), status(s) {}
+};
+void check(int status) {
+  if (status != SPC_OK) throw Failure(status, spc_last_error());
+}
+
+void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+int32_t* ints(const Tensor& t) { return t.defined() ? t.data_ptr<int32_t>() : nullptr; }
+void* data(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+int code_of(at::ScalarType t) {
+  switch (t) {
+    case at::kHalf: return SPC_F16;
+    case at::kBFloat16: return SPC_BF16;
+    case at::kFloat: return SPC_F32;
+    case at::kDouble: return SPC_F64;
+    default: throw Failure(SPC_ERR_UNSUPPORTED, std::string("dtype ") + c10::toString(t) + " is not supported by spconv_triton_b200");
+  }
+}
+
+// ---- rulebooks -------------------------------------------------------------------------------------------
+
+struct Geometry {
+  spc_geometry g{};
+  int kv = 1, kvp = 4;
+  bool subm = false;
+  std::vector<int64_t> out_shape;
+};
+
+std::shared_ptr<Geometry> make_geometry(int batch, const std::vector<int>& in, const std::vector<int>& out,
+                                        const std::vector<int>& ksize, const std::vector<int>& stride,
+                                        const std::vector<int>& pad, const std::vector<int>& dil, bool subm, bool transpose) {
+  auto q = std::make_shared<Geometry>();
+  q->g.ndim = static_cast<int32_t>(in.size());
+  if (in.empty() || in.size() > SPC_MAX_NDIM) throw Failure(SPC_ERR_INVALID_ARGUMENT, "geometry: bad number of dimensions");
+  q->g.batch_size = batch;
+  q->g.subm = subm;
+  q->g.transpose = transpose;
+  for (size_t d = 0; d < in.size(); ++d) {
+    q->g.in_shape[d] = in[d];
+    q->g.out_shape[d] = out.at(d);
+    q->g.ksize[d] = ksize.at(d);
+    q->g.stride[d] = stride.at(d);
+    q->g.padding[d] = pad.at(d);
+    q->g.dilation[d] = dil.at(d);
+    q->kv *= ksize[d];
+    q->out_shape.push_back(out[d]);
+  }
+  q->kvp = (q->kv + 3) & ~3;
+  q->subm = subm;
+  return q;
+}
+
+// Rows from which on the GEMM's row order is worth its sort: with a tile or less there is nothing to group.
+constexpr int64_t kOrderRows = 256;
+
+// The tables of one rulebook, output side and input side, made as they are asked for.  The kernels read the
+// row-major tables; the column-major ones serve the CUDA-core and weight-gradient kernels.
+struct Rulebook {
+  std::shared_ptr<Geometry> geo;
+  Tensor indices, out_indices, workspace;
+  int64_t n_in = 0, n_out = 0;
+  struct Side {
+    Tensor rm, cm, order;
+  } fwd, bwd;
+  std::mutex lock;
+
+  bool subm() const { return geo->subm; }
+  Tensor make(int64_t a, int64_t b) const { return at::empty({a, b}, indices.options()); }
+  bool ordered(int64_t n) const { return geo->kv > 1 && geo->kv <= 32 && n > kOrderRows; }
+
+  void tables(const Tensor& oi, const Side& f, const Side& b) {
+    check(spc_rulebook_tables(&geo->g, ints(indices), n_in, n_out, workspace.data_ptr(), workspace.numel(), ints(oi), ints(f.cm),
+                              ints(f.rm), ints(f.order), ints(b.cm), ints(b.rm), ints(b.order), stream_of(indices)));
+  }
+  Side new_side(int64_t n, bool colmajor, bool order = true) const {
+    Side s;
+    s.rm = make(n, geo->kvp);
+    if (colmajor) s.cm = make(geo->kv, n);
+    if (order && ordered(n)) s.order = at::empty({n}, indices.options());
+    return s;
+  }
+  // The side whose rows are the output rows (of the layer, or of its inverse with `input`).
+  const Side& side(bool input, bool colmajor) {
+    std::lock_guard<std::mutex> hold(lock);
+    if (input && subm()) throw Failure(SPC_ERR_INVALID_ARGUMENT, "a submanifold rulebook has one side");
+    Side& s = input ? bwd : fwd;
+    if (!s.rm.defined()) {
+      c10::cuda::CUDAGuard guard(indices.device());
+      Side made = new_side(n_in, colmajor);
+      tables(Tensor(), Side(), made);
+      s = made;
+    }
+    if (colmajor && !s.cm.defined()) {
+      c10::cuda::CUDAGuard guard(indices.device());
+      const int64_t n = s.rm.size(0);
+      Tensor cm = make(geo->kv, n);
+      check(spc_rowmajor_to_pairs(ints(s.rm), geo->kv, n, ints(cm), stream_of(indices)));
+      s.cm = cm;
+    }
+    return s;
+  }
+  std::vector<Tensor> parts() const {
+    std::vector<Tensor> all;
+    for (const Tensor& t : {indices, out_indices, workspace, fwd.rm, fwd.cm, fwd.order, bwd.rm, bwd.cm, bwd.order})
+      if (t.defined()) all.push_back(t);
+    return all;
+  }
+};
+using Book = std::shared_ptr<Rulebook>;
+
+// Returns a rulebook with n_out == 0 where no point is left.
+Book build_rulebook(const std::shared_ptr<Geometry>& geo, Tensor indices, bool input_side, bool colmajor, bool order) {
+  pybind11::gil_scoped_release release;
+  c10::cuda::CUDAGuard guard(indices.device());
+  auto rb = std::make_shared<Rulebook>();
+  rb->geo = geo;
+  rb->indices = indices = indices.contiguous();
+  rb->n_in = indices.size(0);
+  const size_t bytes = spc_rulebook_workspace_bytes(&geo->g, rb->n_in);
+  if (bytes == 0) throw pybind11::value_error("rulebook geometry rejected by libspconv_b200");
+  rb->workspace = at::empty({static_cast<int64_t>(bytes)}, indices.options().dtype(at::kByte));
+  check(spc_rulebook_prepare(&geo->g, ints(indices), rb->n_in, rb->workspace.data_ptr(), bytes, &rb->n_out, stream_of(indices)));
+  if (rb->n_out == 0) return rb;
+  Rulebook::Side f = rb->new_side(rb->n_out, colmajor, order), b;
+  rb->out_indices = geo->subm ? indices : rb->make(rb->n_out, geo->g.ndim + 1);
+  if (input_side && !geo->subm) b = rb->new_side(rb->n_in, false, order);
+  rb->tables(geo->subm ? Tensor() : rb->out_indices, f, b);
+  rb->fwd = f;
+  rb->bwd = b;
+  if (geo->subm || b.rm.defined()) rb->workspace = Tensor();  // nothing is made from it any more
+  return rb;
+}
+
+void record_stream(const Book& rb, const Tensor& like) {
+  const auto st = c10::cuda::getCurrentCUDAStream(like.device().index());
+  for (const Tensor& t : rb->parts()) t.record_stream(st);
+}
+
+// ---- fp32 operands for the tensor cores ----------------------------------------------------------------------
+
+// How fp32 operands are multiplied: on the CUDA cores, or prepared as TF32 numbers (rounded once, or split in
+// two for IEEE accuracy, where the reduction is short enough for the tensor cores' accumulator).
+struct Fp32Plan {
+  bool tensor = false;
+  int rows_mode = 0, weight_mode = 0, mult = 1;
+};
+Fp32Plan fp32_plan(int n_dim, int r_dim, int kv, bool tf32, int split_most) {
+  Fp32Plan p;
+  if (n_dim % 16 || n_dim < 16 || n_dim > 256 || r_dim % 8) return p;
+  if (tf32) {
+    p.tensor = true;
+    p.rows_mode = p.weight_mode = SPC_TF32_ROUND;
+  } else if (kv * r_dim <= split_most) {
+    p.tensor = true;
+    p.rows_mode = SPC_TF32_SPLIT_A;
+    p.weight_mode = SPC_TF32_SPLIT_B;
+    p.mult = 3;
+  }
+  return p;
+}
+Tensor prepared_rows(const Tensor& x, const Fp32Plan& p) {
+  Tensor out = at::empty({x.size(0), p.mult * x.size(1)}, x.options());
+  check(spc_tf32_prepare(x.data_ptr<float>(), out.data_ptr<float>(), x.size(0), x.size(1), p.rows_mode, stream_of(x)));
+  return out;
+}
+
+// Prepared copies of weights, kept until the weight changes or goes away.  At most 256 weights.
+class WeightCache {
+ public:
+  // transposed: 0 as it is, 1 as the input gradient reads it, 2 with the offsets reversed as well
+  Tensor get(const Tensor& w, int transposed, const Fp32Plan& p) {
+    const int slot = transposed * 8 + p.weight_mode;
+    auto* key = w.unsafeGetTensorImpl();
+    const uint32_t version = w.is_inference() ? 0 : w._version();
+    const auto stream = c10::cuda::getCurrentCUDAStream(w.device().index());
+    {
+      std::lock_guard<std::mutex> hold(lock_);
+      auto it = kept_.find(key);
+      if (it != kept_.end() && !w.is_inference()) {
+        Entry& e = it->second;
+        if (!e.owner.expired() && e.version == version && e.at == w.data_ptr() && e.stream == stream.stream()) {
+          auto hit = e.made.find(slot);
+          if (hit != e.made.end()) return hit->second;
+        }
+      }
+    }
+    const int64_t k_out = w.size(0), c_in = w.size(w.dim() - 1), kv = w.numel() / (k_out * c_in);
+    Tensor out = transposed ? at::empty({c_in, kv, p.mult * k_out}, w.options()) : at::empty({k_out, kv, p.mult * c_in}, w.options());
+    check(spc_tf32_prepare_weight(w.data_ptr<float>(), out.data_ptr<float>(), k_out, kv, c_in, transposed, p.weight_mode, stream.stream()));
+    if (w.is_inference()) return out;
+    std::lock_guard<std::mutex> hold(lock_);
+    Entry& e = kept_[key];
+    if (e.owner.expired() || e.version != version || e.at != w.data_ptr() || e.stream != stream.stream())
+      e = Entry{c10::weak_intrusive_ptr<c10::TensorImpl>(w.getIntrusivePtr()), version, w.data_ptr(), stream.stream(), {}};
+    e.made[slot] = out;
+    if (kept_.size() > 256)
+      for (auto it = kept_.begin(); it != kept_.end();)
+        it = it->second.owner.expired() || (kept_.size() > 256 && it->first != key) ? kept_.erase(it) : std::next(it);
+    return out;
+  }
+
+ private:
+  struct Entry {
+    c10::weak_intrusive_ptr<c10::TensorImpl> owner{c10::intrusive_ptr<c10::TensorImpl>()};
+    uint32_t version = 0;
+    void* at = nullptr;
+    void* stream = nullptr;
+    std::unordered_map<int, Tensor> made;
+  };
+  std::mutex lock_;
+  std::unordered_map<c10::TensorImpl*, Entry> kept_;
+};
+WeightCache& weight_cache() {
+  static WeightCache* c = new WeightCache();  // (tensors must not outlive the CUDA context's end)
+  return *c;
+}
+
+// ---- convolution -------------------------------------------------------------------------------------------------
+
+struct ConvOptions {
+  bool inverse = false;  // the rulebook of a strided layer run backwards
+  bool tf32 = false;
+  int split_most = 0;    // longest reduction that the split fp32 operands may have
+};
+
+Tensor conv_forward_raw(const Tensor& features, const Tensor& weight, const Tensor& bias, const Tensor& residual, const Book& rb,
+                        const ConvOptions& o, at::ScalarType out_type, Tensor scale, Tensor shift, int act, double alpha) {
+  c10::cuda::CUDAGuard guard(features.device());
+  Tensor x = features.contiguous(), w = weight.contiguous();
+  if (w.scalar_type() != x.scalar_type()) w = w.to(x.scalar_type());
+  int64_t k_out = w.size(0), c_in = w.size(w.dim() - 1), kv = rb->geo->kv;
+  const int64_t n_in = o.inverse ? rb->n_out : rb->n_in, n_out = o.inverse ? rb->n_in : rb->n_out;
+  if (x.size(0) != n_in || x.size(1) != c_in || w.numel() != k_out * kv * c_in)
+    throw pybind11::value_error("features do not match the rulebook or the weight of the layer");
+  Tensor b = bias;
+  if (b.defined() && b.scalar_type() != x.scalar_type()) {
+    if (!shift.defined() && b.scalar_type() == at::kFloat) {
+      shift = b.contiguous();  // added in fp32
+      b = Tensor();
+    } else {
+      b = b.to(x.scalar_type());
+    }
+  }
+  if (b.defined()) b = b.contiguous();
+  Tensor r = residual.defined() ? residual.contiguous() : residual;
+  Tensor out = at::empty({n_out, k_out}, x.options().dtype(out_type));
+  int precision = x.scalar_type() == at::kFloat && o.tf32 ? SPC_PREC_TF32 : SPC_PREC_IEEE;
+  if (x.scalar_type() == at::kFloat && out_type == at::kFloat) {
+    const Fp32Plan plan = fp32_plan(k_out, c_in, kv, o.tf32, o.split_most);
+    if (plan.tensor) {
+      x = prepared_rows(x, plan);
+      w = weight_cache().get(w, 0, plan);
+      c_in *= plan.mult;
+      precision = SPC_PREC_TF32;
+    }
+  }
+  const int type = code_of(x.scalar_type()), out_code = code_of(out_type);
+  const bool colmajor = spc_conv_forward_needs_colmajor(c_in, k_out, kv, type, out_code, precision, SPC_GEMM_AUTO);
+  const Rulebook::Side& t = rb->side(o.inverse, colmajor);
+  check(spc_conv_forward_residual(x.data_ptr(), w.data_ptr(), data(b), ints(t.cm), ints(t.rm), ints(t.order), out.data_ptr(), n_in, n_out,
+                                  c_in, k_out, kv, type, out_code, precision, SPC_GEMM_AUTO,
+                                  scale.defined() ? scale.data_ptr<float>() : nullptr, shift.defined() ? shift.data_ptr<float>() : nullptr,
+                                  act, static_cast<float>(alpha), data(r), stream_of(x)));
+  return out;
+}
+
+Tensor conv_backward_input_raw(const Tensor& grad, const Tensor& weight, const Book& rb, const ConvOptions& o) {
+  const int64_t k_out = weight.size(0), c_in = weight.size(weight.dim() - 1), kv = rb->geo->kv;
+  const int64_t n_grad = o.inverse ? rb->n_in : rb->n_out, n_in = o.inverse ? rb->n_out : rb->n_in;
+  Tensor w = weight.scalar_type() == grad.scalar_type() ? weight : weight.to(grad.scalar_type());
+  Tensor din = at::empty({n_in, c_in}, grad.options());
+  // a submanifold layer's input side is its output side with the offsets reversed
+  const bool reversed = rb->subm(), input = !reversed && !o.inverse;
+  const int type = code_of(grad.scalar_type());
+  const int precision = type == SPC_F32 && o.tf32 ? SPC_PREC_TF32 : SPC_PREC_IEEE;
+  const Fp32Plan plan = type == SPC_F32 ? fp32_plan(c_in, k_out, kv, o.tf32, o.split_most) : Fp32Plan();
+  if (plan.tensor) {
+    // as a forward convolution of grad with the transposed weight
+    Tensor g = prepared_rows(grad, plan), wt = weight_cache().get(w, reversed ? 2 : 1, plan);
+    const bool colmajor = spc_conv_forward_needs_colmajor(plan.mult * k_out, c_in, kv, type, type, SPC_PREC_TF32, SPC_GEMM_AUTO);
+    const Rulebook::Side& t = rb->side(input, colmajor);
+    check(spc_conv_forward(g.data_ptr(), wt.data_ptr(), nullptr, ints(t.cm), ints(t.rm), ints(t.order), din.data_ptr(), n_grad, n_in,
+                           plan.mult * k_out, c_in, kv, type, type, SPC_PREC_TF32, SPC_GEMM_AUTO, nullptr, nullptr, SPC_ACT_NONE, 0.f,
+                           stream_of(g)));
+    return din;
+  }
+  const bool colmajor = spc_conv_backward_input_needs_colmajor(c_in, k_out, kv, type, precision, SPC_GEMM_AUTO);
+  const Rulebook::Side& t = rb->side(input, colmajor);
+  check(spc_conv_backward_input_tables(grad.data_ptr(), w.data_ptr(), ints(t.cm), ints(t.rm), ints(t.order), din.data_ptr(), n_in, n_grad,
+                                       c_in, k_out, kv, reversed, type, precision, SPC_GEMM_AUTO, stream_of(grad)));
+  return din;
+}
+
+Tensor conv_backward_weight_raw(const Tensor& features, const Tensor& grad, at::IntArrayRef sizes, const Book& rb, const ConvOptions& o) {
+  const int64_t k_out = sizes[0], c_in = sizes[sizes.size() - 1], kv = rb->geo->kv;
+  Tensor dw = at::empty(sizes, grad.options());
+  Tensor x = features.scalar_type() == grad.scalar_type() ? features : features.to(grad.scalar_type());
+  const Rulebook::Side& t = rb->side(o.inverse, true);
+  const int64_t n_out = grad.size(0);
+  const size_t bytes = spc_conv_backward_weight_workspace_bytes(n_out, c_in, k_out, kv);
+  Tensor ws = at::empty({static_cast<int64_t>(std::max<size_t>(bytes, 16))}, grad.options().dtype(at::kByte));
+  const int type = code_of(grad.scalar_type());
+  check(spc_conv_backward_weight(x.data_ptr(), grad.data_ptr(), ints(t.cm), dw.data_ptr(), ws.data_ptr(), ws.numel(), x.size(0), n_out,
+                                 c_in, k_out, kv, type, type == SPC_F32 && o.tf32 ? SPC_PREC_TF32 : SPC_PREC_IEEE, SPC_GEMM_AUTO,
+                                 stream_of(grad)));
+  return dw;
+}
+
+Tensor column_sums(const Tensor& x, at::ScalarType out_type) {
+  const int64_t rows = x.size(0), cols = x.size(1);
+  Tensor out = at::empty({cols}, x.options().dtype(out_type));
+  Tensor ws = at::empty({static_cast<int64_t>(std::max<size_t>(spc_column_sums_workspace_bytes(rows, cols), 16))}, x.options().dtype(at::kByte));
+  check(spc_column_sums(x.data_ptr(), rows, cols, code_of(x.scalar_type()), out.data_ptr(), code_of(out_type), ws.data_ptr(), ws.numel(),
+                        stream_of(x)));
+  return out;
+}
+
+// Backward of these layers cannot be differentiated again: with create_graph the gradients carry an error.
+variable_list once_differentiable(variable_list&& out, const variable_list& grads, bool create_graph) {
+  bool any = false;
+  for (const Tensor& g : grads) any = any || (g.defined() && g.requires_grad());
+  if (!create_graph || !any) return std::move(out);
+  at::AutoGradMode grad(true);
+  auto error = std::shared_ptr<torch::autograd::DelayedError>(
+      new torch::autograd::DelayedError("trying to differentiate twice a function that was marked with @once_differentiable", out.size()),
+      torch::autograd::deleteNode);
+  for (Tensor& t : out)
+    if (t.defined()) t = t.detach().set_requires_grad(true);
+  return (*error)(std::move(out));
+}
+
+bool wants_grad(std::initializer_list<const Tensor*> ts) {
+  if (!at::GradMode::is_enabled()) return false;
+  for (const Tensor* t : ts)
+    if (t->defined() && t->requires_grad()) return true;
+  return false;
+}
+
+// Inside autocast these layers compute in fp16 whatever its type, as the reference's functions do.
+Tensor cast_for_autocast(const Tensor& t) {
+  if (!at::autocast::is_autocast_enabled(at::kCUDA) || !t.defined() || !t.is_floating_point() || t.scalar_type() == at::kDouble) return t;
+  return t.to(at::kHalf);
+}
+
+struct ConvBackward : public torch::autograd::Node {
+  SavedVariable features_, weight_;
+  Book rb;
+  ConvOptions options;
+  bool bias = false, residual = false;
+  at::ScalarType bias_type = at::kFloat;
+
+  variable_list apply(variable_list&& grads) override {
+    std::lock_guard<std::mutex> hold(mutex_);
+    variable_list out(4);
+    if (!grads[0].defined()) return out;
+    const Tensor weight = weight_.unpack();
+    Tensor features;
+    if (task_should_compute_output(1)) features = features_.unpack();
+    const bool create_graph = at::GradMode::is_enabled();
+    at::AutoGradMode no_grad(false);
+    c10::cuda::CUDAGuard guard(grads[0].device());
+    Tensor grad = grads[0].contiguous();
+    if (bias && task_should_compute_output(2)) out[2] = column_sums(grad, bias_type);
+    if (task_should_compute_output(0)) out[0] = conv_backward_input_raw(grad, weight, rb, options);
+    if (task_should_compute_output(1)) out[1] = conv_backward_weight_raw(features, grad, weight.sizes(), rb, options);
+    if (residual && task_should_compute_output(3)) out[3] = grads[0];
+    return once_differentiable(std::move(out), grads, create_graph);
+  }
+  void release_variables() override {
+    std::lock_guard<std::mutex> hold(mutex_);
+    features_.reset_data();
+    weight_.reset_data();
+  }
+  std::string name() const override { return "SparseImplicitGemmFunctionBackward"; }
+};
+
+// A convolution in training: out = gather-GEMM (+ bias) (+ residual), with its place in the autograd graph.
+Tensor conv_train(const Tensor& features, const Tensor& weight, const c10::optional<Tensor>& bias_opt, const c10::optional<Tensor>& residual_opt,
+                  const Book& rb, bool inverse, bool tf32, int split_most) {
+  pybind11::gil_scoped_release release;
+  const Tensor bias = bias_opt.value_or(Tensor()), residual = residual_opt.value_or(Tensor());
+  const bool grad = wants_grad({&features, &weight, &bias, &residual});
+  ConvOptions o{inverse, tf32, split_most};
+  Tensor x, w, out;
+  {
+    at::NoGradGuard no_grad;
+    x = cast_for_autocast(features).contiguous();
+    w = cast_for_autocast(weight).contiguous();
+    out = conv_forward_raw(x, w, bias, residual, rb, o, x.scalar_type(), Tensor(), Tensor(), SPC_ACT_NONE, 0.0);
+  }
+  if (!grad) return out;
+  auto node = std::shared_ptr<ConvBackward>(new ConvBackward(), torch::autograd::deleteNode);
+  node->set_next_edges(torch::autograd::collect_next_edges(features, weight, bias, residual));
+  node->features_ = SavedVariable(x, false);
+  node->weight_ = SavedVariable(w, false);
+  node->rb = rb;
+  node->options = o;
+  node->bias = bias.defined();
+  node->residual = residual.defined();
+  if (bias.defined()) node->bias_type = bias.scalar_type();
+  torch::autograd::set_history(out, node);
+  return out;
+}
+
+Tensor conv_eval(const Tensor& features, const Tensor& weight, const c10::optional<Tensor>& bias, const Book& rb, bool inverse, bool tf32,
+                 int split_most, const c10::optional<Tensor>& scale, const c10::optional<Tensor>& shift, int act, double alpha) {
+  pybind11::gil_scoped_release release;
+  at::NoGradGuard no_grad;
+  return conv_forward_raw(features, weight, bias.value_or(Tensor()), Tensor(), rb, ConvOptions{inverse, tf32, split_most},
+                          weight.scalar_type(), scale.value_or(Tensor()), shift.value_or(Tensor()), act, alpha);
+}
+
+// ---- pooling -------------------------------------------------------------------------------------------------------
+
+Tensor pool_rows(int op, const Tensor& src, const Tensor& own, const Tensor& ref, const Book& rb, bool input, const Tensor& aux_in,
+                 const Tensor& aux_out) {
+  const int64_t c = src.size(1);
+  const bool flip = rb->subm() && input;  // (a pool over a submanifold neighbourhood: the table of the other side)
+  const Rulebook::Side& t = rb->side(input && !flip, false);
+  const int64_t n = t.rm.size(0);
+  Tensor out = at::empty({n, c}, src.options());
+  if (c == 0) return out;
+  check(spc_pool(op, src.data_ptr(), data(own), data(ref), ints(t.rm), rb->geo->kvp, ints(aux_in), out.data_ptr(), ints(aux_out), n, c,
+                 rb->geo->kv, code_of(src.scalar_type()), stream_of(src)));
+  return out;
+}
+
+struct PoolBackward : public torch::autograd::Node {
+  SavedVariable features_, out_, count_;
+  Book rb;
+  bool average = false;
+
+  variable_list apply(variable_list&& grads) override {
+    std::lock_guard<std::mutex> hold(mutex_);
+    variable_list result(1);
+    if (!grads[0].defined() || !task_should_compute_output(0)) return result;
+    Tensor features, out, count;
+    if (average) {
+      count = count_.unpack();
+    } else {
+      features = features_.unpack();
+      out = out_.unpack(shared_from_this());
+    }
+    const bool create_graph = at::GradMode::is_enabled();
+    at::AutoGradMode no_grad(false);
+    c10::cuda::CUDAGuard guard(grads[0].device());
+    Tensor grad = grads[0].contiguous();
+    if (average) {
+      result[0] = pool_rows(SPC_POOL_AVG_BACKWARD, grad, Tensor(), Tensor(), rb, true, count, Tensor());
+    } else {
+      if (grad.scalar_type() != features.scalar_type()) grad = grad.to(features.scalar_type());
+      result[0] = pool_rows(SPC_POOL_MAX_BACKWARD, grad, features, out, rb, true, Tensor(), Tensor());
+    }
+    return once_differentiable(std::move(result), grads, create_graph);
+  }
+  void release_variables() override {
+    std::lock_guard<std::mutex> hold(mutex_);
+    features_.reset_data();
+    out_.reset_data();
+    count_.reset_data();
+  }
+  std::string name() const override {
+    return average ? "SparseAvgPoolImplicitGemmFunctionBackward" : "SparseMaxPoolImplicitGemmFunctionBackward";
+  }
+};
+
+Tensor pool(const Tensor& features, const Book& rb, bool average) {
+  pybind11::gil_scoped_release release;
+  const bool grad = wants_grad({&features});
+  Tensor x, out, count;
+  {
+    at::NoGradGuard no_grad;
+    c10::cuda::CUDAGuard guard(features.device());
+    x = cast_for_autocast(features).contiguous();
+    if (x.size(0) != rb->n_in) throw pybind11::value_error("features do not match the rulebook of the layer");
+    if (average) count = at::empty({rb->n_out}, rb->indices.options());
+    out = pool_rows(average ? SPC_POOL_AVG_FORWARD : SPC_POOL_MAX_FORWARD, x, Tensor(), Tensor(), rb, false, Tensor(), count);
+  }
+  if (!grad) return out;
+  auto node = std::shared_ptr<PoolBackward>(new PoolBackward(), torch::autograd::deleteNode);
+  node->set_next_edges(torch::autograd::collect_next_edges(features));
+  node->rb = rb;
+  node->average = average;
+  torch::autograd::set_history(out, node);
+  if (average) {
+    node->count_ = SavedVariable(count, false);
+  } else {
+    node->features_ = SavedVariable(x, false);
+    node->out_ = SavedVariable(out, true);
+  }
+  return out;
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_host, m) {
+  namespace py = pybind11;
+  static PyObject* error_type = nullptr;  // SpconvB200Error(status, message), handed over by the package
+  m.def("set_error_type", [](py::object t) { error_type = t.release().ptr(); });
+  py::register_exception_translator([](std::exception_ptr p) {
+    try {
+      if (p) std::rethrow_exception(p);
+    } catch (const Failure& f) {
+      py::object e = py::reinterpret_borrow<py::object>(error_type)(f.status, std::string(f.what()));
+      PyErr_SetObject(error_type, e.ptr());
+    }
+  });
+  py::class_<Geometry, std::shared_ptr<Geometry>>(m, "Geometry")
+      .def(py::init(&make_geometry))
+      .def_readonly("kv", &Geometry::kv)
+      .def_readonly("subm", &Geometry::subm)
+      .def_readonly("out_shape", &Geometry::out_shape);
+  py::class_<Rulebook, Book>(m, "Rulebook")
+      .def_readonly("n_in", &Rulebook::n_in)
+      .def_readonly("n_out", &Rulebook::n_out)
+      .def_readonly("geometry", &Rulebook::geo)
+      .def_readonly("indices", &Rulebook::indices)
+      .def_readonly("out_indices", &Rulebook::out_indices)
+      .def("rowmajor", [](Rulebook& r, bool input) { return r.side(input, false).rm; }, py::call_guard<py::gil_scoped_release>())
+      .def("colmajor", [](Rulebook& r, bool input) { return r.side(input, true).cm; }, py::call_guard<py::gil_scoped_release>());
+  m.def("build_rulebook", &build_rulebook);
+  m.def("record_stream", &record_stream);
+  m.def("conv_train", &conv_train);
+  m.def("conv_eval", &conv_eval);
+  m.def("pool", &pool);
+}

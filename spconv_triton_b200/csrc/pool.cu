@@ -211,7 +211,7 @@ template <typename T, int VEC, int U, int OP, int LGNT>
 __global__ void __launch_bounds__(256)
 pool_group_kernel(const T* __restrict__ src, const T* __restrict__ own, const T* __restrict__ ref,
                   const int32_t* __restrict__ table, const int32_t* __restrict__ aux_in, T* __restrict__ dst,
-                  int32_t* __restrict__ aux_out, long long n_rows, int channels, int kv) {
+                  int32_t* __restrict__ aux_out, long long n_rows, int channels, int kv, long long sk, int sr) {
   // the threads per row are a compile-time power of two: the entry loops below unroll to
   // exactly 32 / nt loads, ballots and selects
   constexpr int lg_nt = LGNT;
@@ -231,7 +231,7 @@ pool_group_kernel(const T* __restrict__ src, const T* __restrict__ own, const T*
 #pragma unroll
     for (int e = 0; e < kE; ++e) {
       const int k = k0 + e * nt + kl;
-      v[e] = (row < n_rows && e < per_lane && k < kv) ? __ldg(&table[static_cast<long long>(k) * n_rows + row]) : -1;
+      v[e] = (row < n_rows && e < per_lane && k < kv) ? __ldg(&table[k * sk + row * sr]) : -1;
     }
   };
 
@@ -289,7 +289,8 @@ template <typename T, int VEC, int U, int OP>
 __global__ void __launch_bounds__(256)
 pool_compact_kernel(const T* __restrict__ src, const T* __restrict__ own, const T* __restrict__ ref,
                     const int32_t* __restrict__ table, const int32_t* __restrict__ aux_in, T* __restrict__ dst,
-                    int32_t* __restrict__ aux_out, long long n_rows, int channels, int kv, PoolGeom g) {
+                    int32_t* __restrict__ aux_out, long long n_rows, int channels, int kv, long long sk, int sr,
+                    PoolGeom g) {
   constexpr int B = PoolTune<OP>::in_flight / U > 0 ? PoolTune<OP>::in_flight / U : 1;
   __shared__ int32_t tab[kChunk][kMaxRows + 1];
   __shared__ int32_t lst[kMaxRows][kChunk];
@@ -310,9 +311,10 @@ pool_compact_kernel(const T* __restrict__ src, const T* __restrict__ own, const 
     const int kc = min(kChunk, kv - k0);
     if (k0 != 0) __syncthreads();
     for (int i = t; i < kc * g.rpb; i += nthr) {
-      const int k = i / g.rpb, r = i - k * g.rpb;
+      // consecutive threads read consecutive entries of the table
+      const int k = sr == 1 ? i / g.rpb : i % kc, r = sr == 1 ? i - k * g.rpb : i / kc;
       const long long rr = row0 + r;
-      tab[k][r] = rr < n_rows ? __ldg(&table[static_cast<long long>(k0 + k) * n_rows + rr]) : -1;
+      tab[k][r] = rr < n_rows ? __ldg(&table[(k0 + k) * sk + rr * sr]) : -1;
     }
     __syncthreads();
     for (int r = warp; r < g.rpb; r += nwarps) {
@@ -344,7 +346,9 @@ int vec_for(int channels, const void* a, const void* b, const void* c = nullptr,
 
 template <typename T, int VEC, int U, int OP>
 void pool_launch_u(const T* src, const T* own, const T* ref, const int32_t* table, const int32_t* aux_in, T* dst,
-                   int32_t* aux_out, int64_t n_rows, int channels, int kv, cudaStream_t st) {
+                   int32_t* aux_out, int64_t n_rows, int channels, int kv, int pitch, cudaStream_t st) {
+  const long long sk = pitch ? 1 : n_rows;
+  const int sr = pitch ? pitch : 1;
   PoolGeom g;
   g.nt = channels / (VEC * U);
   g.tpb = std::min(g.nt, 256);
@@ -358,20 +362,20 @@ void pool_launch_u(const T* src, const T* own, const T* ref, const int32_t* tabl
     const long long warps = ceil_div(static_cast<long long>(n_rows), (32 >> lg) * kGroupIters);
     const unsigned blocks = static_cast<unsigned>(ceil_div(warps, 8));
     switch (lg) {
-      case 2: pool_group_kernel<T, VEC, U, OP, 2><<<blocks, 256, 0, st>>>(src, own, ref, table, aux_in, dst, aux_out, n_rows, channels, kv); break;
-      case 3: pool_group_kernel<T, VEC, U, OP, 3><<<blocks, 256, 0, st>>>(src, own, ref, table, aux_in, dst, aux_out, n_rows, channels, kv); break;
-      case 4: pool_group_kernel<T, VEC, U, OP, 4><<<blocks, 256, 0, st>>>(src, own, ref, table, aux_in, dst, aux_out, n_rows, channels, kv); break;
-      default: pool_group_kernel<T, VEC, U, OP, 5><<<blocks, 256, 0, st>>>(src, own, ref, table, aux_in, dst, aux_out, n_rows, channels, kv); break;
+      case 2: pool_group_kernel<T, VEC, U, OP, 2><<<blocks, 256, 0, st>>>(src, own, ref, table, aux_in, dst, aux_out, n_rows, channels, kv, sk, sr); break;
+      case 3: pool_group_kernel<T, VEC, U, OP, 3><<<blocks, 256, 0, st>>>(src, own, ref, table, aux_in, dst, aux_out, n_rows, channels, kv, sk, sr); break;
+      case 4: pool_group_kernel<T, VEC, U, OP, 4><<<blocks, 256, 0, st>>>(src, own, ref, table, aux_in, dst, aux_out, n_rows, channels, kv, sk, sr); break;
+      default: pool_group_kernel<T, VEC, U, OP, 5><<<blocks, 256, 0, st>>>(src, own, ref, table, aux_in, dst, aux_out, n_rows, channels, kv, sk, sr); break;
     }
   } else {
     pool_compact_kernel<T, VEC, U, OP><<<grid, threads, 0, st>>>(src, own, ref, table, aux_in, dst, aux_out,
-                                                                n_rows, channels, kv, g);
+                                                                n_rows, channels, kv, sk, sr, g);
   }
 }
 
 template <typename T, int OP>
 int pool_launch(const void* src_, const void* own_, const void* ref_, const int32_t* table,
-                const int32_t* aux_in, void* dst_, int32_t* aux_out, int64_t n_rows, int channels, int kv,
+                const int32_t* aux_in, void* dst_, int32_t* aux_out, int64_t n_rows, int channels, int kv, int pitch,
                 cudaStream_t st) {
   constexpr int full = 16 / sizeof(T);
   const T* src = static_cast<const T*>(src_);
@@ -379,18 +383,18 @@ int pool_launch(const void* src_, const void* own_, const void* ref_, const int3
   const T* ref = static_cast<const T*>(ref_);
   T* dst = static_cast<T*>(dst_);
   if (vec_for<T>(channels, src_, own_, ref_, dst_) != full) {
-    pool_launch_u<T, 1, 1, OP>(src, own, ref, table, aux_in, dst, aux_out, n_rows, channels, kv, st);
+    pool_launch_u<T, 1, 1, OP>(src, own, ref, table, aux_in, dst, aux_out, n_rows, channels, kv, pitch, st);
   } else {
     // most vectors per thread that still leave a row at least 4 threads (the warp-group kernel)
     const int tpr = channels / full;
     int u = PoolTune<OP>::max_u;
     while (u > 1 && (tpr % u != 0 || tpr / u < 4)) u /= 2;
     if (u == 4)
-      pool_launch_u<T, full, 4, OP>(src, own, ref, table, aux_in, dst, aux_out, n_rows, channels, kv, st);
+      pool_launch_u<T, full, 4, OP>(src, own, ref, table, aux_in, dst, aux_out, n_rows, channels, kv, pitch, st);
     else if (u == 2)
-      pool_launch_u<T, full, 2, OP>(src, own, ref, table, aux_in, dst, aux_out, n_rows, channels, kv, st);
+      pool_launch_u<T, full, 2, OP>(src, own, ref, table, aux_in, dst, aux_out, n_rows, channels, kv, pitch, st);
     else
-      pool_launch_u<T, full, 1, OP>(src, own, ref, table, aux_in, dst, aux_out, n_rows, channels, kv, st);
+      pool_launch_u<T, full, 1, OP>(src, own, ref, table, aux_in, dst, aux_out, n_rows, channels, kv, pitch, st);
   }
   SPC_LAUNCH_OK();
   return SPC_OK;
@@ -420,7 +424,7 @@ extern "C" int spc_maxpool_forward(const void* features, const int32_t* pair_fwd
     return fail(SPC_ERR_INVALID_ARGUMENT, "maxpool_forward: bad arguments");
   if (n_out == 0) return SPC_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  SPC_POOL_DISPATCH(dtype, (pool_launch<T, kMaxFwd>(features, nullptr, nullptr, pair_fwd, nullptr, out, nullptr, n_out, channels, kv, st)));
+  SPC_POOL_DISPATCH(dtype, (pool_launch<T, kMaxFwd>(features, nullptr, nullptr, pair_fwd, nullptr, out, nullptr, n_out, channels, kv, 0, st)));
 }
 
 extern "C" int spc_avgpool_forward(const void* features, const int32_t* pair_fwd, void* out, int32_t* count,
@@ -429,7 +433,7 @@ extern "C" int spc_avgpool_forward(const void* features, const int32_t* pair_fwd
     return fail(SPC_ERR_INVALID_ARGUMENT, "avgpool_forward: bad arguments");
   if (n_out == 0) return SPC_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  SPC_POOL_DISPATCH(dtype, (pool_launch<T, kAvgFwd>(features, nullptr, nullptr, pair_fwd, nullptr, out, count, n_out, channels, kv, st)));
+  SPC_POOL_DISPATCH(dtype, (pool_launch<T, kAvgFwd>(features, nullptr, nullptr, pair_fwd, nullptr, out, count, n_out, channels, kv, 0, st)));
 }
 
 extern "C" int spc_maxpool_backward(const void* features, const void* out_features, const void* grad_out,
@@ -439,7 +443,7 @@ extern "C" int spc_maxpool_backward(const void* features, const void* out_featur
     return fail(SPC_ERR_INVALID_ARGUMENT, "maxpool_backward: bad arguments");
   if (n_in == 0) return SPC_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  SPC_POOL_DISPATCH(dtype, (pool_launch<T, kMaxBwd>(grad_out, features, out_features, pair_bwd, nullptr, din, nullptr, n_in, channels, kv, st)));
+  SPC_POOL_DISPATCH(dtype, (pool_launch<T, kMaxBwd>(grad_out, features, out_features, pair_bwd, nullptr, din, nullptr, n_in, channels, kv, 0, st)));
 }
 
 extern "C" int spc_avgpool_backward(const void* grad_out, const int32_t* pair_bwd, const int32_t* count,
@@ -448,5 +452,21 @@ extern "C" int spc_avgpool_backward(const void* grad_out, const int32_t* pair_bw
     return fail(SPC_ERR_INVALID_ARGUMENT, "avgpool_backward: bad arguments");
   if (n_in == 0) return SPC_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  SPC_POOL_DISPATCH(dtype, (pool_launch<T, kAvgBwd>(grad_out, nullptr, nullptr, pair_bwd, count, din, nullptr, n_in, channels, kv, st)));
+  SPC_POOL_DISPATCH(dtype, (pool_launch<T, kAvgBwd>(grad_out, nullptr, nullptr, pair_bwd, count, din, nullptr, n_in, channels, kv, 0, st)));
+}
+
+extern "C" int spc_pool(int op, const void* src, const void* own, const void* ref, const int32_t* table, int pitch,
+                        const int32_t* aux_in, void* dst, int32_t* aux_out, int64_t n_rows, int channels, int kv,
+                        int dtype, void* stream) {
+  if (!pool_args_ok(src, table, dst, n_rows, channels, kv) || (pitch != 0 && pitch < kv) || op < kMaxFwd || op > kMaxBwd ||
+      (op == kMaxBwd && (!own || !ref)) || (op == kAvgBwd && !aux_in))
+    return fail(SPC_ERR_INVALID_ARGUMENT, "pool: bad arguments");
+  if (n_rows == 0) return SPC_OK;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  switch (op) {
+    case kMaxFwd: SPC_POOL_DISPATCH(dtype, (pool_launch<T, kMaxFwd>(src, nullptr, nullptr, table, nullptr, dst, nullptr, n_rows, channels, kv, pitch, st)));
+    case kAvgFwd: SPC_POOL_DISPATCH(dtype, (pool_launch<T, kAvgFwd>(src, nullptr, nullptr, table, nullptr, dst, aux_out, n_rows, channels, kv, pitch, st)));
+    case kAvgBwd: SPC_POOL_DISPATCH(dtype, (pool_launch<T, kAvgBwd>(src, nullptr, nullptr, table, aux_in, dst, nullptr, n_rows, channels, kv, pitch, st)));
+    default: SPC_POOL_DISPATCH(dtype, (pool_launch<T, kMaxBwd>(src, own, ref, table, nullptr, dst, nullptr, n_rows, channels, kv, pitch, st)));
+  }
 }

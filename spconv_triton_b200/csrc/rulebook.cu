@@ -1282,6 +1282,19 @@ pairs_to_rowmajor_kernel(const int32_t* __restrict__ pairs, int kv, int kvp, lon
   *reinterpret_cast<int4*>(&out[row * kvp + k0]) = make_int4(v[0], v[1], v[2], v[3]);
 }
 
+// 32 x 32 entries through shared memory: both sides are read and written in full rows.
+__global__ void __launch_bounds__(kThreads)
+rowmajor_to_pairs_kernel(const int32_t* __restrict__ rowmajor, int kv, int kvp, long long n, int32_t* __restrict__ pairs) {
+  __shared__ int32_t tile[32][33];
+  const long long row0 = blockIdx.x * 32ll;
+  const int k0 = blockIdx.y * 32;
+  for (int r = threadIdx.y; r < 32; r += 8)
+    if (row0 + r < n && k0 + threadIdx.x < kv) tile[r][threadIdx.x] = rowmajor[(row0 + r) * kvp + k0 + threadIdx.x];
+  __syncthreads();
+  for (int k = threadIdx.y; k < 32; k += 8)
+    if (row0 + threadIdx.x < n && k0 + k < kv) pairs[static_cast<long long>(k0 + k) * n + row0 + threadIdx.x] = tile[threadIdx.x][k];
+}
+
 __global__ void __launch_bounds__(kThreads)
 native_to_tables_kernel(const int32_t* __restrict__ pair_in, const int32_t* __restrict__ pair_out,
                         int kv, long long n_pair, int32_t* __restrict__ pair_fwd, long long n_out,
@@ -1323,6 +1336,7 @@ struct Layout {
   const uint32_t* shared_cells = nullptr;  // the cells of those rows
 };
 // counts and taken of the tile order
+// (one set for each side of a layer)
 constexpr size_t kOrderCountBytes = 2 * ((kTileBuckets * 4 + 255) / 256) * 256;
 
 inline int cell_blocks(int64_t words) { return static_cast<int>(ceil_div(words, kCellBlock)); }
@@ -1474,7 +1488,7 @@ Layout make_layout(const Geo& g, int64_t n_in) {
   L.off_cub = take(L.cub_bytes);
   L.off_native = take(static_cast<size_t>(L.n_blocks_native) * g.kv * 4);
   L.off_order_pairs = take(g.kv <= 32 ? static_cast<size_t>(n_max) * 8 : 0);
-  L.off_order_counts = take(kOrderCountBytes);
+  L.off_order_counts = take(2 * kOrderCountBytes);
   L.off_ibits = take(static_cast<size_t>(L.ibits_words) * 4);
   L.off_iprefix = take(static_cast<size_t>(L.ibits_words) * 4);
   L.off_istarts = take(L.ibits_words ? static_cast<size_t>(cell_blocks(L.ibits_words) + 1) * 4 : 0);
@@ -1635,7 +1649,7 @@ int prepare_impl(const Geo& g, const Layout& L, const int32_t* idx, int64_t n_in
     clear.add(ws + L.off_tout, 0xFF, static_cast<size_t>(L.cap_out) * 8);
     if (K64) clear.add(ws + L.off_tout_vals, 0x7F, static_cast<size_t>(L.cap_out) * 4);
   }
-  clear.add(ws + L.off_order_counts, 0, kOrderCountBytes);
+  clear.add(ws + L.off_order_counts, 0, 2 * kOrderCountBytes);
   int rc = launch_clear(clear, st);
   if (rc != SPC_OK) return rc;
   Table<K64> tin = tin_at<K64>(ws, L);
@@ -1823,30 +1837,36 @@ struct MaskSplits {
   int n = 1, do_sort = 0;
 };
 
-uint32_t* bucket_counts(const Layout& L, char* ws, int64_t n) {
-  return tile_order_needs_buckets(n) ? reinterpret_cast<uint32_t*>(ws + L.off_order_counts) : nullptr;
+// Scratch of the tile order; the input side of a strided layer has keys and counts of its own, so that both
+// sides come out of one pass.
+uint32_t* order_keys(const Layout& L, char* ws, bool input) {
+  return reinterpret_cast<uint32_t*>(ws + (input ? L.off_keys_b : L.off_keys_a));
 }
-int emit_order(const Layout& L, char* ws, int64_t n, int kv, int32_t* order, cudaStream_t st) {
-  uint32_t* counts = reinterpret_cast<uint32_t*>(ws + L.off_order_counts);
-  return tile_order(reinterpret_cast<const uint32_t*>(ws + L.off_keys_a), n, kv, counts, counts + kOrderCountBytes / 8,
+uint32_t* bucket_counts(const Layout& L, char* ws, int64_t n, bool input) {
+  return tile_order_needs_buckets(n) ? reinterpret_cast<uint32_t*>(ws + L.off_order_counts + (input ? kOrderCountBytes : 0)) : nullptr;
+}
+int emit_order(const Layout& L, char* ws, int64_t n, int kv, int32_t* order, bool input, cudaStream_t st) {
+  uint32_t* counts = reinterpret_cast<uint32_t*>(ws + L.off_order_counts + (input ? kOrderCountBytes : 0));
+  return tile_order(order_keys(L, ws, input), n, kv, counts, counts + kOrderCountBytes / 8,
                     reinterpret_cast<uint2*>(ws + L.off_order_pairs), order, st);
 }
 // Keys or words of the rows that a fill kernel owns.
-void ask_fill(const Layout& L, char* ws, int64_t n, const SideTables& t, const MaskSplits& m, FillOut* out) {
+void ask_fill(const Layout& L, char* ws, int64_t n, const SideTables& t, const MaskSplits& m, bool input, FillOut* out) {
   out->cm = t.cm;
   out->rm = t.rm;
   if (t.order != nullptr) {
-    out->keys = reinterpret_cast<uint32_t*>(ws + L.off_keys_a);
-    out->counts = bucket_counts(L, ws, n);
+    out->keys = order_keys(L, ws, input);
+    out->counts = bucket_counts(L, ws, n, input);
   }
   if (t.mask != nullptr) {
     out->words = reinterpret_cast<uint32_t*>(ws + L.off_words);
     out->iota = mask_iota(L, ws, m.words, m.n, m.do_sort);
   }
 }
-int emit_side(const Geo& g, const Layout& L, char* ws, int64_t n, const SideTables& t, const MaskSplits& m, cudaStream_t st) {
+int emit_side(const Geo& g, const Layout& L, char* ws, int64_t n, const SideTables& t, const MaskSplits& m, bool input,
+              cudaStream_t st) {
   if (t.order != nullptr) {
-    const int rc = emit_order(L, ws, n, g.kv, t.order, st);
+    const int rc = emit_order(L, ws, n, g.kv, t.order, input, st);
     if (rc != SPC_OK) return rc;
   }
   return t.mask != nullptr ? emit_masks(L, ws, n, g.kv, m.words, m.n, m.do_sort, t.mask, t.argsort, st) : SPC_OK;
@@ -1856,21 +1876,15 @@ int emit_side(const Geo& g, const Layout& L, char* ws, int64_t n, const SideTabl
 template <int ND, bool K64>
 int backward_impl(const Geo& g, const Layout& L, const int32_t* idx, int64_t n_in, int64_t n_out, char* ws,
                   const SideTables& bwd, const MaskSplits& m, cudaStream_t st) {
-  if (bwd.order != nullptr && tile_order_needs_buckets(n_in)) {  // the counts of the output side's order are still there
-    Clear c;
-    c.add(ws + L.off_order_counts, 0, kOrderCountBytes);
-    const int rc = launch_clear(c, st);
-    if (rc != SPC_OK) return rc;
-  }
   FillOut out{};
-  ask_fill(L, ws, n_in, bwd, m, &out);
+  ask_fill(L, ws, n_in, bwd, m, true, &out);
   const int rc = launch_fill<ND, K64, true>(g, idx, n_in, n_out, tout_at<K64>(ws, L), out, L.mic, st);
-  return rc != SPC_OK ? rc : emit_side(g, L, ws, n_in, bwd, m, st);
+  return rc != SPC_OK ? rc : emit_side(g, L, ws, n_in, bwd, m, true, st);
 }
 
 // Both sides of a strided / transposed layer: clear the output side's tables, one pass over the input rows,
-// one over the output rows.  The input side's keys or words wait for their sort until the output side's is
-// done with the shared scratch, so an ordered or masked input side is a pass of its own.
+// one over the output rows.  The exactly sorted masks of both sides share their scratch, so an input side with
+// masks is a pass of its own.
 template <int ND, bool K64>
 int strided_impl(const Geo& g, const Layout& L, const int32_t* idx, int64_t n_in, int64_t n_out, char* ws,
                  int32_t* out_indices, const SideTables& fwd, const SideTables& bwd, const MaskSplits& m, cudaStream_t st) {
@@ -1892,8 +1906,8 @@ int strided_impl(const Geo& g, const Layout& L, const int32_t* idx, int64_t n_in
   if (c.total != 0) rc = launch_clear(c, st);
   if (rc != SPC_OK) return rc;
   FillOut out{};
-  const bool together = bwd.wanted() && bwd.order == nullptr && bwd.mask == nullptr;
-  if (together) ask_fill(L, ws, n_in, bwd, m, &out);
+  const bool together = bwd.wanted() && bwd.mask == nullptr;
+  if (together) ask_fill(L, ws, n_in, bwd, m, true, &out);
   out.out_cm = fwd.cm;
   out.out_rm = fwd.rm;
   out.out_words = words;
@@ -1903,10 +1917,11 @@ int strided_impl(const Geo& g, const Layout& L, const int32_t* idx, int64_t n_in
   finish_outputs_kernel<ND, K64><<<blocks_for(n_out), kThreads, 0, st>>>(
       g, reinterpret_cast<const key_t*>(ws + L.off_sorted), n_out, out_indices,
       fwd.mask ? mask_iota(L, ws, m.words, m.n, m.do_sort) : nullptr, fwd.order ? words : nullptr,
-      reinterpret_cast<uint32_t*>(ws + L.off_keys_a), bucket_counts(L, ws, n_out));
+      order_keys(L, ws, false), bucket_counts(L, ws, n_out, false));
   SPC_LAUNCH_OK();
-  rc = emit_side(g, L, ws, n_out, fwd, m, st);
-  if (rc != SPC_OK || !bwd.wanted() || together) return rc;
+  rc = emit_side(g, L, ws, n_out, fwd, m, false, st);
+  if (rc != SPC_OK || !bwd.wanted()) return rc;
+  if (together) return emit_side(g, L, ws, n_in, bwd, m, true, st);
   return backward_impl<ND, K64>(g, L, idx, n_in, n_out, ws, bwd, m, st);
 }
 
@@ -1915,11 +1930,11 @@ template <int ND, bool K64>
 int subm_impl(const Geo& g, const Layout& L, const int32_t* idx, int64_t n, char* ws, const SideTables& fwd, int32_t* rev_cm,
               int32_t* rev_rm, const MaskSplits& m, cudaStream_t st) {
   FillOut out{};
-  ask_fill(L, ws, n, fwd, m, &out);
+  ask_fill(L, ws, n, fwd, m, false, &out);
   out.cm_rev = rev_cm;
   out.rm_rev = rev_rm;
   const int rc = launch_fill<ND, K64, false>(g, idx, n, n, tin_at<K64>(ws, L), out, L.mic, st);
-  return rc != SPC_OK ? rc : emit_side(g, L, ws, n, fwd, m, st);
+  return rc != SPC_OK ? rc : emit_side(g, L, ws, n, fwd, m, false, st);
 }
 
 template <int ND, bool K64>
@@ -2184,6 +2199,16 @@ extern "C" int spc_pairs_to_rowmajor(const int32_t* pairs, int kv, int64_t n, in
   const int kvp = (kv + 3) & ~3;
   pairs_to_rowmajor_kernel<<<blocks_for(n * (kvp / 4)), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
       pairs, kv, kvp, n, out);
+  SPC_LAUNCH_OK();
+  return SPC_OK;
+}
+
+extern "C" int spc_rowmajor_to_pairs(const int32_t* rowmajor, int kv, int64_t n, int32_t* pairs, void* stream) {
+  if (!rowmajor || !pairs || kv <= 0 || n < 0) return fail(SPC_ERR_INVALID_ARGUMENT, "rowmajor_to_pairs: bad arguments");
+  if (n == 0) return SPC_OK;
+  const int kvp = (kv + 3) & ~3;
+  const dim3 grid(static_cast<unsigned>(ceil_div(n, 32)), static_cast<unsigned>(ceil_div(kv, 32)));
+  rowmajor_to_pairs_kernel<<<grid, dim3(32, 8), 0, static_cast<cudaStream_t>(stream)>>>(rowmajor, kv, kvp, n, pairs);
   SPC_LAUNCH_OK();
   return SPC_OK;
 }

@@ -59,7 +59,7 @@ tf32_prepare_kernel(const float* __restrict__ src, float* __restrict__ dst, long
 }
 
 // weight [c_out, kv, c_in] -> dst [c_out, kv, m * c_in], or with `transpose` [c_in, kv, m * c_out]
-// (dst[c][k][n] = w[n][k][c]): the reduction index innermost, as the forward-form kernel reads it.
+// (dst[c][k][n] = w[n][k][c]; 2: dst[c][kv - 1 - k][n]): the reduction index innermost, as the forward-form kernel reads it.
 __global__ void __launch_bounds__(256)
 tf32_prepare_weight_kernel(const float* __restrict__ w, float* __restrict__ dst, int c_out, int kv, int c_in,
                            int transpose, int mode) {
@@ -68,6 +68,7 @@ tf32_prepare_weight_kernel(const float* __restrict__ w, float* __restrict__ dst,
   if (i >= total) return;
   const int c = static_cast<int>(i % c_in);
   const int k = static_cast<int>((i / c_in) % kv);
+  const int ko = transpose == 2 ? kv - 1 - k : k;
   const int n = static_cast<int>(i / (static_cast<long long>(c_in) * kv));
   const float x = w[i];
   const float hi = rna_tf32(x);
@@ -75,7 +76,7 @@ tf32_prepare_weight_kernel(const float* __restrict__ w, float* __restrict__ dst,
   const int red = transpose ? c_out : c_in;   // reduction extent of the prepared weight
   const int r = transpose ? n : c;            // this element's reduction index
   const int o = transpose ? c : n;            // and its output-channel index
-  float* row = dst + (static_cast<long long>(o) * kv + k) * m * red;
+  float* row = dst + (static_cast<long long>(o) * kv + ko) * m * red;
   row[r] = hi;
   if (m == 3) {
     const float lo = rna_tf32(x - hi);
