@@ -51,6 +51,27 @@ class IndiceData(_Record):
                  is_subm: bool, algo: ConvAlgo, ksize, stride, dilation, padding, voxel_num: Any = None):
         self._assign(locals())
 
+    # An entry made from a layer's rulebook (``_rb``) has no pair lists until somebody reads them.
+    def _resolved_pairs(self, name):
+        d = self.__dict__
+        thunk = d.get("_pairs_thunk")
+        if thunk is not None:
+            d["_pairs_thunk"] = None
+            pairs, num = thunk()
+            for key, value in (("_indice_pairs", pairs), ("_indice_pair_num", num)):
+                if d.get(key) is None:
+                    d[key] = value
+        return d[name]
+
+    def _set_pairs(self, name, v):
+        self.__dict__["_rb"] = None  # the user's tables count from now on
+        self.__dict__[name] = v
+
+    indice_pairs = property(lambda self: self._resolved_pairs("_indice_pairs"),
+                            lambda self, v: self._set_pairs("_indice_pairs", v))
+    indice_pair_num = property(lambda self: self._resolved_pairs("_indice_pair_num"),
+                               lambda self, v: self._set_pairs("_indice_pair_num", v))
+
 
 class ImplicitGemmIndiceData(_Record):
     """Implicit-gemm rulebook cached under an ``indice_key`` (reference: core.py:79-120)."""
@@ -89,7 +110,12 @@ class ImplicitGemmIndiceData(_Record):
 
     def _set_fwd(self, v):
         self.__dict__["_pair_fwd_thunk"] = None
-        self.__dict__["_pair_fwd"] = v
+        self._set("_pair_fwd", v)
+
+    # A table that the user assigns counts from then on, not the layer's rulebook.
+    def _set(self, name, v):
+        self.__dict__["_rb"] = None
+        self.__dict__[name] = v
 
     pair_fwd = property(_resolved_fwd, _set_fwd)
 
@@ -108,15 +134,34 @@ class ImplicitGemmIndiceData(_Record):
         return d[name]
 
     pair_mask_fwd_splits = property(lambda self: self._resolved_masks("_pair_mask_fwd_splits"),
-                                    lambda self, v: self.__dict__.__setitem__("_pair_mask_fwd_splits", v))
+                                    lambda self, v: self._set("_pair_mask_fwd_splits", v))
     mask_argsort_fwd_splits = property(lambda self: self._resolved_masks("_mask_argsort_fwd_splits"),
-                                       lambda self, v: self.__dict__.__setitem__("_mask_argsort_fwd_splits", v))
+                                       lambda self, v: self._set("_mask_argsort_fwd_splits", v))
     pair_bwd = property(lambda self: self._resolved("_pair_bwd"),
-                        lambda self, v: self.__dict__.__setitem__("_pair_bwd", v))
+                        lambda self, v: self._set("_pair_bwd", v))
     pair_mask_bwd_splits = property(lambda self: self._resolved("_pair_mask_bwd_splits"),
-                                    lambda self, v: self.__dict__.__setitem__("_pair_mask_bwd_splits", v))
+                                    lambda self, v: self._set("_pair_mask_bwd_splits", v))
     mask_argsort_bwd_splits = property(lambda self: self._resolved("_mask_argsort_bwd_splits"),
-                                       lambda self, v: self.__dict__.__setitem__("_mask_argsort_bwd_splits", v))
+                                       lambda self, v: self._set("_mask_argsort_bwd_splits", v))
+
+
+def entry_of_rulebook(layer, rb, tables, indices, spatial_shape, out_spatial_shape):
+    """The ``indice_dict`` entry of a layer's rulebook (``tables``: what it shows, see _impl/host.py)."""
+    native = layer.algo == ConvAlgo.Native
+    cls = IndiceData if native else ImplicitGemmIndiceData
+    data = cls.__new__(cls)
+    d = data.__dict__
+    d.update(out_indices=rb.out_indices, indices=indices, spatial_shape=spatial_shape, out_spatial_shape=out_spatial_shape,
+             is_subm=layer.subm, algo=layer.algo, ksize=layer.kernel_size, stride=layer.stride, dilation=layer.dilation,
+             padding=layer.padding, _rb=rb)
+    if native:
+        d.update(voxel_num=None, _pairs_thunk=tables, _indice_pairs=None, _indice_pair_num=None)
+    else:
+        d.update(masks=[np.array([0xFFFFFFFF], dtype=np.uint32)], in_voxel_num=None, out_voxel_num=None, _late=tables,
+                 _pair_fwd_thunk=tables.forward, _masks_fwd_thunk=tables.masks, _pair_fwd=None, _pair_bwd=None,
+                 _pair_mask_fwd_splits=None, _pair_mask_bwd_splits=None, _mask_argsort_fwd_splits=None,
+                 _mask_argsort_bwd_splits=None)
+    return data
 
 
 def register_implicit_gemm_indice_data(indice_dict, indice_key, res, indices, *, is_subm, spatial_shape,
@@ -198,17 +243,21 @@ class SparseConvTensor(metaclass=SpConvTensorMeta):
         other._planner = self._planner
         return other
 
+    # Siblings share every member; they are made without the constructor (its checks hold already, and three
+    # of them per layer were a tenth of a small layer's host time).
     def replace_feature(self, feature: torch.Tensor):
-        new = SparseConvTensor(feature, self.indices, self.spatial_shape, self.batch_size, self.grid,
-                               self.voxel_num, self.indice_dict)
-        new.benchmark = self.benchmark
-        return self._carry_over(new)
+        if feature.ndim != 2 and not SPCONV_FX_TRACE_MODE:
+            raise AssertionError
+        new = self.shadow_copy()
+        new._features = feature
+        return new
 
     def shadow_copy(self) -> "SparseConvTensor":
         """New object sharing every member with this one."""
-        new = SparseConvTensor(self.features, self.indices, self.spatial_shape, self.batch_size, self.grid,
-                               self.voxel_num, self.indice_dict, self.benchmark)
-        return self._carry_over(new)
+        new = SparseConvTensor.__new__(SparseConvTensor)
+        new.__dict__.update(self.__dict__)
+        new.spatial_shape = list(self.spatial_shape)
+        return new
 
     def select_by_index(self, valid_indices: torch.Tensor):
         # assigning to the read-only property raises, as upstream does
