@@ -9,6 +9,7 @@ and GEMMs underneath run in libspconv_b200.so.
 
 from __future__ import annotations
 
+import functools
 import math
 import time as _time
 
@@ -20,14 +21,24 @@ from torch.nn.parameter import Parameter
 
 from spconv_triton_b200 import SPCONV_VERSION_NUMBERS  # noqa: F401  (re-export)
 from spconv_triton_b200.compat import Activation, tv
+from spconv_triton_b200 import constants
 from spconv_triton_b200.constants import SAVED_WEIGHT_LAYOUT, SPCONV_DEBUG_WEIGHT
 from spconv_triton_b200.core import ConvAlgo
 from spconv_triton_b200.tools import nullcontext  # noqa: F401
 
 from . import functional as Fsp
 from . import ops
+from ._impl import gemm as _gemm
+from ._impl import host as _host
 from ._impl import pairs as _pairs
-from .core import ImplicitGemmIndiceData, IndiceData, SparseConvTensor, expand_nd, register_implicit_gemm_indice_data
+from .core import (
+    ImplicitGemmIndiceData,
+    IndiceData,
+    SparseConvTensor,
+    entry_of_rulebook,
+    expand_nd,
+    register_implicit_gemm_indice_data,
+)
 from .modules import SparseModule
 
 FILTER_HWIO = False
@@ -230,6 +241,11 @@ class SparseConvolutionBase:
             out_tensor.spatial_shape = out_spatial_shape
             return out_tensor
 
+        if channel_scale is None and output_scale is None:
+            out = self._forward_native_host(training, x, weight, bias, add_input, out_spatial_shape, act_type, act_alpha, bn_fold)
+            if out is not None:
+                return out
+
         indice_dict = x.indice_dict.copy()
         features = x.features.contiguous()
         if self.indice_key is not None:
@@ -301,6 +317,91 @@ class SparseConvolutionBase:
         if add_input is not None:
             out_tensor = out_tensor.replace_feature(ops._apply_act_inplace(
                 out_tensor.features + add_input.features, self.act_type, self.act_alpha, self.act_beta))
+        return out_tensor
+
+    # -- the layer on CUDA tensors: rulebook and arithmetic in one native call each --------------------
+
+    def host_plannable(self) -> bool:
+        """Whether the layer's rulebook can be a native one (its tensors permitting)."""
+        return not self.conv1x1 and (self.algo == ConvAlgo.Native or
+                                     (self.algo == ConvAlgo.MaskImplicitGemm and int(np.prod(self.kernel_size)) <= 32))
+
+    def host_rulebook(self, indices, batch_size, spatial_shape, training):
+        """A new native rulebook, or None where the operator functions have to raise."""
+        geo = _host.geometry_of(self, batch_size, spatial_shape)
+        if geo is None or indices.shape[0] == 0:
+            return None
+        # training reads column-major tables for the weight gradient, and layers too narrow for the tensor
+        # cores read them in the forward direction
+        colmajor = training or self.in_channels % 16 != 0 or self.out_channels % 16 != 0
+        return _host.build(self, geo[0], indices, spatial_shape, training and not self.subm, colmajor)
+
+    def host_entry(self, rb, indices, batch_size, spatial_shape, out_spatial_shape, training):
+        if self.algo == ConvAlgo.Native:
+            tables = functools.partial(self._native_pairs, indices, batch_size, list(spatial_shape))
+        else:
+            tables = _host.Tables(rb, training or not self.subm)
+        return entry_of_rulebook(self, rb, tables, indices, spatial_shape, out_spatial_shape)
+
+    def _native_pairs(self, indices, batch_size, spatial_shape):
+        return ops.get_indice_pairs(indices, batch_size, spatial_shape, self.algo, self.kernel_size, self.stride, self.padding,
+                                    self.dilation, self.output_padding, self.subm, self.transposed)[1:]
+
+    def _forward_native_host(self, training, x, weight, bias, add_input, out_spatial_shape, act_type, act_alpha, bn_fold):
+        """The forward pass through the host extension; None where a setting or a cached rulebook needs the
+        operator functions."""
+        features = x.features
+        if (x.benchmark or not self.host_plannable() or not _host.takes(features, x.indices) or not weight.is_cuda
+                or not ops.unreplaced() or act_type.name not in ("None_", "ReLU", "Sigmoid", "LeakyReLU")
+                or weight.dtype not in _host.FLOATS):
+            return None
+        datas = x.find_indice_pair(self.indice_key)
+        entry_type = IndiceData if self.algo == ConvAlgo.Native else ImplicitGemmIndiceData
+        if datas is None and self.inverse:
+            return None
+        if datas is not None and (not isinstance(datas, entry_type) or datas.algo != self.algo or datas.__dict__.get("_rb") is None
+                                  or datas.is_subm is not self.subm or (not self.subm and not self.inverse)):
+            return None  # reused or rejected by the checks of the general path
+        indice_dict = x.indice_dict.copy()
+        if datas is None:
+            planned = x._planner.take_host(self, x) if x._planner is not None else None
+            rb = planned or self.host_rulebook(x.indices, x.batch_size, x.spatial_shape, training)
+            if rb is None:
+                return None
+            if self.indice_key is not None:
+                indice_dict[self.indice_key] = self.host_entry(rb, x.indices, x.batch_size, x.spatial_shape, out_spatial_shape, training)
+            out_indices = rb.out_indices
+        elif self.inverse:
+            self._check_inverse_reuse_valid(x, x.spatial_shape, datas)
+            rb, out_indices, out_spatial_shape = datas._rb, datas.indices, datas.spatial_shape
+        else:
+            self._check_subm_reuse_valid(x, x.spatial_shape, datas)
+            rb, out_indices = datas._rb, datas.out_indices
+        tf32, split_most = bool(constants.SPCONV_ALLOW_TF32), _gemm.FP32_SPLIT_MAX_REDUCTION
+        if training:
+            # a residual input is added inside the kernel's store
+            residual = None
+            if add_input is not None and add_input.features.shape == (out_indices.shape[0], self.out_channels):
+                out_type = torch.float16 if torch.is_autocast_enabled() else features.dtype
+                if add_input.features.dtype == out_type and add_input.features.device == features.device:
+                    residual, add_input = add_input.features, None
+            out_features = _host.ext().conv_train(features, weight, bias, residual, rb, self.inverse, tf32, split_most)
+        else:
+            if add_input is not None and features.dtype != torch.qint8:
+                raise AssertionError("fused residual add only support int8")
+            scale, shift = bn_fold if bn_fold is not None else (None, None)
+            out_features = _host.ext().conv_eval(features, weight, bias, rb, self.inverse, tf32, split_most, scale, shift,
+                                                 ops._act_code(act_type), float(act_alpha))
+        if (not self.subm and not self.inverse and self.record_voxel_count
+                and hasattr(self, _MAX_NUM_VOXELS_DURING_TRAINING)):
+            ops.maximum_value_int_(getattr(self, _MAX_NUM_VOXELS_DURING_TRAINING), rb.n_out)
+        out_tensor = x.shadow_copy()
+        out_tensor._features = out_features
+        out_tensor.indices = out_indices
+        out_tensor.indice_dict = indice_dict
+        out_tensor.spatial_shape = out_spatial_shape
+        if add_input is not None:
+            out_tensor = out_tensor.replace_feature(out_tensor.features + add_input.features)
         return out_tensor
 
     # -- reuse checks ------------------------------------------------------------------------

@@ -256,3 +256,20 @@ def global_pool_rearrange(coords: torch.Tensor, batch_size: int):
     sorted_b = b[order]
     out_indices[sorted_b, torch.arange(n, device=device) - starts[sorted_b]] = order.to(torch.int32)
     return out_indices, counts.to(torch.int32)
+
+
+# The layers run these operators' work natively; a program that has put functions of its own in their place
+# (to count, to record, to compute otherwise) gets them called.
+_LAYER_OPERATORS = {name: globals()[name] for name in (
+    "get_indice_pairs", "get_indice_pairs_implicit_gemm", "implicit_gemm", "implicit_gemm_backward", "indice_conv",
+    "indice_conv_backward", "indice_maxpool_implicit_gemm", "indice_maxpool_implicit_gemm_backward",
+    "indice_avgpool_implicit_gemm", "indice_avgpool_implicit_gemm_backward")}
+
+
+def unreplaced() -> bool:
+    """Whether the operators above are the package's own."""
+    here = globals()
+    for name, fn in _LAYER_OPERATORS.items():
+        if here[name] is not fn:
+            return False
+    return True

@@ -7,12 +7,14 @@ import time as _time
 import numpy as np
 import torch
 
+from spconv_triton_b200 import constants
 from spconv_triton_b200.core import ConvAlgo
 
 from . import functional as Fsp
 from . import ops
+from ._impl import host as _host
 from .conv import _MAX_NUM_VOXELS_DURING_TRAINING
-from .core import IndiceData, SparseConvTensor, expand_nd, register_implicit_gemm_indice_data
+from .core import IndiceData, SparseConvTensor, entry_of_rulebook, expand_nd, register_implicit_gemm_indice_data
 from .modules import SparseModule
 
 CPU_ONLY_BUILD = False
@@ -66,6 +68,29 @@ class _SparsePoolBase(SparseModule):
                 ksize=self.kernel_size, stride=self.stride, dilation=self.dilation, padding=self.padding)
         return res[0], res[2], res[3]
 
+    def _forward_native_host(self, x, average):
+        """The pass through the host extension (rulebook and pooling, one native call each); None where the
+        operator functions are needed."""
+        features = x.features
+        if (self.algo != ConvAlgo.MaskImplicitGemm or x.benchmark or not features.is_cuda or not x.indices.is_cuda
+                or features.dtype not in _host.POOL_FLOATS or x.indices.dtype != torch.int32 or x.indices.shape[0] == 0
+                or not constants.SPCONV_DO_SORT or not ops.unreplaced()):
+            return None
+        if self.indice_key is not None and (self.indice_key in x.indice_dict or int(np.prod(self.kernel_size)) > 32):
+            return None  # rejected, or has masks of several words to show
+        geo = _host.geometry_of(self, x.batch_size, x.spatial_shape)
+        if geo is None:
+            return None
+        # pooling needs no row order; a layer that reuses the rulebook backwards goes without
+        rb = _host.build(self, geo[0], x.indices, x.spatial_shape, torch.is_grad_enabled() and features.requires_grad and not self.subm,
+                         False, order=False)
+        indice_dict = x.indice_dict.copy()
+        if self.indice_key is not None:
+            indice_dict[self.indice_key] = entry_of_rulebook(self, rb, _host.Tables(rb, self.training or not self.subm), x.indices,
+                                                             x.spatial_shape, list(geo[1]))
+        out = _host.ext().pool(features, rb, average)
+        return self._finish(x, x.shadow_copy(), out, rb.out_indices, indice_dict, list(geo[1]))
+
     def _finish(self, x, out_tensor, out_features, outids, indice_dict, out_spatial_shape):
         if not self.subm and self.record_voxel_count and hasattr(self, _MAX_NUM_VOXELS_DURING_TRAINING):
             ops.maximum_value_int_(getattr(self, _MAX_NUM_VOXELS_DURING_TRAINING), outids.shape[0])
@@ -94,6 +119,9 @@ class SparseMaxPool(_SparsePoolBase):
             raise NotImplementedError("int8 is not supported by spconv_triton")
         if not isinstance(x, SparseConvTensor):
             raise AssertionError
+        out = self._forward_native_host(x, False)
+        if out is not None:
+            return out
         features = x.features
         out_spatial_shape = self._out_shape(x.spatial_shape)
         out_tensor = x.shadow_copy()
@@ -158,6 +186,9 @@ class SparseAvgPool(_SparsePoolBase):
             raise NotImplementedError("int8 is not supported by spconv_triton")
         if not isinstance(x, SparseConvTensor):
             raise AssertionError
+        out = self._forward_native_host(x, True)
+        if out is not None:
+            return out
         out_spatial_shape = self._out_shape(x.spatial_shape)
         out_tensor = x.shadow_copy()
         indice_dict = x.indice_dict.copy()

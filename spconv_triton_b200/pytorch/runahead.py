@@ -30,6 +30,7 @@ from spconv_triton_b200.core import ConvAlgo
 
 from .. import constants
 from . import ops
+from ._impl import host as _host
 from ._impl import pairs as _pairs
 from .core import ImplicitGemmIndiceData, SparseConvTensor, register_implicit_gemm_indice_data
 
@@ -96,6 +97,7 @@ class RulebookPlanner:
         self.keys = dict(x.indice_dict)
         self.allocator = x.thrust_allocator
         self.timer = x._timer
+        self.host = _host.takes(x.features, x.indices) and ops.unreplaced()
         self.main = torch.cuda.current_stream(device)
         self.side = _side_stream(device, 0)
         # input-side tables of strided layers: needed by inverse layers and the backward
@@ -138,6 +140,18 @@ class RulebookPlanner:
             self.indices, self.spatial_shape = datas.out_indices, out_shape
             return True
         src = self.indices
+        if self.host and conv.host_plannable():
+            with torch.cuda.stream(self.side):
+                rb = conv.host_rulebook(src, self.batch_size, self.spatial_shape, conv.training)
+                if rb is None:
+                    return False
+                event = torch.cuda.Event()
+                event.record(self.side)
+            self.ready[id(conv)] = (rb, event, src, list(self.spatial_shape))
+            if conv.indice_key is not None:
+                self.keys[conv.indice_key] = conv.host_entry(rb, src, self.batch_size, self.spatial_shape, out_shape, conv.training)
+            self.indices, self.spatial_shape = rb.out_indices, out_shape
+            return True
         # training: the input-side tables go to the third stream; inference: they stay pending
         with torch.cuda.stream(self.side), _pairs.deferred_backward(self.late if conv.training else "late"):
             res = ops.get_indice_pairs_implicit_gemm(
@@ -160,9 +174,10 @@ class RulebookPlanner:
     def take(self, conv, x: SparseConvTensor):
         """The planned rulebook of ``conv`` if it was made from exactly ``x``'s
         indices; the caller's stream is made to wait for it."""
-        entry = self.ready.pop(id(conv), None)
-        if entry is None:
-            return None
+        entry = self.ready.get(id(conv))
+        if entry is None or not isinstance(entry[0], tuple):
+            return None  # (a native rulebook: take_host)
+        del self.ready[id(conv)]
         res, event, src, shape = entry
         if src is not x.indices or shape != list(x.spatial_shape) or x.batch_size != self.batch_size:
             self.pos = len(self.queue)  # the data flow left the plan
@@ -174,6 +189,20 @@ class RulebookPlanner:
                 t.record_stream(main)
         return res
 
+
+    def take_host(self, conv, x: SparseConvTensor):
+        """The same for a native rulebook."""
+        entry = self.ready.get(id(conv))
+        if entry is None or isinstance(entry[0], tuple):
+            return None
+        del self.ready[id(conv)]
+        rb, event, src, shape = entry
+        if src is not x.indices or shape != list(x.spatial_shape) or x.batch_size != self.batch_size:
+            self.pos = len(self.queue)  # the data flow left the plan
+            return None
+        torch.cuda.current_stream(x.indices.device).wait_event(event)
+        _host.ext().record_stream(rb, x.indices)
+        return rb
 
     def join_late(self) -> None:
         """Makes the caller's stream wait for every input-side table built so far."""

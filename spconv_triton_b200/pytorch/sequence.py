@@ -31,6 +31,7 @@ from spconv_triton_b200 import _lib, constants
 from spconv_triton_b200.core import ConvAlgo
 
 from ._impl import gemm as _gemm
+from ._impl.host import exact_masks as _exact_masks
 from ._impl import pairs as _pairs
 from .core import ImplicitGemmIndiceData, SparseConvTensor
 
@@ -283,18 +284,6 @@ def _column_major(rowmajor, kv, late, table=None):
     if late is not None:
         table._spc_late = late
     return table
-
-
-def _exact_masks(rowmajor, kv):
-    """``pair_mask_fwd_splits`` / ``mask_argsort_fwd_splits`` as the rulebook generator emits them (one
-    split): the rows' mask words sorted ascending, stable, and their argsort.  The pass itself orders
-    the rows by a different key (rows that share kernel offsets end up in the same GEMM tile), so
-    these two are made from the row-major table when somebody reads them."""
-    weights = torch.ones(kv, dtype=torch.int64, device=rowmajor.device) << torch.arange(kv, device=rowmajor.device)
-    words = ((rowmajor[:, :kv] >= 0).to(torch.int64) * weights).sum(1)
-    vals, args = torch.sort(words, stable=True)
-    vals = torch.where(vals >= 2 ** 31, vals - 2 ** 32, vals)  # the words are unsigned, the tensor is int32
-    return [vals.to(torch.int32).reshape(-1, 1)], [args.to(torch.int32)]
 
 
 def _wrap(plan, x, indices, arena, dev, keep):
