@@ -232,12 +232,28 @@ int spc_native_to_tables(const int32_t* pair, int kv, int64_t n_pair, int invers
  *   reference's bit for bit.  *num_voxels_host receives the number of voxels
  *   written (the call synchronises the stream once to read it, where the
  *   reference reads uniq.numel()).  Grids of 2^32 cells or more are rejected. */
-size_t spc_voxelize_workspace_bytes(int64_t n_points, int64_t max_voxels);
+size_t spc_voxelize_workspace_bytes(int64_t n_points, int64_t max_voxels, int max_points);
 int spc_voxelize(const float* points, int64_t n_points, int point_stride, int ndim, int num_features,
                  const float* cmin, const float* vsize, const int32_t* grid_xyz, int64_t max_voxels,
                  int max_points, int clear_voxels, int empty_mean, void* workspace,
                  size_t workspace_bytes, float* voxels, int32_t* indices, int32_t* num_per_voxel,
                  int64_t* pc_voxel_id, int64_t* num_voxels_host, void* stream);
+
+/* spc_voxelize in two halves, for callers that return copies of the filled rows: the
+ * first numbers the voxels (indices, num_per_voxel, pc_voxel_id) and tells the host how
+ * many there are; the second writes the voxel buffer and, in the same pass, the copies
+ * voxels_out [num_voxels, max_points, num_features], indices_out and num_out (may be
+ * NULL).  `sorted` is what the first said; the workspace is the same, untouched. */
+int spc_voxelize_number(const float* points, int64_t n_points, int point_stride, int ndim, int num_features,
+                        const float* cmin, const float* vsize, const int32_t* grid_xyz, int64_t max_voxels,
+                        int max_points, void* workspace, size_t workspace_bytes, int32_t* indices,
+                        int32_t* num_per_voxel, int64_t* pc_voxel_id, int64_t* num_voxels_host, int* sorted,
+                        void* stream);
+int spc_voxelize_store(const float* points, int64_t n_points, int point_stride, int ndim, int num_features,
+                       int64_t max_voxels, int max_points, int clear_voxels, int empty_mean, void* workspace,
+                       size_t workspace_bytes, int64_t num_voxels, int sorted, const int32_t* indices,
+                       const int32_t* num_per_voxel, const int64_t* pc_voxel_id, float* voxels, float* voxels_out,
+                       int32_t* indices_out, int32_t* num_out, void* stream);
 
 /* ---- sparse -> dense (the step after the backbone) ----------------------- */
 

@@ -100,7 +100,10 @@ _PROTOTYPES = {
     "spc_coords_to_keys": (c_int, [_P, c_int64, c_int, POINTER(c_int64), c_int, _P, _P]),
     "spc_rows_scatter_add": (c_int, [_P, _P, c_int64, c_int, c_int, c_int64, _P, _P, c_int, _P, _P]),
     "spc_rows_gather": (c_int, [_P, _P, c_int64, c_int, c_int, c_int64, _P, _P]),
-    "spc_voxelize_workspace_bytes": (c_size_t, [c_int64, c_int64]),
+    "spc_voxelize_workspace_bytes": (c_size_t, [c_int64, c_int64, c_int]),
+    "spc_voxelize_number": (c_int, [_P, c_int64, c_int, c_int, c_int, _P, _P, _P, c_int64, c_int, _P, c_size_t, _P, _P, _P,
+                                    POINTER(c_int64), POINTER(c_int), _P]),
+    "spc_voxelize_store": (c_int, [_P, c_int64, c_int, c_int, c_int, c_int64, c_int, c_int, c_int, _P, c_size_t, c_int64, c_int] + [_P] * 8),
     "spc_voxelize": (c_int, [_P, c_int64, c_int, c_int, c_int, POINTER(ctypes.c_float), POINTER(ctypes.c_float),
                              POINTER(ctypes.c_int32), c_int64, c_int, c_int, c_int, _P, c_size_t, _P, _P, _P, _P,
                              POINTER(c_int64), _P]),

@@ -520,6 +520,48 @@ Tensor pool(const Tensor& features, const Book& rb, bool average) {
   return out;
 }
 
+// ---- voxelisation ----------------------------------------------------------------------------------------------------
+
+// (voxels, indices, num_per_voxel of the voxels found, pc_voxel_id); the persistent buffers hold the same.
+std::tuple<Tensor, Tensor, Tensor, Tensor> voxelize(const Tensor& points, const Tensor& voxels, const Tensor& indices, const Tensor& num,
+                                                    const std::vector<float>& cmin, const std::vector<float>& vsize,
+                                                    const std::vector<int32_t>& grid, bool clear, bool empty_mean) {
+  pybind11::gil_scoped_release release;
+  at::NoGradGuard no_grad;
+  c10::cuda::CUDAGuard guard(points.device());
+  const Tensor pc = points.contiguous();
+  const int64_t n = pc.size(0), most = voxels.size(0);
+  const int nd = static_cast<int>(cmin.size()), slots = static_cast<int>(voxels.size(1)), f = static_cast<int>(voxels.size(2));
+  const int stride = static_cast<int>(pc.size(1));
+  const size_t bytes = spc_voxelize_workspace_bytes(n, most, slots);
+  if (bytes == 0) throw Failure(SPC_ERR_SIZE_LIMIT, "voxelize: sizes out of range");
+  Tensor id = at::empty({n}, pc.options().dtype(at::kLong)), ws = at::empty({static_cast<int64_t>(bytes)}, pc.options().dtype(at::kByte));
+  void* st = stream_of(pc);
+  int64_t found = 0;
+  int sorted = 0;
+  float* at_points = n ? pc.data_ptr<float>() : nullptr;
+  int64_t* at_id = n ? id.data_ptr<int64_t>() : nullptr;
+  check(spc_voxelize_number(at_points, n, stride, nd, f, cmin.data(), vsize.data(), grid.data(), most, slots, ws.data_ptr(), bytes,
+                            ints(indices), ints(num), at_id, &found, &sorted, st));
+  // without the clear the copy shows what the slots held before
+  const bool together = clear;
+  Tensor v, i, c;
+  if (together) {
+    v = at::empty({found, slots, f}, voxels.options());
+    i = at::empty({found, nd}, indices.options());
+    c = at::empty({found}, num.options());
+  }
+  check(spc_voxelize_store(at_points, n, stride, nd, f, most, slots, clear, empty_mean, ws.data_ptr(), bytes, found, sorted, ints(indices),
+                           ints(num), at_id, voxels.data_ptr<float>(), together ? v.data_ptr<float>() : nullptr,
+                           together ? ints(i) : nullptr, together ? ints(c) : nullptr, st));
+  if (!together) {
+    v = voxels.narrow(0, 0, found).clone();
+    i = indices.narrow(0, 0, found).clone();
+    c = num.narrow(0, 0, found).clone();
+  }
+  return {v, i, c, id};
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_host, m) {
@@ -552,4 +594,5 @@ PYBIND11_MODULE(_host, m) {
   m.def("conv_train", &conv_train);
   m.def("conv_eval", &conv_eval);
   m.def("pool", &pool);
+  m.def("voxelize", &voxelize);
 }

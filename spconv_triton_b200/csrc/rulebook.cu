@@ -1564,61 +1564,6 @@ int launch_clear(const Clear& c, cudaStream_t st) {
   return SPC_OK;
 }
 
-// A few page-locked words per host thread and device that kernels write and the host reads after
-// synchronising (host memory: the library still allocates no device memory).
-// One per host thread and device, with the ticket of the next message.
-int host_mailbox(volatile int** out, int* ticket) {
-  static thread_local int* boxes[kMaxDevices] = {nullptr};
-  static thread_local int tickets[kMaxDevices] = {0};
-  const int dev = current_device_slot();
-  if (dev < 0) return fail(SPC_ERR_CUDA, "rulebook: no current device");
-  if (boxes[dev] == nullptr) {
-    void* p = nullptr;
-    SPC_CUDA_OK(cudaHostAlloc(&p, 64, cudaHostAllocPortable | cudaHostAllocMapped));
-    boxes[dev] = static_cast<int*>(p);
-    boxes[dev][0] = 0;
-  }
-  *out = boxes[dev];
-  tickets[dev] = (tickets[dev] + 1) & 0x7fffffff;
-  if (tickets[dev] == 0) tickets[dev] = 1;
-  *ticket = tickets[dev];
-  return SPC_OK;
-}
-
-// How the host waits for a count: it spins on the page-locked ticket that the publishing kernel writes last,
-// which is the fastest wake-up (the count is there before the stream has drained and without the driver's
-// completion signal) but needs an idle core per pass in flight; with SPC_HOST_WAIT=block in the
-// environment (read once) the thread sleeps on a blocking event instead, for processes that keep several
-// passes in flight on few cores (one process per GPU, eight GPUs, three host threads each).  A stream that
-// has drained, or failed, without the ticket ends the spin.  One event per host thread and device.
-int wait_for_ticket(volatile int* box, int ticket, cudaStream_t st) {
-  static const bool block = [] {
-    const char* v = std::getenv("SPC_HOST_WAIT");
-    return v != nullptr && std::strcmp(v, "block") == 0;
-  }();
-  if (!block) {
-    for (unsigned spin = 1; box[0] != ticket; ++spin) {
-      __builtin_ia32_pause();
-      if ((spin & 0xfffu) != 0) continue;
-      const cudaError_t e = cudaStreamQuery(st);
-      if (e == cudaErrorNotReady) continue;
-      SPC_CUDA_OK(e);
-      if (box[0] != ticket) return fail(SPC_ERR_CUDA, "rulebook: the output count did not arrive");
-    }
-    std::atomic_thread_fence(std::memory_order_acquire);
-    return SPC_OK;
-  }
-  static thread_local cudaEvent_t events[kMaxDevices] = {nullptr};
-  const int dev = current_device_slot();
-  if (dev < 0) return fail(SPC_ERR_CUDA, "rulebook: no current device");
-  if (events[dev] == nullptr)
-    SPC_CUDA_OK(cudaEventCreateWithFlags(&events[dev], cudaEventBlockingSync | cudaEventDisableTiming));
-  SPC_CUDA_OK(cudaEventRecord(events[dev], st));
-  SPC_CUDA_OK(cudaEventSynchronize(events[dev]));
-  if (box[0] != ticket) return fail(SPC_ERR_CUDA, "rulebook: the output count did not arrive");
-  return SPC_OK;
-}
-
 inline unsigned blocks_for(int64_t n) { return static_cast<unsigned>(ceil_div(std::max<int64_t>(n, 1), kThreads)); }
 
 // ------------------------------------------------------------------------
@@ -2005,6 +1950,61 @@ void adopt_producer_bits(const Geo& g, Layout* L, const RulebookProducer* produc
 }
 
 }  // namespace
+
+// A few page-locked words per host thread and device that kernels write and the host reads after
+// synchronising (host memory: the library still allocates no device memory).
+// One per host thread and device, with the ticket of the next message.
+int host_mailbox(volatile int** out, int* ticket) {
+  static thread_local int* boxes[kMaxDevices] = {nullptr};
+  static thread_local int tickets[kMaxDevices] = {0};
+  const int dev = current_device_slot();
+  if (dev < 0) return fail(SPC_ERR_CUDA, "rulebook: no current device");
+  if (boxes[dev] == nullptr) {
+    void* p = nullptr;
+    SPC_CUDA_OK(cudaHostAlloc(&p, 64, cudaHostAllocPortable | cudaHostAllocMapped));
+    boxes[dev] = static_cast<int*>(p);
+    boxes[dev][0] = 0;
+  }
+  *out = boxes[dev];
+  tickets[dev] = (tickets[dev] + 1) & 0x7fffffff;
+  if (tickets[dev] == 0) tickets[dev] = 1;
+  *ticket = tickets[dev];
+  return SPC_OK;
+}
+
+// How the host waits for a count: it spins on the page-locked ticket that the publishing kernel writes last,
+// which is the fastest wake-up (the count is there before the stream has drained and without the driver's
+// completion signal) but needs an idle core per pass in flight; with SPC_HOST_WAIT=block in the
+// environment (read once) the thread sleeps on a blocking event instead, for processes that keep several
+// passes in flight on few cores (one process per GPU, eight GPUs, three host threads each).  A stream that
+// has drained, or failed, without the ticket ends the spin.  One event per host thread and device.
+int wait_for_ticket(volatile int* box, int ticket, cudaStream_t st) {
+  static const bool block = [] {
+    const char* v = std::getenv("SPC_HOST_WAIT");
+    return v != nullptr && std::strcmp(v, "block") == 0;
+  }();
+  if (!block) {
+    for (unsigned spin = 1; box[0] != ticket; ++spin) {
+      __builtin_ia32_pause();
+      if ((spin & 0xfffu) != 0) continue;
+      const cudaError_t e = cudaStreamQuery(st);
+      if (e == cudaErrorNotReady) continue;
+      SPC_CUDA_OK(e);
+      if (box[0] != ticket) return fail(SPC_ERR_CUDA, "rulebook: the output count did not arrive");
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
+    return SPC_OK;
+  }
+  static thread_local cudaEvent_t events[kMaxDevices] = {nullptr};
+  const int dev = current_device_slot();
+  if (dev < 0) return fail(SPC_ERR_CUDA, "rulebook: no current device");
+  if (events[dev] == nullptr)
+    SPC_CUDA_OK(cudaEventCreateWithFlags(&events[dev], cudaEventBlockingSync | cudaEventDisableTiming));
+  SPC_CUDA_OK(cudaEventRecord(events[dev], st));
+  SPC_CUDA_OK(cudaEventSynchronize(events[dev]));
+  if (box[0] != ticket) return fail(SPC_ERR_CUDA, "rulebook: the output count did not arrive");
+  return SPC_OK;
+}
 
 int rulebook_prepare_chained(const spc_geometry* sg, const int32_t* indices, int64_t n_in, void* workspace,
                              size_t workspace_bytes, int64_t* n_out_host, const RulebookProducer* producer,

@@ -42,4 +42,9 @@ int rulebook_tables_chained(const spc_geometry* g, const int32_t* indices, int64
                             size_t workspace_bytes, const RulebookTables& tables, const RulebookProducer* producer,
                             cudaStream_t stream);
 
+// Numbers that the host needs during a call: kernels write words 1.. of the box and the ticket to word 0 last
+// (__threadfence_system between); the wait ends when the ticket is there.
+int host_mailbox(volatile int** out, int* ticket);
+int wait_for_ticket(volatile int* box, int ticket, cudaStream_t st);
+
 }  // namespace spc

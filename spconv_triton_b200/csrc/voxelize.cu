@@ -14,26 +14,29 @@
 //     points (utils.py:146-153).
 // The result is deterministic and equal to the reference's, bit for bit.
 //
-// How it is computed here (no global sort of the points by voxel key):
+// How it is computed here (no sort):
 //   1. quantize_insert: key per point; a hash table keeps, per key, the lowest
-//      point index (one packed 64-bit atomicMin: key << 32 | index);
-//   2. mark_first: a point is "first" when the table returns its own index;
-//      an exclusive prefix sum over these flags IS the voxel number of each
-//      first point, because voxel order = order of first points;
-//   3. the host reads the number of voxels (the reference reads uniq.numel() too);
-//   4. assign: every point looks up its voxel's number, counts itself in and
-//      becomes a (voxel number, point index) pair; first points write the
-//      voxel coordinates;
-//   5. a stable radix sort of the pairs by voxel number keeps arrival order
-//      inside a voxel; position - (start of the voxel's segment) is the slot;
-//   6. scatter copies the stored points; fill_mean pads when asked.
-// HBM-bound; algorithmic bytes per point: 4*F read + 4*F written (stored
-// points) + 8 (voxel id) + the clear of the voxel buffer when requested.
+//      point index (one packed 64-bit atomicMin: key << 32 | index) and a count
+//      that also gives the point a place among its voxel's points, in any order;
+//   2. a point is "first" when the table returns its own index; the number of
+//      first points before it IS its voxel's number.  count_first adds them up per
+//      block and hands the total to the host, number_voxels numbers them and
+//      reserves room for each voxel's points in one list;
+//   3. place: every point goes to its place in its voxel's stretch of the list;
+//   4. rank: a point's slot is the number of lower indices in that stretch (a few
+//      points; voxels of more than 256 points take a radix sort instead);
+//   5. emit: the voxel buffer and the caller's copy of it are written row by row,
+//      points and zeros alike, so that nothing is cleared or copied first.
+// HBM-bound; bytes per point: 4*F read + 4*F written (stored points) + 8 (voxel id)
+// + the rows of the voxel buffer.  1.2 M points: the sort (three passes, a scan, nine
+// memsets) and the three copies were 110 of 215 us of device time.
 #include <cub/cub.cuh>
 
 #include <algorithm>
+#include <atomic>
 
 #include "common.cuh"
+#include "rulebook_internal.cuh"
 
 namespace spc {
 namespace {
@@ -62,9 +65,21 @@ __device__ __forceinline__ uint32_t vox_mix(uint32_t h) {
 inline unsigned vox_blocks(int64_t n) { return static_cast<unsigned>(ceil_div(std::max<int64_t>(n, 1), kVoxThreads)); }
 
 __global__ void __launch_bounds__(kVoxThreads)
+vox_clear_kernel(uint4* __restrict__ status, uint4* __restrict__ slots, long long n_slots16, uint4* __restrict__ counts,
+                 long long n_counts16) {
+  const long long stride = static_cast<long long>(gridDim.x) * kVoxThreads, t = blockIdx.x * static_cast<long long>(kVoxThreads) + threadIdx.x;
+  if (t < 16) status[t] = make_uint4(0u, 0u, 0u, 0u);
+  for (long long i = t; i < n_slots16; i += stride) slots[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+  for (long long i = t; i < n_counts16; i += stride) counts[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+enum VoxStatus { kVoxError = 0, kVoxTotal = 1, kVoxMost = 2, kVoxTicket = 3, kVoxCursor = 4 };
+
+__global__ void __launch_bounds__(kVoxThreads)
 quantize_insert_kernel(const __grid_constant__ VoxGeo g, const float* __restrict__ points, long long n,
                        int point_stride, unsigned long long* __restrict__ slots, uint32_t cap_mask,
-                       uint32_t* __restrict__ keys, int* __restrict__ status) {
+                       uint32_t* __restrict__ counts, uint32_t* __restrict__ slot_of, uint32_t* __restrict__ place,
+                       int* __restrict__ status) {
   const long long i = blockIdx.x * static_cast<long long>(kVoxThreads) + threadIdx.x;
   if (i >= n) return;
   const float* p = points + i * point_stride;
@@ -79,105 +94,239 @@ quantize_insert_kernel(const __grid_constant__ VoxGeo g, const float* __restrict
     }
     key = key * static_cast<uint32_t>(g.grid[d]) + static_cast<uint32_t>(q);
   }
-  if (!in_range) {
-    keys[i] = kNoKey;
-    return;
-  }
-  keys[i] = key;
+  slot_of[i] = kNoKey;
+  if (!in_range) return;
   const unsigned long long packed = (static_cast<unsigned long long>(key) << 32) | static_cast<uint32_t>(i);
   uint32_t s = vox_mix(key) & cap_mask;
   for (uint32_t probe = 0; probe <= cap_mask; ++probe) {
     const unsigned long long old = atomicCAS(&slots[s], kVoxEmpty, packed);
-    if (old == kVoxEmpty) return;
-    if (static_cast<uint32_t>(old >> 32) == key) {
-      atomicMin(&slots[s], packed);
+    if (old == kVoxEmpty || static_cast<uint32_t>(old >> 32) == key) {
+      if (old != kVoxEmpty) atomicMin(&slots[s], packed);
+      slot_of[i] = s;
+      place[i] = atomicAdd(&counts[s], 1u);
       return;
     }
     s = (s + 1) & cap_mask;
   }
-  atomicExch(status, SPC_ERR_HASH_TABLE_FULL);
+  atomicExch(&status[kVoxError], SPC_ERR_HASH_TABLE_FULL);
 }
 
-__device__ __forceinline__ int vox_find(const unsigned long long* __restrict__ slots, uint32_t cap_mask, uint32_t key) {
-  uint32_t s = vox_mix(key) & cap_mask;
-  for (uint32_t probe = 0; probe <= cap_mask; ++probe) {
-    const unsigned long long v = slots[s];
-    if (v == kVoxEmpty) return -1;
-    if (static_cast<uint32_t>(v >> 32) == key) return static_cast<int>(v & 0xffffffffu);
-    s = (s + 1) & cap_mask;
+constexpr int kVoxBlock = 2048;  // points a block counts and numbers
+constexpr int kVoxEach = kVoxBlock / kVoxThreads;
+
+__device__ __forceinline__ uint32_t vox_block_sum(uint32_t v, uint32_t* warp_sums, uint32_t* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t incl = v;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += t;
   }
-  return -1;
-}
-
-// first[i] = index of the first point of i's voxel (or -1); flag[i] = 1 when that is i itself.
-__global__ void __launch_bounds__(kVoxThreads)
-mark_first_kernel(const uint32_t* __restrict__ keys, long long n, const unsigned long long* __restrict__ slots,
-                  uint32_t cap_mask, int* __restrict__ first, int* __restrict__ flag) {
-  const long long i = blockIdx.x * static_cast<long long>(kVoxThreads) + threadIdx.x;
-  if (i >= n) return;
-  const uint32_t key = keys[i];
-  const int f = key == kNoKey ? -1 : vox_find(slots, cap_mask, key);
-  first[i] = f;
-  flag[i] = (f == static_cast<int>(i)) ? 1 : 0;
-}
-
-// status[1] = number of voxels found (rank of the last point + its flag): one word for the host to read.
-__global__ void total_kernel(const int* __restrict__ rank, const int* __restrict__ flag, long long n, int* __restrict__ status) {
-  status[1] = rank[n - 1] + flag[n - 1];
-}
-
-__global__ void __launch_bounds__(kVoxThreads)
-assign_kernel(const __grid_constant__ VoxGeo g, const uint32_t* __restrict__ keys, const int* __restrict__ first,
-              const int* __restrict__ rank, long long n, long long num_voxels, int* __restrict__ counts,
-              uint32_t* __restrict__ sort_keys, int* __restrict__ sort_vals, long long* __restrict__ pc_voxel_id,
-              int32_t* __restrict__ indices) {
-  const long long i = blockIdx.x * static_cast<long long>(kVoxThreads) + threadIdx.x;
-  if (i >= n) return;
-  const int f = first[i];
-  long long vid = -1;
-  if (f >= 0) {
-    vid = rank[f];
-    if (vid >= num_voxels) vid = -1;  // beyond the voxel cap
+  __syncthreads();
+  if (lane == 31) warp_sums[warp] = incl;
+  __syncthreads();
+  uint32_t before = 0, all = 0;
+#pragma unroll
+  for (int w = 0; w < kVoxThreads / 32; ++w) {
+    if (w < warp) before += warp_sums[w];
+    all += warp_sums[w];
   }
-  pc_voxel_id[i] = vid;
-  sort_keys[i] = vid >= 0 ? static_cast<uint32_t>(vid) : static_cast<uint32_t>(num_voxels);  // dropped: behind every voxel
-  sort_vals[i] = static_cast<int>(i);
-  if (vid < 0) return;
-  atomicAdd(&counts[vid], 1);
-  if (f == static_cast<int>(i)) {
-    // the voxel's coordinates, reversed to (z, y, x)
-    uint32_t rem = keys[i];
-    for (int d = g.ndim - 1; d >= 0; --d) {
-      const uint32_t gd = static_cast<uint32_t>(g.grid[d]);
-      indices[vid * g.ndim + (g.ndim - 1 - d)] = static_cast<int32_t>(rem % gd);
-      rem /= gd;
+  *total = all;
+  return before + incl - v;  // exclusive
+}
+
+// First points per block; the last block to finish turns the sums into starts and hands the number of voxels
+// and the largest count of points in one to the host.
+__global__ void __launch_bounds__(kVoxThreads)
+count_first_kernel(const uint32_t* __restrict__ slot_of, long long n, const unsigned long long* __restrict__ slots,
+                   const uint32_t* __restrict__ counts, uint32_t* __restrict__ starts, int* __restrict__ status,
+                   volatile int* host_box, int ticket) {
+  __shared__ uint32_t warp_sums[kVoxThreads / 32];
+  __shared__ int last;
+  const long long base = blockIdx.x * static_cast<long long>(kVoxBlock);
+  uint32_t mine = 0, most = 0;
+#pragma unroll
+  for (int e = 0; e < kVoxEach; ++e) {
+    const long long i = base + e * kVoxThreads + threadIdx.x;
+    const uint32_t s = i < n ? slot_of[i] : kNoKey;
+    if (s == kNoKey || static_cast<uint32_t>(slots[s]) != static_cast<uint32_t>(i)) continue;
+    ++mine;
+    most = max(most, counts[s]);
+  }
+  most = __reduce_max_sync(0xffffffffu, most);
+  if ((threadIdx.x & 31) == 0 && most > 0) atomicMax(&status[kVoxMost], static_cast<int>(most));
+  uint32_t total;
+  vox_block_sum(mine, warp_sums, &total);
+  if (threadIdx.x == 0) {
+    starts[blockIdx.x] = total;
+    __threadfence();
+    last = atomicAdd(&status[kVoxTicket], 1) == static_cast<int>(gridDim.x) - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  volatile uint32_t* st = starts;
+  uint32_t carry = 0;
+  for (int b0 = 0; b0 < static_cast<int>(gridDim.x); b0 += kVoxThreads) {
+    const int b = b0 + threadIdx.x;
+    const uint32_t v = b < static_cast<int>(gridDim.x) ? st[b] : 0u;
+    uint32_t all;
+    const uint32_t before = vox_block_sum(v, warp_sums, &all);
+    if (b < static_cast<int>(gridDim.x)) st[b] = carry + before;
+    carry += all;
+  }
+  if (threadIdx.x == 0) {
+    status[kVoxTotal] = static_cast<int>(carry);
+    host_box[1] = *reinterpret_cast<volatile int*>(&status[kVoxError]);
+    host_box[2] = static_cast<int>(carry);
+    host_box[3] = *reinterpret_cast<volatile int*>(&status[kVoxMost]);
+    __threadfence_system();
+    host_box[0] = ticket;
+  }
+}
+
+// Voxel number of every slot that has one below the cap (else -1), its stretch of the list, its coordinates
+// and its count.
+__global__ void __launch_bounds__(kVoxThreads)
+number_voxels_kernel(const __grid_constant__ VoxGeo g, const uint32_t* __restrict__ slot_of, long long n,
+                     const unsigned long long* __restrict__ slots, const uint32_t* __restrict__ counts,
+                     const uint32_t* __restrict__ starts, long long max_voxels, int max_points, int* __restrict__ voxel_of,
+                     uint32_t* __restrict__ seg, int* __restrict__ status, int32_t* __restrict__ indices,
+                     int32_t* __restrict__ num_per_voxel) {
+  __shared__ uint32_t warp_sums[kVoxThreads / 32];
+  __shared__ uint32_t room;
+  // a thread numbers consecutive points, so that the numbers of a block follow the order of its points
+  const long long base = blockIdx.x * static_cast<long long>(kVoxBlock) + threadIdx.x * kVoxEach;
+  uint32_t slot[kVoxEach], mine = 0, points = 0;
+#pragma unroll
+  for (int e = 0; e < kVoxEach; ++e) {
+    const long long i = base + e;
+    slot[e] = i < n ? slot_of[i] : kNoKey;
+    if (slot[e] != kNoKey && static_cast<uint32_t>(slots[slot[e]]) != static_cast<uint32_t>(i)) slot[e] = kNoKey;
+    if (slot[e] == kNoKey) continue;
+    ++mine;
+    points += counts[slot[e]];
+  }
+  uint32_t total, all_points;
+  uint32_t vid = starts[blockIdx.x] + vox_block_sum(mine, warp_sums, &total);
+  uint32_t at = vox_block_sum(points, warp_sums, &all_points);
+  if (threadIdx.x == 0) room = atomicAdd(reinterpret_cast<uint32_t*>(&status[kVoxCursor]), all_points);
+  __syncthreads();
+  at += room;
+#pragma unroll
+  for (int e = 0; e < kVoxEach; ++e) {
+    const uint32_t s = slot[e];
+    if (s == kNoKey) continue;
+    const uint32_t c = counts[s];
+    seg[s] = at;
+    at += c;
+    if (vid < max_voxels) {
+      voxel_of[s] = static_cast<int>(vid);
+      num_per_voxel[vid] = min(static_cast<int>(c), max_points);
+      // the voxel's coordinates, reversed to (z, y, x)
+      uint32_t rem = static_cast<uint32_t>(slots[s] >> 32);
+      for (int d = g.ndim - 1; d >= 0; --d) {
+        const uint32_t gd = static_cast<uint32_t>(g.grid[d]);
+        indices[static_cast<long long>(vid) * g.ndim + (g.ndim - 1 - d)] = static_cast<int32_t>(rem % gd);
+        rem /= gd;
+      }
+    } else {
+      voxel_of[s] = -1;
     }
+    ++vid;
   }
 }
 
+// pc_voxel_id, and the point's index at its place in its voxel's stretch.
 __global__ void __launch_bounds__(kVoxThreads)
-clamp_counts_kernel(const int* __restrict__ counts, long long num_voxels, int max_points,
-                    int32_t* __restrict__ num_per_voxel) {
-  const long long v = blockIdx.x * static_cast<long long>(kVoxThreads) + threadIdx.x;
-  if (v < num_voxels) num_per_voxel[v] = min(counts[v], max_points);
+place_kernel(const uint32_t* __restrict__ slot_of, const uint32_t* __restrict__ place, long long n, const int* __restrict__ voxel_of,
+             const uint32_t* __restrict__ seg, int* __restrict__ list, long long* __restrict__ pc_voxel_id) {
+  const long long i = blockIdx.x * static_cast<long long>(kVoxThreads) + threadIdx.x;
+  if (i >= n) return;
+  const uint32_t s = slot_of[i];
+  const int v = s == kNoKey ? -1 : voxel_of[s];
+  pc_voxel_id[i] = v;
+  if (v >= 0) list[seg[s] + place[i]] = static_cast<int>(i);
 }
 
-// One thread per (sorted position, feature).
+// chosen[voxel, slot] = the point stored there: the slot of a point is the number of earlier points of its voxel.
 __global__ void __launch_bounds__(kVoxThreads)
-scatter_points_kernel(const float* __restrict__ points, int point_stride, int num_features,
-                      const uint32_t* __restrict__ sorted_vid, const int* __restrict__ sorted_idx,
-                      const int* __restrict__ seg_start, long long n_kept, long long num_voxels, int max_points,
-                      float* __restrict__ voxels) {
+rank_kernel(const uint32_t* __restrict__ slot_of, long long n, const int* __restrict__ voxel_of, const uint32_t* __restrict__ seg,
+            const uint32_t* __restrict__ counts, const int* __restrict__ list, int max_points, int* __restrict__ chosen) {
+  const long long i = blockIdx.x * static_cast<long long>(kVoxThreads) + threadIdx.x;
+  if (i >= n) return;
+  const uint32_t s = slot_of[i];
+  if (s == kNoKey) return;
+  const int v = voxel_of[s];
+  if (v < 0) return;
+  const uint32_t c = counts[s];
+  int rank = 0;
+  if (c > 1) {
+    const int* l = list + seg[s];
+    for (uint32_t q = 0; q < c; ++q) rank += __ldg(&l[q]) < static_cast<int>(i);
+  }
+  if (rank < max_points) chosen[static_cast<long long>(v) * max_points + rank] = static_cast<int>(i);
+}
+
+// The same from the points sorted by (voxel number, index): for voxels of so many points that counting the
+// earlier ones of each would take longer than the sort.
+__global__ void __launch_bounds__(kVoxThreads)
+sort_keys_kernel(const long long* __restrict__ pc_voxel_id, long long n, uint32_t behind, uint32_t* __restrict__ keys, int* __restrict__ vals) {
+  const long long i = blockIdx.x * static_cast<long long>(kVoxThreads) + threadIdx.x;
+  if (i >= n) return;
+  const long long v = pc_voxel_id[i];
+  keys[i] = v < 0 ? behind : static_cast<uint32_t>(v);
+  vals[i] = static_cast<int>(i);
+}
+__global__ void __launch_bounds__(kVoxThreads)
+choose_sorted_kernel(const uint32_t* __restrict__ keys, const int* __restrict__ vals, long long n, uint32_t behind, int max_points,
+                     int* __restrict__ chosen) {
+  const long long i = blockIdx.x * static_cast<long long>(kVoxThreads) + threadIdx.x;
+  if (i >= n) return;
+  const uint32_t v = keys[i];
+  if (v == behind) return;
+  // the slot is the distance to the first position of this voxel, if that is less than max_points
+  long long lo = i - max_points < 0 ? 0 : i - max_points, hi = i;
+  if (lo < i && keys[lo] == v && i - lo >= max_points) return;
+  while (lo < hi) {
+    const long long mid = (lo + hi) >> 1;
+    if (keys[mid] == v) hi = mid;
+    else lo = mid + 1;
+  }
+  chosen[static_cast<long long>(v) * max_points + (i - lo)] = vals[i];
+}
+
+// Rows of the voxel buffer and of the caller's copy (`out`, may be null).  With `clear`: every element of every
+// row, zeros where there is no point; without: only the stored points.
+template <int VEC>
+__global__ void __launch_bounds__(kVoxThreads)
+emit_voxels_kernel(const float* __restrict__ points, int point_stride, int num_features, const int* __restrict__ chosen,
+                   const int32_t* __restrict__ num_per_voxel, long long num_voxels, long long rows, int max_points, int clear,
+                   float* __restrict__ voxels, float* __restrict__ out) {
+  struct alignas(4 * VEC) Pack { float v[VEC]; };
+  const int per = num_features / VEC;
   const long long e = blockIdx.x * static_cast<long long>(kVoxThreads) + threadIdx.x;
-  const long long pos = e / num_features;
-  if (pos >= n_kept) return;
-  const int c = static_cast<int>(e - pos * num_features);
-  const uint32_t vid = sorted_vid[pos];
-  if (vid >= num_voxels) return;  // out of range or beyond the voxel cap: sorted behind every kept point
-  const long long slot = pos - seg_start[vid];
-  if (slot >= max_points) return;
-  voxels[(static_cast<long long>(vid) * max_points + slot) * num_features + c] =
-      __ldg(&points[static_cast<long long>(sorted_idx[pos]) * point_stride + c]);
+  const long long ps = e / per;  // (voxel, slot)
+  if (ps >= rows * max_points) return;
+  const int c = static_cast<int>(e - ps * per) * VEC;
+  const long long v = ps / max_points;
+  const int slot = static_cast<int>(ps - v * max_points);
+  Pack x;
+#pragma unroll
+  for (int q = 0; q < VEC; ++q) x.v[q] = 0.f;
+  const bool have = v < num_voxels && slot < num_per_voxel[v];
+  if (have) x = *reinterpret_cast<const Pack*>(points + static_cast<long long>(chosen[ps]) * point_stride + c);
+  const long long at = ps * num_features + c;
+  if (have || clear) *reinterpret_cast<Pack*>(voxels + at) = x;
+  if (out != nullptr && v < num_voxels) *reinterpret_cast<Pack*>(out + at) = x;
+}
+
+__global__ void __launch_bounds__(kVoxThreads)
+copy_rows_kernel(const int32_t* __restrict__ a, int32_t* __restrict__ a_out, long long na, const int32_t* __restrict__ b,
+                 int32_t* __restrict__ b_out, long long nb) {
+  const long long i = blockIdx.x * static_cast<long long>(kVoxThreads) + threadIdx.x;
+  if (i < na) a_out[i] = a[i];
+  if (i < nb) b_out[i] = b[i];
 }
 
 // One thread per (voxel, feature): unused slots take the mean of the stored points,
@@ -203,21 +352,32 @@ uint32_t vox_pow2_at_least(int64_t v) {
   return c;
 }
 
+// Voxels of more points than this take the radix sort: counting earlier points is quadratic in a voxel's points.
+constexpr int kVoxMostRanked = 256;
+
 struct VoxLayout {
   uint32_t cap;
-  size_t off_status, off_slots, off_keys, off_first, off_flag, off_rank, off_counts, off_seg, off_sk_a, off_sk_b,
-      off_sv_a, off_sv_b, off_cub, cub_bytes, total;
+  size_t off_status, off_slots, off_counts, off_slot_of, off_place, off_voxel_of, off_seg, off_list, off_starts, off_chosen, off_sk_a,
+      off_sk_b, off_sv_a, off_sv_b, off_cub, cub_bytes, total;
 };
 
-VoxLayout vox_layout(int64_t n, int64_t max_voxels) {
+size_t vox_sort_bytes(int64_t n) {
+  static std::atomic<size_t> known[64];
+  int e = 0;
+  while ((1ll << e) < n) ++e;
+  size_t have = known[e].load(std::memory_order_relaxed);
+  if (have != 0) return have;
+  cub::DeviceRadixSort::SortPairs(nullptr, have, static_cast<uint32_t*>(nullptr), static_cast<uint32_t*>(nullptr),
+                                  static_cast<int*>(nullptr), static_cast<int*>(nullptr), static_cast<int>(1ll << e));
+  have = std::max<size_t>(have, 16);
+  known[e].store(have, std::memory_order_relaxed);
+  return have;
+}
+
+VoxLayout vox_layout(int64_t n, int64_t max_voxels, int max_points) {
   VoxLayout L{};
-  L.cap = vox_pow2_at_least(2 * std::max<int64_t>(n, 1));
-  size_t scan_bytes = 0, sort_bytes = 0;
-  cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, static_cast<int*>(nullptr), static_cast<int*>(nullptr),
-                                static_cast<int>(std::max<int64_t>(n, max_voxels)));
-  cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, static_cast<uint32_t*>(nullptr), static_cast<uint32_t*>(nullptr),
-                                  static_cast<int*>(nullptr), static_cast<int*>(nullptr), static_cast<int>(n));
-  L.cub_bytes = std::max(scan_bytes, sort_bytes);
+  L.cap = std::max<uint32_t>(vox_pow2_at_least(2 * std::max<int64_t>(n, 1)), 64);
+  L.cub_bytes = vox_sort_bytes(std::max<int64_t>(n, 1));
   size_t off = 0;
   auto take = [&](size_t bytes) {
     const size_t at = off;
@@ -225,15 +385,17 @@ VoxLayout vox_layout(int64_t n, int64_t max_voxels) {
     return at;
   };
   const size_t np = static_cast<size_t>(std::max<int64_t>(n, 1));
-  const size_t nv = static_cast<size_t>(std::max<int64_t>(max_voxels, 1));
+  const size_t nv = static_cast<size_t>(std::min<int64_t>(std::max<int64_t>(max_voxels, 1), np));
   L.off_status = take(256);
   L.off_slots = take(static_cast<size_t>(L.cap) * 8);
-  L.off_keys = take(np * 4);
-  L.off_first = take(np * 4);
-  L.off_flag = take(np * 4);
-  L.off_rank = take(np * 4);
-  L.off_counts = take(nv * 4);
-  L.off_seg = take(nv * 4);
+  L.off_counts = take(static_cast<size_t>(L.cap) * 4);
+  L.off_voxel_of = take(static_cast<size_t>(L.cap) * 4);
+  L.off_seg = take(static_cast<size_t>(L.cap) * 4);
+  L.off_slot_of = take(np * 4);
+  L.off_place = take(np * 4);
+  L.off_list = take(np * 4);
+  L.off_starts = take(static_cast<size_t>(ceil_div(static_cast<int64_t>(np), kVoxBlock)) * 4);
+  L.off_chosen = take(nv * max_points * 4);
   L.off_sk_a = take(np * 4);
   L.off_sk_b = take(np * 4);
   L.off_sv_a = take(np * 4);
@@ -243,14 +405,164 @@ VoxLayout vox_layout(int64_t n, int64_t max_voxels) {
   return L;
 }
 
+struct VoxArgs {
+  const float* points;
+  int64_t n;
+  int point_stride, num_features;
+  int64_t max_voxels;
+  int max_points;
+  VoxGeo g{};
+};
+int vox_check(const float* points, int64_t n_points, int point_stride, int ndim, int num_features, const float* cmin, const float* vsize,
+              const int32_t* grid_xyz, int64_t max_voxels, int max_points, VoxArgs* a) {
+  if (!cmin || !vsize || !grid_xyz || ndim < 1 || ndim > kVoxMaxDim || num_features < 1 ||
+      point_stride < std::max(ndim, num_features) || max_voxels <= 0 || max_points <= 0 || n_points < 0)
+    return fail(SPC_ERR_INVALID_ARGUMENT, "voxelize: bad arguments");
+  if (n_points >= (1ll << 30)) return fail(SPC_ERR_SIZE_LIMIT, "voxelize: %lld points", static_cast<long long>(n_points));
+  a->points = points;
+  a->n = n_points;
+  a->point_stride = point_stride;
+  a->num_features = num_features;
+  a->max_voxels = max_voxels;
+  a->max_points = max_points;
+  a->g.ndim = ndim;
+  double volume = 1;
+  for (int d = 0; d < ndim; ++d) {
+    if (grid_xyz[d] <= 0 || !(vsize[d] > 0.f)) return fail(SPC_ERR_INVALID_ARGUMENT, "voxelize: bad grid");
+    a->g.cmin[d] = cmin[d];
+    a->g.vsize[d] = vsize[d];
+    a->g.grid[d] = grid_xyz[d];
+    volume *= grid_xyz[d];
+  }
+  if (volume >= 4294967295.0) return fail(SPC_ERR_SIZE_LIMIT, "voxelize: grid of %.0f cells needs keys beyond 32 bits", volume);
+  return SPC_OK;
+}
+
 }  // namespace
 }  // namespace spc
 
 using namespace spc;
 
-extern "C" size_t spc_voxelize_workspace_bytes(int64_t n_points, int64_t max_voxels) {
-  if (n_points < 0 || max_voxels <= 0 || n_points >= (1ll << 30)) return 0;
-  return vox_layout(n_points, max_voxels).total;
+extern "C" size_t spc_voxelize_workspace_bytes(int64_t n_points, int64_t max_voxels, int max_points) {
+  if (n_points < 0 || max_voxels <= 0 || max_points <= 0 || n_points >= (1ll << 30)) return 0;
+  return vox_layout(n_points, max_voxels, max_points).total;
+}
+
+extern "C" int spc_voxelize_number(const float* points, int64_t n_points, int point_stride, int ndim, int num_features, const float* cmin,
+                                   const float* vsize, const int32_t* grid_xyz, int64_t max_voxels, int max_points, void* workspace,
+                                   size_t workspace_bytes, int32_t* indices, int32_t* num_per_voxel, int64_t* pc_voxel_id,
+                                   int64_t* num_voxels_host, int* sorted_host, void* stream) {
+  VoxArgs a;
+  int rc = vox_check(points, n_points, point_stride, ndim, num_features, cmin, vsize, grid_xyz, max_voxels, max_points, &a);
+  if (rc != SPC_OK) return rc;
+  if (!num_voxels_host || !sorted_host || !indices || !num_per_voxel || !workspace || (n_points > 0 && (!points || !pc_voxel_id)))
+    return fail(SPC_ERR_INVALID_ARGUMENT, "voxelize: bad arguments");
+  *num_voxels_host = 0;
+  *sorted_host = 0;
+  if (n_points == 0) return SPC_OK;
+  const VoxLayout L = vox_layout(n_points, max_voxels, max_points);
+  if (workspace_bytes < L.total)
+    return fail(SPC_ERR_WORKSPACE_TOO_SMALL, "voxelize: workspace %zu < %zu bytes", workspace_bytes, L.total);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  char* ws = static_cast<char*>(workspace);
+  int* status = reinterpret_cast<int*>(ws + L.off_status);
+  unsigned long long* slots = reinterpret_cast<unsigned long long*>(ws + L.off_slots);
+  uint32_t* counts = reinterpret_cast<uint32_t*>(ws + L.off_counts);
+  int* voxel_of = reinterpret_cast<int*>(ws + L.off_voxel_of);
+  uint32_t* seg = reinterpret_cast<uint32_t*>(ws + L.off_seg);
+  uint32_t* slot_of = reinterpret_cast<uint32_t*>(ws + L.off_slot_of);
+  uint32_t* place = reinterpret_cast<uint32_t*>(ws + L.off_place);
+  uint32_t* starts = reinterpret_cast<uint32_t*>(ws + L.off_starts);
+  const uint32_t cap_mask = L.cap - 1;
+  volatile int* box = nullptr;
+  int ticket = 0;
+  rc = host_mailbox(&box, &ticket);
+  if (rc != SPC_OK) return rc;
+  vox_clear_kernel<<<static_cast<unsigned>(std::min<int64_t>(ceil_div(L.cap / 2, kVoxThreads), 16ll * sm_count())), kVoxThreads, 0, st>>>(
+      reinterpret_cast<uint4*>(status), reinterpret_cast<uint4*>(slots), L.cap / 2, reinterpret_cast<uint4*>(counts), L.cap / 4);
+  SPC_LAUNCH_OK();
+  quantize_insert_kernel<<<vox_blocks(a.n), kVoxThreads, 0, st>>>(a.g, points, a.n, point_stride, slots, cap_mask, counts, slot_of, place,
+                                                               status);
+  SPC_LAUNCH_OK();
+  const unsigned blocks = static_cast<unsigned>(ceil_div(a.n, kVoxBlock));
+  count_first_kernel<<<blocks, kVoxThreads, 0, st>>>(slot_of, a.n, slots, counts, starts, status, box, ticket);
+  SPC_LAUNCH_OK();
+  number_voxels_kernel<<<blocks, kVoxThreads, 0, st>>>(a.g, slot_of, a.n, slots, counts, starts, max_voxels, max_points, voxel_of, seg, status,
+                                                       indices, num_per_voxel);
+  SPC_LAUNCH_OK();
+  place_kernel<<<vox_blocks(a.n), kVoxThreads, 0, st>>>(slot_of, place, a.n, voxel_of, seg, reinterpret_cast<int*>(ws + L.off_list),
+                                                     reinterpret_cast<long long*>(pc_voxel_id));
+  SPC_LAUNCH_OK();
+  rc = wait_for_ticket(box, ticket, st);
+  if (rc != SPC_OK) return rc;
+  if (box[1] != 0) return fail(box[1], "voxelize: hash table full (status %d)", box[1]);
+  *num_voxels_host = std::min<int64_t>(box[2], max_voxels);
+  *sorted_host = box[3] > kVoxMostRanked;
+  return SPC_OK;
+}
+
+extern "C" int spc_voxelize_store(const float* points, int64_t n_points, int point_stride, int ndim, int num_features, int64_t max_voxels,
+                                  int max_points, int clear_voxels, int empty_mean, void* workspace, size_t workspace_bytes,
+                                  int64_t num_voxels, int sorted, const int32_t* indices, const int32_t* num_per_voxel,
+                                  const int64_t* pc_voxel_id, float* voxels, float* voxels_out, int32_t* indices_out, int32_t* num_out,
+                                  void* stream) {
+  if (!workspace || !indices || !num_per_voxel || !voxels || n_points < 0 || num_voxels < 0 || num_voxels > max_voxels || num_features < 1 ||
+      max_points <= 0 || ndim < 1 || (n_points > 0 && (!points || !pc_voxel_id)))
+    return fail(SPC_ERR_INVALID_ARGUMENT, "voxelize: bad arguments");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const VoxLayout L = vox_layout(n_points, max_voxels, max_points);
+  if (workspace_bytes < L.total)
+    return fail(SPC_ERR_WORKSPACE_TOO_SMALL, "voxelize: workspace %zu < %zu bytes", workspace_bytes, L.total);
+  char* ws = static_cast<char*>(workspace);
+  int* chosen = reinterpret_cast<int*>(ws + L.off_chosen);
+  if (num_voxels > 0 && !sorted) {
+    rank_kernel<<<vox_blocks(n_points), kVoxThreads, 0, st>>>(
+        reinterpret_cast<uint32_t*>(ws + L.off_slot_of), n_points, reinterpret_cast<int*>(ws + L.off_voxel_of),
+        reinterpret_cast<uint32_t*>(ws + L.off_seg), reinterpret_cast<uint32_t*>(ws + L.off_counts), reinterpret_cast<int*>(ws + L.off_list),
+        max_points, chosen);
+    SPC_LAUNCH_OK();
+  } else if (num_voxels > 0) {
+    uint32_t* sk_a = reinterpret_cast<uint32_t*>(ws + L.off_sk_a);
+    uint32_t* sk_b = reinterpret_cast<uint32_t*>(ws + L.off_sk_b);
+    int* sv_a = reinterpret_cast<int*>(ws + L.off_sv_a);
+    int* sv_b = reinterpret_cast<int*>(ws + L.off_sv_b);
+    const uint32_t behind = static_cast<uint32_t>(num_voxels);  // dropped points sort behind every voxel
+    sort_keys_kernel<<<vox_blocks(n_points), kVoxThreads, 0, st>>>(reinterpret_cast<const long long*>(pc_voxel_id), n_points, behind, sk_a, sv_a);
+    SPC_LAUNCH_OK();
+    int bits = 1;
+    while (bits < 32 && (1ll << bits) <= num_voxels) ++bits;
+    size_t cub_bytes = L.cub_bytes;
+    SPC_CUDA_OK(cub::DeviceRadixSort::SortPairs(ws + L.off_cub, cub_bytes, sk_a, sk_b, sv_a, sv_b, static_cast<int>(n_points), 0, bits, st));
+    choose_sorted_kernel<<<vox_blocks(n_points), kVoxThreads, 0, st>>>(sk_b, sv_b, n_points, behind, max_points, chosen);
+    SPC_LAUNCH_OK();
+  }
+  const int64_t rows = clear_voxels ? max_voxels : num_voxels;
+  const bool wide = num_features % 4 == 0 && point_stride % 4 == 0 &&
+                    ((reinterpret_cast<uintptr_t>(points) | reinterpret_cast<uintptr_t>(voxels) | reinterpret_cast<uintptr_t>(voxels_out)) & 15u) == 0;
+  if (rows > 0) {
+    const unsigned blocks = vox_blocks(rows * max_points * (wide ? num_features / 4 : num_features));
+    if (wide)
+      emit_voxels_kernel<4><<<blocks, kVoxThreads, 0, st>>>(points, point_stride, num_features, chosen, num_per_voxel, num_voxels, rows,
+                                                           max_points, clear_voxels, voxels, voxels_out);
+    else
+      emit_voxels_kernel<1><<<blocks, kVoxThreads, 0, st>>>(points, point_stride, num_features, chosen, num_per_voxel, num_voxels, rows,
+                                                           max_points, clear_voxels, voxels, voxels_out);
+    SPC_LAUNCH_OK();
+  }
+  if (num_voxels == 0) return SPC_OK;
+  if (empty_mean) {
+    for (float* v : {voxels, voxels_out}) {
+      if (v == nullptr) continue;
+      fill_mean_kernel<<<vox_blocks(num_voxels * num_features), kVoxThreads, 0, st>>>(v, num_per_voxel, num_voxels, max_points, num_features);
+      SPC_LAUNCH_OK();
+    }
+  }
+  if (indices_out != nullptr && num_out != nullptr) {
+    copy_rows_kernel<<<vox_blocks(num_voxels * ndim), kVoxThreads, 0, st>>>(indices, indices_out, num_voxels * ndim, num_per_voxel, num_out,
+                                                                         num_voxels);
+    SPC_LAUNCH_OK();
+  }
+  return SPC_OK;
 }
 
 extern "C" int spc_voxelize(const float* points, int64_t n_points, int point_stride, int ndim, int num_features,
@@ -258,90 +570,12 @@ extern "C" int spc_voxelize(const float* points, int64_t n_points, int point_str
                             int max_points, int clear_voxels, int empty_mean, void* workspace,
                             size_t workspace_bytes, float* voxels, int32_t* indices, int32_t* num_per_voxel,
                             int64_t* pc_voxel_id, int64_t* num_voxels_host, void* stream) {
-  if (!num_voxels_host || !cmin || !vsize || !grid_xyz || ndim < 1 || ndim > kVoxMaxDim || num_features < 1 ||
-      point_stride < std::max(ndim, num_features) || max_voxels <= 0 || max_points <= 0 || n_points < 0 ||
-      !voxels || !indices || !num_per_voxel || !workspace)
-    return fail(SPC_ERR_INVALID_ARGUMENT, "voxelize: bad arguments");
-  if (n_points >= (1ll << 30)) return fail(SPC_ERR_SIZE_LIMIT, "voxelize: %lld points", static_cast<long long>(n_points));
-  VoxGeo g{};
-  g.ndim = ndim;
-  double volume = 1;
-  for (int d = 0; d < ndim; ++d) {
-    if (grid_xyz[d] <= 0 || !(vsize[d] > 0.f)) return fail(SPC_ERR_INVALID_ARGUMENT, "voxelize: bad grid");
-    g.cmin[d] = cmin[d];
-    g.vsize[d] = vsize[d];
-    g.grid[d] = grid_xyz[d];
-    volume *= grid_xyz[d];
-  }
-  if (volume >= 4294967295.0) return fail(SPC_ERR_SIZE_LIMIT, "voxelize: grid of %.0f cells needs keys beyond 32 bits", volume);
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  *num_voxels_host = 0;
-  if (clear_voxels)
-    SPC_CUDA_OK(cudaMemsetAsync(voxels, 0, static_cast<size_t>(max_voxels) * max_points * num_features * sizeof(float), st));
-  if (n_points == 0) return SPC_OK;
-  if (!points || !pc_voxel_id) return fail(SPC_ERR_INVALID_ARGUMENT, "voxelize: null points");
-  const VoxLayout L = vox_layout(n_points, max_voxels);
-  if (workspace_bytes < L.total)
-    return fail(SPC_ERR_WORKSPACE_TOO_SMALL, "voxelize: workspace %zu < %zu bytes", workspace_bytes, L.total);
-  char* ws = static_cast<char*>(workspace);
-  int* status = reinterpret_cast<int*>(ws + L.off_status);
-  unsigned long long* slots = reinterpret_cast<unsigned long long*>(ws + L.off_slots);
-  uint32_t* keys = reinterpret_cast<uint32_t*>(ws + L.off_keys);
-  int* first = reinterpret_cast<int*>(ws + L.off_first);
-  int* flag = reinterpret_cast<int*>(ws + L.off_flag);
-  int* rank = reinterpret_cast<int*>(ws + L.off_rank);
-  int* counts = reinterpret_cast<int*>(ws + L.off_counts);
-  int* seg = reinterpret_cast<int*>(ws + L.off_seg);
-  uint32_t* sk_a = reinterpret_cast<uint32_t*>(ws + L.off_sk_a);
-  uint32_t* sk_b = reinterpret_cast<uint32_t*>(ws + L.off_sk_b);
-  int* sv_a = reinterpret_cast<int*>(ws + L.off_sv_a);
-  int* sv_b = reinterpret_cast<int*>(ws + L.off_sv_b);
-  const uint32_t cap_mask = L.cap - 1;
-  const int n = static_cast<int>(n_points);
-
-  SPC_CUDA_OK(cudaMemsetAsync(status, 0, 256, st));
-  SPC_CUDA_OK(cudaMemsetAsync(slots, 0xFF, static_cast<size_t>(L.cap) * 8, st));
-  quantize_insert_kernel<<<vox_blocks(n), kVoxThreads, 0, st>>>(g, points, n, point_stride, slots, cap_mask, keys, status);
-  SPC_LAUNCH_OK();
-  mark_first_kernel<<<vox_blocks(n), kVoxThreads, 0, st>>>(keys, n, slots, cap_mask, first, flag);
-  SPC_LAUNCH_OK();
-  size_t cub_bytes = L.cub_bytes;
-  SPC_CUDA_OK(cub::DeviceScan::ExclusiveSum(ws + L.off_cub, cub_bytes, flag, rank, n, st));
-  total_kernel<<<1, 1, 0, st>>>(rank, flag, n, status);
-  SPC_LAUNCH_OK();
-  int host[2] = {0, 0};  // status, voxels found
-  SPC_CUDA_OK(cudaMemcpyAsync(host, status, sizeof(host), cudaMemcpyDeviceToHost, st));
-  SPC_CUDA_OK(cudaStreamSynchronize(st));
-  if (host[0] != 0) return fail(host[0], "voxelize: hash table full (status %d)", host[0]);
-  const int64_t total_voxels = host[1];
-  const int64_t num_voxels = std::min<int64_t>(total_voxels, max_voxels);
-  *num_voxels_host = num_voxels;
-  if (num_voxels == 0) {
-    SPC_CUDA_OK(cudaMemsetAsync(pc_voxel_id, 0xFF, static_cast<size_t>(n) * sizeof(int64_t), st));
-    return SPC_OK;
-  }
-  SPC_CUDA_OK(cudaMemsetAsync(counts, 0, static_cast<size_t>(num_voxels) * 4, st));
-  assign_kernel<<<vox_blocks(n), kVoxThreads, 0, st>>>(g, keys, first, rank, n, num_voxels, counts, sk_a, sv_a,
-                                                    reinterpret_cast<long long*>(pc_voxel_id), indices);
-  SPC_LAUNCH_OK();
-  clamp_counts_kernel<<<vox_blocks(num_voxels), kVoxThreads, 0, st>>>(counts, num_voxels, max_points, num_per_voxel);
-  SPC_LAUNCH_OK();
-  cub_bytes = L.cub_bytes;
-  SPC_CUDA_OK(cub::DeviceScan::ExclusiveSum(ws + L.off_cub, cub_bytes, counts, seg, static_cast<int>(num_voxels), st));
-  // stable: arrival order survives inside a voxel; dropped points carry the key num_voxels and
-  // sort behind all others; only the bits that key needs are sorted
-  int bits = 1;
-  while (bits < 32 && (1ll << bits) <= num_voxels) ++bits;
-  cub_bytes = L.cub_bytes;
-  SPC_CUDA_OK(cub::DeviceRadixSort::SortPairs(ws + L.off_cub, cub_bytes, sk_a, sk_b, sv_a, sv_b, n, 0, bits, st));
-  const long long work = static_cast<long long>(n) * num_features;
-  scatter_points_kernel<<<vox_blocks(work), kVoxThreads, 0, st>>>(points, point_stride, num_features, sk_b, sv_b, seg,
-                                                                 n, num_voxels, max_points, voxels);
-  SPC_LAUNCH_OK();
-  if (empty_mean) {
-    fill_mean_kernel<<<vox_blocks(num_voxels * num_features), kVoxThreads, 0, st>>>(voxels, num_per_voxel, num_voxels,
-                                                                                    max_points, num_features);
-    SPC_LAUNCH_OK();
-  }
-  return SPC_OK;
+  if (!voxels) return fail(SPC_ERR_INVALID_ARGUMENT, "voxelize: bad arguments");
+  int sorted = 0;
+  const int rc = spc_voxelize_number(points, n_points, point_stride, ndim, num_features, cmin, vsize, grid_xyz, max_voxels, max_points,
+                                     workspace, workspace_bytes, indices, num_per_voxel, pc_voxel_id, num_voxels_host, &sorted, stream);
+  if (rc != SPC_OK) return rc;
+  return spc_voxelize_store(points, n_points, point_stride, ndim, num_features, max_voxels, max_points, clear_voxels, empty_mean, workspace,
+                            workspace_bytes, *num_voxels_host, sorted, indices, num_per_voxel, pc_voxel_id, voxels, nullptr, nullptr, nullptr,
+                            stream);
 }

@@ -2,18 +2,16 @@
 
 ``PointToVoxel`` keeps the reference's constructor, persistent buffers, return
 values and first-come-first-served semantics; the work is done by
-``spc_voxelize`` of the CUDA library (hash table + prefix sum + one stable
-radix sort) and its results equal the reference's bit for bit.  CUDA tensors
+``spc_voxelize_number`` / ``spc_voxelize_store`` of the CUDA library (hash table,
+prefix sums, ranks inside a voxel) and its results equal the reference's bit for bit.  CUDA tensors
 only: there is no CPU path.
 """
 
 from __future__ import annotations
 
-import ctypes
-
 import torch
 
-from spconv_triton_b200 import _lib
+from ._impl import host as _host
 
 
 class PointToVoxel:
@@ -63,28 +61,8 @@ class PointToVoxel:
             raise NotImplementedError("points must be float32 (voxel boundaries are computed in the points' dtype)")
         if pc.dim() != 2 or pc.shape[1] < max(self.ndim, self.num_point_features):
             raise AssertionError("points must be [N, >= max(ndim, num_point_features)]")
-        pc = pc.contiguous()
-        n = int(pc.shape[0])
-        lib = _lib.load()
-        nd = self.ndim
-        cmin = (ctypes.c_float * nd)(*[float(v) for v in self._coors_range_xyz[:nd]])
-        vsize = (ctypes.c_float * nd)(*[float(v) for v in self._vsize_xyz])
-        grid = (ctypes.c_int32 * nd)(*[int(v) for v in self._grid_size_xyz])
-        with torch.no_grad(), torch.cuda.device(pc.device):
-            pc_voxel_id = torch.empty([n], dtype=torch.int64, device=pc.device)
-            nbytes = int(lib.spc_voxelize_workspace_bytes(n, self.max_num_voxels))
-            if nbytes == 0:
-                raise _lib.SpconvB200Error("voxelize: sizes out of range")
-            ws = torch.empty(nbytes, dtype=torch.uint8, device=pc.device)
-            num = ctypes.c_int64(0)
-            _lib.check(lib.spc_voxelize(
-                _lib.ptr(pc) if n else None, n, int(pc.stride(0)) if n else max(nd, self.num_point_features), nd,
-                self.num_point_features, cmin, vsize, grid, self.max_num_voxels, self.max_num_points_per_voxel,
-                int(bool(clear_voxels)), int(bool(empty_mean)), _lib.ptr(ws), nbytes, _lib.ptr(self.voxels),
-                _lib.ptr(self.indices), _lib.ptr(self.num_per_voxel), _lib.ptr(pc_voxel_id) if n else None,
-                ctypes.byref(num), _lib.current_stream(pc.device)))
-            m = int(num.value)
-            return (self.voxels[:m].clone(), self.indices[:m].clone(), self.num_per_voxel[:m].clone(), pc_voxel_id)
+        return _host.ext().voxelize(pc, self.voxels, self.indices, self.num_per_voxel, self._coors_range_xyz[:self.ndim], self._vsize_xyz,
+                                    self._grid_size_xyz, bool(clear_voxels), bool(empty_mean))
 
 
 def gather_features_by_pc_voxel_id(seg_res_features: torch.Tensor, pc_voxel_id: torch.Tensor,
