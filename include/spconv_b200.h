@@ -242,8 +242,8 @@ int spc_voxelize(const float* points, int64_t n_points, int point_stride, int nd
 /* spc_voxelize in two halves, for callers that return copies of the filled rows: the
  * first numbers the voxels (indices, num_per_voxel, pc_voxel_id) and tells the host how
  * many there are; the second writes the voxel buffer and, in the same pass, the copies
- * voxels_out [num_voxels, max_points, num_features], indices_out and num_out (may be
- * NULL).  `sorted` is what the first said; the workspace is the same, untouched. */
+ * voxels_out [num_voxels, max_points, num_features], indices_out and num_out (all three or
+ * none).  `sorted` is what the first said; the workspace is the same, untouched. */
 int spc_voxelize_number(const float* points, int64_t n_points, int point_stride, int ndim, int num_features,
                         const float* cmin, const float* vsize, const int32_t* grid_xyz, int64_t max_voxels,
                         int max_points, void* workspace, size_t workspace_bytes, int32_t* indices,

@@ -64,21 +64,32 @@ __device__ __forceinline__ uint32_t vox_mix(uint32_t h) {
 
 inline unsigned vox_blocks(int64_t n) { return static_cast<unsigned>(ceil_div(std::max<int64_t>(n, 1), kVoxThreads)); }
 
+// One slot of the hash table, 16 bytes so that whatever a point asks of its voxel is one sector.  While points
+// are entered: key << 32 | lowest point index (all ones: free) and their count.  Once numbered: the voxel
+// (-1: beyond the cap), its stretch of the list, the count.
+struct alignas(16) VoxSlot {
+  union {
+    unsigned long long packed;
+    struct {
+      int voxel;
+      uint32_t seg;
+    };
+  };
+  uint32_t count, unused;
+};
+
 __global__ void __launch_bounds__(kVoxThreads)
-vox_clear_kernel(uint4* __restrict__ status, uint4* __restrict__ slots, long long n_slots16, uint4* __restrict__ counts,
-                 long long n_counts16) {
+vox_clear_kernel(uint4* __restrict__ status, uint4* __restrict__ slots, long long n_slots) {
   const long long stride = static_cast<long long>(gridDim.x) * kVoxThreads, t = blockIdx.x * static_cast<long long>(kVoxThreads) + threadIdx.x;
   if (t < 16) status[t] = make_uint4(0u, 0u, 0u, 0u);
-  for (long long i = t; i < n_slots16; i += stride) slots[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
-  for (long long i = t; i < n_counts16; i += stride) counts[i] = make_uint4(0u, 0u, 0u, 0u);
+  for (long long i = t; i < n_slots; i += stride) slots[i] = make_uint4(~0u, ~0u, 0u, 0u);
 }
 
 enum VoxStatus { kVoxError = 0, kVoxTotal = 1, kVoxMost = 2, kVoxTicket = 3, kVoxCursor = 4 };
 
 __global__ void __launch_bounds__(kVoxThreads)
 quantize_insert_kernel(const __grid_constant__ VoxGeo g, const float* __restrict__ points, long long n,
-                       int point_stride, unsigned long long* __restrict__ slots, uint32_t cap_mask,
-                       uint32_t* __restrict__ counts, uint32_t* __restrict__ slot_of, uint32_t* __restrict__ place,
+                       int point_stride, VoxSlot* __restrict__ slots, uint32_t cap_mask, uint32_t* __restrict__ slot_of, uint32_t* __restrict__ place,
                        int* __restrict__ status) {
   const long long i = blockIdx.x * static_cast<long long>(kVoxThreads) + threadIdx.x;
   if (i >= n) return;
@@ -99,11 +110,11 @@ quantize_insert_kernel(const __grid_constant__ VoxGeo g, const float* __restrict
   const unsigned long long packed = (static_cast<unsigned long long>(key) << 32) | static_cast<uint32_t>(i);
   uint32_t s = vox_mix(key) & cap_mask;
   for (uint32_t probe = 0; probe <= cap_mask; ++probe) {
-    const unsigned long long old = atomicCAS(&slots[s], kVoxEmpty, packed);
+    const unsigned long long old = atomicCAS(&slots[s].packed, kVoxEmpty, packed);
     if (old == kVoxEmpty || static_cast<uint32_t>(old >> 32) == key) {
-      if (old != kVoxEmpty) atomicMin(&slots[s], packed);
+      if (old != kVoxEmpty) atomicMin(&slots[s].packed, packed);
       slot_of[i] = s;
-      place[i] = atomicAdd(&counts[s], 1u);
+      place[i] = atomicAdd(&slots[s].count, 1u);
       return;
     }
     s = (s + 1) & cap_mask;
@@ -135,23 +146,34 @@ __device__ __forceinline__ uint32_t vox_block_sum(uint32_t v, uint32_t* warp_sum
   return before + incl - v;  // exclusive
 }
 
-// First points per block; the last block to finish turns the sums into starts and hands the number of voxels
-// and the largest count of points in one to the host.
+// First points: their bits, and how many a block has; the last block to finish turns the sums into starts and
+// hands the number of voxels and the largest count of points in one to the host.
 __global__ void __launch_bounds__(kVoxThreads)
-count_first_kernel(const uint32_t* __restrict__ slot_of, long long n, const unsigned long long* __restrict__ slots,
-                   const uint32_t* __restrict__ counts, uint32_t* __restrict__ starts, int* __restrict__ status,
-                   volatile int* host_box, int ticket) {
+count_first_kernel(const uint32_t* __restrict__ slot_of, long long n, const VoxSlot* __restrict__ slots, uint32_t* __restrict__ first_bits,
+                   uint32_t* __restrict__ starts, int* __restrict__ status, volatile int* host_box, int ticket) {
   __shared__ uint32_t warp_sums[kVoxThreads / 32];
   __shared__ int last;
   const long long base = blockIdx.x * static_cast<long long>(kVoxBlock);
   uint32_t mine = 0, most = 0;
+  uint32_t slot[kVoxEach];
 #pragma unroll
   for (int e = 0; e < kVoxEach; ++e) {
     const long long i = base + e * kVoxThreads + threadIdx.x;
-    const uint32_t s = i < n ? slot_of[i] : kNoKey;
-    if (s == kNoKey || static_cast<uint32_t>(slots[s]) != static_cast<uint32_t>(i)) continue;
+    slot[e] = i < n ? slot_of[i] : kNoKey;
+  }
+  uint4 held[kVoxEach];  // all requested before any is used
+#pragma unroll
+  for (int e = 0; e < kVoxEach; ++e)
+    held[e] = slot[e] != kNoKey ? *reinterpret_cast<const uint4*>(&slots[slot[e]]) : make_uint4(kNoKey, 0u, 0u, 0u);
+#pragma unroll
+  for (int e = 0; e < kVoxEach; ++e) {
+    const long long i = base + e * kVoxThreads + threadIdx.x;
+    const bool first = slot[e] != kNoKey && held[e].x == static_cast<uint32_t>(i);  // (the low word of `packed`)
+    const unsigned bits = __ballot_sync(0xffffffffu, first);
+    if ((threadIdx.x & 31) == 0) first_bits[(base + e * kVoxThreads + threadIdx.x) >> 5] = bits;
+    if (!first) continue;
     ++mine;
-    most = max(most, counts[s]);
+    most = max(most, held[e].z);
   }
   most = __reduce_max_sync(0xffffffffu, most);
   if ((threadIdx.x & 31) == 0 && most > 0) atomicMax(&status[kVoxMost], static_cast<int>(most));
@@ -185,84 +207,99 @@ count_first_kernel(const uint32_t* __restrict__ slot_of, long long n, const unsi
   }
 }
 
-// Voxel number of every slot that has one below the cap (else -1), its stretch of the list, its coordinates
-// and its count.
+// The voxel number of every first point below the cap (else -1), its stretch of the list, its coordinates and
+// its count.  Only first points touch their slot, so it can take its second meaning in place.
 __global__ void __launch_bounds__(kVoxThreads)
-number_voxels_kernel(const __grid_constant__ VoxGeo g, const uint32_t* __restrict__ slot_of, long long n,
-                     const unsigned long long* __restrict__ slots, const uint32_t* __restrict__ counts,
-                     const uint32_t* __restrict__ starts, long long max_voxels, int max_points, int* __restrict__ voxel_of,
-                     uint32_t* __restrict__ seg, int* __restrict__ status, int32_t* __restrict__ indices,
-                     int32_t* __restrict__ num_per_voxel) {
-  __shared__ uint32_t warp_sums[kVoxThreads / 32];
-  __shared__ uint32_t room;
-  // a thread numbers consecutive points, so that the numbers of a block follow the order of its points
-  const long long base = blockIdx.x * static_cast<long long>(kVoxBlock) + threadIdx.x * kVoxEach;
-  uint32_t slot[kVoxEach], mine = 0, points = 0;
+number_voxels_kernel(const __grid_constant__ VoxGeo g, const uint32_t* __restrict__ slot_of, long long n, VoxSlot* __restrict__ slots,
+                     const uint32_t* __restrict__ first_bits, const uint32_t* __restrict__ starts, long long max_voxels, int max_points,
+                     int* __restrict__ status, int32_t* __restrict__ indices, int32_t* __restrict__ num_per_voxel) {
+  constexpr int kWords = kVoxBlock / 32;
+  __shared__ uint32_t before[kWords], bits_s[kWords];
+  __shared__ uint32_t points, room;
+  const long long base = blockIdx.x * static_cast<long long>(kVoxBlock);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) points = 0;
+  if (warp == 0) {
+    static_assert(kWords == 64, "two words a lane");
+    const uint32_t a = first_bits[(base >> 5) + 2 * lane], b = first_bits[(base >> 5) + 2 * lane + 1];
+    uint32_t incl = __popc(a) + __popc(b);
+    const uint32_t both = incl;
 #pragma unroll
-  for (int e = 0; e < kVoxEach; ++e) {
-    const long long i = base + e;
-    slot[e] = i < n ? slot_of[i] : kNoKey;
-    if (slot[e] != kNoKey && static_cast<uint32_t>(slots[slot[e]]) != static_cast<uint32_t>(i)) slot[e] = kNoKey;
-    if (slot[e] == kNoKey) continue;
-    ++mine;
-    points += counts[slot[e]];
-  }
-  uint32_t total, all_points;
-  uint32_t vid = starts[blockIdx.x] + vox_block_sum(mine, warp_sums, &total);
-  uint32_t at = vox_block_sum(points, warp_sums, &all_points);
-  if (threadIdx.x == 0) room = atomicAdd(reinterpret_cast<uint32_t*>(&status[kVoxCursor]), all_points);
-  __syncthreads();
-  at += room;
-#pragma unroll
-  for (int e = 0; e < kVoxEach; ++e) {
-    const uint32_t s = slot[e];
-    if (s == kNoKey) continue;
-    const uint32_t c = counts[s];
-    seg[s] = at;
-    at += c;
-    if (vid < max_voxels) {
-      voxel_of[s] = static_cast<int>(vid);
-      num_per_voxel[vid] = min(static_cast<int>(c), max_points);
-      // the voxel's coordinates, reversed to (z, y, x)
-      uint32_t rem = static_cast<uint32_t>(slots[s] >> 32);
-      for (int d = g.ndim - 1; d >= 0; --d) {
-        const uint32_t gd = static_cast<uint32_t>(g.grid[d]);
-        indices[static_cast<long long>(vid) * g.ndim + (g.ndim - 1 - d)] = static_cast<int32_t>(rem % gd);
-        rem /= gd;
-      }
-    } else {
-      voxel_of[s] = -1;
+    for (int off = 1; off < 32; off <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, off);
+      if (lane >= off) incl += t;
     }
-    ++vid;
+    bits_s[2 * lane] = a;
+    bits_s[2 * lane + 1] = b;
+    before[2 * lane] = incl - both;
+    before[2 * lane + 1] = incl - both + __popc(a);
+  }
+  __syncthreads();
+  const uint32_t start = starts[blockIdx.x];
+  uint32_t slot[kVoxEach], at[kVoxEach];
+  uint4 held[kVoxEach];
+#pragma unroll
+  for (int e = 0; e < kVoxEach; ++e) {
+    const bool first = (bits_s[e * (kVoxThreads / 32) + warp] >> lane) & 1u;
+    slot[e] = first ? slot_of[base + e * kVoxThreads + threadIdx.x] : kNoKey;
+  }
+#pragma unroll
+  for (int e = 0; e < kVoxEach; ++e)
+    if (slot[e] != kNoKey) held[e] = *reinterpret_cast<const uint4*>(&slots[slot[e]]);
+#pragma unroll
+  for (int e = 0; e < kVoxEach; ++e)
+    if (slot[e] != kNoKey) at[e] = atomicAdd(&points, held[e].z);
+  __syncthreads();
+  if (threadIdx.x == 0) room = atomicAdd(reinterpret_cast<uint32_t*>(&status[kVoxCursor]), points);
+  __syncthreads();
+#pragma unroll
+  for (int e = 0; e < kVoxEach; ++e) {
+    if (slot[e] == kNoKey) continue;
+    const int w = e * (kVoxThreads / 32) + warp;
+    const long long vid = static_cast<long long>(start) + before[w] + __popc(bits_s[w] & ((1u << lane) - 1u));
+    const bool kept = vid < max_voxels;
+    *reinterpret_cast<uint4*>(&slots[slot[e]]) =
+        make_uint4(kept ? static_cast<uint32_t>(vid) : 0xffffffffu, room + at[e], held[e].z, 0u);
+    if (!kept) continue;
+    num_per_voxel[vid] = min(static_cast<int>(held[e].z), max_points);
+    // the voxel's coordinates, reversed to (z, y, x)
+    uint32_t rem = held[e].y;  // the key
+    for (int d = g.ndim - 1; d >= 0; --d) {
+      const uint32_t gd = static_cast<uint32_t>(g.grid[d]);
+      indices[vid * g.ndim + (g.ndim - 1 - d)] = static_cast<int32_t>(rem % gd);
+      rem /= gd;
+    }
   }
 }
 
 // pc_voxel_id, and the point's index at its place in its voxel's stretch.
 __global__ void __launch_bounds__(kVoxThreads)
-place_kernel(const uint32_t* __restrict__ slot_of, const uint32_t* __restrict__ place, long long n, const int* __restrict__ voxel_of,
-             const uint32_t* __restrict__ seg, int* __restrict__ list, long long* __restrict__ pc_voxel_id) {
+place_kernel(const uint32_t* __restrict__ slot_of, const uint32_t* __restrict__ place, long long n, const VoxSlot* __restrict__ slots,
+             int* __restrict__ list, long long* __restrict__ pc_voxel_id) {
   const long long i = blockIdx.x * static_cast<long long>(kVoxThreads) + threadIdx.x;
   if (i >= n) return;
   const uint32_t s = slot_of[i];
-  const int v = s == kNoKey ? -1 : voxel_of[s];
+  const uint4 held = s == kNoKey ? make_uint4(0xffffffffu, 0u, 0u, 0u) : __ldg(reinterpret_cast<const uint4*>(&slots[s]));
+  const int v = static_cast<int>(held.x);
   pc_voxel_id[i] = v;
-  if (v >= 0) list[seg[s] + place[i]] = static_cast<int>(i);
+  if (v >= 0) list[held.y + place[i]] = static_cast<int>(i);
 }
 
 // chosen[voxel, slot] = the point stored there: the slot of a point is the number of earlier points of its voxel.
 __global__ void __launch_bounds__(kVoxThreads)
-rank_kernel(const uint32_t* __restrict__ slot_of, long long n, const int* __restrict__ voxel_of, const uint32_t* __restrict__ seg,
-            const uint32_t* __restrict__ counts, const int* __restrict__ list, int max_points, int* __restrict__ chosen) {
+rank_kernel(const uint32_t* __restrict__ slot_of, long long n, const VoxSlot* __restrict__ slots, const int* __restrict__ list,
+            int max_points, int* __restrict__ chosen) {
   const long long i = blockIdx.x * static_cast<long long>(kVoxThreads) + threadIdx.x;
   if (i >= n) return;
   const uint32_t s = slot_of[i];
   if (s == kNoKey) return;
-  const int v = voxel_of[s];
+  const uint4 held = __ldg(reinterpret_cast<const uint4*>(&slots[s]));
+  const int v = static_cast<int>(held.x);
   if (v < 0) return;
-  const uint32_t c = counts[s];
+  const uint32_t c = held.z;
   int rank = 0;
   if (c > 1) {
-    const int* l = list + seg[s];
+    const int* l = list + held.y;
     for (uint32_t q = 0; q < c; ++q) rank += __ldg(&l[q]) < static_cast<int>(i);
   }
   if (rank < max_points) chosen[static_cast<long long>(v) * max_points + rank] = static_cast<int>(i);
@@ -296,37 +333,35 @@ choose_sorted_kernel(const uint32_t* __restrict__ keys, const int* __restrict__ 
   chosen[static_cast<long long>(v) * max_points + (i - lo)] = vals[i];
 }
 
-// Rows of the voxel buffer and of the caller's copy (`out`, may be null).  With `clear`: every element of every
-// row, zeros where there is no point; without: only the stored points.
-template <int VEC>
+// Rows of the voxel buffer and of the caller's copies (`out` .. `num_out`, may be null).  With `clear`: every
+// element of every row, zeros where there is no point; without: only the stored points.
+template <int VEC, typename Index>
 __global__ void __launch_bounds__(kVoxThreads)
 emit_voxels_kernel(const float* __restrict__ points, int point_stride, int num_features, const int* __restrict__ chosen,
-                   const int32_t* __restrict__ num_per_voxel, long long num_voxels, long long rows, int max_points, int clear,
-                   float* __restrict__ voxels, float* __restrict__ out) {
+                   const int32_t* __restrict__ num_per_voxel, const int32_t* __restrict__ indices, int ndim, Index num_voxels, Index rows,
+                   int max_points, int clear, float* __restrict__ voxels, float* __restrict__ out, int32_t* __restrict__ indices_out,
+                   int32_t* __restrict__ num_out) {
   struct alignas(4 * VEC) Pack { float v[VEC]; };
-  const int per = num_features / VEC;
-  const long long e = blockIdx.x * static_cast<long long>(kVoxThreads) + threadIdx.x;
-  const long long ps = e / per;  // (voxel, slot)
-  if (ps >= rows * max_points) return;
+  const Index per = static_cast<Index>(num_features / VEC);
+  const Index e = static_cast<Index>(blockIdx.x) * kVoxThreads + threadIdx.x;
+  const Index ps = e / per;  // (voxel, slot)
+  if (ps >= rows * static_cast<Index>(max_points)) return;
   const int c = static_cast<int>(e - ps * per) * VEC;
-  const long long v = ps / max_points;
-  const int slot = static_cast<int>(ps - v * max_points);
+  const Index v = ps / static_cast<Index>(max_points);
+  const int slot = static_cast<int>(ps - v * static_cast<Index>(max_points));
   Pack x;
 #pragma unroll
   for (int q = 0; q < VEC; ++q) x.v[q] = 0.f;
-  const bool have = v < num_voxels && slot < num_per_voxel[v];
-  if (have) x = *reinterpret_cast<const Pack*>(points + static_cast<long long>(chosen[ps]) * point_stride + c);
-  const long long at = ps * num_features + c;
-  if (have || clear) *reinterpret_cast<Pack*>(voxels + at) = x;
-  if (out != nullptr && v < num_voxels) *reinterpret_cast<Pack*>(out + at) = x;
-}
-
-__global__ void __launch_bounds__(kVoxThreads)
-copy_rows_kernel(const int32_t* __restrict__ a, int32_t* __restrict__ a_out, long long na, const int32_t* __restrict__ b,
-                 int32_t* __restrict__ b_out, long long nb) {
-  const long long i = blockIdx.x * static_cast<long long>(kVoxThreads) + threadIdx.x;
-  if (i < na) a_out[i] = a[i];
-  if (i < nb) b_out[i] = b[i];
+  const int stored = v < num_voxels ? num_per_voxel[v] : 0;
+  if (slot < stored) x = *reinterpret_cast<const Pack*>(points + static_cast<long long>(chosen[ps]) * point_stride + c);
+  const long long at = static_cast<long long>(ps) * num_features + c;
+  if (slot < stored || clear) *reinterpret_cast<Pack*>(voxels + at) = x;
+  if (out == nullptr || v >= num_voxels) return;
+  *reinterpret_cast<Pack*>(out + at) = x;
+  if (slot == 0 && c == 0) {
+    num_out[v] = stored;
+    for (int d = 0; d < ndim; ++d) indices_out[static_cast<long long>(v) * ndim + d] = indices[static_cast<long long>(v) * ndim + d];
+  }
 }
 
 // One thread per (voxel, feature): unused slots take the mean of the stored points,
@@ -357,7 +392,7 @@ constexpr int kVoxMostRanked = 256;
 
 struct VoxLayout {
   uint32_t cap;
-  size_t off_status, off_slots, off_counts, off_slot_of, off_place, off_voxel_of, off_seg, off_list, off_starts, off_chosen, off_sk_a,
+  size_t off_status, off_slots, off_slot_of, off_place, off_first, off_list, off_starts, off_chosen, off_sk_a,
       off_sk_b, off_sv_a, off_sv_b, off_cub, cub_bytes, total;
 };
 
@@ -376,7 +411,7 @@ size_t vox_sort_bytes(int64_t n) {
 
 VoxLayout vox_layout(int64_t n, int64_t max_voxels, int max_points) {
   VoxLayout L{};
-  L.cap = std::max<uint32_t>(vox_pow2_at_least(2 * std::max<int64_t>(n, 1)), 64);
+  L.cap = std::max<uint32_t>(vox_pow2_at_least(n + n / 2), 64);
   L.cub_bytes = vox_sort_bytes(std::max<int64_t>(n, 1));
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -387,10 +422,8 @@ VoxLayout vox_layout(int64_t n, int64_t max_voxels, int max_points) {
   const size_t np = static_cast<size_t>(std::max<int64_t>(n, 1));
   const size_t nv = static_cast<size_t>(std::min<int64_t>(std::max<int64_t>(max_voxels, 1), np));
   L.off_status = take(256);
-  L.off_slots = take(static_cast<size_t>(L.cap) * 8);
-  L.off_counts = take(static_cast<size_t>(L.cap) * 4);
-  L.off_voxel_of = take(static_cast<size_t>(L.cap) * 4);
-  L.off_seg = take(static_cast<size_t>(L.cap) * 4);
+  L.off_slots = take(static_cast<size_t>(L.cap) * sizeof(VoxSlot));
+  L.off_first = take(static_cast<size_t>(ceil_div(static_cast<int64_t>(np), kVoxBlock)) * (kVoxBlock / 8));
   L.off_slot_of = take(np * 4);
   L.off_place = take(np * 4);
   L.off_list = take(np * 4);
@@ -466,10 +499,8 @@ extern "C" int spc_voxelize_number(const float* points, int64_t n_points, int po
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   char* ws = static_cast<char*>(workspace);
   int* status = reinterpret_cast<int*>(ws + L.off_status);
-  unsigned long long* slots = reinterpret_cast<unsigned long long*>(ws + L.off_slots);
-  uint32_t* counts = reinterpret_cast<uint32_t*>(ws + L.off_counts);
-  int* voxel_of = reinterpret_cast<int*>(ws + L.off_voxel_of);
-  uint32_t* seg = reinterpret_cast<uint32_t*>(ws + L.off_seg);
+  VoxSlot* slots = reinterpret_cast<VoxSlot*>(ws + L.off_slots);
+  uint32_t* first_bits = reinterpret_cast<uint32_t*>(ws + L.off_first);
   uint32_t* slot_of = reinterpret_cast<uint32_t*>(ws + L.off_slot_of);
   uint32_t* place = reinterpret_cast<uint32_t*>(ws + L.off_place);
   uint32_t* starts = reinterpret_cast<uint32_t*>(ws + L.off_starts);
@@ -478,19 +509,18 @@ extern "C" int spc_voxelize_number(const float* points, int64_t n_points, int po
   int ticket = 0;
   rc = host_mailbox(&box, &ticket);
   if (rc != SPC_OK) return rc;
-  vox_clear_kernel<<<static_cast<unsigned>(std::min<int64_t>(ceil_div(L.cap / 2, kVoxThreads), 16ll * sm_count())), kVoxThreads, 0, st>>>(
-      reinterpret_cast<uint4*>(status), reinterpret_cast<uint4*>(slots), L.cap / 2, reinterpret_cast<uint4*>(counts), L.cap / 4);
+  vox_clear_kernel<<<static_cast<unsigned>(std::min<int64_t>(ceil_div(L.cap, kVoxThreads), 16ll * sm_count())), kVoxThreads, 0, st>>>(
+      reinterpret_cast<uint4*>(status), reinterpret_cast<uint4*>(slots), L.cap);
   SPC_LAUNCH_OK();
-  quantize_insert_kernel<<<vox_blocks(a.n), kVoxThreads, 0, st>>>(a.g, points, a.n, point_stride, slots, cap_mask, counts, slot_of, place,
-                                                               status);
+  quantize_insert_kernel<<<vox_blocks(a.n), kVoxThreads, 0, st>>>(a.g, points, a.n, point_stride, slots, cap_mask, slot_of, place, status);
   SPC_LAUNCH_OK();
   const unsigned blocks = static_cast<unsigned>(ceil_div(a.n, kVoxBlock));
-  count_first_kernel<<<blocks, kVoxThreads, 0, st>>>(slot_of, a.n, slots, counts, starts, status, box, ticket);
+  count_first_kernel<<<blocks, kVoxThreads, 0, st>>>(slot_of, a.n, slots, first_bits, starts, status, box, ticket);
   SPC_LAUNCH_OK();
-  number_voxels_kernel<<<blocks, kVoxThreads, 0, st>>>(a.g, slot_of, a.n, slots, counts, starts, max_voxels, max_points, voxel_of, seg, status,
-                                                       indices, num_per_voxel);
+  number_voxels_kernel<<<blocks, kVoxThreads, 0, st>>>(a.g, slot_of, a.n, slots, first_bits, starts, max_voxels, max_points, status, indices,
+                                                       num_per_voxel);
   SPC_LAUNCH_OK();
-  place_kernel<<<vox_blocks(a.n), kVoxThreads, 0, st>>>(slot_of, place, a.n, voxel_of, seg, reinterpret_cast<int*>(ws + L.off_list),
+  place_kernel<<<vox_blocks(a.n), kVoxThreads, 0, st>>>(slot_of, place, a.n, slots, reinterpret_cast<int*>(ws + L.off_list),
                                                      reinterpret_cast<long long*>(pc_voxel_id));
   SPC_LAUNCH_OK();
   rc = wait_for_ticket(box, ticket, st);
@@ -507,7 +537,7 @@ extern "C" int spc_voxelize_store(const float* points, int64_t n_points, int poi
                                   const int64_t* pc_voxel_id, float* voxels, float* voxels_out, int32_t* indices_out, int32_t* num_out,
                                   void* stream) {
   if (!workspace || !indices || !num_per_voxel || !voxels || n_points < 0 || num_voxels < 0 || num_voxels > max_voxels || num_features < 1 ||
-      max_points <= 0 || ndim < 1 || (n_points > 0 && (!points || !pc_voxel_id)))
+      max_points <= 0 || ndim < 1 || (n_points > 0 && (!points || !pc_voxel_id)) || (voxels_out && (!indices_out || !num_out)))
     return fail(SPC_ERR_INVALID_ARGUMENT, "voxelize: bad arguments");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const VoxLayout L = vox_layout(n_points, max_voxels, max_points);
@@ -517,8 +547,8 @@ extern "C" int spc_voxelize_store(const float* points, int64_t n_points, int poi
   int* chosen = reinterpret_cast<int*>(ws + L.off_chosen);
   if (num_voxels > 0 && !sorted) {
     rank_kernel<<<vox_blocks(n_points), kVoxThreads, 0, st>>>(
-        reinterpret_cast<uint32_t*>(ws + L.off_slot_of), n_points, reinterpret_cast<int*>(ws + L.off_voxel_of),
-        reinterpret_cast<uint32_t*>(ws + L.off_seg), reinterpret_cast<uint32_t*>(ws + L.off_counts), reinterpret_cast<int*>(ws + L.off_list),
+        reinterpret_cast<uint32_t*>(ws + L.off_slot_of), n_points, reinterpret_cast<VoxSlot*>(ws + L.off_slots),
+        reinterpret_cast<int*>(ws + L.off_list),
         max_points, chosen);
     SPC_LAUNCH_OK();
   } else if (num_voxels > 0) {
@@ -540,13 +570,18 @@ extern "C" int spc_voxelize_store(const float* points, int64_t n_points, int poi
   const bool wide = num_features % 4 == 0 && point_stride % 4 == 0 &&
                     ((reinterpret_cast<uintptr_t>(points) | reinterpret_cast<uintptr_t>(voxels) | reinterpret_cast<uintptr_t>(voxels_out)) & 15u) == 0;
   if (rows > 0) {
-    const unsigned blocks = vox_blocks(rows * max_points * (wide ? num_features / 4 : num_features));
-    if (wide)
-      emit_voxels_kernel<4><<<blocks, kVoxThreads, 0, st>>>(points, point_stride, num_features, chosen, num_per_voxel, num_voxels, rows,
-                                                           max_points, clear_voxels, voxels, voxels_out);
-    else
-      emit_voxels_kernel<1><<<blocks, kVoxThreads, 0, st>>>(points, point_stride, num_features, chosen, num_per_voxel, num_voxels, rows,
-                                                           max_points, clear_voxels, voxels, voxels_out);
+    const int64_t work = rows * max_points * (wide ? num_features / 4 : num_features);
+    const bool small = work < (1ll << 31);
+    const auto emit = [&](auto kernel, auto index) {
+      using Index = decltype(index);
+      kernel<<<vox_blocks(work), kVoxThreads, 0, st>>>(points, point_stride, num_features, chosen, num_per_voxel, indices, ndim,
+                                                      static_cast<Index>(num_voxels), static_cast<Index>(rows), max_points, clear_voxels, voxels,
+                                                      voxels_out, indices_out, num_out);
+    };
+    if (wide && small) emit(emit_voxels_kernel<4, uint32_t>, uint32_t{});
+    else if (wide) emit(emit_voxels_kernel<4, long long>, 0ll);
+    else if (small) emit(emit_voxels_kernel<1, uint32_t>, uint32_t{});
+    else emit(emit_voxels_kernel<1, long long>, 0ll);
     SPC_LAUNCH_OK();
   }
   if (num_voxels == 0) return SPC_OK;
@@ -556,11 +591,6 @@ extern "C" int spc_voxelize_store(const float* points, int64_t n_points, int poi
       fill_mean_kernel<<<vox_blocks(num_voxels * num_features), kVoxThreads, 0, st>>>(v, num_per_voxel, num_voxels, max_points, num_features);
       SPC_LAUNCH_OK();
     }
-  }
-  if (indices_out != nullptr && num_out != nullptr) {
-    copy_rows_kernel<<<vox_blocks(num_voxels * ndim), kVoxThreads, 0, st>>>(indices, indices_out, num_voxels * ndim, num_per_voxel, num_out,
-                                                                         num_voxels);
-    SPC_LAUNCH_OK();
   }
   return SPC_OK;
 }
