@@ -24,6 +24,11 @@ bool want_tc(int path, int n_dim, int r_dim, int kv, int dtype, int out_dtype, i
   return ok;
 }
 
+// (tensors of the caching allocator are; a caller's view need not be)
+bool f32_aligned(const void* a, const void* b, const void* c) {
+  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15u) == 0;
+}
+
 }  // namespace
 
 extern "C" int spc_conv_forward_needs_colmajor(int c_in, int c_out, int kv, int dtype, int out_dtype, int precision,
@@ -31,7 +36,9 @@ extern "C" int spc_conv_forward_needs_colmajor(int c_in, int c_out, int kv, int 
   const bool tma = path != SPC_GEMM_SIMT && path != SPC_GEMM_TCGEN05_CPASYNC &&
                    gather_gemm_tc_supported(c_out, c_in, kv, dtype, out_dtype, precision, false) &&
                    gather_gemm_tma_supported(c_out, c_in, kv, dtype, out_dtype, precision, false);
-  return tma ? 0 : 1;
+  if (tma) return 0;
+  const bool tc = path != SPC_GEMM_SIMT && gather_gemm_tc_supported(c_out, c_in, kv, dtype, out_dtype, precision, false);
+  return path == SPC_GEMM_AUTO && !tc && gather_gemm_f32_supported(c_out, c_in, dtype, out_dtype) ? 0 : 1;
 }
 
 extern "C" int spc_conv_forward(const void* features, const void* weight, const void* bias,
@@ -75,6 +82,10 @@ extern "C" int spc_conv_forward_residual(const void* features, const void* weigh
                           /*transposed_weight=*/false, /*reversed=*/false, dtype, out_dtype, precision, st);
   }
   if (status != SPC_OK) return status;
+  if (path == SPC_GEMM_AUTO && gather_gemm_f32_supported(c_out, c_in, dtype, out_dtype) && f32_aligned(features, weight, out))
+    return gather_gemm_f32(features, weight, epi, pair_fwd, pair_fwd_rowmajor, mask_argsort, out, n_out, c_out, c_in, kv,
+                           /*transposed_weight=*/false, /*reversed=*/false, st);
+  if (!pair_fwd) return fail(SPC_ERR_INVALID_ARGUMENT, "conv_forward: this layer reads the column-major table");
   // weight[n, k, c]: reduction index c has stride 1, output channel n stride kv*c_in.
   return gather_gemm_simt(features, weight, epi, pair_fwd, mask_argsort, out, n_out, c_out, c_in, kv,
                           /*s_wk=*/c_in, /*s_wr=*/1, /*s_wn=*/static_cast<long long>(kv) * c_in, dtype,
@@ -94,7 +105,9 @@ extern "C" int spc_conv_backward_input_needs_colmajor(int c_in, int c_out, int k
   const bool tma = path != SPC_GEMM_SIMT && path != SPC_GEMM_TCGEN05_CPASYNC &&
                    gather_gemm_tc_supported(c_in, c_out, kv, dtype, dtype, precision, true) &&
                    gather_gemm_tma_supported(c_in, c_out, kv, dtype, dtype, precision, true);
-  return tma ? 0 : 1;
+  if (tma) return 0;
+  const bool tc = path != SPC_GEMM_SIMT && gather_gemm_tc_supported(c_in, c_out, kv, dtype, dtype, precision, true);
+  return path == SPC_GEMM_AUTO && !tc && gather_gemm_f32_supported(c_in, c_out, dtype, dtype) ? 0 : 1;
 }
 
 extern "C" int spc_conv_backward_input_tables(const void* grad_out, const void* weight, const int32_t* pair_bwd,
@@ -116,6 +129,10 @@ extern "C" int spc_conv_backward_input_tables(const void* grad_out, const void* 
                           /*transposed_weight=*/true, reversed != 0, dtype, dtype, precision, st);
   }
   if (status != SPC_OK) return status;
+  if (path == SPC_GEMM_AUTO && gather_gemm_f32_supported(c_in, c_out, dtype, dtype) && f32_aligned(grad_out, weight, din))
+    return gather_gemm_f32(grad_out, weight, Epilogue{}, pair_bwd, pair_bwd_rowmajor, mask_argsort, din, n_in, c_in, c_out, kv,
+                           /*transposed_weight=*/true, reversed != 0, st);
+  if (!pair_bwd) return fail(SPC_ERR_INVALID_ARGUMENT, "conv_backward_input: this layer reads the column-major table");
   // output channel is c (stride 1), reduction index is n (stride kv*c_in); reversed offsets: from the last one down
   const char* w = static_cast<const char*>(weight) + (reversed ? static_cast<size_t>(kv - 1) * c_in * dtype_size(dtype) : 0);
   return gather_gemm_simt(grad_out, w, Epilogue{}, pair_bwd, mask_argsort, din, n_in, c_in, c_out, kv,
@@ -126,7 +143,8 @@ extern "C" int spc_conv_backward_input_tables(const void* grad_out, const void* 
 extern "C" size_t spc_conv_backward_weight_workspace_bytes(int64_t n_out, int c_in, int c_out, int kv) {
   if (n_out < 0 || c_in <= 0 || c_out <= 0 || kv <= 0) return 0;
   // enough for whichever kernel the call ends up using
-  return std::max(wgrad_split(n_out, c_in, c_out, kv).bytes, wgrad_tc_split(n_out, c_in, c_out, kv).bytes);
+  return std::max(std::max(wgrad_split(n_out, c_in, c_out, kv).bytes, wgrad_f32_split(n_out, c_in, c_out, kv).bytes),
+                  wgrad_tc_split(n_out, c_in, c_out, kv).bytes);
 }
 
 extern "C" int spc_conv_backward_weight(const void* features, const void* grad_out, const int32_t* pair_fwd,
@@ -156,6 +174,14 @@ extern "C" int spc_conv_backward_weight(const void* features, const void* grad_o
   if (path == SPC_GEMM_TCGEN05)
     return fail(SPC_ERR_UNSUPPORTED, "conv_backward_weight: the tcgen05 kernel does not take this shape/dtype "
                 "(c_in=%d c_out=%d dtype=%d)", c_in, c_out, dtype);
+  if (path == SPC_GEMM_AUTO && wgrad_f32_supported(c_in, c_out, dtype) && f32_aligned(features, grad_out, workspace)) {
+    const WgradSplit fs = wgrad_f32_split(n_out, c_in, c_out, kv);
+    if (!workspace || workspace_bytes < fs.bytes)
+      return fail(SPC_ERR_WORKSPACE_TOO_SMALL, "conv_backward_weight: workspace %zu < %zu bytes", workspace_bytes, fs.bytes);
+    const int rc = wgrad_f32(features, grad_out, pair_fwd, static_cast<float*>(workspace), n_out, c_in, c_out, kv, fs, st);
+    if (rc != SPC_OK) return rc;
+    return wgrad_reduce(static_cast<const float*>(workspace), dweight, static_cast<long long>(c_out) * kv * c_in, fs.splits, dtype, st);
+  }
   const WgradSplit s = wgrad_split(n_out, c_in, c_out, kv);
   if (!workspace || workspace_bytes < s.bytes)
     return fail(SPC_ERR_WORKSPACE_TOO_SMALL, "conv_backward_weight: workspace %zu < %zu bytes", workspace_bytes,

@@ -27,6 +27,16 @@ WgradSplit wgrad_split(int64_t n_out, int c_in, int c_out, int kv);
 int wgrad_simt(const void* feats, const void* gout, const int32_t* pair_fwd, void* dw, float* partial,
                int64_t n_out, int c_in, int c_out, int kv, int dtype, cudaStream_t st);
 
+// IEEE fp32 kernels for channel counts that are multiples of four (gemm_f32.cu).
+bool gather_gemm_f32_supported(int n_dim, int r_dim, int dtype, int out_dtype);
+int gather_gemm_f32(const void* src, const void* w, const Epilogue& epi, const int32_t* pairs, const int32_t* pairs_rowmajor,
+                    const int32_t* order, void* out, long long m_rows, int n_dim, int r_dim, int kv, bool transposed_weight, bool reversed,
+                    cudaStream_t st);
+bool wgrad_f32_supported(int c_in, int c_out, int dtype);
+WgradSplit wgrad_f32_split(int64_t n_out, int c_in, int c_out, int kv);
+int wgrad_f32(const void* feats, const void* gout, const int32_t* pair_fwd, float* partial, int64_t n_out, int c_in, int c_out, int kv,
+              const WgradSplit& split, cudaStream_t st);
+
 // tcgen05 kernels (gemm_tc.cu).  `transposed_weight` selects the input-gradient
 // view of the KRSC weight; `reversed`: offset k of the table meets weight kv - 1 - k.  Return SPC_ERR_UNSUPPORTED for shapes they do not take.
 bool gather_gemm_tc_supported(int n_dim, int r_dim, int kv, int dtype, int out_dtype, int precision,
