@@ -788,9 +788,19 @@ __device__ __forceinline__ void count_buckets(int bucket, int* slot_bucket, uint
 // on L2 latency otherwise (32 us for 2 000 rows with one line at a time).  The first of three axes stays a
 // loop, and a hash chain is followed in a loop of its own: unrolled completely the code no longer fits the
 // instruction cache, and on few rows fetching it is what takes the time (20 us for the same rows).
+//
+// A plane is the K * K offsets of the last two axes; one call looks a slab of planes up, at most 32 offsets,
+// which is what the shared tile holds: all of a 3x3x3 kernel, a plane of a 5x5x5 one, 27 of 81 in four dimensions.
+template <int ND, int K>
+struct Cube {
+  static constexpr int plane = ND == 1 ? K : K * K;
+  static constexpr int planes = ND <= 2 ? 1 : ND == 3 ? K : K * K;
+  static constexpr int together = plane * planes <= 32 ? planes : plane * K <= 32 ? K : 1;  // planes of a slab
+  static constexpr int slab = plane * together;
+};
 template <int ND, bool K64, int K, typename Emit>
 __device__ __forceinline__ void look_up_cube(const Geo& g, bool div, const int* own, const int* limit,
-                                             const Table<K64>& table, const Emit& emit) {
+                                             const Table<K64>& table, int first_plane, const Emit& emit) {
   using key_t = typename Table<K64>::key_t;
   constexpr int kLast = ND - 1, kMid = ND >= 2 ? ND - 2 : 0;
   constexpr int kLinesHere = ND == 1 ? 1 : K;
@@ -810,14 +820,20 @@ __device__ __forceinline__ void look_up_cube(const Geo& g, bool div, const int* 
   const uint32_t* prefix = dense_prefix(table);
   const int32_t* perm = row_permutation(table);
 #pragma unroll 1
-  for (int p = 0; p < (ND == 3 ? K : 1); ++p) {
+  for (int p = first_plane; p < first_plane + Cube<ND, K>::together; ++p) {
     key_t lead = static_cast<key_t>(own[0]);
-    if (ND == 3) {
-      const int x0 = axis_cell(g, div, 0, own[1], p, limit[0]);
+    if (ND == 4) {
+      const int x0 = axis_cell(g, div, 0, own[1], p / K, limit[0]);
       if (x0 < 0) continue;
       lead = lead * static_cast<key_t>(limit[0]) + static_cast<key_t>(x0);
     }
-    const int k0 = p * K * K;
+    if (ND >= 3) {
+      constexpr int kAxis = ND >= 3 ? ND - 3 : 0;
+      const int x0 = axis_cell(g, div, kAxis, own[kAxis + 1], p % K, limit[kAxis]);
+      if (x0 < 0) continue;
+      lead = lead * static_cast<key_t>(limit[kAxis]) + static_cast<key_t>(x0);
+    }
+    const int k0 = p * Cube<ND, K>::plane;
     key_t base[kLinesHere];
 #pragma unroll
     for (int l = 0; l < kLinesHere; ++l)
@@ -872,10 +888,11 @@ __device__ __forceinline__ void look_up_cube(const Geo& g, bool div, const int* 
 #pragma unroll
         for (int k = 0; k < K; ++k) {
           const int q = l * K + k;
-          if (probe[q] == Table<K64>::kEmpty) continue;
           int j;
-          if (table.settled(base[l] + static_cast<key_t>(xl[k]), probe[q], &j)) emit(k0 + q, j);
-          else far |= 1u << q;
+          const bool taken = probe[q] != Table<K64>::kEmpty;
+          const bool own_key = table.settled(base[l] + static_cast<key_t>(xl[k]), probe[q], &j) && taken;
+          emit(k0 + q, own_key ? j : -1);
+          far |= static_cast<uint32_t>(taken && !own_key) << q;
         }
 #pragma unroll 1
       for (; far != 0; far &= far - 1) {
@@ -938,9 +955,11 @@ fill_kernel(const __grid_constant__ Geo g, const int32_t* __restrict__ idx, long
     x_span = (xa < xb ? xb : xa) - x_lo;
   }
   uint32_t order_word = 0;
-  for (int c0 = 0; c0 < g.kv; c0 += 32) {
+  constexpr int kPiece = K == 0 ? 32 : Cube<ND, K == 0 ? 1 : K>::slab;  // offsets looked up and written at a time
+  // (the pieces of a large kernel are dealt over grid.y: a few thousand rows fill the chip only together with them)
+  for (int c0 = static_cast<int>(blockIdx.y) * kPiece; c0 < g.kv; c0 += kPiece * static_cast<int>(gridDim.y)) {
     const int width = min(32, kvp - c0);           // entries of a row in this piece, a multiple of four
-    const int c1 = min(g.kv, c0 + 32);
+    const int c1 = min(g.kv, c0 + kPiece);
     __syncwarp();  // the previous piece has been copied out
     {
       const int4 none = make_int4(-1, -1, -1, -1);
@@ -949,19 +968,24 @@ fill_kernel(const __grid_constant__ Geo g, const int32_t* __restrict__ idx, long
     __syncwarp();
     uint32_t word = 0;
     auto emit = [&](int k, int j) {
-      if (k < c0 || k >= c1 || j < 0 || (BWD && j >= n_limit)) return;
-      mine[k - c0] = j;
-      word |= 1u << (k - c0);
-      if (out.keys != nullptr) order_word |= 1u << g.key_pos[k];
-      if (BWD && out.out_rm != nullptr)
-        atomicMin(reinterpret_cast<unsigned*>(&out.out_rm[static_cast<long long>(j) * kvp + k]), static_cast<unsigned>(r));
-      if (BWD && out.out_cm != nullptr)
-        atomicMin(reinterpret_cast<unsigned*>(&out.out_cm[k * n_limit + j]), static_cast<unsigned>(r));
-      if (BWD && out.out_words != nullptr)
-        atomicOr(&out.out_words[static_cast<long long>(j) * mic + (k >> 5)], 1u << (out.order_bits ? g.key_pos[k] : (k & 31)));
+      if constexpr (K != 0 && !BWD) {
+        // every entry is stored, absent ones too: no branch, so the lanes of a warp stay together
+        mine[k - c0] = j;
+        word |= static_cast<uint32_t>(j >= 0) << (k - c0);
+      } else {
+        if ((K == 0 && (k < c0 || k >= c1)) || j < 0 || (BWD && j >= n_limit)) return;
+        mine[k - c0] = j;
+        word |= 1u << (k - c0);
+        if (BWD && out.out_rm != nullptr)
+          atomicMin(reinterpret_cast<unsigned*>(&out.out_rm[static_cast<long long>(j) * kvp + k]), static_cast<unsigned>(r));
+        if (BWD && out.out_cm != nullptr)
+          atomicMin(reinterpret_cast<unsigned*>(&out.out_cm[k * n_limit + j]), static_cast<unsigned>(r));
+        if (BWD && out.out_words != nullptr)
+          atomicOr(&out.out_words[static_cast<long long>(j) * mic + (k >> 5)], 1u << (out.order_bits ? g.key_pos[k] : (k & 31)));
+      }
     };
     if constexpr (K != 0) {
-      if (ok) look_up_cube<ND, K64, K>(g, div, own, limit, table, emit);
+      if (ok) look_up_cube<ND, K64, K>(g, div, own, limit, table, c0 / Cube<ND, K>::plane, emit);
     } else if (ok && g.axes_fit && q_hi >= 0) {
       int pos[ND];  // offsets of the leading axes
       const int l0 = c0 / kl, l1 = (c1 - 1) / kl;
@@ -1078,11 +1102,19 @@ fill_kernel(const __grid_constant__ Geo g, const int32_t* __restrict__ idx, long
       }
     }
     if (live && out.words != nullptr) out.words[r * mic + (c0 >> 5)] = word;
+    if (out.keys != nullptr)  // (one piece)
+      for (uint32_t m = word; m != 0; m &= m - 1) order_word |= 1u << g.key_pos[__ffs(m) - 1];
     __syncwarp();
     const int rows = static_cast<int>(n - row0 < 32 ? (n - row0 > 0 ? n - row0 : 0) : 32);
     if (out.rm != nullptr) {
       const int quads = width / 4;
-      if (pitch == kvp) {
+      if (kPiece != 32 && g.kv > kPiece) {
+        // pieces that do not start at multiples of four entries: a row's are written by consecutive lanes
+        for (int row = 0; row < rows; ++row)
+          if (lane < c1 - c0) out.rm[(row0 + row) * kvp + c0 + lane] = tile[row * pitch + lane];
+        if (c1 == g.kv && live)
+          for (int k = g.kv; k < kvp; ++k) out.rm[r * kvp + k] = -1;
+      } else if (pitch == kvp) {
         int4* dst = reinterpret_cast<int4*>(out.rm + row0 * kvp);
         for (int i = lane; i < rows * quads; i += 32) dst[i] = reinterpret_cast<const int4*>(tile)[i];
       } else {
@@ -1460,7 +1492,9 @@ Layout make_layout(const Geo& g, int64_t n_in) {
     L.ibits_words = static_cast<int64_t>(vol_in / 32.0) + 1;
   // the output bitmap also numbers the outputs, which a hash table needs a sort for
   if (!g.subm && !L.k64 && vol_out <= max_bits) L.obits_words = static_cast<int64_t>(vol_out / 32.0) + 1;
-  L.cap_in = !g.subm || L.ibits_words ? 0 : pow2_at_least(4 * n_in);  // load <= 0.25: most look-ups miss, keep their probe chains short
+  // Most look-ups miss, so a loaded table costs probe chains, which a warp follows one after the other: a sixteenth
+  // full while that is a few MB to clear (2 000 rows: the look-up 17 -> 11 us), a quarter beyond.
+  L.cap_in = !g.subm || L.ibits_words ? 0 : pow2_at_least((n_in <= 32768 ? 16 : 4) * n_in);
   L.cap_out = g.subm || L.obits_words ? 0 : pow2_at_least(2 * L.bound);
   const int64_t n_max = std::max<int64_t>(n_in, L.bound);
   L.n_blocks_native = ceil_div(std::max<int64_t>(n_in, 1), kThreads);
@@ -1741,11 +1775,14 @@ int emit_masks(const Layout& L, char* ws, int64_t n, int kv, const uint32_t* spl
   return SPC_OK;
 }
 
-// Kernel width of a cube-shaped kernel with a fill kernel of its own, else 0.
-int cube_width(const Geo& g) {
+// Kernel width of a cube-shaped kernel with a fill kernel of its own, else 0.  (The mask words of several
+// pieces start at multiples of 32 offsets, which the pieces of these kernels do not.)
+int cube_width(const Geo& g, bool words) {
   for (int d = 0; d < g.ndim; ++d)
     if (g.ksize[d] != g.ksize[0] || g.dil[d] != 1) return 0;
-  return g.ndim <= 3 && (g.ksize[0] == 2 || g.ksize[0] == 3) ? g.ksize[0] : 0;
+  const int k = g.ksize[0];
+  if (words && g.kv > 32) return 0;
+  return k == 2 || k == 3 || (k == 5 && g.ndim <= 3) ? k : 0;
 }
 size_t fill_smem_bytes(int kvp) { return static_cast<size_t>(kThreads / 32) * 32 * fill_pitch(kvp) * 4; }
 
@@ -1755,15 +1792,16 @@ int launch_fill(const Geo& g, const int32_t* idx, int64_t n, int64_t n_limit, co
   const int kvp = (g.kv + 3) & ~3;
   const unsigned blocks = blocks_for(n);
   const size_t smem = fill_smem_bytes(kvp);
-  const int width = cube_width(g);
-  if constexpr (ND <= 3) {
-    if (width == 3)
-      fill_kernel<ND, K64, BWD, 3><<<blocks, kThreads, smem, st>>>(g, idx, n, n_limit, table, out, mic, kvp);
-    else if (width == 2 && BWD)  // (submanifold kernels are odd)
-      fill_kernel<ND, K64, BWD, BWD ? 2 : 0><<<blocks, kThreads, smem, st>>>(g, idx, n, n_limit, table, out, mic, kvp);
-  }
-  if (ND > 3 || width == 0 || (width == 2 && !BWD))
-    fill_kernel<ND, K64, BWD, 0><<<blocks, kThreads, smem, st>>>(g, idx, n, n_limit, table, out, mic, kvp);
+  const auto launch = [&](auto width) {
+    constexpr int K = decltype(width)::value;
+    const int pieces = K == 0 ? 1 : g.kv / Cube<ND, K == 0 ? 1 : K>::slab;
+    fill_kernel<ND, K64, BWD, K><<<dim3(blocks, static_cast<unsigned>(pieces)), kThreads, smem, st>>>(g, idx, n, n_limit, table, out, mic, kvp);
+  };
+  const int width = cube_width(g, out.words != nullptr || out.out_words != nullptr);
+  if (width == 3) launch(std::integral_constant<int, 3>{});
+  else if (width == 2 && BWD) launch(std::integral_constant<int, BWD ? 2 : 0>{});  // (submanifold kernels are odd)
+  else if (ND <= 3 && width == 5) launch(std::integral_constant<int, ND <= 3 ? 5 : 0>{});
+  else launch(std::integral_constant<int, 0>{});
   SPC_LAUNCH_OK();
   return SPC_OK;
 }
