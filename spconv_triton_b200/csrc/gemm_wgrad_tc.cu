@@ -6,8 +6,10 @@
 // For one kernel offset k this is a dense contraction D[n, c] = G^T F over the
 // list of existing (output row, input row) pairs, with the pairs as the
 // reduction dimension.  One CTA owns (offset k, a contiguous range of output
-// rows, a block of <= 128 output channels) and keeps D (128 lanes x c_in fp32
-// columns) in tensor memory:
+// rows, one or two blocks of <= 128 output channels) and keeps D (128 lanes x
+// c_in fp32 columns a block) in tensor memory; with 256 output channels both
+// blocks multiply the same feature rows, which two CTAs would gather twice
+// (k5 256 -> 256, 13.6 M pairs: 5.5 -> 3.9 ms):
 //   warps 0-7  scan pair_fwd[k, lo:hi] 256 entries at a time, compact the
 //              existing pairs into a shared-memory ring with warp ballots (no
 //              host-side nonzero(), unlike spconv_triton/pytorch/_impl/gemm.py:663),
@@ -48,7 +50,8 @@ struct WgParams {
   long long n_out, rows_per_split;
   int c_in, c_out, kv, splits;
   int g_row_bytes, f_row_bytes;  // swizzle span of the grad_out / feature rows (32, 64 or 128)
-  int g_stage_bytes, f_stage_bytes, stages, tmem_cols;
+  int n_blocks;  // blocks of 128 output channels of a CTA
+  int g_stage_bytes, f_stage_bytes, stages, tmem_cols, cols;
   int* status;
 };
 
@@ -56,39 +59,42 @@ __host__ __device__ inline uint32_t wg_layout_type(int row_bytes) {
   return row_bytes == 128 ? 2u : (row_bytes == 64 ? 4u : 6u);
 }
 
-// Copies `pieces_per_row` 16-byte pieces of `n_rows` gathered rows into an
-// MN-major stage region: column block b of row p lands at
-// base + b * (kPairsPerStage * row_bytes) + p * row_bytes (+ swizzle).
-template <int ELEM>
-__device__ __forceinline__ void copy_rows(uint32_t dst_base, const uint8_t* src, uint32_t src_pitch,
-                                          const int* rows, int n_rows, int n_rows_padded, int pieces_per_row,
-                                          int row_bytes, int tid, int nthreads) {
+// Copies `pieces` 16-byte pieces of each of `n` gathered rows into an MN-major stage region: column block b
+// of row p lands at base + b * (kPairsPerStage * row_bytes) + p * row_bytes (+ swizzle); rows n .. n_pad are
+// zero filled.  A thread keeps its piece and steps over the rows by a multiple of eight, the period of the
+// swizzle, so that a copy costs it one list read and two additions.
+template <int THREADS>
+__device__ __forceinline__ void copy_rows(uint32_t dst_base, const uint8_t* src, uint32_t src_pitch, const int* rows, int n, int n_pad,
+                                          int pieces, int row_bytes, int tid) {
   const int per_block = row_bytes / 16;  // 2, 4 or 8
   const uint32_t swz_mask = static_cast<uint32_t>(per_block - 1);
   const int lg_pb = per_block == 8 ? 3 : (per_block == 4 ? 2 : 1);
-  const int total = n_rows_padded * pieces_per_row;
-  const bool pow2 = (pieces_per_row & (pieces_per_row - 1)) == 0;
-  const int lg_ppr = 31 - __clz(pieces_per_row);
-  for (int q = tid; q < total; q += nthreads) {
-    int p, piece;
-    if (pow2) {  // the usual case: no integer division per copy
-      p = q >> lg_ppr;
-      piece = q & (pieces_per_row - 1);
-    } else {
-      p = q / pieces_per_row;
-      piece = q - p * pieces_per_row;
+  const auto place = [&](int p, int piece) {
+    const uint32_t lin = static_cast<uint32_t>(p * row_bytes + (piece & (per_block - 1)) * 16);
+    return static_cast<uint32_t>((piece >> lg_pb) * kPairsPerStage * row_bytes) + (lin ^ (((lin >> 7) & swz_mask) << 4));
+  };
+  const int step = THREADS / pieces;
+  if ((pieces & (pieces - 1)) == 0 && step >= 8) {
+    const int lg = 31 - __clz(pieces);
+    const int p0 = tid >> lg, piece = tid & (pieces - 1);
+    uint32_t dst = dst_base + place(p0, piece);
+    const uint32_t dst_step = static_cast<uint32_t>(step * row_bytes);
+    const uint8_t* at = src + piece * 16;
+    for (int p = p0; p < n_pad; p += step, dst += dst_step) {
+      const uint32_t row = p < n ? static_cast<uint32_t>(rows[p]) : 0u;
+      cp_async16(dst, at + static_cast<unsigned long long>(row) * src_pitch, p < n ? 16u : 0u);
     }
-    const int block = piece >> lg_pb, chunk = piece & (per_block - 1);
-    const uint32_t lin = static_cast<uint32_t>(p * row_bytes + chunk * 16);
-    const uint32_t off = static_cast<uint32_t>(block * kPairsPerStage * row_bytes) + (lin ^ (((lin >> 7) & swz_mask) << 4));
-    const bool live = p < n_rows;
-    const uint32_t row = live ? static_cast<uint32_t>(rows[p]) : 0u;
-    cp_async16(dst_base + off, src + static_cast<unsigned long long>(row) * src_pitch + piece * 16, live ? 16u : 0u);
+    return;
+  }
+  for (int q = tid; q < n_pad * pieces; q += THREADS) {
+    const int p = q / pieces, piece = q - p * pieces;
+    const uint32_t row = p < n ? static_cast<uint32_t>(rows[p]) : 0u;
+    cp_async16(dst_base + place(p, piece), src + static_cast<unsigned long long>(row) * src_pitch + piece * 16, p < n ? 16u : 0u);
   }
 }
 
 template <typename T, int W>
-__global__ void __maxnreg__(W == 4 ? 96 : 80)
+__global__ void __launch_bounds__(W * 32 + 32, W == 4 ? 3 : 1)
 wgrad_tc_kernel(const __grid_constant__ WgParams p) {
   constexpr int kWgIssueWarps = W;
   constexpr int kWgIssueThreads = W * 32;
@@ -114,7 +120,7 @@ wgrad_tc_kernel(const __grid_constant__ WgParams p) {
   const int warp = tid >> 5, lane = tid & 31;
   if (*reinterpret_cast<volatile int*>(p.status) != 0) return;
   const int k = blockIdx.x / p.splits, split = blockIdx.x % p.splits;
-  const int n0 = blockIdx.y * kTileM;  // first output channel of this CTA
+  const int n0 = blockIdx.y * p.n_blocks * kTileM;  // first output channel of this CTA
   const long long lo = split * p.rows_per_split;
   const long long hi = min(p.n_out, lo + p.rows_per_split);
   const uint32_t bar_full = smem_u32(bars);
@@ -145,7 +151,7 @@ wgrad_tc_kernel(const __grid_constant__ WgParams p) {
     bool ok = true;
     int head = 0, tail = 0;  // ring positions (uniform over the 256 threads)
     long long pos = lo;
-    const int g_cols = min(kTileM, p.c_out - n0);          // output channels this CTA owns
+    const int g_cols = min(p.n_blocks * kTileM, p.c_out - n0);  // output channels this CTA owns
     const int g_pieces = g_cols * ELEM / 16;
     const int f_pieces = p.c_in * ELEM / 16;
     const uint8_t* g_src = static_cast<const uint8_t*>(p.gout) + static_cast<size_t>(n0) * ELEM;
@@ -219,8 +225,8 @@ wgrad_tc_kernel(const __grid_constant__ WgParams p) {
         const uint32_t g_dst = smem_u32(stage_base + static_cast<size_t>(stage) * stage_bytes);
         const uint32_t f_dst = g_dst + p.g_stage_bytes;
         const uint32_t full = bar_full + 8 * stage;
-        copy_rows<ELEM>(g_dst, g_src, g_pitch, sm, n, n_pad, g_pieces, p.g_row_bytes, tid, kWgIssueThreads);
-        copy_rows<ELEM>(f_dst, f_src, f_pitch, si, n, n_pad, f_pieces, p.f_row_bytes, tid, kWgIssueThreads);
+        copy_rows<kWgIssueThreads>(g_dst, g_src, g_pitch, sm, n, n_pad, g_pieces, p.g_row_bytes, tid);
+        copy_rows<kWgIssueThreads>(f_dst, f_src, f_pitch, si, n, n_pad, f_pieces, p.f_row_bytes, tid);
         cp_async_arrive_noinc(full);
         if (tid == 0) {
           info[stage].ksteps = n_pad / UMMA_K;
@@ -257,22 +263,24 @@ wgrad_tc_kernel(const __grid_constant__ WgParams p) {
       have_acc = __all_sync(0xffffffffu, have_acc);
       tc_fence_after();
       if (have_acc) {
-        const int n = n0 + tid;  // output channel held by this TMEM lane
-        float* dst = p.partial + ((static_cast<long long>(split) * p.c_out + (n < p.c_out ? n : 0)) * p.kv + k) * p.c_in;
         const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
-        for (int c0 = 0; c0 < p.c_in; c0 += 16) {
-          float v[16];
-          if (real_stages > 0) {
-            uint32_t raw[16];
-            tmem_ld16(lane_addr + c0, raw);
-            tmem_ld_wait();
+        for (int b = 0; b < p.n_blocks; ++b) {
+          const int n = n0 + b * kTileM + tid;  // output channel held by this TMEM lane
+          float* dst = p.partial + ((static_cast<long long>(split) * p.c_out + (n < p.c_out ? n : 0)) * p.kv + k) * p.c_in;
+          for (int c0 = 0; c0 < p.c_in; c0 += 16) {
+            float v[16];
+            if (real_stages > 0) {
+              uint32_t raw[16];
+              tmem_ld16(lane_addr + b * p.cols + c0, raw);
+              tmem_ld_wait();
 #pragma unroll
-            for (int q = 0; q < 16; ++q) v[q] = __uint_as_float(raw[q]);
-          } else {
+              for (int q = 0; q < 16; ++q) v[q] = __uint_as_float(raw[q]);
+            } else {
 #pragma unroll
-            for (int q = 0; q < 16; ++q) v[q] = 0.f;
+              for (int q = 0; q < 16; ++q) v[q] = 0.f;
+            }
+            if (n < p.c_out) store_row16<float>(dst + c0, v);
           }
-          if (n < p.c_out) store_row16<float>(dst + c0, v);
         }
       }
       tc_fence_before();
@@ -294,6 +302,7 @@ wgrad_tc_kernel(const __grid_constant__ WgParams p) {
       const uint32_t stage_step = static_cast<uint32_t>(stage_bytes >> 4);
       const uint32_t a_step = static_cast<uint32_t>(UMMA_K * p.g_row_bytes / 16);
       const uint32_t b_step = static_cast<uint32_t>(UMMA_K * p.f_row_bytes / 16);
+      const uint32_t a_block = static_cast<uint32_t>(kTileM * ELEM * kPairsPerStage / 16);  // 128 channels of a stage's rows
       const uint32_t info0 = smem_u32(info);
       uint32_t a_lo = a_lo0, b_lo = b_lo0, full = bar_full, empty = bar_empty, inf = info0;
       int stage = 0;
@@ -312,15 +321,18 @@ wgrad_tc_kernel(const __grid_constant__ WgParams p) {
           tc_commit(bar_accum);
           break;
         }
+        for (int b = 0; b < p.n_blocks; ++b) {
+          const uint32_t d = tmem_base + static_cast<uint32_t>(b * p.cols), a_at = a_lo + b * a_block;
 #pragma unroll
-        for (int ks = 0; ks < kPairsPerStage / UMMA_K; ++ks) {
-          if (static_cast<uint32_t>(ks) < ksteps) {
-            const uint64_t a_desc = (static_cast<uint64_t>(a_hi) << 32) | (a_lo + a_step * ks);
-            const uint64_t b_desc = (static_cast<uint64_t>(b_hi) << 32) | (b_lo + b_step * ks);
-            tc_mma<false>(tmem_base, a_desc, b_desc, idesc, accumulate);
-            accumulate = 1;
+          for (int ks = 0; ks < kPairsPerStage / UMMA_K; ++ks) {
+            if (static_cast<uint32_t>(ks) < ksteps) {
+              const uint64_t a_desc = (static_cast<uint64_t>(a_hi) << 32) | (a_at + a_step * ks);
+              const uint64_t b_desc = (static_cast<uint64_t>(b_hi) << 32) | (b_lo + b_step * ks);
+              tc_mma<false>(d, a_desc, b_desc, idesc, ks == 0 ? accumulate : 1u);
+            }
           }
         }
+        accumulate = 1;
         tc_commit(empty);
         a_lo += stage_step;
         b_lo += stage_step;
@@ -352,18 +364,20 @@ wgrad_tc_kernel(const __grid_constant__ WgParams p) {
   }
 }
 
+// Swizzle span of rows of `elems` channels: the widest of 128, 64 and 32 bytes that divides them.
 int span_of(int elems, int elem_size) {
   const int bytes = elems * elem_size;
-  if (bytes == 32 || bytes == 64) return bytes;
-  if (bytes >= 128 && bytes % 128 == 0) return 128;
-  return 0;
+  return bytes % 128 == 0 ? 128 : bytes % 64 == 0 ? 64 : bytes % 32 == 0 ? 32 : 0;
 }
+
+// Blocks of 128 output channels a CTA takes (two fill tensor memory at 256 input channels: one CTA per SM).
+int wg_blocks(int c_out) { return c_out % (2 * tc::kTileM) == 0 ? 2 : 1; }
 
 template <typename T, int W>
 int launch_wgrad_tc(const WgParams& p, size_t smem_bytes, cudaStream_t st) {
   static bool configured[kMaxDevices] = {false};  // per instantiation and device
-  SPC_CUDA_OK(ensure_dynamic_smem(wgrad_tc_kernel<T, W>, 200 * 1024, configured));
-  dim3 grid(static_cast<unsigned>(p.kv * p.splits), static_cast<unsigned>(ceil_div(p.c_out, kTileM)));
+  SPC_CUDA_OK(ensure_dynamic_smem(wgrad_tc_kernel<T, W>, 226 * 1024, configured));
+  dim3 grid(static_cast<unsigned>(p.kv * p.splits), static_cast<unsigned>(ceil_div(p.c_out, p.n_blocks * kTileM)));
   wgrad_tc_kernel<T, W><<<grid, W * 32 + 32, smem_bytes, st>>>(p);
   SPC_LAUNCH_OK();
   return SPC_OK;
@@ -385,7 +399,7 @@ bool wgrad_tc_supported(int c_in, int c_out, int kv, int dtype) {
 // tensor-core tile (128 output channels x all input channels per CTA).
 WgradSplit wgrad_tc_split(int64_t n_out, int c_in, int c_out, int kv) {
   WgradSplit s;
-  const int64_t tiles = static_cast<int64_t>(kv) * ceil_div(c_out, tc::kTileM);
+  const int64_t tiles = static_cast<int64_t>(kv) * ceil_div(c_out, wg_blocks(c_out) * tc::kTileM);
   // several CTAs per resident slot: offsets differ a lot in how many pairs they have (the centre
   // offset of a submanifold layer has all of them), and surplus CTAs even that out
   int64_t want = ceil_div(16 * static_cast<int64_t>(sm_count()), std::max<int64_t>(tiles, 1));
@@ -405,23 +419,24 @@ int wgrad_tc(const void* feats, const void* gout, const int32_t* pair_fwd, float
   WgParams p{};
   p.feats = feats; p.gout = gout; p.pair_fwd = pair_fwd; p.partial = partial;
   p.n_out = n_out; p.rows_per_split = split.rows_per_split; p.splits = split.splits;
-  p.c_in = c_in; p.c_out = c_out; p.kv = kv;
+  p.c_in = c_in; p.c_out = c_out; p.kv = kv; p.n_blocks = wg_blocks(c_out);
   const int g_cols = std::min(c_out, tc::kTileM);
   p.g_row_bytes = span_of(g_cols, 2);
   p.f_row_bytes = span_of(c_in, 2);
   // the A region always spans 128 channels (M = 128); columns beyond c_out hold stale data
-  p.g_stage_bytes = static_cast<int>(align_up(static_cast<size_t>(tc::kTileM) * 2 * kPairsPerStage, 1024));
+  p.g_stage_bytes = static_cast<int>(align_up(static_cast<size_t>(p.n_blocks) * tc::kTileM * 2 * kPairsPerStage, 1024));
   p.f_stage_bytes = static_cast<int>(align_up(static_cast<size_t>(c_in) * 2 * kPairsPerStage, 1024));
   const int stage_bytes = p.g_stage_bytes + p.f_stage_bytes;
   const size_t fixed = 1024 + 2 * kRing * 4 + 2 * tc::kMaxStages * kPairsPerStage * 4 + (2 * tc::kMaxStages + 1) * 8 +
                        tc::kMaxStages * sizeof(tc::StageInfo) + kScanBatch * kWgMaxIssueWarps * 4 + 64;
-  const bool narrow = (c_in + g_cols) * 2 <= 384;  // bytes of rows per pair
-  const size_t budget = narrow ? 74 * 1024 : 110 * 1024;  // three / two CTAs per SM
+  const bool narrow = (c_in + p.n_blocks * g_cols) * 2 <= 384;  // bytes of rows per pair
+  p.cols = 32;
+  while (p.cols < c_in) p.cols <<= 1;
+  // three, two or (two blocks of 256 columns) one CTA per SM
+  const size_t budget = narrow ? 74 * 1024 : p.n_blocks * p.cols > 256 ? 222 * 1024 : 110 * 1024;
   p.stages = std::max(2, std::min<int>(tc::kMaxStages, static_cast<int>((budget - fixed) / stage_bytes)));
   const size_t smem_bytes = fixed + static_cast<size_t>(p.stages) * stage_bytes;
-  int cols = 32;
-  while (cols < c_in) cols <<= 1;
-  p.tmem_cols = cols;
+  p.tmem_cols = p.n_blocks * p.cols;
   p.status = device_status_ptr();
   if (p.status == nullptr) return fail(SPC_ERR_CUDA, "tcgen05 wgrad: no device status word");
   if (narrow) {
