@@ -39,7 +39,6 @@ using namespace tc;
 // is at most 384 bytes of rows, eight (two CTAs per SM) for wider rows, which need the copy throughput.
 constexpr int kWgMaxIssueWarps = 8;
 constexpr int kPairsPerStage = 64;
-constexpr int kScanBatch = 4;                        // table entries per thread per scan round
 constexpr int kRing = 2048;                          // capacity of the pair list (power of two, > 64 + 1024)
 
 struct WgParams {
@@ -59,47 +58,53 @@ __host__ __device__ inline uint32_t wg_layout_type(int row_bytes) {
   return row_bytes == 128 ? 2u : (row_bytes == 64 ? 4u : 6u);
 }
 
-// Copies `pieces` 16-byte pieces of each of `n` gathered rows into an MN-major stage region: column block b
-// of row p lands at base + b * (kPairsPerStage * row_bytes) + p * row_bytes (+ swizzle); rows n .. n_pad are
-// zero filled.  A thread keeps its piece and steps over the rows by a multiple of eight, the period of the
-// swizzle, so that a copy costs it one list read and two additions.
-template <int THREADS>
-__device__ __forceinline__ void copy_rows(uint32_t dst_base, const uint8_t* src, uint32_t src_pitch, const int* rows, int n, int n_pad,
-                                          int pieces, int row_bytes, int tid) {
+// Copies 16-byte pieces of gathered rows into an MN-major stage region: column block b of row p lands at
+// base + b * (kPairsPerStage * row_bytes) + p * row_bytes (+ swizzle); rows n .. n_pad are zero filled.
+__device__ __forceinline__ uint32_t piece_place(int p, int piece, int row_bytes) {
   const int per_block = row_bytes / 16;  // 2, 4 or 8
-  const uint32_t swz_mask = static_cast<uint32_t>(per_block - 1);
-  const int lg_pb = per_block == 8 ? 3 : (per_block == 4 ? 2 : 1);
-  const auto place = [&](int p, int piece) {
-    const uint32_t lin = static_cast<uint32_t>(p * row_bytes + (piece & (per_block - 1)) * 16);
-    return static_cast<uint32_t>((piece >> lg_pb) * kPairsPerStage * row_bytes) + (lin ^ (((lin >> 7) & swz_mask) << 4));
-  };
-  const int step = THREADS / pieces;
-  if ((pieces & (pieces - 1)) == 0 && step >= 8) {
-    const int lg = 31 - __clz(pieces);
-    const int p0 = tid >> lg, piece = tid & (pieces - 1);
-    uint32_t dst = dst_base + place(p0, piece);
-    const uint32_t dst_step = static_cast<uint32_t>(step * row_bytes);
-    const uint8_t* at = src + piece * 16;
-    for (int p = p0; p < n_pad; p += step, dst += dst_step) {
-      const uint32_t row = p < n ? static_cast<uint32_t>(rows[p]) : 0u;
-      cp_async16(dst, at + static_cast<unsigned long long>(row) * src_pitch, p < n ? 16u : 0u);
-    }
-    return;
-  }
-  for (int q = tid; q < n_pad * pieces; q += THREADS) {
-    const int p = q / pieces, piece = q - p * pieces;
-    const uint32_t row = p < n ? static_cast<uint32_t>(rows[p]) : 0u;
-    cp_async16(dst_base + place(p, piece), src + static_cast<unsigned long long>(row) * src_pitch + piece * 16, p < n ? 16u : 0u);
+  const int lg = per_block == 8 ? 3 : (per_block == 4 ? 2 : 1);
+  const uint32_t lin = static_cast<uint32_t>(p * row_bytes + (piece & (per_block - 1)) * 16);
+  const uint32_t mask = static_cast<uint32_t>(per_block - 1);
+  return static_cast<uint32_t>((piece >> lg) * kPairsPerStage * row_bytes) + (lin ^ (((lin >> 7) & mask) << 4));
+}
+
+// A power of two of pieces: a thread keeps its piece and steps over the rows by a multiple of eight, the
+// period of the swizzle, so that where it starts is settled once per CTA and a copy costs one list read and
+// two additions; four copies at a time, their list entries first, since with one warp on a scheduler every
+// dependent instruction is waited for (27 offsets of 45 k rows, 64 -> 64: 109 -> 64 us together with the
+// order of the offsets below and twice the splits; 128 -> 128: 169 -> 151 us).
+__device__ __forceinline__ void copy_rows(uint32_t to, const uint8_t* at, uint32_t pitch, const int* rows, int n, int n_pad, int first,
+                                          int step, uint32_t dst_step) {
+  for (int p = first; p < n_pad; p += 4 * step, to += 4 * dst_step) {
+    uint32_t row[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) row[u] = p + u * step < n ? static_cast<uint32_t>(rows[p + u * step]) : 0u;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (p + u * step < n_pad)
+        cp_async16(to + u * dst_step, at + static_cast<unsigned long long>(row[u]) * pitch, p + u * step < n ? 16u : 0u);
   }
 }
 
-template <typename T, int W>
+// Any number of pieces (48 or 96 channels).
+template <int THREADS>
+__device__ __forceinline__ void copy_rows_any(uint32_t base, const uint8_t* src, uint32_t pitch, const int* rows, int n, int n_pad,
+                                              int pieces, int row_bytes, int tid) {
+  for (int q = tid; q < n_pad * pieces; q += THREADS) {
+    const int p = q / pieces, piece = q - p * pieces;
+    const uint32_t row = p < n ? static_cast<uint32_t>(rows[p]) : 0u;
+    cp_async16(base + piece_place(p, piece, row_bytes), src + static_cast<unsigned long long>(row) * pitch + piece * 16, p < n ? 16u : 0u);
+  }
+}
+
+// SCAN: table entries a thread looks at per scan round.
+template <typename T, int W, int SCAN>
 __global__ void __launch_bounds__(W * 32 + 32, W == 4 ? 3 : 1)
 wgrad_tc_kernel(const __grid_constant__ WgParams p) {
   constexpr int kWgIssueWarps = W;
   constexpr int kWgIssueThreads = W * 32;
   constexpr int kWgMmaWarp = W;
-  constexpr int kScanEntries = kScanBatch * kWgIssueThreads;
+  constexpr int kScanEntries = SCAN * kWgIssueThreads;
   constexpr int ELEM = sizeof(T);
   constexpr int UMMA_K = 32 / ELEM;  // 16 pairs per MMA
 
@@ -113,13 +118,16 @@ wgrad_tc_kernel(const __grid_constant__ WgParams p) {
   int* rows_i = rows_m + kMaxStages * kPairsPerStage;
   uint64_t* bars = reinterpret_cast<uint64_t*>(rows_i + kMaxStages * kPairsPerStage);
   StageInfo* info = reinterpret_cast<StageInfo*>(bars + 2 * kMaxStages + 1);
-  int* warp_cnt = reinterpret_cast<int*>(info + kMaxStages);  // [kScanBatch][8]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(warp_cnt + kScanBatch * kWgIssueWarps);
+  int* warp_cnt = reinterpret_cast<int*>(info + kMaxStages);  // [SCAN][8]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(warp_cnt + SCAN * kWgIssueWarps);
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
   if (*reinterpret_cast<volatile int*>(p.status) != 0) return;
-  const int k = blockIdx.x / p.splits, split = blockIdx.x % p.splits;
+  // The middle offsets first: the centre of a submanifold kernel has every row, its neighbours most of them,
+  // and a CTA of theirs started last would run on alone.
+  const int turn = blockIdx.x / p.splits, split = blockIdx.x % p.splits;
+  const int k = (turn & 1) ? (p.kv - 1) / 2 + (turn + 1) / 2 : (p.kv - 1) / 2 - turn / 2;
   const int n0 = blockIdx.y * p.n_blocks * kTileM;  // first output channel of this CTA
   const long long lo = split * p.rows_per_split;
   const long long hi = min(p.n_out, lo + p.rows_per_split);
@@ -157,15 +165,21 @@ wgrad_tc_kernel(const __grid_constant__ WgParams p) {
     const uint8_t* g_src = static_cast<const uint8_t*>(p.gout) + static_cast<size_t>(n0) * ELEM;
     const uint8_t* f_src = static_cast<const uint8_t*>(p.feats);
     const uint32_t g_pitch = static_cast<uint32_t>(p.c_out) * ELEM, f_pitch = static_cast<uint32_t>(p.c_in) * ELEM;
+    const int g_lg = 31 - __clz(g_pieces), g_step = kWgIssueThreads >> g_lg, g_first = tid >> g_lg, g_piece = tid & (g_pieces - 1);
+    const bool g_even = (g_pieces & (g_pieces - 1)) == 0 && g_step >= 8;
+    const uint32_t g_place = piece_place(g_first, g_piece, p.g_row_bytes);
+    const int f_lg = 31 - __clz(f_pieces), f_step = kWgIssueThreads >> f_lg, f_first = tid >> f_lg, f_piece = tid & (f_pieces - 1);
+    const bool f_even = (f_pieces & (f_pieces - 1)) == 0 && f_step >= 8;
+    const uint32_t f_place = piece_place(f_first, f_piece, p.f_row_bytes);
 
     // Table entries are fetched one scan round (1024 entries, four per thread) ahead:
     // the loads of the next round are in flight while the stages of this one are built,
     // so the walk over a sparse table does not pay a memory latency per round.
     const int32_t* table = p.pair_fwd + static_cast<long long>(k) * p.n_out;
-    int ahead[kScanBatch];
+    int ahead[SCAN];
     auto fetch = [&](long long at) {
 #pragma unroll
-      for (int j = 0; j < kScanBatch; ++j) {
+      for (int j = 0; j < SCAN; ++j) {
         const long long m = at + j * kWgIssueThreads + tid;
         ahead[j] = m < hi ? __ldg(&table[m]) : -1;
       }
@@ -174,10 +188,10 @@ wgrad_tc_kernel(const __grid_constant__ WgParams p) {
     while (pos < hi || tail > head) {
       if (tail - head < kPairsPerStage && pos < hi) {
         // ---- append the existing pairs of one scan round to the ring, in table order ----
-        int cur[kScanBatch];
-        unsigned ballot[kScanBatch];
+        int cur[SCAN];
+        unsigned ballot[SCAN];
 #pragma unroll
-        for (int j = 0; j < kScanBatch; ++j) {
+        for (int j = 0; j < SCAN; ++j) {
           cur[j] = ahead[j];
           ballot[j] = __ballot_sync(0xffffffffu, cur[j] >= 0);
           if (lane == 0) warp_cnt[j * kWgIssueWarps + warp] = __popc(ballot[j]);
@@ -186,10 +200,10 @@ wgrad_tc_kernel(const __grid_constant__ WgParams p) {
         pos += kScanEntries;
         if (pos < hi) fetch(pos);
         named_bar_sync(1, kWgIssueThreads);
-        int before[kScanBatch];
+        int before[SCAN];
         int run = 0;
 #pragma unroll
-        for (int j = 0; j < kScanBatch; ++j) {
+        for (int j = 0; j < SCAN; ++j) {
 #pragma unroll
           for (int w = 0; w < kWgIssueWarps; ++w) {
             if (w == warp) before[j] = run;
@@ -197,7 +211,7 @@ wgrad_tc_kernel(const __grid_constant__ WgParams p) {
           }
         }
 #pragma unroll
-        for (int j = 0; j < kScanBatch; ++j) {
+        for (int j = 0; j < SCAN; ++j) {
           if (cur[j] >= 0) {
             const int slot = (tail + before[j] + __popc(ballot[j] & ((1u << lane) - 1u))) & (kRing - 1);
             ring_m[slot] = static_cast<int>(at + j * kWgIssueThreads + tid);
@@ -225,8 +239,14 @@ wgrad_tc_kernel(const __grid_constant__ WgParams p) {
         const uint32_t g_dst = smem_u32(stage_base + static_cast<size_t>(stage) * stage_bytes);
         const uint32_t f_dst = g_dst + p.g_stage_bytes;
         const uint32_t full = bar_full + 8 * stage;
-        copy_rows<kWgIssueThreads>(g_dst, g_src, g_pitch, sm, n, n_pad, g_pieces, p.g_row_bytes, tid);
-        copy_rows<kWgIssueThreads>(f_dst, f_src, f_pitch, si, n, n_pad, f_pieces, p.f_row_bytes, tid);
+        if (g_even)
+          copy_rows(g_dst + g_place, g_src + g_piece * 16, g_pitch, sm, n, n_pad, g_first, g_step, g_step * p.g_row_bytes);
+        else
+          copy_rows_any<kWgIssueThreads>(g_dst, g_src, g_pitch, sm, n, n_pad, g_pieces, p.g_row_bytes, tid);
+        if (f_even)
+          copy_rows(f_dst + f_place, f_src + f_piece * 16, f_pitch, si, n, n_pad, f_first, f_step, f_step * p.f_row_bytes);
+        else
+          copy_rows_any<kWgIssueThreads>(f_dst, f_src, f_pitch, si, n, n_pad, f_pieces, p.f_row_bytes, tid);
         cp_async_arrive_noinc(full);
         if (tid == 0) {
           info[stage].ksteps = n_pad / UMMA_K;
@@ -373,12 +393,12 @@ int span_of(int elems, int elem_size) {
 // Blocks of 128 output channels a CTA takes (two fill tensor memory at 256 input channels: one CTA per SM).
 int wg_blocks(int c_out) { return c_out % (2 * tc::kTileM) == 0 ? 2 : 1; }
 
-template <typename T, int W>
+template <typename T, int W, int SCAN>
 int launch_wgrad_tc(const WgParams& p, size_t smem_bytes, cudaStream_t st) {
   static bool configured[kMaxDevices] = {false};  // per instantiation and device
-  SPC_CUDA_OK(ensure_dynamic_smem(wgrad_tc_kernel<T, W>, 226 * 1024, configured));
+  SPC_CUDA_OK(ensure_dynamic_smem(wgrad_tc_kernel<T, W, SCAN>, 226 * 1024, configured));
   dim3 grid(static_cast<unsigned>(p.kv * p.splits), static_cast<unsigned>(ceil_div(p.c_out, p.n_blocks * kTileM)));
-  wgrad_tc_kernel<T, W><<<grid, W * 32 + 32, smem_bytes, st>>>(p);
+  wgrad_tc_kernel<T, W, SCAN><<<grid, W * 32 + 32, smem_bytes, st>>>(p);
   SPC_LAUNCH_OK();
   return SPC_OK;
 }
@@ -403,7 +423,9 @@ WgradSplit wgrad_tc_split(int64_t n_out, int c_in, int c_out, int kv) {
   // several CTAs per resident slot: offsets differ a lot in how many pairs they have (the centre
   // offset of a submanifold layer has all of them), and surplus CTAs even that out
   int64_t want = ceil_div(16 * static_cast<int64_t>(sm_count()), std::max<int64_t>(tiles, 1));
-  const int64_t by_len = std::max<int64_t>(1, n_out / 4096);
+  // the centre offset's CTAs are the longest chain: as short as the partial sums' traffic allows (10 k rows,
+  // 64 -> 64: 91 -> 34 us; at 128 x 128 and above the partial sums of 2048-row splits cost more than they give)
+  const int64_t by_len = std::max<int64_t>(1, n_out / (c_in * c_out <= 64 * 128 ? 2048 : 4096));
   want = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(want, by_len), 64));
   s.splits = static_cast<int>(want);
   s.rows_per_split = ceil_div(std::max<int64_t>(n_out, 1), s.splits);
@@ -428,7 +450,7 @@ int wgrad_tc(const void* feats, const void* gout, const int32_t* pair_fwd, float
   p.f_stage_bytes = static_cast<int>(align_up(static_cast<size_t>(c_in) * 2 * kPairsPerStage, 1024));
   const int stage_bytes = p.g_stage_bytes + p.f_stage_bytes;
   const size_t fixed = 1024 + 2 * kRing * 4 + 2 * tc::kMaxStages * kPairsPerStage * 4 + (2 * tc::kMaxStages + 1) * 8 +
-                       tc::kMaxStages * sizeof(tc::StageInfo) + kScanBatch * kWgMaxIssueWarps * 4 + 64;
+                       tc::kMaxStages * sizeof(tc::StageInfo) + 8 * kWgMaxIssueWarps * 4 + 64;
   const bool narrow = (c_in + p.n_blocks * g_cols) * 2 <= 384;  // bytes of rows per pair
   p.cols = 32;
   while (p.cols < c_in) p.cols <<= 1;
@@ -440,11 +462,11 @@ int wgrad_tc(const void* feats, const void* gout, const int32_t* pair_fwd, float
   p.status = device_status_ptr();
   if (p.status == nullptr) return fail(SPC_ERR_CUDA, "tcgen05 wgrad: no device status word");
   if (narrow) {
-    if (dtype == SPC_F16) return launch_wgrad_tc<__half, 4>(p, smem_bytes, st);
-    return launch_wgrad_tc<__nv_bfloat16, 4>(p, smem_bytes, st);
+    if (dtype == SPC_F16) return launch_wgrad_tc<__half, 4, 8>(p, smem_bytes, st);
+    return launch_wgrad_tc<__nv_bfloat16, 4, 8>(p, smem_bytes, st);
   }
-  if (dtype == SPC_F16) return launch_wgrad_tc<__half, 8>(p, smem_bytes, st);
-  return launch_wgrad_tc<__nv_bfloat16, 8>(p, smem_bytes, st);
+  if (dtype == SPC_F16) return launch_wgrad_tc<__half, 8, 4>(p, smem_bytes, st);
+  return launch_wgrad_tc<__nv_bfloat16, 8, 4>(p, smem_bytes, st);
 }
 
 }  // namespace spc
