@@ -14,8 +14,8 @@
 //     (one per column block for the input gradient) completing on the same
 //     mbarrier with complete_tx::bytes.
 // The row pitch in shared memory equals the swizzle span (32 / 64 / 128 bytes),
-// so channel counts of 16, 32 and multiples of 64 (16-bit) or 8, 16 and
-// multiples of 32 (TF32) are taken; other widths stay with gemm_tc.cu.
+// and is the widest that divides a row of channels: multiples of 16 channels
+// (16-bit) or 8 (TF32) are taken; other widths stay with gemm_tc.cu.
 //
 // Measured alternatives on B200 (64 -> 64 channels, 723k rows, 7.1M pairs):
 // feeding the rows with TMA tile::gather4 (4 rows per instruction) reached
@@ -471,13 +471,11 @@ CUtensorMapDataType tma_dtype(int dtype) {
                           : (dtype == SPC_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32);
 }
 
-// Swizzle span of rows holding `elems` contiguous elements: 32, 64 or 128 bytes
-// (the latter for any multiple of 128 bytes); 0 if the width does not fit.
+// Swizzle span of rows holding `elems` contiguous elements: the widest of 128, 64 and 32 bytes that
+// divides them (48 channels of 16 bits: 32 bytes, 96 channels: 64), so that no copy is padding; 0 if none does.
 int row_span(int elems, int elem_size) {
   const int bytes = elems * elem_size;
-  if (bytes == 32 || bytes == 64) return bytes;
-  if (bytes >= 128 && bytes % 128 == 0) return 128;
-  return 0;
+  return bytes % 128 == 0 ? 128 : bytes % 64 == 0 ? 64 : bytes % 32 == 0 ? 32 : 0;
 }
 
 template <typename T, typename TO, bool B_MN, int LPR>
