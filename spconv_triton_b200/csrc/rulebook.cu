@@ -3,16 +3,16 @@
 // Design (differs from the reference on purpose): the reference materialises
 // the kv*N candidate grid (out_lin, valid, out_row) in HBM, sorts the input
 // coordinates, runs kv*N binary searches and scatters into -1 pre-filled
-// tables (spconv_triton/pytorch/_impl/pairs.py:126-426).  Here two open-addressing hash
-// tables keyed by the batch-major linear coordinate replace the sorts and
-// searches, and every table is produced by a GATHER pass with one thread per
-// table column: thread r owns column r of pair_fwd, looks each of the kv
-// neighbour coordinates up (the tables are a few MB and stay in the 126 MB
-// L2), writes pair_fwd[k*n+r] fully coalesced and keeps the row's offset
-// bitmask in a register.  No candidate grid, no pre-fill, no atomics on the
-// tables, and the only ordered step is a radix sort of the n_out unique
-// output coordinates, which reproduces the ascending row numbering that
-// torch.unique gives the reference.
+// tables (spconv_triton/pytorch/_impl/pairs.py:126-426).  Here an occupancy bitmap of the
+// input grid and a hash table keyed by the batch-major linear coordinate replace
+// the sorts and searches (grids too large for a bitmap: hash tables alone).  A
+// thread owns a row: of a submanifold layer it looks the neighbours up, one
+// bitmap window per line of offsets, the present ones in the hash table; of a
+// strided or transposed layer it walks the one to eight outputs of an INPUT row
+// and scatters the pair into both tables.  Output rows are numbered by the rank
+// of their bit, which is the ascending order torch.unique gives the reference,
+// without a sort.  No candidate grid, no atomics on the tables; the tables are
+// L2-resident (126 MB) up to a few hundred thousand rows.
 #include <cub/device/device_radix_sort.cuh>
 
 #include <algorithm>
