@@ -75,3 +75,99 @@ def _invert(table, n_in):
         m = (t[k] >= 0).nonzero()[:, 0]
         inv[k][t[k][m].long()] = m.int()
     return inv.to(DEV)
+
+
+# (shape, rows, batch, kernel, stride, subm, transposed): cells and rows at the edges of 256-thread blocks, of the
+# 8192-row pieces of the tile order, of the windows of a bitmap line, of the slabs of a 125-offset and a
+# four-dimensional kernel; a grid too large for a bitmap
+BOOKS = [
+    ((64, 64, 64), 1, 1, 3, 1, True, False), ((64, 64, 64), 8191, 2, 3, 1, True, False),
+    ((40, 33, 65), 8193, 1, 3, 1, True, False), ((128, 128, 32), 16385, 2, 5, 1, True, False),
+    ((9, 9, 9, 10), 2000, 1, 3, 1, True, False), ((512, 512), 5000, 3, 3, 1, True, False),
+    ((64, 64, 64), 257, 1, 3, 2, False, False), ((41, 50, 63), 8193, 2, 3, 2, False, False),
+    ((40, 40, 40), 6000, 1, 2, 2, False, False), ((30, 30, 30), 1500, 2, 3, 1, False, False),
+    ((20, 20, 21), 700, 1, 3, 2, False, True), ((1500, 1500, 1500), 3000, 1, 3, 2, False, False),
+    ((1500, 1500, 1500), 3000, 1, 3, 1, True, False),
+]
+
+
+@pytest.mark.parametrize("shape,n,batch,k,stride,subm,transposed", BOOKS)
+@pytest.mark.parametrize("ordered", [False, True])
+def test_layer_rulebook_tables(shape, n, batch, k, stride, subm, transposed, ordered):
+    """Tables and coordinates of both sides equal the oracle's, bit for bit."""
+    from spconv_triton_b200.pytorch._impl import host
+
+    nd = len(shape)
+    idx = unique_coords(n, n, batch, shape)
+    if ordered:
+        idx = idx[np.lexsort(idx.T[::-1])]
+    one, pad = (1,) * nd, ((k // 2,) * nd if k % 2 else (0,) * nd)
+    geo, _ = host.geometry(batch, shape, (k,) * nd, (stride,) * nd, pad, one, (0,) * nd, subm, transposed)
+    rb = host.ext().build_rulebook(geo, torch.from_numpy(idx).to(DEV), True, True, True)
+    exp = orb.igemm_pairs(idx, batch, list(shape), [k] * nd, [stride] * nd, list(pad), [1] * nd, [0] * nd, subm, transposed,
+                          True, False)
+    np.testing.assert_array_equal(to_np(rb.out_indices), exp[0])
+    np.testing.assert_array_equal(to_np(rb.colmajor(False)), exp[2])
+    np.testing.assert_array_equal(to_np(rb.rowmajor(False))[:, :geo.kv].T, exp[2])
+    if not subm:  # the input side of a submanifold layer is its forward table, offsets reversed
+        np.testing.assert_array_equal(to_np(rb.colmajor(True)), exp[3])
+        np.testing.assert_array_equal(to_np(rb.rowmajor(True))[:, :geo.kv].T, exp[3])
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("kind,n,k", [("subm", 8193, 3), ("subm", 500, 5), ("down", 4097, 3), ("up", 129, 3)])
+def test_trained_layer(kind, n, k, dtype):
+    """Output, input, weight and bias gradient of a layer through its autograd node, against fp64 sums over the
+    oracle's tables: a row that the tile order lost or doubled would be wrong in one of them."""
+    import spconv_triton_b200.pytorch as sp
+
+    shape, ci, co = (48, 48, 48), 32, 48
+    idx = unique_coords(n, n, 1, shape)
+    cls = {"subm": sp.SubMConv3d, "down": sp.SparseConv3d, "up": sp.SparseConvTranspose3d}[kind]
+    stride = 1 if kind == "subm" else 2
+    torch.manual_seed(2)
+    layer = cls(ci, co, k, stride=stride, padding=k // 2, bias=True).to(DEV).to(dtype)
+    x = torch.randn(n, ci).to(DEV).to(dtype).requires_grad_()
+    y = layer(sp.SparseConvTensor(x, torch.from_numpy(idx).to(DEV), list(shape), 1)).features
+    g = torch.randn(y.shape).to(DEV).to(dtype)
+    y.backward(g)
+    table = torch.from_numpy(orb.igemm_pairs(idx, 1, list(shape), [k] * 3, [stride] * 3, [k // 2] * 3, [1] * 3, [0] * 3,
+                                             kind == "subm", kind == "up", True, False)[2]).to(DEV)
+    w = layer.weight.detach().reshape(co, -1, ci)
+    out, dw = _dense_statement(x.detach(), g, w, table)
+    din = torch.zeros((n, ci), dtype=torch.float64, device=DEV)
+    for q in range(table.shape[0]):
+        m = (table[q] >= 0).nonzero()[:, 0]
+        din.index_add_(0, table[q][m].long(), g[m].double() @ w[:, q].double())
+    for got, want in ((y.detach(), out + layer.bias.detach().double()), (x.grad, din), (layer.weight.grad.reshape(w.shape), dw),
+                      (layer.bias.grad, g.double().sum(0))):
+        assert rel_err(to_np(got.double()), to_np(want)) <= TOL[dtype]
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 8), (255, 16), (4097, 48), (70000, 128)])
+def test_bias_gradient_sums(rows, cols):
+    import spconv_triton_b200.pytorch as sp
+
+    idx = unique_coords(rows, rows, 1, (80, 80, 80))
+    layer = sp.SubMConv3d(16, cols, 1, bias=True).to(DEV).half()
+    y = layer(sp.SparseConvTensor(torch.ones(rows, 16, device=DEV).half(), torch.from_numpy(idx).to(DEV), [80] * 3, 1)).features
+    g = torch.randn(rows, cols, device=DEV).half()
+    y.backward(g)
+    assert rel_err(to_np(layer.bias.grad.double()), to_np(g.double().sum(0))) <= TOL[torch.float16]
+
+
+@pytest.mark.parametrize("heavy", [255, 256, 257, 3000])
+def test_voxels_with_many_points(heavy):
+    """Voxels around the number of points up to which a point ranks itself by comparisons."""
+    from oracle.voxelize import point_to_voxel
+    from spconv_triton_b200.pytorch.utils import PointToVoxel
+
+    g = torch.Generator().manual_seed(heavy)
+    pts = torch.rand((5000 + heavy, 4), generator=g) * 50
+    at = torch.randperm(len(pts), generator=g)[:heavy]
+    pts[at, :3] = torch.rand((heavy, 3), generator=g) * 0.4 + 20.05
+    ctor = dict(vsize_xyz=[0.5] * 3, coors_range_xyz=[0.0, 0.0, 0.0, 50.0, 50.0, 50.0], num_point_features=4,
+                max_num_voxels=100_000, max_num_points_per_voxel=300)
+    out = PointToVoxel(device=torch.device(DEV), **ctor).generate_voxel_with_id(pts.to(DEV))
+    for got, want in zip(out, point_to_voxel(pts.numpy(), **ctor)):
+        np.testing.assert_array_equal(to_np(got), want)
