@@ -503,8 +503,9 @@ int spc_avgpool_backward(const void* grad_out, const int32_t* pair_bwd, const in
 
 /* The same four operators over a row-major table [n_rows, pitch] (pitch 0: column-major
  * [kv, n_rows]).  src: features forward, grad_out backward; own / ref: features and
- * pooled output (max backward); aux_in / aux_out: the counts of the average.  Every
- * element of dst (and aux_out) is written. */
+ * pooled output (max backward); aux_in / aux_out: the counts of the average; order:
+ * a permutation of the rows, the order in which the average's gradient works on them
+ * (NULL: as they are; the other operators take none).  Every element of dst (and aux_out) is written. */
 typedef enum {
   SPC_POOL_MAX_FORWARD = 0,
   SPC_POOL_AVG_FORWARD = 1,
@@ -512,8 +513,15 @@ typedef enum {
   SPC_POOL_MAX_BACKWARD = 3
 } spc_pool_op;
 int spc_pool(int op, const void* src, const void* own, const void* ref, const int32_t* table, int pitch,
-             const int32_t* aux_in, void* dst, int32_t* aux_out, int64_t n_rows, int channels, int kv, int dtype,
+             const int32_t* order, const int32_t* aux_in, void* dst, int32_t* aux_out, int64_t n_rows, int channels, int kv, int dtype,
              void* stream);
+
+/* An order for spc_pool: the rows of a row-major table [n_rows, pitch] (pitch a
+ * multiple of 4) by the first row they read, so that rows that share targets run
+ * close together. */
+size_t spc_pool_row_order_workspace_bytes(int64_t n_rows);
+int spc_pool_row_order(const int32_t* table, int pitch, int kv, int64_t n_rows, int64_t n_targets, int32_t* order,
+                       void* workspace, size_t workspace_bytes, void* stream);
 
 /* ---- a chain of convolutions in one call --------------------------------- */
 

@@ -441,6 +441,13 @@ Tensor conv_eval(const Tensor& features, const Tensor& weight, const c10::option
 
 // ---- pooling -------------------------------------------------------------------------------------------------------
 
+// Bytes of gathered rows from which on the gradient of an average works on the input rows in the order of the
+// outputs they read.  Input rows come as the user has them, outputs in cell order: up to about the size of the L2
+// (126 MB) that does not matter, beyond it every gather of an unordered row is a miss (27 outputs of 512 bytes each,
+// 300 k rows: 741 -> 439 us, the order itself 28 us in four launches).  The maximum's gradient, which reads few
+// outputs a row and its own row besides, gains nothing (213 against 227 us).
+constexpr size_t kPoolOrderBytes = size_t{96} << 20;
+
 Tensor pool_rows(int op, const Tensor& src, const Tensor& own, const Tensor& ref, const Book& rb, bool input, const Tensor& aux_in,
                  const Tensor& aux_out) {
   const int64_t c = src.size(1);
@@ -449,7 +456,14 @@ Tensor pool_rows(int op, const Tensor& src, const Tensor& own, const Tensor& ref
   const int64_t n = t.rm.size(0);
   Tensor out = at::empty({n, c}, src.options());
   if (c == 0) return out;
-  check(spc_pool(op, src.data_ptr(), data(own), data(ref), ints(t.rm), rb->geo->kvp, ints(aux_in), out.data_ptr(), ints(aux_out), n, c,
+  Tensor order;
+  if (op == SPC_POOL_AVG_BACKWARD && n > 0 && src.nbytes() >= kPoolOrderBytes) {
+    order = at::empty({n}, rb->indices.options());
+    Tensor scratch = at::empty({static_cast<int64_t>(spc_pool_row_order_workspace_bytes(n))}, rb->indices.options().dtype(at::kByte));
+    check(spc_pool_row_order(ints(t.rm), rb->geo->kvp, rb->geo->kv, n, src.size(0), ints(order), scratch.data_ptr(), scratch.numel(),
+                             stream_of(src)));
+  }
+  check(spc_pool(op, src.data_ptr(), data(own), data(ref), ints(t.rm), rb->geo->kvp, ints(order), ints(aux_in), out.data_ptr(), ints(aux_out), n, c,
                  rb->geo->kv, code_of(src.scalar_type()), stream_of(src)));
   return out;
 }

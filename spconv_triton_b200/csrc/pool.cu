@@ -17,6 +17,7 @@
 // (pool.py:200-201) and its backward MULTIPLIES by that count (pool.py:250-252).
 // fp16/bf16/fp32 accumulate in fp32, fp64 in fp64 (pool.py:72-74).
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -95,19 +96,71 @@ __device__ __forceinline__ Pack<__nv_bfloat16, 8> pack<__nv_bfloat16, 8>(const f
   return o;
 }
 
+// Sums of two neighbouring channels per instruction; the same IEEE results as one at a time.
+__device__ __forceinline__ void add2(float& a0, float& a1, float x0, float x1) {
+  asm("{\n\t.reg .b64 a, x;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 x, {%2, %3};\n\t"
+      "add.rn.f32x2 a, a, x;\n\tmov.b64 {%0, %1}, a;\n\t}"
+      : "+f"(a0), "+f"(a1) : "f"(x0), "f"(x1));
+}
+__device__ __forceinline__ void fma2(float& a0, float& a1, float x0, float x1, float w) {
+  asm("{\n\t.reg .b64 a, x, w;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 x, {%2, %3};\n\tmov.b64 w, {%4, %4};\n\t"
+      "fma.rn.f32x2 a, x, w, a;\n\tmov.b64 {%0, %1}, a;\n\t}"
+      : "+f"(a0), "+f"(a1) : "f"(x0), "f"(x1), "f"(w));
+}
+// o = x * w + a
+__device__ __forceinline__ void fma2(float x0, float x1, float w, float a0, float a1, float& o0, float& o1) {
+  o0 = a0;
+  o1 = a1;
+  fma2(o0, o1, x0, x1, w);
+}
+__device__ __forceinline__ void mul2(float& o0, float& o1, float x0, float x1, float w) {
+  asm("{\n\t.reg .b64 o, x, w;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 w, {%4, %4};\n\t"
+      "mul.rn.f32x2 o, x, w;\n\tmov.b64 {%0, %1}, o;\n\t}"
+      : "=f"(o0), "=f"(o1) : "f"(x0), "f"(x1), "f"(w));
+}
+
+// a + x in one instruction; x is exact in fp32.
+__device__ __forceinline__ void add_mixed(float& a, __half x) { asm("add.rn.f32.f16 %0, %1, %0;" : "+f"(a) : "h"(__half_as_ushort(x))); }
+__device__ __forceinline__ void add_mixed(float& a, __nv_bfloat16 x) { asm("add.rn.f32.bf16 %0, %1, %0;" : "+f"(a) : "h"(__bfloat16_as_ushort(x))); }
+
+// a / d for a whole number d, correctly rounded by one correction of a * (1 / d) with the exact remainder
+// (Markstein 1990), two channels an instruction, instead of a division's ten instructions a value: a window
+// of few present rows spent a quarter of its time there.  Used where the quotient is then rounded to 16 bits;
+// where the remainder is no number (an infinity), the quotient is a * (1 / d).
+template <int VEC>
+__device__ __forceinline__ void divide_by_count(float (&a)[VEC], float d) {
+  const float inverse = 1.f / d;
+  float q[VEC], check0 = 0.f, check1 = 0.f;
+#pragma unroll
+  for (int v = 0; v < VEC; v += 2) {
+    float rest0 = a[v], rest1 = a[v + 1];
+    mul2(q[v], q[v + 1], a[v], a[v + 1], inverse);
+    fma2(rest0, rest1, q[v], q[v + 1], -d);
+    add2(check0, check1, rest0, rest1);
+    fma2(rest0, rest1, inverse, q[v], q[v + 1], a[v], a[v + 1]);
+  }
+  if (check0 + check1 == check0 + check1) return;
+#pragma unroll
+  for (int v = 0; v < VEC; ++v)
+    if (!(a[v] == a[v])) a[v] = q[v];
+}
+
 enum PoolOp { kMaxFwd = 0, kAvgFwd = 1, kAvgBwd = 2, kMaxBwd = 3 };
 // Independent 16-byte gathers one thread keeps in flight (rows in flight = in_flight / U), and
 // 16-byte vectors of a row one thread owns, per operator; each pair is the measured best on B200
 // for 512-byte rows (C = 256 fp16): max forward has few present entries per row and gains from
 // four rows in flight with two vectors each (0.26 ms = 0.81 of the copy peak, against 0.31 with
-// 4 x 2); average forward over a 3^3 window prefers four vectors and one row; max backward
+// 4 x 2); average forward over a 3^3 window prefers two vectors and two rows; max backward
 // reads two rows per entry and keeps its own row in registers: one vector and one row per thread
-// (more resident threads) is best for it.
+// (more resident threads) is best for it.  `ctas` per SM bounds the registers (0: the
+// compiler's choice): the forward average issues
+// instructions most of the time and gains by a fourth CTA (1.1 M rows of 512 bytes, 7.4 entries: 494 to 447 us,
+// 565 before its sums and quotients were packed), its gradient, bound by L2, loses by it (439 to 547).
 template <int OP> struct PoolTune;
-template <> struct PoolTune<0> { static constexpr int in_flight = 8, max_u = 2; };  // kMaxFwd
-template <> struct PoolTune<1> { static constexpr int in_flight = 4, max_u = 4; };  // kAvgFwd
-template <> struct PoolTune<2> { static constexpr int in_flight = 8, max_u = 2; };  // kAvgBwd
-template <> struct PoolTune<3> { static constexpr int in_flight = 1, max_u = 1; };  // kMaxBwd
+template <> struct PoolTune<0> { static constexpr int in_flight = 8, max_u = 2, ctas = 3; };  // kMaxFwd
+template <> struct PoolTune<1> { static constexpr int in_flight = 4, max_u = 2, ctas = 4; };  // kAvgFwd
+template <> struct PoolTune<2> { static constexpr int in_flight = 8, max_u = 2, ctas = 3; };  // kAvgBwd
+template <> struct PoolTune<3> { static constexpr int in_flight = 1, max_u = 1, ctas = 0; };  // kMaxBwd
 constexpr int kChunk = 32;    // table entries of one row compacted per pass (one per lane)
 constexpr int kMaxRows = 64;  // rows per CTA
 
@@ -160,11 +213,24 @@ struct PoolRow {
       ++total;
 #pragma unroll
       for (int u = 0; u < U; ++u) {
+        if constexpr (OP == kAvgFwd && sizeof(T) == 2) {
+#pragma unroll
+          for (int v = 0; v < VEC; ++v) add_mixed(acc[u][v], pk[b][u].v[v]);
+          continue;
+        }
         A x[VEC], r[VEC], o[VEC];
         unpack<T, VEC>(pk[b][u], x);
         if (OP == kMaxBwd) {
           unpack<T, VEC>(rk[b][u], r);
           unpack<T, VEC>(f[u], o);
+        }
+        if constexpr ((OP == kAvgFwd || OP == kAvgBwd) && VEC % 2 == 0 && std::is_same<A, float>::value) {
+#pragma unroll
+          for (int v = 0; v < VEC; v += 2) {
+            if (OP == kAvgFwd) add2(acc[u][v], acc[u][v + 1], x[v], x[v + 1]);
+            else fma2(acc[u][v], acc[u][v + 1], x[v], x[v + 1], w[b]);
+          }
+          continue;
         }
 #pragma unroll
         for (int v = 0; v < VEC; ++v) {
@@ -182,7 +248,9 @@ struct PoolRow {
     const A d = static_cast<A>(total > 1 ? total : 1);
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      if (OP == kAvgFwd) {
+      if constexpr (OP == kAvgFwd && sizeof(T) == 2 && VEC % 2 == 0) {
+        divide_by_count<VEC>(acc[u], d);
+      } else if (OP == kAvgFwd) {
 #pragma unroll
         for (int v = 0; v < VEC; ++v) acc[u][v] /= d;
       }
@@ -208,10 +276,10 @@ struct PoolGeom { int nt, tpb, rpb; };
 constexpr int kGroupIters = 8;  // row groups per warp
 
 template <typename T, int VEC, int U, int OP, int LGNT>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, PoolTune<OP>::ctas)
 pool_group_kernel(const T* __restrict__ src, const T* __restrict__ own, const T* __restrict__ ref,
-                  const int32_t* __restrict__ table, const int32_t* __restrict__ aux_in, T* __restrict__ dst,
-                  int32_t* __restrict__ aux_out, long long n_rows, int channels, int kv, long long sk, int sr) {
+                  const int32_t* __restrict__ table, const int32_t* __restrict__ order, const int32_t* __restrict__ aux_in,
+                  T* __restrict__ dst, int32_t* __restrict__ aux_out, long long n_rows, int channels, int kv, long long sk, int sr) {
   // the threads per row are a compile-time power of two: the entry loops below unroll to
   // exactly 32 / nt loads, ballots and selects
   constexpr int lg_nt = LGNT;
@@ -226,31 +294,57 @@ pool_group_kernel(const T* __restrict__ src, const T* __restrict__ own, const T*
   constexpr int per_lane = kE;
   const long long warp_id = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const long long row_first = warp_id * kGroupIters * per_lane + (lane >> lg_nt);
+  // The average's kernels keep the rows of the warp's groups in registers, requested at once where there is an
+  // order; the forward pass, which has none, still gains by the shorter row arithmetic (505 to 450 us), the
+  // maximum loses (116 to 144 and 216 to 268 us).
+  constexpr bool kOrdered = OP == kAvgBwd || OP == kAvgFwd;
+  int rows_of[(kGroupIters * kE + 31) / 32];
+#pragma unroll
+  for (int i = 0; i < (kGroupIters * kE + 31) / 32; ++i) {
+    const long long slot = warp_id * kGroupIters * per_lane + i * 32 + lane;
+    rows_of[i] = !kOrdered || order == nullptr ? static_cast<int>(slot) : (i * 32 + lane < kGroupIters * kE && slot < n_rows ? __ldg(&order[slot]) : 0);
+  }
+  auto row_at = [&](int it) {
+    if (!kOrdered) return row_first + static_cast<long long>(it) * per_lane;
+    const int at = it * kE + (lane >> lg_nt);
+    int r = __shfl_sync(kFull, rows_of[0], at & 31);
+#pragma unroll
+    for (int i = 1; i < (kGroupIters * kE + 31) / 32; ++i) {
+      const int other = __shfl_sync(kFull, rows_of[i], at & 31);
+      r = (at >> 5) == i ? other : r;
+    }
+    return static_cast<long long>(r);
+  };
 
-  auto load_entries = [&](long long row, int k0, int (&v)[kE]) {
+  auto load_entries = [&](long long row, bool there, int k0, int (&v)[kE]) {
 #pragma unroll
     for (int e = 0; e < kE; ++e) {
       const int k = k0 + e * nt + kl;
-      v[e] = (row < n_rows && e < per_lane && k < kv) ? __ldg(&table[k * sk + row * sr]) : -1;
+      v[e] = (there && k < kv) ? __ldg(&table[k * sk + row * sr]) : -1;
     }
   };
 
   int vn[kE];
-  load_entries(row_first, 0, vn);
+  long long next = row_at(0);
+  load_entries(next, row_first < n_rows, 0, vn);
 #pragma unroll 1
   for (int it = 0; it < kGroupIters; ++it) {
-    const long long row = row_first + static_cast<long long>(it) * per_lane;
-    if (row - (lane >> lg_nt) >= n_rows) break;  // warp-uniform: the whole group is past the end
-    const bool live = row < n_rows;
+    const long long slot = row_first + static_cast<long long>(it) * per_lane;
+    if (slot - (lane >> lg_nt) >= n_rows) break;  // warp-uniform: the whole group is past the end
+    const bool live = slot < n_rows;
+    const long long row = kOrdered ? next : slot;
     int v[kE];
 #pragma unroll
     for (int e = 0; e < kE; ++e) v[e] = vn[e];
-    if (it + 1 < kGroupIters) load_entries(row + per_lane, 0, vn);
+    if (it + 1 < kGroupIters) {
+      if (kOrdered) next = row_at(it + 1);
+      load_entries(kOrdered ? next : slot + per_lane, slot + per_lane < n_rows, 0, vn);
+    }
 
     PoolRow<T, VEC, U, OP> pr;
     if (live) pr.begin(own, row, channels, c0, cstep);
     for (int k0 = 0; k0 < kv; k0 += 32) {
-      if (k0 != 0) load_entries(row, k0, v);
+      if (k0 != 0) load_entries(row, live, k0, v);
       unsigned gm = 0;
 #pragma unroll
       for (int e = 0; e < kE; ++e) {
@@ -288,7 +382,7 @@ pool_group_kernel(const T* __restrict__ src, const T* __restrict__ own, const T*
 template <typename T, int VEC, int U, int OP>
 __global__ void __launch_bounds__(256)
 pool_compact_kernel(const T* __restrict__ src, const T* __restrict__ own, const T* __restrict__ ref,
-                    const int32_t* __restrict__ table, const int32_t* __restrict__ aux_in, T* __restrict__ dst,
+                    const int32_t* __restrict__ table, const int32_t* __restrict__ order, const int32_t* __restrict__ aux_in, T* __restrict__ dst,
                     int32_t* __restrict__ aux_out, long long n_rows, int channels, int kv, long long sk, int sr,
                     PoolGeom g) {
   constexpr int B = PoolTune<OP>::in_flight / U > 0 ? PoolTune<OP>::in_flight / U : 1;
@@ -300,8 +394,8 @@ pool_compact_kernel(const T* __restrict__ src, const T* __restrict__ own, const 
   const long long row0 = static_cast<long long>(blockIdx.x) * g.rpb;
   const int rl = t / g.tpb;
   const int ct = t - rl * g.tpb + static_cast<int>(blockIdx.y) * g.tpb;
-  const long long row = row0 + rl;
-  const bool live = rl < g.rpb && row < n_rows && ct < g.nt;
+  const bool live = rl < g.rpb && row0 + rl < n_rows && ct < g.nt;
+  const long long row = OP == kAvgBwd && order != nullptr && live ? __ldg(&order[row0 + rl]) : row0 + rl;
   const int c0 = ct * VEC, cstep = g.nt * VEC;
 
   PoolRow<T, VEC, U, OP> pr;
@@ -313,8 +407,9 @@ pool_compact_kernel(const T* __restrict__ src, const T* __restrict__ own, const 
     for (int i = t; i < kc * g.rpb; i += nthr) {
       // consecutive threads read consecutive entries of the table
       const int k = sr == 1 ? i / g.rpb : i % kc, r = sr == 1 ? i - k * g.rpb : i / kc;
-      const long long rr = row0 + r;
-      tab[k][r] = rr < n_rows ? __ldg(&table[(k0 + k) * sk + rr * sr]) : -1;
+      const bool there = row0 + r < n_rows;
+      const long long rr = OP == kAvgBwd && there && order != nullptr ? __ldg(&order[row0 + r]) : row0 + r;
+      tab[k][r] = there ? __ldg(&table[(k0 + k) * sk + rr * sr]) : -1;
     }
     __syncthreads();
     for (int r = warp; r < g.rpb; r += nwarps) {
@@ -336,6 +431,65 @@ pool_compact_kernel(const T* __restrict__ src, const T* __restrict__ own, const 
   if (live) pr.finish(dst, aux_out, row, channels, c0, cstep);
 }
 
+// Rows in the order of the rows they read: by the first present entry of their table row, in up to 8192
+// buckets of neighbouring targets, any order inside a bucket.
+constexpr int kOrderBuckets = 8192;
+
+__global__ void __launch_bounds__(1024) clear_buckets_kernel(int* counts) { counts[blockIdx.x * 1024 + threadIdx.x] = 0; }
+
+__global__ void __launch_bounds__(256)
+count_buckets_kernel(const int4* __restrict__ table, int words, int n_rows, int shift, int* __restrict__ counts,
+                     int2* __restrict__ placed) {
+  const int r = blockIdx.x * 256 + threadIdx.x;
+  if (r >= n_rows) return;
+  int first = 0;  // a row that reads nothing goes anywhere
+  for (int q = 0; q < words; ++q) {
+    const int4 e = __ldg(&table[static_cast<long long>(r) * words + q]);
+    const int hit = e.x >= 0 ? e.x : e.y >= 0 ? e.y : e.z >= 0 ? e.z : e.w;  // (beyond kv the table holds -1)
+    if (hit >= 0) {
+      first = hit;
+      break;
+    }
+  }
+  const int b = first >> shift;
+  placed[r] = make_int2(b, atomicAdd(&counts[b], 1));
+}
+
+__global__ void __launch_bounds__(1024) scan_buckets_kernel(int* counts) {
+  __shared__ int sums[32];
+  constexpr int kEach = kOrderBuckets / 1024;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  int c[kEach], own = 0;
+#pragma unroll
+  for (int i = 0; i < kEach; ++i) {
+    c[i] = counts[t * kEach + i];
+    own += c[i];
+  }
+  int incl = own;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) sums[warp] = incl;
+  __syncthreads();
+  int before = incl - own;
+  for (int w = 0; w < warp; ++w) before += sums[w];
+#pragma unroll
+  for (int i = 0; i < kEach; ++i) {
+    counts[t * kEach + i] = before;
+    before += c[i];
+  }
+}
+
+__global__ void __launch_bounds__(256)
+deal_buckets_kernel(const int2* __restrict__ placed, const int* __restrict__ starts, int n_rows, int32_t* __restrict__ order) {
+  const int r = blockIdx.x * 256 + threadIdx.x;
+  if (r >= n_rows) return;
+  const int2 p = placed[r];
+  order[starts[p.x] + p.y] = r;
+}
+
 template <typename T>
 int vec_for(int channels, const void* a, const void* b, const void* c = nullptr, const void* d = nullptr) {
   constexpr int full = 16 / sizeof(T);
@@ -345,7 +499,7 @@ int vec_for(int channels, const void* a, const void* b, const void* c = nullptr,
 }
 
 template <typename T, int VEC, int U, int OP>
-void pool_launch_u(const T* src, const T* own, const T* ref, const int32_t* table, const int32_t* aux_in, T* dst,
+void pool_launch_u(const T* src, const T* own, const T* ref, const int32_t* table, const int32_t* order, const int32_t* aux_in, T* dst,
                    int32_t* aux_out, int64_t n_rows, int channels, int kv, int pitch, cudaStream_t st) {
   const long long sk = pitch ? 1 : n_rows;
   const int sr = pitch ? pitch : 1;
@@ -362,19 +516,19 @@ void pool_launch_u(const T* src, const T* own, const T* ref, const int32_t* tabl
     const long long warps = ceil_div(static_cast<long long>(n_rows), (32 >> lg) * kGroupIters);
     const unsigned blocks = static_cast<unsigned>(ceil_div(warps, 8));
     switch (lg) {
-      case 2: pool_group_kernel<T, VEC, U, OP, 2><<<blocks, 256, 0, st>>>(src, own, ref, table, aux_in, dst, aux_out, n_rows, channels, kv, sk, sr); break;
-      case 3: pool_group_kernel<T, VEC, U, OP, 3><<<blocks, 256, 0, st>>>(src, own, ref, table, aux_in, dst, aux_out, n_rows, channels, kv, sk, sr); break;
-      case 4: pool_group_kernel<T, VEC, U, OP, 4><<<blocks, 256, 0, st>>>(src, own, ref, table, aux_in, dst, aux_out, n_rows, channels, kv, sk, sr); break;
-      default: pool_group_kernel<T, VEC, U, OP, 5><<<blocks, 256, 0, st>>>(src, own, ref, table, aux_in, dst, aux_out, n_rows, channels, kv, sk, sr); break;
+      case 2: pool_group_kernel<T, VEC, U, OP, 2><<<blocks, 256, 0, st>>>(src, own, ref, table, order, aux_in, dst, aux_out, n_rows, channels, kv, sk, sr); break;
+      case 3: pool_group_kernel<T, VEC, U, OP, 3><<<blocks, 256, 0, st>>>(src, own, ref, table, order, aux_in, dst, aux_out, n_rows, channels, kv, sk, sr); break;
+      case 4: pool_group_kernel<T, VEC, U, OP, 4><<<blocks, 256, 0, st>>>(src, own, ref, table, order, aux_in, dst, aux_out, n_rows, channels, kv, sk, sr); break;
+      default: pool_group_kernel<T, VEC, U, OP, 5><<<blocks, 256, 0, st>>>(src, own, ref, table, order, aux_in, dst, aux_out, n_rows, channels, kv, sk, sr); break;
     }
   } else {
-    pool_compact_kernel<T, VEC, U, OP><<<grid, threads, 0, st>>>(src, own, ref, table, aux_in, dst, aux_out,
+    pool_compact_kernel<T, VEC, U, OP><<<grid, threads, 0, st>>>(src, own, ref, table, order, aux_in, dst, aux_out,
                                                                 n_rows, channels, kv, sk, sr, g);
   }
 }
 
 template <typename T, int OP>
-int pool_launch(const void* src_, const void* own_, const void* ref_, const int32_t* table,
+int pool_launch(const void* src_, const void* own_, const void* ref_, const int32_t* table, const int32_t* order,
                 const int32_t* aux_in, void* dst_, int32_t* aux_out, int64_t n_rows, int channels, int kv, int pitch,
                 cudaStream_t st) {
   constexpr int full = 16 / sizeof(T);
@@ -383,18 +537,18 @@ int pool_launch(const void* src_, const void* own_, const void* ref_, const int3
   const T* ref = static_cast<const T*>(ref_);
   T* dst = static_cast<T*>(dst_);
   if (vec_for<T>(channels, src_, own_, ref_, dst_) != full) {
-    pool_launch_u<T, 1, 1, OP>(src, own, ref, table, aux_in, dst, aux_out, n_rows, channels, kv, pitch, st);
+    pool_launch_u<T, 1, 1, OP>(src, own, ref, table, order, aux_in, dst, aux_out, n_rows, channels, kv, pitch, st);
   } else {
     // most vectors per thread that still leave a row at least 4 threads (the warp-group kernel)
     const int tpr = channels / full;
     int u = PoolTune<OP>::max_u;
     while (u > 1 && (tpr % u != 0 || tpr / u < 4)) u /= 2;
     if (u == 4)
-      pool_launch_u<T, full, 4, OP>(src, own, ref, table, aux_in, dst, aux_out, n_rows, channels, kv, pitch, st);
+      pool_launch_u<T, full, 4, OP>(src, own, ref, table, order, aux_in, dst, aux_out, n_rows, channels, kv, pitch, st);
     else if (u == 2)
-      pool_launch_u<T, full, 2, OP>(src, own, ref, table, aux_in, dst, aux_out, n_rows, channels, kv, pitch, st);
+      pool_launch_u<T, full, 2, OP>(src, own, ref, table, order, aux_in, dst, aux_out, n_rows, channels, kv, pitch, st);
     else
-      pool_launch_u<T, full, 1, OP>(src, own, ref, table, aux_in, dst, aux_out, n_rows, channels, kv, pitch, st);
+      pool_launch_u<T, full, 1, OP>(src, own, ref, table, order, aux_in, dst, aux_out, n_rows, channels, kv, pitch, st);
   }
   SPC_LAUNCH_OK();
   return SPC_OK;
@@ -424,7 +578,7 @@ extern "C" int spc_maxpool_forward(const void* features, const int32_t* pair_fwd
     return fail(SPC_ERR_INVALID_ARGUMENT, "maxpool_forward: bad arguments");
   if (n_out == 0) return SPC_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  SPC_POOL_DISPATCH(dtype, (pool_launch<T, kMaxFwd>(features, nullptr, nullptr, pair_fwd, nullptr, out, nullptr, n_out, channels, kv, 0, st)));
+  SPC_POOL_DISPATCH(dtype, (pool_launch<T, kMaxFwd>(features, nullptr, nullptr, pair_fwd, nullptr, nullptr, out, nullptr, n_out, channels, kv, 0, st)));
 }
 
 extern "C" int spc_avgpool_forward(const void* features, const int32_t* pair_fwd, void* out, int32_t* count,
@@ -433,7 +587,7 @@ extern "C" int spc_avgpool_forward(const void* features, const int32_t* pair_fwd
     return fail(SPC_ERR_INVALID_ARGUMENT, "avgpool_forward: bad arguments");
   if (n_out == 0) return SPC_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  SPC_POOL_DISPATCH(dtype, (pool_launch<T, kAvgFwd>(features, nullptr, nullptr, pair_fwd, nullptr, out, count, n_out, channels, kv, 0, st)));
+  SPC_POOL_DISPATCH(dtype, (pool_launch<T, kAvgFwd>(features, nullptr, nullptr, pair_fwd, nullptr, nullptr, out, count, n_out, channels, kv, 0, st)));
 }
 
 extern "C" int spc_maxpool_backward(const void* features, const void* out_features, const void* grad_out,
@@ -443,7 +597,7 @@ extern "C" int spc_maxpool_backward(const void* features, const void* out_featur
     return fail(SPC_ERR_INVALID_ARGUMENT, "maxpool_backward: bad arguments");
   if (n_in == 0) return SPC_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  SPC_POOL_DISPATCH(dtype, (pool_launch<T, kMaxBwd>(grad_out, features, out_features, pair_bwd, nullptr, din, nullptr, n_in, channels, kv, 0, st)));
+  SPC_POOL_DISPATCH(dtype, (pool_launch<T, kMaxBwd>(grad_out, features, out_features, pair_bwd, nullptr, nullptr, din, nullptr, n_in, channels, kv, 0, st)));
 }
 
 extern "C" int spc_avgpool_backward(const void* grad_out, const int32_t* pair_bwd, const int32_t* count,
@@ -452,21 +606,49 @@ extern "C" int spc_avgpool_backward(const void* grad_out, const int32_t* pair_bw
     return fail(SPC_ERR_INVALID_ARGUMENT, "avgpool_backward: bad arguments");
   if (n_in == 0) return SPC_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  SPC_POOL_DISPATCH(dtype, (pool_launch<T, kAvgBwd>(grad_out, nullptr, nullptr, pair_bwd, count, din, nullptr, n_in, channels, kv, 0, st)));
+  SPC_POOL_DISPATCH(dtype, (pool_launch<T, kAvgBwd>(grad_out, nullptr, nullptr, pair_bwd, nullptr, count, din, nullptr, n_in, channels, kv, 0, st)));
 }
 
 extern "C" int spc_pool(int op, const void* src, const void* own, const void* ref, const int32_t* table, int pitch,
-                        const int32_t* aux_in, void* dst, int32_t* aux_out, int64_t n_rows, int channels, int kv,
+                        const int32_t* order, const int32_t* aux_in, void* dst, int32_t* aux_out, int64_t n_rows, int channels, int kv,
                         int dtype, void* stream) {
   if (!pool_args_ok(src, table, dst, n_rows, channels, kv) || (pitch != 0 && pitch < kv) || op < kMaxFwd || op > kMaxBwd ||
-      (op == kMaxBwd && (!own || !ref)) || (op == kAvgBwd && !aux_in))
+      (op == kMaxBwd && (!own || !ref)) || (op == kAvgBwd && !aux_in) || (order != nullptr && op != kAvgBwd))
     return fail(SPC_ERR_INVALID_ARGUMENT, "pool: bad arguments");
   if (n_rows == 0) return SPC_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   switch (op) {
-    case kMaxFwd: SPC_POOL_DISPATCH(dtype, (pool_launch<T, kMaxFwd>(src, nullptr, nullptr, table, nullptr, dst, nullptr, n_rows, channels, kv, pitch, st)));
-    case kAvgFwd: SPC_POOL_DISPATCH(dtype, (pool_launch<T, kAvgFwd>(src, nullptr, nullptr, table, nullptr, dst, aux_out, n_rows, channels, kv, pitch, st)));
-    case kAvgBwd: SPC_POOL_DISPATCH(dtype, (pool_launch<T, kAvgBwd>(src, nullptr, nullptr, table, aux_in, dst, nullptr, n_rows, channels, kv, pitch, st)));
-    default: SPC_POOL_DISPATCH(dtype, (pool_launch<T, kMaxBwd>(src, own, ref, table, nullptr, dst, nullptr, n_rows, channels, kv, pitch, st)));
+    case kMaxFwd: SPC_POOL_DISPATCH(dtype, (pool_launch<T, kMaxFwd>(src, nullptr, nullptr, table, order, nullptr, dst, nullptr, n_rows, channels, kv, pitch, st)));
+    case kAvgFwd: SPC_POOL_DISPATCH(dtype, (pool_launch<T, kAvgFwd>(src, nullptr, nullptr, table, order, nullptr, dst, aux_out, n_rows, channels, kv, pitch, st)));
+    case kAvgBwd: SPC_POOL_DISPATCH(dtype, (pool_launch<T, kAvgBwd>(src, nullptr, nullptr, table, order, aux_in, dst, nullptr, n_rows, channels, kv, pitch, st)));
+    default: SPC_POOL_DISPATCH(dtype, (pool_launch<T, kMaxBwd>(src, own, ref, table, order, nullptr, dst, nullptr, n_rows, channels, kv, pitch, st)));
   }
+}
+
+extern "C" size_t spc_pool_row_order_workspace_bytes(int64_t n_rows) {
+  return kOrderBuckets * sizeof(int) + static_cast<size_t>(std::max<int64_t>(n_rows, 0)) * sizeof(int2);
+}
+
+extern "C" int spc_pool_row_order(const int32_t* table, int pitch, int kv, int64_t n_rows, int64_t n_targets, int32_t* order,
+                                  void* workspace, size_t workspace_bytes, void* stream) {
+  if (!table || !order || !workspace || pitch < kv || pitch % 4 != 0 || kv <= 0 || n_rows < 0 || n_rows >= (1ll << 31) ||
+      n_targets <= 0 || n_targets >= (1ll << 31) || workspace_bytes < spc_pool_row_order_workspace_bytes(n_rows) ||
+      ((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(workspace)) & 15u))
+    return fail(SPC_ERR_INVALID_ARGUMENT, "pool_row_order: bad arguments");
+  if (n_rows == 0) return SPC_OK;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  int* counts = static_cast<int*>(workspace);
+  int2* placed = reinterpret_cast<int2*>(counts + kOrderBuckets);
+  int shift = 0;
+  while (((n_targets - 1) >> shift) >= kOrderBuckets) ++shift;
+  const unsigned blocks = static_cast<unsigned>(ceil_div(n_rows, 256));
+  clear_buckets_kernel<<<kOrderBuckets / 1024, 1024, 0, st>>>(counts);
+  SPC_LAUNCH_OK();
+  count_buckets_kernel<<<blocks, 256, 0, st>>>(reinterpret_cast<const int4*>(table), pitch / 4, static_cast<int>(n_rows), shift, counts, placed);
+  SPC_LAUNCH_OK();
+  scan_buckets_kernel<<<1, 1024, 0, st>>>(counts);
+  SPC_LAUNCH_OK();
+  deal_buckets_kernel<<<blocks, 256, 0, st>>>(placed, counts, static_cast<int>(n_rows), order);
+  SPC_LAUNCH_OK();
+  return SPC_OK;
 }

@@ -171,3 +171,43 @@ def test_voxels_with_many_points(heavy):
     out = PointToVoxel(device=torch.device(DEV), **ctor).generate_voxel_with_id(pts.to(DEV))
     for got, want in zip(out, point_to_voxel(pts.numpy(), **ctor)):
         np.testing.assert_array_equal(to_np(got), want)
+
+
+@pytest.mark.parametrize("n,targets,channels", [(1, 1, 8), (255, 9000, 64), (1025, 8192, 256), (5000, 100_000, 40)])
+@pytest.mark.parametrize("average", [False, True])
+def test_pool_gradient_in_any_row_order(n, targets, channels, average):
+    """The order is a permutation by the first row read, and the average's gradient has the same bits with it and
+    without; the maximum's (no order) beside it."""
+    from spconv_triton_b200 import _lib
+
+    lib, kv, pitch = _lib.load(), 27, 28
+    gen = torch.Generator().manual_seed(n)
+    table = torch.randint(0, targets, (n, pitch), generator=gen, dtype=torch.int32)
+    table[torch.rand((n, pitch), generator=gen) < 0.6] = -1
+    table[:, kv:] = -1
+    first = torch.where(table >= 0, table, 0).gather(1, (table >= 0).int().argmax(1, keepdim=True))[:, 0]
+    table = table.to(DEV)
+    order = torch.empty(n, dtype=torch.int32, device=DEV)
+    scratch = torch.empty(lib.spc_pool_row_order_workspace_bytes(n), dtype=torch.uint8, device=DEV)
+    st = _lib.current_stream(table.device)
+    _lib.check(lib.spc_pool_row_order(_lib.ptr(table), pitch, kv, n, targets, _lib.ptr(order), _lib.ptr(scratch),
+                                      scratch.numel(), st))
+    assert torch.equal(order.sort().values.cpu(), torch.arange(n, dtype=torch.int32))
+    bucket = -(-targets // 8192)
+    assert bool((first[order.cpu().long()].diff() > -2 * bucket).all())
+    mk = lambda r: torch.randn((r, channels), generator=gen).to(DEV).half()  # noqa: E731
+    grad, own, ref = mk(targets), mk(n), mk(targets)
+    ref[::2] = own[torch.arange(0, targets, 2) % n]
+    count = torch.randint(1, 28, (targets,), generator=gen, dtype=torch.int32).to(DEV)
+    got = []
+    for rows in (None, order) if average else (None,):
+        dst = torch.full((n, channels), 7.0, device=DEV).half()
+        _lib.check(lib.spc_pool(2 if average else 3, _lib.ptr(grad), _lib.ptr(own), _lib.ptr(ref), _lib.ptr(table), pitch,
+                                _lib.ptr(rows), _lib.ptr(count), _lib.ptr(dst), None, n, channels, kv,
+                                _lib.dtype_code(torch.float16), st))
+        got.append(dst)
+    assert torch.equal(got[0], got[-1])
+    t = table[:, :kv].long()
+    there, t = (t >= 0)[:, :, None], t.clamp(min=0)
+    g = grad.double()[t] * (count.double()[t][:, :, None] if average else (ref[t] == own[:, None]).double())
+    assert rel_err(to_np(got[0].double()), to_np((g * there).sum(1))) <= TOL[torch.float16]
