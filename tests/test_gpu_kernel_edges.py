@@ -211,3 +211,22 @@ def test_pool_gradient_in_any_row_order(n, targets, channels, average):
     there, t = (t >= 0)[:, :, None], t.clamp(min=0)
     g = grad.double()[t] * (count.double()[t][:, :, None] if average else (ref[t] == own[:, None]).double())
     assert rel_err(to_np(got[0].double()), to_np((g * there).sum(1))) <= TOL[torch.float16]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("channels", [32, 128, 40])
+def test_average_of_16_bit_rows_is_the_rounded_fp32_average(dtype, channels):
+    """Sums and quotients of 16-bit rows have the bits of fp32 sums divided by the count, infinities, NaNs, zeros of
+    either sign and the smallest values among them."""
+    import spconv_triton_b200.pytorch as sp
+
+    idx = torch.from_numpy(unique_coords(5, 3000, 1, (24, 24, 24))).to(DEV)
+    x = torch.randn(3000, channels, device=DEV).to(dtype)
+    for at, value in enumerate((float("inf"), -float("inf"), float("nan"), -0.0, 6e-8, 65504.0)):
+        x[at::97, at % channels] = value
+    pool = sp.SparseAvgPool3d(3, 1, padding=1)
+    got = pool(sp.SparseConvTensor(x, idx, [24] * 3, 1)).features
+    exp = pool(sp.SparseConvTensor(x.float(), idx, [24] * 3, 1)).features.to(dtype)
+    assert torch.equal(got.isnan(), exp.isnan())
+    assert torch.equal(got.nan_to_num(7.0), exp.nan_to_num(7.0))
+    assert torch.equal(torch.signbit(got)[~got.isnan()], torch.signbit(exp)[~exp.isnan()])
