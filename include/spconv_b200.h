@@ -422,6 +422,9 @@ int spc_conv_backward_input(const void* grad_out, const void* weight,
 int spc_tf32_prepare(const float* src, float* dst, int64_t rows, int cols, int mode, void* stream);
 int spc_tf32_prepare_weight(const float* weight, float* dst, int c_out, int kv, int c_in,
                             int transpose, int mode, void* stream);
+/* Both in one launch, for callers that prepare the operands of one call. */
+int spc_tf32_prepare_operands(const float* src, float* dst, int64_t rows, int cols, int mode, const float* weight,
+                              float* weight_dst, int c_out, int kv, int c_in, int transpose, int weight_mode, void* stream);
 
 /* Bytes of device scratch spc_conv_backward_weight needs (fp32 partial sums
  * of the split reduction). */

@@ -15,7 +15,6 @@
 
 #include <memory>
 #include <mutex>
-#include <unordered_map>
 
 #include "../../include/spconv_b200.h"
 
@@ -187,61 +186,24 @@ Fp32Plan fp32_plan(int n_dim, int r_dim, int kv, bool tf32, int split_most) {
   }
   return p;
 }
-Tensor prepared_rows(const Tensor& x, const Fp32Plan& p) {
-  Tensor out = at::empty({x.size(0), p.mult * x.size(1)}, x.options());
-  check(spc_tf32_prepare(x.data_ptr<float>(), out.data_ptr<float>(), x.size(0), x.size(1), p.rows_mode, stream_of(x)));
-  return out;
-}
-
-// Prepared copies of weights, kept until the weight changes or goes away.  At most 256 weights.
-class WeightCache {
- public:
-  // transposed: 0 as it is, 1 as the input gradient reads it, 2 with the offsets reversed as well
-  Tensor get(const Tensor& w, int transposed, const Fp32Plan& p) {
-    const int slot = transposed * 8 + p.weight_mode;
-    auto* key = w.unsafeGetTensorImpl();
-    const uint32_t version = w.is_inference() ? 0 : w._version();
-    const auto stream = c10::cuda::getCurrentCUDAStream(w.device().index());
-    {
-      std::lock_guard<std::mutex> hold(lock_);
-      auto it = kept_.find(key);
-      if (it != kept_.end() && !w.is_inference()) {
-        Entry& e = it->second;
-        if (!e.owner.expired() && e.version == version && e.at == w.data_ptr() && e.stream == stream.stream()) {
-          auto hit = e.made.find(slot);
-          if (hit != e.made.end()) return hit->second;
-        }
-      }
-    }
-    const int64_t k_out = w.size(0), c_in = w.size(w.dim() - 1), kv = w.numel() / (k_out * c_in);
-    Tensor out = transposed ? at::empty({c_in, kv, p.mult * k_out}, w.options()) : at::empty({k_out, kv, p.mult * c_in}, w.options());
-    check(spc_tf32_prepare_weight(w.data_ptr<float>(), out.data_ptr<float>(), k_out, kv, c_in, transposed, p.weight_mode, stream.stream()));
-    if (w.is_inference()) return out;
-    std::lock_guard<std::mutex> hold(lock_);
-    Entry& e = kept_[key];
-    if (e.owner.expired() || e.version != version || e.at != w.data_ptr() || e.stream != stream.stream())
-      e = Entry{c10::weak_intrusive_ptr<c10::TensorImpl>(w.getIntrusivePtr()), version, w.data_ptr(), stream.stream(), {}};
-    e.made[slot] = out;
-    if (kept_.size() > 256)
-      for (auto it = kept_.begin(); it != kept_.end();)
-        it = it->second.owner.expired() || (kept_.size() > 256 && it->first != key) ? kept_.erase(it) : std::next(it);
-    return out;
-  }
-
- private:
-  struct Entry {
-    c10::weak_intrusive_ptr<c10::TensorImpl> owner{c10::intrusive_ptr<c10::TensorImpl>()};
-    uint32_t version = 0;
-    void* at = nullptr;
-    void* stream = nullptr;
-    std::unordered_map<int, Tensor> made;
-  };
-  std::mutex lock_;
-  std::unordered_map<c10::TensorImpl*, Entry> kept_;
+// The prepared copies of a call's operands, in one block and one launch; they live as long as the call.  (Kept from
+// one call for the next, a copy of the weight would have to notice every way in which a weight can change, those that
+// pass its version counter by among them, and outlive captures.)
+// transposed: 0 as it is, 1 as the input gradient reads it, 2 with the offsets reversed as well.
+struct Prepared {
+  Tensor block;
+  const float *rows, *weight;
 };
-WeightCache& weight_cache() {
-  static WeightCache* c = new WeightCache();  // (tensors must not outlive the CUDA context's end)
-  return *c;
+Prepared prepared(const Tensor& x, const Tensor& w, int transposed, const Fp32Plan& p) {
+  const int64_t k_out = w.size(0), c_in = w.size(w.dim() - 1), kv = w.numel() / (k_out * c_in);
+  const int64_t rows = p.mult * x.numel();  // (a multiple of eight: the weight's part starts at a 32-byte boundary)
+  Prepared out{at::empty({rows + p.mult * w.numel()}, x.options()), nullptr, nullptr};
+  float* at = out.block.data_ptr<float>();
+  check(spc_tf32_prepare_operands(x.data_ptr<float>(), at, x.size(0), x.size(1), p.rows_mode, w.data_ptr<float>(), at + rows, k_out, kv, c_in,
+                                  transposed, p.weight_mode, stream_of(x)));
+  out.rows = at;
+  out.weight = at + rows;
+  return out;
 }
 
 // ---- convolution -------------------------------------------------------------------------------------------------
@@ -273,12 +235,15 @@ Tensor conv_forward_raw(const Tensor& features, const Tensor& weight, const Tens
   if (b.defined()) b = b.contiguous();
   Tensor r = residual.defined() ? residual.contiguous() : residual;
   Tensor out = at::empty({n_out, k_out}, x.options().dtype(out_type));
+  const void *from = x.data_ptr(), *weights = w.data_ptr();
+  Prepared copies;
   int precision = x.scalar_type() == at::kFloat && o.tf32 ? SPC_PREC_TF32 : SPC_PREC_IEEE;
   if (x.scalar_type() == at::kFloat && out_type == at::kFloat) {
     const Fp32Plan plan = fp32_plan(k_out, c_in, kv, o.tf32, o.split_most);
     if (plan.tensor) {
-      x = prepared_rows(x, plan);
-      w = weight_cache().get(w, 0, plan);
+      copies = prepared(x, w, 0, plan);
+      from = copies.rows;
+      weights = copies.weight;
       c_in *= plan.mult;
       precision = SPC_PREC_TF32;
     }
@@ -286,7 +251,7 @@ Tensor conv_forward_raw(const Tensor& features, const Tensor& weight, const Tens
   const int type = code_of(x.scalar_type()), out_code = code_of(out_type);
   const bool colmajor = spc_conv_forward_needs_colmajor(c_in, k_out, kv, type, out_code, precision, SPC_GEMM_AUTO);
   const Rulebook::Side& t = rb->side(o.inverse, colmajor);
-  check(spc_conv_forward_residual(x.data_ptr(), w.data_ptr(), data(b), ints(t.cm), ints(t.rm), ints(t.order), out.data_ptr(), n_in, n_out,
+  check(spc_conv_forward_residual(from, weights, data(b), ints(t.cm), ints(t.rm), ints(t.order), out.data_ptr(), n_in, n_out,
                                   c_in, k_out, kv, type, out_code, precision, SPC_GEMM_AUTO,
                                   scale.defined() ? scale.data_ptr<float>() : nullptr, shift.defined() ? shift.data_ptr<float>() : nullptr,
                                   act, static_cast<float>(alpha), data(r), stream_of(x)));
@@ -305,12 +270,12 @@ Tensor conv_backward_input_raw(const Tensor& grad, const Tensor& weight, const B
   const Fp32Plan plan = type == SPC_F32 ? fp32_plan(c_in, k_out, kv, o.tf32, o.split_most) : Fp32Plan();
   if (plan.tensor) {
     // as a forward convolution of grad with the transposed weight
-    Tensor g = prepared_rows(grad, plan), wt = weight_cache().get(w, reversed ? 2 : 1, plan);
+    const Prepared copies = prepared(grad, w, reversed ? 2 : 1, plan);
     const bool colmajor = spc_conv_forward_needs_colmajor(plan.mult * k_out, c_in, kv, type, type, SPC_PREC_TF32, SPC_GEMM_AUTO);
     const Rulebook::Side& t = rb->side(input, colmajor);
-    check(spc_conv_forward(g.data_ptr(), wt.data_ptr(), nullptr, ints(t.cm), ints(t.rm), ints(t.order), din.data_ptr(), n_grad, n_in,
+    check(spc_conv_forward(copies.rows, copies.weight, nullptr, ints(t.cm), ints(t.rm), ints(t.order), din.data_ptr(), n_grad, n_in,
                            plan.mult * k_out, c_in, kv, type, type, SPC_PREC_TF32, SPC_GEMM_AUTO, nullptr, nullptr, SPC_ACT_NONE, 0.f,
-                           stream_of(g)));
+                           stream_of(grad)));
     return din;
   }
   const bool colmajor = spc_conv_backward_input_needs_colmajor(c_in, k_out, kv, type, precision, SPC_GEMM_AUTO);

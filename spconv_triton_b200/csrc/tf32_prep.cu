@@ -27,11 +27,11 @@ __device__ __forceinline__ float rna_tf32(float x) {
   return __uint_as_float(r);
 }
 
-// ROUND mode on 16-byte vectors (the whole matrix is one contiguous run)
-__global__ void __launch_bounds__(256)
-tf32_round4_kernel(const float4* __restrict__ src, float4* __restrict__ dst, long long n4) {
-  const long long stride = static_cast<long long>(gridDim.x) * 256;
-  for (long long i = blockIdx.x * 256ll + threadIdx.x; i < n4; i += stride) {
+// ROUND mode on 16-byte vectors (the whole matrix is one contiguous run), by `blocks` CTAs of which this is `block`
+__device__ __forceinline__ void round_rows(const float4* __restrict__ src, float4* __restrict__ dst, long long n4, unsigned block,
+                                           unsigned blocks) {
+  const long long stride = static_cast<long long>(blocks) * 256;
+  for (long long i = block * 256ll + threadIdx.x; i < n4; i += stride) {
     float4 v = __ldg(src + i);
     v.x = rna_tf32(v.x); v.y = rna_tf32(v.y); v.z = rna_tf32(v.z); v.w = rna_tf32(v.w);
     dst[i] = v;
@@ -39,9 +39,9 @@ tf32_round4_kernel(const float4* __restrict__ src, float4* __restrict__ dst, lon
 }
 
 // one thread per source element
-__global__ void __launch_bounds__(256)
-tf32_prepare_kernel(const float* __restrict__ src, float* __restrict__ dst, long long rows, int cols, int mode) {
-  const long long i = blockIdx.x * 256ll + threadIdx.x;
+__device__ __forceinline__ void prepare_rows(const float* __restrict__ src, float* __restrict__ dst, long long rows, int cols, int mode,
+                                             unsigned block) {
+  const long long i = block * 256ll + threadIdx.x;
   if (i >= rows * cols) return;
   const long long r = i / cols;
   const int c = static_cast<int>(i - r * cols);
@@ -60,10 +60,9 @@ tf32_prepare_kernel(const float* __restrict__ src, float* __restrict__ dst, long
 
 // weight [c_out, kv, c_in] -> dst [c_out, kv, m * c_in], or with `transpose` [c_in, kv, m * c_out]
 // (dst[c][k][n] = w[n][k][c]; 2: dst[c][kv - 1 - k][n]): the reduction index innermost, as the forward-form kernel reads it.
-__global__ void __launch_bounds__(256)
-tf32_prepare_weight_kernel(const float* __restrict__ w, float* __restrict__ dst, int c_out, int kv, int c_in,
-                           int transpose, int mode) {
-  const long long i = blockIdx.x * 256ll + threadIdx.x;
+__device__ __forceinline__ void prepare_weight(const float* __restrict__ w, float* __restrict__ dst, int c_out, int kv, int c_in,
+                                               int transpose, int mode, unsigned block) {
+  const long long i = block * 256ll + threadIdx.x;
   const long long total = static_cast<long long>(c_out) * kv * c_in;
   if (i >= total) return;
   const int c = static_cast<int>(i % c_in);
@@ -85,38 +84,77 @@ tf32_prepare_weight_kernel(const float* __restrict__ w, float* __restrict__ dst,
   }
 }
 
-}  // namespace
-}  // namespace spc
+struct Rows {
+  const float* src;
+  float* dst;
+  long long rows;
+  int cols, mode;
+  bool wide;        // whole 16-byte vectors
+  unsigned blocks;
+};
+struct Weight {
+  const float* src;
+  float* dst;
+  int c_out, kv, c_in, transpose, mode;
+  unsigned blocks;
+};
+// The first CTAs take the rows, the others the weight.
+__global__ void __launch_bounds__(256) tf32_prepare_kernel(const __grid_constant__ Rows x, const __grid_constant__ Weight w) {
+  if (blockIdx.x >= x.blocks)
+    prepare_weight(w.src, w.dst, w.c_out, w.kv, w.c_in, w.transpose, w.mode, blockIdx.x - x.blocks);
+  else if (x.wide)
+    round_rows(reinterpret_cast<const float4*>(x.src), reinterpret_cast<float4*>(x.dst), x.rows * x.cols / 4, blockIdx.x, x.blocks);
+  else
+    prepare_rows(x.src, x.dst, x.rows, x.cols, x.mode, blockIdx.x);
+}
 
-extern "C" int spc_tf32_prepare(const float* src, float* dst, int64_t rows, int cols, int mode, void* stream) {
-  using namespace spc;
+int rows_of(const float* src, float* dst, int64_t rows, int cols, int mode, Rows* x) {
   if (!src || !dst || rows < 0 || cols <= 0 || mode < SPC_TF32_ROUND || mode > SPC_TF32_SPLIT_B)
     return fail(SPC_ERR_INVALID_ARGUMENT, "tf32_prepare: bad arguments");
-  if (rows == 0) return SPC_OK;
   const long long total = static_cast<long long>(rows) * cols;
   const bool aligned = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15u) == 0;
-  if (mode == SPC_TF32_ROUND && total % 4 == 0 && aligned) {
-    const long long n4 = total / 4;
-    const unsigned blocks = static_cast<unsigned>(std::min<long long>(ceil_div(n4, 256), 8ll * sm_count()));
-    tf32_round4_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), n4);
-    SPC_LAUNCH_OK();
-    return SPC_OK;
-  }
-  tf32_prepare_kernel<<<static_cast<unsigned>(ceil_div(total, 256)), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      src, dst, rows, cols, mode);
+  const bool wide = mode == SPC_TF32_ROUND && total % 4 == 0 && aligned;
+  const long long blocks = wide ? std::min<long long>(ceil_div(total / 4, 256), 8ll * sm_count()) : ceil_div(total, 256);
+  *x = Rows{src, dst, rows, cols, mode, wide, static_cast<unsigned>(blocks)};
+  return SPC_OK;
+}
+int weight_of(const float* weight, float* dst, int c_out, int kv, int c_in, int transpose, int mode, Weight* w) {
+  if (!weight || !dst || c_out <= 0 || kv <= 0 || c_in <= 0 || mode < SPC_TF32_ROUND || mode > SPC_TF32_SPLIT_B)
+    return fail(SPC_ERR_INVALID_ARGUMENT, "tf32_prepare_weight: bad arguments");
+  const long long total = static_cast<long long>(c_out) * kv * c_in;
+  *w = Weight{weight, dst, c_out, kv, c_in, transpose, mode, static_cast<unsigned>(ceil_div(total, 256))};
+  return SPC_OK;
+}
+int launch(const Rows& x, const Weight& w, void* stream) {
+  if (x.blocks + w.blocks == 0) return SPC_OK;
+  tf32_prepare_kernel<<<x.blocks + w.blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(x, w);
   SPC_LAUNCH_OK();
   return SPC_OK;
 }
 
+}  // namespace
+}  // namespace spc
+
+using namespace spc;
+
+extern "C" int spc_tf32_prepare(const float* src, float* dst, int64_t rows, int cols, int mode, void* stream) {
+  Rows x{};
+  const int rc = rows_of(src, dst, rows, cols, mode, &x);
+  return rc != SPC_OK ? rc : launch(x, Weight{}, stream);
+}
+
 extern "C" int spc_tf32_prepare_weight(const float* weight, float* dst, int c_out, int kv, int c_in, int transpose,
                                        int mode, void* stream) {
-  using namespace spc;
-  if (!weight || !dst || c_out <= 0 || kv <= 0 || c_in <= 0 || mode < SPC_TF32_ROUND || mode > SPC_TF32_SPLIT_B)
-    return fail(SPC_ERR_INVALID_ARGUMENT, "tf32_prepare_weight: bad arguments");
-  const long long total = static_cast<long long>(c_out) * kv * c_in;
-  tf32_prepare_weight_kernel<<<static_cast<unsigned>(ceil_div(total, 256)), 256, 0,
-                               static_cast<cudaStream_t>(stream)>>>(weight, dst, c_out, kv, c_in, transpose, mode);
-  SPC_LAUNCH_OK();
-  return SPC_OK;
+  Weight w{};
+  const int rc = weight_of(weight, dst, c_out, kv, c_in, transpose, mode, &w);
+  return rc != SPC_OK ? rc : launch(Rows{}, w, stream);
+}
+
+extern "C" int spc_tf32_prepare_operands(const float* src, float* dst, int64_t rows, int cols, int mode, const float* weight,
+                                         float* weight_dst, int c_out, int kv, int c_in, int transpose, int weight_mode, void* stream) {
+  Rows x{};
+  Weight w{};
+  int rc = rows_of(src, dst, rows, cols, mode, &x);
+  if (rc == SPC_OK) rc = weight_of(weight, weight_dst, c_out, kv, c_in, transpose, weight_mode, &w);
+  return rc != SPC_OK ? rc : launch(x, w, stream);
 }

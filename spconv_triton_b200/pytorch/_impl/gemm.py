@@ -78,25 +78,12 @@ def _prepared_rows(x, mode, mult):
 
 
 def _prepared_weight(w, transpose, mode, mult):
-    """Prepared copy of the KRSC weight, remembered on the tensor until it changes."""
-    owner = w._base if w._base is not None else w  # the layer's parameter when ``w`` is a reshaped view of it
-    key = (w._version, w.data_ptr(), tuple(w.shape), bool(transpose), mode)
-    cache = getattr(owner, "_spc_tf32", None)
-    if cache is None:
-        cache = {}
-        try:
-            owner._spc_tf32 = cache
-        except AttributeError:
-            pass
-    hit = cache.get((bool(transpose), mode))
-    if hit is not None and hit[0] == key:
-        return hit[1]
+    """Prepared copy of the KRSC weight [K, kv, C]."""
     k_out, kv, c_in = w.shape
     shape = (c_in, kv, mult * k_out) if transpose else (k_out, kv, mult * c_in)
     out = torch.empty(shape, dtype=torch.float32, device=w.device)
     _lib.check(_lib.load().spc_tf32_prepare_weight(_lib.ptr(w), _lib.ptr(out), k_out, kv, c_in, int(bool(transpose)),
                                                    mode, _lib.current_stream(w.device)))
-    cache[(bool(transpose), mode)] = (key, out)
     return out
 
 
