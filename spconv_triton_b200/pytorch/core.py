@@ -40,6 +40,23 @@ class _Record:
         for name in self._fields:
             setattr(self, name, values[name])
 
+    # A copy (copy.deepcopy, pickle, torch.save) holds the tables themselves, not what would make them or the
+    # layer's rulebook, which belong to this process.
+    _on_demand: tuple = ()
+
+    def __getstate__(self):
+        for name in self._fields:
+            getattr(self, name)
+        state = dict(self.__dict__)
+        for name in ("_rb", *self._on_demand):
+            if name in state:
+                state[name] = None
+        for name, value in state.items():
+            if isinstance(value, torch.Tensor) and getattr(value, "_spc_late", None) is not None:
+                state[name] = plain = value.detach()
+                plain._spc_rowmajor = getattr(value, "_spc_rowmajor", None)
+        return state
+
 
 class IndiceData(_Record):
     """Native-format rulebook cached under an ``indice_key`` (reference: core.py:47-76)."""
@@ -50,6 +67,8 @@ class IndiceData(_Record):
     def __init__(self, out_indices, indices, indice_pairs, indice_pair_num, spatial_shape, out_spatial_shape,
                  is_subm: bool, algo: ConvAlgo, ksize, stride, dilation, padding, voxel_num: Any = None):
         self._assign(locals())
+
+    _on_demand = ("_pairs_thunk",)
 
     # An entry made from a layer's rulebook (``_rb``) has no pair lists until somebody reads them.
     def _resolved_pairs(self, name):
@@ -87,6 +106,8 @@ class ImplicitGemmIndiceData(_Record):
                  out_voxel_num: Any = None):
         self._late = None
         self._assign(locals())
+
+    _on_demand = ("_late", "_pair_fwd_thunk", "_masks_fwd_thunk")
 
     # The input-side tables of a strided layer may be pending (an inference forward does
     # not build them); reading any of the three attributes builds them.

@@ -1,0 +1,42 @@
+"""Host-side records: entries read by several threads or written by the user, containers that are copied after a
+pass, folded statistics.  No GPU needed."""
+
+import copy
+import pickle
+import threading
+import time
+
+import numpy as np
+import torch
+
+import spconv_triton_b200.pytorch as sp
+from spconv_triton_b200.core import ConvAlgo
+from spconv_triton_b200.pytorch.core import ImplicitGemmIndiceData
+
+
+def _entry():
+    return ImplicitGemmIndiceData(torch.zeros(3, 4), torch.zeros(3, 4), None, torch.Tensor(), None, [], None, [],
+                                  [np.array([0xFFFFFFFF], dtype=np.uint32)], [4] * 3, [2] * 3, False,
+                                  ConvAlgo.MaskImplicitGemm, [3] * 3, [2] * 3, [1] * 3, [1] * 3)
+
+
+class _Late:
+    def __init__(self):
+        self.calls = 0
+
+    def get(self):
+        self.calls += 1
+        time.sleep(0.05)
+        return torch.ones(2), [torch.ones(3)], [torch.ones(4)]
+
+
+def test_copies_of_an_entry_hold_its_tables():
+    entry = _entry()
+    entry._late = _Late()
+    entry._pair_fwd_thunk = lambda: torch.zeros(5)
+    entry._rb = threading.Lock()  # (like a native rulebook: cannot be copied)
+    for clone in (copy.deepcopy, lambda e: pickle.loads(pickle.dumps(e))):
+        got = clone(entry)
+        assert got.pair_fwd.numel() == 5 and got.pair_bwd.numel() == 2 and got.__dict__.get("_rb") is None
+        assert got.ksize == [3] * 3 and got.algo == ConvAlgo.MaskImplicitGemm
+    assert entry._rb is not None
