@@ -106,6 +106,7 @@ class ImplicitGemmIndiceData(_Record):
                  out_voxel_num: Any = None):
         self._late = None
         self._assign(locals())
+        self._assigned = frozenset()
 
     _on_demand = ("_late", "_pair_fwd_thunk", "_masks_fwd_thunk")
 
@@ -115,8 +116,8 @@ class ImplicitGemmIndiceData(_Record):
         late = self.__dict__.get("_late")
         if late is not None:
             self.__dict__["_late"] = None
-            pair_bwd, pm_bwd, ma_bwd = late.get()
-            self.__dict__.update(_pair_bwd=pair_bwd, _pair_mask_bwd_splits=pm_bwd, _mask_argsort_bwd_splits=ma_bwd)
+            made = zip(("_pair_bwd", "_pair_mask_bwd_splits", "_mask_argsort_bwd_splits"), late.get(), strict=True)
+            self.__dict__.update((k, v) for k, v in made if k not in self._assigned)
         return self.__dict__[name]
 
     # The column-major table may be pending too (the native pass writes only the row-major copy when
@@ -136,7 +137,10 @@ class ImplicitGemmIndiceData(_Record):
     # A table that the user assigns counts from then on, not the layer's rulebook.
     def _set(self, name, v):
         self.__dict__["_rb"] = None
+        self._assigned |= {name}
         self.__dict__[name] = v
+
+    _assigned: frozenset = frozenset()
 
     pair_fwd = property(_resolved_fwd, _set_fwd)
 

@@ -30,6 +30,18 @@ class _Late:
         return torch.ones(2), [torch.ones(3)], [torch.ones(4)]
 
 
+def test_a_table_that_the_user_assigns_stays():
+    entry = _entry()
+    entry._late = _Late()
+    entry._masks_fwd_thunk = lambda: ([torch.zeros(6)], [torch.zeros(7)])
+    mine = torch.full((9,), 3.0)
+    entry.pair_bwd = mine
+    entry.mask_argsort_fwd_splits = [mine]
+    assert entry.pair_bwd is mine and entry.mask_argsort_fwd_splits[0] is mine
+    assert entry.pair_mask_bwd_splits[0].numel() == 3 and entry.pair_mask_fwd_splits[0].numel() == 6
+    assert entry.pair_bwd is mine and entry.mask_argsort_fwd_splits[0] is mine
+
+
 def test_copies_of_an_entry_hold_its_tables():
     entry = _entry()
     entry._late = _Late()
