@@ -6,6 +6,7 @@ spconv_triton/pytorch/core.py so that user models run unchanged.
 
 from __future__ import annotations
 
+import threading
 from typing import Any, Union
 
 import numpy as np
@@ -31,14 +32,38 @@ class ThrustSortAllocator:
         self.device = device
 
 
+_on_demand_lock = threading.RLock()  # held while tables are made; entries may be read by several threads
+
+
 class _Record:
-    """Plain attribute bag; subclasses list their fields in ``_fields``."""
+    """Plain attribute bag; subclasses list their fields in ``_fields``.  Some tables are made when first read:
+    ``_on_demand`` names the attributes that hold what makes them."""
 
     _fields: tuple = ()
+    _assigned: frozenset = frozenset()  # tables that the user has put in the place of pending ones: they stay
 
     def _assign(self, values: dict):
         for name in self._fields:
             setattr(self, name, values[name])
+        self._assigned = frozenset()
+
+    def _set(self, name, v):
+        with _on_demand_lock:
+            self.__dict__["_rb"] = None  # a table that the user assigns counts from then on, not the layer's rulebook
+            self._assigned |= {name}
+            self.__dict__[name] = v
+
+    def _made(self, name, maker, fields, make):
+        """The table ``name`` of ``fields``, which ``make`` makes from the attribute ``maker`` (None: they are there)."""
+        d = self.__dict__
+        if d.get(maker) is not None:
+            with _on_demand_lock:
+                source = d.get(maker)
+                if source is not None:
+                    made = zip(fields, make(source), strict=True)
+                    d.update((k, v) for k, v in made if k not in self._assigned)
+                    d[maker] = None  # last: who finds it gone finds the tables
+        return d[name]
 
     # A copy (copy.deepcopy, pickle, torch.save) holds the tables themselves, not what would make them or the
     # layer's rulebook, which belong to this process.
@@ -72,24 +97,12 @@ class IndiceData(_Record):
 
     # An entry made from a layer's rulebook (``_rb``) has no pair lists until somebody reads them.
     def _resolved_pairs(self, name):
-        d = self.__dict__
-        thunk = d.get("_pairs_thunk")
-        if thunk is not None:
-            d["_pairs_thunk"] = None
-            pairs, num = thunk()
-            for key, value in (("_indice_pairs", pairs), ("_indice_pair_num", num)):
-                if d.get(key) is None:
-                    d[key] = value
-        return d[name]
-
-    def _set_pairs(self, name, v):
-        self.__dict__["_rb"] = None  # the user's tables count from now on
-        self.__dict__[name] = v
+        return self._made(name, "_pairs_thunk", ("_indice_pairs", "_indice_pair_num"), lambda thunk: thunk())
 
     indice_pairs = property(lambda self: self._resolved_pairs("_indice_pairs"),
-                            lambda self, v: self._set_pairs("_indice_pairs", v))
+                            lambda self, v: self._set("_indice_pairs", v))
     indice_pair_num = property(lambda self: self._resolved_pairs("_indice_pair_num"),
-                               lambda self, v: self._set_pairs("_indice_pair_num", v))
+                               lambda self, v: self._set("_indice_pair_num", v))
 
 
 class ImplicitGemmIndiceData(_Record):
@@ -106,57 +119,29 @@ class ImplicitGemmIndiceData(_Record):
                  out_voxel_num: Any = None):
         self._late = None
         self._assign(locals())
-        self._assigned = frozenset()
 
     _on_demand = ("_late", "_pair_fwd_thunk", "_masks_fwd_thunk")
 
     # The input-side tables of a strided layer may be pending (an inference forward does
     # not build them); reading any of the three attributes builds them.
     def _resolved(self, name):
-        late = self.__dict__.get("_late")
-        if late is not None:
-            self.__dict__["_late"] = None
-            made = zip(("_pair_bwd", "_pair_mask_bwd_splits", "_mask_argsort_bwd_splits"), late.get(), strict=True)
-            self.__dict__.update((k, v) for k, v in made if k not in self._assigned)
-        return self.__dict__[name]
+        return self._made(name, "_late", ("_pair_bwd", "_pair_mask_bwd_splits", "_mask_argsort_bwd_splits"), lambda late: late.get())
 
     # The column-major table may be pending too (the native pass writes only the row-major copy when
     # that is all its kernels read): it is then the transpose of the copy, made when first read.
     def _resolved_fwd(self):
-        d = self.__dict__
-        thunk = d.get("_pair_fwd_thunk")
-        if thunk is not None:
-            d["_pair_fwd_thunk"] = None
-            d["_pair_fwd"] = thunk()
-        return d["_pair_fwd"]
+        return self._made("_pair_fwd", "_pair_fwd_thunk", ("_pair_fwd",), lambda thunk: (thunk(),))
 
     def _set_fwd(self, v):
         self.__dict__["_pair_fwd_thunk"] = None
         self._set("_pair_fwd", v)
-
-    # A table that the user assigns counts from then on, not the layer's rulebook.
-    def _set(self, name, v):
-        self.__dict__["_rb"] = None
-        self._assigned |= {name}
-        self.__dict__[name] = v
-
-    _assigned: frozenset = frozenset()
 
     pair_fwd = property(_resolved_fwd, _set_fwd)
 
     # ... and so may the sorted masks and their argsort: the native pass orders the rows for its own
     # kernels by a different key and leaves a thunk that makes the exactly sorted pair.
     def _resolved_masks(self, name):
-        d = self.__dict__
-        thunk = d.get("_masks_fwd_thunk")
-        if thunk is not None:
-            d["_masks_fwd_thunk"] = None
-            pm, ma = thunk()
-            if d.get("_pair_mask_fwd_splits") is None:  # not assigned by the user in the meantime
-                d["_pair_mask_fwd_splits"] = pm
-            if d.get("_mask_argsort_fwd_splits") is None:
-                d["_mask_argsort_fwd_splits"] = ma
-        return d[name]
+        return self._made(name, "_masks_fwd_thunk", ("_pair_mask_fwd_splits", "_mask_argsort_fwd_splits"), lambda thunk: thunk())
 
     pair_mask_fwd_splits = property(lambda self: self._resolved_masks("_pair_mask_fwd_splits"),
                                     lambda self, v: self._set("_pair_mask_fwd_splits", v))

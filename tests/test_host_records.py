@@ -30,6 +30,35 @@ class _Late:
         return torch.ones(2), [torch.ones(3)], [torch.ones(4)]
 
 
+def test_threads_read_an_entry_whose_tables_are_made_on_demand():
+    entry = _entry()
+    late, made = _Late(), []
+
+    def slow(result):
+        made.append(result)
+        time.sleep(0.05)
+        return result
+
+    entry._late = late
+    entry._pair_fwd_thunk = lambda: slow(torch.zeros(5))
+    entry._masks_fwd_thunk = lambda: slow(([torch.zeros(6)], [torch.zeros(7)]))
+    seen, gate = [], threading.Barrier(4)
+
+    def read():
+        gate.wait()
+        seen.append((entry.pair_fwd, entry.pair_mask_fwd_splits, entry.mask_argsort_fwd_splits, entry.pair_bwd,
+                     entry.pair_mask_bwd_splits, entry.mask_argsort_bwd_splits))
+
+    threads = [threading.Thread(target=read) for _ in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(seen) == 4 and late.calls == 1 and len(made) == 2
+    for values in seen:
+        assert [v.numel() if isinstance(v, torch.Tensor) else v[0].numel() for v in values] == [5, 6, 7, 2, 3, 4]
+
+
 def test_a_table_that_the_user_assigns_stays():
     entry = _entry()
     entry._late = _Late()
