@@ -5,6 +5,8 @@
 // direction, more than the kernels of a layer of a few thousand voxels take.  Here a layer is two calls (its
 // rulebook, its arithmetic) that release the interpreter lock; backward never enters Python.
 #include <ATen/autocast_mode.h>
+#include <ATen/cuda/CUDAEvent.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/function.h>
@@ -83,14 +85,23 @@ constexpr int64_t kOrderRows = 256;
 
 // The tables of one rulebook, output side and input side, made as they are asked for.  The kernels read the
 // row-major tables; the column-major ones serve the CUDA-core and weight-gradient kernels.
+//
+// Whoever builds a rulebook orders its streams as for any tensor.  Tables made later are made on the stream of the
+// call that asks first; `late` lets a call on another stream wait for them.
 struct Rulebook {
   std::shared_ptr<Geometry> geo;
   Tensor indices, out_indices, workspace;
   int64_t n_in = 0, n_out = 0;
   struct Side {
     Tensor rm, cm, order;
-  } fwd, bwd;
-  std::mutex lock;
+  };
+  struct Late {
+    c10::optional<c10::cuda::CUDAStream> stream;
+    at::cuda::CUDAEvent made;
+  };
+  Side fwd, bwd;
+  Late late_fwd, late_bwd;
+  mutable std::mutex lock;
 
   bool subm() const { return geo->subm; }
   Tensor make(int64_t a, int64_t b) const { return at::empty({a, b}, indices.options()); }
@@ -108,26 +119,44 @@ struct Rulebook {
     return s;
   }
   // The side whose rows are the output rows (of the layer, or of its inverse with `input`).
-  const Side& side(bool input, bool colmajor) {
-    std::lock_guard<std::mutex> hold(lock);
+  Side side(bool input, bool colmajor) {
     if (input && subm()) throw Failure(SPC_ERR_INVALID_ARGUMENT, "a submanifold rulebook has one side");
-    Side& s = input ? bwd : fwd;
+    std::lock_guard<std::mutex> hold(lock);
+    c10::cuda::CUDAGuard guard(indices.device());
+    const auto now = c10::cuda::getCurrentCUDAStream();
+    Side& kept = input ? bwd : fwd;
+    Late& late = input ? late_bwd : late_fwd;
+    const bool missing = !kept.rm.defined() || (colmajor && !kept.cm.defined());
+    if (!missing && !late.stream) return kept;
+    // A capture records its kernels and does not run them: it waits for nothing (what came before a capture is
+    // done when the graph runs), and tables that it makes are its own.
+    const bool capturing = c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
+    Side s = kept;
+    if (late.stream && *late.stream != now && !capturing) {
+      late.made.block(now);
+      for (const Tensor& t : {s.rm, s.cm, s.order})
+        if (t.defined()) t.record_stream(now);
+    }
+    if (!missing) return s;
     if (!s.rm.defined()) {
-      c10::cuda::CUDAGuard guard(indices.device());
-      Side made = new_side(n_in, colmajor);
-      tables(Tensor(), Side(), made);
-      s = made;
-    }
-    if (colmajor && !s.cm.defined()) {
-      c10::cuda::CUDAGuard guard(indices.device());
+      for (const Tensor& t : {indices, workspace}) t.record_stream(now);
+      s = new_side(n_in, colmajor);
+      tables(Tensor(), Side(), s);
+    } else {
       const int64_t n = s.rm.size(0);
-      Tensor cm = make(geo->kv, n);
-      check(spc_rowmajor_to_pairs(ints(s.rm), geo->kv, n, ints(cm), stream_of(indices)));
-      s.cm = cm;
+      s.rm.record_stream(now);
+      s.cm = make(geo->kv, n);
+      check(spc_rowmajor_to_pairs(ints(s.rm), geo->kv, n, ints(s.cm), now.stream()));
     }
+    if (capturing) return s;
+    kept = s;
+    late.made.record(now);
+    late.stream = now;
+    if (bwd.rm.defined()) workspace = Tensor();  // nothing is made from it any more
     return s;
   }
   std::vector<Tensor> parts() const {
+    std::lock_guard<std::mutex> hold(lock);
     std::vector<Tensor> all;
     for (const Tensor& t : {indices, out_indices, workspace, fwd.rm, fwd.cm, fwd.order, bwd.rm, bwd.cm, bwd.order})
       if (t.defined()) all.push_back(t);
@@ -155,7 +184,7 @@ Book build_rulebook(const std::shared_ptr<Geometry>& geo, Tensor indices, bool i
   rb->tables(geo->subm ? Tensor() : rb->out_indices, f, b);
   rb->fwd = f;
   rb->bwd = b;
-  if (geo->subm || b.rm.defined()) rb->workspace = Tensor();  // nothing is made from it any more
+  if (geo->subm || b.rm.defined()) rb->workspace = Tensor();
   return rb;
 }
 
@@ -250,7 +279,7 @@ Tensor conv_forward_raw(const Tensor& features, const Tensor& weight, const Tens
   }
   const int type = code_of(x.scalar_type()), out_code = code_of(out_type);
   const bool colmajor = spc_conv_forward_needs_colmajor(c_in, k_out, kv, type, out_code, precision, SPC_GEMM_AUTO);
-  const Rulebook::Side& t = rb->side(o.inverse, colmajor);
+  const Rulebook::Side t = rb->side(o.inverse, colmajor);
   check(spc_conv_forward_residual(from, weights, data(b), ints(t.cm), ints(t.rm), ints(t.order), out.data_ptr(), n_in, n_out,
                                   c_in, k_out, kv, type, out_code, precision, SPC_GEMM_AUTO,
                                   scale.defined() ? scale.data_ptr<float>() : nullptr, shift.defined() ? shift.data_ptr<float>() : nullptr,
@@ -272,14 +301,14 @@ Tensor conv_backward_input_raw(const Tensor& grad, const Tensor& weight, const B
     // as a forward convolution of grad with the transposed weight
     const Prepared copies = prepared(grad, w, reversed ? 2 : 1, plan);
     const bool colmajor = spc_conv_forward_needs_colmajor(plan.mult * k_out, c_in, kv, type, type, SPC_PREC_TF32, SPC_GEMM_AUTO);
-    const Rulebook::Side& t = rb->side(input, colmajor);
+    const Rulebook::Side t = rb->side(input, colmajor);
     check(spc_conv_forward(copies.rows, copies.weight, nullptr, ints(t.cm), ints(t.rm), ints(t.order), din.data_ptr(), n_grad, n_in,
                            plan.mult * k_out, c_in, kv, type, type, SPC_PREC_TF32, SPC_GEMM_AUTO, nullptr, nullptr, SPC_ACT_NONE, 0.f,
                            stream_of(grad)));
     return din;
   }
   const bool colmajor = spc_conv_backward_input_needs_colmajor(c_in, k_out, kv, type, precision, SPC_GEMM_AUTO);
-  const Rulebook::Side& t = rb->side(input, colmajor);
+  const Rulebook::Side t = rb->side(input, colmajor);
   check(spc_conv_backward_input_tables(grad.data_ptr(), w.data_ptr(), ints(t.cm), ints(t.rm), ints(t.order), din.data_ptr(), n_in, n_grad,
                                        c_in, k_out, kv, reversed, type, precision, SPC_GEMM_AUTO, stream_of(grad)));
   return din;
@@ -289,7 +318,7 @@ Tensor conv_backward_weight_raw(const Tensor& features, const Tensor& grad, at::
   const int64_t k_out = sizes[0], c_in = sizes[sizes.size() - 1], kv = rb->geo->kv;
   Tensor dw = at::empty(sizes, grad.options());
   Tensor x = features.scalar_type() == grad.scalar_type() ? features : features.to(grad.scalar_type());
-  const Rulebook::Side& t = rb->side(o.inverse, true);
+  const Rulebook::Side t = rb->side(o.inverse, true);
   const int64_t n_out = grad.size(0);
   const size_t bytes = spc_conv_backward_weight_workspace_bytes(n_out, c_in, k_out, kv);
   Tensor ws = at::empty({static_cast<int64_t>(std::max<size_t>(bytes, 16))}, grad.options().dtype(at::kByte));
@@ -417,7 +446,7 @@ Tensor pool_rows(int op, const Tensor& src, const Tensor& own, const Tensor& ref
                  const Tensor& aux_out) {
   const int64_t c = src.size(1);
   const bool flip = rb->subm() && input;  // (a pool over a submanifold neighbourhood: the table of the other side)
-  const Rulebook::Side& t = rb->side(input && !flip, false);
+  const Rulebook::Side t = rb->side(input && !flip, false);
   const int64_t n = t.rm.size(0);
   Tensor out = at::empty({n, c}, src.options());
   if (c == 0) return out;

@@ -1,0 +1,94 @@
+"""Tables that are made when somebody asks for them: on any stream and thread, and under capture."""
+
+import threading
+
+import numpy as np
+import pytest
+import torch
+
+from gpu_util import DEV, to_np, unique_coords
+from oracle import rulebook as orb
+
+pytestmark = pytest.mark.gpu
+
+SHAPE, N = (40, 40, 40), 9000
+
+
+def _book(colmajor=False):
+    """A strided rulebook without its input side, and the oracle's tables of both sides."""
+    from spconv_triton_b200.pytorch._impl import host
+
+    idx = unique_coords(11, N, 2, SHAPE)
+    geo, _ = host.geometry(2, SHAPE, (3,) * 3, (2,) * 3, (1,) * 3, (1,) * 3, (0,) * 3, False, False)
+    rb = host.ext().build_rulebook(geo, torch.from_numpy(idx).to(DEV), False, colmajor, True)
+    exp = orb.igemm_pairs(idx, 2, list(SHAPE), [3] * 3, [2] * 3, [1] * 3, [1] * 3, [0] * 3, False, False, True, False)
+    return rb, exp[2], exp[3]
+
+
+def test_a_table_made_on_one_stream_is_read_on_another():
+    """Behind 50 ms of other work on the stream that makes it, the table is not there yet when the second stream asks."""
+    rb, fwd, bwd = _book()
+    torch.cuda.synchronize()
+    first, second = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(first):
+        torch.cuda._sleep(100_000_000)
+        rb.colmajor(False)
+        rb.rowmajor(True)
+    with torch.cuda.stream(second):
+        got = [rb.colmajor(False).clone(), rb.rowmajor(True).clone(), rb.colmajor(True).clone()]
+    second.synchronize()
+    np.testing.assert_array_equal(to_np(got[0]), fwd)
+    np.testing.assert_array_equal(to_np(got[1])[:, :27].T, bwd)
+    np.testing.assert_array_equal(to_np(got[2]), bwd)
+
+
+def test_threads_ask_for_the_same_tables():
+    bad = []
+    for _ in range(8):
+        rb, fwd, bwd = _book()
+        torch.cuda.synchronize()
+        gate = threading.Barrier(4)
+
+        def work(colmajor_first):
+            with torch.cuda.stream(torch.cuda.Stream()):
+                gate.wait()
+                for input_side, want in ((True, bwd), (False, fwd)):
+                    cm = rb.colmajor(input_side) if colmajor_first else None
+                    rm = rb.rowmajor(input_side).clone()
+                    cm = (rb.colmajor(input_side) if cm is None else cm).clone()
+                    torch.cuda.current_stream().synchronize()
+                    if not (np.array_equal(to_np(cm), want) and np.array_equal(to_np(rm)[:, :27].T, want)):
+                        bad.append(input_side)
+
+        threads = [threading.Thread(target=work, args=(i % 2 == 0,)) for i in range(4)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    assert not bad
+
+
+def test_tables_asked_for_under_capture():
+    """A capture records the making of a table but does not run it: later calls make their own."""
+    rb, fwd, bwd = _book()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        inside = [rb.colmajor(False), rb.colmajor(True)]
+    np.testing.assert_array_equal(to_np(rb.colmajor(True)), bwd)
+    np.testing.assert_array_equal(to_np(rb.colmajor(False)), fwd)
+    graph.replay()
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(to_np(inside[0]), fwd)
+    np.testing.assert_array_equal(to_np(inside[1]), bwd)
+
+
+def test_scratch_goes_with_its_use():
+    """The scratch of a rulebook goes once both sides are there."""
+    rb, _, _ = _book()
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    rb.rowmajor(True)
+    made = rb.n_in * 28 * 4 + rb.n_in * 4
+    torch.cuda.synchronize()
+    assert torch.cuda.memory_allocated() <= before + made - 100_000  # (the scratch is larger than that)
