@@ -179,8 +179,10 @@ class LateTables:
                     p.workspace.numel(), _lib.ptr(pair_bwd), _lib.ptr(pm_bwd), _lib.ptr(ma_bwd), self.split_words,
                     self.n_split, int(bool(self.do_sort)), _lib.ptr(bwd_rm), _lib.current_stream(dev)))
                 pair_bwd._spc_rowmajor = bwd_rm
-            self.value = (pair_bwd, [pm_bwd[s] for s in range(self.n_split)],
-                          [ma_bwd[s] for s in range(self.n_split)])
+            value = (pair_bwd, [pm_bwd[s] for s in range(self.n_split)], [ma_bwd[s] for s in range(self.n_split)])
+            if torch.cuda.is_current_stream_capturing():
+                return value  # recorded, not made: it belongs to the graph
+            self.value = value
             self.p = None  # the workspace is no longer needed
         return self.value
 
@@ -304,7 +306,8 @@ def native_pair_to_tables(pair, indice_pair_num, n_in, n_out, inverse, need_bwd=
             _lib.check(_lib.load().spc_native_to_tables(
                 _lib.ptr(src), kv, n_pair, int(bool(inverse)), _lib.ptr(pf), int(n_out), _lib.ptr(pb),
                 int(n_in), _lib.current_stream(dev)))
-        cache[key] = (pf, pb)
+        if not torch.cuda.is_current_stream_capturing():  # (recorded, not made: it belongs to the graph)
+            cache[key] = (pf, pb)
     return pf, pb
 
 
@@ -319,8 +322,9 @@ def rowmajor_of(pair_table):
         with torch.cuda.device(dev):
             rm = torch.empty((n, (kv + 3) // 4 * 4), dtype=torch.int32, device=dev)
             _lib.check(_lib.load().spc_pairs_to_rowmajor(_lib.ptr(src), kv, n, _lib.ptr(rm), _lib.current_stream(dev)))
-        try:
-            pair_table._spc_rowmajor = rm
-        except AttributeError:
-            pass
+        if not torch.cuda.is_current_stream_capturing():
+            try:
+                pair_table._spc_rowmajor = rm
+            except AttributeError:
+                pass
     return rm

@@ -32,6 +32,20 @@ class ThrustSortAllocator:
         self.device = device
 
 
+def _tensors_of(res):
+    """Every tensor that nested lists and tuples hold, with the row-major copies of tables."""
+    stack = [res]
+    while stack:
+        item = stack.pop()
+        if isinstance(item, torch.Tensor):
+            yield item
+            extra = getattr(item, "_spc_rowmajor", None)
+            if extra is not None:
+                yield extra
+        elif isinstance(item, (list, tuple)):
+            stack.extend(item)
+
+
 _on_demand_lock = threading.RLock()  # held while tables are made; entries may be read by several threads
 
 
@@ -41,6 +55,7 @@ class _Record:
 
     _fields: tuple = ()
     _assigned: frozenset = frozenset()  # tables that the user has put in the place of pending ones: they stay
+    _ready: dict = {}  # of tables made on demand: (stream, event)
 
     def _assign(self, values: dict):
         for name in self._fields:
@@ -51,19 +66,36 @@ class _Record:
         with _on_demand_lock:
             self.__dict__["_rb"] = None  # a table that the user assigns counts from then on, not the layer's rulebook
             self._assigned |= {name}
+            self._ready = {k: e for k, e in self._ready.items() if k != name}
             self.__dict__[name] = v
 
     def _made(self, name, maker, fields, make):
-        """The table ``name`` of ``fields``, which ``make`` makes from the attribute ``maker`` (None: they are there)."""
+        """The table ``name`` of ``fields``, which ``make`` makes from the attribute ``maker`` (None: they are there).
+        They are made on the stream of the first reader; readers on other streams wait for them.  What a stream
+        capture makes belongs to its graph."""
         d = self.__dict__
         if d.get(maker) is not None:
             with _on_demand_lock:
                 source = d.get(maker)
                 if source is not None:
-                    made = zip(fields, make(source), strict=True)
-                    d.update((k, v) for k, v in made if k not in self._assigned)
+                    made = dict(zip(fields, make(source), strict=True))
+                    on_device = [t for t in _tensors_of(list(made.values())) if t.is_cuda]
+                    if on_device and torch.cuda.is_current_stream_capturing():
+                        return made[name] if name not in self._assigned else d[name]
+                    if on_device:
+                        stream = torch.cuda.current_stream(on_device[0].device)
+                        self._ready = {**self._ready, **dict.fromkeys(fields, (stream, stream.record_event()))}
+                    d.update((k, v) for k, v in made.items() if k not in self._assigned)
                     d[maker] = None  # last: who finds it gone finds the tables
-        return d[name]
+        value = d[name]
+        if name in self._ready:
+            stream, event = self._ready[name]
+            now = torch.cuda.current_stream(stream.device)
+            if now != stream and not torch.cuda.is_current_stream_capturing():
+                now.wait_event(event)
+                for t in _tensors_of(value):
+                    t.record_stream(now)
+        return value
 
     # A copy (copy.deepcopy, pickle, torch.save) holds the tables themselves, not what would make them or the
     # layer's rulebook, which belong to this process.
@@ -72,7 +104,7 @@ class _Record:
     def __getstate__(self):
         for name in self._fields:
             getattr(self, name)
-        state = dict(self.__dict__)
+        state = dict(self.__dict__, _ready={})
         for name in ("_rb", *self._on_demand):
             if name in state:
                 state[name] = None

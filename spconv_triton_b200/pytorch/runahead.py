@@ -32,7 +32,7 @@ from .. import constants
 from . import ops
 from ._impl import host as _host
 from ._impl import pairs as _pairs
-from .core import ImplicitGemmIndiceData, SparseConvTensor, register_implicit_gemm_indice_data
+from .core import ImplicitGemmIndiceData, SparseConvTensor, _tensors_of, register_implicit_gemm_indice_data
 
 _side_streams: dict = {}
 
@@ -44,20 +44,6 @@ def _side_stream(device: torch.device, which: int) -> torch.cuda.Stream:
     if key not in _side_streams:
         _side_streams[key] = torch.cuda.Stream(device=device, priority=-1)
     return _side_streams[key]
-
-
-def _tensors_of(res):
-    """Every tensor a rulebook tuple holds, with the row-major table copies."""
-    stack = [res]
-    while stack:
-        item = stack.pop()
-        if isinstance(item, torch.Tensor):
-            yield item
-            extra = getattr(item, "_spc_rowmajor", None)
-            if extra is not None:
-                yield extra
-        elif isinstance(item, (list, tuple)):
-            stack.extend(item)
 
 
 def flatten_convs(container) -> list:

@@ -92,3 +92,53 @@ def test_scratch_goes_with_its_use():
     made = rb.n_in * 28 * 4 + rb.n_in * 4
     torch.cuda.synchronize()
     assert torch.cuda.memory_allocated() <= before + made - 100_000  # (the scratch is larger than that)
+
+
+def test_an_entry_read_on_two_streams():
+    import spconv_triton_b200.pytorch as sp
+
+    idx = unique_coords(11, N, 2, SHAPE)
+    layer = sp.SparseConv3d(16, 16, 3, stride=2, padding=1, indice_key="d").to(DEV).half().eval()
+    with torch.no_grad():
+        y = layer(sp.SparseConvTensor(torch.randn(N, 16, device=DEV).half(), torch.from_numpy(idx).to(DEV), list(SHAPE), 2))
+    entry = y.indice_dict["d"]
+    torch.cuda.synchronize()
+    first, second = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(first):
+        torch.cuda._sleep(100_000_000)
+        entry.pair_fwd, entry.pair_bwd, entry.mask_argsort_fwd_splits
+    with torch.cuda.stream(second):
+        got = [entry.pair_fwd.clone(), entry.pair_bwd.clone(), entry.mask_argsort_fwd_splits[0].clone()]
+    second.synchronize()
+    exp = orb.igemm_pairs(idx, 2, list(SHAPE), [3] * 3, [2] * 3, [1] * 3, [1] * 3, [0] * 3, False, False, True, False)
+    for g, e in zip(got, (exp[2], exp[3], exp[6][0])):
+        np.testing.assert_array_equal(to_np(g), e)
+
+
+def test_tables_of_the_operator_functions_under_capture():
+    """What the operator functions remember on a pair list or a table is not what a capture has recorded."""
+    import spconv_triton_b200.pytorch as sp
+    from spconv_triton_b200.core import ConvAlgo
+    from spconv_triton_b200.pytorch import ops
+    from spconv_triton_b200.pytorch._impl import pairs
+
+    idx = torch.from_numpy(unique_coords(11, N, 2, SHAPE)).to(DEV)
+    _, lists, num = ops.get_indice_pairs(idx, 2, list(SHAPE), ConvAlgo.Native, [3] * 3, [1] * 3, [1] * 3, [1] * 3, [0] * 3, True)
+    layer = sp.SparseConv3d(16, 16, 3, stride=2, padding=1, indice_key="d").to(DEV).half().eval()
+    with torch.no_grad(), pairs.deferred_backward("late"):
+        res = ops.get_indice_pairs_implicit_gemm(idx, 2, list(SHAPE), layer.algo, layer.kernel_size, layer.stride, layer.padding,
+                                                 layer.dilation, [0] * 3)
+    late = res[2]._spc_late
+    plain = res[2].clone()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(torch.cuda.CUDAGraph()):
+        pairs.native_pair_to_tables(lists, num, N, N, False)
+        pairs.rowmajor_of(plain)
+        late.get()
+    exp = orb.igemm_pairs(to_np(idx), 2, list(SHAPE), [3] * 3, [2] * 3, [1] * 3, [1] * 3, [0] * 3, False, False, True, False)
+    fwd, bwd = pairs.native_pair_to_tables(lists, num, N, N, False)
+    want = orb.native_pair_to_tables(to_np(lists), N, N, False, True)
+    np.testing.assert_array_equal(to_np(fwd), want[0])
+    np.testing.assert_array_equal(to_np(bwd), want[1])
+    np.testing.assert_array_equal(to_np(pairs.rowmajor_of(plain))[:, :27].T, exp[2])
+    np.testing.assert_array_equal(to_np(late.get()[0]), exp[3])
