@@ -393,6 +393,7 @@ struct ConvBackward : public torch::autograd::Node {
     std::lock_guard<std::mutex> hold(mutex_);
     features_.reset_data();
     weight_.reset_data();
+    rb.reset();
   }
   std::string name() const override { return "SparseImplicitGemmFunctionBackward"; }
 };
@@ -495,6 +496,7 @@ struct PoolBackward : public torch::autograd::Node {
     features_.reset_data();
     out_.reset_data();
     count_.reset_data();
+    rb.reset();
   }
   std::string name() const override {
     return average ? "SparseAvgPoolImplicitGemmFunctionBackward" : "SparseMaxPoolImplicitGemmFunctionBackward";

@@ -142,3 +142,29 @@ def test_tables_of_the_operator_functions_under_capture():
     np.testing.assert_array_equal(to_np(bwd), want[1])
     np.testing.assert_array_equal(to_np(pairs.rowmajor_of(plain))[:, :27].T, exp[2])
     np.testing.assert_array_equal(to_np(late.get()[0]), exp[3])
+
+
+def test_tables_go_when_backward_has_run():
+    """... and not with the last tensor that keeps the graph's nodes."""
+    import spconv_triton_b200.pytorch as sp
+
+    layer = sp.SparseConv3d(16, 16, 3, stride=2, padding=1).to(DEV)
+    idx = torch.from_numpy(unique_coords(11, N, 2, SHAPE)).to(DEV)
+    x = torch.randn(N, 16, device=DEV, requires_grad=True)
+    loss = layer(sp.SparseConvTensor(x, idx, list(SHAPE), 2)).features.sum()
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    loss.backward()  # (`loss` keeps the graph's nodes)
+    grads = sum(t.grad.numel() * 4 for t in (x, *layer.parameters()))
+    torch.cuda.synchronize()
+    assert torch.cuda.memory_allocated() <= before + grads - N * 28 * 4
+    with pytest.raises(RuntimeError, match="second time"):
+        loss.backward()
+    pool = sp.SparseMaxPool3d(2, 2)
+    x = torch.randn(N, 16, device=DEV, requires_grad=True)
+    loss = pool(sp.SparseConvTensor(x, idx, list(SHAPE), 2)).features.sum()
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    loss.backward()
+    torch.cuda.synchronize()
+    assert torch.cuda.memory_allocated() <= before + x.grad.numel() * 4 - N * 8 * 4
