@@ -1367,9 +1367,8 @@ struct Layout {
   const uint32_t* shared_prefix = nullptr;
   const uint32_t* shared_cells = nullptr;  // the cells of those rows
 };
-// counts and taken of the tile order
-// (one set for each side of a layer)
-constexpr size_t kOrderCountBytes = 2 * ((kTileBuckets * 4 + 255) / 256) * 256;
+// bucket counts of the tile order (one set for each side of a layer)
+constexpr size_t kOrderCountBytes = kTileOrderWords * 4;
 
 inline int cell_blocks(int64_t words) { return static_cast<int>(ceil_div(words, kCellBlock)); }
 
@@ -1821,7 +1820,7 @@ struct MaskSplits {
 };
 
 // Scratch of the tile order; the input side of a strided layer has keys and counts of its own, so that both
-// sides come out of one pass.
+// sides come out of one pass.  The counts are zero after phase 1 and after every order.
 uint32_t* order_keys(const Layout& L, char* ws, bool input) {
   return reinterpret_cast<uint32_t*>(ws + (input ? L.off_keys_b : L.off_keys_a));
 }
@@ -1830,8 +1829,7 @@ uint32_t* bucket_counts(const Layout& L, char* ws, int64_t n, bool input) {
 }
 int emit_order(const Layout& L, char* ws, int64_t n, int kv, int32_t* order, bool input, cudaStream_t st) {
   uint32_t* counts = reinterpret_cast<uint32_t*>(ws + L.off_order_counts + (input ? kOrderCountBytes : 0));
-  return tile_order(order_keys(L, ws, input), n, kv, counts, counts + kOrderCountBytes / 8,
-                    reinterpret_cast<uint2*>(ws + L.off_order_pairs), order, st);
+  return tile_order(order_keys(L, ws, input), n, kv, counts, reinterpret_cast<uint2*>(ws + L.off_order_pairs), order, st);
 }
 // Keys or words of the rows that a fill kernel owns.
 void ask_fill(const Layout& L, char* ws, int64_t n, const SideTables& t, const MaskSplits& m, bool input, FillOut* out) {

@@ -90,15 +90,18 @@ deal_rows_kernel(const uint32_t* __restrict__ keys, long long n, const uint32_t*
 // offsets of a 3x3x3 kernel.  A warp ranks its rows 32 at a time (lanes with the same digit find each other
 // with nine ballots, the first of them adds to the warp's count of that digit), then the counts of all warps
 // become places by one block-wide sum in (digit, warp) order, which keeps the sort stable.
+// `used` (may be null): the bucket counts that the rows have been dealt by, zeroed for the next order.
 template <int ITEMS>
 __global__ void __launch_bounds__(kPieceThreads)
 sort_piece_kernel(const uint32_t* __restrict__ keys, const uint2* __restrict__ pairs, long long n, int key_bits,
-                  int32_t* __restrict__ order) {
+                  int32_t* __restrict__ order, uint32_t* __restrict__ used) {
   extern __shared__ __align__(16) unsigned char smem[];
   uint2* item = reinterpret_cast<uint2*>(smem);                                   // [kPieceThreads * ITEMS]
   uint16_t* count = reinterpret_cast<uint16_t*>(item + kPieceThreads * ITEMS);    // [kDigits][kPieceWarps]
   __shared__ uint32_t warp_sum[kPieceWarps];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (used != nullptr)
+    for (int i = blockIdx.x * kPieceThreads + tid; i < kTileOrderWords; i += gridDim.x * kPieceThreads) used[i] = 0u;
   const long long first = blockIdx.x * static_cast<long long>(kPieceThreads * ITEMS);
   const int left = static_cast<int>(n - first < kPieceThreads * ITEMS ? n - first : kPieceThreads * ITEMS);
   uint2 mine[ITEMS];
@@ -181,34 +184,33 @@ sort_piece_kernel(const uint32_t* __restrict__ keys, const uint2* __restrict__ p
 }
 
 template <int ITEMS>
-int launch_sort(const uint32_t* keys, const uint2* pairs, int64_t n, int key_bits, int32_t* order, cudaStream_t st) {
+int launch_sort(const uint32_t* keys, const uint2* pairs, int64_t n, int key_bits, int32_t* order, uint32_t* used, cudaStream_t st) {
   static bool configured[kMaxDevices] = {false};
   constexpr int bytes = kPieceThreads * ITEMS * static_cast<int>(sizeof(uint2)) + kDigits * kPieceWarps * 2;
   SPC_CUDA_OK(ensure_dynamic_smem(sort_piece_kernel<ITEMS>, bytes, configured));
   const unsigned blocks = static_cast<unsigned>(ceil_div(n, kPieceThreads * ITEMS));
-  sort_piece_kernel<ITEMS><<<blocks, kPieceThreads, bytes, st>>>(keys, pairs, n, key_bits, order);
+  sort_piece_kernel<ITEMS><<<blocks, kPieceThreads, bytes, st>>>(keys, pairs, n, key_bits, order, used);
   SPC_LAUNCH_OK();
   return SPC_OK;
 }
 
 }  // namespace
 
-int tile_order(const uint32_t* keys, int64_t n, int kv, const uint32_t* counts, uint32_t* taken, uint2* pairs,
-               int32_t* order, cudaStream_t st) {
+int tile_order(const uint32_t* keys, int64_t n, int kv, uint32_t* counts, uint2* pairs, int32_t* order, cudaStream_t st) {
   constexpr int kItems = kTileOrderPiece / kPieceThreads;
   if (!tile_order_needs_buckets(n)) {
     // one piece: exact, and no larger than it has to be (the fewer rows a thread holds, the sooner it is done)
-    if (n <= kPieceThreads) return launch_sort<1>(keys, nullptr, n, kv, order, st);
-    if (n <= 2 * kPieceThreads) return launch_sort<2>(keys, nullptr, n, kv, order, st);
-    if (n <= 4 * kPieceThreads) return launch_sort<4>(keys, nullptr, n, kv, order, st);
-    return launch_sort<kItems>(keys, nullptr, n, kv, order, st);
+    if (n <= kPieceThreads) return launch_sort<1>(keys, nullptr, n, kv, order, nullptr, st);
+    if (n <= 2 * kPieceThreads) return launch_sort<2>(keys, nullptr, n, kv, order, nullptr, st);
+    if (n <= 4 * kPieceThreads) return launch_sort<4>(keys, nullptr, n, kv, order, nullptr, st);
+    return launch_sort<kItems>(keys, nullptr, n, kv, order, nullptr, st);
   }
   // pieces of 4096 rows where they still fit one wave of CTAs: the sort is as long as one piece takes
   const bool small = n <= static_cast<int64_t>(sm_count()) * kTileOrderPiece / 2;
   const unsigned blocks = static_cast<unsigned>(ceil_div(n, kDealThreads * kDealItems));
-  deal_rows_kernel<<<blocks, kDealThreads, 0, st>>>(keys, n, counts, taken, pairs);
+  deal_rows_kernel<<<blocks, kDealThreads, 0, st>>>(keys, n, counts, counts + kTileOrderWords / 2, pairs);
   SPC_LAUNCH_OK();
-  return small ? launch_sort<kItems / 2>(keys, pairs, n, kv, order, st) : launch_sort<kItems>(keys, pairs, n, kv, order, st);
+  return small ? launch_sort<kItems / 2>(keys, pairs, n, kv, order, counts, st) : launch_sort<kItems>(keys, pairs, n, kv, order, counts, st);
 }
 
 }  // namespace spc

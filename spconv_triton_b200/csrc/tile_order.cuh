@@ -13,6 +13,9 @@ constexpr int kTileOrderPiece = 8192;
 // Sets of at most three of 32 offsets: 1 + 32 + 496 + 4960.
 constexpr int kTileBuckets = 5489;
 
+// Words of scratch of one order: the rows of every bucket, then how many of them have been dealt.
+constexpr int kTileOrderWords = 2 * ((kTileBuckets + 63) / 64 * 64);
+
 inline bool tile_order_needs_buckets(int64_t n) { return n > kTileOrderPiece; }
 
 // The order the gather-GEMM wants is not the numeric order of the mask words but one in which the
@@ -52,9 +55,10 @@ __device__ __forceinline__ int bucket_of(uint32_t word) {
   return upto3 + (upto2 - 1 - inner);
 }
 
-// Ascending order (as above) of `n` rows by key; kv <= 32 offsets make the keys.  `counts` (rows per bucket, made
-// by the caller), `taken` (zeroed) and `pairs` (n entries) are read only where tile_order_needs_buckets(n).
-int tile_order(const uint32_t* keys, int64_t n, int kv, const uint32_t* counts, uint32_t* taken, uint2* pairs,
-               int32_t* order, cudaStream_t st);
+// Ascending order (as above) of `n` rows by key; kv <= 32 offsets make the keys.  `counts` (kTileOrderWords words, the
+// rows per bucket made by the caller, the rest zero) and `pairs` (n entries) are used only where
+// tile_order_needs_buckets(n); every word of `counts` is zero again afterwards, so that the next order of the same
+// scratch can be counted into it.
+int tile_order(const uint32_t* keys, int64_t n, int kv, uint32_t* counts, uint2* pairs, int32_t* order, cudaStream_t st);
 
 }  // namespace spc

@@ -1,0 +1,48 @@
+"""The C ABI of the rulebooks called as its header allows."""
+
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from gpu_util import DEV, to_np, unique_coords
+from oracle import rulebook as orb
+
+pytestmark = pytest.mark.gpu
+
+
+def _prepared(shape, n, batch, stride, subm):
+    from spconv_triton_b200 import _lib
+
+    lib, nd = _lib.load(), len(shape)
+    out = list(shape) if subm else [(s + 2 - 3) // stride + 1 for s in shape]
+    geo = _lib.make_geometry(batch, list(shape), out, [3] * nd, [stride] * nd, [1] * nd, [1] * nd, subm, False)
+    coords = unique_coords(n, n, batch, shape)
+    idx = torch.from_numpy(coords).to(DEV)
+    ws = torch.empty(int(lib.spc_rulebook_workspace_bytes(ctypes.byref(geo), n)), dtype=torch.uint8, device=DEV)
+    n_out = ctypes.c_int64(0)
+    st = _lib.current_stream(idx.device)
+    _lib.check(lib.spc_rulebook_prepare(ctypes.byref(geo), _lib.ptr(idx), n, _lib.ptr(ws), ws.numel(), ctypes.byref(n_out), st))
+
+    def tables(**want):
+        names = ("out_indices", "pair_fwd", "pair_fwd_rowmajor", "order_fwd", "pair_bwd", "pair_bwd_rowmajor", "order_bwd")
+        _lib.check(lib.spc_rulebook_tables(ctypes.byref(geo), _lib.ptr(idx), n, n_out.value, _lib.ptr(ws), ws.numel(),
+                                           *[_lib.ptr(want.get(k)) for k in names], _lib.current_stream(idx.device)))
+
+    exp = orb.igemm_pairs(coords, batch, list(shape), [3] * nd, [stride] * nd, [1] * nd, [1] * nd, [0] * nd, subm, False, True, False)
+    return tables, n, int(n_out.value), exp
+
+
+@pytest.mark.parametrize("n,subm", [(8191, True), (8193, True), (30000, True), (9000, False), (40000, False)])
+def test_a_row_order_asked_for_again(n, subm):
+    """... is an order of the rows again, of either side, whether or not the rows fit one piece."""
+    tables, n_in, n_out, _ = _prepared((64, 64, 48), n, 2, 2, subm)
+    for _ in range(3):
+        order = torch.full((n_out,), -1, dtype=torch.int32, device=DEV)
+        tables(order_fwd=order, **({} if subm else {"out_indices": torch.empty((n_out, 4), dtype=torch.int32, device=DEV)}))
+        assert torch.equal(order.sort().values.cpu(), torch.arange(n_out, dtype=torch.int32))
+        if not subm:
+            order = torch.full((n_in,), -1, dtype=torch.int32, device=DEV)
+            tables(order_bwd=order)
+            assert torch.equal(order.sort().values.cpu(), torch.arange(n_in, dtype=torch.int32))
