@@ -58,9 +58,11 @@ class _Record:
     _ready: dict = {}  # of tables made on demand: (stream, event)
 
     def _assign(self, values: dict):
-        for name in self._fields:
-            setattr(self, name, values[name])
-        self._assigned = frozenset()
+        tables = type(self)._tables
+        self.__dict__.update(("_" + name if name in tables else name, values[name]) for name in self._fields)
+
+    def __init_subclass__(cls):
+        cls._tables = frozenset(name for name in cls._fields if isinstance(vars(cls).get(name), property))
 
     def _set(self, name, v):
         with _on_demand_lock:
@@ -149,7 +151,6 @@ class ImplicitGemmIndiceData(_Record):
                  mask_argsort_fwd_splits, mask_argsort_bwd_splits, masks, spatial_shape, out_spatial_shape,
                  is_subm: bool, algo: ConvAlgo, ksize, stride, dilation, padding, in_voxel_num: Any = None,
                  out_voxel_num: Any = None):
-        self._late = None
         self._assign(locals())
 
     _on_demand = ("_late", "_pair_fwd_thunk", "_masks_fwd_thunk")
