@@ -326,20 +326,26 @@ enum Counter { kUniqueCount = 0, kStatus = 1, kUnsorted = 2, kTicket = 3 };
 // ------------------------------------------------------------------------
 // Scratch regions are cleared by a kernel rather than by cudaMemsetAsync, and all of them by one launch: a
 // kernel can neither be routed to a copy engine (where it would queue behind a large transfer of the
-// application) nor cost a driver memset's set-up.  Regions are 16-byte multiples at 16-byte offsets.
+// application) nor cost a driver memset's set-up.  Regions are whole words and may start and end anywhere: the
+// caller's tables do.
 struct Clear {
   static constexpr int kMost = 8;
-  uint4* at[kMost];
+  uint4* at[kMost];         // the 16-byte vectors of a region,
   long long n16[kMost];
+  int head[kMost], tail[kMost];  // and up to three words before and behind them
   uint32_t word[kMost];
   int n = 0;
   long long total = 0;
   void add(void* p, int byte, size_t bytes) {
     if (bytes == 0) return;
-    at[n] = static_cast<uint4*>(p);
-    n16[n] = static_cast<long long>((bytes + 15) / 16);
+    const size_t words = bytes / 4;
+    const size_t before = std::min<size_t>((16 - (reinterpret_cast<uintptr_t>(p) & 15u)) % 16 / 4, words);
+    at[n] = reinterpret_cast<uint4*>(static_cast<uint32_t*>(p) + before);
+    n16[n] = static_cast<long long>((words - before) / 4);
+    head[n] = static_cast<int>(before);
+    tail[n] = static_cast<int>((words - before) % 4);
     word[n] = 0x01010101u * (static_cast<uint32_t>(byte) & 0xffu);
-    total += n16[n++];
+    total += n16[n++] + 1;
   }
 };
 __global__ void __launch_bounds__(256) clear_kernel(const __grid_constant__ Clear c) {
@@ -348,6 +354,11 @@ __global__ void __launch_bounds__(256) clear_kernel(const __grid_constant__ Clea
     const uint4 v = make_uint4(c.word[s], c.word[s], c.word[s], c.word[s]);
     uint4* __restrict__ dst = c.at[s];
     for (long long i = blockIdx.x * 256ll + threadIdx.x; i < c.n16[s]; i += stride) dst[i] = v;
+    if (blockIdx.x == 0 && threadIdx.x < 8) {
+      const int t = threadIdx.x & 3;
+      if (threadIdx.x < 4 && t < c.head[s]) (reinterpret_cast<uint32_t*>(dst) - c.head[s])[t] = v.x;
+      if (threadIdx.x >= 4 && t < c.tail[s]) reinterpret_cast<uint32_t*>(dst + c.n16[s])[t] = v.x;
+    }
   }
 }
 
@@ -1875,16 +1886,8 @@ int strided_impl(const Geo& g, const Layout& L, const int32_t* idx, int64_t n_in
   Clear c;
   c.add(fwd.rm, 0xFF, fwd.rm ? static_cast<size_t>(n_out) * kvp * 4 : 0);
   c.add(words, 0, words ? static_cast<size_t>(n_out) * L.mic * 4 : 0);
-  int rc = SPC_OK;
-  if (fwd.cm != nullptr) {
-    // (a table of the caller's: neither its start nor its size need be a multiple of 16 bytes)
-    const size_t bytes = static_cast<size_t>(g.kv) * n_out * 4;
-    if ((reinterpret_cast<uintptr_t>(fwd.cm) | bytes) & 15u)
-      SPC_CUDA_OK(cudaMemsetAsync(fwd.cm, 0xFF, bytes, st));
-    else
-      c.add(fwd.cm, 0xFF, bytes);
-  }
-  if (c.total != 0) rc = launch_clear(c, st);
+  c.add(fwd.cm, 0xFF, fwd.cm ? static_cast<size_t>(g.kv) * n_out * 4 : 0);
+  int rc = c.total != 0 ? launch_clear(c, st) : SPC_OK;
   if (rc != SPC_OK) return rc;
   FillOut out{};
   const bool together = bwd.wanted() && bwd.mask == nullptr;
@@ -1929,7 +1932,10 @@ int native_impl(const Geo& g, const Layout& L, const int32_t* idx, int64_t n_in,
   int* block_counts = reinterpret_cast<int*>(ws + L.off_native);
   const unsigned nb = static_cast<unsigned>(L.n_blocks_native);
   dim3 grid(nb, static_cast<unsigned>(g.kv));
-  SPC_CUDA_OK(cudaMemsetAsync(pair, 0xFF, static_cast<size_t>(2) * g.kv * n_in * sizeof(int32_t), st));
+  Clear c;
+  c.add(pair, 0xFF, static_cast<size_t>(2) * g.kv * n_in * sizeof(int32_t));
+  const int rc = launch_clear(c, st);
+  if (rc != SPC_OK) return rc;
   native_count_kernel<ND, K64><<<grid, kThreads, 0, st>>>(g, idx, n_in, n_out, lookup, block_counts);
   SPC_LAUNCH_OK();
   native_scan_kernel<<<g.kv, kThreads, 0, st>>>(block_counts, static_cast<int>(nb), npl, g.kv, g.subm);
@@ -2255,9 +2261,11 @@ extern "C" int spc_native_to_tables(const int32_t* pair, int kv, int64_t n_pair,
   if (!pair || !pair_fwd || kv <= 0 || n_pair < 0 || n_out < 0 || n_in < 0)
     return fail(SPC_ERR_INVALID_ARGUMENT, "native_to_tables: bad arguments");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (n_out > 0) SPC_CUDA_OK(cudaMemsetAsync(pair_fwd, 0xFF, static_cast<size_t>(kv) * n_out * 4, st));
-  if (pair_bwd && n_in > 0) SPC_CUDA_OK(cudaMemsetAsync(pair_bwd, 0xFF, static_cast<size_t>(kv) * n_in * 4, st));
-  if (n_pair == 0) return SPC_OK;
+  Clear c;
+  c.add(pair_fwd, 0xFF, static_cast<size_t>(kv) * n_out * 4);
+  if (pair_bwd) c.add(pair_bwd, 0xFF, static_cast<size_t>(kv) * n_in * 4);
+  const int rc = c.total != 0 ? launch_clear(c, st) : SPC_OK;
+  if (rc != SPC_OK || n_pair == 0) return rc;
   const int32_t* pair_in = pair + static_cast<int64_t>(inverse ? 1 : 0) * kv * n_pair;
   const int32_t* pair_out = pair + static_cast<int64_t>(inverse ? 0 : 1) * kv * n_pair;
   dim3 grid(blocks_for(n_pair), static_cast<unsigned>(kv));

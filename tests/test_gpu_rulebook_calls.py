@@ -46,3 +46,35 @@ def test_a_row_order_asked_for_again(n, subm):
             order = torch.full((n_in,), -1, dtype=torch.int32, device=DEV)
             tables(order_bwd=order)
             assert torch.equal(order.sort().values.cpu(), torch.arange(n_in, dtype=torch.int32))
+
+
+def _node_types(graph):
+    """The kinds of nodes of a captured graph."""
+    cuda, count = ctypes.CDLL("libcuda.so.1"), ctypes.c_size_t(0)
+    handle = ctypes.c_void_p(graph.raw_cuda_graph())
+    assert cuda.cuGraphGetNodes(handle, None, ctypes.byref(count)) == 0
+    nodes = (ctypes.c_void_p * count.value)()
+    assert cuda.cuGraphGetNodes(handle, nodes, ctypes.byref(count)) == 0
+    kinds, kind = set(), ctypes.c_int(0)
+    for node in nodes:
+        assert cuda.cuGraphNodeGetType(ctypes.c_void_p(node), ctypes.byref(kind)) == 0
+        kinds.add({0: "kernel", 1: "memcpy", 2: "memset"}.get(kind.value, kind.value))
+    return kinds
+
+
+@pytest.mark.parametrize("start", [0, 1, 2, 3])
+@pytest.mark.parametrize("n", [777, 778, 779, 780])
+def test_a_table_that_starts_and_ends_anywhere(n, start):
+    """The column-major table of a strided layer is a caller's: cleared to its last entry, and nothing beside it,
+    by a kernel (no driver memset, which may wait behind the application's transfers)."""
+    tables, _, n_out, exp = _prepared((20, 24, 22), n, 1, 2, False)
+    room = torch.full((27 * n_out + 8,), 7, dtype=torch.int32, device=DEV)
+    table = room[start:start + 27 * n_out]
+    out_indices = torch.empty((n_out, 4), dtype=torch.int32, device=DEV)
+    tables(pair_fwd=table, out_indices=out_indices)
+    np.testing.assert_array_equal(to_np(table).reshape(27, n_out), exp[2])
+    assert bool((room[:start] == 7).all()) and bool((room[start + 27 * n_out:] == 7).all())
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        tables(pair_fwd=table, out_indices=out_indices)
+    assert _node_types(graph) == {"kernel"}
