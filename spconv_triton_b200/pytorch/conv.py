@@ -355,6 +355,10 @@ class SparseConvolutionBase:
                 or not ops.unreplaced() or act_type.name not in ("None_", "ReLU", "Sigmoid", "LeakyReLU")
                 or weight.dtype not in _host.FLOATS):
             return None
+        if not training and self.algo == ConvAlgo.Native and (
+                add_input is not None or features.dtype != weight.dtype or torch.is_autocast_enabled()
+                or (torch.is_grad_enabled() and (features.requires_grad or weight.requires_grad))):
+            return None  # layers of pair lists are autograd functions in evaluation mode too
         datas = x.find_indice_pair(self.indice_key)
         entry_type = IndiceData if self.algo == ConvAlgo.Native else ImplicitGemmIndiceData
         if datas is None and self.inverse:

@@ -1,0 +1,52 @@
+"""What the layers take and refuse, on CUDA tensors, does not depend on which host path runs them."""
+
+import numpy as np
+import pytest
+import torch
+
+from gpu_util import DEV, rel_err, to_np, unique_coords
+
+pytestmark = pytest.mark.gpu
+
+SHAPE, N = [20, 20, 20], 1500
+
+
+def _input(channels, dtype=torch.float32, grad=False):
+    import spconv_triton_b200.pytorch as sp
+
+    torch.manual_seed(4)
+    idx = torch.from_numpy(unique_coords(3, N, 1, SHAPE)).to(DEV)
+    return sp.SparseConvTensor(torch.randn(N, channels, device=DEV).to(dtype).requires_grad_(grad), idx, SHAPE, 1)
+
+
+def _both_paths(monkeypatch, run):
+    """run() through the layers' native host side and through the operator functions."""
+    from spconv_triton_b200.pytorch._impl import host
+
+    first = run()
+    monkeypatch.setattr(host, "takes", lambda *a: False)
+    return first, run()
+
+
+@pytest.mark.parametrize("what", ["gradient", "autocast", "mixed", "residual"])
+def test_pair_list_layers_in_evaluation_mode(what, monkeypatch):
+    """Layers of more than 32 offsets are differentiable, follow autocast, keep the type of their features and add
+    `add_input` in evaluation mode too."""
+    import spconv_triton_b200.pytorch as sp
+
+    torch.manual_seed(5)
+    layer = sp.SubMConv3d(16, 16, 5, padding=2).to(DEV).eval()
+
+    def run():
+        x = _input(16, torch.float16 if what == "mixed" else torch.float32, grad=what == "gradient")
+        layer.zero_grad()
+        with torch.set_grad_enabled(what == "gradient"), torch.autocast("cuda", enabled=what == "autocast"):
+            y = layer(x, add_input=x) if what == "residual" else layer(x)
+        if what != "gradient":
+            return [y.features]
+        y.features.square().sum().backward()
+        return [y.features.detach(), x.features.grad, layer.weight.grad]
+
+    for a, b in zip(*_both_paths(monkeypatch, run)):
+        assert a.dtype == b.dtype
+        assert rel_err(to_np(a.double()), to_np(b.double())) <= (2e-3 if a.dtype == torch.float16 else 1e-5)
