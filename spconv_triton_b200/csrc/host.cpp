@@ -35,6 +35,12 @@ void check(int status) {
 }
 
 void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+// An operand as the kernels read it, in 16-byte words: contiguous (a view that starts elsewhere is copied; the
+// CUDA-core kernels that take such views read column-major tables, which are not made for the others).
+Tensor operand(const Tensor& t) {
+  const Tensor c = t.contiguous();
+  return (reinterpret_cast<uintptr_t>(c.const_data_ptr()) & 15u) != 0 ? c.clone() : c;
+}
 int32_t* ints(const Tensor& t) { return t.defined() ? t.data_ptr<int32_t>() : nullptr; }
 void* data(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 int code_of(at::ScalarType t) {
@@ -246,8 +252,7 @@ struct ConvOptions {
 Tensor conv_forward_raw(const Tensor& features, const Tensor& weight, const Tensor& bias, const Tensor& residual, const Book& rb,
                         const ConvOptions& o, at::ScalarType out_type, Tensor scale, Tensor shift, int act, double alpha) {
   c10::cuda::CUDAGuard guard(features.device());
-  Tensor x = features.contiguous(), w = weight.contiguous();
-  if (w.scalar_type() != x.scalar_type()) w = w.to(x.scalar_type());
+  Tensor x = operand(features), w = operand(weight.scalar_type() == x.scalar_type() ? weight : weight.to(x.scalar_type()));
   int64_t k_out = w.size(0), c_in = w.size(w.dim() - 1), kv = rb->geo->kv;
   const int64_t n_in = o.inverse ? rb->n_out : rb->n_in, n_out = o.inverse ? rb->n_in : rb->n_out;
   if (x.size(0) != n_in || x.size(1) != c_in || w.numel() != k_out * kv * c_in)
@@ -262,7 +267,7 @@ Tensor conv_forward_raw(const Tensor& features, const Tensor& weight, const Tens
     }
   }
   if (b.defined()) b = b.contiguous();
-  Tensor r = residual.defined() ? residual.contiguous() : residual;
+  Tensor r = residual.defined() ? operand(residual) : residual;
   Tensor out = at::empty({n_out, k_out}, x.options().dtype(out_type));
   const void *from = x.data_ptr(), *weights = w.data_ptr();
   Prepared copies;
@@ -290,7 +295,7 @@ Tensor conv_forward_raw(const Tensor& features, const Tensor& weight, const Tens
 Tensor conv_backward_input_raw(const Tensor& grad, const Tensor& weight, const Book& rb, const ConvOptions& o) {
   const int64_t k_out = weight.size(0), c_in = weight.size(weight.dim() - 1), kv = rb->geo->kv;
   const int64_t n_grad = o.inverse ? rb->n_in : rb->n_out, n_in = o.inverse ? rb->n_out : rb->n_in;
-  Tensor w = weight.scalar_type() == grad.scalar_type() ? weight : weight.to(grad.scalar_type());
+  Tensor w = operand(weight.scalar_type() == grad.scalar_type() ? weight : weight.to(grad.scalar_type()));
   Tensor din = at::empty({n_in, c_in}, grad.options());
   // a submanifold layer's input side is its output side with the offsets reversed
   const bool reversed = rb->subm(), input = !reversed && !o.inverse;
@@ -317,7 +322,7 @@ Tensor conv_backward_input_raw(const Tensor& grad, const Tensor& weight, const B
 Tensor conv_backward_weight_raw(const Tensor& features, const Tensor& grad, at::IntArrayRef sizes, const Book& rb, const ConvOptions& o) {
   const int64_t k_out = sizes[0], c_in = sizes[sizes.size() - 1], kv = rb->geo->kv;
   Tensor dw = at::empty(sizes, grad.options());
-  Tensor x = features.scalar_type() == grad.scalar_type() ? features : features.to(grad.scalar_type());
+  Tensor x = operand(features.scalar_type() == grad.scalar_type() ? features : features.to(grad.scalar_type()));
   const Rulebook::Side t = rb->side(o.inverse, true);
   const int64_t n_out = grad.size(0);
   const size_t bytes = spc_conv_backward_weight_workspace_bytes(n_out, c_in, k_out, kv);
@@ -382,7 +387,7 @@ struct ConvBackward : public torch::autograd::Node {
     const bool create_graph = at::GradMode::is_enabled();
     at::AutoGradMode no_grad(false);
     c10::cuda::CUDAGuard guard(grads[0].device());
-    Tensor grad = grads[0].contiguous();
+    Tensor grad = operand(grads[0]);
     if (bias && task_should_compute_output(2)) out[2] = column_sums(grad, bias_type);
     if (task_should_compute_output(0)) out[0] = conv_backward_input_raw(grad, weight, rb, options);
     if (task_should_compute_output(1)) out[1] = conv_backward_weight_raw(features, grad, weight.sizes(), rb, options);

@@ -50,3 +50,34 @@ def test_pair_list_layers_in_evaluation_mode(what, monkeypatch):
     for a, b in zip(*_both_paths(monkeypatch, run)):
         assert a.dtype == b.dtype
         assert rel_err(to_np(a.double()), to_np(b.double())) <= (2e-3 if a.dtype == torch.float16 else 1e-5)
+
+
+def _misaligned(t):
+    """The same values, contiguous, four bytes off a 16-byte boundary."""
+    off = 4 // t.element_size()
+    return torch.cat([t.new_zeros(off), t.detach().reshape(-1)])[off:].view(t.shape)
+
+
+@pytest.mark.parametrize("channels", [16, 64])
+@pytest.mark.parametrize("which", ["features", "weight", "gradient"])
+def test_operands_that_start_anywhere(channels, which):
+    """Views into a larger buffer (flat parameters, slices) need not start at a multiple of 16 bytes."""
+    import spconv_triton_b200.pytorch as sp
+
+    torch.manual_seed(6)
+    layer = sp.SubMConv3d(channels, channels, 3, padding=1).to(DEV)
+    x, g = _input(channels).features, torch.randn(N, channels, device=DEV)
+    results = []
+    for moved in (False, True):
+        if moved and which == "weight":
+            layer.weight.data = _misaligned(layer.weight.data)
+        feats = (_misaligned(x) if moved and which == "features" else x.clone()).requires_grad_()
+        layer.zero_grad()
+        y = layer(_input(channels).replace_feature(feats)).features
+        y.backward(_misaligned(g) if moved and which == "gradient" else g)
+        results.append([y.detach(), feats.grad, layer.weight.grad, layer.bias.grad])
+        with torch.no_grad():
+            results[-1].append(layer.eval()(_input(channels).replace_feature(feats.detach())).features)
+        layer.train()
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
