@@ -2071,7 +2071,8 @@ bool rulebook_adopts(const spc_geometry* sg, int64_t n_in, const RulebookProduce
   if (!make_geo(sg, &g)) return false;
   Layout L = make_layout(g, n_in);
   adopt_producer_bits(g, &L, producer);
-  return L.shared_bits != nullptr;
+  // (outputs that are not marked in a bitmap are enumerated from the coordinates)
+  return L.shared_bits != nullptr && (g.subm || (L.obits_words != 0 && g.axes_fit));
 }
 
 int rulebook_tables_chained(const spc_geometry* sg, const int32_t* indices, int64_t n_in, int64_t n_out,

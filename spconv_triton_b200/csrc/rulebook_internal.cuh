@@ -36,7 +36,7 @@ struct RulebookTables {
 int rulebook_prepare_chained(const spc_geometry* g, const int32_t* indices, int64_t n_in, void* workspace,
                              size_t workspace_bytes, int64_t* n_out_host, const RulebookProducer* producer,
                              cudaStream_t stream);
-// Whether rulebook_prepare_chained would take the rows from `producer`: it then reads nothing of `indices`.
+// Whether rulebook_prepare_chained would take all it needs from `producer`: it then reads nothing of `indices`.
 bool rulebook_adopts(const spc_geometry* g, int64_t n_in, const RulebookProducer* producer);
 int rulebook_tables_chained(const spc_geometry* g, const int32_t* indices, int64_t n_in, int64_t n_out, void* workspace,
                             size_t workspace_bytes, const RulebookTables& tables, const RulebookProducer* producer,

@@ -78,3 +78,28 @@ def test_a_table_that_starts_and_ends_anywhere(n, start):
     with torch.cuda.graph(graph):
         tables(pair_fwd=table, out_indices=out_indices)
     assert _node_types(graph) == {"kernel"}
+
+
+def test_outputs_numbered_by_hash_after_outputs_numbered_by_bitmap():
+    """In a pass of one call, the outputs of a transposed layer on a grid beyond the bitmap's limit are enumerated
+    from the coordinates that the strided layer before it writes, not before it has written them."""
+    import spconv_triton_b200.pytorch as sp
+    from spconv_triton_b200 import constants
+
+    shape, n, batch = [100, 1000, 1000], 20000, 3  # 37 M cells behind the first layer, 296 M behind the second
+    net = sp.SparseSequential(sp.SparseConv3d(16, 16, 3, stride=2, padding=1, bias=False),
+                              sp.SparseConvTranspose3d(16, 16, 3, stride=2, padding=1, bias=False)).to(DEV).half().eval()
+    idx = torch.from_numpy(unique_coords(5, n, batch, shape)).to(DEV)
+    x = torch.randn(n, 16, device=DEV).half()
+    outs = []
+    with torch.no_grad():
+        for native in (False, True, True, True):
+            old, constants.SPCONV_NATIVE_SEQUENCE = constants.SPCONV_NATIVE_SEQUENCE, native
+            try:
+                y = net(sp.SparseConvTensor(x, idx, shape, batch))
+            finally:
+                constants.SPCONV_NATIVE_SEQUENCE = old
+            outs.append((y.indices, y.features))
+    for indices, features in outs[1:]:
+        assert torch.equal(indices, outs[0][0])
+        assert torch.equal(features, outs[0][1])
