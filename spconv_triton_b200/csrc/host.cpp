@@ -364,6 +364,15 @@ bool wants_grad(std::initializer_list<const Tensor*> ts) {
   return false;
 }
 
+// These layers have no forward-mode derivative (nor had the autograd functions whose place their nodes take).
+void refuse_forward_mode(std::initializer_list<const Tensor*> ts) {
+  for (const Tensor* t : ts)
+    if (t->defined() && t->_fw_grad(0).defined()) {
+      PyErr_SetString(PyExc_NotImplementedError, "sparse convolution and pooling layers do not support forward mode AD");
+      throw pybind11::error_already_set();
+    }
+}
+
 // Inside autocast these layers compute in fp16 whatever its type, as the reference's functions do.
 Tensor cast_for_autocast(const Tensor& t) {
   if (!at::autocast::is_autocast_enabled(at::kCUDA) || !t.defined() || !t.is_floating_point() || t.scalar_type() == at::kDouble) return t;
@@ -406,8 +415,9 @@ struct ConvBackward : public torch::autograd::Node {
 // A convolution in training: out = gather-GEMM (+ bias) (+ residual), with its place in the autograd graph.
 Tensor conv_train(const Tensor& features, const Tensor& weight, const c10::optional<Tensor>& bias_opt, const c10::optional<Tensor>& residual_opt,
                   const Book& rb, bool inverse, bool tf32, int split_most) {
-  pybind11::gil_scoped_release release;
   const Tensor bias = bias_opt.value_or(Tensor()), residual = residual_opt.value_or(Tensor());
+  refuse_forward_mode({&features, &weight, &bias, &residual});
+  pybind11::gil_scoped_release release;
   const bool grad = wants_grad({&features, &weight, &bias, &residual});
   ConvOptions o{inverse, tf32, split_most};
   Tensor x, w, out;
@@ -509,6 +519,7 @@ struct PoolBackward : public torch::autograd::Node {
 };
 
 Tensor pool(const Tensor& features, const Book& rb, bool average) {
+  refuse_forward_mode({&features});
   pybind11::gil_scoped_release release;
   const bool grad = wants_grad({&features});
   Tensor x, out, count;

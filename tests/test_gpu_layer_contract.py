@@ -81,3 +81,33 @@ def test_operands_that_start_anywhere(channels, which):
         layer.train()
     for a, b in zip(*results):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("kind", ["subm", "down", "max", "avg"])
+def test_forward_mode_derivatives_are_refused(kind):
+    """... not dropped: the layers have no forward-mode derivative."""
+    import spconv_triton_b200.pytorch as sp
+
+    layer = {"subm": lambda: sp.SubMConv3d(16, 16, 3, padding=1), "down": lambda: sp.SparseConv3d(16, 16, 3, 2, 1),
+             "max": lambda: sp.SparseMaxPool3d(2, 2), "avg": lambda: sp.SparseAvgPool3d(2, 2)}[kind]().to(DEV).train()
+    x = _input(16)
+    with torch.autograd.forward_ad.dual_level():
+        dual = torch.autograd.forward_ad.make_dual(x.features, torch.ones_like(x.features))
+        with pytest.raises((NotImplementedError, RuntimeError), match="forward"):
+            layer(x.replace_feature(dual))
+
+
+@pytest.mark.parametrize("kind", ["subm", "max"])
+@pytest.mark.parametrize("transform", ["grad", "vmap"])
+def test_function_transforms_are_refused(kind, transform):
+    import spconv_triton_b200.pytorch as sp
+
+    layer = (sp.SubMConv3d(16, 16, 3, padding=1) if kind == "subm" else sp.SparseMaxPool3d(2, 2)).to(DEV).train()
+    x = _input(16)
+
+    def run(feats):
+        y = layer(x.replace_feature(feats)).features
+        return y.sum() if transform == "grad" else y
+
+    with pytest.raises(RuntimeError):
+        torch.func.grad(run)(x.features) if transform == "grad" else torch.func.vmap(run)(x.features[None])
