@@ -38,12 +38,14 @@ __device__ __forceinline__ void round_rows(const float4* __restrict__ src, float
   }
 }
 
-// one thread per source element
+// one thread per source element; Index: 32 bits where they hold the element count (four 64-bit divisions in a row
+// are as long as the rest of the kernel on few elements)
+template <typename Index>
 __device__ __forceinline__ void prepare_rows(const float* __restrict__ src, float* __restrict__ dst, long long rows, int cols, int mode,
                                              unsigned block) {
-  const long long i = block * 256ll + threadIdx.x;
-  if (i >= rows * cols) return;
-  const long long r = i / cols;
+  const Index i = static_cast<Index>(block) * 256 + threadIdx.x;
+  if (i >= static_cast<Index>(rows * cols)) return;
+  const Index r = i / static_cast<Index>(cols);
   const int c = static_cast<int>(i - r * cols);
   const float x = src[i];
   const float hi = rna_tf32(x);
@@ -52,7 +54,7 @@ __device__ __forceinline__ void prepare_rows(const float* __restrict__ src, floa
     return;
   }
   const float lo = rna_tf32(x - hi);
-  float* row = dst + r * 3 * cols;
+  float* row = dst + static_cast<long long>(r) * 3 * cols;
   row[c] = hi;
   row[cols + c] = mode == SPC_TF32_SPLIT_A ? lo : hi;
   row[2 * cols + c] = mode == SPC_TF32_SPLIT_A ? hi : lo;
@@ -60,15 +62,16 @@ __device__ __forceinline__ void prepare_rows(const float* __restrict__ src, floa
 
 // weight [c_out, kv, c_in] -> dst [c_out, kv, m * c_in], or with `transpose` [c_in, kv, m * c_out]
 // (dst[c][k][n] = w[n][k][c]; 2: dst[c][kv - 1 - k][n]): the reduction index innermost, as the forward-form kernel reads it.
+template <typename Index>
 __device__ __forceinline__ void prepare_weight(const float* __restrict__ w, float* __restrict__ dst, int c_out, int kv, int c_in,
                                                int transpose, int mode, unsigned block) {
-  const long long i = block * 256ll + threadIdx.x;
-  const long long total = static_cast<long long>(c_out) * kv * c_in;
-  if (i >= total) return;
-  const int c = static_cast<int>(i % c_in);
-  const int k = static_cast<int>((i / c_in) % kv);
+  const Index i = static_cast<Index>(block) * 256 + threadIdx.x;
+  if (i >= static_cast<Index>(c_out) * kv * c_in) return;
+  const Index row_of = i / static_cast<Index>(c_in);  // (output channel, offset)
+  const int c = static_cast<int>(i - row_of * c_in);
+  const int n = static_cast<int>(row_of / static_cast<Index>(kv));
+  const int k = static_cast<int>(row_of - static_cast<Index>(n) * kv);
   const int ko = transpose == 2 ? kv - 1 - k : k;
-  const int n = static_cast<int>(i / (static_cast<long long>(c_in) * kv));
   const float x = w[i];
   const float hi = rna_tf32(x);
   const int m = mode == SPC_TF32_ROUND ? 1 : 3;
@@ -99,13 +102,14 @@ struct Weight {
   unsigned blocks;
 };
 // The first CTAs take the rows, the others the weight.
+template <typename Index>
 __global__ void __launch_bounds__(256) tf32_prepare_kernel(const __grid_constant__ Rows x, const __grid_constant__ Weight w) {
   if (blockIdx.x >= x.blocks)
-    prepare_weight(w.src, w.dst, w.c_out, w.kv, w.c_in, w.transpose, w.mode, blockIdx.x - x.blocks);
+    prepare_weight<Index>(w.src, w.dst, w.c_out, w.kv, w.c_in, w.transpose, w.mode, blockIdx.x - x.blocks);
   else if (x.wide)
     round_rows(reinterpret_cast<const float4*>(x.src), reinterpret_cast<float4*>(x.dst), x.rows * x.cols / 4, blockIdx.x, x.blocks);
   else
-    prepare_rows(x.src, x.dst, x.rows, x.cols, x.mode, blockIdx.x);
+    prepare_rows<Index>(x.src, x.dst, x.rows, x.cols, x.mode, blockIdx.x);
 }
 
 int rows_of(const float* src, float* dst, int64_t rows, int cols, int mode, Rows* x) {
@@ -127,7 +131,10 @@ int weight_of(const float* weight, float* dst, int c_out, int kv, int c_in, int 
 }
 int launch(const Rows& x, const Weight& w, void* stream) {
   if (x.blocks + w.blocks == 0) return SPC_OK;
-  tf32_prepare_kernel<<<x.blocks + w.blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(x, w);
+  const long long most = std::max<long long>(x.rows * x.cols, static_cast<long long>(w.c_out) * w.kv * w.c_in) + 256;
+  const unsigned blocks = x.blocks + w.blocks;
+  if (most <= 0xffffffffll) tf32_prepare_kernel<uint32_t><<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(x, w);
+  else tf32_prepare_kernel<unsigned long long><<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(x, w);
   SPC_LAUNCH_OK();
   return SPC_OK;
 }
