@@ -26,6 +26,13 @@ def check_device_status(device=None):
         _lib.check(_lib.load().spc_check_device_status(_lib.current_stream(dev)))
 
 
+def on_one_device(first, *others):
+    """Raises where a kernel would be handed an address of another device (or of the host)."""
+    for t in others:
+        if t is not None and t.device != first.device:
+            raise ValueError(f"expected all tensors on {first.device}, found one on {t.device}")
+
+
 def _precision(t: torch.Tensor) -> int:
     # TF32 only for fp32 inputs and only while the live flag is set (gemm.py:460-463)
     if t.dtype == torch.float32 and bool(constants.SPCONV_ALLOW_TF32):
@@ -115,6 +122,9 @@ def conv_forward(features, filters_krsc, pair_fwd, n_out, bias=None, out_dtype=N
     k_out, kv, c_in = filters_krsc.shape
     if out_dtype is None:
         out_dtype = features.dtype
+    on_one_device(features, filters_krsc, pair_fwd, bias, mask_argsort)
+    if bias is not None and bias.numel() != k_out:
+        raise ValueError(f"a bias of {bias.numel()} values for {k_out} channels")
     dev = features.device
     with torch.cuda.device(dev):
         out = torch.empty((n_out, k_out), dtype=out_dtype, device=dev)
@@ -158,6 +168,7 @@ def conv_backward_input(grad_out, filters_krsc, pair_bwd, n_in, pair_mask=None, 
                         fp32_accum=None):
     """din [n_in, C] = sum_k grad_out[pair_bwd[k, :]] @ W[k]."""
     k_out, kv, c_in = filters_krsc.shape
+    on_one_device(grad_out, filters_krsc, pair_bwd, mask_argsort)
     dev = grad_out.device
     with torch.cuda.device(dev):
         din = torch.empty((n_in, c_in), dtype=grad_out.dtype, device=dev)
@@ -189,6 +200,7 @@ def conv_backward_weight(features, grad_out, pair_fwd, weight_shape_krsc, fp32_a
     """dW [K, kv, C] (contiguous, grad_out.dtype)."""
     k_out, kv, c_in = (int(v) for v in weight_shape_krsc)
     n_out = int(grad_out.shape[0])
+    on_one_device(grad_out, features, pair_fwd)
     dev = grad_out.device
     with torch.cuda.device(dev):
         dw = torch.empty((k_out, kv, c_in), dtype=grad_out.dtype, device=dev)

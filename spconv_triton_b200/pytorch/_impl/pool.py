@@ -10,9 +10,12 @@ import torch
 
 from spconv_triton_b200 import _lib
 
+from .gemm import on_one_device
+
 
 def maxpool_forward(features, pair_fwd, n_out):
     kv = int(pair_fwd.shape[0])
+    on_one_device(features, pair_fwd)
     feats = features.contiguous()
     c = int(feats.shape[1])
     dev = feats.device
@@ -28,6 +31,7 @@ def maxpool_forward(features, pair_fwd, n_out):
 
 def maxpool_backward(features, out_features, grad_out, pair_bwd):
     kv = int(pair_bwd.shape[0])
+    on_one_device(features, out_features, grad_out, pair_bwd)
     feats = features.contiguous()
     out = out_features.contiguous()
     g = grad_out.contiguous()
@@ -48,6 +52,7 @@ def maxpool_backward(features, out_features, grad_out, pair_bwd):
 
 def avgpool_forward(features, pair_fwd, n_out, calc_count=True):
     kv = int(pair_fwd.shape[0])
+    on_one_device(features, pair_fwd)
     feats = features.contiguous()
     c = int(feats.shape[1])
     dev = feats.device
@@ -65,6 +70,7 @@ def avgpool_forward(features, pair_fwd, n_out, calc_count=True):
 
 def avgpool_backward(grad_out, pair_bwd, count):
     kv = int(pair_bwd.shape[0])
+    on_one_device(grad_out, pair_bwd, count)
     g = grad_out.contiguous()
     n_in = int(pair_bwd.shape[1])
     c = int(g.shape[1])

@@ -228,7 +228,6 @@ class SparseConvolutionBase:
         bias_after = bias if training else None
         bias_fused = None if training else bias
         out_spatial_shape = self._output_spatial_shape(x.spatial_shape)
-        out_tensor = x.shadow_copy()
         if x.benchmark:
             self._open_benchmark_record(x, name)
 
@@ -237,7 +236,7 @@ class SparseConvolutionBase:
             feats = torch.mm(x.features, weight.view(self.in_channels, self.out_channels))
             if bias is not None:
                 feats += bias
-            out_tensor = out_tensor.replace_feature(feats)
+            out_tensor = x.replace_feature(feats)
             out_tensor.spatial_shape = out_spatial_shape
             return out_tensor
 
@@ -246,6 +245,7 @@ class SparseConvolutionBase:
             if out is not None:
                 return out
 
+        out_tensor = x.shadow_copy()
         indice_dict = x.indice_dict.copy()
         features = x.features.contiguous()
         if self.indice_key is not None:
@@ -351,10 +351,13 @@ class SparseConvolutionBase:
         """The forward pass through the host extension; None where a setting or a cached rulebook needs the
         operator functions."""
         features = x.features
-        if (x.benchmark or not self.host_plannable() or not _host.takes(features, x.indices) or not weight.is_cuda
-                or not ops.unreplaced() or act_type.name not in ("None_", "ReLU", "Sigmoid", "LeakyReLU")
+        dev = features.device
+        if (x.benchmark or not self.host_plannable() or not _host.takes(features, x.indices) or weight.device != dev
+                or x.indices.device != dev or not ops.unreplaced() or act_type.name not in ("None_", "ReLU", "Sigmoid", "LeakyReLU")
                 or weight.dtype not in _host.FLOATS):
             return None
+        if bias is not None and (bias.device != dev or bias.shape != (self.out_channels,) or bias.dtype not in _host.FLOATS):
+            return None  # broadcast or refused by the general path
         if not training and self.algo == ConvAlgo.Native and (
                 add_input is not None or features.dtype != weight.dtype or torch.is_autocast_enabled()
                 or (torch.is_grad_enabled() and (features.requires_grad or weight.requires_grad))):
@@ -387,7 +390,7 @@ class SparseConvolutionBase:
             residual = None
             if add_input is not None and add_input.features.shape == (out_indices.shape[0], self.out_channels):
                 out_type = torch.float16 if torch.is_autocast_enabled() else features.dtype
-                if add_input.features.dtype == out_type and add_input.features.device == features.device:
+                if add_input.features.dtype == out_type and add_input.features.device == dev:
                     residual, add_input = add_input.features, None
             out_features = _host.ext().conv_train(features, weight, bias, residual, rb, self.inverse, tf32, split_most)
         else:

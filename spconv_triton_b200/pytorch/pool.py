@@ -72,7 +72,7 @@ class _SparsePoolBase(SparseModule):
         """The pass through the host extension (rulebook and pooling, one native call each); None where the
         operator functions are needed."""
         features = x.features
-        if (self.algo != ConvAlgo.MaskImplicitGemm or x.benchmark or not features.is_cuda or not x.indices.is_cuda
+        if (self.algo != ConvAlgo.MaskImplicitGemm or x.benchmark or not features.is_cuda or x.indices.device != features.device
                 or features.dtype not in _host.POOL_FLOATS or x.indices.dtype != torch.int32 or x.indices.shape[0] == 0
                 or not constants.SPCONV_DO_SORT or not ops.unreplaced()):
             return None

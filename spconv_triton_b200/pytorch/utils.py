@@ -55,7 +55,7 @@ class PointToVoxel:
     def generate_voxel_with_id(self, pc: torch.Tensor, clear_voxels: bool = True, empty_mean: bool = False):
         """``(voxels [M, P, F], indices [M, ndim] zyx, num_per_voxel [M], pc_voxel_id [N])``
         (reference: utils.py:72-163)."""
-        if pc.device.type != self.device.type:
+        if pc.device != self.voxels.device:
             raise AssertionError("your pc device is wrong")
         if pc.dtype != torch.float32:
             raise NotImplementedError("points must be float32 (voxel boundaries are computed in the points' dtype)")

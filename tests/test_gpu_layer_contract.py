@@ -111,3 +111,34 @@ def test_function_transforms_are_refused(kind, transform):
 
     with pytest.raises(RuntimeError):
         torch.func.grad(run)(x.features) if transform == "grad" else torch.func.vmap(run)(x.features[None])
+
+
+@pytest.mark.parametrize("train", [False, True])
+def test_a_bias_that_does_not_fit_is_no_operand_of_a_kernel(train):
+    """A bias of one value is broadcast in training; other shapes, and a bias elsewhere, are errors."""
+    import spconv_triton_b200.pytorch as sp
+
+    layer, x = sp.SubMConv3d(16, 16, 3, padding=1, bias=True).to(DEV).train(train), _input(16)
+    with torch.set_grad_enabled(train):
+        layer.bias = torch.nn.Parameter(torch.zeros(16, device=DEV))
+        plain = layer(x).features
+        layer.bias = torch.nn.Parameter(torch.full((1,), 0.5, device=DEV))
+        if train:
+            y = layer(x).features
+            assert torch.equal(y, plain + 0.5)
+            y.sum().backward()
+            assert layer.bias.grad.shape == (1,) and float(layer.bias.grad) == 16 * N
+        else:
+            with pytest.raises(ValueError):
+                layer(x)
+        for bias in (torch.zeros(15, device=DEV), torch.zeros(16)):
+            layer.bias = torch.nn.Parameter(bias)
+            with pytest.raises((ValueError, RuntimeError)):
+                layer(x)
+
+
+def test_weights_on_another_device_are_refused():
+    import spconv_triton_b200.pytorch as sp
+
+    with pytest.raises((ValueError, RuntimeError, AssertionError)):
+        sp.SubMConv3d(16, 16, 3, padding=1)(_input(16))
