@@ -52,6 +52,10 @@ class SparseSequential(SparseModule):
                 raise ValueError("name exists.")
             self.add_module(name, module)
 
+    # What the native pass keeps on a container (plans of this process's threads, arena size) is not part of a copy.
+    def __getstate__(self):
+        return {k: v for k, v in self.__dict__.items() if k not in ("_spc_plans", "_spc_arena_floor")}
+
     def __len__(self):
         return len(self._modules)
 

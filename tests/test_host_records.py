@@ -81,3 +81,23 @@ def test_copies_of_an_entry_hold_its_tables():
         assert got.pair_fwd.numel() == 5 and got.pair_bwd.numel() == 2 and got.__dict__.get("_rb") is None
         assert got.ksize == [3] * 3 and got.algo == ConvAlgo.MaskImplicitGemm
     assert entry._rb is not None
+
+
+def _net():
+    return sp.SparseSequential(sp.SubMConv3d(16, 16, 3, padding=1, bias=False, indice_key="s"), torch.nn.BatchNorm1d(16),
+                               torch.nn.ReLU()).eval()
+
+
+def test_a_container_that_has_run_can_be_copied():
+    """Plans of the native pass belong to the object that made them, not to its copies."""
+    from spconv_triton_b200.pytorch import sequence
+
+    net = _net()
+    x = sp.SparseConvTensor(torch.zeros(3, 16), torch.zeros(3, 4, dtype=torch.int32), [4] * 3, 1)
+    net.__dict__["_spc_plans"] = {threading.get_ident(): sequence._compile(net, x)}
+    net.__dict__["_spc_arena_floor"] = [1 << 30, 6144.0]
+    for clone in (copy.deepcopy, lambda n: pickle.loads(pickle.dumps(n))):
+        got = clone(net)
+        assert "_spc_plans" not in got.__dict__ and "_spc_arena_floor" not in got.__dict__
+        assert torch.equal(got[0].weight, net[0].weight)
+    assert net.__dict__["_spc_plans"]
