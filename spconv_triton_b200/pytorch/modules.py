@@ -129,11 +129,12 @@ class SparseSequential(SparseModule):
 
 def _folded_bn(bn: nn.BatchNorm1d):
     """fp32 (scale, shift) with bn(x) == x * scale + shift in evaluation mode;
-    memoised on the module until one of its tensors changes."""
-    tensors = (bn.weight, bn.bias, bn.running_mean, bn.running_var)
+    memoised on the module until one of its tensors changes.  (The counter of batches among them: a forward
+    pass in training mode writes the running statistics past their version counters.)"""
+    tensors = (bn.weight, bn.bias, bn.running_mean, bn.running_var, bn.num_batches_tracked)
     key = tuple((t._version, t.data_ptr()) if t is not None else None for t in tensors) + (bn.eps,)
     cached = getattr(bn, "_spc_folded", None)
-    if cached is not None and cached[0] == key:
+    if cached is not None and cached[0] == key and all(a is b for a, b in zip(cached[3], tensors, strict=True)):
         return cached[1], cached[2]
     with torch.no_grad():
         scale = torch.rsqrt(bn.running_var.float() + bn.eps)
@@ -143,7 +144,7 @@ def _folded_bn(bn: nn.BatchNorm1d):
         if bn.bias is not None:
             shift = shift + bn.bias.float()
         scale, shift = scale.contiguous(), shift.contiguous()
-    bn._spc_folded = (key, scale, shift)
+    bn._spc_folded = (key, scale, shift, tensors)
     return scale, shift
 
 

@@ -101,3 +101,30 @@ def test_a_container_that_has_run_can_be_copied():
         assert "_spc_plans" not in got.__dict__ and "_spc_arena_floor" not in got.__dict__
         assert torch.equal(got[0].weight, net[0].weight)
     assert net.__dict__["_spc_plans"]
+
+
+def test_folded_statistics_follow_a_forward_in_training_mode():
+    """Training moves the running statistics without telling their version counters."""
+    from spconv_triton_b200.pytorch.modules import _folded_bn
+
+    bn = torch.nn.BatchNorm1d(4)
+    bn.eval()
+    before = [t.clone() for t in _folded_bn(bn)]
+    bn.train()(torch.randn(64, 4) * 3 + 1)
+    bn.eval()
+    x = torch.randn(8, 4)
+    scale, shift = _folded_bn(bn)
+    assert not torch.equal(shift, before[1])
+    torch.testing.assert_close(x * scale + shift, bn(x))
+
+
+def test_folded_statistics_follow_other_tensors_at_the_same_address():
+    from spconv_triton_b200.pytorch.modules import _folded_bn
+
+    bn, store = torch.nn.BatchNorm1d(4).eval(), torch.zeros(4)
+    for value in (0.0, 1.0):
+        store.fill_(value)
+        bn.running_mean = store.data  # (a new tensor on the same memory, its version counter at its start)
+        scale, shift = _folded_bn(bn)
+        x = torch.randn(8, 4)
+        torch.testing.assert_close(x * scale + shift, bn(x))
