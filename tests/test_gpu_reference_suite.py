@@ -5,7 +5,8 @@ environment variable ``SPCONV_TEST_IMPL`` (its ``tests/helpers.py:24-47``);
 ``spconv_triton_b200`` exposes every module that loader imports.  The test
 files are taken from a checkout of the reference: ``$SPCONV_REFERENCE_ROOT`` or
 the git-ignored copy ``baseline/_ref/reference`` made by
-``baseline/install_reference.py``; without either the tests are skipped.
+``baseline/install_reference.py``; without either the tests are skipped.  ``SPCONV_REFERENCE_SUITE_LOG`` names a
+file to which one line of counts per test file is added.
 
 Files whose golden vectors are listed in the reference's
 ``.MISSING_LARGE_BLOBS`` (not part of the checkout) cannot be collected and
@@ -69,8 +70,8 @@ def test_reference_file(name, tmp_path):
     res = subprocess.run(cmd, cwd=str(ref), env=env, capture_output=True, text=True, timeout=1500)
     tail = "\n".join((res.stdout + "\n" + res.stderr).splitlines()[-40:])
     summary = re.findall(r"(\d+) (passed|failed|error|errors|skipped|deselected)", res.stdout)
-    out_dir = ROOT / "gpurun_out"
-    if out_dir.is_dir():
-        with open(out_dir / "reference_suite.txt", "a") as f:
+    log = os.environ.get("SPCONV_REFERENCE_SUITE_LOG")
+    if log:
+        with open(log, "a") as f:
             f.write(f"{name}: rc={res.returncode} " + " ".join(f"{n} {k}" for n, k in summary) + "\n")
     assert res.returncode == 0, f"{name} against spconv_triton_b200:\n{tail}"
