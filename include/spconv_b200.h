@@ -53,12 +53,12 @@ typedef enum { SPC_PREC_IEEE = 0, SPC_PREC_TF32 = 1 } spc_precision;
 /* Operand preparations for fp32 layers on the tensor cores (spc_tf32_prepare). */
 typedef enum { SPC_TF32_ROUND = 0, SPC_TF32_SPLIT_A = 1, SPC_TF32_SPLIT_B = 2 } spc_tf32_mode;
 
-/* Which implementation a GEMM entry point may use.  AUTO picks a tcgen05
- * kernel whenever the shape allows it (gathered rows copied with cp.async;
- * weight slabs loaded by tiled TMA when the channel widths fit a swizzle span,
- * by cp.async otherwise) and the CUDA-core kernel for the rest.  SIMT forces the CUDA-core kernels; TCGEN05 demands a
- * tensor-core kernel (SPC_ERR_UNSUPPORTED if the shape does not fit);
- * TCGEN05_CPASYNC behaves like AUTO but never uses the TMA-fed kernel. */
+/* Which implementation a GEMM entry point may use.  AUTO picks the tcgen05
+ * kernel whenever the shape allows it (gathered rows copied with cp.async,
+ * weight slabs loaded by tiled TMA) and a CUDA-core kernel for the rest.  SIMT
+ * forces the CUDA-core kernels; TCGEN05 demands the tensor-core kernel
+ * (SPC_ERR_UNSUPPORTED if the shape does not fit).  TCGEN05_CPASYNC named a second
+ * tensor-core kernel, for widths that the first did not take, and is AUTO now. */
 typedef enum {
   SPC_GEMM_AUTO = 0,
   SPC_GEMM_SIMT = 1,

@@ -1,5 +1,5 @@
 // C-ABI entry points of the implicit gather-GEMM and the choice between the
-// tcgen05 kernels and the CUDA-core kernels.
+// tcgen05 kernel and the CUDA-core kernels.
 #include <algorithm>
 
 #include "common.cuh"
@@ -9,12 +9,15 @@ using namespace spc;
 
 namespace {
 
-// The tensor-core kernels take 16-bit inputs always and fp32 inputs only when
+// (the code of a kernel that is gone)
+int known_path(int path) { return path == SPC_GEMM_TCGEN05_CPASYNC ? SPC_GEMM_AUTO : path; }
+
+// The tensor-core kernel takes 16-bit inputs always and fp32 inputs only when
 // the caller allows TF32; IEEE fp32 stays on the CUDA cores.
 bool want_tc(int path, int n_dim, int r_dim, int kv, int dtype, int out_dtype, int precision, bool transposed,
              int* status) {
   *status = SPC_OK;
-  const bool ok = gather_gemm_tc_supported(n_dim, r_dim, kv, dtype, out_dtype, precision, transposed);
+  const bool ok = gather_gemm_tma_supported(n_dim, r_dim, kv, dtype, out_dtype, precision, transposed);
   if (path == SPC_GEMM_SIMT) return false;
   if (path == SPC_GEMM_TCGEN05) {
     if (!ok) *status = fail(SPC_ERR_UNSUPPORTED, "tcgen05 path does not take this shape/dtype "
@@ -33,12 +36,9 @@ bool f32_aligned(const void* a, const void* b, const void* c) {
 
 extern "C" int spc_conv_forward_needs_colmajor(int c_in, int c_out, int kv, int dtype, int out_dtype, int precision,
                                                int path) {
-  const bool tma = path != SPC_GEMM_SIMT && path != SPC_GEMM_TCGEN05_CPASYNC &&
-                   gather_gemm_tc_supported(c_out, c_in, kv, dtype, out_dtype, precision, false) &&
-                   gather_gemm_tma_supported(c_out, c_in, kv, dtype, out_dtype, precision, false);
-  if (tma) return 0;
-  const bool tc = path != SPC_GEMM_SIMT && gather_gemm_tc_supported(c_out, c_in, kv, dtype, out_dtype, precision, false);
-  return path == SPC_GEMM_AUTO && !tc && gather_gemm_f32_supported(c_out, c_in, dtype, out_dtype) ? 0 : 1;
+  path = known_path(path);
+  if (path != SPC_GEMM_SIMT && gather_gemm_tma_supported(c_out, c_in, kv, dtype, out_dtype, precision, false)) return 0;
+  return path == SPC_GEMM_AUTO && gather_gemm_f32_supported(c_out, c_in, dtype, out_dtype) ? 0 : 1;
 }
 
 extern "C" int spc_conv_forward(const void* features, const void* weight, const void* bias,
@@ -58,6 +58,7 @@ extern "C" int spc_conv_forward_residual(const void* features, const void* weigh
                                          int c_in, int c_out, int kv, int dtype, int out_dtype, int precision,
                                          int path, const float* out_scale, const float* out_shift, int act,
                                          float act_alpha, const void* residual, void* stream) {
+  path = known_path(path);
   if (!features || !weight || !out || n_in < 0 || n_out < 0 || c_in <= 0 || c_out <= 0 || kv <= 0)
     return fail(SPC_ERR_INVALID_ARGUMENT, "conv_forward: bad arguments");
   if (!pair_fwd && (!pair_fwd_rowmajor ||
@@ -74,12 +75,8 @@ extern "C" int spc_conv_forward_residual(const void* features, const void* weigh
     return fail(SPC_ERR_INVALID_ARGUMENT, "conv_forward: the residual must be 16-byte aligned");
   int status;
   if (want_tc(path, c_out, c_in, kv, dtype, out_dtype, precision, false, &status)) {
-    if (path != SPC_GEMM_TCGEN05_CPASYNC &&
-        gather_gemm_tma_supported(c_out, c_in, kv, dtype, out_dtype, precision, false))
-      return gather_gemm_tma(features, weight, epi, pair_fwd, pair_fwd_rowmajor, mask_argsort, out, n_in, n_out, c_out, c_in, kv,
-                             /*transposed_weight=*/false, /*reversed=*/false, dtype, out_dtype, precision, st);
-    return gather_gemm_tc(features, weight, epi, pair_fwd, mask_argsort, out, n_out, c_out, c_in, kv,
-                          /*transposed_weight=*/false, /*reversed=*/false, dtype, out_dtype, precision, st);
+    return gather_gemm_tma(features, weight, epi, pair_fwd, pair_fwd_rowmajor, mask_argsort, out, n_in, n_out, c_out, c_in, kv,
+                           /*transposed_weight=*/false, /*reversed=*/false, dtype, out_dtype, precision, st);
   }
   if (status != SPC_OK) return status;
   if (path == SPC_GEMM_AUTO && gather_gemm_f32_supported(c_out, c_in, dtype, out_dtype) && f32_aligned(features, weight, out))
@@ -102,18 +99,16 @@ extern "C" int spc_conv_backward_input(const void* grad_out, const void* weight,
 }
 
 extern "C" int spc_conv_backward_input_needs_colmajor(int c_in, int c_out, int kv, int dtype, int precision, int path) {
-  const bool tma = path != SPC_GEMM_SIMT && path != SPC_GEMM_TCGEN05_CPASYNC &&
-                   gather_gemm_tc_supported(c_in, c_out, kv, dtype, dtype, precision, true) &&
-                   gather_gemm_tma_supported(c_in, c_out, kv, dtype, dtype, precision, true);
-  if (tma) return 0;
-  const bool tc = path != SPC_GEMM_SIMT && gather_gemm_tc_supported(c_in, c_out, kv, dtype, dtype, precision, true);
-  return path == SPC_GEMM_AUTO && !tc && gather_gemm_f32_supported(c_in, c_out, dtype, dtype) ? 0 : 1;
+  path = known_path(path);
+  if (path != SPC_GEMM_SIMT && gather_gemm_tma_supported(c_in, c_out, kv, dtype, dtype, precision, true)) return 0;
+  return path == SPC_GEMM_AUTO && gather_gemm_f32_supported(c_in, c_out, dtype, dtype) ? 0 : 1;
 }
 
 extern "C" int spc_conv_backward_input_tables(const void* grad_out, const void* weight, const int32_t* pair_bwd,
                                               const int32_t* pair_bwd_rowmajor, const int32_t* mask_argsort, void* din,
                                               int64_t n_in, int64_t n_out, int c_in, int c_out, int kv, int reversed, int dtype,
                                               int precision, int path, void* stream) {
+  path = known_path(path);
   if (!grad_out || !weight || !din || n_in < 0 || n_out < 0 || c_in <= 0 || c_out <= 0 || kv <= 0)
     return fail(SPC_ERR_INVALID_ARGUMENT, "conv_backward_input: bad arguments");
   if (!pair_bwd && (!pair_bwd_rowmajor || spc_conv_backward_input_needs_colmajor(c_in, c_out, kv, dtype, precision, path)))
@@ -122,11 +117,8 @@ extern "C" int spc_conv_backward_input_tables(const void* grad_out, const void* 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int status;
   if (want_tc(path, c_in, c_out, kv, dtype, dtype, precision, true, &status)) {
-    if (path != SPC_GEMM_TCGEN05_CPASYNC && gather_gemm_tma_supported(c_in, c_out, kv, dtype, dtype, precision, true))
-      return gather_gemm_tma(grad_out, weight, Epilogue{}, pair_bwd, pair_bwd_rowmajor, mask_argsort, din, n_out, n_in, c_in, c_out, kv,
-                             /*transposed_weight=*/true, reversed != 0, dtype, dtype, precision, st);
-    return gather_gemm_tc(grad_out, weight, Epilogue{}, pair_bwd, mask_argsort, din, n_in, c_in, c_out, kv,
-                          /*transposed_weight=*/true, reversed != 0, dtype, dtype, precision, st);
+    return gather_gemm_tma(grad_out, weight, Epilogue{}, pair_bwd, pair_bwd_rowmajor, mask_argsort, din, n_out, n_in, c_in, c_out, kv,
+                           /*transposed_weight=*/true, reversed != 0, dtype, dtype, precision, st);
   }
   if (status != SPC_OK) return status;
   if (path == SPC_GEMM_AUTO && gather_gemm_f32_supported(c_in, c_out, dtype, dtype) && f32_aligned(grad_out, weight, din))
@@ -153,6 +145,7 @@ extern "C" int spc_conv_backward_weight(const void* features, const void* grad_o
                                         int path, void* stream) {
   (void)n_in;
   (void)precision;
+  path = known_path(path);
   if (!features || !grad_out || !pair_fwd || !dweight || n_out < 0 || c_in <= 0 || c_out <= 0 || kv <= 0)
     return fail(SPC_ERR_INVALID_ARGUMENT, "conv_backward_weight: bad arguments");
   cudaStream_t st = static_cast<cudaStream_t>(stream);

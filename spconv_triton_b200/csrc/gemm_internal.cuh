@@ -37,14 +37,6 @@ WgradSplit wgrad_f32_split(int64_t n_out, int c_in, int c_out, int kv);
 int wgrad_f32(const void* feats, const void* gout, const int32_t* pair_fwd, float* partial, int64_t n_out, int c_in, int c_out, int kv,
               const WgradSplit& split, cudaStream_t st);
 
-// tcgen05 kernels (gemm_tc.cu).  `transposed_weight` selects the input-gradient
-// view of the KRSC weight; `reversed`: offset k of the table meets weight kv - 1 - k.  Return SPC_ERR_UNSUPPORTED for shapes they do not take.
-bool gather_gemm_tc_supported(int n_dim, int r_dim, int kv, int dtype, int out_dtype, int precision,
-                              bool transposed_weight);
-int gather_gemm_tc(const void* src, const void* w, const Epilogue& epi, const int32_t* pairs,
-                   const int32_t* order, void* out, long long m_rows, int n_dim, int r_dim, int kv,
-                   bool transposed_weight, bool reversed, int dtype, int out_dtype, int precision, cudaStream_t st);
-
 // dw[e] = sum over splits of partial[s, e], added in split order (deterministic).
 int wgrad_reduce(const float* partial, void* dw, long long elems, int splits, int dtype, cudaStream_t st);
 
@@ -56,8 +48,9 @@ int wgrad_tc(const void* feats, const void* gout, const int32_t* pair_fwd, float
 
 int* device_status_ptr();
 
-// Variant of the tcgen05 kernel (gemm_tma.cu) whose weight slabs arrive by tiled TMA loads;
-// the gathered feature rows are copied with cp.async.
+// tcgen05 kernel (gemm_tma.cu): weight slabs by tiled TMA loads, gathered feature rows by cp.async.
+// `transposed_weight` selects the input-gradient view of the KRSC weight; `reversed`: offset k of the table
+// meets weight kv - 1 - k.
 bool gather_gemm_tma_supported(int n_dim, int r_dim, int kv, int dtype, int out_dtype, int precision,
                                bool transposed_weight);
 int gather_gemm_tma(const void* src, const void* w, const Epilogue& epi, const int32_t* pairs,

@@ -1,9 +1,14 @@
 // Implicit gather-GEMM on tcgen05: cp.async-gathered feature rows, TMA-loaded
 // weight slabs.
 //
-// Same computation and tiling as gemm_tc.cu (128 output rows per CTA, fp32
-// accumulator in tensor memory).  What differs is how a shared-memory stage is
-// filled:
+//   out[rm, n] = sum_k sum_r src[pairs[k, rm], r] * B_k[r, n]  (+ epilogue)
+//
+// for the forward pass (B_k[r, n] = W[n, k, r]) and, with the weight read
+// "transposed", for the input gradient (B_k[r, n] = W[r, k, n]).  One CTA owns
+// a tile of 128 output rows, taken in an order in which the rows of a tile share
+// kernel offsets; the accumulator, 128 lanes x N fp32 columns, lives in tensor
+// memory.  For every offset that a row of the tile has, and every chunk of the
+// reduction, a shared-memory stage is filled:
 //   * the 128 gathered feature rows are copied with 16-byte cp.async by two
 //     groups of two warps that take the stages in turn (a row's pieces go to
 //     neighbouring lanes, a thread copies one piece of 16, 8 or 4 rows, absent
@@ -13,9 +18,11 @@
 //   * the weight slab W[:, k, chunk] arrives through one tiled 3-D TMA load
 //     (one per column block for the input gradient) completing on the same
 //     mbarrier with complete_tx::bytes.
-// The row pitch in shared memory equals the swizzle span (32 / 64 / 128 bytes),
-// and is the widest that divides a row of channels: multiples of 16 channels
-// (16-bit) or 8 (TF32) are taken; other widths stay with gemm_tc.cu.
+// Operands lie in shared memory in the canonical layouts of tcgen05.mma: the rows
+// and the forward weight K-major, the input gradient's weight MN-major (a row is
+// one reduction index).  The row pitch equals the swizzle span (32 / 64 / 128
+// bytes), the widest that divides a row of channels: multiples of 16 channels
+// (16-bit) or 8 (TF32) are taken; other widths run on the CUDA cores.
 //
 // Measured alternatives on B200 (64 -> 64 channels, 723k rows, 7.1M pairs):
 // feeding the rows with TMA tile::gather4 (4 rows per instruction) reached
@@ -115,6 +122,7 @@ constexpr int kThreadsHybrid = kIssueThreads + 32;    // 160
 constexpr int kCopyGroups = 2;                        // halves of the copy warps; stages alternate between them
 constexpr int kGroupThreads = kIssueThreads / kCopyGroups;  // 64
 constexpr int kPassBytes = kGroupThreads * 16;        // one copy per thread of a group covers 1024 bytes of the tile
+constexpr int kMostSmem = 226 * 1024;                 // dynamic shared memory of a CTA
 constexpr int kMaxCtasPerSm = 4;                      // 4 x 160 threads x 96 registers fit the register file
 
 // 16-byte copy into shared memory; zeros instead when row < 0 (the source is then not read).
@@ -366,7 +374,7 @@ gather_gemm_tma_kernel(const __grid_constant__ TmaParams p, const __grid_constan
             if (p.epi.residual != nullptr)
               add_residual16<TO>(v, static_cast<const TO*>(p.epi.residual) + my_row * p.n_dim + c0);
           }
-          TO line[16];
+          alignas(16) TO line[16];
           store_row16<TO>(line, v);
 #pragma unroll
           for (int q = 0; q < static_cast<int>(sizeof(TO)); ++q)
@@ -501,16 +509,16 @@ CUtensorMapDataType tma_dtype(int dtype) {
 }
 
 // Swizzle span of rows holding `elems` contiguous elements: the widest of 128, 64 and 32 bytes that
-// divides them (48 channels of 16 bits: 32 bytes, 96 channels: 64), so that no copy is padding; 0 if none does.
+// divides them (48 channels of 16 bits: 32 bytes, 96 channels: 64), so that no copy is padding.
 int row_span(int elems, int elem_size) {
   const int bytes = elems * elem_size;
-  return bytes % 128 == 0 ? 128 : bytes % 64 == 0 ? 64 : bytes % 32 == 0 ? 32 : 0;
+  return bytes % 128 == 0 ? 128 : bytes % 64 == 0 ? 64 : 32;
 }
 
 template <typename T, typename TO, bool B_MN, int LPR>
 int launch_tma_rows(const TmaParams& p, const CUtensorMap& map_b, size_t smem_bytes, cudaStream_t st) {
   static bool configured[kMaxDevices] = {false};  // per instantiation and device
-  SPC_CUDA_OK(ensure_dynamic_smem(gather_gemm_tma_kernel<T, TO, B_MN, LPR>, 226 * 1024, configured));
+  SPC_CUDA_OK(ensure_dynamic_smem(gather_gemm_tma_kernel<T, TO, B_MN, LPR>, kMostSmem, configured));
   const unsigned grid = static_cast<unsigned>(ceil_div(p.m_rows, kTileM));
   gather_gemm_tma_kernel<T, TO, B_MN, LPR><<<grid, kThreadsHybrid, smem_bytes, st>>>(p, map_b);
   SPC_LAUNCH_OK();
@@ -528,10 +536,17 @@ int launch_tma(const TmaParams& p, const CUtensorMap& map_b, size_t smem_bytes, 
 
 bool gather_gemm_tma_supported(int n_dim, int r_dim, int kv, int dtype, int out_dtype, int precision,
                                bool transposed_weight) {
-  if (!gather_gemm_tc_supported(n_dim, r_dim, kv, dtype, out_dtype, precision, transposed_weight)) return false;
-  const int elem = (dtype == SPC_F32) ? 4 : 2;
-  if (row_span(r_dim, elem) == 0) return false;
-  if (transposed_weight && row_span(n_dim, elem) == 0) return false;
+  (void)kv;
+  const bool sixteen = dtype == SPC_F16 || dtype == SPC_BF16;
+  const bool tf32 = dtype == SPC_F32 && precision == SPC_PREC_TF32;
+  if (!sixteen && !tf32) return false;
+  // The MN-major weight slab of the input gradient is laid out for 16-bit elements only; a TF32 input gradient
+  // comes as a forward convolution with a prepared, transposed weight.
+  if (tf32 && (transposed_weight || out_dtype != SPC_F32)) return false;
+  if (sixteen && out_dtype != dtype && out_dtype != SPC_F32) return false;
+  if (n_dim < 16 || n_dim > 256 || n_dim % 16 != 0) return false;
+  const int step = sixteen ? 16 : 8;  // reduction elements of one tcgen05.mma: 32 bytes, the narrowest span
+  if (r_dim < step || r_dim % step != 0) return false;
   return encode_fn() != nullptr;
 }
 
@@ -586,8 +601,7 @@ int gather_gemm_tma(const void* src, const void* w, const Epilogue& epi, const i
     const size_t per_cta = (228 * 1024 - static_cast<size_t>(ctas) * 1024) / ctas - 256;
     p.stages = per_cta > fixed ? std::min<int>(kMaxStages, static_cast<int>((per_cta - fixed) / stage_bytes)) : 0;
   }
-  // the kernel's dynamic shared memory limit is set to 200 KB
-  while (p.stages > 2 && fixed + static_cast<size_t>(p.stages) * stage_bytes > 226 * 1024) --p.stages;
+  while (p.stages > 2 && fixed + static_cast<size_t>(p.stages) * stage_bytes > kMostSmem) --p.stages;
   // shared memory is carved out of the L1: beyond two stages, keep about 36 KB of the SM as cache
   // for the table and epilogue traffic (a third stage that took it cost 8 % on 64 -> 128)
   // (layers whose reduction spans several stages per offset keep the deeper pipeline: 128 -> 128

@@ -9,10 +9,6 @@ namespace spc {
 namespace tc {
 
 constexpr int kTileM = 128;
-constexpr int kRowBytes = 128;
-constexpr int kAStageBytes = kTileM * kRowBytes;  // 16 KB
-constexpr int kProducers = 128;
-constexpr int kThreadsTc = 160;
 constexpr int kGroup = 32;  // kernel offsets voted on together
 constexpr int kMaxStages = 8;
 // A wait polls kSpinLimit times, then keeps polling against a wall-clock limit, so that a slow

@@ -34,7 +34,7 @@ def gemm_path(request):
 
     g = _gemm()
     old = g.GEMM_PATH
-    # "cpasync": like auto, but the tcgen05 kernels are fed by cp.async, never by TMA
+    # "cpasync": the code of a kernel that is gone, which callers may still pass: as auto
     g.GEMM_PATH = {"simt": _lib.SPC_GEMM_SIMT, "auto": _lib.SPC_GEMM_AUTO,
                    "cpasync": _lib.SPC_GEMM_TCGEN05_CPASYNC}[request.param]
     yield request.param
