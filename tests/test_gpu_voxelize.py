@@ -115,3 +115,29 @@ def test_empty_and_wrong_inputs():
     feats = torch.arange(6.0, device=DEV).view(3, 2)
     back = gather_features_by_pc_voxel_id(feats, torch.tensor([2, -1, 0], device=DEV), invalid_value=-7)
     assert back.tolist() == [[4.0, 5.0], [-7.0, -7.0], [0.0, 1.0]]
+
+
+@pytest.mark.parametrize("clear,mean", [(True, False), (True, True), (False, False)])
+def test_the_combined_call_equals_its_two_halves(clear, mean):
+    """``spc_voxelize`` of the C ABI writes what ``spc_voxelize_number`` and ``spc_voxelize_store`` (the class) write."""
+    import ctypes
+
+    from spconv_triton_b200 import _lib
+    from spconv_triton_b200.pytorch.utils import PointToVoxel
+
+    lib, n, most, slots = _lib.load(), 20000, 3000, 5
+    g = torch.Generator().manual_seed(9)
+    pts = (torch.rand((n, 4), generator=g) * 12).to("cuda")
+    op = PointToVoxel([0.5] * 3, [0.0, 0.0, 0.0, 10.0, 10.0, 10.0], 4, most, slots, torch.device("cuda"))
+    exp = op.generate_voxel_with_id(pts, clear, mean)
+    voxels = torch.zeros((most, slots, 4), device="cuda")
+    indices, num = (torch.zeros(s, dtype=torch.int32, device="cuda") for s in ((most, 3), (most,)))
+    ids, found = torch.empty(n, dtype=torch.int64, device="cuda"), ctypes.c_int64(0)
+    ws = torch.empty(int(lib.spc_voxelize_workspace_bytes(n, most, slots)), dtype=torch.uint8, device="cuda")
+    floats, ints = ctypes.c_float * 3, ctypes.c_int32 * 3
+    _lib.check(lib.spc_voxelize(_lib.ptr(pts), n, 4, 3, 4, floats(0, 0, 0), floats(0.5, 0.5, 0.5), ints(20, 20, 20), most, slots,
+                                int(clear), int(mean), _lib.ptr(ws), ws.numel(), _lib.ptr(voxels), _lib.ptr(indices), _lib.ptr(num),
+                                _lib.ptr(ids), ctypes.byref(found), _lib.current_stream(pts.device)))
+    for got, want in zip((voxels, indices, num), exp):
+        assert torch.equal(got[:found.value], want)
+    assert torch.equal(ids, exp[3])
