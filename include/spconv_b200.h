@@ -191,7 +191,8 @@ int spc_rulebook_igemm_backward(const spc_geometry* g, const int32_t* indices, i
  *   kernel offsets; rows of the same offsets come in any order.
  * The input side (pair_bwd, pair_bwd_rowmajor, order_bwd) exists for strided and
  * transposed layers only; it may be asked for by a later call of its own with the
- * same workspace. */
+ * same workspace.  Calls on one workspace, repeated ones too, follow one another on
+ * one stream or are ordered by the caller: they share scratch. */
 int spc_rulebook_tables(const spc_geometry* g, const int32_t* indices, int64_t n_in, int64_t n_out,
                         void* workspace, size_t workspace_bytes, int32_t* out_indices,
                         int32_t* pair_fwd, int32_t* pair_fwd_rowmajor, int32_t* order_fwd,
@@ -426,8 +427,6 @@ int spc_tf32_prepare_weight(const float* weight, float* dst, int c_out, int kv, 
 int spc_tf32_prepare_operands(const float* src, float* dst, int64_t rows, int cols, int mode, const float* weight,
                               float* weight_dst, int c_out, int kv, int c_in, int transpose, int weight_mode, void* stream);
 
-/* Bytes of device scratch spc_conv_backward_weight needs (fp32 partial sums
- * of the split reduction). */
 /* spc_conv_backward_input for callers that hold one table: pair_bwd may be NULL when
  * pair_bwd_rowmajor is given and spc_conv_backward_input_needs_colmajor says 0.  With
  * `reversed` the tables are the forward tables of a submanifold layer, whose input
@@ -445,6 +444,8 @@ size_t spc_column_sums_workspace_bytes(int64_t rows, int cols);
 int spc_column_sums(const void* x, int64_t rows, int cols, int dtype, void* out, int out_dtype, void* workspace,
                     size_t workspace_bytes, void* stream);
 
+/* Bytes of device scratch spc_conv_backward_weight needs (fp32 partial sums
+ * of the split reduction). */
 size_t spc_conv_backward_weight_workspace_bytes(int64_t n_out, int c_in, int c_out, int kv);
 
 /* Weight gradient: replaces conv_backward_weight, _impl/gemm.py:634-713.

@@ -5,9 +5,9 @@
 // reads three 16-byte words for 32 multiply-adds (16 packed fma.rn.f32x2, the same IEEE results), a warp
 // four shared-memory wavefronts.  The tile's rows come in an order that groups rows with common offsets, a
 // warp skips the offsets that none of its 16 rows has, and the next stage's operands are in flight during the
-// multiplications.  SubM 64 -> 64, 100 k rows, 6.2 of 27 neighbours: forward and input gradient 425 us each in
-// natural order, 240 sorted, with 4 x 4 outputs a thread, scalar shared-memory reads and a barrier twice every
-// 16 channels; weight gradient 727 us.
+// multiplications.  SubM 64 -> 64, 100 k rows, 6.2 of 27 neighbours: forward 104 us, input gradient 97, weight
+// gradient 123 (49 - 51, 48 % of the issue slots; 128 registers, four CTAs a multiprocessor).  With 4 x 4 outputs a
+// thread, scalar shared-memory reads and a barrier twice every 16 channels: 425, 425 (240 with sorted rows), 727.
 #include <algorithm>
 
 #include "common.cuh"

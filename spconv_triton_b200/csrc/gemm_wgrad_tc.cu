@@ -8,15 +8,19 @@
 // reduction dimension.  One CTA owns (offset k, a contiguous range of output
 // rows, one or two blocks of <= 128 output channels) and keeps D (128 lanes x
 // c_in fp32 columns a block) in tensor memory; with 256 output channels both
-// blocks multiply the same feature rows, which two CTAs would gather twice
-// (k5 256 -> 256, 13.6 M pairs: 5.5 -> 3.9 ms):
-//   warps 0-7  scan pair_fwd[k, lo:hi] 256 entries at a time, compact the
+// blocks multiply the same feature rows, which two CTAs would gather twice.
+// Bound by the gathered rows on narrow layers (64 -> 128, 1.6 M pairs of a 27 x 1.36 M
+// table: 222 us, 631 MB read, a quarter of it the table; the tensor pipe at 5 %).  k5
+// 256 -> 256, 13.6 M pairs: 5.5 ms with a block a CTA, 2.53 now (704 TFLOP/s, 0.44 of
+// the measured peak).
+// W (four or eight) copy warps and one that multiplies:
+//   warps 0 .. W-1  scan pair_fwd[k, lo:hi] 1024 entries a round, compact the
 //              existing pairs into a shared-memory ring with warp ballots (no
 //              host-side nonzero(), unlike spconv_triton/pytorch/_impl/gemm.py:663),
 //              and for every 64 pairs copy the 64 grad_out rows and the 64
 //              feature rows into a swizzled stage with 16-byte cp.async
 //              (completion delivered by cp.async.mbarrier.arrive.noinc)
-//   warp 8     issues tcgen05.mma with BOTH operands MN-major: a stage row is
+//   warp W     issues tcgen05.mma with BOTH operands MN-major: a stage row is
 //              one pair and holds its channels contiguously, which is exactly
 //              how gathered rows arrive, so nothing is transposed
 //   warps 0-3  finally read TMEM and write the fp32 partial tile
@@ -157,7 +161,7 @@ wgrad_tc_kernel(const __grid_constant__ WgParams p) {
     int stage = 0;
     uint32_t empty_parity = 1;
     bool ok = true;
-    int head = 0, tail = 0;  // ring positions (uniform over the 256 threads)
+    int head = 0, tail = 0;  // ring positions (uniform over the copy threads)
     long long pos = lo;
     const int g_cols = min(p.n_blocks * kTileM, p.c_out - n0);  // output channels this CTA owns
     const int g_pieces = g_cols * ELEM / 16;
@@ -172,7 +176,7 @@ wgrad_tc_kernel(const __grid_constant__ WgParams p) {
     const bool f_even = (f_pieces & (f_pieces - 1)) == 0 && f_step >= 8;
     const uint32_t f_place = piece_place(f_first, f_piece, p.f_row_bytes);
 
-    // Table entries are fetched one scan round (1024 entries, four per thread) ahead:
+    // Table entries are fetched one scan round (1024 entries, SCAN per thread) ahead:
     // the loads of the next round are in flight while the stages of this one are built,
     // so the walk over a sparse table does not pay a memory latency per round.
     const int32_t* table = p.pair_fwd + static_cast<long long>(k) * p.n_out;
@@ -423,8 +427,17 @@ WgradSplit wgrad_tc_split(int64_t n_out, int c_in, int c_out, int kv) {
   // several CTAs per resident slot: offsets differ a lot in how many pairs they have (the centre
   // offset of a submanifold layer has all of them), and surplus CTAs even that out
   int64_t want = ceil_div(16 * static_cast<int64_t>(sm_count()), std::max<int64_t>(tiles, 1));
-  // the centre offset's CTAs are the longest chain: as short as the partial sums' traffic allows (10 k rows,
-  // 64 -> 64: 91 -> 34 us; at 128 x 128 and above the partial sums of 2048-row splits cost more than they give)
+  // Two costs: the centre offset's CTAs are the longest chain (as long as a split has rows), and every split writes
+  // c_out * kv * c_in partial sums that the reduction reads.  Few channels: short splits, many: long ones.  Rows a
+  // split 2048 / 4096, fp16, submanifold scenes a quarter full, microseconds:
+  //                    32->32     64->64     96->96    64->128    96->128   128->128   256->256
+  //   27, 10 k rows   42 / 70    44 / 73    83 / 149   50 / 85    55 / 95    48 / 79   83 / 128
+  //   27, 45 k        40 / 67    46 / 71    83 / 145   56 / 83    85 / 89    81 / 79  161 / 130
+  //   27, 150 k       81 / 76    93 / 85   205 / 185  118 / 103  243 / 216  239 / 202 486 / 357
+  //   125, 10 k       44 / 73    48 / 75    93 / 159   58 / 91    79 / 99    75 / 87  167 / 155
+  //   125, 40 k       89 / 79   103 / 87   239 / 191  138 / 107  290 / 218  284 / 204 620 / 398
+  // The line lies at 64 x 128: up to there 2048 rows gain a third at 10 - 45 k rows and lose a tenth at 150 k; beyond,
+  // 4096 gain from 45 k on and lose below (96 -> 96 up to 45 k as well).
   const int64_t by_len = std::max<int64_t>(1, n_out / (c_in * c_out <= 64 * 128 ? 2048 : 4096));
   want = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(want, by_len), 64));
   s.splits = static_cast<int>(want);

@@ -11,8 +11,11 @@
 // strided or transposed layer it walks the one to eight outputs of an INPUT row
 // and scatters the pair into both tables.  Output rows are numbered by the rank
 // of their bit, which is the ascending order torch.unique gives the reference,
-// without a sort.  No candidate grid, no atomics on the tables; the tables are
-// L2-resident (126 MB) up to a few hundred thousand rows.
+// without a sort (grids too large for a bitmap: a hash table and a library radix
+// sort of its keys).  No candidate grid.  A submanifold layer's entries are plain
+// stores; a strided layer's output side is cleared and scattered to with atomicMin
+// (the lowest input row of equal coordinates wins) and atomicOr (mask words).  The
+// tables are L2-resident (126 MB) up to a few hundred thousand rows.
 #include <cub/device/device_radix_sort.cuh>
 
 #include <algorithm>
