@@ -41,6 +41,13 @@ Tensor operand(const Tensor& t) {
   const Tensor c = t.contiguous();
   return (reinterpret_cast<uintptr_t>(c.const_data_ptr()) & 15u) != 0 ? c.clone() : c;
 }
+// Refuses operands of several GPUs: a kernel would be handed another GPU's addresses.
+void on_one_device(std::initializer_list<const Tensor*> ts) {
+  const Tensor& first = **ts.begin();
+  for (const Tensor* t : ts)
+    if (t->defined() && t->device() != first.device())
+      throw pybind11::value_error("expected all tensors on " + first.device().str() + ", found one on " + t->device().str());
+}
 int32_t* ints(const Tensor& t) { return t.defined() ? t.data_ptr<int32_t>() : nullptr; }
 void* data(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 int code_of(at::ScalarType t) {
@@ -128,12 +135,12 @@ struct Rulebook {
   Side side(bool input, bool colmajor) {
     if (input && subm()) throw Failure(SPC_ERR_INVALID_ARGUMENT, "a submanifold rulebook has one side");
     std::lock_guard<std::mutex> hold(lock);
-    c10::cuda::CUDAGuard guard(indices.device());
-    const auto now = c10::cuda::getCurrentCUDAStream();
     Side& kept = input ? bwd : fwd;
     Late& late = input ? late_bwd : late_fwd;
     const bool missing = !kept.rm.defined() || (colmajor && !kept.cm.defined());
     if (!missing && !late.stream) return kept;
+    c10::cuda::CUDAGuard guard(indices.device());
+    const auto now = c10::cuda::getCurrentCUDAStream();
     // A capture records its kernels and does not run them: it waits for nothing (what came before a capture is
     // done when the graph runs), and tables that it makes are its own.
     const bool capturing = c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
@@ -251,6 +258,7 @@ struct ConvOptions {
 
 Tensor conv_forward_raw(const Tensor& features, const Tensor& weight, const Tensor& bias, const Tensor& residual, const Book& rb,
                         const ConvOptions& o, at::ScalarType out_type, Tensor scale, Tensor shift, int act, double alpha) {
+  on_one_device({&features, &weight, &bias, &residual, &scale, &shift, &rb->indices});
   c10::cuda::CUDAGuard guard(features.device());
   Tensor x = operand(features), w = operand(weight.scalar_type() == x.scalar_type() ? weight : weight.to(x.scalar_type()));
   int64_t k_out = w.size(0), c_in = w.size(w.dim() - 1), kv = rb->geo->kv;
@@ -397,7 +405,7 @@ struct ConvBackward : public torch::autograd::Node {
     at::AutoGradMode no_grad(false);
     c10::cuda::CUDAGuard guard(grads[0].device());
     Tensor grad = operand(grads[0]);
-    if (bias && task_should_compute_output(2)) out[2] = column_sums(grad, bias_type);
+    if (bias && task_should_compute_output(2)) out[2] = bias_type == at::kDouble ? column_sums(grad, at::kFloat).to(at::kDouble) : column_sums(grad, bias_type);
     if (task_should_compute_output(0)) out[0] = conv_backward_input_raw(grad, weight, rb, options);
     if (task_should_compute_output(1)) out[1] = conv_backward_weight_raw(features, grad, weight.sizes(), rb, options);
     if (residual && task_should_compute_output(3)) out[3] = grads[0];
@@ -527,6 +535,7 @@ Tensor pool(const Tensor& features, const Book& rb, bool average) {
     at::NoGradGuard no_grad;
     c10::cuda::CUDAGuard guard(features.device());
     x = cast_for_autocast(features).contiguous();
+    on_one_device({&x, &rb->indices});
     if (x.size(0) != rb->n_in) throw pybind11::value_error("features do not match the rulebook of the layer");
     if (average) count = at::empty({rb->n_out}, rb->indices.options());
     out = pool_rows(average ? SPC_POOL_AVG_FORWARD : SPC_POOL_MAX_FORWARD, x, Tensor(), Tensor(), rb, false, Tensor(), count);
@@ -554,6 +563,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> voxelize(const Tensor& points, const 
                                                     const std::vector<int32_t>& grid, bool clear, bool empty_mean) {
   pybind11::gil_scoped_release release;
   at::NoGradGuard no_grad;
+  on_one_device({&points, &voxels, &indices, &num});
   c10::cuda::CUDAGuard guard(points.device());
   const Tensor pc = points.contiguous();
   const int64_t n = pc.size(0), most = voxels.size(0);

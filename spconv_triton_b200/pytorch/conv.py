@@ -351,12 +351,11 @@ class SparseConvolutionBase:
         """The forward pass through the host extension; None where a setting or a cached rulebook needs the
         operator functions."""
         features = x.features
-        dev = features.device
-        if (x.benchmark or not self.host_plannable() or not _host.takes(features, x.indices) or weight.device != dev
-                or x.indices.device != dev or not ops.unreplaced() or act_type.name not in ("None_", "ReLU", "Sigmoid", "LeakyReLU")
+        if (x.benchmark or not self.host_plannable() or not _host.takes(features, x.indices) or not weight.is_cuda
+                or not ops.unreplaced() or act_type.name not in ("None_", "ReLU", "Sigmoid", "LeakyReLU")
                 or weight.dtype not in _host.FLOATS):
             return None
-        if bias is not None and (bias.device != dev or bias.shape != (self.out_channels,) or bias.dtype not in _host.FLOATS):
+        if bias is not None and (not bias.is_cuda or bias.shape != (self.out_channels,)):
             return None  # broadcast or refused by the general path
         if not training and self.algo == ConvAlgo.Native and (
                 add_input is not None or features.dtype != weight.dtype or torch.is_autocast_enabled()
@@ -390,7 +389,7 @@ class SparseConvolutionBase:
             residual = None
             if add_input is not None and add_input.features.shape == (out_indices.shape[0], self.out_channels):
                 out_type = torch.float16 if torch.is_autocast_enabled() else features.dtype
-                if add_input.features.dtype == out_type and add_input.features.device == dev:
+                if add_input.features.dtype == out_type and add_input.features.device == features.device:
                     residual, add_input = add_input.features, None
             out_features = _host.ext().conv_train(features, weight, bias, residual, rb, self.inverse, tf32, split_most)
         else:

@@ -2,6 +2,7 @@
 
 from __future__ import annotations
 
+import operator
 import threading
 import time
 from collections import OrderedDict
@@ -127,14 +128,18 @@ class SparseSequential(SparseModule):
         return x
 
 
+_BN_TENSORS = ("weight", "bias", "running_mean", "running_var", "num_batches_tracked")
+
+
 def _folded_bn(bn: nn.BatchNorm1d):
     """fp32 (scale, shift) with bn(x) == x * scale + shift in evaluation mode;
     memoised on the module until one of its tensors changes.  (The counter of batches among them: a forward
     pass in training mode writes the running statistics past their version counters.)"""
-    tensors = (bn.weight, bn.bias, bn.running_mean, bn.running_var, bn.num_batches_tracked)
+    own = {**bn._parameters, **bn._buffers}  # (attributes of a module are a slow look-up)
+    tensors = tuple([own[n] if n in own else getattr(bn, n) for n in _BN_TENSORS])
     key = tuple((t._version, t.data_ptr()) if t is not None else None for t in tensors) + (bn.eps,)
     cached = getattr(bn, "_spc_folded", None)
-    if cached is not None and cached[0] == key and all(a is b for a, b in zip(cached[3], tensors, strict=True)):
+    if cached is not None and cached[0] == key and all(map(operator.is_, cached[3], tensors)):
         return cached[1], cached[2]
     with torch.no_grad():
         scale = torch.rsqrt(bn.running_var.float() + bn.eps)
