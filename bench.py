@@ -2,8 +2,7 @@
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 
-Workload (the configuration its metric is quoted on):
-VoxelNet-style sparse middle encoder, fp16 inference: SubMConv3d 4->16, then
+Workload: the VoxelNet-style sparse middle encoder, fp16 inference: SubMConv3d 4->16, then
 three stages of [SparseConv3d k3 s2 p1 + 2 x SubMConv3d k3] at 32 / 64 / 64
 channels, BatchNorm + ReLU after every convolution, grid [41, 1600, 1408],
 batch 8, 16k-24k voxels per sample drawn by the seeded plane-plus-clusters
@@ -120,7 +119,7 @@ UNET_WIDTHS = (32, 64, 128, 256)
 
 
 def build_unet(c_in=4, widths=UNET_WIDTHS):
-    """BASELINE configs[3]: encoder of SubM / stride-2 convolutions at 32 / 64 / 128 / 256
+    """encoder of SubM / stride-2 convolutions at 32 / 64 / 128 / 256
     channels, decoder of SparseInverseConv3d layers that reuse the encoder's
     indice_keys, BatchNorm + ReLU after every convolution."""
     import spconv_triton_b200.pytorch as sp
@@ -155,7 +154,7 @@ def make_unet_scenes(n_scenes=2, batch=UNET_BATCH, n_range=UNET_N_RANGE, grid=UN
 
 
 def run_train_arm(dev, rank, world, steps, warmup):
-    """BASELINE configs[3]: one training step = forward + backward of the sparse
+    """one training step = forward + backward of the sparse
     UNet under fp16 autocast, the data-parallel all-reduce of the parameter
     gradients (bucketed, overlapped with backward) and an SGD update.  The batch
     of 8 samples is sharded by sample over the ranks (strong scaling); returns
@@ -215,7 +214,7 @@ def run_train_arm(dev, rank, world, steps, warmup):
     reducer = GradientReducer(net.parameters(), bucket_bytes=4 << 20) if world > 1 else None
     ms, loss = timed(reducer)
     rec = {
-        "workload": "BASELINE configs[3]: sparse UNet 32/64/128/256 with SparseInverseConv3d decoder, fp16 autocast, "
+        "workload": "sparse UNet 32/64/128/256 with SparseInverseConv3d decoder, fp16 autocast, "
                     "forward + backward + gradient all-reduce + SGD step, grid [512,512,64], batch 8 over all ranks",
         "scaling": "strong", "n_gpus": world, "steps": steps, "warmup": warmup,
         "voxels_per_step": int(np.mean(voxels)), "ms_per_step": ms / steps,
@@ -461,7 +460,7 @@ def run_reference_arm(args):
         "n_gpus": args.gpus, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": 1e3 * sum(times) / len(times), "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f32", "data": "synthetic",
-        "config": {"workload": "BASELINE configs[2]: VoxelNet-style backbone, one sample per step (bounded sample)",
+        "config": {"workload": "VoxelNet-style backbone, one sample per step (bounded sample)",
                    "grid": GRID, "voxels_per_sample": list(N_RANGE)},
         "cpu_baseline": {"value": value, "unit": "Mvoxels/s", "cores": cores, "kind": "port",
                          "sample": f"{args.steps} steps of one sample each ({int(np.mean(voxels))} voxels avg), "
@@ -596,7 +595,7 @@ def run_backbone_reference_gpu(dev, steps, warmup):
 
 
 def blob_scene(seed, batch, n_per_sample, grid=256):
-    """Dense-ish random blobs: n_per_sample unique voxels per sample filling
+    """Dense-ish random blobs (30 % occupancy): n_per_sample unique voxels per sample filling
     random solid blobs of a grid^3 volume to 30 % occupancy."""
     from spconv_triton_b200.scenes import blob_batch
 
@@ -604,10 +603,10 @@ def blob_scene(seed, batch, n_per_sample, grid=256):
 
 
 def run_op_bench(args):
-    """Single-operator timings at the other BASELINE configurations (not the
-    headline line): ``--op pool`` = configs[4] SparseMaxPool3d k2 s2 and
+    """Single-operator timings of the other workloads (not the
+    headline line): ``--op pool`` = SparseMaxPool3d k2 s2 and
     SparseAvgPool3d k3 s1 at C = 256 fp16, 4 x 400k voxels in 256^3;
-    ``--op conv_s2`` = configs[1] SparseConv3d k3 s2 64 -> 128 fp16, 4 x 120k
+    ``--op conv_s2`` = SparseConv3d k3 s2 64 -> 128 fp16, 4 x 120k
     voxels; ``--op conv_subm`` = SubMConv3d k3 (forward, input and weight gradient)
     at 32, 64 and 128 channels on the voxel set two stride-2 layers leave of a
     4-sample LiDAR-like batch; ``--op voxelize`` = PointToVoxel on 1.2M points.
@@ -664,7 +663,7 @@ def run_op_bench(args):
         run_backbone_reference_gpu(dev, max(args.steps, 5), args.warmup)
         return
     if args.op == "conv_k5":
-        # BASELINE configs[4]: SubMConv3d k5 256 -> 256 fp16 (kv 125, Native rulebook) on 4 x 400k blob voxels
+        # SubMConv3d k5 256 -> 256 fp16 (kv 125, Native rulebook) on 4 x 400k blob voxels
         batch, c, n_per = 4, 256, args.k5_voxels
         idx = blob_scene(7, batch, n_per).to(dev)
         n = int(idx.shape[0])
@@ -898,7 +897,7 @@ def main():
                     help="independent steps in flight at a time, each issued by its own host thread and CUDA stream "
                          "(1 = one pass after the other); lowered to what the host cores of this rank allow")
     ap.add_argument("--no-train", action="store_true",
-                    help="skip the training-step record (BASELINE configs[3]) that follows the headline measurement")
+                    help="skip the training-step record (sparse UNet) that follows the headline measurement")
     ap.add_argument("--voxel-order", default="random", choices=["random", "sorted"],
                     help="--op pool: input voxel order (random = as a voxeliser emits them, sorted = as a previous layer's rulebook emits them)")
     args = ap.parse_args()
@@ -1150,7 +1149,7 @@ def main():
                       for d in idict.values())
     out = None
 
-    # ---- BASELINE configs[3]: the training step with the gradient all-reduce ---------------
+    # ---- the training step with the gradient all-reduce ---------------
     train = None
     if not args.no_train:
         torch.cuda.empty_cache()
@@ -1177,7 +1176,7 @@ def main():
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": dev_ms / args.steps, "higher_is_better": True,
         "scaling": "weak", "vs_baseline": None, "dtype": "f16", "data": "synthetic",
         "config": {
-            "workload": "BASELINE configs[2]: VoxelNet-style sparse middle encoder, fp16 inference, "
+            "workload": "VoxelNet-style sparse middle encoder, fp16 inference, "
                         "grid [41,1600,1408], batch 8 per GPU, 16k-24k voxels/sample, rulebooks rebuilt every step",
             "voxels_per_step": int(np.mean(voxels_per_scene)), "scenes": N_SCENES,
             "l2": f"inputs larger than L2: rulebook tables of one step hold {table_bytes / 1e6:.0f} MB "

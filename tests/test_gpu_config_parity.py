@@ -2,11 +2,11 @@
 module API (the composition of rulebook, GEMM, fused epilogue, run-ahead and
 autograd), at sizes the oracle finishes in seconds:
 
-* configs[2]  the VoxelNet-style backbone of bench.py on one ~20k-voxel sample,
+* the VoxelNet-style backbone of bench.py on one ~20k-voxel sample,
               BatchNorm/ReLU fold and rulebook run-ahead on and off;
-* configs[4]  SubMConv3d k5 256 -> 256 (kv 125, Native rulebook) on 120k blob
+* SubMConv3d k5 256 -> 256 (kv 125, Native rulebook) on 120k blob
               voxels, SubMConv4d k3 64 -> 64 on 50k voxels;
-* configs[3]  encoder / decoder with SparseInverseConv3d reusing the encoder's
+* encoder / decoder with SparseInverseConv3d reusing the encoder's
               rulebook, forward + backward under fp16 autocast, gradients
               against an fp64 gather-matmul over the oracle's tables;
 * fp32        TF32 mode against fp64 of the TF32-rounded operands (1e-5: the same
@@ -33,7 +33,7 @@ DEV = "cuda"
 
 
 # ---------------------------------------------------------------------------------------------
-# configs[2]: the backbone
+# the backbone
 # ---------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("fold", [True, False])
 @pytest.mark.parametrize("runahead", [True, False])
@@ -64,7 +64,7 @@ def test_config3_backbone_matches_oracle(fold, runahead):
 
 
 # ---------------------------------------------------------------------------------------------
-# configs[4]: k5 256 -> 256 (Native) and the 4-D layer
+# k5 256 -> 256 (Native) and the 4-D layer
 # ---------------------------------------------------------------------------------------------
 def test_config5_subm_k5_native_120k():
     import bench
@@ -136,7 +136,7 @@ def test_config5_subm4d_k3_50k():
 
 
 # ---------------------------------------------------------------------------------------------
-# configs[3]: encoder / decoder, forward + backward under autocast
+# encoder / decoder, forward + backward under autocast
 # ---------------------------------------------------------------------------------------------
 class _GatherMatmul(torch.nn.Module):
     """fp64 CPU restatement of one sparse convolution over given tables:

@@ -64,7 +64,7 @@ def _check_rulebook(res, n_in, out_shape, subm):
 
 
 def test_config2_strided_conv_64_128_fp16():
-    """BASELINE configs[1]: SparseConv3d k3 s2 p1, 64 -> 128, fp16, batch 4, ~120k voxels/sample."""
+    """SparseConv3d k3 s2 p1, 64 -> 128, fp16, batch 4, ~120k voxels/sample."""
     from spconv_triton_b200.pytorch._impl import gemm as G
     from spconv_triton_b200.pytorch._impl import pairs as P
 
@@ -100,7 +100,7 @@ def test_config2_strided_conv_64_128_fp16():
 
 
 def test_config3_backbone_rulebooks_and_determinism():
-    """BASELINE configs[2]: the VoxelNet-style backbone, batch 8, 16k-24k voxels/sample."""
+    """the VoxelNet-style backbone, batch 8, 16k-24k voxels/sample."""
     import bench
     import spconv_triton_b200.pytorch as sp
 
@@ -131,7 +131,7 @@ def test_config3_backbone_rulebooks_and_determinism():
 
 
 def test_config5_pools_256_channels():
-    """BASELINE configs[4]: SparseMaxPool3d k2 s2 and SparseAvgPool3d k3 s1 at C = 256 on ~30 %-occupancy blobs."""
+    """SparseMaxPool3d k2 s2 and SparseAvgPool3d k3 s1 at C = 256 on ~30 %-occupancy blobs."""
     import spconv_triton_b200.pytorch as sp
 
     rng = np.random.default_rng(3)
