@@ -207,11 +207,11 @@ def forward(container, x):
     for st, L in zip(steps, plan.layers):
         c = st.conv
         w = c.weight
-        if w.dtype != feats.dtype or w.device != dev or not w.is_contiguous():
+        if w.dtype != feats.dtype or w.device != dev or not w.is_contiguous() or w.numel() != c.out_channels * st.kv * c.in_channels:
             return None
         L.weight = w.data_ptr()
         b = c.bias
-        if b is not None and (b.dtype != feats.dtype or b.device != dev):
+        if b is not None and (b.dtype != feats.dtype or b.device != dev or b.shape != (c.out_channels,) or not b.is_contiguous()):
             return None
         L.bias = b.data_ptr() if b is not None else None
         if st.bn is not None:

@@ -23,13 +23,10 @@ def _torch_save(obj):
 
 @pytest.mark.parametrize("clone", [copy.deepcopy, lambda o: pickle.loads(pickle.dumps(o)), _torch_save],
                          ids=["deepcopy", "pickle", "torch.save"])
-@pytest.mark.parametrize("train", [False, True])
-@pytest.mark.parametrize("how", ["layers", "one call"])
+@pytest.mark.parametrize("train,how", [(False, "layers"), (True, "layers"), (False, "one call")])
 def test_copies_of_an_indice_dict(clone, train, how):
     import spconv_triton_b200.pytorch as sp
 
-    if how == "one call" and train:
-        pytest.skip("the native pass is inference")
     shape = [24, 22, 20]
     idx = unique_coords(7, 2500, 2, shape)
     net = sp.SparseSequential(sp.SubMConv3d(16, 16, 3, padding=1, indice_key="s"),

@@ -142,3 +142,26 @@ def test_weights_on_another_device_are_refused():
 
     with pytest.raises((ValueError, RuntimeError, AssertionError)):
         sp.SubMConv3d(16, 16, 3, padding=1)(_input(16))
+
+
+def test_a_bias_that_does_not_fit_stays_out_of_the_native_pass():
+    import spconv_triton_b200.pytorch as sp
+
+    net = sp.SparseSequential(sp.SubMConv3d(16, 16, 3, padding=1, bias=True)).to(DEV).half().eval()
+    x = _input(16, torch.float16)
+    with torch.no_grad():
+        net(x)
+        net[0].bias = torch.nn.Parameter(torch.zeros(1, device=DEV).half())
+        with pytest.raises(ValueError):
+            net(x)
+
+
+def test_a_bias_in_double_precision():
+    import spconv_triton_b200.pytorch as sp
+
+    layer, x = sp.SubMConv3d(16, 16, 3, padding=1, bias=True).to(DEV), _input(16)
+    layer.bias = torch.nn.Parameter(layer.bias.detach().double())
+    y = layer(x).features
+    y.sum().backward()
+    assert y.dtype == torch.float32 and layer.bias.grad.dtype == torch.float64
+    assert torch.equal(layer.bias.grad, torch.full_like(layer.bias.grad, N))
