@@ -360,7 +360,7 @@ int spc_rows_gather(const void* src, const int32_t* rows, int64_t n, int channel
  *   bias [c_out] dtype or NULL; out [n_out, c_out] out_dtype;
  *   mask_argsort [n_out] or NULL: the order in which rows are grouped into
  *   tiles (rows with equal offset bitmasks become neighbours);
- *   pair_fwd_rowmajor [n_out, kvp] or NULL: the row-major copy of pair_fwd
+ *   pair_fwd_rowmajor [n_out, kvp] or NULL, 16-byte aligned: the row-major copy of pair_fwd
  *   (spc_rulebook_igemm / spc_pairs_to_rowmajor); optional, only faster;
  *   out_scale, out_shift: fp32 [c_out] or both NULL; when given the store is
  *   out = act((acc + bias) * out_scale + out_shift), i.e. an inference

@@ -355,8 +355,8 @@ bool gather_gemm_f32_supported(int n_dim, int r_dim, int dtype, int out_dtype) {
 int gather_gemm_f32(const void* src, const void* w, const Epilogue& epi, const int32_t* pairs, const int32_t* pairs_rowmajor,
                     const int32_t* order, void* out, long long m_rows, int n_dim, int r_dim, int kv, bool transposed_weight, bool reversed,
                     cudaStream_t st) {
-  if (!aligned16(src) || !aligned16(w) || !aligned16(out))
-    return fail(SPC_ERR_UNSUPPORTED, "fp32 gather-GEMM: operands must be 16-byte aligned");
+  if (!aligned16(src) || !aligned16(w) || !aligned16(out) || !aligned16(pairs_rowmajor))
+    return fail(SPC_ERR_UNSUPPORTED, "fp32 gather-GEMM: operands and the row-major table must be 16-byte aligned");
   F32Params p{static_cast<const float*>(src), static_cast<const float*>(w), epi, pairs, pairs_rowmajor, order, static_cast<float*>(out),
               m_rows, n_dim, r_dim, kv, (kv + 3) & ~3, reversed};
   const dim3 grid(static_cast<unsigned>(ceil_div(m_rows, kTile)), static_cast<unsigned>(ceil_div(n_dim, kTile)));

@@ -557,8 +557,9 @@ int gather_gemm_tma(const void* src, const void* w, const Epilogue& epi, const i
     return fail(SPC_ERR_UNSUPPORTED, "TMA gather-GEMM: unsupported shape");
   if (src_rows <= 0 || src_rows >= (1ll << 31) - 1)
     return fail(SPC_ERR_SIZE_LIMIT, "TMA gather-GEMM: %lld source rows", static_cast<long long>(src_rows));
-  if ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(out)) & 15u)
-    return fail(SPC_ERR_UNSUPPORTED, "TMA gather-GEMM: operands must be 16-byte aligned");
+  if ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(out) |
+       reinterpret_cast<uintptr_t>(pairs_rowmajor)) & 15u)
+    return fail(SPC_ERR_UNSUPPORTED, "TMA gather-GEMM: operands and the row-major table must be 16-byte aligned");
   const int elem = (dtype == SPC_F32) ? 4 : 2;
   EncodeTiledFn encode = encode_fn();
 

@@ -54,6 +54,21 @@ def test_workspace_query_needs_no_gpu():
     assert _lib.load().spc_conv_backward_weight_workspace_bytes(100000, 64, 64, 27) > 0
 
 
+def test_a_row_major_table_off_its_boundary_is_refused():
+    """Its entries are read 16 bytes at a time; the check comes before anything is launched."""
+    from spconv_triton_b200 import _lib
+
+    at = lambda n: ctypes.c_void_p(n)  # noqa: E731  (never read)
+    for transposed in (False, True):
+        if transposed:
+            rc = _lib.load().spc_conv_backward_input(at(4096), at(4096), at(4096), at(4100), None, at(4096), 10, 10, 64, 64, 27, _lib.SPC_F32,
+                                                     _lib.SPC_PREC_IEEE, _lib.SPC_GEMM_AUTO, None)
+        else:
+            rc = _lib.load().spc_conv_forward(at(4096), at(4096), None, at(4096), at(4100), None, at(4096), 10, 10, 64, 64, 27, _lib.SPC_F32,
+                                              _lib.SPC_F32, _lib.SPC_PREC_IEEE, _lib.SPC_GEMM_AUTO, None, None, 0, 0.0, None)
+        assert rc == 5 and b"row-major table" in _lib.load().spc_last_error()
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     from spconv_triton_b200 import _lib
 
