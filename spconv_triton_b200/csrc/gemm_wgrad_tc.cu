@@ -102,8 +102,10 @@ __device__ __forceinline__ void copy_rows_any(uint32_t base, const uint8_t* src,
 }
 
 // SCAN: table entries a thread looks at per scan round.
+// The registers of three or two CTAs a multiprocessor: left to the compiler, eight copy warps took 115 a thread, which
+// is one CTA (128 -> 128, 383 k rows, 3.8 M pairs: 526 us; two, with 94: 350).
 template <typename T, int W, int SCAN>
-__global__ void __launch_bounds__(W * 32 + 32, W == 4 ? 3 : 1)
+__global__ void __launch_bounds__(W * 32 + 32, W == 4 ? 3 : 2)
 wgrad_tc_kernel(const __grid_constant__ WgParams p) {
   constexpr int kWgIssueWarps = W;
   constexpr int kWgIssueThreads = W * 32;
@@ -431,13 +433,13 @@ WgradSplit wgrad_tc_split(int64_t n_out, int c_in, int c_out, int kv) {
   // c_out * kv * c_in partial sums that the reduction reads.  Few channels: short splits, many: long ones.  Rows a
   // split 2048 / 4096, fp16, submanifold scenes a quarter full, microseconds:
   //                    32->32     64->64     96->96    64->128    96->128   128->128   256->256
-  //   27, 10 k rows   42 / 70    44 / 73    83 / 149   50 / 85    55 / 95    48 / 79   83 / 128
-  //   27, 45 k        40 / 67    46 / 71    83 / 145   56 / 83    85 / 89    81 / 79  161 / 130
-  //   27, 150 k       81 / 76    93 / 85   205 / 185  118 / 103  243 / 216  239 / 202 486 / 357
-  //   125, 10 k       44 / 73    48 / 75    93 / 159   58 / 91    79 / 99    75 / 87  167 / 155
-  //   125, 40 k       89 / 79   103 / 87   239 / 191  138 / 107  290 / 218  284 / 204 620 / 398
+  //   27, 10 k rows   42 / 70    44 / 74    83 / 149   50 / 85    54 / 93    50 / 81   81 / 130
+  //   27, 45 k        40 / 67    48 / 71    85 / 144   56 / 83    65 / 95    61 / 85  163 / 130
+  //   27, 150 k       81 / 77    95 / 87   206 / 185  119 / 106  173 / 151  177 / 142 486 / 359
+  //   125, 10 k       44 / 71    48 / 77    93 / 157   58 / 91    69 / 106   65 / 93  167 / 153
+  //   125, 40 k       89 / 79   104 / 89   239 / 189  138 / 108  208 / 157  212 / 148 622 / 400
   // The line lies at 64 x 128: up to there 2048 rows gain a third at 10 - 45 k rows and lose a tenth at 150 k; beyond,
-  // 4096 gain from 45 k on and lose below (96 -> 96 up to 45 k as well).
+  // 4096 gain a fifth and more from 150 k on (256 -> 256 from 45 k) and lose a third on few rows.
   const int64_t by_len = std::max<int64_t>(1, n_out / (c_in * c_out <= 64 * 128 ? 2048 : 4096));
   want = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(want, by_len), 64));
   s.splits = static_cast<int>(want);
