@@ -56,5 +56,11 @@ bool gather_gemm_tma_supported(int n_dim, int r_dim, int kv, int dtype, int out_
 int gather_gemm_tma(const void* src, const void* w, const Epilogue& epi, const int32_t* pairs,
                     const int32_t* pairs_rowmajor, const int32_t* order, void* out, long long src_rows, long long m_rows, int n_dim, int r_dim,
                     int kv, bool transposed_weight, bool reversed, int dtype, int out_dtype, int precision, cudaStream_t st);
+// The kernel behind it for many rows of one stage (gemm_stream.cu).
+bool gather_gemm_stream_takes(int n_dim, int r_dim, long long m_rows, int dtype);
+int gather_gemm_stream(const void* src, const void* w, const Epilogue& epi, const int32_t* pairs, const int32_t* pairs_rowmajor,
+                       const int32_t* order, void* out, long long m_rows, int n_dim, int r_dim, int kv, bool transposed_weight,
+                       bool reversed, int dtype, int out_dtype, cudaStream_t st);
+
 
 }  // namespace spc

@@ -50,34 +50,17 @@
 // epilogue; the first thread of a copy group also issues its stages' TMA
 // weight loads; warp 4 issues tcgen05.mma and counts the stages from the same
 // vote.  All waits are bounded.
-#include <cuda.h>
-
 #include <algorithm>
 #include <type_traits>
 
 #include "common.cuh"
 #include "gemm_internal.cuh"
-#include "tc_common.cuh"
+#include "gemm_tma_common.cuh"
 
 namespace spc {
 namespace {
 
 using namespace tc;
-
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2,
-                                            uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3, %4}], [%5];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
-      : "memory");
-}
-__device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
-  asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
-}
 
 struct TmaParams {
   const void* src;
@@ -99,10 +82,6 @@ struct TmaParams {
   int* status;
 };
 
-__host__ __device__ inline uint32_t layout_type_for(int row_bytes) {
-  return row_bytes == 128 ? 2u : (row_bytes == 64 ? 4u : 6u);
-}
-
 // Four copy warps + the MMA warp: 160 threads.  A small CTA lets three or four of them share an SM
 // (shared memory permitting), i.e. three or four MMA issuers and that many tiles whose table
 // load, pipeline drain and epilogue overlap the others' stages: 64 -> 64 went from 166 us with
@@ -122,17 +101,7 @@ constexpr int kThreadsHybrid = kIssueThreads + 32;    // 160
 constexpr int kCopyGroups = 2;                        // halves of the copy warps; stages alternate between them
 constexpr int kGroupThreads = kIssueThreads / kCopyGroups;  // 64
 constexpr int kPassBytes = kGroupThreads * 16;        // one copy per thread of a group covers 1024 bytes of the tile
-constexpr int kMostSmem = 226 * 1024;                 // dynamic shared memory of a CTA
 constexpr int kMaxCtasPerSm = 4;                      // 4 x 160 threads x 96 registers fit the register file
-
-// 16-byte copy into shared memory; zeros instead when row < 0 (the source is then not read).
-__device__ __forceinline__ void cp_async16_row(uint32_t dst, const void* src, int row) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.lt.s32 p, %2, 0;\n\t"
-      "cp.async.cg.shared.global [%0], [%1], 16, p;\n\t}" ::"r"(dst), "l"(src), "r"(row)
-      : "memory");
-}
 
 // LPR: lanes per row = 16-byte pieces of one A row in a stage (8, 4 or 2 for rows of 128, 64 or 32
 // bytes).  128 / LPR rows are covered by one copy per thread, so a thread copies piece
@@ -148,7 +117,8 @@ gather_gemm_tma_kernel(const __grid_constant__ TmaParams p, const __grid_constan
   constexpr int CP = kTileM / kRowsPass;          // copies per thread and stage: 16, 8, 4
 
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  // (an offset, not a rounded pointer: the compiler keeps knowing that these are shared-memory addresses)
+  uint8_t* const smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   const int stage_bytes = p.a_stage_bytes + p.b_stage_bytes;
   uint8_t* stage_base = smem;
   // table entries of the group, [offset][row / kRowsPass-th copy of thread row % kRowsPass]
@@ -476,45 +446,6 @@ gather_gemm_tma_kernel(const __grid_constant__ TmaParams p, const __grid_constan
 }
 
 // ---- host side ------------------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-  // The driver call needs the thread's context, which a thread that has made no runtime call yet (autograd's,
-  // whose first step may be an input gradient) does not have: an empty free makes it current.
-  static thread_local bool current = false;
-  if (!current) current = cudaFree(nullptr) == cudaSuccess;
-  static EncodeTiledFn fn = nullptr;
-  static bool tried = false;
-  if (!tried) {
-    tried = true;
-    void* raw = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &raw, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(raw);
-  }
-  return fn;
-}
-
-CUtensorMapSwizzle swizzle_for(int row_bytes) {
-  return row_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
-                          : (row_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
-}
-
-CUtensorMapDataType tma_dtype(int dtype) {
-  return dtype == SPC_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
-                          : (dtype == SPC_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32);
-}
-
-// Swizzle span of rows holding `elems` contiguous elements: the widest of 128, 64 and 32 bytes that
-// divides them (48 channels of 16 bits: 32 bytes, 96 channels: 64), so that no copy is padding.
-int row_span(int elems, int elem_size) {
-  const int bytes = elems * elem_size;
-  return bytes % 128 == 0 ? 128 : bytes % 64 == 0 ? 64 : 32;
-}
-
 template <typename T, typename TO, bool B_MN, int LPR>
 int launch_tma_rows(const TmaParams& p, const CUtensorMap& map_b, size_t smem_bytes, cudaStream_t st) {
   static bool configured[kMaxDevices] = {false};  // per instantiation and device
@@ -561,7 +492,9 @@ int gather_gemm_tma(const void* src, const void* w, const Epilogue& epi, const i
        reinterpret_cast<uintptr_t>(pairs_rowmajor)) & 15u)
     return fail(SPC_ERR_UNSUPPORTED, "TMA gather-GEMM: operands and the row-major table must be 16-byte aligned");
   const int elem = (dtype == SPC_F32) ? 4 : 2;
-  EncodeTiledFn encode = encode_fn();
+  if (gather_gemm_stream_takes(n_dim, r_dim, m_rows, dtype))
+    return gather_gemm_stream(src, w, epi, pairs, pairs_rowmajor, order, out, m_rows, n_dim, r_dim, kv, transposed_weight, reversed, dtype,
+                              out_dtype, st);
 
   TmaParams p{};
   p.src = src; p.epi = epi; p.pairs = pairs; p.pairs_rm = pairs_rowmajor; p.kvp = (kv + 3) & ~3; p.order = order; p.out = out;
@@ -620,29 +553,8 @@ int gather_gemm_tma(const void* src, const void* w, const Epilogue& epi, const i
   if (p.status == nullptr) return fail(SPC_ERR_CUDA, "TMA gather-GEMM: no device status word");
 
   CUtensorMap map_b;
-  // B: the KRSC weight [c_out][kv][c_in] as a 3-D tensor (c_in innermost)
-  {
-    const int c_in = transposed_weight ? n_dim : r_dim;
-    const int c_out = transposed_weight ? r_dim : n_dim;
-    const cuuint64_t dims[3] = {static_cast<cuuint64_t>(c_in), static_cast<cuuint64_t>(kv),
-                                static_cast<cuuint64_t>(c_out)};
-    const cuuint64_t strides[2] = {static_cast<cuuint64_t>(c_in) * elem, static_cast<cuuint64_t>(kv) * c_in * elem};
-    cuuint32_t box[3];
-    if (transposed_weight) {
-      box[0] = static_cast<cuuint32_t>(p.b_row_bytes / elem);  // output channels of one column block
-      box[1] = 1;
-      box[2] = static_cast<cuuint32_t>(epr);                   // reduction rows of one stage
-    } else {
-      box[0] = static_cast<cuuint32_t>(epr);
-      box[1] = 1;
-      box[2] = static_cast<cuuint32_t>(n_dim);
-    }
-    const cuuint32_t estr[3] = {1, 1, 1};
-    const CUresult r = encode(&map_b, tma_dtype(dtype), 3, const_cast<void*>(w), dims, strides, box, estr,
-                              CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_for(p.b_row_bytes),
-                              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(SPC_ERR_CUDA, "cuTensorMapEncodeTiled(B) failed: %d", static_cast<int>(r));
-  }
+  const int rc = weight_map(&map_b, w, n_dim, r_dim, kv, transposed_weight, p.b_row_bytes, epr, dtype);
+  if (rc != SPC_OK) return rc;
 
 #define SPC_TMA(T, TO)                                                                                   \
   return transposed_weight ? launch_tma<T, TO, true>(p, map_b, smem_bytes, st)                    \

@@ -60,6 +60,28 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     if (mbar_try_wait(bar, parity)) return true;
   return mbar_wait_slow(bar, parity);
 }
+// The same without a call, for places where many values are live: polls until the phase is complete or the time is up.
+__device__ __forceinline__ bool mbar_wait_timed(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 t0, t1;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "@p bra WAIT_DONE;\n\t"
+      "mov.u64 t0, %%globaltimer;\n\t"
+      "WAIT_AGAIN:\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "@p bra WAIT_DONE;\n\t"
+      "mov.u64 t1, %%globaltimer;\n\t"
+      "sub.u64 t1, t1, t0;\n\t"
+      "setp.lt.u64 q, t1, %4;\n\t"
+      "@q bra WAIT_AGAIN;\n\t"
+      "WAIT_DONE:\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity), "r"(kWaitHintNs), "l"(kWaitLimitNs)
+      : "memory");
+  return ok != 0;
+}
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t src_bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
 }
