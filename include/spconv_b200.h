@@ -444,6 +444,23 @@ size_t spc_column_sums_workspace_bytes(int64_t rows, int cols);
 int spc_column_sums(const void* x, int64_t rows, int cols, int dtype, void* out, int out_dtype, void* workspace,
                     size_t workspace_bytes, void* stream);
 
+/* Batch normalisation in training of x [rows, cols] (row-major, 16-byte aligned, cols a multiple of 16 bytes and at
+ * most 4096, rows >= 2), with the activation that follows it:
+ *   y = act((x - mean) * invstd * weight + bias),   mean, var over the rows, invstd = 1 / sqrt(var + eps)
+ * weight, bias [cols] fp32 or NULL; y of x's dtype (fp16, bf16, fp32; arithmetic in fp32, one rounding).
+ * save_mean, save_invstd [cols] are written for the backward call.  running_mean / running_var (both or neither) become
+ * (1 - momentum) * old + momentum * new (unbiased variance), *batches (device, or NULL) goes up by one.
+ * Backward: dx (or NULL), dweight, dbias (or NULL) of dy.  The workspace of both is spc_norm_act_workspace_bytes, 0 for
+ * shapes that the kernels do not take.  No counterpart in the reference, which runs the torch modules. */
+typedef enum { SPC_NORM_NONE = 0, SPC_NORM_RELU = 1, SPC_NORM_SILU = 2 } spc_norm_activation;
+size_t spc_norm_act_workspace_bytes(int64_t rows, int cols, int dtype);
+int spc_norm_act_forward(const void* x, const float* weight, const float* bias, float* running_mean, float* running_var,
+                         int64_t* batches, float momentum, float eps, int act, void* y, float* save_mean, float* save_invstd,
+                         void* workspace, size_t workspace_bytes, int64_t rows, int cols, int dtype, void* stream);
+int spc_norm_act_backward(const void* x, const void* dy, const float* weight, const float* bias, const float* save_mean,
+                          const float* save_invstd, int act, void* dx, float* dweight, float* dbias, void* workspace,
+                          size_t workspace_bytes, int64_t rows, int cols, int dtype, void* stream);
+
 /* Bytes of device scratch spc_conv_backward_weight needs (fp32 partial sums
  * of the split reduction). */
 size_t spc_conv_backward_weight_workspace_bytes(int64_t n_out, int c_in, int c_out, int kv);

@@ -115,6 +115,9 @@ _PROTOTYPES = {
     "spc_conv_backward_input_needs_colmajor": (c_int, [c_int] * 6),
     "spc_column_sums_workspace_bytes": (c_size_t, [c_int64, c_int]),
     "spc_column_sums": (c_int, [_P, c_int64, c_int, c_int, _P, c_int, _P, c_size_t, _P]),
+    "spc_norm_act_workspace_bytes": (c_size_t, [c_int64, c_int, c_int]),
+    "spc_norm_act_forward": (c_int, [_P] * 6 + [ctypes.c_float, ctypes.c_float, c_int] + [_P] * 4 + [c_size_t, c_int64, c_int, c_int, _P]),
+    "spc_norm_act_backward": (c_int, [_P] * 6 + [c_int] + [_P] * 4 + [c_size_t, c_int64, c_int, c_int, _P]),
     "spc_pool_row_order_workspace_bytes": (c_size_t, [c_int64]),
     "spc_pool_row_order": (c_int, [_P, c_int, c_int, c_int64, c_int64, _P, _P, c_size_t, _P]),
     "spc_pool": (c_int, [c_int, _P, _P, _P, _P, c_int, _P, _P, _P, _P, c_int64, c_int, c_int, c_int, _P]),

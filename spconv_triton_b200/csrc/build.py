@@ -18,7 +18,7 @@ from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
 HERE = Path(__file__).resolve().parent
-SOURCES = ["capi.cu", "rulebook.cu", "tile_order.cu", "gemm_simt.cu", "gemm_tma.cu", "gemm_stream.cu", "gemm_wgrad_tc.cu", "gemm.cu", "pool.cu", "voxelize.cu", "dense.cu", "hash.cu", "global_pool.cu", "from_dense.cu", "tf32_prep.cu", "sequence.cu", "column_sums.cu", "gemm_f32.cu"]
+SOURCES = ["capi.cu", "rulebook.cu", "tile_order.cu", "gemm_simt.cu", "gemm_tma.cu", "gemm_stream.cu", "gemm_wgrad_tc.cu", "gemm.cu", "pool.cu", "voxelize.cu", "dense.cu", "hash.cu", "global_pool.cu", "from_dense.cu", "tf32_prep.cu", "sequence.cu", "column_sums.cu", "norm.cu", "gemm_f32.cu"]
 LIB = HERE / "libspconv_b200.so"
 HOST = HERE / "_host.so"  # the layers' host side (host.cpp): a Python module over torch's C++ interface
 STAMP = HERE / "build" / "sources.sha256"

@@ -9,6 +9,7 @@
 #include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/autograd.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/basic_ops.h>
 #include <torch/csrc/autograd/functions/utils.h>
@@ -457,6 +458,121 @@ Tensor conv_eval(const Tensor& features, const Tensor& weight, const c10::option
                           weight.scalar_type(), scale.value_or(Tensor()), shift.value_or(Tensor()), act, alpha);
 }
 
+// ---- normalisation and activation -----------------------------------------------------------------------------------
+
+Tensor norm_scratch(const Tensor& x, int type) {
+  const size_t bytes = spc_norm_act_workspace_bytes(x.size(0), static_cast<int>(x.size(1)), type);
+  return at::empty({static_cast<int64_t>(std::max<size_t>(bytes, 16))}, x.options().dtype(at::kByte));
+}
+float* floats(const Tensor& t) { return t.defined() ? t.data_ptr<float>() : nullptr; }
+
+struct NormActBackward : public torch::autograd::Node {
+  SavedVariable x_, weight_, bias_;
+  Tensor mean, invstd;  // (of the forward pass; nobody else has them)
+  int act = 0;
+  double eps = 0.0;
+
+  variable_list apply(variable_list&& grads) override {
+    std::lock_guard<std::mutex> hold(mutex_);
+    variable_list out(3);
+    if (!grads[0].defined()) return out;
+    const Tensor x = x_.unpack(), weight = weight_.unpack(), bias = bias_.unpack();
+    TORCH_CHECK(mean.defined(), torch::autograd::ERR_BACKWARD_TWICE);
+    c10::cuda::CUDAGuard guard(grads[0].device());
+    if (at::GradMode::is_enabled()) {
+      // Gradients that are to be differentiated themselves: those of torch's functions of the same operands.
+      const Tensor z = at::batch_norm(x, weight, bias, Tensor(), Tensor(), true, 0.0, eps, false);
+      const Tensor y = act == SPC_NORM_SILU ? at::silu(z) : act == SPC_NORM_RELU ? at::relu(z) : z;
+      variable_list wanted;
+      std::vector<int> at;
+      const Tensor operands[3] = {x, weight, bias};
+      for (int i = 0; i < 3; ++i)
+        if (task_should_compute_output(i) && operands[i].defined()) {
+          wanted.push_back(operands[i]);
+          at.push_back(i);
+        }
+      if (wanted.empty()) return out;
+      const variable_list found = torch::autograd::grad({y}, wanted, {grads[0]}, true, true, true);
+      for (size_t i = 0; i < at.size(); ++i) out[at[i]] = found[i];
+      return out;
+    }
+    Tensor dy = grads[0].scalar_type() == x.scalar_type() ? grads[0] : grads[0].to(x.scalar_type());
+    dy = operand(dy);
+    Tensor dx, dweight, dbias;
+    if (task_should_compute_output(0)) dx = at::empty_like(x);
+    if (weight.defined() && task_should_compute_output(1)) dweight = at::empty_like(weight);
+    if (bias.defined() && task_should_compute_output(2)) dbias = at::empty_like(bias);
+    const int type = code_of(x.scalar_type());
+    const Tensor ws = norm_scratch(x, type);
+    check(spc_norm_act_backward(x.data_ptr(), dy.data_ptr(), floats(weight), floats(bias), floats(mean), floats(invstd), act, data(dx),
+                                floats(dweight), floats(dbias), ws.data_ptr(), ws.numel(), x.size(0), x.size(1), type, stream_of(x)));
+    out[0] = dx;
+    out[1] = dweight;
+    out[2] = dbias;
+    return out;
+  }
+  void release_variables() override {
+    std::lock_guard<std::mutex> hold(mutex_);
+    x_.reset_data();
+    weight_.reset_data();
+    bias_.reset_data();
+    mean.reset();
+    invstd.reset();
+  }
+  std::string name() const override { return "SparseBatchNormActBackward"; }
+};
+
+bool wide_floats(const Tensor& t, int64_t n, const Tensor& like) {
+  return t.scalar_type() == at::kFloat && t.dim() == 1 && t.size(0) == n && t.is_contiguous() && t.device() == like.device() &&
+         t.layout() == at::kStrided && !t._fw_grad(0).defined();
+}
+
+// BatchNorm1d in training and the activation after it; nothing where the operands are not what the kernels take (the
+// modules run then, and refuse what they refuse).
+c10::optional<Tensor> norm_act_train(const Tensor& x, const c10::optional<Tensor>& weight_opt, const c10::optional<Tensor>& bias_opt,
+                                     const Tensor& running_mean, const Tensor& running_var, const Tensor& batches, double momentum, double eps,
+                                     int act) {
+  const Tensor weight = weight_opt.value_or(Tensor()), bias = bias_opt.value_or(Tensor());
+  const auto type = x.scalar_type();
+  if ((type != at::kHalf && type != at::kBFloat16 && type != at::kFloat) || !x.is_cuda() || x.layout() != at::kStrided || x.dim() != 2 ||
+      !x.is_contiguous() || (reinterpret_cast<uintptr_t>(x.const_data_ptr()) & 15u) != 0 || x._fw_grad(0).defined() ||
+      weight.defined() != bias.defined())
+    return c10::nullopt;
+  const int64_t rows = x.size(0), cols = x.size(1);
+  if (cols > 4096 || spc_norm_act_workspace_bytes(rows, static_cast<int>(cols), code_of(type)) == 0) return c10::nullopt;
+  for (const Tensor* t : {&weight, &bias, &running_mean, &running_var})
+    if (t->defined() && !wide_floats(*t, cols, x)) return c10::nullopt;
+  if (batches.scalar_type() != at::kLong || batches.numel() != 1 || batches.device() != x.device()) return c10::nullopt;
+  pybind11::gil_scoped_release release;
+  const bool grad = wants_grad({&x, &weight, &bias});
+  Tensor y, mean, invstd;
+  {
+    at::NoGradGuard no_grad;
+    c10::cuda::CUDAGuard guard(x.device());
+    y = at::empty_like(x);
+    mean = at::empty({cols}, x.options().dtype(at::kFloat));
+    invstd = at::empty_like(mean);
+    const Tensor ws = norm_scratch(x, code_of(type));
+    check(spc_norm_act_forward(x.data_ptr(), floats(weight), floats(bias), floats(running_mean), floats(running_var),
+                               batches.data_ptr<int64_t>(), static_cast<float>(momentum), static_cast<float>(eps), act, y.data_ptr(),
+                               floats(mean), floats(invstd), ws.data_ptr(), ws.numel(), rows, static_cast<int>(cols), code_of(type),
+                               stream_of(x)));
+    batches.unsafeGetTensorImpl()->bump_version();  // (as its own increment does)
+  }
+  if (!grad) return y;
+  auto node = std::shared_ptr<NormActBackward>(new NormActBackward(), torch::autograd::deleteNode);
+  node->set_next_edges(torch::autograd::collect_next_edges(x, weight, bias));
+  node->x_ = SavedVariable(x, false);
+  node->weight_ = SavedVariable(weight, false);
+  node->bias_ = SavedVariable(bias, false);
+  node->mean = mean;
+  node->invstd = invstd;
+  node->act = act;
+  node->eps = eps;
+  torch::autograd::set_history(y, node);
+  return y;
+}
+
 // ---- pooling -------------------------------------------------------------------------------------------------------
 
 // Bytes of gathered rows from which on the gradient of an average works on the input rows in the order of the
@@ -629,6 +745,7 @@ PYBIND11_MODULE(_host, m) {
   m.def("record_stream", &record_stream);
   m.def("conv_train", &conv_train);
   m.def("conv_eval", &conv_eval);
+  m.def("norm_act_train", &norm_act_train);
   m.def("pool", &pool);
   m.def("voxelize", &voxelize);
 }

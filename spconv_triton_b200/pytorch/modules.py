@@ -12,6 +12,7 @@ from torch import nn
 
 from spconv_triton_b200 import _lib
 
+from ._impl import host as _host
 from .core import SparseConvTensor
 
 _depth = threading.local()  # nesting depth of SparseSequential.forward on this thread
@@ -110,7 +111,7 @@ class SparseSequential(SparseModule):
         i = 0
         while i < len(mods):
             module = mods[i]
-            fused = _try_fold_bn_relu(mods, i, x)
+            fused = _try_fold_bn_relu(mods, i, x) or _try_train_bn_act(mods, i, x)
             if fused is not None:
                 x, i = fused
             else:
@@ -182,6 +183,49 @@ def _try_fold_bn_relu(mods, i, x):
     if scale.device != x.features.device:
         return None
     return conv(x, _fold=(scale, shift, relu)), i + 2 + int(relu)
+
+
+_HOOKS = ("_forward_hooks", "_forward_pre_hooks", "_backward_hooks", "_backward_pre_hooks")
+_GLOBAL_HOOKS = ("_global_forward_hooks", "_global_forward_pre_hooks", "_global_backward_hooks", "_global_backward_pre_hooks")
+
+
+def _plain(module) -> bool:
+    """Nobody looks at what goes in and out of this module."""
+    own = module.__dict__
+    return "forward" not in own and not any(own.get(h) for h in _HOOKS)
+
+
+def _watched() -> bool:
+    """Something sees or changes the torch functions that the modules would call."""
+    return (any(getattr(torch.nn.modules.module, h, None) for h in _GLOBAL_HOOKS) or torch._C._len_torch_function_stack() > 0
+            or torch._C._len_torch_dispatch_stack() > 0 or torch._C._functorch.peek_interpreter_stack() is not None
+            or torch.compiler.is_compiling() or torch.jit.is_tracing())
+
+
+def _try_train_bn_act(mods, i, x):
+    """In training a BatchNorm1d and the ReLU or SiLU after it run as one operator (``spc_norm_act_*``) that passes over
+    the features twice in each direction; the activation sees the normalised features before they are rounded.  Returns
+    ``(new_x, next_index)``, or None where the modules run one by one: whatever the operator does not take, and wherever
+    something could see the tensor between the two."""
+    bn = mods[i]
+    if type(bn) not in (nn.BatchNorm1d, SparseBatchNorm) or not bn.training or not isinstance(x, SparseConvTensor):
+        return None
+    features = x.features
+    if (type(features) is not torch.Tensor or not features.is_cuda or features.dim() != 2 or x.indices.shape[0] == 0
+            or features.shape[1] != bn.num_features or bn.momentum is None or not bn.track_running_stats
+            or bn.running_mean is None or bn.running_var is None or bn.num_batches_tracked is None
+            or not _plain(bn) or _watched()):
+        return None
+    if any(type(t) not in (torch.Tensor, nn.Parameter) for t in (bn.weight, bn.bias) if t is not None):
+        return None
+    act, after = 0, i + 1
+    if after < len(mods) and _plain(mods[after]):
+        kind = type(mods[after])
+        act = 1 if kind in (nn.ReLU, SparseReLU) else 2 if kind is nn.SiLU else 0
+        after += 1 if act else 0
+    out = _host.ext().norm_act_train(features, bn.weight, bn.bias, bn.running_mean, bn.running_var, bn.num_batches_tracked,
+                                     bn.momentum, bn.eps, act)
+    return None if out is None else (x.replace_feature(out), after)
 
 
 def assign_name_for_sparse_modules(module: nn.Module):
