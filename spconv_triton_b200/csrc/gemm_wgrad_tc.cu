@@ -115,7 +115,8 @@ wgrad_tc_kernel(const __grid_constant__ WgParams p) {
   constexpr int UMMA_K = 32 / ELEM;  // 16 pairs per MMA
 
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  // (an offset, not a rounded pointer: the compiler keeps knowing that these are shared-memory addresses)
+  uint8_t* const smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   const int stage_bytes = p.g_stage_bytes + p.f_stage_bytes;
   uint8_t* stage_base = smem;
   int* ring_m = reinterpret_cast<int*>(smem + static_cast<size_t>(p.stages) * stage_bytes);  // output rows
@@ -430,17 +431,19 @@ WgradSplit wgrad_tc_split(int64_t n_out, int c_in, int c_out, int kv) {
   // offset of a submanifold layer has all of them), and surplus CTAs even that out
   int64_t want = ceil_div(16 * static_cast<int64_t>(sm_count()), std::max<int64_t>(tiles, 1));
   // Two costs: the centre offset's CTAs are the longest chain (as long as a split has rows), and every split writes
-  // c_out * kv * c_in partial sums that the reduction reads.  Few channels: short splits, many: long ones.  Rows a
-  // split 2048 / 4096, fp16, submanifold scenes a quarter full, microseconds:
-  //                    32->32     64->64     96->96    64->128    96->128   128->128   256->256
-  //   27, 10 k rows   42 / 70    44 / 74    83 / 149   50 / 85    54 / 93    50 / 81   81 / 130
-  //   27, 45 k        40 / 67    48 / 71    85 / 144   56 / 83    65 / 95    61 / 85  163 / 130
-  //   27, 150 k       81 / 77    95 / 87   206 / 185  119 / 106  173 / 151  177 / 142 486 / 359
-  //   125, 10 k       44 / 71    48 / 77    93 / 157   58 / 91    69 / 106   65 / 93  167 / 153
-  //   125, 40 k       89 / 79   104 / 89   239 / 189  138 / 108  208 / 157  212 / 148 622 / 400
-  // The line lies at 64 x 128: up to there 2048 rows gain a third at 10 - 45 k rows and lose a tenth at 150 k; beyond,
-  // 4096 gain a fifth and more from 150 k on (256 -> 256 from 45 k) and lose a third on few rows.
-  const int64_t by_len = std::max<int64_t>(1, n_out / (c_in * c_out <= 64 * 128 ? 2048 : 4096));
+  // c_out * kv * c_in partial sums that the reduction reads.  Few table entries (rows times offsets) leave the chip idle
+  // with long splits, many pay for short ones; wide layers have the larger sums.  Rows a split 1024 / 2048 / 4096,
+  // fp16, submanifold scenes a quarter full, microseconds:
+  //                         32->32            64->64          64->128          128->128          256->256
+  //   27 offsets, 10 k   27 /  42 /  70   30 /  44 /  74   34 /  50 /  85   38 /  50 /  81   67 /  81 / 130
+  //   125, 10 k          36 /  44 /  71   44 /  48 /  77   56 /  58 /  91   83 /  65 /  93  261 / 167 / 153
+  //   27, 45 k           40 /  40 /  67   46 /  48 /  71   58 /  56 /  83   93 /  61 /  85  276 / 163 / 130
+  //   27, 150 k          81 /  81 /  77   95 /  95 /  87  119 / 119 / 106  177 / 177 / 142  489 / 486 / 359
+  //   125, 40 k          89 /  89 /  79  105 / 104 /  89  138 / 138 / 108  212 / 212 / 148  622 / 622 / 400
+  // Entries: 0.27, 1.25, 1.2, 4.1 and 5 million; the lines lie between the rows where the better side changes.
+  const int64_t entries = n_out * kv, sums = static_cast<int64_t>(c_in) * c_out;
+  const int64_t few = sums <= 64 * 128 ? 1250000 : 400000, some = sums <= 128 * 128 ? 2400000 : 600000;
+  const int64_t by_len = std::max<int64_t>(1, n_out / (entries <= few ? 1024 : entries <= some ? 2048 : 4096));
   want = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(want, by_len), 64));
   s.splits = static_cast<int>(want);
   s.rows_per_split = ceil_div(std::max<int64_t>(n_out, 1), s.splits);
