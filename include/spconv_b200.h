@@ -382,6 +382,10 @@ int spc_conv_forward(const void* features, const void* weight, const void* bias,
 int spc_conv_forward_needs_colmajor(int c_in, int c_out, int kv, int dtype, int out_dtype, int precision,
                                     int path);
 
+/* 1 if a convolution in fp32 with so many rows of n_dim channels, r_dim channels added up, runs on the kernel for few
+ * rows (it reads the row-major table and no row order), given SPC_PREC_IEEE and SPC_GEMM_AUTO. */
+int spc_conv_small(int64_t rows, int n_dim, int r_dim, int kv);
+
 /* spc_conv_forward with a residual connection fused into the store:
  *   out[m, n] = act((acc + bias[n]) * scale[n] + shift[n]) + residual[m, n]
  * residual [n_out, c_out] has the OUTPUT dtype (16-byte aligned, NULL = none) and is

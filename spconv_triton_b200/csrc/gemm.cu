@@ -34,6 +34,10 @@ bool f32_aligned(const void* a, const void* b, const void* c) {
 
 }  // namespace
 
+extern "C" int spc_conv_small(int64_t rows, int n_dim, int r_dim, int kv) {
+  return rows > 0 && n_dim > 0 && r_dim > 0 && kv > 0 && gather_gemm_small_takes(rows, n_dim, r_dim, kv) ? 1 : 0;
+}
+
 extern "C" int spc_conv_forward_needs_colmajor(int c_in, int c_out, int kv, int dtype, int out_dtype, int precision,
                                                int path) {
   path = known_path(path);
@@ -79,6 +83,9 @@ extern "C" int spc_conv_forward_residual(const void* features, const void* weigh
                            /*transposed_weight=*/false, /*reversed=*/false, dtype, out_dtype, precision, st);
   }
   if (status != SPC_OK) return status;
+  if (path == SPC_GEMM_AUTO && dtype == SPC_F32 && out_dtype == SPC_F32 && pair_fwd_rowmajor != nullptr &&
+      gather_gemm_small_takes(n_out, c_out, c_in, kv) && f32_aligned(features, weight, pair_fwd_rowmajor))
+    return gather_gemm_small(features, weight, epi, pair_fwd_rowmajor, out, n_out, c_out, c_in, kv, false, false, st);
   if (path == SPC_GEMM_AUTO && gather_gemm_f32_supported(c_out, c_in, dtype, out_dtype) && f32_aligned(features, weight, out))
     return gather_gemm_f32(features, weight, epi, pair_fwd, pair_fwd_rowmajor, mask_argsort, out, n_out, c_out, c_in, kv,
                            /*transposed_weight=*/false, /*reversed=*/false, st);
@@ -121,6 +128,9 @@ extern "C" int spc_conv_backward_input_tables(const void* grad_out, const void* 
                            /*transposed_weight=*/true, reversed != 0, dtype, dtype, precision, st);
   }
   if (status != SPC_OK) return status;
+  if (path == SPC_GEMM_AUTO && dtype == SPC_F32 && pair_bwd_rowmajor != nullptr && gather_gemm_small_takes(n_in, c_in, c_out, kv) &&
+      f32_aligned(grad_out, weight, pair_bwd_rowmajor))
+    return gather_gemm_small(grad_out, weight, Epilogue{}, pair_bwd_rowmajor, din, n_in, c_in, c_out, kv, true, reversed != 0, st);
   if (path == SPC_GEMM_AUTO && gather_gemm_f32_supported(c_in, c_out, dtype, dtype) && f32_aligned(grad_out, weight, din))
     return gather_gemm_f32(grad_out, weight, Epilogue{}, pair_bwd, pair_bwd_rowmajor, mask_argsort, din, n_in, c_in, c_out, kv,
                            /*transposed_weight=*/true, reversed != 0, st);

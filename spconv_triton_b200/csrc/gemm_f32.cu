@@ -345,9 +345,96 @@ wgrad_f32_kernel(const float* __restrict__ feats, const float* __restrict__ gout
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+// Few rows (the rule is at gather_gemm_small_takes): a tile of any kernel that stages operands is one chain of 10 - 20 offsets
+// on a chip that is nearly empty.  Here 16 lanes have a row, an output channel each (up to four), find the row's offsets in
+// its own table entries and read rows and weights through the caches: as many rounds as a row has neighbours.
+// Bound: latency of two or three dependent loads a neighbour.  2 000 rows, 16 -> 16, 1.2 neighbours: 4.4 us, against 17 for
+// the tensor cores, 2 for their operands' copies and 9 for the row order that the copies' kernel wants and this one does not.
+constexpr int kSmallRows = kThreads / 16;
+
+template <bool W_MN, int NC>  // NC: output channels of a lane
+__global__ void __launch_bounds__(kThreads)
+gather_gemm_small_kernel(const __grid_constant__ F32Params p) {
+  __shared__ __align__(16) int entries[kSmallRows][32];
+  const int group = threadIdx.x >> 4, lane = threadIdx.x & 15;
+  const long long row = static_cast<long long>(blockIdx.x) * kSmallRows + group;
+  uint32_t mine = 0;
+  if (lane < 8) {
+    int4 e = make_int4(-1, -1, -1, -1);
+    if (row < p.m_rows && 4 * lane < p.kvp) e = __ldg(reinterpret_cast<const int4*>(p.pairs_rm + row * p.kvp) + lane);
+    *reinterpret_cast<int4*>(&entries[group][4 * lane]) = e;
+    mine = ((e.x >= 0 ? 1u : 0u) | (e.y >= 0 ? 2u : 0u) | (e.z >= 0 ? 4u : 0u) | (e.w >= 0 ? 8u : 0u)) << (4 * lane);
+  }
+#pragma unroll
+  for (int s = 8; s > 0; s >>= 1) mine |= __shfl_xor_sync(0xffffffffu, mine, s);
+  __syncwarp();
+  float acc[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) acc[c] = 0.f;
+  for (uint32_t rest = mine; rest != 0; rest &= rest - 1) {
+    const int kk = __ffs(rest) - 1, k = p.reversed ? p.kv - 1 - kk : kk;
+    const float4* const x = reinterpret_cast<const float4*>(p.src + static_cast<long long>(entries[group][kk]) * p.r_dim);
+#pragma unroll 4
+    for (int r = 0; r < p.r_dim; r += 4) {
+      const float4 a = __ldg(x + (r >> 2));
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const int n = lane + 16 * c;
+        float4 b;
+        if (W_MN) {
+          const float* const w = p.w + (static_cast<long long>(r) * p.kv + k) * p.n_dim + n;
+          const long long pitch = static_cast<long long>(p.kv) * p.n_dim;
+          b = make_float4(__ldg(w), __ldg(w + pitch), __ldg(w + 2 * pitch), __ldg(w + 3 * pitch));
+        } else {
+          b = __ldg(reinterpret_cast<const float4*>(p.w + (static_cast<long long>(n) * p.kv + k) * p.r_dim + r));
+        }
+        acc[c] = fmaf(a.x, b.x, acc[c]);
+        acc[c] = fmaf(a.y, b.y, acc[c]);
+        acc[c] = fmaf(a.z, b.z, acc[c]);
+        acc[c] = fmaf(a.w, b.w, acc[c]);
+      }
+    }
+  }
+  if (row >= p.m_rows) return;
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const int n = lane + 16 * c;
+    float v = apply_epilogue<float>(acc[c], p.epi, n);
+    if (p.epi.residual != nullptr) v += static_cast<const float*>(p.epi.residual)[row * p.n_dim + n];
+    p.out[row * p.n_dim + n] = v;
+  }
+}
+
 }  // namespace
 
 // Thin layers (at most 8 reduction channels) have kernels of their own.
+// 9 to 64 channels, one table word of offsets, and at most 2 M row-channel-channel products an offset: beyond that the
+// weights' way through the L1 (a kilobyte a pair at 16 x 16) costs more than the tiles save.
+bool gather_gemm_small_takes(long long m_rows, int n_dim, int r_dim, int kv) {
+  return kv <= 32 && n_dim % 16 == 0 && n_dim <= 64 && r_dim % 4 == 0 && r_dim > 8 && r_dim <= 64 && m_rows * n_dim * r_dim <= (2ll << 20);
+}
+
+int gather_gemm_small(const void* src, const void* w, const Epilogue& epi, const int32_t* pairs_rowmajor, void* out, long long m_rows,
+                      int n_dim, int r_dim, int kv, bool transposed_weight, bool reversed, cudaStream_t st) {
+  F32Params p{static_cast<const float*>(src), static_cast<const float*>(w), epi, nullptr, pairs_rowmajor, nullptr,
+              static_cast<float*>(out), m_rows, n_dim, r_dim, kv, (kv + 3) & ~3, reversed ? 1 : 0};
+  const unsigned grid = static_cast<unsigned>(ceil_div(m_rows, kSmallRows));
+#define SPC_SMALL(NC)                                                                    \
+  case NC:                                                                               \
+    if (transposed_weight) gather_gemm_small_kernel<true, NC><<<grid, kThreads, 0, st>>>(p); \
+    else gather_gemm_small_kernel<false, NC><<<grid, kThreads, 0, st>>>(p);              \
+    break;
+  switch (n_dim / 16) {
+    SPC_SMALL(1)
+    SPC_SMALL(2)
+    SPC_SMALL(3)
+    SPC_SMALL(4)
+  }
+#undef SPC_SMALL
+  SPC_LAUNCH_OK();
+  return SPC_OK;
+}
+
 bool gather_gemm_f32_supported(int n_dim, int r_dim, int dtype, int out_dtype) {
   return dtype == SPC_F32 && out_dtype == SPC_F32 && n_dim % 4 == 0 && r_dim % 4 == 0 && r_dim > 8;
 }

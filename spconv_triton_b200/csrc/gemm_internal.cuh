@@ -28,6 +28,9 @@ int wgrad_simt(const void* feats, const void* gout, const int32_t* pair_fwd, voi
                int64_t n_out, int c_in, int c_out, int kv, int dtype, cudaStream_t st);
 
 // IEEE fp32 kernels for channel counts that are multiples of four (gemm_f32.cu).
+bool gather_gemm_small_takes(long long m_rows, int n_dim, int r_dim, int kv);
+int gather_gemm_small(const void* src, const void* w, const Epilogue& epi, const int32_t* pairs_rowmajor, void* out, long long m_rows,
+                      int n_dim, int r_dim, int kv, bool transposed_weight, bool reversed, cudaStream_t st);
 bool gather_gemm_f32_supported(int n_dim, int r_dim, int dtype, int out_dtype);
 int gather_gemm_f32(const void* src, const void* w, const Epilogue& epi, const int32_t* pairs, const int32_t* pairs_rowmajor,
                     const int32_t* order, void* out, long long m_rows, int n_dim, int r_dim, int kv, bool transposed_weight, bool reversed,

@@ -215,8 +215,9 @@ struct Fp32Plan {
   bool tensor = false;
   int rows_mode = 0, weight_mode = 0, mult = 1;
 };
-Fp32Plan fp32_plan(int n_dim, int r_dim, int kv, bool tf32, int split_most) {
+Fp32Plan fp32_plan(int64_t rows, int n_dim, int r_dim, int kv, bool tf32, int split_most) {
   Fp32Plan p;
+  if (!tf32 && spc_conv_small(rows, n_dim, r_dim, kv)) return p;
   if (n_dim % 16 || n_dim < 16 || n_dim > 256 || r_dim % 8) return p;
   if (tf32) {
     p.tensor = true;
@@ -282,7 +283,7 @@ Tensor conv_forward_raw(const Tensor& features, const Tensor& weight, const Tens
   Prepared copies;
   int precision = x.scalar_type() == at::kFloat && o.tf32 ? SPC_PREC_TF32 : SPC_PREC_IEEE;
   if (x.scalar_type() == at::kFloat && out_type == at::kFloat) {
-    const Fp32Plan plan = fp32_plan(k_out, c_in, kv, o.tf32, o.split_most);
+    const Fp32Plan plan = fp32_plan(n_out, k_out, c_in, kv, o.tf32, o.split_most);
     if (plan.tensor) {
       copies = prepared(x, w, 0, plan);
       from = copies.rows;
@@ -310,7 +311,7 @@ Tensor conv_backward_input_raw(const Tensor& grad, const Tensor& weight, const B
   const bool reversed = rb->subm(), input = !reversed && !o.inverse;
   const int type = code_of(grad.scalar_type());
   const int precision = type == SPC_F32 && o.tf32 ? SPC_PREC_TF32 : SPC_PREC_IEEE;
-  const Fp32Plan plan = type == SPC_F32 ? fp32_plan(c_in, k_out, kv, o.tf32, o.split_most) : Fp32Plan();
+  const Fp32Plan plan = type == SPC_F32 ? fp32_plan(n_in, c_in, k_out, kv, o.tf32, o.split_most) : Fp32Plan();
   if (plan.tensor) {
     // as a forward convolution of grad with the transposed weight
     const Prepared copies = prepared(grad, w, reversed ? 2 : 1, plan);
@@ -746,6 +747,10 @@ PYBIND11_MODULE(_host, m) {
   m.def("conv_train", &conv_train);
   m.def("conv_eval", &conv_eval);
   m.def("norm_act_train", &norm_act_train);
+  // both directions of an IEEE fp32 layer run on the kernel for few rows
+  m.def("small", [](int64_t rows, int c_out, int c_in, int kv) {
+    return spc_conv_small(rows, c_out, c_in, kv) != 0 && spc_conv_small(rows, c_in, c_out, kv) != 0;
+  });
   m.def("pool", &pool);
   m.def("voxelize", &voxelize);
 }

@@ -64,6 +64,12 @@ FP32_ON_TENSOR_CORES = True
 FP32_SPLIT_MAX_REDUCTION = 1024
 
 
+def _small(rows, n_dim, r_dim, kv, t, out_dtype=torch.float32):
+    """Whether an IEEE fp32 layer runs on the CUDA-core kernel for few rows (it reads the row-major table)."""
+    return (t.dtype == torch.float32 and out_dtype == torch.float32 and GEMM_PATH == _lib.SPC_GEMM_AUTO and FP32_ON_TENSOR_CORES
+            and not constants.SPCONV_ALLOW_TF32 and bool(_lib.load().spc_conv_small(rows, n_dim, r_dim, kv)))
+
+
 def _fp32_plan(n_dim, r_dim, kv):
     """(mode for the gathered operand, mode for the weight, reduction multiplier) if an fp32 layer
     with ``n_dim`` outputs and reduction ``r_dim`` per kernel offset can run on the tcgen05
@@ -147,6 +153,8 @@ def conv_forward(features, filters_krsc, pair_fwd, n_out, bias=None, out_dtype=N
             scale, shift, act, alpha = epilogue
         precision, tensor_cores = _precision(feats), None
         plan = _fp32_plan(k_out, c_in, kv) if feats.dtype == torch.float32 and out_dtype == torch.float32 else None
+        if _small(n_out, k_out, c_in, kv, feats, out_dtype):
+            plan, tensor_cores = None, True  # (the row-major table, as for the tensor cores)
         if plan is not None:
             feats = _prepared_rows(feats, plan[0], plan[2])
             w = _prepared_weight(w, False, plan[1], plan[2])
@@ -181,7 +189,8 @@ def conv_backward_input(grad_out, filters_krsc, pair_bwd, n_in, pair_mask=None, 
         pb = pair_bwd if pair_bwd.is_contiguous() else pair_bwd.contiguous()
         order = _order(kv, pair_mask, mask_argsort)
         plan = _fp32_plan(c_in, k_out, kv) if g.dtype == torch.float32 else None
-        if plan is not None:
+        small = _small(n_in, c_in, k_out, kv, g)
+        if plan is not None and not small:
             # the input gradient as a forward convolution of grad_out with the transposed weight
             gp = _prepared_rows(g, plan[0], plan[2])
             wt = _prepared_weight(w, True, plan[1], plan[2])
@@ -191,7 +200,7 @@ def conv_backward_input(grad_out, filters_krsc, pair_bwd, n_in, pair_mask=None, 
                 _lib.SPC_PREC_TF32, GEMM_PATH, None, None, _lib.SPC_ACT_NONE, 0.0, _lib.current_stream(dev)))
             return din
         _lib.check(_lib.load().spc_conv_backward_input(
-            _lib.ptr(g), _lib.ptr(w), _lib.ptr(pb), _lib.ptr(_rowmajor(pair_bwd, g)), _lib.ptr(order), _lib.ptr(din), n_in, g.shape[0], c_in,
+            _lib.ptr(g), _lib.ptr(w), _lib.ptr(pb), _lib.ptr(_rowmajor(pair_bwd, g, True if small else None)), _lib.ptr(order), _lib.ptr(din), n_in, g.shape[0], c_in,
             k_out, kv, _lib.dtype_code(g.dtype), _precision(g), GEMM_PATH, _lib.current_stream(dev)))
     return din
 

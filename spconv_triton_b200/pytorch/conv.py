@@ -324,7 +324,7 @@ class SparseConvolutionBase:
     def host_plannable(self) -> bool:
         """Whether the layer's rulebook can be a native one (its tensors permitting)."""
         return not self.conv1x1 and (self.algo == ConvAlgo.Native or
-                                     (self.algo == ConvAlgo.MaskImplicitGemm and int(np.prod(self.kernel_size)) <= 32))
+                                     (self.algo == ConvAlgo.MaskImplicitGemm and math.prod(self.kernel_size) <= 32))
 
     def host_rulebook(self, indices, batch_size, spatial_shape, training):
         """A new native rulebook, or None where the operator functions have to raise."""
@@ -334,7 +334,13 @@ class SparseConvolutionBase:
         # training reads column-major tables for the weight gradient, and layers too narrow for the tensor
         # cores read them in the forward direction
         colmajor = training or self.in_channels % 16 != 0 or self.out_channels % 16 != 0
-        return _host.build(self, geo[0], indices, spatial_shape, training and not self.subm, colmajor)
+        # an fp32 layer of few rows wants no row order (layers that share its rulebook may: at 32 tiles 9 us of sorting
+        # against 4 us a layer)
+        rows = indices.shape[0]
+        small = (self.subm and rows <= 4096 and self.weight.dtype == torch.float32 and not constants.SPCONV_ALLOW_TF32
+                 and not torch.is_autocast_enabled()
+                 and _host.ext().small(rows, self.out_channels, self.in_channels, math.prod(self.kernel_size)))
+        return _host.build(self, geo[0], indices, spatial_shape, training and not self.subm, colmajor, not small)
 
     def host_entry(self, rb, indices, batch_size, spatial_shape, out_spatial_shape, training):
         if self.algo == ConvAlgo.Native:

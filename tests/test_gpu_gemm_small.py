@@ -1,0 +1,73 @@
+"""The fp32 gather-GEMM for few rows (csrc/gemm_f32.cu) against fp64, and the layers that run on it."""
+
+import ctypes
+
+import pytest
+import torch
+
+import spconv_triton_b200.pytorch as sp
+from spconv_triton_b200 import _lib, constants
+
+pytestmark = pytest.mark.gpu
+
+
+def _p(t):
+    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+
+
+@pytest.mark.parametrize("rows,n,r,kv", [(1, 16, 12, 27), (7, 64, 64, 1), (8, 48, 16, 8), (9, 32, 20, 32), (2000, 16, 16, 27),
+                                         (512, 64, 64, 27), (8191, 16, 16, 3)])
+def test_against_fp64(rows, n, r, kv):
+    lib = _lib.load()
+    assert lib.spc_conv_small(rows, n, r, kv) == 1
+    gen = torch.Generator("cuda").manual_seed(rows)
+    n_in = rows + 5
+    x, w = torch.randn(n_in, r, generator=gen, device="cuda"), torch.randn(n, kv, r, generator=gen, device="cuda")
+    bias, residual = torch.randn(n, generator=gen, device="cuda"), torch.randn(rows, n, generator=gen, device="cuda")
+    table = torch.randint(0, n_in, (rows, kv), generator=gen, device="cuda").int()
+    table[torch.rand(rows, kv, generator=gen, device="cuda") < 0.7] = -1
+    rm = torch.full((rows, (kv + 3) // 4 * 4), -1, dtype=torch.int32, device="cuda")
+    rm[:, :kv] = table
+    f = torch.cat([x.double(), x.new_zeros(1, r).double()])[table.long()]  # [rows, kv, r], absent rows zero (index -1)
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # one fp32 rounding a product and sum, kv * r of them at most
+    bound = 2.0 ** -24 * (kv * r + 4)
+
+    def near(got, want, size):
+        assert ((got.double() - want).abs() <= bound * (size + 1)).all()
+
+    out = torch.full((rows, n), float("nan"), device="cuda")
+    assert lib.spc_conv_forward_residual(_p(x), _p(w), _p(bias), None, _p(rm), None, _p(out), n_in, rows, r, n, kv, _lib.SPC_F32, _lib.SPC_F32,
+                                         _lib.SPC_PREC_IEEE, 0, None, None, 1, 0.0, _p(residual), stream) == 0
+    want = torch.einsum("akr,nkr->an", f, w.double())
+    near(out, torch.relu(want + bias) + residual, torch.einsum("akr,nkr->an", f.abs(), w.double().abs()) + bias.abs() + residual.abs())
+    back = w.permute(2, 1, 0).contiguous()  # [r, kv, n] of a layer n -> r
+    for reverse in (0, 1):
+        din = torch.full((rows, n), float("nan"), device="cuda")
+        assert lib.spc_conv_backward_input_tables(_p(x), _p(back), None, _p(rm), None, _p(din), rows, n_in, n, r, kv, reverse, _lib.SPC_F32,
+                                                  _lib.SPC_PREC_IEEE, 0, stream) == 0
+        m = back.flip(1) if reverse else back
+        near(din, torch.einsum("akr,rkn->an", f, m.double()), torch.einsum("akr,rkn->an", f.abs(), m.double().abs()))
+
+
+@pytest.mark.parametrize("tf32", [False, True])
+def test_layers_that_share_the_rulebook(tf32, monkeypatch):
+    """A small layer builds it without a row order; a wide one and a 16-bit one use it after."""
+    monkeypatch.setattr(constants, "SPCONV_ALLOW_TF32", tf32)
+    gen = torch.Generator().manual_seed(3)
+    cells = torch.randperm(24 ** 3, generator=gen)[:1500]
+    idx = torch.stack([torch.zeros_like(cells), cells // 576, cells // 24 % 24, cells % 24], 1).int().cuda()
+    x = torch.randn(1500, 16, generator=gen).cuda()
+    small, wide = sp.SubMConv3d(16, 16, 3, indice_key="a").cuda(), sp.SubMConv3d(16, 128, 3, indice_key="a").cuda()
+    t = small(sp.SparseConvTensor(x, idx, [24] * 3, 1))
+    dense = torch.zeros(1, 16, 24, 24, 24, dtype=torch.float64, device="cuda")
+    at = idx.long()
+    for layer, bound in ((small, 2e-3 if tf32 else 1e-5), (wide, 2e-3 if tf32 else 1e-5)):
+        y = layer(t.replace_feature(x)).features.double()
+        dense[0, :, at[:, 1], at[:, 2], at[:, 3]] = x.double().t()
+        z = torch.nn.functional.conv3d(dense, layer.weight.double().permute(0, 4, 1, 2, 3), layer.bias.double(), padding=1)
+        z = z[0, :, at[:, 1], at[:, 2], at[:, 3]].t()
+        assert (y - z).norm() <= bound * z.norm()
+    with torch.autocast("cuda", dtype=torch.float16):
+        half = small(t.replace_feature(x)).features
+    assert half.dtype == torch.float16
