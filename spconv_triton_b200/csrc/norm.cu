@@ -7,7 +7,7 @@
 // activation saw are made again from x.
 //
 // torch runs the two modules as three kernels forward and three backward.  The thirteen pairs of a UNet training step (two indoor
-// scans of 120 000 voxels, fp16, SiLU): forward 1.68 -> 0.50 ms, backward 1.59 -> 1.09 ms.
+// scans of 120 000 voxels, fp16, SiLU): forward 1.68 -> 0.45 ms, backward 1.59 -> 0.69 ms.
 //
 // Statistics: a thread takes four rows at a time to their mean and squared deviations and merges these into its running
 // pair, threads, chunks and the final value are merged the same way (Chan, Golub, LeVeque: "Updating formulae and a
@@ -21,7 +21,8 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kAhead = 4;        // rows of a thread in flight
-constexpr int kMostChunks = 592; // four CTAs a multiprocessor: partial results stay few enough to merge in one launch
+constexpr int kCtas = 4;         // CTAs a multiprocessor, all of them at once: a chunk each, few enough to merge in one launch
+constexpr int kMostChunks = kCtas * 148;
 
 template <typename T> struct Vec {
   static constexpr int N = 16 / sizeof(T);
@@ -82,7 +83,7 @@ __device__ __forceinline__ void merge(Moments& a, float n, float mean, float m2)
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, kCtas)
 moments_kernel(const T* __restrict__ x, long long rows, int cols, long long chunk, float2* __restrict__ partial) {
   constexpr int N = Vec<T>::N;
   extern __shared__ float2 shared2[];  // [lanes][width * N]
@@ -141,36 +142,63 @@ moments_kernel(const T* __restrict__ x, long long rows, int cols, long long chun
   }
 }
 
-__device__ __forceinline__ double warp_sum(double v) {
+// The finishing kernels: eight channels a CTA (64 bytes of a chunk's results), 32 threads a channel that hold the results of
+// all their chunks at once, so that each kernel waits for memory once (a warp a channel, four loads ahead: 8 and 5 us).
+constexpr int kFinishChannels = 8, kFinishLanes = kThreads / kFinishChannels;
+constexpr int kHeld = (kMostChunks + kFinishLanes - 1) / kFinishLanes;
+struct Held {
+  float2 v[kHeld];
+};
+__device__ __forceinline__ Held held_chunks(const float2* partial, int chunks, int cols, int c, int first) {
+  Held h;
 #pragma unroll
-  for (int s = 16; s > 0; s >>= 1) v += __shfl_xor_sync(0xffffffffu, v, s);
-  return v;
+  for (int i = 0; i < kHeld; ++i) {
+    const int at = first + i * kFinishLanes;
+    h.v[i] = at < chunks && c < cols ? __ldg(&partial[static_cast<long long>(at) * cols + c]) : make_float2(0.f, 0.f);
+  }
+  return h;
+}
+// Sum over the threads of a channel, for each of them.
+__device__ __forceinline__ double channel_sum(double v) {
+  __shared__ double sums[kThreads / 32][kFinishChannels];
+  v += __shfl_xor_sync(0xffffffffu, v, 8);
+  v += __shfl_xor_sync(0xffffffffu, v, 16);
+  const int channel = threadIdx.x % kFinishChannels;
+  __syncthreads();
+  if ((threadIdx.x & 31) < kFinishChannels) sums[threadIdx.x >> 5][channel] = v;
+  __syncthreads();
+  double all = 0.;
+#pragma unroll
+  for (int w = 0; w < kThreads / 32; ++w) all += sums[w][channel];
+  return all;
 }
 
-// One warp a channel: the mean of the chunks' means, then their squared deviations and those of their means from it, in
-// fp64 (merged pair by pair, a division each, it took 13 us instead of 4); kept in fp32 as the user's running ones are.
+// The mean of the chunks' means, then their squared deviations and those of their means from it, in fp64; kept in fp32 as
+// the user's running ones are.
 __global__ void __launch_bounds__(kThreads)
 finish_moments_kernel(const float2* __restrict__ partial, int chunks, long long chunk, long long rows, int cols, float eps, float momentum,
                       float* __restrict__ save_mean, float* __restrict__ save_invstd, float* __restrict__ running_mean,
                       float* __restrict__ running_var, long long* __restrict__ batches) {
-  const int c = (blockIdx.x * kThreads + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  const int c = blockIdx.x * kFinishChannels + threadIdx.x % kFinishChannels, lane = threadIdx.x / kFinishChannels;
   if (blockIdx.x == 0 && threadIdx.x == 0 && batches != nullptr) *batches += 1;
-  if (c >= cols) return;
+  const Held h = held_chunks(partial, chunks, cols, c, lane);
   const double n = static_cast<double>(rows);
-  const auto size = [&](int i) { return static_cast<double>(min(chunk, rows - i * chunk)); };
+  const auto size = [&](int i) {
+    const int at = lane + i * kFinishLanes;
+    return at < chunks ? static_cast<double>(min(chunk, rows - at * chunk)) : 0.;
+  };
   double sum = 0.;
-#pragma unroll 4
-  for (int i = lane; i < chunks; i += 32) sum += size(i) * __ldg(&partial[static_cast<long long>(i) * cols + c].x);
-  const double mean = warp_sum(sum) / n;
+#pragma unroll
+  for (int i = 0; i < kHeld; ++i) sum += size(i) * h.v[i].x;
+  const double mean = channel_sum(sum) / n;
   double m2 = 0.;
-#pragma unroll 4
-  for (int i = lane; i < chunks; i += 32) {
-    const float2 b = __ldg(&partial[static_cast<long long>(i) * cols + c]);
-    const double d = b.x - mean;
-    m2 += b.y + size(i) * d * d;
+#pragma unroll
+  for (int i = 0; i < kHeld; ++i) {
+    const double d = h.v[i].x - mean;
+    m2 += h.v[i].y + size(i) * d * d;
   }
-  m2 = warp_sum(m2);
-  if (lane != 0) return;
+  m2 = channel_sum(m2);
+  if (lane != 0 || c >= cols) return;
   const double var = m2 / n;
   save_mean[c] = static_cast<float>(mean);
   save_invstd[c] = static_cast<float>(1. / sqrt(var + static_cast<double>(eps)));
@@ -197,7 +225,7 @@ __device__ __forceinline__ Channel<N> channel(const float* mean, const float* in
 }
 
 template <typename T, int ACT>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, kCtas)
 normalize_kernel(const T* __restrict__ x, const float* __restrict__ mean, const float* __restrict__ invstd, const float* __restrict__ weight,
                  const float* __restrict__ bias, long long rows, int cols, long long chunk, T* __restrict__ y) {
   constexpr int N = Vec<T>::N;
@@ -225,7 +253,7 @@ normalize_kernel(const T* __restrict__ x, const float* __restrict__ mean, const 
 
 // Per chunk and channel: sum of dz and of dz (x - mean), dz the gradient at the normalisation's output.
 template <typename T, int ACT>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, kCtas)
 gradient_sums_kernel(const T* __restrict__ x, const T* __restrict__ dy, const float* __restrict__ mean, const float* __restrict__ invstd,
                      const float* __restrict__ weight, const float* __restrict__ bias, long long rows, int cols, long long chunk,
                      float2* __restrict__ partial) {
@@ -280,18 +308,17 @@ gradient_sums_kernel(const T* __restrict__ x, const T* __restrict__ dy, const fl
 __global__ void __launch_bounds__(kThreads)
 finish_sums_kernel(const float2* __restrict__ partial, int chunks, long long rows, int cols, const float* __restrict__ invstd,
                    float* __restrict__ dweight, float* __restrict__ dbias, float2* __restrict__ means) {
-  const int c = (blockIdx.x * kThreads + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (c >= cols) return;
+  const int c = blockIdx.x * kFinishChannels + threadIdx.x % kFinishChannels, lane = threadIdx.x / kFinishChannels;
+  const Held h = held_chunks(partial, chunks, cols, c, lane);
   double a = 0., b = 0.;
-#pragma unroll 4
-  for (int i = lane; i < chunks; i += 32) {
-    const float2 q = __ldg(&partial[static_cast<long long>(i) * cols + c]);
-    a += q.x;
-    b += q.y;
+#pragma unroll
+  for (int i = 0; i < kHeld; ++i) {
+    a += h.v[i].x;
+    b += h.v[i].y;
   }
-  a = warp_sum(a);
-  b = warp_sum(b);
-  if (lane != 0) return;
+  a = channel_sum(a);
+  b = channel_sum(b);
+  if (lane != 0 || c >= cols) return;
   const double inv = invstd[c];
   if (dweight != nullptr) dweight[c] = static_cast<float>(b * inv);
   if (dbias != nullptr) dbias[c] = static_cast<float>(a);
@@ -299,7 +326,7 @@ finish_sums_kernel(const float2* __restrict__ partial, int chunks, long long row
 }
 
 template <typename T, int ACT>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, kCtas)
 input_gradient_kernel(const T* __restrict__ x, const T* __restrict__ dy, const float* __restrict__ mean, const float* __restrict__ invstd,
                       const float* __restrict__ weight, const float* __restrict__ bias, const float2* __restrict__ means, long long rows,
                       int cols, long long chunk, T* __restrict__ dx) {
@@ -376,7 +403,7 @@ int forward(const void* x, const float* weight, const float* bias, float* runnin
   const dim3 grid(p.chunks, p.across);
   moments_kernel<T><<<grid, kThreads, p.shared, st>>>(static_cast<const T*>(x), rows, cols, p.chunk, partial);
   SPC_LAUNCH_OK();
-  finish_moments_kernel<<<static_cast<unsigned>(ceil_div(cols, kThreads / 32)), kThreads, 0, st>>>(
+  finish_moments_kernel<<<static_cast<unsigned>(ceil_div(cols, kFinishChannels)), kThreads, 0, st>>>(
       partial, p.chunks, p.chunk, rows, cols, eps, momentum, save_mean, save_invstd, running_mean, running_var, batches);
   SPC_LAUNCH_OK();
   normalize_kernel<T, ACT><<<grid, kThreads, 0, st>>>(static_cast<const T*>(x), save_mean, save_invstd, weight, bias, rows, cols, p.chunk,
@@ -395,7 +422,7 @@ int backward(const void* x, const void* dy, const float* weight, const float* bi
   gradient_sums_kernel<T, ACT><<<grid, kThreads, p.shared, st>>>(static_cast<const T*>(x), static_cast<const T*>(dy), save_mean, save_invstd,
                                                                  weight, bias, rows, cols, p.chunk, partial);
   SPC_LAUNCH_OK();
-  finish_sums_kernel<<<static_cast<unsigned>(ceil_div(cols, kThreads / 32)), kThreads, 0, st>>>(partial, p.chunks, rows, cols, save_invstd,
+  finish_sums_kernel<<<static_cast<unsigned>(ceil_div(cols, kFinishChannels)), kThreads, 0, st>>>(partial, p.chunks, rows, cols, save_invstd,
                                                                                                dweight, dbias, means);
   SPC_LAUNCH_OK();
   if (dx == nullptr) return SPC_OK;
