@@ -6,7 +6,7 @@
 // four shared-memory wavefronts.  The tile's rows come in an order that groups rows with common offsets, a
 // warp skips the offsets that none of its 16 rows has, and the next stage's operands are in flight during the
 // multiplications.  SubM 64 -> 64, 100 k rows, 6.2 of 27 neighbours: forward 104 us, input gradient 97, weight
-// gradient 123 (49 - 51, 48 % of the issue slots; 128 registers, four CTAs a multiprocessor).  With 4 x 4 outputs a
+// gradient 75 (49 - 51 % of the issue slots in the first two; 128 registers, four CTAs a multiprocessor).  With 4 x 4 outputs a
 // thread, scalar shared-memory reads and a barrier twice every 16 channels: 425, 425 (240 with sorted rows), 727.
 #include <algorithm>
 
@@ -249,7 +249,9 @@ wgrad_f32_kernel(const float* __restrict__ feats, const float* __restrict__ gout
   __shared__ int warp_cnt[kListRows / 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int tx = tid & 15, ty = tid >> 4;
-  const int k = blockIdx.x / splits, split = blockIdx.x % splits;
+  // the middle offsets first: they have the most pairs
+  const int turn = blockIdx.x / splits, split = blockIdx.x % splits;
+  const int k = (turn & 1) ? (kv - 1) / 2 + (turn + 1) / 2 : (kv - 1) / 2 - turn / 2;
   const int c0 = blockIdx.y * kTile, n0 = blockIdx.z * kTile;
   const long long lo = split * rows_per_split, hi = min(n_out, lo + rows_per_split);
   const int32_t* col = pair_fwd + static_cast<long long>(k) * n_out;
@@ -459,8 +461,10 @@ bool wgrad_f32_supported(int c_in, int c_out, int dtype) { return dtype == SPC_F
 WgradSplit wgrad_f32_split(int64_t n_out, int c_in, int c_out, int kv) {
   WgradSplit s;
   const int64_t tiles = static_cast<int64_t>(kv) * ceil_div(c_in, kTile) * ceil_div(c_out, kTile);
-  int64_t want = ceil_div(8 * static_cast<int64_t>(sm_count()), std::max<int64_t>(tiles, 1));
-  want = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(want, n_out / 2048), 64));
+  // The centre offset of a submanifold layer has a pair a row and is the longest chain: splits short enough that one is not
+  // longer than the rest of the work (SubM 64 -> 64, 100 k rows: 44 splits in offset order 136 us, 64 and the middle first 75).
+  int64_t want = ceil_div(16 * static_cast<int64_t>(sm_count()), std::max<int64_t>(tiles, 1));
+  want = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(want, n_out / 1024), 64));
   s.splits = static_cast<int>(want);
   s.rows_per_split = ceil_div(std::max<int64_t>(n_out, 1), s.splits);
   s.bytes = static_cast<size_t>(s.splits) * c_out * kv * c_in * sizeof(float);
