@@ -57,21 +57,25 @@ column_sums_kernel(const T* __restrict__ x, long long rows, int cols, long long 
   }
 }
 
-// out[c] = sum of partial[chunk, c]; 32 columns a CTA, eight chunk lanes.
+// out[c] = sum of partial[chunk, c]; 32 columns a CTA, 32 chunk lanes with eight loads under way each (eight lanes, four
+// loads: 14.6 us for 1184 chunks of 128 columns, all of it waiting).
+constexpr int kAddLanes = 32;
 template <typename TO>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(32 * kAddLanes)
 add_chunks_kernel(const float* __restrict__ partial, int chunks, int cols, TO* __restrict__ out) {
-  __shared__ float s[8][32];
+  __shared__ float s[kAddLanes][32];
   const int c = blockIdx.x * 32 + (threadIdx.x & 31), lane = threadIdx.x >> 5;
   float sum = 0.f;
-  if (c < cols)
-    for (int i = lane; i < chunks; i += 8) sum += partial[static_cast<long long>(i) * cols + c];
+  if (c < cols) {
+#pragma unroll 8
+    for (int i = lane; i < chunks; i += kAddLanes) sum += __ldg(&partial[static_cast<long long>(i) * cols + c]);
+  }
   s[lane][threadIdx.x & 31] = sum;
   __syncthreads();
   if (lane == 0 && c < cols) {
     float all = 0.f;
 #pragma unroll
-    for (int l = 0; l < 8; ++l) all += s[l][threadIdx.x & 31];
+    for (int l = 0; l < kAddLanes; ++l) all += s[l][threadIdx.x & 31];
     out[c] = from_float<TO>(all);
   }
 }
@@ -96,9 +100,9 @@ int column_sums(const void* x, int64_t rows, int cols, void* out, int out_dtype,
   SPC_LAUNCH_OK();
   const unsigned blocks = static_cast<unsigned>(ceil_div(cols, 32));
   switch (out_dtype) {
-    case SPC_F16: add_chunks_kernel<<<blocks, kThreads, 0, st>>>(partial, chunks, cols, static_cast<__half*>(out)); break;
-    case SPC_BF16: add_chunks_kernel<<<blocks, kThreads, 0, st>>>(partial, chunks, cols, static_cast<__nv_bfloat16*>(out)); break;
-    case SPC_F32: add_chunks_kernel<<<blocks, kThreads, 0, st>>>(partial, chunks, cols, static_cast<float*>(out)); break;
+    case SPC_F16: add_chunks_kernel<<<blocks, 32 * kAddLanes, 0, st>>>(partial, chunks, cols, static_cast<__half*>(out)); break;
+    case SPC_BF16: add_chunks_kernel<<<blocks, 32 * kAddLanes, 0, st>>>(partial, chunks, cols, static_cast<__nv_bfloat16*>(out)); break;
+    case SPC_F32: add_chunks_kernel<<<blocks, 32 * kAddLanes, 0, st>>>(partial, chunks, cols, static_cast<float*>(out)); break;
     default: return fail(SPC_ERR_UNSUPPORTED, "column_sums: dtype %d not supported", out_dtype);
   }
   SPC_LAUNCH_OK();
