@@ -335,6 +335,8 @@ choose_sorted_kernel(const uint32_t* __restrict__ keys, const int* __restrict__ 
 
 // Rows of the voxel buffer and of the caller's copies (`out` .. `num_out`, may be null).  With `clear`: every
 // element of every row, zeros where there is no point; without: only the stored points.
+// Four elements a thread, their counts and point numbers on their way together: a pass of three dependent loads an element.
+constexpr int kEmitEach = 4;
 template <int VEC, typename Index>
 __global__ void __launch_bounds__(kVoxThreads)
 emit_voxels_kernel(const float* __restrict__ points, int point_stride, int num_features, const int* __restrict__ chosen,
@@ -342,25 +344,38 @@ emit_voxels_kernel(const float* __restrict__ points, int point_stride, int num_f
                    int max_points, int clear, float* __restrict__ voxels, float* __restrict__ out, int32_t* __restrict__ indices_out,
                    int32_t* __restrict__ num_out) {
   struct alignas(4 * VEC) Pack { float v[VEC]; };
-  const Index per = static_cast<Index>(num_features / VEC);
-  const Index e = static_cast<Index>(blockIdx.x) * kVoxThreads + threadIdx.x;
-  const Index ps = e / per;  // (voxel, slot)
-  if (ps >= rows * static_cast<Index>(max_points)) return;
-  const int c = static_cast<int>(e - ps * per) * VEC;
-  const Index v = ps / static_cast<Index>(max_points);
-  const int slot = static_cast<int>(ps - v * static_cast<Index>(max_points));
-  Pack x;
+  const Index per = static_cast<Index>(num_features / VEC), all = rows * static_cast<Index>(max_points) * per;
+  const Index first = static_cast<Index>(blockIdx.x) * (kVoxThreads * kEmitEach) + threadIdx.x;
+  Index at[kEmitEach];   // of the element's first float
+  int stored[kEmitEach], from[kEmitEach];
 #pragma unroll
-  for (int q = 0; q < VEC; ++q) x.v[q] = 0.f;
-  const int stored = v < num_voxels ? num_per_voxel[v] : 0;
-  if (slot < stored) x = *reinterpret_cast<const Pack*>(points + static_cast<long long>(chosen[ps]) * point_stride + c);
-  const long long at = static_cast<long long>(ps) * num_features + c;
-  if (slot < stored || clear) *reinterpret_cast<Pack*>(voxels + at) = x;
-  if (out == nullptr || v >= num_voxels) return;
-  *reinterpret_cast<Pack*>(out + at) = x;
-  if (slot == 0 && c == 0) {
-    num_out[v] = stored;
-    for (int d = 0; d < ndim; ++d) indices_out[static_cast<long long>(v) * ndim + d] = indices[static_cast<long long>(v) * ndim + d];
+  for (int i = 0; i < kEmitEach; ++i) {
+    const Index e = first + static_cast<Index>(i * kVoxThreads), ps = e / per;  // (voxel, slot)
+    at[i] = e;
+    stored[i] = from[i] = 0;
+    if (e < all && ps < num_voxels * static_cast<Index>(max_points)) {
+      stored[i] = num_per_voxel[ps / static_cast<Index>(max_points)];
+      from[i] = chosen[ps];  // (read beside the count; of no meaning from the count on)
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < kEmitEach; ++i) {
+    const Index e = at[i];
+    if (e >= all) break;
+    const Index ps = e / per, v = ps / static_cast<Index>(max_points);
+    const int c = static_cast<int>(e - ps * per) * VEC, slot = static_cast<int>(ps - v * static_cast<Index>(max_points));
+    Pack x;
+#pragma unroll
+    for (int q = 0; q < VEC; ++q) x.v[q] = 0.f;
+    if (slot < stored[i]) x = *reinterpret_cast<const Pack*>(points + static_cast<long long>(from[i]) * point_stride + c);
+    const long long to = static_cast<long long>(e) * VEC;
+    if (slot < stored[i] || clear) *reinterpret_cast<Pack*>(voxels + to) = x;
+    if (out == nullptr || v >= num_voxels) continue;
+    *reinterpret_cast<Pack*>(out + to) = x;
+    if (slot == 0 && c == 0) {
+      num_out[v] = stored[i];
+      for (int d = 0; d < ndim; ++d) indices_out[static_cast<long long>(v) * ndim + d] = indices[static_cast<long long>(v) * ndim + d];
+    }
   }
 }
 
@@ -574,7 +589,7 @@ extern "C" int spc_voxelize_store(const float* points, int64_t n_points, int poi
     const bool small = work < (1ll << 31);
     const auto emit = [&](auto kernel, auto index) {
       using Index = decltype(index);
-      kernel<<<vox_blocks(work), kVoxThreads, 0, st>>>(points, point_stride, num_features, chosen, num_per_voxel, indices, ndim,
+      kernel<<<vox_blocks(ceil_div(work, kEmitEach)), kVoxThreads, 0, st>>>(points, point_stride, num_features, chosen, num_per_voxel, indices, ndim,
                                                       static_cast<Index>(num_voxels), static_cast<Index>(rows), max_points, clear_voxels, voxels,
                                                       voxels_out, indices_out, num_out);
     };
