@@ -509,15 +509,13 @@ int launch(const StreamParams& p, int a_row_bytes, const CUtensorMap& map_b, int
 // 193 k 31 / 35, 373 k 51 / 48; 32 -> 64 with 4, 269 k 41 / 43, 523 k 70 / 61.
 bool gather_gemm_stream_takes(int n_dim, int r_dim, long long m_rows, int dtype) {
   if (dtype != SPC_F16 && dtype != SPC_BF16) return false;
-  if (r_dim * 2 != row_span(r_dim, 2) || n_dim > 128) return false;
+  if (r_dim * 2 != row_span(r_dim, 2) || n_dim > 128 || m_rows >= (1ll << 31) - kTileM) return false;
   return ceil_div(m_rows, kTileM) >= (n_dim > 64 ? 8ll : 20ll) * sm_count();
 }
 
 int gather_gemm_stream(const void* src, const void* w, const Epilogue& epi, const int32_t* pairs, const int32_t* pairs_rowmajor,
                        const int32_t* order, void* out, long long m_rows, int n_dim, int r_dim, int kv, bool transposed_weight,
                        bool reversed, int dtype, int out_dtype, cudaStream_t st) {
-  if (m_rows >= (1ll << 31) - kTileM)
-    return fail(SPC_ERR_SIZE_LIMIT, "TMA gather-GEMM: %lld rows", static_cast<long long>(m_rows));
   StreamParams p{};
   p.src = src; p.epi = epi; p.pairs = pairs; p.pairs_rm = pairs_rowmajor; p.kvp = (kv + 3) & ~3; p.order = order; p.out = out;
   p.m_rows = static_cast<int>(m_rows);

@@ -10,8 +10,8 @@
 // c_in fp32 columns a block) in tensor memory; with 256 output channels both
 // blocks multiply the same feature rows, which two CTAs would gather twice.
 // Bound by the gathered rows on narrow layers (64 -> 128, 1.6 M pairs of a 27 x 1.36 M
-// table: 222 us, 631 MB read, a quarter of it the table; the tensor pipe at 5 %).  k5
-// 256 -> 256, 13.6 M pairs: 5.5 ms with a block a CTA, 2.53 now (704 TFLOP/s, 0.44 of
+// table: 188 us, 631 MB read, a quarter of it the table; the tensor pipe at 5 %).  k5
+// 256 -> 256, 13.6 M pairs: 5.5 ms with a block a CTA, 2.35 now (760 TFLOP/s, 0.46 of
 // the measured peak).
 // W (four or eight) copy warps and one that multiplies:
 //   warps 0 .. W-1  scan pair_fwd[k, lo:hi] 1024 entries a round, compact the
