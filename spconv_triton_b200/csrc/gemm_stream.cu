@@ -128,7 +128,8 @@ gather_gemm_stream_kernel(const __grid_constant__ StreamParams p, const __grid_c
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
-  if (*reinterpret_cast<volatile int*>(p.status) != 0) return;
+  // (one thread's reading, acted on by the whole CTA below: threads that saw different values must not part)
+  const int stopped = tid == 32 ? *reinterpret_cast<volatile int*>(p.status) : 0;
   const uint32_t bar0 = smem_u32(bars);
   const auto bar = [bar0](int i) { return bar0 + 8u * i; };
 
@@ -156,9 +157,13 @@ gather_gemm_stream_kernel(const __grid_constant__ StreamParams p, const __grid_c
   const bool has_epilogue = p.epi.bias != nullptr || p.epi.shift != nullptr || p.epi.act != SPC_ACT_NONE;
   if (has_epilogue) stage_epilogue<T>(p.epi, p.n_dim, epi_scale, epi_shift, tid, kThreads);
   tc_fence_before();
-  __syncthreads();
+  const int stop = __syncthreads_or(stopped);
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (stop != 0) {
+    if (warp == kMmaWarp) tmem_dealloc(tmem_base, static_cast<uint32_t>(p.tmem_cols));
+    return;
+  }
   const uint32_t stage0 = smem_u32(smem);
   // tiles are taken from the END of the mask-sorted order first: those rows have the most kernel offsets, and starting
   // the long tiles first leaves the short ones to fill the tail

@@ -130,7 +130,8 @@ wgrad_tc_kernel(const __grid_constant__ WgParams p) {
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
-  if (*reinterpret_cast<volatile int*>(p.status) != 0) return;
+  // (one thread's reading, acted on by the whole CTA below: threads that saw different values must not part)
+  const int stopped = tid == 32 ? *reinterpret_cast<volatile int*>(p.status) : 0;
   // The middle offsets first: the centre of a submanifold kernel has every row, its neighbours most of them,
   // and a CTA of theirs started last would run on alone.
   const int turn = blockIdx.x / p.splits, split = blockIdx.x % p.splits;
@@ -155,9 +156,13 @@ wgrad_tc_kernel(const __grid_constant__ WgParams p) {
     tmem_relinquish();
   }
   tc_fence_before();
-  __syncthreads();
+  const int stop = __syncthreads_or(stopped);
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (stop != 0) {
+    if (warp == kWgMmaWarp) tmem_dealloc(tmem_base, static_cast<uint32_t>(p.tmem_cols));
+    return;
+  }
 
   int real_stages = 0;
   if (warp < kWgIssueWarps) {
