@@ -141,3 +141,18 @@ def test_the_combined_call_equals_its_two_halves(clear, mean):
     for got, want in zip((voxels, indices, num), exp):
         assert torch.equal(got[:found.value], want)
     assert torch.equal(ids, exp[3])
+
+
+@pytest.mark.parametrize("features", [3, 4])
+@pytest.mark.parametrize("beyond", [0, 1])
+def test_cap_either_side_of_one_element_a_thread(features, beyond):
+    """The cap sets the elements that are written: up to 6144 a multiprocessor a thread has one, beyond it four."""
+    slots = 5
+    each = slots * (1 if features == 4 else features)
+    limit = 6144 * torch.cuda.get_device_properties(0).multi_processor_count // each
+    pts = torch.rand(3001, features, generator=torch.Generator().manual_seed(features)) * 12
+    ctor = dict(vsize_xyz=[1.0] * 3, coors_range_xyz=[0.0, 0.0, 0.0, 10.0, 10.0, 10.0], num_point_features=features,
+                max_num_voxels=limit + beyond, max_num_points_per_voxel=slots)
+    out = P2V(**ctor).generate_voxel_with_id(pts.to(DEV))
+    exp = point_to_voxel(pts.numpy(), **ctor)
+    check(out, dict(voxels=exp[0], indices=exp[1], num_per_voxel=exp[2], pc_voxel_id=exp[3]))
