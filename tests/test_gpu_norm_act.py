@@ -80,6 +80,61 @@ def test_no_worse_than_the_modules():
     assert own.norm() <= 1.05 * apart.norm()
 
 
+@pytest.mark.parametrize("act", list(ACTS))
+@pytest.mark.parametrize("dtype,rows,channels", [(torch.float16, 4099, 32), (torch.float16, 60000, 64), (torch.bfloat16, 4099, 32),
+                                                 (torch.bfloat16, 60000, 64), (torch.float32, 4099, 32), (torch.float32, 60000, 64)])
+def test_no_output_is_further_from_fp64_than_the_modules(act, dtype, rows, channels):
+    """Result, input gradient and both parameters' gradients, in every type and with every activation."""
+    g = torch.Generator("cuda").manual_seed(rows + channels)
+    x = (0.5 + torch.randn(rows, channels, generator=g, device="cuda") * (0.5 + torch.rand(channels, generator=g, device="cuda"))).to(dtype)
+    dy = torch.randn(rows, channels, generator=g, device="cuda").to(dtype)
+    net = _net(channels, act)
+
+    def outputs(run, net, x, dy):
+        f = x.clone().requires_grad_()
+        y = run(net, f)
+        y.backward(dy)
+        return [t.double() for t in (y.detach(), f.grad, net[0].weight.grad, net[0].bias.grad)]
+
+    exact = outputs(lambda n, f: _apart(n, _tensor(f)), copy.deepcopy(net).double(), x.double(), dy.double())
+    own = outputs(lambda n, f: n(_tensor(f)).features, copy.deepcopy(net), x, dy)
+    apart = outputs(lambda n, f: _apart(n, _tensor(f)), copy.deepcopy(net), x, dy)
+    for what, a, b, e in zip(("y", "dx", "dweight", "dbias"), own, apart, exact):
+        # (both sides round y and dx once to the features' type at least: equal but for the values' luck.  The parameters'
+        # gradients are fp32 sums; without an activation those of dy alone, of which both sides see all but the last bits)
+        slack = 2.0 ** -24 * 4 * e.norm() if what.startswith("d") else 0.0
+        assert (a - e).norm() <= 1.05 * (b - e).norm() + slack, what
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+def test_silu_far_from_zero(dtype):
+    """Each value, and the parameters' gradients of rows whose activation is all but flat, where exp(-z) is large."""
+    lim = 15.0 if dtype == torch.float16 else 88.0  # below, results of that type are none
+    n = 4096
+    x = torch.linspace(-1, 1, n, device="cuda", dtype=torch.float64)[torch.randperm(n, generator=torch.Generator().manual_seed(1)).cuda()]
+    x = x[:, None].expand(n, 8).contiguous().to(dtype)
+    net = _net(8, "silu")
+    net[0].weight.data.fill_(lim / 3 ** 0.5)  # (a uniform variable's largest value is 3 ** 0.5 deviations)
+    net[0].bias.data.zero_()
+    f = x.clone().requires_grad_()
+    y = net(_tensor(f)).features
+    d = x.double().requires_grad_()
+    wide = copy.deepcopy(net).double()
+    z = wide[0](d)
+    e = nn.functional.silu(z)
+    low = (z < -0.8 * lim).float()
+    y.backward(low.to(dtype))
+    e.backward(low.double())
+    # one rounding of the result, a few of exp and the division; z is off by a few roundings of itself and by the mean's error
+    # (2^-24 of values up to 1, twice) times the gain, and the activation's slope takes that on
+    s, dz = torch.sigmoid(z), 2.0 ** -24 * (8 * z.abs() + 2 * lim)
+    bound = (EPS[dtype] + 2.0 ** -24 * 8) * e.abs() + dz * (s * (1 + z * (1 - s))).abs() + dz ** 2 * s
+    tiny = 2.0 ** -24 if dtype == torch.float16 else torch.finfo(dtype).tiny
+    assert ((y.double() - e).abs() <= bound + tiny).all()
+    for a, b in zip(net.parameters(), wide.parameters()):
+        assert (a.grad.double() - b.grad).abs().max() <= 2.0 ** -24 * 16 * (1 + lim) * b.grad.abs().max()  # (s is off by dz of itself)
+
+
 def test_without_affine_and_non_finite():
     net = _net(16, "relu", affine=False)
     x = torch.randn(100, 16, device="cuda")
