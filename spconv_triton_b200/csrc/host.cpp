@@ -115,6 +115,7 @@ struct Rulebook {
   };
   Side fwd, bwd;
   Late late_fwd, late_bwd;
+  bool captured = false;  // by a graph, whose replays read the tables and what it makes tables from
   mutable std::mutex lock;
 
   bool subm() const { return geo->subm; }
@@ -135,16 +136,17 @@ struct Rulebook {
   // The side whose rows are the output rows (of the layer, or of its inverse with `input`).
   Side side(bool input, bool colmajor) {
     if (input && subm()) throw Failure(SPC_ERR_INVALID_ARGUMENT, "a submanifold rulebook has one side");
+    c10::cuda::CUDAGuard guard(indices.device());
+    // A capture records its kernels and does not run them: it waits for nothing (what came before a capture is
+    // done when the graph runs), and tables that it makes are its own.
+    const bool capturing = c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
     std::lock_guard<std::mutex> hold(lock);
+    captured = captured || capturing;
     Side& kept = input ? bwd : fwd;
     Late& late = input ? late_bwd : late_fwd;
     const bool missing = !kept.rm.defined() || (colmajor && !kept.cm.defined());
     if (!missing && !late.stream) return kept;
-    c10::cuda::CUDAGuard guard(indices.device());
     const auto now = c10::cuda::getCurrentCUDAStream();
-    // A capture records its kernels and does not run them: it waits for nothing (what came before a capture is
-    // done when the graph runs), and tables that it makes are its own.
-    const bool capturing = c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
     Side s = kept;
     if (late.stream && *late.stream != now && !capturing) {
       late.made.block(now);
@@ -166,7 +168,7 @@ struct Rulebook {
     kept = s;
     late.made.record(now);
     late.stream = now;
-    if (bwd.rm.defined()) workspace = Tensor();  // nothing is made from it any more
+    if (bwd.rm.defined() && !captured) workspace = Tensor();  // nothing is made from it any more
     return s;
   }
   std::vector<Tensor> parts() const {
@@ -740,6 +742,7 @@ PYBIND11_MODULE(_host, m) {
       .def_readonly("geometry", &Rulebook::geo)
       .def_readonly("indices", &Rulebook::indices)
       .def_readonly("out_indices", &Rulebook::out_indices)
+      .def_readonly("captured", &Rulebook::captured)
       .def("rowmajor", [](Rulebook& r, bool input) { return r.side(input, false).rm; }, py::call_guard<py::gil_scoped_release>())
       .def("colmajor", [](Rulebook& r, bool input) { return r.side(input, true).cm; }, py::call_guard<py::gil_scoped_release>());
   m.def("build_rulebook", &build_rulebook);

@@ -160,7 +160,7 @@ class LateTables:
     def __init__(self, prepared, n_out, split_words, n_split, do_sort, mic):
         self.p, self.n_out, self.split_words, self.n_split = prepared, n_out, split_words, n_split
         self.do_sort, self.mic = do_sort, mic
-        self.value = None
+        self.value, self.captured = None, False
 
     def get(self):
         if self.value is None:
@@ -181,9 +181,11 @@ class LateTables:
                 pair_bwd._spc_rowmajor = bwd_rm
             value = (pair_bwd, [pm_bwd[s] for s in range(self.n_split)], [ma_bwd[s] for s in range(self.n_split)])
             if torch.cuda.is_current_stream_capturing():
+                self.captured = True
                 return value  # recorded, not made: it belongs to the graph
             self.value = value
-            self.p = None  # the workspace is no longer needed
+            if not self.captured:  # (a graph makes them again, from the workspace, at every replay)
+                self.p = None
         return self.value
 
 

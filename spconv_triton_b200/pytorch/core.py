@@ -56,6 +56,7 @@ class _Record:
     _fields: tuple = ()
     _assigned: frozenset = frozenset()  # tables that the user has put in the place of pending ones: they stay
     _ready: dict = {}  # of tables made on demand: (stream, event)
+    _captured: tuple = ()  # what graphs make tables from, or read them from, at every replay
 
     def _assign(self, values: dict):
         tables = type(self)._tables
@@ -64,8 +65,15 @@ class _Record:
     def __init_subclass__(cls):
         cls._tables = frozenset(name for name in cls._fields if isinstance(vars(cls).get(name), property))
 
+    def _keep_for_graphs(self, source):
+        if not any(source is s for s in self._captured):
+            self._captured += (source,)
+
     def _set(self, name, v):
         with _on_demand_lock:
+            rb = self.__dict__.get("_rb")
+            if rb is not None and rb.captured:
+                self._keep_for_graphs(rb)
             self.__dict__["_rb"] = None  # a table that the user assigns counts from then on, not the layer's rulebook
             self._assigned |= {name}
             self._ready = {k: e for k, e in self._ready.items() if k != name}
@@ -83,6 +91,7 @@ class _Record:
                     made = dict(zip(fields, make(source), strict=True))
                     on_device = [t for t in _tensors_of(list(made.values())) if t.is_cuda]
                     if on_device and torch.cuda.is_current_stream_capturing():
+                        self._keep_for_graphs(source)
                         return made[name] if name not in self._assigned else d[name]
                     if on_device:
                         stream = torch.cuda.current_stream(on_device[0].device)
@@ -106,7 +115,7 @@ class _Record:
     def __getstate__(self):
         for name in self._fields:
             getattr(self, name)
-        state = dict(self.__dict__, _ready={})
+        state = dict(self.__dict__, _ready={}, _captured=())
         for name in ("_rb", *self._on_demand):
             if name in state:
                 state[name] = None

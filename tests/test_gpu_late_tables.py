@@ -83,6 +83,50 @@ def test_tables_asked_for_under_capture():
     np.testing.assert_array_equal(to_np(inside[1]), bwd)
 
 
+def test_a_graph_keeps_what_it_makes_tables_from():
+    """... also when a later call has made them for good and other tensors have come and gone."""
+    rb, _, bwd = _book()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        inside = rb.colmajor(True)
+    assert rb.captured
+    np.testing.assert_array_equal(to_np(rb.colmajor(True)), bwd)
+    others = [torch.full((size,), 0x55, dtype=torch.uint8, device=DEV) for size in (1 << 16, 1 << 18, 1 << 20, 1 << 22) for _ in range(16)]
+    torch.cuda.synchronize()
+    for _ in range(2):
+        inside.fill_(-7)
+        graph.replay()
+        np.testing.assert_array_equal(to_np(inside), bwd)
+    assert all(bool((t == 0x55).all()) for t in others)
+
+
+def test_a_graph_keeps_what_a_pending_side_is_made_from():
+    """The same for the input side that an inference pass of the operator functions leaves pending."""
+    import spconv_triton_b200.pytorch as sp
+    from spconv_triton_b200.pytorch import ops
+    from spconv_triton_b200.pytorch._impl import pairs
+
+    idx = torch.from_numpy(unique_coords(11, N, 2, SHAPE)).to(DEV)
+    layer = sp.SparseConv3d(16, 16, 3, stride=2, padding=1, indice_key="d").to(DEV).half().eval()
+    with torch.no_grad(), pairs.deferred_backward("late"):
+        res = ops.get_indice_pairs_implicit_gemm(idx, 2, list(SHAPE), layer.algo, layer.kernel_size, layer.stride, layer.padding,
+                                                 layer.dilation, [0] * 3)
+    late = res[2]._spc_late
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        inside = late.get()[0]
+    want = late.get()[0].clone()
+    assert late.p is not None
+    others = [torch.full((size,), 0x55, dtype=torch.uint8, device=DEV) for size in (1 << 16, 1 << 18, 1 << 20, 1 << 22) for _ in range(16)]
+    torch.cuda.synchronize()
+    inside.fill_(-7)
+    graph.replay()
+    assert torch.equal(inside, want)
+    assert all(bool((t == 0x55).all()) for t in others)
+
+
 def test_scratch_goes_with_its_use():
     """The scratch of a rulebook goes once both sides are there."""
     rb, _, _ = _book()

@@ -5,6 +5,8 @@ import copy
 import pickle
 import threading
 import time
+import weakref
+from types import SimpleNamespace
 
 import numpy as np
 import torch
@@ -101,6 +103,40 @@ def test_a_container_that_has_run_can_be_copied():
         assert "_spc_plans" not in got.__dict__ and "_spc_arena_floor" not in got.__dict__
         assert torch.equal(got[0].weight, net[0].weight)
     assert net.__dict__["_spc_plans"]
+
+
+class _OnDevice(torch.Tensor):
+    is_cuda = True
+
+
+def test_what_a_graph_makes_tables_from_stays(monkeypatch):
+    """... also when a later call outside the capture has made them for good, and when the user has put others there."""
+    capturing = True
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: capturing)
+    stream = SimpleNamespace(record_event=lambda: None, device="cuda")
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device: stream)
+
+    class Late(_Late):
+        def get(self):
+            return torch.ones(2).as_subclass(_OnDevice), [], []
+
+    entry = _entry()
+    entry._late = Late()
+    late = weakref.ref(entry._late)
+    entry.pair_bwd, entry.pair_bwd  # (recorded twice, kept once)
+    capturing = False
+    entry.pair_bwd
+    assert entry._late is None and late() is not None and len(entry._captured) == 1
+    rb = SimpleNamespace(captured=True)
+    entry._rb = rb
+    entry.pair_mask_bwd_splits = []
+    assert entry._rb is None and entry._captured[-1] is rb
+    entry._rb = SimpleNamespace(captured=False)
+    entry.mask_argsort_bwd_splits = []
+    assert len(entry._captured) == 2
+    assert copy.copy(entry)._captured == ()
+    entry = None
+    assert late() is None
 
 
 def test_folded_statistics_follow_a_forward_in_training_mode():
