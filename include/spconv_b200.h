@@ -548,6 +548,19 @@ size_t spc_pool_row_order_workspace_bytes(int64_t n_rows);
 int spc_pool_row_order(const int32_t* table, int pitch, int kv, int64_t n_rows, int64_t n_targets, int32_t* order,
                        void* workspace, size_t workspace_bytes, void* stream);
 
+/* Evaluation-mode batch normalisations as out_scale / out_shift of spc_conv_forward:
+ * scale = weight / sqrt(var + eps), shift = bias - mean * scale, in fp32, all of them
+ * in one launch.  The statistics and parameters are fp16, bf16 or fp32 (`types`: an
+ * spc_dtype each, in the order mean, var, weight, bias); weight and bias may be NULL. */
+typedef struct {
+  const void *mean, *var, *weight, *bias;  /* [channels] */
+  float *scale, *shift;                    /* [channels], written */
+  int32_t types[4];
+  int32_t channels;
+  float eps;
+} spc_norm_fold;
+int spc_fold_norms(const spc_norm_fold* norms, int n, void* stream);
+
 /* ---- a chain of convolutions in one call --------------------------------- */
 
 /* One layer of spc_sequence_forward: a sparse convolution with kernel volume <= 32
@@ -605,6 +618,14 @@ int spc_sequence_forward(const spc_seq_layer* layers, int n_layers, const int32_
                          const void* features, int64_t n_in, int dtype, void* arena,
                          size_t arena_bytes, size_t* arena_needed, spc_seq_result* results,
                          void* stream_main, void* stream_chain, void* stream_side);
+/* The same after spc_fold_norms of `norms`, which writes what layers[i].scale and
+ * layers[i].shift point to: queued on `stream_main` behind the rulebook of the first
+ * layer, so that nothing waits for it but the GEMMs. */
+int spc_sequence_forward_norms(const spc_seq_layer* layers, int n_layers, const int32_t* indices,
+                               const void* features, int64_t n_in, int dtype, void* arena,
+                               size_t arena_bytes, size_t* arena_needed, spc_seq_result* results,
+                               void* stream_main, void* stream_chain, void* stream_side,
+                               const spc_norm_fold* norms, int n_norms);
 
 #ifdef __cplusplus
 }

@@ -70,6 +70,7 @@ _PROTOTYPES = {
     "spc_post_device_status": (c_int, [_P, _P]),
     "spc_tf32_prepare": (c_int, [_P, _P, c_int64, c_int, c_int, _P]),
     "spc_sequence_forward": (c_int, [_P, c_int, _P, _P, c_int64, c_int, _P, c_size_t, _P, _P, _P, _P, _P]),
+    "spc_sequence_forward_norms": (c_int, [_P, c_int, _P, _P, c_int64, c_int, _P, c_size_t, _P, _P, _P, _P, _P, _P, c_int]),
     "spc_tf32_prepare_operands": (c_int, [_P, _P, c_int64, c_int, c_int, _P, _P, c_int, c_int, c_int, c_int, c_int, _P]),
     "spc_tf32_prepare_weight": (c_int, [_P, _P, c_int, c_int, c_int, c_int, c_int, _P]),
     "spc_conv_output_size": (c_int, [c_int, POINTER(c_int32), POINTER(c_int32), POINTER(c_int32),
@@ -118,6 +119,7 @@ _PROTOTYPES = {
     "spc_norm_act_workspace_bytes": (c_size_t, [c_int64, c_int, c_int]),
     "spc_norm_act_forward": (c_int, [_P] * 6 + [ctypes.c_float, ctypes.c_float, c_int] + [_P] * 4 + [c_size_t, c_int64, c_int, c_int, _P]),
     "spc_norm_act_backward": (c_int, [_P] * 6 + [c_int] + [_P] * 4 + [c_size_t, c_int64, c_int, c_int, _P]),
+    "spc_fold_norms": (c_int, [_P, c_int, _P]),
     "spc_pool_row_order_workspace_bytes": (c_size_t, [c_int64]),
     "spc_pool_row_order": (c_int, [_P, c_int, c_int, c_int64, c_int64, _P, _P, c_size_t, _P]),
     "spc_pool": (c_int, [c_int, _P, _P, _P, _P, c_int, _P, _P, _P, _P, c_int64, c_int, c_int, c_int, _P]),

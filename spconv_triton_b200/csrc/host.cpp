@@ -16,6 +16,8 @@
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/extension.h>
 
+#include <pybind11/stl.h>
+
 #include <memory>
 #include <mutex>
 
@@ -576,6 +578,49 @@ c10::optional<Tensor> norm_act_train(const Tensor& x, const c10::optional<Tensor
   return y;
 }
 
+// Scale and shift of evaluation-mode normalisations (mean, variance, weight, bias, eps, channels): a block for them, where in it
+// each pair lies, and the argument of spc_fold_norms, which fills it; nothing where a tensor is not what the kernel takes.
+using Norm = std::tuple<Tensor, Tensor, c10::optional<Tensor>, c10::optional<Tensor>, double, int64_t>;
+using Places = std::vector<std::pair<int64_t, int64_t>>;
+c10::optional<std::tuple<Tensor, Places, pybind11::bytes>> norm_folds(const std::vector<Norm>& norms, const Tensor& like) {
+  std::vector<spc_norm_fold> folds(norms.size());
+  Places places(norms.size());
+  int64_t total = 0;
+  for (size_t i = 0; i < norms.size(); ++i) {
+    const auto& [mean, var, weight, bias, eps, c] = norms[i];
+    const Tensor none, *ts[4] = {&mean, &var, weight ? &*weight : &none, bias ? &*bias : &none};
+    const void* at[4];
+    for (int t = 0; t < 4; ++t) {
+      at[t] = nullptr;
+      folds[i].types[t] = SPC_F32;
+      if (!ts[t]->defined()) continue;
+      const auto type = ts[t]->scalar_type();
+      if (ts[t]->layout() != at::kStrided || ts[t]->device() != like.device() || ts[t]->dim() != 1 || ts[t]->numel() != c || c == 0 ||
+          !ts[t]->is_contiguous() || (type != at::kHalf && type != at::kBFloat16 && type != at::kFloat))
+        return c10::nullopt;
+      at[t] = ts[t]->const_data_ptr();
+      folds[i].types[t] = code_of(type);
+    }
+    folds[i].mean = at[0];
+    folds[i].var = at[1];
+    folds[i].weight = at[2];
+    folds[i].bias = at[3];
+    folds[i].channels = static_cast<int32_t>(c);
+    folds[i].eps = static_cast<float>(eps);
+    const int64_t room = (c + 3) & ~int64_t{3};
+    places[i] = {total, total + room};
+    total += 2 * room;
+  }
+  at::NoGradGuard no_grad;
+  c10::cuda::CUDAGuard guard(like.device());
+  Tensor block = at::empty({total}, like.options().dtype(at::kFloat));
+  for (size_t i = 0; i < norms.size(); ++i) {
+    folds[i].scale = block.data_ptr<float>() + places[i].first;
+    folds[i].shift = block.data_ptr<float>() + places[i].second;
+  }
+  return std::make_tuple(block, places, pybind11::bytes(reinterpret_cast<const char*>(folds.data()), folds.size() * sizeof(spc_norm_fold)));
+}
+
 // ---- pooling -------------------------------------------------------------------------------------------------------
 
 // Bytes of gathered rows from which on the gradient of an average works on the input rows in the order of the
@@ -750,6 +795,7 @@ PYBIND11_MODULE(_host, m) {
   m.def("conv_train", &conv_train);
   m.def("conv_eval", &conv_eval);
   m.def("norm_act_train", &norm_act_train);
+  m.def("norm_folds", &norm_folds);
   // both directions of an IEEE fp32 layer run on the kernel for few rows
   m.def("small", [](int64_t rows, int c_out, int c_in, int kv) {
     return spc_conv_small(rows, c_out, c_in, kv) != 0 && spc_conv_small(rows, c_in, c_out, kv) != 0;

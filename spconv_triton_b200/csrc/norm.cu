@@ -375,6 +375,31 @@ input_gradient_kernel(const T* __restrict__ x, const T* __restrict__ dy, const f
     one(*reinterpret_cast<const Vec<T>*>(from + r * cols), *reinterpret_cast<const Vec<T>*>(grad + r * cols), r);
 }
 
+// Evaluation mode: scale and shift for the store of the GEMM before the normalisation.  Latency of one launch (2 us), a CTA a
+// normalisation; made for each pass, so that nobody has to notice when the statistics change.
+constexpr int kMostFolds = 48;  // a launch's parameters are at most 4 KB
+struct Folds {
+  spc_norm_fold of[kMostFolds];
+};
+__device__ __forceinline__ float value_at(const void* p, int type, int c) {
+  if (type == SPC_F16) return to_float(static_cast<const __half*>(p)[c]);
+  if (type == SPC_BF16) return to_float(static_cast<const __nv_bfloat16*>(p)[c]);
+  return static_cast<const float*>(p)[c];
+}
+__global__ void __launch_bounds__(kThreads)
+fold_norms_kernel(const __grid_constant__ Folds folds) {
+  const spc_norm_fold& f = folds.of[blockIdx.x];
+  for (int c = threadIdx.x; c < f.channels; c += kThreads) {
+    float scale = rsqrtf(value_at(f.var, f.types[1], c) + f.eps);
+    if (f.weight != nullptr) scale *= value_at(f.weight, f.types[2], c);
+    // (rounded after each step, as torch's functions of these tensors round)
+    float shift = __fmul_rn(-value_at(f.mean, f.types[0], c), scale);
+    if (f.bias != nullptr) shift = __fadd_rn(shift, value_at(f.bias, f.types[3], c));
+    f.scale[c] = scale;
+    f.shift[c] = shift;
+  }
+}
+
 struct Plan {
   int chunks, across, lanes;  // chunks of rows, CTAs across the columns, threads a column vector
   long long chunk;
@@ -446,6 +471,24 @@ using namespace spc;
 extern "C" size_t spc_norm_act_workspace_bytes(int64_t rows, int cols, int dtype) {
   if (!takes(rows, cols, dtype)) return 0;
   return (static_cast<size_t>(plan(rows, cols, dtype).chunks) + 1) * cols * sizeof(float2);
+}
+
+extern "C" int spc_fold_norms(const spc_norm_fold* norms, int n, void* stream) {
+  if (norms == nullptr || n < 0) return fail(SPC_ERR_INVALID_ARGUMENT, "fold_norms: bad arguments");
+  for (int i = 0; i < n; ++i) {
+    const spc_norm_fold& f = norms[i];
+    if (!f.mean || !f.var || !f.scale || !f.shift || f.channels <= 0) return fail(SPC_ERR_INVALID_ARGUMENT, "fold_norms: bad arguments");
+    for (int t : f.types)
+      if (t != SPC_F16 && t != SPC_BF16 && t != SPC_F32) return fail(SPC_ERR_UNSUPPORTED, "fold_norms: unsupported dtype");
+  }
+  for (int first = 0; first < n; first += kMostFolds) {
+    Folds folds{};
+    const int count = std::min(n - first, kMostFolds);
+    std::copy(norms + first, norms + first + count, folds.of);
+    fold_norms_kernel<<<count, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(folds);
+    SPC_LAUNCH_OK();
+  }
+  return SPC_OK;
 }
 
 #define SPC_NORM_TYPES(CALL)                                                      \

@@ -71,6 +71,15 @@ extern "C" int spc_sequence_forward(const spc_seq_layer* layers, int n_layers, c
                                     const void* features, int64_t n_in, int dtype, void* arena_ptr,
                                     size_t arena_bytes, size_t* arena_needed, spc_seq_result* results,
                                     void* stream_main, void* stream_chain, void* stream_side) {
+  return spc_sequence_forward_norms(layers, n_layers, indices, features, n_in, dtype, arena_ptr, arena_bytes, arena_needed, results,
+                                    stream_main, stream_chain, stream_side, nullptr, 0);
+}
+
+extern "C" int spc_sequence_forward_norms(const spc_seq_layer* layers, int n_layers, const int32_t* indices,
+                                          const void* features, int64_t n_in, int dtype, void* arena_ptr,
+                                          size_t arena_bytes, size_t* arena_needed, spc_seq_result* results,
+                                          void* stream_main, void* stream_chain, void* stream_side,
+                                          const spc_norm_fold* norms, int n_norms) {
   if (!layers || n_layers <= 0 || n_layers > kMaxSeqLayers || !indices || !features || n_in <= 0 || !arena_ptr ||
       !arena_needed || !results || !stream_chain || !stream_side)
     return fail(SPC_ERR_INVALID_ARGUMENT, "sequence_forward: bad arguments");
@@ -175,6 +184,10 @@ extern "C" int spc_sequence_forward(const spc_seq_layer* layers, int n_layers, c
 
     // ---- the GEMM, on the caller's stream, once its rulebook is there ---------------------------
     const spc_seq_result& G = results[L.rulebook];
+    if (i == 0 && n_norms > 0) {
+      rc = spc_fold_norms(norms, n_norms, main);
+      if (rc != SPC_OK) return rc;
+    }
     SPC_CUDA_OK(cudaStreamWaitEvent(main, ev[L.rulebook], 0));
     R.features = arena.take(static_cast<size_t>(R.n_out) * L.c_out * esize);
     if (arena.overflow) break;

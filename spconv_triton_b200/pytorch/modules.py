@@ -2,7 +2,6 @@
 
 from __future__ import annotations
 
-import operator
 import threading
 import time
 from collections import OrderedDict
@@ -129,19 +128,8 @@ class SparseSequential(SparseModule):
         return x
 
 
-_BN_TENSORS = ("weight", "bias", "running_mean", "running_var", "num_batches_tracked")
-
-
 def _folded_bn(bn: nn.BatchNorm1d):
-    """fp32 (scale, shift) with bn(x) == x * scale + shift in evaluation mode;
-    memoised on the module until one of its tensors changes.  (The counter of batches among them: a forward
-    pass in training mode writes the running statistics past their version counters.)"""
-    own = {**bn._parameters, **bn._buffers}  # (attributes of a module are a slow look-up)
-    tensors = tuple([own[n] if n in own else getattr(bn, n) for n in _BN_TENSORS])
-    key = tuple((t._version, t.data_ptr()) if t is not None else None for t in tensors) + (bn.eps,)
-    cached = getattr(bn, "_spc_folded", None)
-    if cached is not None and cached[0] == key and all(map(operator.is_, cached[3], tensors)):
-        return cached[1], cached[2]
+    """fp32 (scale, shift) with bn(x) == x * scale + shift in evaluation mode."""
     with torch.no_grad():
         scale = torch.rsqrt(bn.running_var.float() + bn.eps)
         if bn.weight is not None:
@@ -149,9 +137,35 @@ def _folded_bn(bn: nn.BatchNorm1d):
         shift = -bn.running_mean.float() * scale
         if bn.bias is not None:
             shift = shift + bn.bias.float()
-        scale, shift = scale.contiguous(), shift.contiguous()
-    bn._spc_folded = (key, scale, shift, tensors)
-    return scale, shift
+        return scale.contiguous(), shift.contiguous()
+
+
+def _bn_operands(bn):
+    params, buffers = bn._parameters, bn._buffers  # (attributes of a module are a slow look-up)
+    if "weight" in params and "bias" in params and "running_mean" in buffers and "running_var" in buffers:
+        return buffers["running_mean"], buffers["running_var"], params["weight"], params["bias"], bn.eps, bn.num_features
+    return bn.running_mean, bn.running_var, bn.weight, bn.bias, bn.eps, bn.num_features
+
+
+def _folded_norms(norms, like, launch=True):
+    """``_folded_bn`` of each of ``norms`` for features like ``like``: a block of fp32 values, where in it each (scale, shift)
+    lies, and the argument of ``spc_fold_norms``, which fills the block (queued here unless ``launch`` is False; empty where
+    torch's functions have filled it).  None where a tensor is on another device or of another length.  Made anew by each
+    pass: a pair kept from one for the next would have to notice every way in which statistics can change (training writes
+    them past their version counters, as ``.data`` does) and wait for the stream that made it."""
+    done = _host.ext().norm_folds([_bn_operands(bn) for bn in norms], like)
+    if done is None:
+        parts = [t for bn in norms for t in _folded_bn(bn)]
+        if any(t.device != like.device for t in parts) or [t.shape for t in parts[::2]] != [(bn.num_features,) for bn in norms]:
+            return None
+        starts = [0]
+        for t in parts:
+            starts.append(starts[-1] + t.numel())
+        return torch.cat(parts), list(zip(starts[0::2], starts[1::2])), b""
+    if launch:
+        with torch.cuda.device(like.device):
+            _lib.check(_lib.load().spc_fold_norms(done[2], len(norms), _lib.current_stream(like.device)))
+    return done
 
 
 def _try_fold_bn_relu(mods, i, x):
@@ -179,10 +193,12 @@ def _try_fold_bn_relu(mods, i, x):
     if x.benchmark or x.indices.shape[0] == 0:
         return None
     relu = i + 2 < len(mods) and type(mods[i + 2]) in (nn.ReLU, SparseReLU)
-    scale, shift = _folded_bn(bn)
-    if scale.device != x.features.device:
+    folded = _folded_norms([bn], x.features)
+    if folded is None:
         return None
-    return conv(x, _fold=(scale, shift, relu)), i + 2 + int(relu)
+    block, ((at, to),), _ = folded
+    c = bn.num_features
+    return conv(x, _fold=(block[at:at + c], block[to:to + c], relu)), i + 2 + int(relu)
 
 
 _HOOKS = ("_forward_hooks", "_forward_pre_hooks", "_backward_hooks", "_backward_pre_hooks")

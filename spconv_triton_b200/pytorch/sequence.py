@@ -1,4 +1,4 @@
-"""Inference pass of a SparseSequential through ``spc_sequence_forward`` (not in
+"""Inference pass of a SparseSequential through ``spc_sequence_forward_norms`` (not in
 the reference).
 
 The reference runs a network layer by layer from Python
@@ -199,11 +199,10 @@ def forward(container, x):
     if steps[0].conv.in_channels != feats.shape[1]:
         return None
     dev = feats.device
-    from .modules import _folded_bn
+    from .modules import _folded_norms
     from .runahead import _side_stream
 
-    # pointers of this pass (weights and folded statistics may have changed since the last one)
-    keep = []
+    # pointers of this pass (weights may have changed since the last one)
     for st, L in zip(steps, plan.layers):
         c = st.conv
         w = c.weight
@@ -214,14 +213,6 @@ def forward(container, x):
         if b is not None and (b.dtype != feats.dtype or b.device != dev or b.shape != (c.out_channels,) or not b.is_contiguous()):
             return None
         L.bias = b.data_ptr() if b is not None else None
-        if st.bn is not None:
-            scale, shift = _folded_bn(st.bn)
-            if scale.device != dev:
-                return None
-            keep += [scale, shift]
-            L.scale, L.shift = scale.data_ptr(), shift.data_ptr()
-        else:
-            L.scale = L.shift = None
         L.act = _lib.SPC_ACT_RELU if st.relu else _lib.SPC_ACT_NONE
         L.act_alpha = 0.0
 
@@ -231,6 +222,15 @@ def forward(container, x):
     lib = _lib.load()
     with torch.cuda.device(dev):
         main = torch.cuda.current_stream(dev)
+        folds, normed = b"", [(st.bn, L) for st, L in zip(steps, plan.layers) if st.bn is not None]
+        if normed:
+            folded = _folded_norms([bn for bn, _ in normed], feats, launch=False)
+            if folded is None:
+                return None
+            block, places, folds = folded
+            base = block.data_ptr()
+            for (_, L), (scale, shift) in zip(normed, places):
+                L.scale, L.shift = base + 4 * scale, base + 4 * shift
         chain, side = _side_stream(dev, 0), _side_stream(dev, 1)
         # sized from the largest need per input voxel seen so far and rounded up coarsely, so that
         # passes over scenes of similar size ask the caching allocator for the same block again
@@ -251,11 +251,11 @@ def forward(container, x):
             # arena is a block of the caller's stream like any other (no record_stream, whose
             # deferred frees made the pool grow in bursts when several threads run passes).
             arena = torch.empty(arena_bytes, dtype=torch.uint8, device=dev)
-            rc = lib.spc_sequence_forward(ctypes.cast(plan.layers, ctypes.c_void_p), len(steps), indices.data_ptr(),
-                                          feats.data_ptr(), n_in, _lib.dtype_code(feats.dtype), arena.data_ptr(),
-                                          arena_bytes, ctypes.cast(ctypes.pointer(needed), ctypes.c_void_p),
-                                          ctypes.cast(plan.results, ctypes.c_void_p), main.cuda_stream,
-                                          chain.cuda_stream, side.cuda_stream)
+            rc = lib.spc_sequence_forward_norms(ctypes.cast(plan.layers, ctypes.c_void_p), len(steps), indices.data_ptr(),
+                                                feats.data_ptr(), n_in, _lib.dtype_code(feats.dtype), arena.data_ptr(),
+                                                arena_bytes, ctypes.cast(ctypes.pointer(needed), ctypes.c_void_p),
+                                                ctypes.cast(plan.results, ctypes.c_void_p), main.cuda_stream,
+                                                chain.cuda_stream, side.cuda_stream, folds, len(normed) if folds else 0)
             if rc == _lib.SPC_OK:
                 break
             # whatever was queued wrote into this arena: let it finish before the arena goes away
@@ -269,7 +269,7 @@ def forward(container, x):
         else:
             return None
         plan.bytes_per_voxel = floor[1] = max(plan.bytes_per_voxel, floor[1], needed.value / n_in)
-        return _wrap(plan, x, indices, arena, dev, keep)
+        return _wrap(plan, x, indices, arena)
 
 
 _ABSENT = 0xFFFFFFFFFFFFFFFF  # offset of a table the pass did not produce
@@ -286,7 +286,7 @@ def _column_major(rowmajor, kv, late, table=None):
     return table
 
 
-def _wrap(plan, x, indices, arena, dev, keep):
+def _wrap(plan, x, indices, arena):
     """The output tensor and the rulebook cache entries, as views of the arena."""
     steps, results = plan.steps, plan.results
     ndim = len(x.spatial_shape)
@@ -329,5 +329,4 @@ def _wrap(plan, x, indices, arena, dev, keep):
     out = SparseConvTensor(feats, cur_indices, plan.out_shape, x.batch_size, x.grid, x.voxel_num, indice_dict)
     x._carry_over(out)
     out._planner = None
-    out._spc_keep = keep  # folded statistics in use by kernels that may still be queued
     return out
