@@ -57,7 +57,7 @@ struct StreamParams {
   int stages, a_stage_bytes, b_stage_bytes;
   int copiers;     // copy warps at work: no more than there are stages (a slot's last round but one must be over)
   int acc_cols, tmem_cols;  // columns of one accumulator and of both
-  int epi_bytes;   // bytes of a row that the epilogue passes through shared memory at a time: 32, 64 or 128
+  int epi_bytes;   // bytes of a row that the epilogue passes through shared memory at a time: 32, 64 or 128, and 16 channels at least
   int epi_pad;     // output channels rounded up to 16; sizes the epilogue scale / shift arrays
   int b_row_bytes;  // swizzle span of the MN-major B rows
   int* status;
@@ -550,9 +550,12 @@ int gather_gemm_stream(const void* src, const void* w, const Epilogue& epi, cons
   };
   const int widest = p.epi_bytes;
   const auto stages = [&] { return static_cast<int>(std::min<size_t>(kMaxStages, (per_cta - fixed()) / stage_bytes)); };
-  // a stage per copy warp, if need be with a narrower epilogue; where even that leaves two, a wide one
-  while (p.epi_bytes > 32 && stages() < kCopyWarps) p.epi_bytes /= 2;
+  // a stage per copy warp, if need be with a narrower epilogue (the 16 channels of a step fit it: 32 bytes of 16-bit results,
+  // 64 of fp32 ones); where even that leaves two, a wide one
+  const int narrowest = 16 * (out_dtype == SPC_F32 ? 4 : 2);
+  while (p.epi_bytes > narrowest && stages() < kCopyWarps) p.epi_bytes /= 2;
   if (stages() < kCopyWarps) p.epi_bytes = widest;
+  if (p.epi_bytes < narrowest || row_bytes % narrowest != 0) return fail(SPC_ERR_UNSUPPORTED, "TMA gather-GEMM: store of %d channels", n_dim);
   p.stages = stages();
   p.copiers = std::min(p.stages, kCopyWarps);
   const size_t smem_bytes = fixed() + static_cast<size_t>(p.stages) * stage_bytes;

@@ -1,5 +1,6 @@
 """The gather-GEMM of many tiles a CTA (csrc/gemm_stream.cu) against fp32 matmuls of the same rows: at the fewest rows it
-takes, with ragged last tiles, tiles without any pair, every span of a row, and each option of the store."""
+takes, with ragged last tiles, tiles without any pair, every span of a row, each option of the store, and stores whose
+pass through shared memory the host narrows to win a third stage."""
 
 import ctypes
 
@@ -55,11 +56,21 @@ def _close(got, want, magnitude, out_type):
     assert (got.float() - want).abs().max().item() <= EPS[out_type] * want.abs().max().item() * 1.01 + 2.0 ** -20 * magnitude
 
 
+# (stages of the kernel and bytes of a row that a store passes through shared memory, beside the cases below)
 @pytest.mark.parametrize("c_in,c_out,kv,dtype,out_type,ordered,colmajor", [
     (64, 128, 27, torch.float16, torch.float16, True, False), (64, 96, 27, torch.bfloat16, torch.bfloat16, False, False),
     (32, 64, 27, torch.float16, torch.float32, True, False), (32, 112, 33, torch.float16, torch.float16, True, False),
     (16, 16, 27, torch.float16, torch.float16, True, True), (16, 128, 3, torch.bfloat16, torch.float32, False, True),
-    (64, 16, 40, torch.float16, torch.float16, True, False)])
+    (64, 16, 40, torch.float16, torch.float16, True, False),
+    (64, 128, 8, torch.float16, torch.float32, True, False),  # 2, 128
+    (64, 128, 9, torch.bfloat16, torch.float32, False, False),  # 2, 128
+    (64, 112, 27, torch.float16, torch.float32, True, False),  # 2, 128
+    (64, 128, 1, torch.float16, torch.float32, True, False),  # 3, 64
+    (64, 96, 27, torch.float16, torch.float32, False, False),  # 3, 64
+    (64, 64, 27, torch.bfloat16, torch.float32, True, False),  # 3, 128
+    (64, 128, 8, torch.float16, torch.float16, True, False),  # 3, 32
+    (64, 128, 9, torch.bfloat16, torch.bfloat16, False, False),  # 3, 32
+    (64, 112, 27, torch.float16, torch.float16, True, False)])  # 3, 32
 def test_forward_and_input_gradient(c_in, c_out, kv, dtype, out_type, ordered, colmajor):
     gen = torch.Generator("cuda").manual_seed(c_in + c_out)
     n_out, n_in = _rows(c_out), 30001
@@ -72,16 +83,18 @@ def test_forward_and_input_gradient(c_in, c_out, kv, dtype, out_type, ordered, c
     order = torch.randperm(n_out, generator=gen, device="cuda").int() if ordered else None
     plain = _reference(x, w, cm)
     lib = _lib.load()
-    for full in (False, True):
+    acts = {1: torch.relu, 2: torch.sigmoid, 3: lambda z: torch.nn.functional.leaky_relu(z, 0.1)}
+    for act in (0, *acts):
+        full = act != 0
         out = torch.full((n_out, c_out), float("nan"), dtype=out_type, device="cuda")
-        extra = (_p(scale), _p(shift), 1, 0.0, _p(residual)) if full else (None, None, 0, 0.0, None)
+        extra = (_p(scale), _p(shift), act, 0.1, _p(residual)) if full else (None, None, 0, 0.0, None)
         rc = lib.spc_conv_forward_residual(_p(x), _p(w), _p(bias if full else None), _p(cm), _p(None if colmajor else rm), _p(order), _p(out),
                                            n_in, n_out, c_in, c_out, kv, CODES[dtype], CODES[out_type], 0, 0, *extra,
                                            ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
         assert rc == 0
         want = plain
         if full:
-            want = torch.relu((plain + bias.float()) * scale + shift) + residual.float()
+            want = acts[act]((plain + bias.float()) * scale + shift) + residual.float()
         _close(out, want, 4 * (1 + scale.abs().max().item()), out_type)
     # the input gradient of a layer with the channels the other way round, of a strided and of a submanifold layer
     weight = w.permute(2, 1, 0).contiguous()  # [c_in, kv, c_out]: its output channels are reduced over
