@@ -48,16 +48,14 @@ inline EncodeTiledFn encode_fn() {
   // whose first step may be an input gradient) does not have: an empty free makes it current.
   static thread_local bool current = false;
   if (!current) current = cudaFree(nullptr) == cudaSuccess;
-  static EncodeTiledFn fn = nullptr;
-  static bool tried = false;
-  if (!tried) {
-    tried = true;
+  // (a thread that comes while another looks the function up waits for it)
+  static const EncodeTiledFn fn = []() -> EncodeTiledFn {
     void* raw = nullptr;
     cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &raw, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(raw);
-  }
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &raw, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess)
+      return nullptr;
+    return reinterpret_cast<EncodeTiledFn>(raw);
+  }();
   return fn;
 }
 
@@ -96,7 +94,9 @@ inline int weight_map(CUtensorMap* map, const void* w, int n_dim, int r_dim, int
     box[2] = static_cast<cuuint32_t>(n_dim);
   }
   const cuuint32_t estr[3] = {1, 1, 1};
-  const CUresult r = encode_fn()(map, tma_dtype(dtype), 3, const_cast<void*>(w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  const EncodeTiledFn encode = encode_fn();
+  if (encode == nullptr) return fail(SPC_ERR_CUDA, "the driver has no cuTensorMapEncodeTiled");
+  const CUresult r = encode(map, tma_dtype(dtype), 3, const_cast<void*>(w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                                  swizzle_for(b_row_bytes), CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? SPC_OK : fail(SPC_ERR_CUDA, "cuTensorMapEncodeTiled(B) failed: %d", static_cast<int>(r));
 }

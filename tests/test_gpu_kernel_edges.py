@@ -230,3 +230,31 @@ def test_average_of_16_bit_rows_is_the_rounded_fp32_average(dtype, channels):
     assert torch.equal(got.isnan(), exp.isnan())
     assert torch.equal(got.nan_to_num(7.0), exp.nan_to_num(7.0))
     assert torch.equal(torch.signbit(got)[~got.isnan()], torch.signbit(exp)[~exp.isnan()])
+
+
+_FIRST_CALLS = """
+import ctypes, sys, threading
+ctypes.CDLL(sys.argv[2]).cudaFree(None)  # the context, so that the threads meet in the call itself
+lib, gate, got = ctypes.CDLL(sys.argv[1]), threading.Barrier(16), []
+def first():
+    gate.wait()
+    got.append(lib.spc_conv_forward_needs_colmajor(64, 64, 27, 0, 0, 0, 0))
+threads = [threading.Thread(target=first) for _ in range(16)]
+for t in threads: t.start()
+for t in threads: t.join()
+sys.exit(any(got))
+"""
+
+
+def test_first_calls_of_many_threads():
+    """All of them find the tensor cores, also the ones that come while another looks the driver's function up (new processes:
+    it happens once in each, and not in each)."""
+    import subprocess
+    import sys
+
+    from spconv_triton_b200.csrc.build import LIB
+
+    with open("/proc/self/maps") as f:
+        runtime = next(line.split()[-1] for line in f if "libcudart.so" in line)
+    for _ in range(6):
+        subprocess.run([sys.executable, "-c", _FIRST_CALLS, str(LIB), runtime], check=True, timeout=60)
