@@ -347,17 +347,28 @@ wgrad_f32_kernel(const float* __restrict__ feats, const float* __restrict__ gout
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-// Few rows (the rule is at gather_gemm_small_takes): a tile of any kernel that stages operands is one chain of 10 - 20 offsets
-// on a chip that is nearly empty.  Here 16 lanes have a row, an output channel each (up to four), find the row's offsets in
-// its own table entries and read rows and weights through the caches: as many rounds as a row has neighbours.
-// Bound: latency of two or three dependent loads a neighbour.  2 000 rows, 16 -> 16, 1.2 neighbours: 4.4 us, against 17 for
-// the tensor cores, 2 for their operands' copies and 9 for the row order that the copies' kernel wants and this one does not.
+// Few rows (the rule is at gather_gemm_small_takes): a tile of 64 or 128 rows is one chain of up to 27 offsets on a chip that
+// is nearly empty.  Here a CTA has eight rows, 16 lanes a row, and passes over the offsets that any of them has: the weights
+// of an offset (read by neighbouring lanes, whichever way they are transposed) and the rows that have it come by cp.async,
+// two offsets ahead, and a row's lanes multiply, NC output channels each, if the row has the offset.
+// Bound: latency: 1 - 1.5 us from the launch to the first stage, then 0.4 us an offset (copies, barrier, multiplications) with
+// one or two CTAs a multiprocessor.  Measured beside the rule.
 constexpr int kSmallRows = kThreads / 16;
+// Floats between staged rows: whole 16-byte words, an odd number of them, so that lanes on neighbouring rows meet different banks.
+__host__ __device__ constexpr int small_pitch(int floats) { return ((floats >> 2) | 1) << 2; }
+constexpr int kSmallStages = 3;  // (four and eight: the same)
+constexpr int kSmallMostBytes = kSmallStages * (64 + kSmallRows) * small_pitch(64) * static_cast<int>(sizeof(float));
+
+__device__ __forceinline__ void copy16(uint32_t to, const float* from) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(from) : "memory");
+}
 
 template <bool W_MN, int NC>  // NC: output channels of a lane
 __global__ void __launch_bounds__(kThreads)
 gather_gemm_small_kernel(const __grid_constant__ F32Params p) {
+  extern __shared__ __align__(16) float small_stages[];
   __shared__ __align__(16) int entries[kSmallRows][32];
+  __shared__ uint32_t votes[kThreads / 32];
   const int group = threadIdx.x >> 4, lane = threadIdx.x & 15;
   const long long row = static_cast<long long>(blockIdx.x) * kSmallRows + group;
   uint32_t mine = 0;
@@ -369,31 +380,82 @@ gather_gemm_small_kernel(const __grid_constant__ F32Params p) {
   }
 #pragma unroll
   for (int s = 8; s > 0; s >>= 1) mine |= __shfl_xor_sync(0xffffffffu, mine, s);
-  __syncwarp();
+  const uint32_t both = mine | __shfl_xor_sync(0xffffffffu, mine, 16);
+  if ((threadIdx.x & 31) == 0) votes[threadIdx.x >> 5] = both;
+  __syncthreads();
+  uint32_t all = 0;
+#pragma unroll
+  for (int w = 0; w < kThreads / 32; ++w) all |= votes[w];
+
+  // A stage: the weights, [n_dim][r_dim] or, read transposed, [r_dim][n_dim] with the pitch of their rows, and the CTA's rows.
+  const int w_rows = W_MN ? p.r_dim : p.n_dim, w_cols = W_MN ? p.n_dim : p.r_dim;
+  const int w_pitch = small_pitch(w_cols), x_pitch = small_pitch(p.r_dim);
+  const int stage_floats = w_rows * w_pitch + kSmallRows * x_pitch;
+  const int x_at = w_rows * w_pitch + group * x_pitch;
+  // this thread's piece of the weight rows `group`, `group` + kSmallRows, ... and of its own row
+  const float* const w_from = p.w + group * p.kv * w_cols + 4 * lane;
+  const float* const x_from = p.src + 4 * lane;
+  const int w_step = kSmallRows * p.kv * w_cols;
+  const uint32_t stages = static_cast<uint32_t>(__cvta_generic_to_shared(small_stages));
+  const uint32_t w_to = 4 * (group * w_pitch + 4 * lane), x_to = 4 * (x_at + 4 * lane);
+  const bool w_lane = 4 * lane < w_cols, x_lane = 4 * lane < p.r_dim;
+  uint32_t ahead = all;  // offsets that have not been asked for
+  uint32_t to = stages;
+  const uint32_t stage_bytes = 4 * stage_floats, end = stages + kSmallStages * stage_bytes;
+  const auto fetch_next = [&] {
+    if (ahead != 0) {
+      const int kk = __ffs(ahead) - 1, k = p.reversed ? p.kv - 1 - kk : kk;
+      ahead &= ahead - 1;
+      if (w_lane) {
+        const float* from = w_from + k * w_cols;
+        uint32_t there = to + w_to;
+#pragma unroll 4
+        for (int i = group; i < w_rows; i += kSmallRows, from += w_step, there += 4 * kSmallRows * w_pitch) copy16(there, from);
+      }
+      if (x_lane && (mine >> kk & 1u)) copy16(to + x_to, x_from + static_cast<long long>(entries[group][kk]) * p.r_dim);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");  // (empty ones too: the wait below counts them)
+    to += stage_bytes;
+    if (to == end) to = stages;
+  };
+#pragma unroll 1
+  for (int s = 0; s < kSmallStages - 1; ++s) fetch_next();
+
   float acc[NC];
 #pragma unroll
   for (int c = 0; c < NC; ++c) acc[c] = 0.f;
-  for (uint32_t rest = mine; rest != 0; rest &= rest - 1) {
-    const int kk = __ffs(rest) - 1, k = p.reversed ? p.kv - 1 - kk : kk;
-    const float4* const x = reinterpret_cast<const float4*>(p.src + static_cast<long long>(entries[group][kk]) * p.r_dim);
+  int at = 0;
+#pragma unroll 1
+  for (uint32_t rest = all; rest != 0; rest &= rest - 1) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kSmallStages - 2) : "memory");
+    __syncthreads();  // this stage is there for everyone, and everyone is done with the one that is filled next
+    fetch_next();
+    const float* const stage = small_stages + at * stage_floats;
+    at = at + 1 == kSmallStages ? 0 : at + 1;
+    if (!(mine >> (__ffs(rest) - 1) & 1u)) continue;
+    const float4* const x = reinterpret_cast<const float4*>(stage + x_at);
 #pragma unroll 4
     for (int r = 0; r < p.r_dim; r += 4) {
-      const float4 a = __ldg(x + (r >> 2));
+      const float4 a = x[r >> 2];
+      float b[4][NC];
+      if (W_MN) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+          for (int c = 0; c < NC; ++c) b[q][c] = stage[(r + q) * w_pitch + lane + 16 * c];
+      } else {
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          const float4 v = *reinterpret_cast<const float4*>(stage + (lane + 16 * c) * w_pitch + r);
+          b[0][c] = v.x; b[1][c] = v.y; b[2][c] = v.z; b[3][c] = v.w;
+        }
+      }
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
-        const int n = lane + 16 * c;
-        float4 b;
-        if (W_MN) {
-          const float* const w = p.w + (static_cast<long long>(r) * p.kv + k) * p.n_dim + n;
-          const long long pitch = static_cast<long long>(p.kv) * p.n_dim;
-          b = make_float4(__ldg(w), __ldg(w + pitch), __ldg(w + 2 * pitch), __ldg(w + 3 * pitch));
-        } else {
-          b = __ldg(reinterpret_cast<const float4*>(p.w + (static_cast<long long>(n) * p.kv + k) * p.r_dim + r));
-        }
-        acc[c] = fmaf(a.x, b.x, acc[c]);
-        acc[c] = fmaf(a.y, b.y, acc[c]);
-        acc[c] = fmaf(a.z, b.z, acc[c]);
-        acc[c] = fmaf(a.w, b.w, acc[c]);
+        acc[c] = fmaf(a.x, b[0][c], acc[c]);
+        acc[c] = fmaf(a.y, b[1][c], acc[c]);
+        acc[c] = fmaf(a.z, b[2][c], acc[c]);
+        acc[c] = fmaf(a.w, b[3][c], acc[c]);
       }
     }
   }
@@ -407,11 +469,31 @@ gather_gemm_small_kernel(const __grid_constant__ F32Params p) {
   }
 }
 
+template <bool W_MN, int NC>
+int launch_small(const F32Params& p, cudaStream_t st) {
+  const int w_rows = W_MN ? p.r_dim : p.n_dim, w_cols = W_MN ? p.n_dim : p.r_dim;
+  const size_t stage_bytes = (static_cast<size_t>(w_rows) * small_pitch(w_cols) + kSmallRows * small_pitch(p.r_dim)) * sizeof(float);
+  static bool configured[kMaxDevices] = {false};  // per instantiation and device
+  SPC_CUDA_OK(ensure_dynamic_smem(gather_gemm_small_kernel<W_MN, NC>, kSmallMostBytes, configured));
+  gather_gemm_small_kernel<W_MN, NC>
+      <<<static_cast<unsigned>(ceil_div(p.m_rows, kSmallRows)), kThreads, kSmallStages * stage_bytes, st>>>(p);
+  SPC_LAUNCH_OK();
+  return SPC_OK;
+}
+
 }  // namespace
 
-// Thin layers (at most 8 reduction channels) have kernels of their own.
-// 9 to 64 channels, one table word of offsets, and at most 2 M row-channel-channel products an offset: beyond that the
-// weights' way through the L1 (a kilobyte a pair at 16 x 16) costs more than the tiles save.
+// 16, 32, 48 or 64 output channels, 12 to 64 reduction channels in steps of four, one table word of offsets, and at most 2 M
+// row-channel-channel products an offset, where the tiles catch up.  Layer of 27 offsets, its rulebook there, forward / input
+// gradient in us, the tensor cores (with their operands' copies and a row order) -> this kernel; and lanes that read rows and
+// weights through the caches, each lane its own channel's weights (16 lines a load), which this one replaces:
+//     channels, rows      1.2 neighbours a row                                20 - 26 neighbours a row
+//     16 -> 16,  2 000   19.0 / 18.8 ->  6.1 /  5.7    4.1 /  9.0            24.0 / 23.8 -> 14.3 / 14.3    16 /  54
+//     16 -> 16,  8 192   19.2 / 19.2 ->  6.4 /  6.1    5.3 /  9.2            24.5 / 24.3 -> 24.7 / 24.3    32 /  43
+//     16 -> 64,  2 048   21.2 / 51.1 ->  6.7 /  9.2    6.7 / 26.9            26.9 / 84.5 -> 21.4 / 27.3    37 / 187
+//     32 -> 32,  2 048   28.9 / 29.6 ->  6.9 /  7.4    7.7 /  9.8            39.9 / 40.8 -> 21.7 / 21.8    60 /  58
+//     48 -> 48,    900   49.8 / 45.0 ->  8.1 /  7.4    9.4 / 18.3            77.6 / 70.7 -> 27.6 / 24.9    51 /  91
+//     64 -> 64,    512   81.0 / 72.4 -> 10.2 / 13.0   18.1 / 27.6            93.7 / 84.6 -> 30.3 / 37.1   131 / 151
 bool gather_gemm_small_takes(long long m_rows, int n_dim, int r_dim, int kv) {
   return kv <= 32 && n_dim % 16 == 0 && n_dim <= 64 && r_dim % 4 == 0 && r_dim > 8 && r_dim <= 64 && m_rows * n_dim * r_dim <= (2ll << 20);
 }
@@ -420,23 +502,16 @@ int gather_gemm_small(const void* src, const void* w, const Epilogue& epi, const
                       int n_dim, int r_dim, int kv, bool transposed_weight, bool reversed, cudaStream_t st) {
   F32Params p{static_cast<const float*>(src), static_cast<const float*>(w), epi, nullptr, pairs_rowmajor, nullptr,
               static_cast<float*>(out), m_rows, n_dim, r_dim, kv, (kv + 3) & ~3, reversed ? 1 : 0};
-  const unsigned grid = static_cast<unsigned>(ceil_div(m_rows, kSmallRows));
-#define SPC_SMALL(NC)                                                                    \
-  case NC:                                                                               \
-    if (transposed_weight) gather_gemm_small_kernel<true, NC><<<grid, kThreads, 0, st>>>(p); \
-    else gather_gemm_small_kernel<false, NC><<<grid, kThreads, 0, st>>>(p);              \
-    break;
   switch (n_dim / 16) {
-    SPC_SMALL(1)
-    SPC_SMALL(2)
-    SPC_SMALL(3)
-    SPC_SMALL(4)
+    case 1: return transposed_weight ? launch_small<true, 1>(p, st) : launch_small<false, 1>(p, st);
+    case 2: return transposed_weight ? launch_small<true, 2>(p, st) : launch_small<false, 2>(p, st);
+    case 3: return transposed_weight ? launch_small<true, 3>(p, st) : launch_small<false, 3>(p, st);
+    case 4: return transposed_weight ? launch_small<true, 4>(p, st) : launch_small<false, 4>(p, st);
   }
-#undef SPC_SMALL
-  SPC_LAUNCH_OK();
-  return SPC_OK;
+  return fail(SPC_ERR_UNSUPPORTED, "fp32 gather-GEMM of few rows: %d output channels", n_dim);
 }
 
+// Thin layers (at most 8 reduction channels) have kernels of their own.
 bool gather_gemm_f32_supported(int n_dim, int r_dim, int dtype, int out_dtype) {
   return dtype == SPC_F32 && out_dtype == SPC_F32 && n_dim % 4 == 0 && r_dim % 4 == 0 && r_dim > 8;
 }
