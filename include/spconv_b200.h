@@ -205,6 +205,10 @@ int spc_pairs_to_rowmajor(const int32_t* pairs, int kv, int64_t n, int32_t* out,
 /* ... and back: the column-major table [kv, n] of a row-major one. */
 int spc_rowmajor_to_pairs(const int32_t* rowmajor, int kv, int64_t n, int32_t* pairs, void* stream);
 
+/* ... and the order that spc_rulebook_tables makes of its rows, for a table that was made
+ * without one: order [n], keys [n] scratch, kernels of at most 32 offsets and n <= 8192. */
+int spc_rowmajor_order(const spc_geometry* g, const int32_t* rowmajor, int64_t n, int32_t* order, uint32_t* keys, void* stream);
+
 /* Phase 2, Native format: replaces native_pairs, _impl/pairs.py:223-278.
  *   pair [2, kv, n_in] (-1 fill): per offset the contributing input rows in
  *   ascending order and their output rows; indice_num_per_loc [kv]. */

@@ -111,6 +111,7 @@ _PROTOTYPES = {
                              POINTER(c_int64), _P]),
     "spc_rulebook_tables": (c_int, [POINTER(Geometry), _P, c_int64, c_int64, _P, c_size_t] + [_P] * 8),
     "spc_rowmajor_to_pairs": (c_int, [_P, c_int, c_int64, _P, _P]),
+    "spc_rowmajor_order": (c_int, [_P, _P, c_int64, _P, _P, _P]),
     "spc_conv_backward_input_tables": (c_int, [_P, _P, _P, _P, _P, _P, c_int64, c_int64, c_int, c_int, c_int, c_int,
                                                c_int, c_int, c_int, _P]),
     "spc_conv_backward_input_needs_colmajor": (c_int, [c_int] * 6),

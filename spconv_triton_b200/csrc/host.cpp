@@ -98,6 +98,8 @@ std::shared_ptr<Geometry> make_geometry(int batch, const std::vector<int>& in, c
 
 // Rows from which on the GEMM's row order is worth its sort: with a tile or less there is nothing to group.
 constexpr int64_t kOrderRows = 256;
+// ... and up to which the order that a submanifold rulebook was built without is made when a layer wants it.
+constexpr int64_t kLateOrderRows = 8192;
 
 // The tables of one rulebook, output side and input side, made as they are asked for.  The kernels read the
 // row-major tables; the column-major ones serve the CUDA-core and weight-gradient kernels.
@@ -135,8 +137,9 @@ struct Rulebook {
     if (order && ordered(n)) s.order = at::empty({n}, indices.options());
     return s;
   }
-  // The side whose rows are the output rows (of the layer, or of its inverse with `input`).
-  Side side(bool input, bool colmajor) {
+  // The side whose rows are the output rows (of the layer, or of its inverse with `input`); with the row order, where
+  // such a rulebook has one, if `order`.
+  Side side(bool input, bool colmajor, bool order) {
     if (input && subm()) throw Failure(SPC_ERR_INVALID_ARGUMENT, "a submanifold rulebook has one side");
     c10::cuda::CUDAGuard guard(indices.device());
     // A capture records its kernels and does not run them: it waits for nothing (what came before a capture is
@@ -146,7 +149,9 @@ struct Rulebook {
     captured = captured || capturing;
     Side& kept = input ? bwd : fwd;
     Late& late = input ? late_bwd : late_fwd;
-    const bool missing = !kept.rm.defined() || (colmajor && !kept.cm.defined());
+    const bool no_cm = colmajor && !kept.cm.defined();
+    const bool no_order = order && subm() && !kept.order.defined() && ordered(n_out) && n_out <= kLateOrderRows;
+    const bool missing = !kept.rm.defined() || no_cm || no_order;
     if (!missing && !late.stream) return kept;
     const auto now = c10::cuda::getCurrentCUDAStream();
     Side s = kept;
@@ -163,8 +168,15 @@ struct Rulebook {
     } else {
       const int64_t n = s.rm.size(0);
       s.rm.record_stream(now);
-      s.cm = make(geo->kv, n);
-      check(spc_rowmajor_to_pairs(ints(s.rm), geo->kv, n, ints(s.cm), now.stream()));
+      if (no_cm) {
+        s.cm = make(geo->kv, n);
+        check(spc_rowmajor_to_pairs(ints(s.rm), geo->kv, n, ints(s.cm), now.stream()));
+      }
+      if (no_order) {
+        s.order = at::empty({n}, indices.options());
+        const Tensor keys = at::empty_like(s.order);
+        check(spc_rowmajor_order(&geo->g, ints(s.rm), n, ints(s.order), reinterpret_cast<uint32_t*>(ints(keys)), now.stream()));
+      }
     }
     if (capturing) return s;
     kept = s;
@@ -219,9 +231,11 @@ struct Fp32Plan {
   bool tensor = false;
   int rows_mode = 0, weight_mode = 0, mult = 1;
 };
+// An IEEE fp32 layer on the kernel for few rows, which reads no row order.
+bool few_rows(int64_t rows, int n_dim, int r_dim, int kv, bool tf32) { return !tf32 && spc_conv_small(rows, n_dim, r_dim, kv) != 0; }
 Fp32Plan fp32_plan(int64_t rows, int n_dim, int r_dim, int kv, bool tf32, int split_most) {
   Fp32Plan p;
-  if (!tf32 && spc_conv_small(rows, n_dim, r_dim, kv)) return p;
+  if (few_rows(rows, n_dim, r_dim, kv, tf32)) return p;
   if (n_dim % 16 || n_dim < 16 || n_dim > 256 || r_dim % 8) return p;
   if (tf32) {
     p.tensor = true;
@@ -298,7 +312,7 @@ Tensor conv_forward_raw(const Tensor& features, const Tensor& weight, const Tens
   }
   const int type = code_of(x.scalar_type()), out_code = code_of(out_type);
   const bool colmajor = spc_conv_forward_needs_colmajor(c_in, k_out, kv, type, out_code, precision, SPC_GEMM_AUTO);
-  const Rulebook::Side t = rb->side(o.inverse, colmajor);
+  const Rulebook::Side t = rb->side(o.inverse, colmajor, !(type == SPC_F32 && out_code == SPC_F32 && few_rows(n_out, k_out, c_in, kv, o.tf32)));
   check(spc_conv_forward_residual(from, weights, data(b), ints(t.cm), ints(t.rm), ints(t.order), out.data_ptr(), n_in, n_out,
                                   c_in, k_out, kv, type, out_code, precision, SPC_GEMM_AUTO,
                                   scale.defined() ? scale.data_ptr<float>() : nullptr, shift.defined() ? shift.data_ptr<float>() : nullptr,
@@ -320,14 +334,14 @@ Tensor conv_backward_input_raw(const Tensor& grad, const Tensor& weight, const B
     // as a forward convolution of grad with the transposed weight
     const Prepared copies = prepared(grad, w, reversed ? 2 : 1, plan);
     const bool colmajor = spc_conv_forward_needs_colmajor(plan.mult * k_out, c_in, kv, type, type, SPC_PREC_TF32, SPC_GEMM_AUTO);
-    const Rulebook::Side t = rb->side(input, colmajor);
+    const Rulebook::Side t = rb->side(input, colmajor, true);
     check(spc_conv_forward(copies.rows, copies.weight, nullptr, ints(t.cm), ints(t.rm), ints(t.order), din.data_ptr(), n_grad, n_in,
                            plan.mult * k_out, c_in, kv, type, type, SPC_PREC_TF32, SPC_GEMM_AUTO, nullptr, nullptr, SPC_ACT_NONE, 0.f,
                            stream_of(grad)));
     return din;
   }
   const bool colmajor = spc_conv_backward_input_needs_colmajor(c_in, k_out, kv, type, precision, SPC_GEMM_AUTO);
-  const Rulebook::Side t = rb->side(input, colmajor);
+  const Rulebook::Side t = rb->side(input, colmajor, !(type == SPC_F32 && few_rows(n_in, c_in, k_out, kv, o.tf32)));
   check(spc_conv_backward_input_tables(grad.data_ptr(), w.data_ptr(), ints(t.cm), ints(t.rm), ints(t.order), din.data_ptr(), n_in, n_grad,
                                        c_in, k_out, kv, reversed, type, precision, SPC_GEMM_AUTO, stream_of(grad)));
   return din;
@@ -337,7 +351,7 @@ Tensor conv_backward_weight_raw(const Tensor& features, const Tensor& grad, at::
   const int64_t k_out = sizes[0], c_in = sizes[sizes.size() - 1], kv = rb->geo->kv;
   Tensor dw = at::empty(sizes, grad.options());
   Tensor x = operand(features.scalar_type() == grad.scalar_type() ? features : features.to(grad.scalar_type()));
-  const Rulebook::Side t = rb->side(o.inverse, true);
+  const Rulebook::Side t = rb->side(o.inverse, true, false);
   const int64_t n_out = grad.size(0);
   const size_t bytes = spc_conv_backward_weight_workspace_bytes(n_out, c_in, k_out, kv);
   Tensor ws = at::empty({static_cast<int64_t>(std::max<size_t>(bytes, 16))}, grad.options().dtype(at::kByte));
@@ -634,7 +648,7 @@ Tensor pool_rows(int op, const Tensor& src, const Tensor& own, const Tensor& ref
                  const Tensor& aux_out) {
   const int64_t c = src.size(1);
   const bool flip = rb->subm() && input;  // (a pool over a submanifold neighbourhood: the table of the other side)
-  const Rulebook::Side t = rb->side(input && !flip, false);
+  const Rulebook::Side t = rb->side(input && !flip, false, false);
   const int64_t n = t.rm.size(0);
   Tensor out = at::empty({n, c}, src.options());
   if (c == 0) return out;
@@ -788,8 +802,8 @@ PYBIND11_MODULE(_host, m) {
       .def_readonly("indices", &Rulebook::indices)
       .def_readonly("out_indices", &Rulebook::out_indices)
       .def_readonly("captured", &Rulebook::captured)
-      .def("rowmajor", [](Rulebook& r, bool input) { return r.side(input, false).rm; }, py::call_guard<py::gil_scoped_release>())
-      .def("colmajor", [](Rulebook& r, bool input) { return r.side(input, true).cm; }, py::call_guard<py::gil_scoped_release>());
+      .def("rowmajor", [](Rulebook& r, bool input) { return r.side(input, false, false).rm; }, py::call_guard<py::gil_scoped_release>())
+      .def("colmajor", [](Rulebook& r, bool input) { return r.side(input, true, false).cm; }, py::call_guard<py::gil_scoped_release>());
   m.def("build_rulebook", &build_rulebook);
   m.def("record_stream", &record_stream);
   m.def("conv_train", &conv_train);

@@ -1194,6 +1194,16 @@ finish_outputs_kernel(const __grid_constant__ Geo g, const typename Table<K64>::
   if (counts != nullptr) count_buckets(live ? bucket_of(word) : -1, slot_bucket, slot_count, counts);
 }
 
+// The keys of the order from a finished row-major table, as the fill makes them on its way.
+__global__ void __launch_bounds__(kThreads)
+rowmajor_keys_kernel(const __grid_constant__ Geo g, const int32_t* __restrict__ rm, int kvp, long long n, uint32_t* __restrict__ keys) {
+  const long long r = blockIdx.x * static_cast<long long>(kThreads) + threadIdx.x;
+  if (r >= n) return;
+  uint32_t word = 0;
+  for (int k = 0; k < g.kv; ++k) word |= (__ldg(&rm[r * kvp + k]) >= 0 ? 1u : 0u) << g.key_pos[k];
+  keys[r] = gray_decode(word);
+}
+
 // keys[i] = words[rows[i], w] & and_mask ; rows == nullptr means identity.
 __global__ void __launch_bounds__(kThreads)
 gather_mask_word_kernel(const uint32_t* __restrict__ words, const int32_t* __restrict__ rows,
@@ -2257,6 +2267,17 @@ extern "C" int spc_rowmajor_to_pairs(const int32_t* rowmajor, int kv, int64_t n,
   rowmajor_to_pairs_kernel<<<grid, dim3(32, 8), 0, static_cast<cudaStream_t>(stream)>>>(rowmajor, kv, kvp, n, pairs);
   SPC_LAUNCH_OK();
   return SPC_OK;
+}
+
+extern "C" int spc_rowmajor_order(const spc_geometry* sg, const int32_t* rowmajor, int64_t n, int32_t* order, uint32_t* keys, void* stream) {
+  Geo g;
+  if (!make_geo(sg, &g) || !rowmajor || !order || !keys || n < 0) return fail(SPC_ERR_INVALID_ARGUMENT, "rowmajor_order: bad arguments");
+  if (g.kv > 32 || tile_order_needs_buckets(n)) return fail(SPC_ERR_UNSUPPORTED, "rowmajor_order: %d offsets, %lld rows", g.kv, static_cast<long long>(n));
+  if (n == 0) return SPC_OK;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  rowmajor_keys_kernel<<<blocks_for(n), kThreads, 0, st>>>(g, rowmajor, (g.kv + 3) & ~3, n, keys);
+  SPC_LAUNCH_OK();
+  return tile_order(keys, n, g.kv, nullptr, nullptr, order, st);
 }
 
 extern "C" int spc_native_to_tables(const int32_t* pair, int kv, int64_t n_pair, int inverse,

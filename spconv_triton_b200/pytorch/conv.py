@@ -334,8 +334,7 @@ class SparseConvolutionBase:
         # training reads column-major tables for the weight gradient, and layers too narrow for the tensor
         # cores read them in the forward direction
         colmajor = training or self.in_channels % 16 != 0 or self.out_channels % 16 != 0
-        # an fp32 layer of few rows wants no row order (layers that share its rulebook may: at 32 tiles 9 us of sorting
-        # against 4 us a layer)
+        # an fp32 layer of few rows wants no row order (9 us of sorting); a layer on its rulebook that does has it made
         rows = indices.shape[0]
         small = (self.subm and rows <= 4096 and self.weight.dtype == torch.float32 and not constants.SPCONV_ALLOW_TF32
                  and not torch.is_autocast_enabled()

@@ -71,3 +71,49 @@ def test_layers_that_share_the_rulebook(tf32, monkeypatch):
     with torch.autocast("cuda", dtype=torch.float16):
         half = small(t.replace_feature(x)).features
     assert half.dtype == torch.float16
+
+
+@pytest.mark.parametrize("rows", [257, 1024, 1025, 4096])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_a_wide_layer_gets_its_row_order(rows, dtype):
+    """... also on the rulebook of a small one, and the same: its results have the bits of a rulebook of its own."""
+    gen = torch.Generator().manual_seed(rows)
+    cells = torch.randperm(32 ** 3, generator=gen)[:rows]
+    idx = torch.stack([torch.zeros_like(cells), cells // 1024, cells // 32 % 32, cells % 32], 1).int().cuda()
+    x = sp.SparseConvTensor(torch.randn(rows, 16, generator=gen).cuda(), idx, [32] * 3, 1)
+    small, wide = sp.SubMConv3d(16, 16, 3, indice_key="a").cuda(), sp.SubMConv3d(128, 128, 3, indice_key="a").cuda().to(dtype)
+    f = torch.randn(rows, 128, generator=gen).cuda().to(dtype)
+    lib, launches = _lib.load(), []
+    own = wide(x.replace_feature(f)).features
+    shared = small(x)
+    for _ in range(2):
+        before = lib.spc_launch_count()
+        assert torch.equal(wide(shared.replace_feature(f)).features, own)
+        launches.append(lib.spc_launch_count() - before)
+    assert launches[0] == launches[1] + 2  # (keys and sort, once)
+
+
+def test_row_order_of_a_table():
+    """Made later it is the order that the tables come with; more rows than one CTA sorts are refused."""
+    from spconv_triton_b200.pytorch._impl import host
+
+    geo = host.geometry(1, (24,) * 3, (3,) * 3, (1,) * 3, (1,) * 3, (1,) * 3, (0,) * 3, True, False)[0]
+    cells = torch.randperm(24 ** 3, generator=torch.Generator().manual_seed(0))[:8193]
+    idx = torch.stack([torch.zeros_like(cells), cells // 576, cells // 24 % 24, cells % 24], 1).int().cuda()
+    lib, stream = _lib.load(), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    g = _lib.make_geometry(1, [24] * 3, [24] * 3, [3] * 3, [1] * 3, [1] * 3, [1] * 3, True, False)
+    for n in (1, 31, 2048, 8192, 8193):
+        at = idx[:n].contiguous()
+        rm = host.ext().build_rulebook(geo, at, False, False, False).rowmajor(False)
+        order, keys = torch.full((n,), -1, dtype=torch.int32, device="cuda"), torch.empty(n, dtype=torch.int32, device="cuda")
+        rc = lib.spc_rowmajor_order(ctypes.byref(g), _p(rm), n, _p(order), _p(keys), stream)
+        if n > 8192:
+            assert rc == _lib.SPC_ERR_UNSUPPORTED
+            continue
+        assert rc == 0
+        ws = torch.empty(lib.spc_rulebook_workspace_bytes(ctypes.byref(g), n), dtype=torch.uint8, device="cuda")
+        n_out, want, table = ctypes.c_int64(), torch.empty_like(order), torch.empty_like(rm)
+        assert lib.spc_rulebook_prepare(ctypes.byref(g), _p(at), n, _p(ws), ws.numel(), ctypes.byref(n_out), stream) == 0
+        assert lib.spc_rulebook_tables(ctypes.byref(g), _p(at), n, n, _p(ws), ws.numel(), None, None, _p(table), _p(want), None, None, None,
+                                       stream) == 0
+        assert torch.equal(order, want) and torch.equal(table, rm)
