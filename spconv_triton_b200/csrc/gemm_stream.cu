@@ -508,14 +508,28 @@ int launch(const StreamParams& p, int a_row_bytes, const CUtensorMap& map_b, int
 }  // namespace
 
 // Rows of one stage, 16-bit, both accumulators of two CTAs in tensor memory, and tiles enough that a CTA takes several:
-// with few, four small CTAs of gemm_tma.cu a multiprocessor are done before the second tile of a long one.  Measured (us, that
-// kernel / this one): 64 -> 128 strided, 96 k rows 29 / 32, 178 k 43 / 39, 287 k 64 / 51, 554 k 117 / 84; 64 -> 64 with 13 stages
-// a tile, 168 k 53 / 60, 353 k 98 / 100, 523 k 141 / 135; 64 -> 64 with 8, 329 k 78 / 84, 443 k 102 / 103; 32 -> 32 with 7,
-// 193 k 31 / 35, 373 k 51 / 48; 32 -> 64 with 4, 269 k 41 / 43, 523 k 70 / 61.
+// with few, four small CTAs of gemm_tma.cu a multiprocessor are done before the second tile of a long one, the later the less a
+// row is (its channels in and out).  Measured (us, that kernel / this one; neighbours a row of a submanifold layer, strided
+// layers by their stages a tile):
+//   64 -> 128   180 k rows, 1.8 neighbours  46 / 46    7.5   85 /  81    27  106 / 103     strided, 1.4:  197 k  43 / 34
+//               205 k                       53 / 53          97 /  94        122 / 116              2:  186 k  50 / 56
+//               260 k                       66 / 57         122 / 119        148 / 143                  243 k  66 / 64
+//   64 ->  96   180 k                       34 / 37          69 /  62         85 /  79                  186 k  38 / 43
+//               205 k                       41 / 41          79 /  71         92 /  87                  243 k  52 / 50
+//   32 -> 128   230 k                       38 / 39          62 /  57         83 /  76                  236 k  36 / 38
+//               400 k                       61 / 62         106 /  91        138 / 123                  385 k  56 / 57
+//   64 ->  64   390 k                       59 / 54         120 / 117        149 / 151
+//               700 k                      101 / 96         211 / 205        256 / 252
+//   32 ->  64   390 k                       48 / 43          84 /  72        109 /  94
+//   32 ->  32   390 k                       42 / 39          71 /  68         87 /  87
+//               700 k                       72 / 67         123 / 113        149 / 154
+//   16 ->  16   390 k                       36 / 32          55 /  52         73 /  69
+// Input gradients (the weight read transposed), outputs and reduction as above: 64 -> 128 at 205 k rows 54 / 55, 103 / 101,
+// 129 / 125; 64 -> 64 at 390 k 59 / 54, 123 / 122, 153 / 155; 32 -> 32 at 390 k 43 / 40, 73 / 72, 92 / 93.
 bool gather_gemm_stream_takes(int n_dim, int r_dim, long long m_rows, int dtype) {
   if (dtype != SPC_F16 && dtype != SPC_BF16) return false;
   if (r_dim * 2 != row_span(r_dim, 2) || n_dim > 128 || m_rows >= (1ll << 31) - kTileM) return false;
-  return ceil_div(m_rows, kTileM) >= (n_dim > 64 ? 8ll : 20ll) * sm_count();
+  return ceil_div(m_rows, kTileM) >= (n_dim > 64 && r_dim == 64 ? 11ll : 20ll) * sm_count();
 }
 
 int gather_gemm_stream(const void* src, const void* w, const Epilogue& epi, const int32_t* pairs, const int32_t* pairs_rowmajor,
@@ -535,10 +549,10 @@ int gather_gemm_stream(const void* src, const void* w, const Epilogue& epi, cons
   p.acc_cols = 32;
   while (p.acc_cols < n_dim) p.acc_cols <<= 1;
   p.tmem_cols = kAccs * p.acc_cols;
-  // one wave of two CTAs a multiprocessor
+  // One wave of two CTAs a multiprocessor, all of them: a CTA that takes a tile less ends with the shortest ones.  (As few CTAs
+  // as end with the same number of tiles left a part of the chip with one CTA: 64 -> 96, 190 k rows, 74 us and 91 for 68 and 84.)
   const int ctas = 2;
-  const int each = static_cast<int>(ceil_div(p.tiles, static_cast<int64_t>(ctas) * sm_count()));
-  const int grid = static_cast<int>(ceil_div(p.tiles, each));
+  const int grid = static_cast<int>(std::min<int64_t>(p.tiles, static_cast<int64_t>(ctas) * sm_count()));
   const int row_bytes = n_dim * (out_dtype == SPC_F32 ? 4 : 2);
   p.epi_bytes = 128;
   while (p.epi_bytes > 32 && p.epi_bytes / 2 >= row_bytes) p.epi_bytes /= 2;
