@@ -495,16 +495,16 @@ struct NormActBackward : public torch::autograd::Node {
     std::lock_guard<std::mutex> hold(mutex_);
     variable_list out(3);
     if (!grads[0].defined()) return out;
-    const Tensor x = x_.unpack(), weight = weight_.unpack(), bias = bias_.unpack();
+    const Tensor saved_x = x_.unpack(), saved_weight = weight_.unpack(), saved_bias = bias_.unpack();
     TORCH_CHECK(mean.defined(), torch::autograd::ERR_BACKWARD_TWICE);
     c10::cuda::CUDAGuard guard(grads[0].device());
     if (at::GradMode::is_enabled()) {
       // Gradients that are to be differentiated themselves: those of torch's functions of the same operands.
-      const Tensor z = at::batch_norm(x, weight, bias, Tensor(), Tensor(), true, 0.0, eps, false);
+      const Tensor z = at::batch_norm(saved_x, saved_weight, saved_bias, Tensor(), Tensor(), true, 0.0, eps, false);
       const Tensor y = act == SPC_NORM_SILU ? at::silu(z) : act == SPC_NORM_RELU ? at::relu(z) : z;
       variable_list wanted;
       std::vector<int> at;
-      const Tensor operands[3] = {x, weight, bias};
+      const Tensor operands[3] = {saved_x, saved_weight, saved_bias};
       for (int i = 0; i < 3; ++i)
         if (task_should_compute_output(i) && operands[i].defined()) {
           wanted.push_back(operands[i]);
@@ -515,8 +515,12 @@ struct NormActBackward : public torch::autograd::Node {
       for (size_t i = 0; i < at.size(); ++i) out[at[i]] = found[i];
       return out;
     }
-    Tensor dy = grads[0].scalar_type() == x.scalar_type() ? grads[0] : grads[0].to(x.scalar_type());
+    Tensor dy = grads[0].scalar_type() == saved_x.scalar_type() ? grads[0] : grads[0].to(saved_x.scalar_type());
     dy = operand(dy);
+    // (a hook of saved tensors may give back other strides than it was given)
+    const Tensor x = operand(saved_x);
+    const Tensor weight = saved_weight.defined() ? saved_weight.contiguous() : saved_weight;
+    const Tensor bias = saved_bias.defined() ? saved_bias.contiguous() : saved_bias;
     Tensor dx, dweight, dbias;
     if (task_should_compute_output(0)) dx = at::empty_like(x);
     if (weight.defined() && task_should_compute_output(1)) dweight = at::empty_like(weight);
@@ -675,10 +679,10 @@ struct PoolBackward : public torch::autograd::Node {
     if (!grads[0].defined() || !task_should_compute_output(0)) return result;
     Tensor features, out, count;
     if (average) {
-      count = count_.unpack();
+      count = count_.unpack().contiguous();  // (a hook of saved tensors may give back other strides than it was given)
     } else {
-      features = features_.unpack();
-      out = out_.unpack(shared_from_this());
+      features = features_.unpack().contiguous();
+      out = out_.unpack(shared_from_this()).contiguous();
     }
     const bool create_graph = at::GradMode::is_enabled();
     at::AutoGradMode no_grad(false);

@@ -208,3 +208,34 @@ def test_saved_tensor_hooks_and_changes_in_place():
     y.sum().backward()
     with pytest.raises(RuntimeError):
         y.sum().backward()
+
+
+@pytest.mark.parametrize("start", [0, 1])
+def test_saved_tensors_come_back_with_other_strides(start):
+    """... or from another address; nets of a convolution, a normalisation and each pooling."""
+
+    def other(t):  # the same values, columns first, or starting off a 16-byte boundary
+        if not t.is_floating_point():
+            return t.clone()
+        if start:
+            room = torch.empty(t.numel() + start, dtype=t.dtype, device=t.device)
+            room[start:].copy_(t.reshape(-1))
+            return room[start:].view(t.shape)
+        return t.reshape(len(t), -1).t().contiguous().t().reshape(t.shape) if t.dim() == 2 else torch.stack([t, t], -1)[..., 0]
+
+    gen = torch.Generator().manual_seed(2)
+    cells = torch.randperm(16 ** 3, generator=gen)[:900]
+    idx = torch.stack([torch.zeros_like(cells), cells // 256, cells // 16 % 16, cells % 16], 1).int().cuda()
+    f = torch.randn(900, 16, generator=gen).cuda().requires_grad_()
+    torch.manual_seed(0)
+    for pool in (sp.SparseMaxPool3d, sp.SparseAvgPool3d):
+        net = sp.SparseSequential(sp.SubMConv3d(16, 32, 3), nn.BatchNorm1d(32), nn.SiLU(), pool(2, 2)).cuda()
+
+        def grads():
+            y = net(sp.SparseConvTensor(f, idx, [16] * 3, 1)).features
+            return torch.autograd.grad(y, [f, *net.parameters()], torch.ones_like(y))
+
+        want = grads()
+        with torch.autograd.graph.saved_tensors_hooks(other, lambda t: t):
+            got = grads()
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
