@@ -52,7 +52,7 @@ struct StreamParams {
   void* out;
   int m_rows, tiles;
   int kvp;
-  int n_dim, r_dim, kv;
+  int n_dim, kv;
   int reversed;  // offset k of the table meets weight kv - 1 - k
   int stages, a_stage_bytes, b_stage_bytes;
   int copiers;     // copy warps at work: no more than there are stages (a slot's last round but one must be over)
@@ -104,7 +104,6 @@ __global__ void __launch_bounds__(kThreads, 2)
 gather_gemm_stream_kernel(const __grid_constant__ StreamParams p, const __grid_constant__ CUtensorMap map_b) {
   constexpr int ELEM = sizeof(T);
   constexpr int UMMA_K = 32 / ELEM;
-  constexpr bool TF32 = TcType<T>::tf32;
   constexpr int A_ROW_BYTES = 16 * LPR;
   constexpr int EPR = A_ROW_BYTES / ELEM;    // reduction elements
   constexpr int kRowsPass = 32 / LPR;        // rows that one copy per lane covers: 4, 8, 16
@@ -447,7 +446,7 @@ gather_gemm_stream_kernel(const __grid_constant__ StreamParams p, const __grid_c
             for (int ks = 0; ks < KSTEPS; ++ks) {
               const uint64_t a_desc = (static_cast<uint64_t>(a_hi) << 32) | (a_lo + 2u * ks);
               const uint64_t b_desc = (static_cast<uint64_t>(b_hi) << 32) | (b_lo + b_step * ks);
-              tc_mma<TF32>(tmem_d, a_desc, b_desc, idesc, accumulate);
+              tc_mma</*TF32=*/false>(tmem_d, a_desc, b_desc, idesc, accumulate);
               accumulate = 1;
             }
             tc_commit(empty);
@@ -539,7 +538,7 @@ int gather_gemm_stream(const void* src, const void* w, const Epilogue& epi, cons
   p.src = src; p.epi = epi; p.pairs = pairs; p.pairs_rm = pairs_rowmajor; p.kvp = (kv + 3) & ~3; p.order = order; p.out = out;
   p.m_rows = static_cast<int>(m_rows);
   p.tiles = static_cast<int>(ceil_div(m_rows, kTileM));
-  p.n_dim = n_dim; p.r_dim = r_dim; p.kv = kv; p.reversed = reversed;
+  p.n_dim = n_dim; p.kv = kv; p.reversed = reversed;
   const int a_row_bytes = 2 * r_dim;
   p.b_row_bytes = transposed_weight ? row_span(n_dim, 2) : a_row_bytes;
   p.a_stage_bytes = static_cast<int>(align_up(static_cast<size_t>(kTileM) * a_row_bytes, 1024));

@@ -71,7 +71,6 @@ struct TmaParams {
   void* out;
   long long m_rows;
   int kvp;
-  int src_rows;  // rows of the gathered matrix; also the "absent row" index
   int n_dim, r_dim, kv;
   int reversed;  // offset k of the table meets weight kv - 1 - k
   int stages, a_stage_bytes, b_stage_bytes, tmem_cols;
@@ -500,7 +499,7 @@ int gather_gemm_tma(const void* src, const void* w, const Epilogue& epi, const i
 
   TmaParams p{};
   p.src = src; p.epi = epi; p.pairs = pairs; p.pairs_rm = pairs_rowmajor; p.kvp = (kv + 3) & ~3; p.order = order; p.out = out;
-  p.m_rows = m_rows; p.src_rows = static_cast<int>(src_rows);
+  p.m_rows = m_rows;
   p.n_dim = n_dim; p.r_dim = r_dim; p.kv = kv; p.reversed = reversed;
   p.a_row_bytes = row_span(r_dim, elem);
   p.b_row_bytes = transposed_weight ? row_span(n_dim, elem) : p.a_row_bytes;
