@@ -348,16 +348,16 @@ wgrad_f32_kernel(const float* __restrict__ feats, const float* __restrict__ gout
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // Few rows (the rule is at gather_gemm_small_takes): a tile of 64 or 128 rows is one chain of up to 27 offsets on a chip that
-// is nearly empty.  Here a CTA has eight rows, 16 lanes a row, and passes over the offsets that any of them has: the weights
-// of an offset (read by neighbouring lanes, whichever way they are transposed) and the rows that have it come by cp.async,
-// two offsets ahead, and a row's lanes multiply, NC output channels each, if the row has the offset.
-// Bound: latency: 1 - 1.5 us from the launch to the first stage, then 0.4 us an offset (copies, barrier, multiplications) with
-// one or two CTAs a multiprocessor.  Measured beside the rule.
+// is nearly empty.  Here a CTA has eight rows, 16 lanes a row, and passes over the offsets that any of them has, a batch of
+// them at a time: the weights of each (read by neighbouring lanes, whichever way they are transposed) and the rows that have
+// it come by cp.async while the batch before is multiplied, by a row's lanes, NC output channels each, for the offsets that
+// the row has.
+// Bound: latency, of the table entries, then of the copies, then of the multiplications of a row.  Measured beside the rule.
 constexpr int kSmallRows = kThreads / 16;
 // Floats between staged rows: whole 16-byte words, an odd number of them, so that lanes on neighbouring rows meet different banks.
 __host__ __device__ constexpr int small_pitch(int floats) { return ((floats >> 2) | 1) << 2; }
-constexpr int kSmallStages = 3;  // (four and eight: the same)
-constexpr int kSmallMostBytes = kSmallStages * (64 + kSmallRows) * small_pitch(64) * static_cast<int>(sizeof(float));
+constexpr int kSmallBatchBytes = 40 * 1024, kSmallMostBatch = 8;  // of the offsets of a batch (two such buffers)
+static_assert((64 + kSmallRows) * small_pitch(64) * sizeof(float) <= kSmallBatchBytes, "an offset at least");
 
 __device__ __forceinline__ void copy16(uint32_t to, const float* from) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(from) : "memory");
@@ -365,8 +365,8 @@ __device__ __forceinline__ void copy16(uint32_t to, const float* from) {
 
 template <bool W_MN, int NC>  // NC: output channels of a lane
 __global__ void __launch_bounds__(kThreads)
-gather_gemm_small_kernel(const __grid_constant__ F32Params p) {
-  extern __shared__ __align__(16) float small_stages[];
+gather_gemm_small_kernel(const __grid_constant__ F32Params p, int batch_most) {
+  extern __shared__ __align__(16) float small_stages[];  // [2][batch_most] stages
   __shared__ __align__(16) int entries[kSmallRows][32];
   __shared__ uint32_t votes[kThreads / 32];
   const int group = threadIdx.x >> 4, lane = threadIdx.x & 15;
@@ -399,63 +399,65 @@ gather_gemm_small_kernel(const __grid_constant__ F32Params p) {
   const uint32_t stages = static_cast<uint32_t>(__cvta_generic_to_shared(small_stages));
   const uint32_t w_to = 4 * (group * w_pitch + 4 * lane), x_to = 4 * (x_at + 4 * lane);
   const bool w_lane = 4 * lane < w_cols, x_lane = 4 * lane < p.r_dim;
+  const uint32_t stage_bytes = 4 * stage_floats;
   uint32_t ahead = all;  // offsets that have not been asked for
-  uint32_t to = stages;
-  const uint32_t stage_bytes = 4 * stage_floats, end = stages + kSmallStages * stage_bytes;
-  const auto fetch_next = [&] {
-    if (ahead != 0) {
+  // The next offsets, into one half of the stages in ascending order.
+  const auto fetch = [&](int half) {
+    const uint32_t before = ahead;
+    uint32_t to = stages + half * batch_most * stage_bytes;
+#pragma unroll 2
+    for (int j = 0; j < batch_most && ahead != 0; ++j, to += stage_bytes) {
       const int kk = __ffs(ahead) - 1, k = p.reversed ? p.kv - 1 - kk : kk;
       ahead &= ahead - 1;
+      const int entry = entries[group][kk];
       if (w_lane) {
         const float* from = w_from + k * w_cols;
         uint32_t there = to + w_to;
 #pragma unroll 4
         for (int i = group; i < w_rows; i += kSmallRows, from += w_step, there += 4 * kSmallRows * w_pitch) copy16(there, from);
       }
-      if (x_lane && (mine >> kk & 1u)) copy16(to + x_to, x_from + static_cast<long long>(entries[group][kk]) * p.r_dim);
+      if (x_lane && entry >= 0) copy16(to + x_to, x_from + static_cast<long long>(entry) * p.r_dim);
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");  // (empty ones too: the wait below counts them)
-    to += stage_bytes;
-    if (to == end) to = stages;
+    return before ^ ahead;
   };
-#pragma unroll 1
-  for (int s = 0; s < kSmallStages - 1; ++s) fetch_next();
 
   float acc[NC];
 #pragma unroll
   for (int c = 0; c < NC; ++c) acc[c] = 0.f;
-  int at = 0;
+  uint32_t next = fetch(0);
 #pragma unroll 1
-  for (uint32_t rest = all; rest != 0; rest &= rest - 1) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(kSmallStages - 2) : "memory");
-    __syncthreads();  // this stage is there for everyone, and everyone is done with the one that is filled next
-    fetch_next();
-    const float* const stage = small_stages + at * stage_floats;
-    at = at + 1 == kSmallStages ? 0 : at + 1;
-    if (!(mine >> (__ffs(rest) - 1) & 1u)) continue;
-    const float4* const x = reinterpret_cast<const float4*>(stage + x_at);
+  for (int half = 0; next != 0; half ^= 1) {
+    const uint32_t batch = next;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();  // this batch is there for everyone, and everyone is done with the one before it
+    next = fetch(half ^ 1);
+#pragma unroll 1
+    for (uint32_t rest = batch & mine; rest != 0; rest &= rest - 1) {
+      const float* const stage = small_stages + (half * batch_most + __popc(batch & ((rest & -rest) - 1u))) * stage_floats;
+      const float4* const x = reinterpret_cast<const float4*>(stage + x_at);
 #pragma unroll 4
-    for (int r = 0; r < p.r_dim; r += 4) {
-      const float4 a = x[r >> 2];
-      float b[4][NC];
-      if (W_MN) {
+      for (int r = 0; r < p.r_dim; r += 4) {
+        const float4 a = x[r >> 2];
+        float b[4][NC];
+        if (W_MN) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
+          for (int q = 0; q < 4; ++q)
 #pragma unroll
-          for (int c = 0; c < NC; ++c) b[q][c] = stage[(r + q) * w_pitch + lane + 16 * c];
-      } else {
+            for (int c = 0; c < NC; ++c) b[q][c] = stage[(r + q) * w_pitch + lane + 16 * c];
+        } else {
+#pragma unroll
+          for (int c = 0; c < NC; ++c) {
+            const float4 v = *reinterpret_cast<const float4*>(stage + (lane + 16 * c) * w_pitch + r);
+            b[0][c] = v.x; b[1][c] = v.y; b[2][c] = v.z; b[3][c] = v.w;
+          }
+        }
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
-          const float4 v = *reinterpret_cast<const float4*>(stage + (lane + 16 * c) * w_pitch + r);
-          b[0][c] = v.x; b[1][c] = v.y; b[2][c] = v.z; b[3][c] = v.w;
+          acc[c] = fmaf(a.x, b[0][c], acc[c]);
+          acc[c] = fmaf(a.y, b[1][c], acc[c]);
+          acc[c] = fmaf(a.z, b[2][c], acc[c]);
+          acc[c] = fmaf(a.w, b[3][c], acc[c]);
         }
-      }
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        acc[c] = fmaf(a.x, b[0][c], acc[c]);
-        acc[c] = fmaf(a.y, b[1][c], acc[c]);
-        acc[c] = fmaf(a.z, b[2][c], acc[c]);
-        acc[c] = fmaf(a.w, b[3][c], acc[c]);
       }
     }
   }
@@ -473,10 +475,11 @@ template <bool W_MN, int NC>
 int launch_small(const F32Params& p, cudaStream_t st) {
   const int w_rows = W_MN ? p.r_dim : p.n_dim, w_cols = W_MN ? p.n_dim : p.r_dim;
   const size_t stage_bytes = (static_cast<size_t>(w_rows) * small_pitch(w_cols) + kSmallRows * small_pitch(p.r_dim)) * sizeof(float);
+  const int batch = std::min(kSmallMostBatch, static_cast<int>(kSmallBatchBytes / stage_bytes));
   static bool configured[kMaxDevices] = {false};  // per instantiation and device
-  SPC_CUDA_OK(ensure_dynamic_smem(gather_gemm_small_kernel<W_MN, NC>, kSmallMostBytes, configured));
+  SPC_CUDA_OK(ensure_dynamic_smem(gather_gemm_small_kernel<W_MN, NC>, 2 * kSmallBatchBytes, configured));
   gather_gemm_small_kernel<W_MN, NC>
-      <<<static_cast<unsigned>(ceil_div(p.m_rows, kSmallRows)), kThreads, kSmallStages * stage_bytes, st>>>(p);
+      <<<static_cast<unsigned>(ceil_div(p.m_rows, kSmallRows)), kThreads, 2 * batch * stage_bytes, st>>>(p, batch);
   SPC_LAUNCH_OK();
   return SPC_OK;
 }
@@ -486,14 +489,14 @@ int launch_small(const F32Params& p, cudaStream_t st) {
 // 16, 32, 48 or 64 output channels, 12 to 64 reduction channels in steps of four, one table word of offsets, and at most 2 M
 // row-channel-channel products an offset, where the tiles catch up.  Layer of 27 offsets, its rulebook there, forward / input
 // gradient in us, the tensor cores (with their operands' copies and a row order) -> this kernel; and lanes that read rows and
-// weights through the caches, each lane its own channel's weights (16 lines a load), which this one replaces:
+// weights through the caches, each lane its own channel's weights (16 lines a load), which this kernel replaces:
 //     channels, rows      1.2 neighbours a row                                20 - 26 neighbours a row
-//     16 -> 16,  2 000   19.0 / 18.8 ->  6.1 /  5.7    4.1 /  9.0            24.0 / 23.8 -> 14.3 / 14.3    16 /  54
-//     16 -> 16,  8 192   19.2 / 19.2 ->  6.4 /  6.1    5.3 /  9.2            24.5 / 24.3 -> 24.7 / 24.3    32 /  43
-//     16 -> 64,  2 048   21.2 / 51.1 ->  6.7 /  9.2    6.7 / 26.9            26.9 / 84.5 -> 21.4 / 27.3    37 / 187
-//     32 -> 32,  2 048   28.9 / 29.6 ->  6.9 /  7.4    7.7 /  9.8            39.9 / 40.8 -> 21.7 / 21.8    60 /  58
-//     48 -> 48,    900   49.8 / 45.0 ->  8.1 /  7.4    9.4 / 18.3            77.6 / 70.7 -> 27.6 / 24.9    51 /  91
-//     64 -> 64,    512   81.0 / 72.4 -> 10.2 / 13.0   18.1 / 27.6            93.7 / 84.6 -> 30.3 / 37.1   131 / 151
+//     16 -> 16,  2 000   18.8 / 18.7 ->  4.7 /  4.5    4.1 /  9.0            24.0 / 23.8 -> 12.5 / 13.0    16 /  54
+//     16 -> 16,  8 192   19.1 / 19.2 ->  5.2 /  5.1    5.3 /  9.2            24.4 / 24.4 -> 21.5 / 24.8    32 /  43
+//     16 -> 64,  2 048   20.7 / 50.5 ->  5.5 /  6.8    6.7 / 26.9            26.9 / 84.5 -> 19.0 / 27.7    37 / 187
+//     32 -> 32,  2 048   28.4 / 29.3 ->  5.4 /  5.7    7.7 /  9.8            40.0 / 40.8 -> 19.4 / 23.4    60 /  58
+//     48 -> 48,    900   49.7 / 45.2 ->  6.8 /  7.0    9.4 / 18.3            77.8 / 70.6 -> 26.2 / 28.2    51 /  91
+//     64 -> 64,    512   81.0 / 72.1 ->  8.7 / 10.0   18.1 / 27.6            93.5 / 84.1 -> 30.6 / 35.2   131 / 151
 bool gather_gemm_small_takes(long long m_rows, int n_dim, int r_dim, int kv) {
   return kv <= 32 && n_dim % 16 == 0 && n_dim <= 64 && r_dim % 4 == 0 && r_dim > 8 && r_dim <= 64 && m_rows * n_dim * r_dim <= (2ll << 20);
 }
