@@ -19,17 +19,16 @@
 // are bounded; after one has run out a warp leaves its loop, the others' waits run out in turn, and everything in flight
 // is awaited before tensor memory goes back.
 //
-// Measured (one B200, us, L2 cold; the kernel of one tile a CTA in gemm_tma.cu -> this one): strided 64 -> 128, 1.36 M rows with
-// 1.4 stages a tile 289 -> 213; 32 -> 64, 1.47 M rows 154 -> 139; 64 -> 64 submanifold, 384 k rows with 1.3 stages
-// 53 -> 48, 716 k rows with 12.5 stages 195 -> 178, 443 k with 17.6: 143 -> 141.  Wider rows stay there: with several
-// stages an offset the multiplications cover the chain, and two accumulators cost the third CTA or stage (128 -> 128 on
-// 74 k rows 33 -> 52).
+// Measured (one B200, us, alone, L2 cold; the kernel of one tile a CTA in gemm_tma.cu -> this one): strided 64 -> 128, 1.36 M
+// rows with 1.4 stages a tile 289 -> 213; 32 -> 64, 1.47 M rows 154 -> 139; other sizes beside the rule at the end.  Wider rows
+// stay there: with several stages an offset the multiplications cover the chain, and two accumulators cost the third CTA or
+// stage (128 -> 128 on 74 k rows 33 -> 52).
 //
 // Measured and dropped: tables and epilogue by the same warps (57 -> 84 us at 64 -> 64: one chain again, and 32 unrolled
 // offsets a tile are more instructions than the fetch keeps up with); table entries copied row by row with cp.async and
 // read from there, stores by warps of their own (178 -> 227: a copy thread then reads an entry a row instead of four at once);
 // stores by cp.async.bulk (about 48 cycles per row and multiprocessor); fewer table warps and more copy warps (equal or
-// slower); two waves of CTAs instead of one (+ 2 - 5 %); test_wait or nanosleep instead of try_wait (+ 5 %).
+// slower); two waves of CTAs instead of one (+ 2 - 5 % of the kernel alone); test_wait or nanosleep instead of try_wait (+ 5 %).
 // A tcgen05.ld waits for the global stores that its warp has under way (17 -> 250 cycles on an idle chip, over 1 000 on a
 // busy one), which is what is left of the epilogue of rows wider than its 128-byte passes.
 #include <algorithm>
@@ -95,7 +94,8 @@ __device__ __forceinline__ float4 lds4(uint32_t at) {
 }
 
 // Offsets whose table entries go through shared memory together: a whole 3 x 3 x 3 kernel where the stages are small, half of
-// it where the room is a stage more (64 -> 128: 235 -> 213 us; 32 -> 64: 139 against 152).
+// it where the room is a stage more (the strided 64 -> 128 above: 235 us with whole kernels, 213 with halves; 32 -> 64: 139 whole,
+// 152 halves).
 __host__ __device__ constexpr int table_group(int lanes_per_row) { return lanes_per_row == 8 ? 16 : 32; }
 
 // LPR: lanes per row = 16-byte pieces of one A row in a stage (8, 4 or 2 for rows of 128, 64 or 32 bytes).
