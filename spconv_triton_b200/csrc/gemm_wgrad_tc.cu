@@ -445,10 +445,13 @@ WgradSplit wgrad_tc_split(int64_t n_out, int c_in, int c_out, int kv) {
   //   27, 45 k           40 /  40 /  67   46 /  48 /  71   58 /  56 /  83   93 /  61 /  85  276 / 163 / 130
   //   27, 150 k          81 /  81 /  77   95 /  95 /  87  119 / 119 / 106  177 / 177 / 142  489 / 486 / 359
   //   125, 40 k          89 /  89 /  79  105 / 104 /  89  138 / 138 / 108  212 / 212 / 148  622 / 622 / 400
-  // Entries: 0.27, 1.25, 1.2, 4.1 and 5 million; the lines lie between the rows where the better side changes.
+  // Entries: 0.27, 1.25, 1.2, 4.1 and 5 million; the lines lie between the rows where the better side changes.  Where few of the
+  // entries are pairs, the centre's chain is all there is to narrow layers: 100 k rows with 1.5 neighbours, 2048 / 4096, 16 -> 16
+  // 30 / 49, 64 -> 64 39 / 56, 64 -> 128 55 / 73 (128 -> 128, with 4096, 86); so these stay at 2048, a tenth behind in full scenes.
   const int64_t entries = n_out * kv, sums = static_cast<int64_t>(c_in) * c_out;
-  const int64_t few = sums <= 64 * 128 ? 1250000 : 400000, some = sums <= 128 * 128 ? 2400000 : 600000;
-  const int64_t by_len = std::max<int64_t>(1, n_out / (entries <= few ? 1024 : entries <= some ? 2048 : 4096));
+  const bool narrow = sums <= 64 * 128;
+  const int64_t few = narrow ? 1250000 : 400000, some = sums <= 128 * 128 ? 2400000 : 600000;
+  const int64_t by_len = std::max<int64_t>(1, n_out / (entries <= few ? 1024 : narrow || entries <= some ? 2048 : 4096));
   want = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(want, by_len), 64));
   s.splits = static_cast<int>(want);
   s.rows_per_split = ceil_div(std::max<int64_t>(n_out, 1), s.splits);
