@@ -242,17 +242,17 @@ constexpr int kListRows = 512;  // table entries compacted at a time
 // The reduction runs over pairs: a stage is 32 of them, 64 channels of both rows, copied as they lie.
 __global__ void __launch_bounds__(kThreads, 4)
 wgrad_f32_kernel(const float* __restrict__ feats, const float* __restrict__ gout, const int32_t* __restrict__ pair_fwd,
-                 float* __restrict__ partial, long long n_out, int c_in, int c_out, int kv, int splits, long long rows_per_split) {
+                 float* __restrict__ partial, long long n_out, int c_in, int c_out, int kv, int first_turn, int splits, long long rows_per_split) {
   __shared__ __align__(16) float g_s[2][kStep * kTile];
   __shared__ __align__(16) float f_s[2][kStep * kTile];
   __shared__ int list_i[kListRows], list_o[kListRows];
   __shared__ int warp_cnt[kListRows / 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int tx = tid & 15, ty = tid >> 4;
-  // the middle offsets first: they have the most pairs
-  const int turn = blockIdx.x / splits, split = blockIdx.x % splits;
+  // the middle offsets first, all channel blocks of one before the next: they have the most pairs
+  const int turn = first_turn + blockIdx.z / splits, split = blockIdx.z % splits;
   const int k = (turn & 1) ? (kv - 1) / 2 + (turn + 1) / 2 : (kv - 1) / 2 - turn / 2;
-  const int c0 = blockIdx.y * kTile, n0 = blockIdx.z * kTile;
+  const int c0 = blockIdx.x * kTile, n0 = blockIdx.y * kTile;
   const long long lo = split * rows_per_split, hi = min(n_out, lo + rows_per_split);
   const int32_t* col = pair_fwd + static_cast<long long>(k) * n_out;
   const int lp = tid >> 4, lc = (tid & 15) * 4;  // loader: sixteen lanes a pair, pairs lp, lp + 8, ..
@@ -552,10 +552,14 @@ WgradSplit wgrad_f32_split(int64_t n_out, int c_in, int c_out, int kv) {
 int wgrad_f32(const void* feats, const void* gout, const int32_t* pair_fwd, float* partial, int64_t n_out, int c_in, int c_out, int kv,
               const WgradSplit& s, cudaStream_t st) {
   if (!aligned16(feats) || !aligned16(gout)) return fail(SPC_ERR_UNSUPPORTED, "fp32 weight gradient: operands must be 16-byte aligned");
-  const dim3 grid(static_cast<unsigned>(kv * s.splits), static_cast<unsigned>(ceil_div(c_in, kTile)), static_cast<unsigned>(ceil_div(c_out, kTile)));
-  wgrad_f32_kernel<<<grid, kThreads, 0, st>>>(static_cast<const float*>(feats), static_cast<const float*>(gout), pair_fwd, partial, n_out, c_in,
-                                              c_out, kv, s.splits, s.rows_per_split);
-  SPC_LAUNCH_OK();
+  const int most = 65535 / s.splits;  // offsets of a launch
+  for (int turn = 0; turn < kv; turn += most) {
+    const dim3 grid(static_cast<unsigned>(ceil_div(c_in, kTile)), static_cast<unsigned>(ceil_div(c_out, kTile)),
+                    static_cast<unsigned>(std::min(most, kv - turn) * s.splits));
+    wgrad_f32_kernel<<<grid, kThreads, 0, st>>>(static_cast<const float*>(feats), static_cast<const float*>(gout), pair_fwd, partial, n_out,
+                                                c_in, c_out, kv, turn, s.splits, s.rows_per_split);
+    SPC_LAUNCH_OK();
+  }
   return SPC_OK;
 }
 

@@ -258,3 +258,27 @@ def test_first_calls_of_many_threads():
         runtime = next(line.split()[-1] for line in f if "libcudart.so" in line)
     for _ in range(6):
         subprocess.run([sys.executable, "-c", _FIRST_CALLS, str(LIB), runtime], check=True, timeout=60)
+
+
+@pytest.mark.parametrize("kv,c_in,c_out,n_out", [(66000, 12, 4, 3), (27, 132, 68, 2100)])
+def test_fp32_weight_gradient_of_many_offsets_and_blocks(kv, c_in, c_out, n_out):
+    """More offsets than a launch takes, several channel blocks with ragged edges, two splits."""
+    import ctypes
+
+    from spconv_triton_b200 import _lib
+
+    lib = _lib.load()
+    gen = torch.Generator(DEV).manual_seed(kv)
+    n_in = 50
+    x, g = torch.randn(n_in, c_in, generator=gen, device=DEV), torch.randn(n_out, c_out, generator=gen, device=DEV)
+    table = torch.randint(-1, n_in, (kv, n_out), generator=gen, device=DEV).int()
+    dw = torch.full((c_out, kv, c_in), float("nan"), device=DEV)
+    ws = torch.empty(lib.spc_conv_backward_weight_workspace_bytes(n_out, c_in, c_out, kv), dtype=torch.uint8, device=DEV)
+    p = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    assert lib.spc_conv_backward_weight(p(x), p(g), p(table), p(dw), p(ws), ws.numel(), n_in, n_out, c_in, c_out, kv, _lib.SPC_F32,
+                                        _lib.SPC_PREC_IEEE, 0, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    wide = torch.cat([x.double(), x.new_zeros(1, c_in).double()])
+    for k in range(0, kv, 1000):  # (index -1: the row of zeros)
+        f = wide[table[k:k + 1000].long()]
+        want, size = torch.einsum("mn,kmc->nkc", g.double(), f), torch.einsum("mn,kmc->nkc", g.double().abs(), f.abs())
+        assert ((dw[:, k:k + 1000].double() - want).abs() <= 2.0 ** -24 * (n_out + 4) * (size + 1e-30)).all()
