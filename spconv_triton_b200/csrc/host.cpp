@@ -600,7 +600,7 @@ c10::optional<Tensor> norm_act_train(const Tensor& x, const c10::optional<Tensor
 // each pair lies, and the argument of spc_fold_norms, which fills it; nothing where a tensor is not what the kernel takes.
 using Norm = std::tuple<Tensor, Tensor, c10::optional<Tensor>, c10::optional<Tensor>, double, int64_t>;
 using Places = std::vector<std::pair<int64_t, int64_t>>;
-c10::optional<std::tuple<Tensor, Places, pybind11::bytes>> norm_folds(const std::vector<Norm>& norms, const Tensor& like) {
+c10::optional<std::tuple<Tensor, Places, std::vector<spc_norm_fold>>> place_folds(const std::vector<Norm>& norms, const Tensor& like) {
   std::vector<spc_norm_fold> folds(norms.size());
   Places places(norms.size());
   int64_t total = 0;
@@ -636,7 +636,24 @@ c10::optional<std::tuple<Tensor, Places, pybind11::bytes>> norm_folds(const std:
     folds[i].scale = block.data_ptr<float>() + places[i].first;
     folds[i].shift = block.data_ptr<float>() + places[i].second;
   }
+  return std::make_tuple(block, std::move(places), std::move(folds));
+}
+c10::optional<std::tuple<Tensor, Places, pybind11::bytes>> norm_folds(const std::vector<Norm>& norms, const Tensor& like) {
+  auto placed = place_folds(norms, like);
+  if (!placed) return c10::nullopt;
+  auto& [block, places, folds] = *placed;
   return std::make_tuple(block, places, pybind11::bytes(reinterpret_cast<const char*>(folds.data()), folds.size() * sizeof(spc_norm_fold)));
+}
+// Scale and shift of one of them, made on the current stream.
+c10::optional<std::pair<Tensor, Tensor>> fold_norm(const Tensor& mean, const Tensor& var, const c10::optional<Tensor>& weight,
+                                                   const c10::optional<Tensor>& bias, double eps, int64_t c, const Tensor& like) {
+  const auto placed = place_folds({Norm{mean, var, weight, bias, eps, c}}, like);
+  if (!placed) return c10::nullopt;
+  const auto& [block, places, folds] = *placed;
+  at::NoGradGuard no_grad;
+  c10::cuda::CUDAGuard guard(like.device());
+  check(spc_fold_norms(folds.data(), 1, stream_of(like)));
+  return std::make_pair(block.narrow(0, places[0].first, c), block.narrow(0, places[0].second, c));
 }
 
 // ---- pooling -------------------------------------------------------------------------------------------------------
@@ -814,6 +831,7 @@ PYBIND11_MODULE(_host, m) {
   m.def("conv_eval", &conv_eval);
   m.def("norm_act_train", &norm_act_train);
   m.def("norm_folds", &norm_folds);
+  m.def("fold_norm", &fold_norm);
   // both directions of an IEEE fp32 layer run on the kernel for few rows
   m.def("small", [](int64_t rows, int c_out, int c_in, int kv) {
     return spc_conv_small(rows, c_out, c_in, kv) != 0 && spc_conv_small(rows, c_in, c_out, kv) != 0;

@@ -193,12 +193,12 @@ def _try_fold_bn_relu(mods, i, x):
     if x.benchmark or x.indices.shape[0] == 0:
         return None
     relu = i + 2 < len(mods) and type(mods[i + 2]) in (nn.ReLU, SparseReLU)
-    folded = _folded_norms([bn], x.features)
+    folded = _host.ext().fold_norm(*_bn_operands(bn), x.features)
     if folded is None:
-        return None
-    block, ((at, to),), _ = folded
-    c = bn.num_features
-    return conv(x, _fold=(block[at:at + c], block[to:to + c], relu)), i + 2 + int(relu)
+        folded = _folded_bn(bn)
+        if any(t.device != x.features.device or t.shape != (bn.num_features,) for t in folded):
+            return None
+    return conv(x, _fold=(*folded, relu)), i + 2 + int(relu)
 
 
 _HOOKS = ("_forward_hooks", "_forward_pre_hooks", "_backward_hooks", "_backward_pre_hooks")
