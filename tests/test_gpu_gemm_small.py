@@ -117,3 +117,25 @@ def test_row_order_of_a_table():
         assert lib.spc_rulebook_tables(ctypes.byref(g), _p(at), n, n, _p(ws), ws.numel(), None, None, _p(table), _p(want), None, None, None,
                                        stream) == 0
         assert torch.equal(order, want) and torch.equal(table, rm)
+
+
+def test_a_row_order_asked_for_under_capture():
+    """It belongs to the graph; a layer outside makes the rulebook's own."""
+    gen = torch.Generator().manual_seed(5)
+    cells = torch.randperm(32 ** 3, generator=gen)[:2000]
+    idx = torch.stack([torch.zeros_like(cells), cells // 1024, cells // 32 % 32, cells % 32], 1).int().cuda()
+    x = sp.SparseConvTensor(torch.randn(2000, 16, generator=gen).cuda(), idx, [32] * 3, 1)
+    small, wide = sp.SubMConv3d(16, 16, 3, indice_key="a").cuda(), sp.SubMConv3d(128, 128, 3, indice_key="a").cuda().half()
+    f = torch.randn(2000, 128, generator=gen).cuda().half()
+    with torch.no_grad():
+        own, shared = wide(x.replace_feature(f)).features, small(x).replace_feature(f)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            inside = wide(shared).features
+        inside.zero_()
+        graph.replay()
+        assert torch.equal(inside, own) and torch.equal(wide(shared).features, own)
+        inside.zero_()
+        graph.replay()
+        assert torch.equal(inside, own)
